@@ -2,10 +2,9 @@
 //
 // The reference decodes with one dense GEMM per (source, target) pair over activations that are more
 // than 99 % zeros, each followed by an all-reduce (clt/models/decoder.py:289-295, clt/models/parallel.py:363-383),
-// and then computes the MSE in separate passes (clt/training/losses.py:76-90).  Here one CTA per token walks
-// that token's active (layer, feature, value) entries, reads each feature's contiguous block of decoder rows
-// (feature-major layout [F, R, d]) and accumulates every target layer's reconstruction in registers
-// (the targets are split over four warp groups to keep the register footprint small).
+// and then computes the MSE in separate passes (clt/training/losses.py:76-90).  Here a warp takes one token and one target
+// layer, walks the token's active (layer, feature, value) entries, reads the decoder row of each (feature-major layout
+// [F, R, d]) and accumulates the reconstruction in registers.
 // The epilogue either writes the fp32 partial reconstruction (tensor parallel: summed across ranks before
 // the loss) or, single rank, finishes in place: bias, optional dense addend (skip connection), residual,
 // per-layer squared-error sum in de-normalised units and the bf16 gradient seed  gs = (y_hat - y) * sigma^2.
@@ -109,244 +108,203 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
   }
 }
 
-constexpr int kGroups = 4;  // warp groups per token; group g owns targets t with t % kGroups == g
+// ------------------------------------------------------------------ gather kernels
+// Both kernels below give a warp one token and one slice of d_model and let it walk the token's active entries with
+// plain 16-byte loads, a few decoder rows at a time; the sums stay in registers.  The work is a read of n_entries * targets
+// decoder rows, several times the size of the touched weights, so what bounds it is how many of those reads L2 serves and how
+// many are in flight.  One warp per (token, target) without a shared-memory ring keeps thousands of tokens resident (the ring
+// of a CTA per token held 444), all at the same target, and because the entries of a token are sorted by (layer, feature) they
+// pass over that target's rows together: 7.9 GB from DRAM become 6.3 GB at the GPT-2 shape.
+// Walk configurations.  Few warps with four rows in flight each finish a short list soonest; with thousands of tokens it is the
+// number of tokens on the chip that counts: seven-warp CTAs of 72 registers, two rows in flight, put 28 warps on an SM.
+// GPT-2 shape, 4096 tokens, k = 200: 2.08 ms with 16 warps of four rows, 1.80 ms with 28 of two; 512 tokens, k = 32: 0.119
+// against 0.151 ms.
+constexpr int kWalkWarps = 8;
+constexpr int kFullWarps = 7;
+constexpr long long kRunningMinWarps = 1024;   // below: too few warps, the (token, target) split has L times as many
+constexpr int kFullMinTokens = 2048;             // from here on the chip is full of tokens
+constexpr long long kSplitBelowWarps = 4096;   // fewer (token, target) warps than that leave SMs idle: the entries are split too
 
-// One CTA per token.  The CTA is split into kGroups warp groups of `gthreads` threads; every group walks
-// all entries of the token but only accumulates its own targets (t = g, g + kGroups, ...), so a thread
-// holds TPG x 8 accumulators instead of L x 8 and many more warps fit on an SM (more than 16 layers:
-// blockIdx.y selects the next 16 targets).  Each thread covers 8
-// consecutive elements of d (one 16-byte load per decoder row).
-template <int TPG>
-__global__ void __launch_bounds__(1024) decode_kernel(const DecodeParams p, int gthreads) {
+__device__ __forceinline__ int decode_token(const DecodeParams& p, int i) {
   // Tensor-parallel push: rank r starts with the tokens owned by rank r + 1, so that at any moment the ranks
   // store into different owners instead of all into the same one.
-  const int tok = p.mode == 2 ? int((blockIdx.x + 1LL * ((p.rank + 1) % p.world) * p.rows_per_rank) % p.B) : int(blockIdx.x);
-  const int g = threadIdx.x / gthreads;
-  const int gt = threadIdx.x - g * gthreads;
-  const int e0 = gt * 8;
-  const bool active = e0 < p.d;
-  float acc[TPG][8];
-#pragma unroll
-  for (int j = 0; j < TPG; ++j)
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[j][i] = 0.f;
-  __shared__ float sq_s[kMaxLayers];
-  __shared__ const t16* w_s[kMaxLayers];  // parameter tables in shared memory: indexed per entry
-  __shared__ int rows_s[kMaxLayers];
-  if (threadIdx.x < kMaxLayers) {
-    sq_s[threadIdx.x] = 0.f;
-    w_s[threadIdx.x] = p.w[threadIdx.x];
-    rows_s[threadIdx.x] = p.rows[threadIdx.x];
-  }
-  __syncthreads();
-  const int L = p.L, d = p.d, tying = p.tying;
-  const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
-  const int t_span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + t_span - 1 of a source layer s
+  return p.mode == 2 ? int((i + 1LL * ((p.rank + 1) % p.world) * p.rows_per_rank) % p.B) : i;
+}
 
-  const int b = p.tok_off[tok], e = p.tok_off[tok + 1];
-  if (active) {
-    for (int i = b; i < e; ++i) {
-      const int col = __ldg(p.tcsr_col + i);  // packed by the CSR build: (layer << 24) | feature
-      const float a = __ldg(p.tcsr_val + i);
-      const int s = col >> 24;
-      const int f = col & 0xFFFFFF;
-      if (a == 0.f) continue;
-      if (!clt_in_bounds(s, L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102)) continue;
-      if (tying == 0) {
-        // row (t - s) of feature f; rows of one feature are contiguous
-        const t16* base = w_s[s] + (1LL * f * rows_s[s] - s) * d + e0;
+// acc += a_j * row_j over the entries whose bits are set in `mask` (lane i of the warp holds entry i of the batch: its
+// activation and the address of its decoder row).  The order of the additions is the order of the entries.
+template <int NV, int R>
+__device__ __forceinline__ void gather_rows(uint32_t mask, float a, const t16* row, const int (&e0)[NV], const bool (&act)[NV], float (&acc)[NV][8]) {
+  const uint32_t row_lo = uint32_t(reinterpret_cast<uintptr_t>(row)), row_hi = uint32_t(reinterpret_cast<uintptr_t>(row) >> 32);
+  while (mask != 0u) {
+    uint4 q[R][NV];
+    float w[R];
+    bool have[R];
 #pragma unroll
-        for (int j = 0; j < TPG; ++j) {
-          const int t = g + (blockIdx.y * TPG + j) * kGroups;
-          if (t < L && t >= s && t - s < t_span) fma8(acc[j], a, __ldg(reinterpret_cast<const uint4*>(base + 1LL * t * d)));
-        }
-      } else if (tying == 1) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(w_s[s] + 1LL * f * d + e0));
+    for (int k = 0; k < R; ++k) {
+      have[k] = mask != 0u;
+      const int src = have[k] ? __ffs(mask) - 1 : 0;
+      mask &= mask - 1u;
+      w[k] = __shfl_sync(0xFFFFFFFFu, a, src);
+      const uintptr_t r = (uintptr_t(__shfl_sync(0xFFFFFFFFu, row_hi, src)) << 32) | uintptr_t(__shfl_sync(0xFFFFFFFFu, row_lo, src));
 #pragma unroll
-        for (int j = 0; j < TPG; ++j) {
-          const int t = g + (blockIdx.y * TPG + j) * kGroups;
-          if (t < p.L && t >= s && t - s < t_span) {
-            float av = a;
-            if (p.feat_offset) av += p.feat_offset[1LL * t * p.col_pitch + f];
-            if (p.feat_scale) av *= p.feat_scale[1LL * t * p.col_pitch + f];
-            fma8(acc[j], av, v);
-          }
-        }
-      } else {
+      for (int v = 0; v < NV; ++v)
+        if (have[k] && act[v]) q[k][v] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const t16*>(r) + e0[v]));
+    }
 #pragma unroll
-        for (int j = 0; j < TPG; ++j) {
-          const int t = g + (blockIdx.y * TPG + j) * kGroups;
-          if (t < p.L && t >= s && t - s < t_span) {
-            float av = a;
-            if (p.feat_offset) av += p.feat_offset[1LL * t * p.col_pitch + f];
-            if (p.feat_scale) av *= p.feat_scale[1LL * t * p.col_pitch + f];
-            fma8(acc[j], av, __ldg(reinterpret_cast<const uint4*>(w_s[t] + 1LL * f * d + e0)));
-          }
-        }
+    for (int k = 0; k < R; ++k) {
+      if (have[k]) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+          if (act[v]) fma8(acc[v], w[k], q[k][v]);
       }
     }
-  }
-
-#pragma unroll
-  for (int j = 0; j < TPG; ++j) {
-    const int t = g + (blockIdx.y * TPG + j) * kGroups;  // the same for all lanes of a warp (gthreads is a multiple of 32)
-    if (t >= p.L) continue;
-    float sq = active ? decode_epilogue(p, tok, t, e0, acc[j], loss_scale) : 0.f;
-    if (p.mode == 1) {
-      sq = warp_sum(sq);
-      if ((threadIdx.x & 31) == 0) atomicAdd(&sq_s[t], sq);
-    }
-  }
-  if (p.mode == 1) {
-    __syncthreads();
-    if (threadIdx.x < p.L && sq_s[threadIdx.x] != 0.f) atomicAdd(&p.sq_err[threadIdx.x], double(sq_s[threadIdx.x]));
   }
 }
 
-// Untied decoders, the flagship path: the rows of one active feature for all its targets are one contiguous
-// block of (L - s) * d bf16.  A producer warp streams these blocks into a shared-memory ring with 1-D bulk
-// copies (cp.async.bulk + mbarrier, no multicast); the four consumer groups take their targets' rows from
-// shared memory.  Large contiguous reads and a ring that is always full keep HBM busy, where the per-row
-// register loads of decode_kernel wait on a dependent load chain.  Every mbarrier wait is bounded.
-constexpr int kDecodeStages = 16;  // at most; the launcher picks the depth so that the ring holds a few tens of KB
-
-struct DecodeBulkShared {
-  uint64_t full[kDecodeStages];
-  uint64_t empty[kDecodeStages];
-  float sq_s[kMaxLayers];
-  const t16* w_s[kMaxLayers];
-  int rows_s[kMaxLayers];
-  int abort_flag;
-  int ent_sl[kDecodeStages];    // source layer and activation of the entry in each stage, written by the producer
-  float ent_a[kDecodeStages];
-};
-
-// V: 8-element column chunks per thread (1 for d <= 1024, 2 up to d = 2048: chunk v of thread gt covers columns
-// (v * gthreads + gt) * 8 ...), so that the CTA stays at four groups of at most 128 threads plus the producer warp.
-template <int TPG, int V>
-__global__ void __launch_bounds__(544) decode_bulk_kernel(const DecodeParams p, int gthreads, int stage_bytes, int nstages, int* status) {
-  extern __shared__ __align__(128) uint8_t smem_raw_dec[];  // bulk copies need 16-byte alignment only
-  uint8_t* ring = smem_raw_dec;
-  DecodeBulkShared* sh = reinterpret_cast<DecodeBulkShared*>(ring + size_t(nstages) * stage_bytes);
-  // per-source tied decoders: one row per feature that serves every target >= its source layer
-  const bool shared_row = p.tying == 1;
-  // Tensor-parallel push: rank r starts with the tokens owned by rank r + 1, so that at any moment the ranks
-  // store into different owners instead of all into the same one.
-  const int tok = p.mode == 2 ? int((blockIdx.x + 1LL * ((p.rank + 1) % p.world) * p.rows_per_rank) % p.B) : int(blockIdx.x);
-  const int nconsumer = kGroups * gthreads;
-  const bool is_producer = int(threadIdx.x) >= nconsumer;
-  const int L = p.L, d = p.d;
-  if (threadIdx.x < kMaxLayers) {
-    sh->sq_s[threadIdx.x] = 0.f;
-    sh->w_s[threadIdx.x] = p.w[threadIdx.x];
-    sh->rows_s[threadIdx.x] = p.rows[threadIdx.x];
-  }
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < nstages; ++s) {
-      mbar_init(&sh->full[s], 1);
-      mbar_init(&sh->empty[s], nconsumer / 32);
-    }
-    sh->abort_flag = 0;
-    fence_barrier_init();
-  }
-  __syncthreads();
-  volatile int* abort_flag = &sh->abort_flag;
-  const int b = p.tok_off[tok], e = p.tok_off[tok + 1];
+// One warp (SPLIT = 1) or one CTA of kWalkWarps warps (SPLIT = kWalkWarps: few tokens, the entries of a token are dealt to
+// the warps and the partial sums meet in shared memory) per (token, target, column chunk of NV * 256).  Every tying mode:
+// `tying` only decides which row an entry reads.  blockIdx.y counts the targets from the last one down: the longest
+// lists come first, so that the short ones fill the tail.
+template <int NV, int SPLIT, bool FULL = false>
+__global__ void __launch_bounds__(32 * (FULL ? kFullWarps : kWalkWarps), FULL ? (NV == 4 ? 3 : 4) : (NV >= 3 ? 2 : (NV == 2 ? 3 : 4))) decode_walk_kernel(const DecodeParams p) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = p.L - 1 - int(blockIdx.y);
+  constexpr int kWarps = FULL ? kFullWarps : kWalkWarps;
+  const int slot = SPLIT == 1 ? int(blockIdx.x) * kWarps + warp : int(blockIdx.x);
+  const int d = p.d;
   const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
+  float sq = 0.f;
+  __shared__ float red_s[kWarps];
+  if (slot < p.B) {
+    const int tok = decode_token(p, slot);
+    int e0[NV];
+    bool act[NV];
+    float acc[NV][8];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      e0[v] = ((int(blockIdx.z) * NV + v) * 32 + lane) * 8;
+      act[v] = e0[v] < d;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
+    }
+    const int span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + span - 1 of a source layer s
+    const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
+    int seen = 0;  // SPLIT: entries dealt so far
+    for (int i0 = b; i0 < e; i0 += 32) {
+      const int i = i0 + lane;
+      const int col = i < e ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
+      float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
+      const int s = col >> 24, f = col & 0xFFFFFF;
+      bool use = a != 0.f && s <= t && t - s < span;
+      if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
+      const t16* row = nullptr;
+      if (use) {
+        const int wi = p.tying == 2 ? t : s;
+        row = p.w[wi] + (p.tying == 0 ? 1LL * f * p.rows[s] + (t - s) : 1LL * f) * d;
+        if (p.tying != 0) {
+          if (p.feat_offset) a += p.feat_offset[1LL * t * p.col_pitch + f];
+          if (p.feat_scale) a *= p.feat_scale[1LL * t * p.col_pitch + f];
+        }
+      }
+      uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
+      if (SPLIT > 1) {
+        const int rank = seen + __popc(mask & ((1u << lane) - 1u));
+        seen += __popc(mask);
+        mask = __ballot_sync(0xFFFFFFFFu, use && rank % SPLIT == warp);
+      }
+      gather_rows<NV, FULL ? 2 : 4>(mask, a, row, e0, act, acc);
+    }
+    if (SPLIT == 1) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
+    } else {
+      __shared__ __align__(16) float part[SPLIT > 1 ? SPLIT : 1][SPLIT > 1 ? NV * 256 : 4];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        float4* dst = reinterpret_cast<float4*>(&part[warp][(v * 32 + lane) * 8]);
+        dst[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+        dst[1] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
+      }
+      __syncthreads();
+      for (int c = threadIdx.x; c < NV * 32; c += blockDim.x) {  // one 8-element slice per thread
+        const int ec = (int(blockIdx.z) * NV * 32 + c) * 8;
+        if (ec >= d) continue;
+        float out[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[i] = 0.f;
+#pragma unroll
+        for (int w = 0; w < SPLIT; ++w) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) out[i] += part[w][c * 8 + i];
+        }
+        sq += decode_epilogue(p, tok, t, ec, out, loss_scale);
+      }
+    }
+  }
+  if (p.mode == 1) {
+    // one shared word per warp and one global atomic per CTA: all warps of the CTA work on the same target
+    sq = warp_sum(sq);
+    if (lane == 0) red_s[warp] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float tot = 0.f;
+      for (int w = 0; w < kWarps; ++w) tot += red_s[w];
+      if (tot != 0.f) atomicAdd(&p.sq_err[t], double(tot));
+    }
+  }
+}
 
-  if (is_producer) {
-    if (threadIdx.x == nconsumer) {
-      int issued = 0;
-      int col_next = b < e ? __ldg(p.tcsr_col + b) : 0;
-      float a_next = b < e ? __ldg(p.tcsr_val + b) : 0.f;
-      for (int i = b; i < e; ++i, ++issued) {
-        const int st = issued % nstages;
-        const uint32_t ph = (issued / nstages) & 1;
-        const int col = col_next;
-        float a = a_next;
-        if (i + 1 < e) {  // the next entry's index is in flight while this stage is waited for
-          col_next = __ldg(p.tcsr_col + i + 1);
-          a_next = __ldg(p.tcsr_val + i + 1);
-        }
-        if (!mbar_wait(&sh->empty[st], ph ^ 1, abort_flag)) break;
-        int sl = col >> 24, f = col & 0xFFFFFF;
-        if (!clt_in_bounds(sl, L, p.dbg_status, 103) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 104)) { sl = 0; f = 0; a = 0.f; }  // decode a harmless row with weight zero
-        const int R = sh->rows_s[sl];
-        const int r_eff = (p.rows_limit > 0 && p.rows_limit < R) ? p.rows_limit : R;
-        const uint32_t bytes = uint32_t(r_eff) * uint32_t(d) * 2u;
-        sh->ent_sl[st] = sl;
-        sh->ent_a[st] = a;
-        mbar_expect_tx(&sh->full[st], bytes);  // release: the two words above are visible to whoever sees the phase
-        bulk_load_1d(ring + size_t(st) * stage_bytes, sh->w_s[sl] + 1LL * f * R * d, bytes, &sh->full[st]);
-      }
-      if (*abort_flag) {
-        // give copies already issued a bounded chance to land before the CTA retires
-        const int first = issued > nstages ? issued - nstages : 0;
-        for (int j = first; j < issued; ++j) {
-          const long long start = clock64();
-          while (!mbar_try_wait(&sh->full[j % nstages], (j / nstages) & 1))
-            if (clock64() - start > kWaitTimeoutCycles) break;
-        }
-      }
+// Per-source tied decoders without affine terms: the row of feature (s, f) serves every target t >= s with the same weight,
+// so the reconstruction of target t is the one of t - 1 plus the entries of layer t.  One warp per (token, column chunk)
+// reads every row once and finishes a target whenever a layer's entries are in.  The list is scanned once per layer
+// (coalesced, a few hundred bytes), which makes the result independent of how the entries of a token are ordered.
+template <int NV>
+__global__ void __launch_bounds__(32 * kWalkWarps, NV >= 2 ? 2 : 3) decode_running_kernel(const DecodeParams p) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int slot = int(blockIdx.x) * kWalkWarps + warp;
+  const int d = p.d;
+  const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
+  __shared__ float sq_s[kMaxLayers];
+  if (threadIdx.x < kMaxLayers) sq_s[threadIdx.x] = 0.f;
+  __syncthreads();
+  if (slot < p.B) {
+    const int tok = decode_token(p, slot);
+    int e0[NV];
+    bool act[NV];
+    float acc[NV][8];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      e0[v] = ((int(blockIdx.y) * NV + v) * 32 + lane) * 8;
+      act[v] = e0[v] < d;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
     }
-  } else {
-    const int g = threadIdx.x / gthreads;
-    const int gt = threadIdx.x - g * gthreads;
-    const int lane = threadIdx.x & 31;
-    int e0[V];
-    bool active[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) { e0[v] = (v * gthreads + gt) * 8; active[v] = e0[v] < d; }
-    float acc[TPG][V][8];
-#pragma unroll
-    for (int j = 0; j < TPG; ++j)
-#pragma unroll
-      for (int v = 0; v < V; ++v)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[j][v][i] = 0.f;
-    int it = 0;
-    bool ok = true;
-    const int t_span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;
-    for (int i = b; i < e; ++i, ++it) {
-      const int st = it % nstages;
-      const uint32_t ph = (it / nstages) & 1;
-      if (!mbar_wait(&sh->full[st], ph, abort_flag)) { ok = false; break; }
-      const int sl = sh->ent_sl[st];
-      const float a = sh->ent_a[st];
-      if (a != 0.f) {
-        const t16* rows = reinterpret_cast<const t16*>(ring + size_t(st) * stage_bytes);
-#pragma unroll
-        for (int j = 0; j < TPG; ++j) {
-          const int t = g + (blockIdx.y * TPG + j) * kGroups;
-          if (t < L && t >= sl && t - sl < t_span) {
-            const t16* row = rows + (shared_row ? 0 : (t - sl) * d);
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-              if (active[v]) fma8(acc[j][v], a, *reinterpret_cast<const uint4*>(row + e0[v]));
-          }
-        }
+    const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
+    for (int t = 0; t < p.L; ++t) {
+      for (int i0 = b; i0 < e; i0 += 32) {
+        const int i = i0 + lane;
+        const int col = i < e ? __ldg(p.tcsr_col + i) : 0;
+        const float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
+        const int f = col & 0xFFFFFF;
+        bool use = a != 0.f && (col >> 24) == t;
+        if (use && !clt_in_bounds(f, p.col_pitch, p.dbg_status, 103)) use = false;
+        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
+        if (mask != 0u) gather_rows<NV, 4>(mask, a, p.w[t] + 1LL * f * d, e0, act, acc);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->empty[st]);  // this warp is done with the stage
-    }
-    // one warp-level sum and one shared atomic per warp and target (the lanes of a warp share their targets)
-#pragma unroll
-    for (int j = 0; j < TPG; ++j) {
-      const int t = g + (blockIdx.y * TPG + j) * kGroups;
-      if (t >= L) continue;
       float sq = 0.f;
 #pragma unroll
-      for (int v = 0; v < V; ++v)
-        if (ok && active[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[j][v], loss_scale);
+      for (int v = 0; v < NV; ++v)
+        if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
       if (p.mode == 1) {
         sq = warp_sum(sq);
-        if (lane == 0) atomicAdd(&sh->sq_s[t], sq);
+        if (lane == 0) atomicAdd(&sq_s[t], sq);
       }
     }
   }
   __syncthreads();
-  if (p.mode == 1 && threadIdx.x < L && sh->sq_s[threadIdx.x] != 0.f) atomicAdd(&p.sq_err[threadIdx.x], double(sh->sq_s[threadIdx.x]));
-  if (threadIdx.x == 0 && sh->abort_flag && status != nullptr) atomicCAS(status, STATUS_OK, STATUS_WAIT_TIMEOUT);
+  if (p.mode == 1 && threadIdx.x < p.L && sq_s[threadIdx.x] != 0.f) atomicAdd(&p.sq_err[threadIdx.x], double(sq_s[threadIdx.x]));
 }
 
 // Epilogue for the tensor-parallel path, run after the partial reconstructions were summed across ranks:
@@ -490,55 +448,34 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   for (int i = 0; i < 8; ++i) p.stage_peers[i] = static_cast<float*>(a->stage_peers[i]);
   p.rows_per_rank = a->rows_per_rank; p.rank = a->rank; p.world = a->world;
   p.ctl = a->ctl; p.rows_limit = a->rows_limit; p.dbg_status = a->status;
-  int gthreads = ((a->d / 8 + 31) / 32) * 32;
-  int threads = gthreads * kGroups;
-  if (threads > 1024) return -1;
-  const int tpg = (a->L + kGroups - 1) / kGroups;  // targets per warp group
-  int max_rows = 0;
-  for (int i = 0; i < a->L; ++i) max_rows = a->rows[i] > max_rows ? a->rows[i] : max_rows;
-  if (a->rows_limit > 0 && a->rows_limit < max_rows) max_rows = a->rows_limit;
-  const int stage_bytes = ((max_rows * a->d * 2 + 127) / 128) * 128;
-  // ring depth: four stages for the long rows of untied decoders, more for short rows so that the copies in flight per
-  // CTA stay in the tens of kilobytes
-  int nstages = 4;
-  while (nstages < kDecodeStages && nstages * stage_bytes < 24 * 1024) nstages *= 2;
-  // long rows (d_model 2048 with many target layers): fewer, larger stages; two column chunks per thread
-  while (nstages > 2 && size_t(nstages) * stage_bytes + sizeof(DecodeBulkShared) + 256 > 200 * 1024) --nstages;
-  const size_t smem = size_t(nstages) * stage_bytes + sizeof(DecodeBulkShared) + 256;
-  const bool plain_tied = a->tying == 1 && a->feat_offset == nullptr && a->feat_scale == nullptr;
-  const int vchunks = a->d > 1024 ? 2 : 1;
-  const int bulk_gthreads = vchunks == 2 ? ((a->d / 16 + 31) / 32) * 32 : gthreads;
-  const bool bulk = (a->tying == 0 || plain_tied) && a->status != nullptr && tpg <= 4 && smem <= 200 * 1024 && bulk_gthreads * kGroups + 32 <= 544;
-  if (bulk) {
-    gthreads = bulk_gthreads;
-    threads = gthreads * kGroups;
-    static size_t attr_set[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    auto launch = [&](auto kern) -> int {
-      size_t& have = attr_set[tpg + 5 * (vchunks - 1)];
-      if (have < smem) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
-        have = smem;
-      }
-      kern<<<dim3(a->B, 1), threads + 32, smem, st>>>(p, gthreads, stage_bytes, nstages, a->status);
-      return 0;
-    };
-    int rc = 0;
-    if (vchunks == 1) {
-      if (tpg <= 1) rc = launch(decode_bulk_kernel<1, 1>);
-      else if (tpg == 2) rc = launch(decode_bulk_kernel<2, 1>);
-      else if (tpg == 3) rc = launch(decode_bulk_kernel<3, 1>);
-      else rc = launch(decode_bulk_kernel<4, 1>);
-    } else {
-      if (tpg <= 1) rc = launch(decode_bulk_kernel<1, 2>);
-      else if (tpg == 2) rc = launch(decode_bulk_kernel<2, 2>);
-      else if (tpg == 3) rc = launch(decode_bulk_kernel<3, 2>);
-      else rc = launch(decode_bulk_kernel<4, 2>);
-    }
-    if (rc != 0) return rc;
-  } else if (tpg <= 1) decode_kernel<1><<<dim3(a->B, 1), threads, 0, st>>>(p, gthreads);
-  else if (tpg == 2) decode_kernel<2><<<dim3(a->B, 1), threads, 0, st>>>(p, gthreads);
-  else if (tpg == 3) decode_kernel<3><<<dim3(a->B, 1), threads, 0, st>>>(p, gthreads);
-  else decode_kernel<4><<<dim3(a->B, (tpg + 3) / 4), threads, 0, st>>>(p, gthreads);  // 16 targets per pass
+  if (a->B <= 0 || a->L <= 0) return 0;
+  // 16-byte vectors per lane: the whole row up to d_model 1024 (a warp then reads an entry's row in one go), half of it above
+  const int chunks = a->d > 1024 ? 2 : 1;
+  const int nv = (a->d / 8 + 32 * chunks - 1) / (32 * chunks);
+  const bool plain_tied = a->tying == 1 && a->feat_offset == nullptr && a->feat_scale == nullptr && a->rows_limit <= 0;
+  auto pick = [&](auto k1, auto k2, auto k3, auto k4, dim3 grid, int block) {
+    if (nv <= 1) k1<<<grid, block, 0, st>>>(p);
+    else if (nv == 2) k2<<<grid, block, 0, st>>>(p);
+    else if (nv == 3) k3<<<grid, block, 0, st>>>(p);
+    else k4<<<grid, block, 0, st>>>(p);
+  };
+  const int token_ctas = (a->B + kWalkWarps - 1) / kWalkWarps;
+  const int run_chunks = (a->d + 511) / 512;  // at most two vectors per lane: the sums stay live across the epilogues of all targets
+  const int block = 32 * kWalkWarps;
+  if (plain_tied && 1LL * a->B * run_chunks >= kRunningMinWarps) {
+    const dim3 grid(token_ctas, run_chunks);
+    if (a->d <= 256) decode_running_kernel<1><<<grid, block, 0, st>>>(p);
+    else decode_running_kernel<2><<<grid, block, 0, st>>>(p);
+  } else if (nv >= 3 && a->B >= kFullMinTokens) {
+    const dim3 grid((a->B + kFullWarps - 1) / kFullWarps, a->L, chunks);
+    if (nv == 3) decode_walk_kernel<3, 1, true><<<grid, 32 * kFullWarps, 0, st>>>(p);
+    else decode_walk_kernel<4, 1, true><<<grid, 32 * kFullWarps, 0, st>>>(p);
+  } else if (1LL * a->B * a->L * chunks >= kSplitBelowWarps) {
+    pick(decode_walk_kernel<1, 1>, decode_walk_kernel<2, 1>, decode_walk_kernel<3, 1>, decode_walk_kernel<4, 1>, dim3(token_ctas, a->L, chunks), block);
+  } else {
+    pick(decode_walk_kernel<1, kWalkWarps>, decode_walk_kernel<2, kWalkWarps>, decode_walk_kernel<3, kWalkWarps>, decode_walk_kernel<4, kWalkWarps>,
+         dim3(a->B, a->L, chunks), block);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -1323,6 +1323,102 @@ __global__ void __launch_bounds__(256) csr_sort_long_segments_kernel(const int* 
   }
 }
 
+// Bitonic network on n 64-bit words in shared memory or on (key, value) pairs in global memory, by all threads of the CTA.  Every
+// comparator puts the smaller key at the lower index (the first step of a merge pairs mirrored positions), so the virtual
+// padding to a power of two, which stands for +infinity at the end of the array, never has to move.
+template <typename CmpSwap>
+__device__ __forceinline__ void bitonic_cta(int n, CmpSwap cmp_swap) {
+  int p2 = 1;
+  while (p2 < n) p2 <<= 1;
+  for (int size = 2; size <= p2; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      __syncthreads();
+      for (int i = threadIdx.x; i < p2 / 2; i += blockDim.x) {
+        const int j = i & (stride - 1);
+        const int lo = 2 * i - j;
+        const int hi = stride == (size >> 1) ? lo + size - 1 - 2 * j : lo + stride;
+        if (hi < n) cmp_swap(lo, hi);
+      }
+    }
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void sort_words_cta(unsigned long long* w, int n) {
+  bitonic_cta(n, [&](int lo, int hi) {
+    const unsigned long long x = w[lo], y = w[hi];
+    if (x > y) { w[lo] = y; w[hi] = x; }
+  });
+}
+__device__ __forceinline__ void sort_pairs_cta(int* k, float* v, int n) {
+  bitonic_cta(n, [&](int lo, int hi) {
+    const int ka = k[lo], kb = k[hi];
+    if (ka > kb) {
+      k[lo] = kb; k[hi] = ka;
+      const float t = v[lo]; v[lo] = v[hi]; v[hi] = t;
+    }
+  });
+}
+__device__ __forceinline__ unsigned long long pack_entry(int key, float val) { return ((unsigned long long)(unsigned int)key << 32) | __float_as_uint(val); }
+
+// Token segments: one CTA per token sorts its entries by (layer, feature).  Up to kTokenRankCap entries every thread counts how
+// many keys are below its own (broadcast reads of shared memory, no barrier in between: 1 us where the 36 barriers of a
+// network on 256 entries take ten) and stores its entry at that rank; more entries, or equal keys, go through the
+// network in shared memory, and lists beyond its buffer through the one in global memory.  The order lets the decode's tokens
+// pass over the decoder rows together (L2) and fixes the order of its sums.
+constexpr int kTokenSortCap = 2048;
+constexpr int kTokenRankCap = 512;
+__global__ void __launch_bounds__(256) csr_sort_token_segments_kernel(const int* __restrict__ off, int* __restrict__ key, float* __restrict__ val) {
+  __shared__ unsigned long long w[kTokenSortCap];
+  const int b = off[blockIdx.x], n = off[blockIdx.x + 1] - b;
+  if (n <= 1) return;
+  if (n > kTokenSortCap) {
+    sort_pairs_cta(key + b, val + b, n);
+    return;
+  }
+  if (n <= kTokenRankCap) {
+    __shared__ __align__(16) int keys[kTokenRankCap];
+    __shared__ int taken[kTokenRankCap];
+    int mine[2];
+    float v[2];
+    int rank[2] = {0, 0};
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int i = threadIdx.x + 256 * m;
+      mine[m] = i < n ? key[b + i] : 0x7FFFFFFF;
+      v[m] = i < n ? val[b + i] : 0.f;
+      keys[i] = mine[m];
+      taken[i] = 0;
+    }
+    __syncthreads();
+    const int4* k4 = reinterpret_cast<const int4*>(keys);
+    if (n <= 256) {
+      for (int j = 0; j < (n + 3) / 4; ++j) {
+        const int4 q = k4[j];
+        rank[0] += (q.x < mine[0]) + (q.y < mine[0]) + (q.z < mine[0]) + (q.w < mine[0]);
+      }
+    } else {
+      for (int j = 0; j < (n + 3) / 4; ++j) {
+        const int4 q = k4[j];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) rank[m] += (q.x < mine[m]) + (q.y < mine[m]) + (q.z < mine[m]) + (q.w < mine[m]);
+      }
+    }
+    bool clash = false;  // equal keys share a rank
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+      if (threadIdx.x + 256 * m < n) clash |= atomicExch(&taken[rank[m]], 1) != 0;
+    if (!__syncthreads_or(clash)) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+        if (threadIdx.x + 256 * m < n) { key[b + rank[m]] = mine[m]; val[b + rank[m]] = v[m]; }
+      return;
+    }
+  }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) w[i] = pack_entry(key[b + i], val[b + i]);
+  sort_words_cta(w, n);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) { key[b + i] = int(w[i] >> 32); val[b + i] = __uint_as_float((unsigned int)(w[i] & 0xFFFFFFFFULL)); }
+}
+
 // Dead-feature counters: +1 per step, reset where the feature fired (reference trainer.py:693-712).
 __global__ void __launch_bounds__(256) dead_counter_kernel(long long* __restrict__ counter, unsigned char* __restrict__ fired, int n) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1629,10 +1725,8 @@ extern "C" int clt_build_csr(const CltCsrArgs* a, cudaStream_t st) {
   launch_exclusive_scan(a->feat_cnt, a->feat_off, a->feat_cursor, a->num_cols, st);
   csr_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->feat_cursor,
                                              a->tcsr_col, a->tcsr_val, a->fcsr_tok, a->fcsr_val, a->col_pitch, a->num_tokens, a->num_cols);
-  if (a->sort_segments & 1) {
-    csr_sort_segments_kernel<<<(a->num_tokens + 255) / 256, 256, 0, st>>>(a->tok_off, a->num_tokens, a->tcsr_col, a->tcsr_val);
-    csr_sort_long_segments_kernel<<<(a->num_tokens + 255) / 256 < 1184 ? (a->num_tokens + 255) / 256 : 1184, 256, 0, st>>>(a->tok_off, a->num_tokens, a->tcsr_col, a->tcsr_val);
-  }
+  if ((a->sort_segments & 1) && a->num_tokens > 0)
+    csr_sort_token_segments_kernel<<<a->num_tokens, 256, 0, st>>>(a->tok_off, a->tcsr_col, a->tcsr_val);
   if (a->sort_segments & 2) {
     csr_sort_segments_kernel<<<(a->num_cols + 255) / 256, 256, 0, st>>>(a->feat_off, a->num_cols, a->fcsr_tok, a->fcsr_val);
     csr_sort_long_segments_kernel<<<(a->num_cols + 255) / 256 < 1184 ? (a->num_cols + 255) / 256 : 1184, 256, 0, st>>>(a->feat_off, a->num_cols, a->fcsr_tok, a->fcsr_val);
@@ -1709,10 +1803,7 @@ extern "C" int clt_build_csr_static(const int* ent_tok, const int* ent_col, cons
   exclusive_scan_kernel<<<1, 1024, 0, stream>>>(feat_cnt, feat_off, feat_cursor, num_cols);
   csr_scatter_kernel<<<blocks, 256, 0, stream>>>(ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cursor, feat_cursor, tcsr_col, tcsr_val,
                                                  fcsr_tok, fcsr_val, col_pitch, num_tokens, num_cols);
-  if (sort_segments & 1) {
-    csr_sort_segments_kernel<<<(num_tokens + 255) / 256, 256, 0, stream>>>(tok_off, num_tokens, tcsr_col, tcsr_val);
-    csr_sort_long_segments_kernel<<<num_tokens < 1184 ? num_tokens : 1184, 256, 0, stream>>>(tok_off, num_tokens, tcsr_col, tcsr_val);
-  }
+  if (sort_segments & 1) csr_sort_token_segments_kernel<<<num_tokens, 256, 0, stream>>>(tok_off, tcsr_col, tcsr_val);
   if (sort_segments & 2) {
     csr_sort_segments_kernel<<<(num_cols + 255) / 256, 256, 0, stream>>>(feat_off, num_cols, fcsr_tok, fcsr_val);
     csr_sort_long_segments_kernel<<<num_cols < 1184 ? num_cols : 1184, 256, 0, stream>>>(feat_off, num_cols, fcsr_tok, fcsr_val);

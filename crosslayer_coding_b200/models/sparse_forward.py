@@ -146,7 +146,7 @@ class SparseForward:
         self.feat_cnt.zero_()
         e.build_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.feat_cnt, self.tok_off,
                     self.feat_off, self.tok_cursor, self.feat_cursor, self.tcsr_col, self.tcsr_val, self.fcsr_tok, self.fcsr_val,
-                    None, 2, self.Fl)
+                    None, 3, self.Fl)
 
     # ------------------------------------------------------------------ decode
     @torch.no_grad()

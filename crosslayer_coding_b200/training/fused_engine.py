@@ -405,7 +405,7 @@ class FusedBatchTopKEngine:
         self.ext.build_csr(
             self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols,
             self.tok_cnt, self.feat_cnt, self.tok_off, self.feat_off, self.tok_cursor, self.feat_cursor,
-            self.tcsr_col, self.tcsr_val, self.fcsr_tok, self.fcsr_val, self.fired, 2, self.Fl,
+            self.tcsr_col, self.tcsr_val, self.fcsr_tok, self.fcsr_val, self.fired, 3, self.Fl,
         )
 
     def encode_select(self, X: torch.Tensor, fresh: bool = True) -> None:

@@ -1,0 +1,116 @@
+"""Kernels of the sparse step at the sizes where their dispatch changes, each against a plain PyTorch restatement."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+I32, F32 = torch.int32, torch.float32
+
+
+@pytest.fixture(scope="module")
+def ext():
+    from crosslayer_coding_b200.ops import ext as ext_mod
+
+    return ext_mod.load()
+
+
+def _dev():
+    return torch.device("cuda:0")
+
+
+def _csr(ext, tok, col, val, B, ncols, pitch, sort=3):
+    """Both CSR views of an entry list, as the engine builds them."""
+    dev, n = tok.device, tok.numel()
+    ctl = torch.zeros(16, dtype=torch.int64, device=dev)
+    ctl[3] = n
+    z = lambda k, dt=I32: torch.zeros(max(k, 1), dtype=dt, device=dev)  # noqa: E731
+    r = dict(tok_off=z(B + 1), feat_off=z(ncols + 1), tcsr_col=z(n), tcsr_val=z(n, F32), fcsr_tok=z(n), fcsr_val=z(n, F32))
+    ext.build_csr(tok, col, val, ctl, B, ncols, z(B), z(ncols), r["tok_off"], r["feat_off"], z(B), z(ncols), r["tcsr_col"], r["tcsr_val"],
+                  r["fcsr_tok"], r["fcsr_val"], None, sort, pitch)
+    return r
+
+
+def _entries(g, L, B, F, n, dev):
+    """n distinct (token, layer, feature) entries in random order; every third value negative, a few exactly zero."""
+    flat = torch.randperm(B * L * F, generator=g)[:n]
+    val = torch.randn(n, generator=g)
+    val[::17] = 0.0
+    return (flat // (L * F)).to(I32).to(dev), (flat % (L * F)).to(I32).to(dev), val.to(dev)
+
+
+# d: one, two, three and four 16-byte vectors per lane, partly filled ones, two column chunks; B: the split walk (few
+# (token, target) warps), the walk and (per source) the running sum, each with a last CTA that is not full
+@pytest.mark.parametrize("tying,affine", [(0, False), (1, False), (1, True), (2, False), (2, True)])
+@pytest.mark.parametrize("L,B,d", [(2, 3, 8), (3, 5, 264), (12, 2, 768), (4, 1030, 256), (5, 1027, 520), (2, 2055, 768), (3, 1500, 1024), (2, 2051, 1032), (3, 700, 2048)])
+def test_gather_decode_matches_dense(ext, L, B, d, tying, affine):
+    dev = _dev()
+    g = torch.Generator().manual_seed(L * 1000 + B + d)
+    F = 24
+    tok, col, val = _entries(g, L, B, F, min(B * L * F, 7 * B), dev)
+    rows = [L - s if tying == 0 else 1 for s in range(L)]
+    W = [(torch.randn(F, r, d, generator=g) / 4).bfloat16().to(dev) for r in rows]
+    off = torch.randn(L, F, generator=g).to(dev) if affine else None
+    sc = torch.randn(L, F, generator=g).to(dev) if affine else None
+    bias = torch.randn(L, d, generator=g).to(dev)
+    y = torch.randn(L, B, d, generator=g).bfloat16().to(dev)
+    sigma = (0.5 + torch.rand(L, d, generator=g)).to(dev)
+    acts = torch.zeros(L, B, F, device=dev, dtype=torch.float64)
+    acts[(col // F).long(), tok.long(), (col % F).long()] = val.double()
+    want = torch.zeros(L, B, d, device=dev, dtype=torch.float64)
+    for t in range(L):
+        for s in range(t + 1):
+            a = acts[s]
+            if affine:
+                a = torch.where(a != 0, (a + off[t].double()) * sc[t].double(), a)
+            w = W[s][:, t - s] if tying == 0 else W[s if tying == 1 else t][:, 0]
+            want[t] += a @ w.double()
+    want += bias.double()[:, None, :]
+    status = torch.zeros(4, dtype=I32, device=dev)
+    for sort in (3, 0):  # the order of a token's entries changes only the order of the sums
+        c = _csr(ext, tok, col, val, B, L * F, F, sort)
+        yhat = torch.full((L, B, d), float("nan"), device=dev)
+        gs = torch.empty(L, B, d, device=dev, dtype=torch.bfloat16)
+        sq = torch.zeros(L, device=dev, dtype=torch.float64)
+        ext.sparse_decode(W, L, B, d, F, tying, c["tok_off"], c["tcsr_col"], c["tcsr_val"], off, sc, None, bias, None, y, sigma, gs, yhat, sq, 1, [], 0, 0,
+                          status)
+        # fp32 sums of at most a few dozen products: 2^-24 each on terms of the size of the result
+        scale = want.abs().max()
+        assert (yhat.double() - want).abs().max() < 1e-5 * scale
+        r = (want - y.double()) * sigma.double()[:, None]
+        assert torch.allclose(sq, r.square().sum((1, 2)), rtol=1e-5)
+        # bf16 keeps 8 bits: half a unit in the last place of the value, plus the fp32 error of the sum
+        assert ((gs.double() - r * sigma.double()[:, None]).abs() <= 2 ** -8 * (r * sigma.double()[:, None]).abs() + 1e-4).all()
+        # partial sums only (the tensor-parallel form before the exchange)
+        part = torch.full((L, B, d), float("nan"), device=dev)
+        ext.sparse_decode(W, L, B, d, F, tying, c["tok_off"], c["tcsr_col"], c["tcsr_val"], off, sc, part, None, None, None, None, None, None, None, 0, [], 0,
+                          0, status)
+        assert (part.double() + bias.double()[:, None] - want).abs().max() < 1e-5 * scale
+    assert int(status[0]) == 0
+
+
+# long segments in shared memory, ranges beyond it, one feature per CTA, tokens beyond the token sort's buffer
+@pytest.mark.parametrize("B,L,F,n", [(40, 2, 300, 900), (3000, 1, 8, 20000), (5000, 1, 2, 9000), (9000, 1, 3, 27000), (2, 2, 4000, 9000), (700, 3, 512, 200000)])
+def test_csr_segments_are_sorted(ext, B, L, F, n):
+    dev = _dev()
+    g = torch.Generator().manual_seed(n)
+    tok, col, val = _entries(g, L, B, F, n, dev)
+    c = _csr(ext, tok, col, val, B, L * F, F)
+    order = torch.argsort(col.long() * B + tok.long())
+    assert torch.equal(c["fcsr_tok"], tok[order]) and torch.equal(c["fcsr_val"], val[order])
+    order = torch.argsort(tok.long() * (L * F) + col.long())
+    packed = ((col // F) << 24) | (col % F)
+    assert torch.equal(c["tcsr_col"], packed[order].to(I32)) and torch.equal(c["tcsr_val"], val[order])
+    assert torch.equal(c["feat_off"].cpu(), torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(col.cpu().long(), minlength=L * F).cumsum(0)]).to(I32))
+    assert torch.equal(c["tok_off"].cpu(), torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(tok.cpu().long(), minlength=B).cumsum(0)]).to(I32))
+
+
+def test_equal_keys_in_a_token_segment_are_all_kept(ext):
+    """A caller's list may name one column twice for a token: both entries stay."""
+    dev = _dev()
+    tok = torch.zeros(40, dtype=I32, device=dev)
+    col = torch.tensor([7] * 20 + list(range(20)), dtype=I32, device=dev)
+    val = torch.arange(40, device=dev).float()
+    c = _csr(ext, tok, col, val, 1, 64, 64)
+    assert torch.equal(c["tcsr_col"].long(), torch.sort(col.long()).values)
+    assert torch.equal(torch.sort(c["tcsr_val"]).values, val)
