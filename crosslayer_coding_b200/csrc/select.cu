@@ -628,12 +628,17 @@ __device__ __forceinline__ void token_rows_scan(const t16* __restrict__ x, const
 
 __global__ void __launch_bounds__(256) token_topk_kernel(const t16* __restrict__ x, const float* __restrict__ mean,
                                                            const float* __restrict__ rstd, ScanGeom g, int col_pitch, int f_valid, int k,
-                                                           long long* __restrict__ ctl, Lists o, int* __restrict__ status) {
+                                                           long long* __restrict__ ctl, Lists o, int* __restrict__ status, int only_marked) {
   extern __shared__ uint8_t tk_smem[];
   TokenTopkShared* sh = reinterpret_cast<TokenTopkShared*>(tk_smem);
   const int tok0 = blockIdx.x * kTokPerCta;
   const int ntok = min(kTokPerCta, g.B - tok0);
   const int tid = threadIdx.x;
+  if (only_marked) {  // every thread reads the marks before any of them is overwritten
+    bool any = false;
+    for (int t = 0; t < ntok; ++t) any |= o.ent_tok[1LL * (tok0 + t) * k] < 0;
+    if (!__syncthreads_or(any)) return;
+  }
   if (tid < kTokPerCta) { sh->prefix[tid] = 0; sh->mask[tid] = 0; sh->need[tid] = (unsigned int)k; sh->emitted[tid] = 0; sh->nties[tid] = 0; }
   if (blockIdx.x == 0 && tid == 0) ctl[CTL_NUM_ENTRIES] = 1LL * g.B * k;
   // ---- exact k-th largest key per token: radix select, most significant digits first
@@ -696,6 +701,156 @@ __global__ void __launch_bounds__(256) token_topk_kernel(const t16* __restrict__
       if (rank < need && above + rank < k) {
         const long long q = 1LL * (tok0 + t) * k + above + rank;
         o.ent_tok[q] = tok0 + t; o.ent_col[q] = ci; o.ent_val[q] = sh->tie_val[t][i];
+      }
+    }
+  }
+}
+
+// The same selection with one scan of the rows instead of four.  A bound from below for a token's k-th largest key comes from
+// a sample of its columns (every step-th block of 2048): every thread keeps the largest key of kTkSlots interleaved parts of
+// the sample, and the k-th largest of those kTkMaxima maxima is reached by at least k elements.  One scan then collects what
+// is at or above the bound (about step * k elements) and the exact cut is searched in that short list, whose 64-bit words
+// (key, inverted column) are distinct and order ties by the lowest index.  A token whose list overflows is marked by a token
+// index of -1 in its first entry, and the radix kernel above takes it.  TPC tokens per CTA share the loads of the column
+// statistics.
+constexpr int kTkSlots = 4;
+constexpr int kTkThreads = 256;
+constexpr int kTkMaxima = kTkSlots * kTkThreads;
+constexpr int kTkList = 2048;
+
+template <int TPC>
+struct TokenListShared {
+  union {
+    uint32_t maxima[TPC][kTkMaxima];
+    unsigned long long list[TPC][kTkList];
+  } u;
+  uint32_t bound[TPC];
+  int n[TPC];
+  unsigned long long cut[TPC];
+  int out[TPC];
+};
+
+template <int TPC, typename Fn>
+__device__ __forceinline__ void token_keys_scan(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, const ScanGeom& g,
+                                                int tok0, int ntok, int groups, int step, Fn fn) {
+  // groups of 8 columns, counted over all layers; 8 elements of TPC tokens per thread and step
+  const int per_layer = g.F / 8;
+  int it = 0;
+  for (int q = int(threadIdx.x); q < groups; q += kTkThreads * step, ++it) {
+    const int l = q / per_layer, c0 = (q - l * per_layer) * 8;
+    float mu[8], rs[8];
+    load_cols8(mean + 1LL * l * g.sp + c0, mu);
+    load_cols8(rstd + 1LL * l * g.sp + c0, rs);
+    uint4 v[TPC];
+#pragma unroll
+    for (int t = 0; t < TPC; ++t)
+      v[t] = t < ntok ? __ldg(reinterpret_cast<const uint4*>(x + 1LL * l * g.layer_stride + 1LL * (tok0 + t) * g.ld + c0)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int t = 0; t < TPC; ++t) {
+      if (t < ntok) {
+        const uint32_t u[4] = {v[t].x, v[t].y, v[t].z, v[t].w};
+        uint32_t key[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) key[j] = float_to_key((((j & 1) ? t16_hi(u[j >> 1]) : t16_lo(u[j >> 1])) - mu[j]) * rs[j]);
+        fn(t, l, c0, it, key);
+      }
+    }
+  }
+}
+
+template <int TPC>
+__global__ void __launch_bounds__(kTkThreads) token_topk_list_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd,
+                                                                     ScanGeom g, int col_pitch, int f_valid, int k, int step, long long* __restrict__ ctl, Lists o) {
+  extern __shared__ __align__(16) uint8_t tl_smem[];
+  TokenListShared<TPC>* sh = reinterpret_cast<TokenListShared<TPC>*>(tl_smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tok0 = blockIdx.x * TPC;
+  const int ntok = min(TPC, g.B - tok0);
+  if (blockIdx.x == 0 && tid == 0) ctl[CTL_NUM_ENTRIES] = 1LL * g.B * k;
+  const int groups = g.L * (g.F / 8);
+  // ---- bound from the sample
+  uint32_t best[TPC][kTkSlots];
+#pragma unroll
+  for (int t = 0; t < TPC; ++t)
+#pragma unroll
+    for (int i = 0; i < kTkSlots; ++i) best[t][i] = 0;
+  token_keys_scan<TPC>(x, mean, rstd, g, tok0, ntok, groups, step, [&](int t, int, int c0, int it, const uint32_t (&key)[8]) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = max(m, c0 + j < f_valid ? key[j] : 0u);
+    const int slot = it % kTkSlots;
+#pragma unroll
+    for (int i = 0; i < kTkSlots; ++i)
+      if (i == slot) best[t][i] = max(best[t][i], m);
+  });
+#pragma unroll
+  for (int t = 0; t < TPC; ++t)
+#pragma unroll
+    for (int i = 0; i < kTkSlots; ++i) sh->u.maxima[t][i * kTkThreads + tid] = best[t][i];
+  __syncthreads();
+  if (warp < ntok) {
+    // largest key with zero low bits that at least k maxima reach
+    uint32_t bound = 0;
+    for (int bit = 31; bit >= 12; --bit) {
+      const uint32_t trial = bound | (1u << bit);
+      int cnt = 0;
+      for (int i = lane; i < kTkMaxima; i += 32) cnt += sh->u.maxima[warp][i] >= trial ? 1 : 0;
+      if (__reduce_add_sync(0xFFFFFFFFu, cnt) >= k) bound = trial;
+    }
+    if (lane == 0) { sh->bound[warp] = bound; sh->n[warp] = 0; sh->out[warp] = 0; }
+  }
+  __syncthreads();
+  uint32_t bound[TPC];
+#pragma unroll
+  for (int t = 0; t < TPC; ++t) bound[t] = t < ntok ? sh->bound[t] : 0xFFFFFFFFu;
+  __syncthreads();
+  // ---- one scan: everything at or above the bound
+  token_keys_scan<TPC>(x, mean, rstd, g, tok0, ntok, groups, 1, [&](int t, int l, int c0, int, const uint32_t (&key)[8]) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = max(m, key[j]);
+    if (m < bound[t]) return;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (key[j] >= bound[t] && c0 + j < f_valid) {  // padding columns of a shard take no part
+        const int slot = atomicAdd(&sh->n[t], 1);
+        if (slot < kTkList) sh->u.list[t][slot] = ((unsigned long long)key[j] << 32) | (0xFFFFFFFFu - (unsigned int)(l * col_pitch + c0 + j));
+      }
+    }
+  });
+  __syncthreads();
+  // ---- exact cut of the list: the largest word that exactly k words reach (one warp per token)
+  if (warp < ntok) {
+    const int n = sh->n[warp];
+    const bool lost = n > kTkList || n < k;
+    if (lost && lane == 0) o.ent_tok[1LL * (tok0 + warp) * k] = -1;
+    if (!lost) {
+      unsigned long long cut = 0;
+      for (int bit = 63; bit >= 0; --bit) {
+        const unsigned long long trial = cut | (1ULL << bit);
+        int cnt = 0;
+        for (int i = lane; i < n; i += 32) cnt += sh->u.list[warp][i] >= trial ? 1 : 0;
+        cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+        if (cnt >= k) cut = trial;
+        if (cnt == k) break;
+      }
+      const long long base = 1LL * (tok0 + warp) * k;
+      int done = 0;
+      for (int i0 = 0; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        const bool keep = i < n && sh->u.list[warp][i] >= cut;
+        const unsigned ball = __ballot_sync(0xFFFFFFFFu, keep);
+        if (keep) {
+          const int slot = done + __popc(ball & ((1u << lane) - 1u));
+          const int col = int(0xFFFFFFFFu - (unsigned int)(sh->u.list[warp][i] & 0xFFFFFFFFULL));
+          const int l = col / col_pitch, c = col - l * col_pitch;
+          if (slot < k) {
+            o.ent_tok[base + slot] = tok0 + warp;
+            o.ent_col[base + slot] = col;
+            o.ent_val[base + slot] = t16_to_float(x[1LL * l * g.layer_stride + 1LL * (tok0 + warp) * g.ld + c]);
+          }
+        }
+        done += __popc(ball);
       }
     }
   }
@@ -1571,6 +1726,24 @@ extern "C" int CLT_FN(clt_threshold_select)(const CltSelectArgs* a, cudaStream_t
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
+template <int TPC>
+static int launch_token_list(const CltSelectArgs* a, const ScanGeom& g, int f_valid, int k, cudaStream_t st) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(token_topk_list_kernel<TPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TokenListShared<TPC>))) != cudaSuccess) return -4;
+    attr_set = true;
+  }
+  // sample: at most every eighth block, at least enough groups for all maxima, and an expected list (step * k) of half its room
+  const int groups = g.L * (g.F / 8);
+  int step = kTkList / 2 / k;
+  step = step > 8 ? 8 : step;
+  if (step > groups / (2 * kTkMaxima)) step = groups / (2 * kTkMaxima);
+  if (step < 1) step = 1;
+  token_topk_list_kernel<TPC><<<(a->B + TPC - 1) / TPC, kTkThreads, sizeof(TokenListShared<TPC>), st>>>(
+      static_cast<const t16*>(a->x), a->mean, a->rstd, g, a->col_pitch, f_valid, k, step, a->ctl, lists_of(a));
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
 // Per-token top-k of the batch z-scores (TokenTopK).  Uses x, mean, rstd, L, B, F, stat_pitch, ld, layer_stride,
 // col_pitch, ctl, ent_* (capacity >= B * k), status of the argument block; k_total carries the per-token k and feat_offset
 // (when positive) the number of valid columns per layer (the rest of F is shard padding).
@@ -1586,8 +1759,14 @@ extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, cudaStream_
     attr_set = true;
   }
   const int grid = (a->B + kTokPerCta - 1) / kTokPerCta;
+  const bool list = k <= kTkMaxima / 2;
+  if (list) {
+    const int rc = a->B >= 1776 ? launch_token_list<4>(a, g, f_valid, int(k), st) : a->B >= 592 ? launch_token_list<2>(a, g, f_valid, int(k), st)
+                                                                                              : launch_token_list<1>(a, g, f_valid, int(k), st);
+    if (rc != 0) return rc;
+  }
   token_topk_kernel<<<grid, 256, sizeof(TokenTopkShared), st>>>(static_cast<const t16*>(a->x), a->mean, a->rstd, g, a->col_pitch,
-                                                                 f_valid, int(k), a->ctl, lists_of(a), a->status);
+                                                                 f_valid, int(k), a->ctl, lists_of(a), a->status, list ? 1 : 0);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -114,3 +114,32 @@ def test_equal_keys_in_a_token_segment_are_all_kept(ext):
     c = _csr(ext, tok, col, val, 1, 64, 64)
     assert torch.equal(c["tcsr_col"].long(), torch.sort(col.long()).values)
     assert torch.equal(torch.sort(c["tcsr_val"]).values, val)
+
+
+# one, two and four tokens per CTA with a last CTA that is not full; k up to the radix rounds; padding columns
+@pytest.mark.parametrize("L,B,Fl,F,k", [(3, 5, 4096, 4096, 64), (2, 601, 2056, 2050, 24), (4, 1779, 520, 520, 7), (2, 33, 1032, 1030, 513), (1, 9, 64, 64, 64),
+                                        (2, 40, 16384, 16384, 300)])
+def test_token_topk(ext, L, B, Fl, F, k):
+    dev = _dev()
+    torch.manual_seed(k)
+    x = torch.randn(L, B, Fl, device=dev).bfloat16()
+    if B == 33:
+        x[0, :, 100:400] = 1.5  # equal columns after standardisation: ties at and around the cut
+    mean, rstd = torch.empty(L, Fl, device=dev), torch.empty(L, Fl, device=dev)
+    ext.colstats(x, mean, rstd)
+    if B == 40:
+        x[1, 3] = 30.0  # a token whose list overflows: half of its keys are far above the bound of the other half
+        ext.colstats(x, mean, rstd)
+    status = torch.zeros(4, dtype=I32, device=dev)
+    ctl = torch.zeros(16, dtype=torch.int64, device=dev)
+    tok, col = torch.zeros(B * k, dtype=I32, device=dev), torch.zeros(B * k, dtype=I32, device=dev)
+    val = torch.zeros(B * k, device=dev)
+    ext.token_topk_select(x, mean, rstd, Fl, k, ctl, tok, col, val, status, F)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0 and int(ctl[3]) == B * k
+    assert torch.equal(tok.view(B, k), torch.arange(B, device=dev, dtype=I32)[:, None].expand(B, k))
+    assert torch.equal(x.float()[(col // Fl).long(), tok.long(), (col % Fl).long()], val)
+    z = ((x.float() - mean[:, None]) * rstd[:, None])[:, :, :F].permute(1, 0, 2).reshape(B, L * F)
+    order = torch.sort(z, dim=1, descending=True, stable=True).indices[:, :k]
+    want = torch.sort((order // F) * Fl + order % F, dim=1).values.to(I32)
+    assert torch.equal(torch.sort(col.view(B, k), dim=1).values, want)
