@@ -4,7 +4,7 @@
 // flattened tensor (clt/models/activations.py:27-32, 281-357).  Here the same selection is a threshold
 // search over the bf16 pre-activations written by the encoder GEMM:
 //
-//   1. colstats      per-feature batch mean and 1/(std+1e-6) (unbiased std, shifted sums)
+//   1. colstats      per-feature batch mean and 1/(std+1e-6) (unbiased std, from the encoder GEMM's row blocks or a pass of its own)
 //   2. zhist         8192-bin histogram of the order-preserving key of z = (x-mean)*rstd, keys >= key_lo
 //   3. find_bin      bin that contains the k_total-th largest key (after the ranks' histograms were summed)
 //   4. compact       entries above the bin go to the output list, entries inside it to a candidate list
@@ -1318,12 +1318,25 @@ __global__ void __launch_bounds__(1024) exclusive_scan_kernel(const int* __restr
 // Multi-CTA variant without scratch memory: CTA t owns elements [4096 t, 4096 (t + 1)).  It first adds up
 // everything in front of its tile (the counts are small and stay in L2, so the repeated reads are cheaper
 // than a second launch or a look-back protocol), then scans its own tile.
-__global__ void __launch_bounds__(1024) exclusive_scan_tiles_kernel(const int* __restrict__ in, int* __restrict__ out,
-                                                                      int* __restrict__ cursor, int n) {
+// Both arrays of the CSR build go in one launch: the first `tiles_a` CTAs scan a, the rest b.
+struct ScanJob {
+  const int* in;
+  int* out;
+  int* cursor;  // optional copy of the offsets for the scatter pass
+  int n;
+};
+__global__ void __launch_bounds__(1024) exclusive_scan_tiles_kernel(ScanJob ja, ScanJob jb, int tiles_a) {
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int base = blockIdx.x * 4096;
+  const bool second = int(blockIdx.x) >= tiles_a;
+  const ScanJob& job = second ? jb : ja;
+  const int tile = second ? int(blockIdx.x) - tiles_a : int(blockIdx.x);
+  const int n = job.n;
+  const int* __restrict__ in = job.in;
+  int* __restrict__ out = job.out;
+  int* __restrict__ cursor = job.cursor;
+  const int base = tile * 4096;
   int front = 0;
   {
     const int4* in4 = reinterpret_cast<const int4*>(in);  // base is a multiple of 4
@@ -1376,14 +1389,18 @@ __global__ void __launch_bounds__(1024) exclusive_scan_tiles_kernel(const int* _
     }
     run += v[k];
   }
-  if (blockIdx.x == gridDim.x - 1 && tid == 1023) out[n] = carry + warp_tot[31];
+  if (base + 4096 >= n && tid == 1023) out[n] = carry + warp_tot[31];
 }
 
-static void launch_exclusive_scan(const int* in, int* out, int* cursor, int n, cudaStream_t st) {
-  const int ntiles = (n + 4095) / 4096;
-  const bool aligned = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
-  if (ntiles >= 2 && ntiles <= 512 && aligned) exclusive_scan_tiles_kernel<<<ntiles, 1024, 0, st>>>(in, out, cursor, n);
-  else exclusive_scan_kernel<<<1, 1024, 0, st>>>(in, out, cursor, n);
+static void launch_exclusive_scans(const ScanJob& a, const ScanJob& b, cudaStream_t st) {
+  const int ta = (a.n + 4095) / 4096, tb = (b.n + 4095) / 4096;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(b.in)) & 15) == 0;
+  if (a.n > 0 && b.n > 0 && ta <= 512 && tb <= 512 && aligned) {
+    exclusive_scan_tiles_kernel<<<ta + tb, 1024, 0, st>>>(a, b, ta);
+  } else {
+    exclusive_scan_kernel<<<1, 1024, 0, st>>>(a.in, a.out, a.cursor, a.n);
+    exclusive_scan_kernel<<<1, 1024, 0, st>>>(b.in, b.out, b.cursor, b.n);
+  }
 }
 
 __global__ void __launch_bounds__(256) csr_scatter_kernel(const int* __restrict__ ent_tok, const int* __restrict__ ent_col,
@@ -1403,78 +1420,6 @@ __global__ void __launch_bounds__(256) csr_scatter_kernel(const int* __restrict_
     if (p >= 0 && p < cap) { tcsr_col[p] = (layer << 24) | (c - layer * col_pitch); tcsr_val[p] = v; }
     const int q = atomicAdd(&feat_cursor[c], 1);
     if (q >= 0 && q < cap) { fcsr_tok[q] = t; fcsr_val[q] = v; }
-  }
-}
-
-// Sort every CSR segment by its integer key (segments are short: insertion sort by one thread), so the
-// order of the entries - and with it every floating-point sum over a segment - is reproducible.
-constexpr int kShortSegment = 32;  // longer segments are sorted by a whole CTA (csr_sort_long_segments_kernel)
-
-__global__ void __launch_bounds__(256) csr_sort_segments_kernel(const int* __restrict__ off, int nseg, int* __restrict__ key,
-                                                                  float* __restrict__ val) {
-  for (int sidx = blockIdx.x * blockDim.x + threadIdx.x; sidx < nseg; sidx += gridDim.x * blockDim.x) {
-    const int b = off[sidx], e = off[sidx + 1];
-    if (e - b > kShortSegment) continue;
-    for (int i = b + 1; i < e; ++i) {
-      const int k = key[i];
-      const float v = val[i];
-      int j = i - 1;
-      while (j >= b && key[j] > k) { key[j + 1] = key[j]; val[j + 1] = val[j]; --j; }
-      key[j + 1] = k; val[j + 1] = v;
-    }
-  }
-}
-
-// Long segments (a feature that fires on most tokens of the batch, a token with a thousand active features): an insertion
-// sort by one thread would take O(n^2) dependent global-memory moves.  Here a CTA walks the segments, skips the short
-// ones and sorts a long one cooperatively with a bitonic network in place (keys inside a segment are distinct, so no
-// stability is needed); out-of-range partners of the virtual power-of-two padding are skipped.
-__global__ void __launch_bounds__(256) csr_sort_long_segments_kernel(const int* __restrict__ off, int nseg, int* __restrict__ key,
-                                                                       float* __restrict__ val) {
-  __shared__ int long_list[256];
-  __shared__ int long_count;
-  // every thread looks at one segment of a block of 256; the few long ones are then sorted one after the other by the CTA
-  for (int base = blockIdx.x * 256; base < nseg; base += gridDim.x * 256) {
-    if (threadIdx.x == 0) long_count = 0;
-    __syncthreads();
-    const int mine = base + threadIdx.x;
-    if (mine < nseg && off[mine + 1] - off[mine] > kShortSegment) long_list[atomicAdd(&long_count, 1)] = mine;
-    __syncthreads();
-    const int nlong = long_count;
-    for (int q = 0; q < nlong; ++q) {
-      const int sidx = long_list[q];
-      const int b = off[sidx], n = off[sidx + 1] - b;
-      int* k = key + b;
-      float* v = val + b;
-      int p2 = 1;
-      while (p2 < n) p2 <<= 1;
-      // every comparator puts the smaller key at the lower index (the first step of a merge pairs mirrored positions), so
-      // the virtual padding, which stands for +infinity at the end of the array, never has to move
-      for (int size = 2; size <= p2; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-          __syncthreads();
-          for (int i = threadIdx.x; i < p2 / 2; i += blockDim.x) {
-            int lo, hi;
-            if (stride == (size >> 1)) {
-              const int blk = i / stride, j = i - blk * stride;
-              lo = blk * size + j;
-              hi = blk * size + size - 1 - j;
-            } else {
-              lo = 2 * i - (i & (stride - 1));
-              hi = lo + stride;
-            }
-            if (hi >= n) continue;
-            const int ka = k[lo], kb = k[hi];
-            if (ka > kb) {
-              k[lo] = kb; k[hi] = ka;
-              const float t = v[lo]; v[lo] = v[hi]; v[hi] = t;
-            }
-          }
-        }
-      }
-      __syncthreads();
-    }
-    __syncthreads();
   }
 }
 
@@ -1514,6 +1459,56 @@ __device__ __forceinline__ void sort_pairs_cta(int* k, float* v, int n) {
   });
 }
 __device__ __forceinline__ unsigned long long pack_entry(int key, float val) { return ((unsigned long long)(unsigned int)key << 32) | __float_as_uint(val); }
+
+// Feature segments (sorted by token, so that every floating-point sum over a segment has one order).  A feature holds a few
+// entries, so a CTA takes up to 256 adjacent features, whose entries are one contiguous range: it comes into shared memory with
+// coalesced loads, one thread sorts one short segment there, and the CTA sorts the long ones together.  Ranges that do not
+// fit (features that fire on most tokens) are sorted in place in global memory.
+constexpr int kShortSegment = 32;
+constexpr int kFeatSortCap = 4096;
+__global__ void __launch_bounds__(256) csr_sort_feature_segments_kernel(const int* __restrict__ off, int nseg, int per_cta,
+                                                                          int* __restrict__ key, float* __restrict__ val) {
+  __shared__ unsigned long long w[kFeatSortCap];
+  __shared__ int long_list[256];
+  __shared__ int long_count;
+  const int s0 = blockIdx.x * per_cta, s1 = min(nseg, s0 + per_cta);
+  const int lo = off[s0], range = off[s1] - lo;
+  if (range <= 1) return;
+  const int mine = s0 + threadIdx.x;  // threads beyond per_cta own no segment
+  const int b = mine < s1 ? off[mine] : 0, n = mine < s1 ? off[mine + 1] - b : 0;
+  if (threadIdx.x == 0) long_count = 0;
+  const bool in_smem = range <= kFeatSortCap;
+  if (in_smem)
+    for (int i = threadIdx.x; i < range; i += 256) w[i] = pack_entry(key[lo + i], val[lo + i]);
+  __syncthreads();
+  if (n > kShortSegment) {
+    long_list[atomicAdd(&long_count, 1)] = mine;
+  } else if (in_smem) {
+    unsigned long long* q = w + (b - lo);
+    for (int i = 1; i < n; ++i) {
+      const unsigned long long x = q[i];
+      int j = i - 1;
+      while (j >= 0 && q[j] > x) { q[j + 1] = q[j]; --j; }
+      q[j + 1] = x;
+    }
+  } else {
+    for (int i = b + 1; i < b + n; ++i) {
+      const int k = key[i];
+      const float v = val[i];
+      int j = i - 1;
+      while (j >= b && key[j] > k) { key[j + 1] = key[j]; val[j + 1] = val[j]; --j; }
+      key[j + 1] = k; val[j + 1] = v;
+    }
+  }
+  __syncthreads();
+  for (int q = 0; q < long_count; ++q) {
+    const int sb = off[long_list[q]], sn = off[long_list[q] + 1] - sb;
+    if (in_smem) sort_words_cta(w + (sb - lo), sn);
+    else sort_pairs_cta(key + sb, val + sb, sn);
+  }
+  if (in_smem)
+    for (int i = threadIdx.x; i < range; i += 256) { key[lo + i] = int(w[i] >> 32); val[lo + i] = __uint_as_float((unsigned int)(w[i] & 0xFFFFFFFFULL)); }
+}
 
 // Token segments: one CTA per token sorts its entries by (layer, feature).  Up to kTokenRankCap entries every thread counts how
 // many keys are below its own (broadcast reads of shared memory, no barrier in between: 1 us where the 36 barriers of a
@@ -1896,20 +1891,25 @@ struct CltCsrArgs {
   int col_pitch;                      // columns are layer * col_pitch + feature (feature < 2^24)
 };
 
+// Features per CTA: as many as fill half of the shared buffer when the list is full, so that small dictionaries with long
+// segments get a CTA per feature instead of a few CTAs that sort hundreds of long segments one after the other.
+static void launch_feature_sort(const int* off, int num_cols, long long ent_cap, int* key, float* val, cudaStream_t st) {
+  if (num_cols <= 0) return;
+  int per_cta = 256;
+  while (per_cta > 1 && double(ent_cap) / num_cols * per_cta > kFeatSortCap / 2) per_cta /= 2;
+  csr_sort_feature_segments_kernel<<<(num_cols + per_cta - 1) / per_cta, 256, 0, st>>>(off, num_cols, per_cta, key, val);
+}
+
 extern "C" int clt_build_csr(const CltCsrArgs* a, cudaStream_t st) {
   const int blocks = 592;
   csr_count_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cnt, a->feat_cnt, a->fired,
                                            a->num_tokens, a->num_cols);
-  launch_exclusive_scan(a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens, st);
-  launch_exclusive_scan(a->feat_cnt, a->feat_off, a->feat_cursor, a->num_cols, st);
+  launch_exclusive_scans({a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens}, {a->feat_cnt, a->feat_off, a->feat_cursor, a->num_cols}, st);
   csr_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->feat_cursor,
                                              a->tcsr_col, a->tcsr_val, a->fcsr_tok, a->fcsr_val, a->col_pitch, a->num_tokens, a->num_cols);
   if ((a->sort_segments & 1) && a->num_tokens > 0)
     csr_sort_token_segments_kernel<<<a->num_tokens, 256, 0, st>>>(a->tok_off, a->tcsr_col, a->tcsr_val);
-  if (a->sort_segments & 2) {
-    csr_sort_segments_kernel<<<(a->num_cols + 255) / 256, 256, 0, st>>>(a->feat_off, a->num_cols, a->fcsr_tok, a->fcsr_val);
-    csr_sort_long_segments_kernel<<<(a->num_cols + 255) / 256 < 1184 ? (a->num_cols + 255) / 256 : 1184, 256, 0, st>>>(a->feat_off, a->num_cols, a->fcsr_tok, a->fcsr_val);
-  }
+  if (a->sort_segments & 2) launch_feature_sort(a->feat_off, a->num_cols, a->ent_cap, a->fcsr_tok, a->fcsr_val, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -1983,10 +1983,7 @@ extern "C" int clt_build_csr_static(const int* ent_tok, const int* ent_col, cons
   csr_scatter_kernel<<<blocks, 256, 0, stream>>>(ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cursor, feat_cursor, tcsr_col, tcsr_val,
                                                  fcsr_tok, fcsr_val, col_pitch, num_tokens, num_cols);
   if (sort_segments & 1) csr_sort_token_segments_kernel<<<num_tokens, 256, 0, stream>>>(tok_off, tcsr_col, tcsr_val);
-  if (sort_segments & 2) {
-    csr_sort_segments_kernel<<<(num_cols + 255) / 256, 256, 0, stream>>>(feat_off, num_cols, fcsr_tok, fcsr_val);
-    csr_sort_long_segments_kernel<<<num_cols < 1184 ? num_cols : 1184, 256, 0, stream>>>(feat_off, num_cols, fcsr_tok, fcsr_val);
-  }
+  if (sort_segments & 2) launch_feature_sort(feat_off, num_cols, ent_cap, fcsr_tok, fcsr_val, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 #endif  // !CLT_T16_IS_HALF
