@@ -154,6 +154,8 @@ struct CltTopkTpArgs {
   int* status;
 };
 int clt_token_topk_tp(const CltTopkTpArgs* a, int phase, cudaStream_t st);
+int clt_theta_accumulate(const int* feat_off, const float* fcsr_val, const float* mean, const float* rstd, int L, int pitch, int width, float eps,
+                         float* sum_min, float* cnt_min, float* mean_acc, float* std_acc, float* batches, cudaStream_t st);
 int clt_aux_compact(const long long* dead_counter, long long window, int L, int F_pitch, int F_valid, int nd_cap, int* dead_cols, int* nd,
                     int* nd_all, int* extra_idx, cudaStream_t st);
 int clt_scatter_add_rows(float* dst, float* dst_bias, const float* src, const float* src_bias, const int* extra_idx, long long n_dst_rows, int d,
@@ -486,7 +488,8 @@ void sparse_decode(const std::vector<Tensor>& dec_w, int64_t L, int64_t B, int64
   } else if (mode == 0) {
     TORCH_CHECK(a.yhat_partial != nullptr, "mode 0 needs yhat_partial");
   } else {
-    TORCH_CHECK(a.bias_sum && a.target && a.gs && a.sq_err, "mode 1 needs bias_sum, target, gs, sq_err");
+    // without a target there is no loss: the reconstruction is the only output
+    TORCH_CHECK(a.bias_sum && ((a.target && a.gs && a.sq_err) || (!a.target && a.yhat_out)), "mode 1 needs bias_sum and either target, gs, sq_err or yhat_out alone");
   }
   c10::cuda::CUDAGuard guard(tok_off.device());
   check(CLT_PICK(half, clt_sparse_decode)(&a, cur_stream()), "sparse_decode");
@@ -752,6 +755,22 @@ void theta_adam(Tensor& log_theta, Tensor& m, Tensor& v, Tensor& theta, const Te
   check(CLT_PICK(half, clt_theta_adam)(&a, cur_stream()), "theta_adam");
 }
 
+void theta_accumulate(const Tensor& feat_off, const Tensor& fcsr_val, const Tensor& mean, const Tensor& rstd, double eps, Tensor& sum_min,
+                      Tensor& cnt_min, Tensor& mean_acc, Tensor& std_acc, Tensor& batches) {
+  need(feat_off, at::kInt, "feat_off"); need(fcsr_val, at::kFloat, "fcsr_val"); need(mean, at::kFloat, "mean"); need(rstd, at::kFloat, "rstd");
+  TORCH_CHECK(mean.dim() == 2 && rstd.sizes() == mean.sizes() && feat_off.numel() == mean.numel() + 1, "mean / rstd [L, F], feat_off [L * F + 1]");
+  for (const Tensor* t : {&sum_min, &cnt_min, &mean_acc, &std_acc}) {
+    need(*t, at::kFloat, "statistics");
+    TORCH_CHECK(t->dim() == 2 && t->size(0) == mean.size(0) && t->size(1) == sum_min.size(1) && t->size(1) <= mean.size(1), "statistics [L, width]");
+  }
+  need(batches, at::kFloat, "batches");
+  TORCH_CHECK(batches.numel() == mean.size(0), "batches [L]");
+  c10::cuda::CUDAGuard guard(mean.device());
+  check(clt_theta_accumulate(feat_off.data_ptr<int>(), fcsr_val.data_ptr<float>(), mean.data_ptr<float>(), rstd.data_ptr<float>(), int(mean.size(0)),
+                             int(mean.size(1)), int(sum_min.size(1)), float(eps), sum_min.data_ptr<float>(), cnt_min.data_ptr<float>(),
+                             mean_acc.data_ptr<float>(), std_acc.data_ptr<float>(), batches.data_ptr<float>(), cur_stream()), "theta_accumulate");
+}
+
 void theta_exp(const Tensor& log_theta, Tensor& theta) {
   const bool w16 = log_theta.scalar_type() != at::kFloat;
   const bool half = w16 && is_half(log_theta, "log_theta");
@@ -994,6 +1013,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("norm2"), py::arg("feat_off"), py::arg("fcsr_val"), py::arg("tying"), py::arg("c_g"), py::arg("lambda_"), py::arg("c"),
         py::arg("bandwidth"), py::arg("hyper"), py::arg("ctl") = none, py::arg("norm_weight") = 0.0, py::arg("grad_out") = none);
   m.def("theta_exp", &theta_exp);
+  m.def("theta_accumulate", &theta_accumulate);
   m.def("dense_gemm", &dense_gemm);
   m.def("transpose16", &transpose16, py::arg("inp"), py::arg("out"), py::arg("mask") = none);
   m.def("negative_indicator", &negative_indicator);

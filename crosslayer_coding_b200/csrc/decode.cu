@@ -76,6 +76,18 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
     dst[1] = make_float4(a[4], a[5], a[6], a[7]);
     return 0.f;
   } else {
+    if (p.target == nullptr) {  // inference: the reconstruction is all there is to write
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i] = a[i] + p.bias_sum[1LL * t * p.d + e0 + i];
+        if (p.addend) v[i] += p.addend[off + i];
+      }
+      float4* dst = reinterpret_cast<float4*>(p.yhat_out + off);
+      dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+      dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+      return 0.f;
+    }
     float y[8], out[8];
     const uint4 tv = *reinterpret_cast<const uint4*>(p.target + off);
     const uint32_t u[4] = {tv.x, tv.y, tv.z, tv.w};
@@ -251,7 +263,7 @@ __global__ void __launch_bounds__(32 * (FULL ? kFullWarps : kWalkWarps), FULL ? 
     if (threadIdx.x == 0) {
       float tot = 0.f;
       for (int w = 0; w < kWarps; ++w) tot += red_s[w];
-      if (tot != 0.f) atomicAdd(&p.sq_err[t], double(tot));
+      if (tot != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[t], double(tot));
     }
   }
 }
@@ -304,7 +316,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps, NV >= 2 ? 2 : 3) decode_runni
     }
   }
   __syncthreads();
-  if (p.mode == 1 && threadIdx.x < p.L && sq_s[threadIdx.x] != 0.f) atomicAdd(&p.sq_err[threadIdx.x], double(sq_s[threadIdx.x]));
+  if (p.mode == 1 && threadIdx.x < p.L && sq_s[threadIdx.x] != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[threadIdx.x], double(sq_s[threadIdx.x]));
 }
 
 // Epilogue for the tensor-parallel path, run after the partial reconstructions were summed across ranks:

@@ -278,6 +278,33 @@ __global__ void __launch_bounds__(256) theta_adam_kernel(const ThetaAdamParams p
   }
 }
 
+// One batch of the threshold statistics (BatchTopK / TopK -> JumpReLU): per feature the batch mean and standard deviation and the
+// smallest z-score among its selected entries with a positive value, added to the running sums.  One thread per feature walks
+// its entry list; everything it touches is 28 bytes per feature plus the entries, so the pass is a few microseconds where the
+// same statistic as tensor operations is some twenty launches over the entry list and the feature planes.
+__global__ void __launch_bounds__(256) theta_accumulate_kernel(const int* __restrict__ feat_off, const float* __restrict__ fcsr_val,
+                                                                 const float* __restrict__ mean, const float* __restrict__ rstd, int L, int pitch,
+                                                                 int width, float eps, float* __restrict__ sum_min, float* __restrict__ cnt_min,
+                                                                 float* __restrict__ mean_acc, float* __restrict__ std_acc, float* __restrict__ batches) {
+  const long long n = 1LL * L * pitch;
+  for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
+    const int l = int(i / pitch), f = int(i - 1LL * l * pitch);
+    if (f == 0) batches[l] += 1.f;
+    if (f >= width) continue;
+    const long long o = 1LL * l * width + f;
+    const float mu = mean[i], rs = rstd[i];
+    mean_acc[o] += mu;
+    std_acc[o] += __frcp_rn(rs) - eps;
+    float low = INFINITY;
+    const int b = __ldg(feat_off + i), e = __ldg(feat_off + i + 1);
+    for (int j = b; j < e; ++j) {
+      const float x = __ldg(fcsr_val + j);
+      if (x > 0.f) low = fminf(low, (x - mu) * rs);
+    }
+    if (low < INFINITY) { sum_min[o] += low; cnt_min[o] += 1.f; }
+  }
+}
+
 // ---------------------------------------------------------------------------------------- batch normalisation
 // Activation batches arrive on the device as stored ([2, L, B, d]: inputs and targets of every layer, bf16 / fp16 /
 // fp32); the store's normalisation (x - mean) / std with per-(side, layer, element) statistics, or x * mul, and the
@@ -471,6 +498,18 @@ extern "C" int CLT_FN(clt_theta_exp)(const void* log_theta, float* theta, long l
   else theta_exp_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(log_theta), theta, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
+
+#if !CLT_T16_IS_HALF
+extern "C" int clt_theta_accumulate(const int* feat_off, const float* fcsr_val, const float* mean, const float* rstd, int L, int pitch, int width,
+                                    float eps, float* sum_min, float* cnt_min, float* mean_acc, float* std_acc, float* batches, cudaStream_t st) {
+  if (width > pitch) return -1;
+  const long long n = 1LL * L * pitch;
+  if (n <= 0) return 0;
+  const int grid = int((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
+  theta_accumulate_kernel<<<grid, 256, 0, st>>>(feat_off, fcsr_val, mean, rstd, L, pitch, width, eps, sum_min, cnt_min, mean_acc, std_acc, batches);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+#endif
 
 // in_type: 0 fp32, 1 bf16, 2 fp16.  mean / inv_std: [rows / rows_per_stat, d] or null (only the multiplier applies).
 extern "C" int CLT_FN(clt_normalize_cast)(const void* in, int in_type, void* out, const float* mean, const float* inv_std, long long rows,

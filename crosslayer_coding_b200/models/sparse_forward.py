@@ -88,15 +88,22 @@ class SparseForward:
         if self.fn == "batchtopk":
             from ..training.fused_engine import histogram_range
 
-            self.hist = torch.zeros(2 * 8192 + 32, dtype=i32, device=dev)
             self.key_lo, self.shift = histogram_range(self.k_total, B * L * Fl)
             cand_cap = int(min(B * L * Fl, max(1 << 20, 4 * self.k_total)))
             self.cand = [torch.empty(cand_cap, dtype=i32, device=dev) for _ in range(3)] + [torch.empty(cand_cap, dtype=f32, device=dev)]
             self.sel_state = torch.tensor([self.key_lo, self.shift], dtype=torch.int64, device=dev) if self.key_lo != 0 else None
             self.pool = torch.empty(4, int(min(B * L * Fl, 3 * self.k_total + (1 << 16))), dtype=i32, device=dev) if self.key_lo != 0 else None
         ncols = self.ncols = L * Fl
-        self.tok_cnt = torch.zeros(B, dtype=i32, device=dev)
-        self.feat_cnt = torch.zeros(ncols, dtype=i32, device=dev)
+        # everything that has to be zero when a call starts sits in one buffer, cleared by one memset; the loss sums come last,
+        # because only `reconstruct` clears them
+        sizes = [2 * 8192 + 32, B, ncols]
+        starts = [0]
+        for n in sizes:
+            starts.append((starts[-1] + n + 63) // 64 * 64)
+        self._zeroed = torch.zeros(starts[-1] + 2 * L, dtype=i32, device=dev)
+        self._zeroed_encode = self._zeroed[: starts[-1]]
+        self.hist, self.tok_cnt, self.feat_cnt = (self._zeroed[o: o + n] for o, n in zip(starts, sizes))
+        self.sq_err = self._zeroed[starts[-1]:].view(torch.float64)
         self.tok_off = torch.zeros(B + 1, dtype=i32, device=dev)
         self.feat_off = torch.zeros(ncols + 1, dtype=i32, device=dev)
         self.tok_cursor = torch.zeros(B, dtype=i32, device=dev)
@@ -106,7 +113,6 @@ class SparseForward:
         self.fcsr_tok = torch.zeros(cap, dtype=i32, device=dev)
         self.fcsr_val = torch.zeros(cap, dtype=f32, device=dev)
         self.gs = torch.empty(L, B, d, dtype=torch.bfloat16, device=dev)
-        self.sq_err = torch.zeros(L, dtype=torch.float64, device=dev)
         if self.tying == 0:
             from .clt import pair_index
 
@@ -118,24 +124,26 @@ class SparseForward:
             sel = torch.tril(torch.ones(L, L, dtype=f32, device=dev))
         else:
             sel = torch.eye(L, dtype=f32, device=dev)
-        self.bias_sel = sel
+        self.bias_sel = sel.contiguous()
+        self.bias_sum = torch.empty(L, d, dtype=f32, device=dev)
+        self.theta = torch.full((L, Fl), _MIN_POSITIVE_BF16, dtype=f32, device=dev) if self.fn in ("jumprelu", "relu") else None
 
     # ------------------------------------------------------------------ selection
     def _theta(self) -> torch.Tensor:
         if self.fn == "jumprelu":
-            return self.model.log_threshold.data.float().exp().contiguous()
-        return torch.full((self.L, self.Fl), _MIN_POSITIVE_BF16, dtype=torch.float32, device=self.dev)
+            torch.exp(self.model.log_threshold.data, out=self.theta)  # re-read on every call: the parameter may have changed
+        return self.theta
 
     @torch.no_grad()
-    def encode(self, X: torch.Tensor) -> None:
+    def encode(self, X: torch.Tensor, clear_loss: bool = False) -> None:
         """Pre-activations, selection and the token-major / feature-major CSR views of the active entries."""
         e, m = self.ext, self.model
         assert X.dtype == torch.bfloat16 and X.shape == (self.L, self.B, self.d), (X.dtype, tuple(X.shape))
+        (self._zeroed if clear_loss else self._zeroed_encode).zero_()
         e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, self.tile_stats)
         if self.tile_stats is not None:
             e.colstats_from_tiles(self.tile_stats, self.mean, self.rstd, self.B)
         if self.fn == "batchtopk":
-            self.hist.zero_()
             e.batchtopk_select(self.preact, self.mean, self.rstd, self.Fl, self.Fl, 0, self.Fl, self.k_total, self.key_lo, self.shift,
                                self.hist, self.ctl, self.ent_tok, self.ent_col, self.ent_val, self.cand[0], self.cand[1], self.cand[2],
                                self.cand[3], self.status, 1, 0, [], [], 0, 0, self.sel_state, self.pool)
@@ -144,8 +152,6 @@ class SparseForward:
                                 self.ent_val, self.status)
         else:
             e.threshold_select(self.preact, self._theta(), self.Fl, self.Fl, self.ctl, self.ent_tok, self.ent_col, self.ent_val, self.status)
-        self.tok_cnt.zero_()
-        self.feat_cnt.zero_()
         e.build_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.feat_cnt, self.tok_off,
                     self.feat_off, self.tok_cursor, self.feat_cursor, self.tcsr_col, self.tcsr_val, self.fcsr_tok, self.fcsr_val,
                     None, 3, self.Fl)
@@ -155,20 +161,19 @@ class SparseForward:
     def reconstruct(self, X: torch.Tensor, Y: Optional[torch.Tensor] = None, sigma: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Reconstructions ``[L, B, d]`` (fp32).  With targets ``Y`` the per-layer sums of squared errors
         (scaled by ``sigma [L, d]`` when given) are left in ``self.sq_err``."""
-        self.encode(X)
+        self.encode(X, clear_loss=True)
         e, m = self.ext, self.model
-        self.sq_err.zero_()
         yhat = torch.empty(self.L, self.B, self.d, dtype=torch.float32, device=self.dev)
-        bias_sum = (self.bias_sel @ m.dec_bias.data.float()).contiguous()
+        e.step_finish(None, None, m.dec_bias.data, self.bias_sel, self.bias_sum)
         off = scale = None
         if m.feature_offset is not None:
             off = m.feature_offset.data.float().contiguous()
         if m.feature_scale is not None:
             scale = m.feature_scale.data.float().contiguous()
-        tgt = Y if Y is not None else torch.zeros_like(X)
         sg = sigma.to(device=self.dev, dtype=torch.float32).reshape(self.L, self.d).contiguous() if sigma is not None else None
+        gs, sq_err = (self.gs, self.sq_err) if Y is not None else (None, None)  # no targets: the reconstruction is the only output
         e.sparse_decode([w.data for w in m.dec_weight], self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col,
-                        self.tcsr_val, off, scale, None, bias_sum, None, tgt, sg, self.gs, yhat, self.sq_err, 1, [], 0, 0, self.status)
+                        self.tcsr_val, off, scale, None, self.bias_sum, None, Y, sg, gs, yhat, sq_err, 1, [], 0, 0, self.status)
         return yhat
 
     def forward_dict(self, inputs: Dict[int, torch.Tensor]) -> Dict[int, torch.Tensor]:

@@ -81,26 +81,11 @@ def accumulate_theta_batch(model, inputs: Dict[int, torch.Tensor], stats: Dict[s
 @torch.no_grad()
 def accumulate_theta_batch_sparse(sf, X: torch.Tensor, stats: Dict[str, torch.Tensor]) -> None:
     """The same statistic from the sparse forward (``models.sparse_forward.SparseForward``): the batch mean / std of
-    every feature come from the column-statistics kernel, the per-feature minimum of the selected z-scores from the
-    entry list - no dense ``[B, L*F]`` selection, which is what the dense path spends its time on."""
+    every feature come from the selection's column statistics, the per-feature minimum of the selected z-scores from the
+    feature-major entry list, one kernel - no dense ``[B, L*F]`` selection, which is what the dense path spends its time on."""
     sf.encode(X)
-    L, Fl = sf.L, sf.Fl
-    std = 1.0 / sf.rstd - act.ZSCORE_EPS
-    stats["mean"] += sf.mean[:, : stats["mean"].shape[1]]
-    stats["std"] += std[:, : stats["std"].shape[1]]
-    stats["batches"] += 1
-    cap = sf.ent_val.numel()
-    n = torch.clamp(sf.ctl[3], max=cap)
-    live = (torch.arange(cap, device=X.device) < n) & (sf.ent_val > 0)
-    col = torch.where(live, sf.ent_col, torch.zeros_like(sf.ent_col)).long()
-    z = (sf.ent_val - sf.mean.reshape(-1)[col]) * sf.rstd.reshape(-1)[col]
-    z = torch.where(live, z, torch.full_like(z, float("inf")))
-    mins = torch.full((L * Fl,), float("inf"), device=X.device)
-    mins.scatter_reduce_(0, col, z, reduce="amin", include_self=True)
-    mins = mins.view(L, Fl)[:, : stats["sum_min"].shape[1]]
-    ok = torch.isfinite(mins)
-    stats["sum_min"] += torch.where(ok, mins, torch.zeros_like(mins))
-    stats["cnt_min"] += ok.float()
+    sf.ext.theta_accumulate(sf.feat_off, sf.fcsr_val, sf.mean, sf.rstd, act.ZSCORE_EPS, stats["sum_min"], stats["cnt_min"], stats["mean"],
+                            stats["std"], stats["batches"])
 
 
 @torch.no_grad()

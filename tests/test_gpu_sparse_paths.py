@@ -179,3 +179,75 @@ def test_encoder_gemm_column_statistics(ext, L, M, N, K, dtype, bias_size):
         assert ((1.0 / rstd.double() - 1e-6 - std).abs() <= 2e-5 * std + 1e-5).all()
     else:
         assert (rstd > 9e5).all()
+
+
+def _serving_model(fn, tying, dev, L=3, d=64, F=512):
+    from crosslayer_coding_b200 import CLTConfig, CrossLayerTranscoder
+
+    torch.manual_seed(0)
+    cfg = CLTConfig(num_features=F, num_layers=L, d_model=d, activation_fn=fn, batchtopk_k=9, topk_k=9, jumprelu_threshold=0.1, clt_dtype="bfloat16",
+                    decoder_tying=tying)
+    model = CrossLayerTranscoder(cfg, device=dev)
+    with torch.no_grad():
+        for w in model.dec_weight:
+            w.uniform_(-0.1, 0.1)
+        model.dec_bias.uniform_(-0.5, 0.5)
+        model.enc_weight.uniform_(-0.02, 0.02)
+    return model
+
+
+@pytest.mark.parametrize("fn,tying", [("batchtopk", "none"), ("topk", "per_source"), ("jumprelu", "per_target"), ("relu", "none")])
+def test_sparse_forward_with_and_without_targets(ext, fn, tying):
+    """Without targets only the reconstruction is written; the loss sums of an earlier call with targets survive `encode`; changed
+    parameters (biases, thresholds) are seen by the next call."""
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model(fn, tying, dev)
+    B = 200
+    sf = SparseForward(model, B)
+    x = torch.randn(3, B, 64, device=dev).bfloat16()
+    y = torch.randn(3, B, 64, device=dev).bfloat16()
+    a = sf.reconstruct(x, y)
+    sq = sf.sq_err.clone()
+    assert torch.allclose(sq, (a.double() - y.double()).square().sum((1, 2)), rtol=1e-5)
+    sf.encode(x)
+    assert torch.equal(sf.sq_err, sq)
+    b = sf.forward_dict({l: x[l] for l in range(3)})
+    for l in range(3):
+        assert torch.equal(a[l], b[l])
+    with torch.no_grad():
+        model.dec_bias.add_(0.25)
+    shift = {"none": torch.arange(1, 4), "per_source": torch.arange(1, 4), "per_target": torch.ones(3)}[tying].to(dev).float() * 0.25
+    c = sf.reconstruct(x)
+    assert torch.allclose(c, a + shift[:, None, None], atol=2e-2)
+    if fn == "jumprelu":
+        n = sf.num_entries()
+        with torch.no_grad():
+            model.log_threshold.add_(0.5)
+        sf.encode(x)
+        assert sf.num_entries() < n
+    sf.check_status()
+
+
+@pytest.mark.parametrize("fn", ["batchtopk", "topk"])
+def test_threshold_statistics_match_the_dense_form(ext, fn):
+    from crosslayer_coding_b200.models import theta
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model(fn, "none", dev)
+    sf = SparseForward(model, 150)
+    dense, sparse = theta._new_stats(model), theta._new_stats(model)
+    for i in range(3):
+        x = torch.randn(3, 150, 64, device=dev).bfloat16()
+        theta.accumulate_theta_batch(model, {l: x[l] for l in range(3)}, dense)
+        theta.accumulate_theta_batch_sparse(sf, x, sparse)
+    sf.check_status()
+    assert torch.equal(sparse["batches"], dense["batches"])
+    # 16-bit pre-activations of two GEMMs: single elements differ by one rounding (2^-8 relative), a selection by few entries
+    for n in ("mean", "std"):
+        assert torch.allclose(sparse[n], dense[n], atol=2e-3, rtol=2e-3), n
+    assert float((sparse["cnt_min"] != dense["cnt_min"]).float().mean()) < 0.02
+    same = sparse["cnt_min"] == dense["cnt_min"]
+    assert float(((sparse["sum_min"] - dense["sum_min"]).abs()[same] > 0.05).float().mean()) < 0.02
