@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(32 * (FULL ? kFullWarps : kWalkWarps), FULL ? 
       const int col = i < e ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
       float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
       const int s = col >> 24, f = col & 0xFFFFFF;
-      bool use = a != 0.f && s <= t && t - s < span;
+      bool use = a != 0.f;
       if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
+      use = use && s <= t && t - s < span;
       const t16* row = nullptr;
       if (use) {
         const int wi = p.tying == 2 ? t : s;
@@ -300,8 +301,9 @@ __global__ void __launch_bounds__(32 * kWalkWarps, NV >= 2 ? 2 : 3) decode_runni
         const int col = i < e ? __ldg(p.tcsr_col + i) : 0;
         const float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
         const int f = col & 0xFFFFFF;
-        bool use = a != 0.f && (col >> 24) == t;
-        if (use && !clt_in_bounds(f, p.col_pitch, p.dbg_status, 103)) use = false;
+        bool use = a != 0.f;
+        if (use && (!clt_in_bounds(col >> 24, p.L, p.dbg_status, 103) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 104))) use = false;
+        use = use && (col >> 24) == t;
         const uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
         if (mask != 0u) gather_rows<NV, 4>(mask, a, p.w[t] + 1LL * f * d, e0, act, acc);
       }
