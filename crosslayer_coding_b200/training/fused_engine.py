@@ -7,7 +7,7 @@ One step is a fixed sequence of hand-written kernels and never materialises a de
  #    kernel (csrc/)                         replaces in the reference
 ====  =====================================  ============================================
  1    encoder_gemm  (tcgen05 + TMA)          L x F.linear + all_gather, run 2-4x per step
- 2    colstats_from_tiles                    per-layer mean/std temporaries (column sums come from the GEMM)
+ 2    colstats                               per-layer mean/std temporaries
  3    batchtopk_select                       torch.topk over B*L*F + mask + multiply
  4    build_csr                              (dense mask is the reference's data structure)
  5    sparse_decode (+ loss epilogue)        P dense decoder GEMMs + P all-reduces + MSELoss
@@ -236,8 +236,7 @@ class FusedBatchTopKEngine:
         self.preact = torch.empty(L, B, Fl, dtype=self.t16, device=dev)
         self.mean = torch.empty(L, Fl, dtype=f32, device=dev)
         self.rstd = torch.empty(L, Fl, dtype=f32, device=dev)
-        # the selections rank z-scores: the encoder GEMM leaves the column statistics of its 128-row blocks here
-        self.tile_stats = torch.empty(L, (B + 127) // 128, Fl, 2, dtype=f32, device=dev) if self.fn in ("batchtopk", "topk") else None
+        self.tile_stats = None  # [L, ceil(B / 128), Fl, 2] fp32 switches the statistics into the GEMM epilogue
         # tracked histogram range {key_lo, shift} and the pool filled by the single pass over the pre-activations
         self.sel_state = torch.tensor([self.key_lo, self.shift], dtype=torch.int64, device=dev) if self.key_lo != 0 else None
         k_local = -(-self.k_total // max(1, self.world))
@@ -418,6 +417,9 @@ class FusedBatchTopKEngine:
         if fresh:
             self._begin_step()
         self._X_last = X
+        # The GEMM can leave the column statistics behind (tile_stats), as the sparse forward uses it.  A training step keeps the
+        # separate pass: the two differ in the last bit, which moves single entries across the cut of the selection, and the
+        # moments of such an entry's rows then differ by their own size from what earlier runs of the same inputs gave.
         e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, self.tile_stats)
         if self.fn in ("jumprelu", "relu"):
             self._ensure_theta()
@@ -425,7 +427,10 @@ class FusedBatchTopKEngine:
             self._build_csr()
             self.kernel_launches += 2 + 5  # gemm, threshold selection, csr (5)
             return
-        e.colstats_from_tiles(self.tile_stats, self.mean, self.rstd, self.B)
+        if self.tile_stats is not None:
+            e.colstats_from_tiles(self.tile_stats, self.mean, self.rstd, self.B)
+        else:
+            e.colstats(self.preact, self.mean, self.rstd)
         if self.fn == "topk" and self.world == 1:
             e.token_topk_select(self.preact, self.mean, self.rstd, self.Fl, self.k_token, self.ctl, self.ent_tok, self.ent_col,
                                 self.ent_val, self.status, self.Fv)
