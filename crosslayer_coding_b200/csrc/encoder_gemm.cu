@@ -6,9 +6,9 @@
 // Counterpart of the reference's per-layer F.linear calls (clt/models/parallel.py:286 through
 // clt/models/encoder.py:101).
 //
-// Structure: one CTA per SM, 10 warps.  Warp 0 feeds a shared-memory ring with TMA tile loads
+// Structure: one CTA per SM, 6 warps.  Warp 0 feeds a 4-stage shared-memory ring with TMA tile loads
 // (no cluster multicast: every CTA fetches its own tiles), warp 1 issues tcgen05.mma 128x256x16 into one
-// of two 256-column TMEM accumulators, warps 2-9 drain the other accumulator with tcgen05.ld, add the
+// of two 256-column TMEM accumulators, warps 2-5 drain the other accumulator with tcgen05.ld, add the
 // bias and store bf16.  Tiles are ordered m-fastest so CTAs that run together share the weight tile in L2.
 // Every mbarrier wait is bounded; on a timeout the CTA records STATUS_WAIT_TIMEOUT, drains its copies,
 // frees its TMEM and returns.
@@ -18,25 +18,19 @@
 
 namespace clt {
 
-// Epilogue warps per CTA: two per TMEM lane quarter, each with half of the tile's columns.  With four, the drain of a tile (TMEM ->
-// registers -> staging -> TMA store) left no time for the column statistics beside the MMAs: [4096 x 768] x [768 x 24576] for
-// 12 layers took 1.54 ms without and 2.15 ms with them, with eight warps 1.46 and 1.61 ms, which saves the separate pass
-// over the pre-activations (0.37 ms).  The staging tiles cost one stage of the ring.
-constexpr int kEpiWarps = 8;
-
 namespace gemm {
 constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzled row
-constexpr int STAGES = 3;
+constexpr int STAGES = 4;
 constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
 constexpr uint32_t B_BYTES = BN * BK * 2;
 constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int NUM_THREADS = 64 + 32 * kEpiWarps;
+constexpr int NUM_THREADS = 192;
 constexpr uint32_t TMEM_COLS = 512;
 // ring + 1024 B alignment slack + barriers/bias
-constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + kEpiWarps * 4096 + 1024 + 10240;  // ring + epilogue staging + slack + barriers
+constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + 4 * 4096 + 1024 + 4096;  // ring + epilogue staging + slack + barriers
 }  // namespace gemm
 
 // Epilogue of one 32-row slab (one warp, lane = row): TMEM -> registers -> + bias -> bf16 -> shared staging
@@ -46,11 +40,12 @@ constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + kEpiWarps * 4096 + 
 constexpr int kEpiCols = 64;
 constexpr uint32_t kEpiStageBytes = 32 * kEpiCols * 2;
 
-// With `colacc` (shared, this slab's [2][BN] floats) the slab's column means and squared deviations of the rounded values are
-// read back from the staging tile (each lane owns two adjacent columns); `nrows` masks the rows beyond the matrix.
+// With `colacc` (shared, [2][BN] floats: sums and sums of squares per tile column) the slab's column statistics
+// of the rounded bf16 values are read back from the staging tile (each lane owns two adjacent columns) and
+// added up over the tile's four slabs; `nrows` masks the rows beyond the matrix.
 __device__ __forceinline__ void epilogue_slab(uint32_t taddr, const CUtensorMap* map_c, uint8_t* stage, const float* bias_s,
-                                              int c_lo, int c_hi, int n_base, int m_base, int l, int lane, float* colacc, int bn_full, int nrows) {
-  for (int c = c_lo; c < c_hi; ++c) {
+                                              int bn, int n_base, int m_base, int l, int lane, float* colacc, int bn_full, int nrows) {
+  for (int c = 0; c < bn / kEpiCols; ++c) {
     uint32_t r0[32], r1[32];
     tmem_ld_32x32(taddr + c * kEpiCols, r0);
     tmem_ld_32x32(taddr + c * kEpiCols + 32, r1);
@@ -78,45 +73,33 @@ __device__ __forceinline__ void epilogue_slab(uint32_t taddr, const CUtensorMap*
     if (colacc != nullptr) {
       float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
       const uint32_t chunk = uint32_t(lane >> 2), inner = uint32_t(lane & 3) * 4u;
-      const uint32_t first = *reinterpret_cast<const uint32_t*>(stage + (chunk << 4) + inner);  // sums about the slab's first row
-      const float h0 = t16_lo(first), h1 = t16_hi(first);
 #pragma unroll 8
-      for (int r = 1; r < 32; ++r) {
+      for (int r = 0; r < 32; ++r) {
         if (r < nrows) {
           const uint32_t u = *reinterpret_cast<const uint32_t*>(stage + r * 128 + ((chunk ^ uint32_t(r & 7)) << 4) + inner);
-          const float a = t16_lo(u) - h0, b = t16_hi(u) - h1;
+          const float a = t16_lo(u), b = t16_hi(u);
           s0 += a; q0 = fmaf(a, a, q0);
           s1 += b; q1 = fmaf(b, b, q1);
         }
       }
-      const float inv = 1.f / float(nrows);
       const int col = c * kEpiCols + 2 * lane;
-      *reinterpret_cast<float2*>(colacc + col) = make_float2(h0 + s0 * inv, h1 + s1 * inv);
-      *reinterpret_cast<float2*>(colacc + bn_full + col) = make_float2(q0 - s0 * s0 * inv, q1 - s1 * s1 * inv);
+      atomicAdd(&colacc[col], s0); atomicAdd(&colacc[col + 1], s1);
+      atomicAdd(&colacc[bn_full + col], q0); atomicAdd(&colacc[bn_full + col + 1], q1);
     }
   }
 }
 
-// Column statistics of a 128-row block -> global [L][row blocks of 128][N] x (mean, sum of squared deviations): merges the means and
-// deviations of the block's four slabs (Chan et al.), `colacc` = [4 slabs][2][BN].
-__device__ __forceinline__ void flush_tile_stats(const float* colacc, int bn_full, float* tile_stats, int l, int row_block, int row_blocks,
-                                                 int n_base, int N, int M, int etid) {
-  const int rows = M - row_block * 128;
-  for (int j = etid; j < bn_full; j += 32 * kEpiWarps) {
+// Per-tile column statistics -> global partials [L][row blocks of 128][N][2], then cleared for the next tile.
+__device__ __forceinline__ void flush_tile_stats(float* colacc, int bn_full, float* tile_stats, int l, int row_block, int row_blocks,
+                                                 int n_base, int N, int etid) {
+  for (int j = etid; j < bn_full; j += 128) {
     const int n = n_base + j;
-    if (n >= N || row_block >= row_blocks) continue;
-    float cnt = 0.f, mu = 0.f, m2 = 0.f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float nb = float(min(32, rows - 32 * q));
-      if (nb <= 0.f) break;
-      const float delta = colacc[2 * q * bn_full + j] - mu;
-      const float tot = cnt + nb;
-      m2 += fmaxf(colacc[(2 * q + 1) * bn_full + j], 0.f) + delta * delta * (cnt * nb / tot);
-      mu += delta * (nb / tot);
-      cnt = tot;
+    if (n < N && row_block < row_blocks) {
+      float2* dst = reinterpret_cast<float2*>(tile_stats) + (1LL * l * row_blocks + row_block) * N + n;
+      *dst = make_float2(colacc[j], colacc[bn_full + j]);
     }
-    *(reinterpret_cast<float2*>(tile_stats) + (1LL * l * row_blocks + row_block) * N + n) = make_float2(mu, m2);
+    colacc[j] = 0.f;
+    colacc[bn_full + j] = 0.f;
   }
 }
 
@@ -129,7 +112,7 @@ struct GemmShared {
   int abort_flag;
   int epi_ok;
   alignas(16) float bias[gemm::BN];
-  alignas(16) float colacc[4 * 2 * gemm::BN];
+  float colacc[2 * gemm::BN];
 };
 
 __global__ void __launch_bounds__(gemm::NUM_THREADS, 1)
@@ -141,8 +124,8 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   // 128-byte-swizzled tiles need 1024-byte alignment
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;  // one 4 KB staging tile per epilogue warp, 1024-byte aligned
-  GemmShared* sh = reinterpret_cast<GemmShared*>(epi_stage + kEpiWarps * kEpiStageBytes);
+  uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;  // four 4 KB staging tiles, 1024-byte aligned
+  GemmShared* sh = reinterpret_cast<GemmShared*>(epi_stage + 4 * kEpiStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -159,11 +142,12 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh->tmem_full[b], 1);
-      mbar_init(&sh->tmem_empty[b], kEpiWarps);
+      mbar_init(&sh->tmem_empty[b], 4);
     }
     sh->abort_flag = 0;
     fence_barrier_init();
   }
+  for (int j = threadIdx.x; j < 2 * BN; j += NUM_THREADS) sh->colacc[j] = 0.f;
   if (warp == 1) {
     tmem_alloc(&sh->tmem_base, TMEM_COLS);
     tmem_relinquish();
@@ -241,7 +225,6 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   } else {
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) belong to this warp
-    const int half = (warp - 2) >> 2;  // column half of the tile
     const int etid = (warp - 2) * 32 + lane;
     const int row_blocks = (M + 127) / 128;
     int prev_l = -1, prev_rb = 0, prev_n = 0;
@@ -253,30 +236,30 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int l = int(t / (1LL * tiles_m * tiles_n));
       const uint32_t buf = local_tile & 1;
       const uint32_t tph = (local_tile >> 1) & 1;
-      named_barrier_sync(1, 32 * kEpiWarps);  // previous tile's bias reads and column sums are done
-      if (tile_stats != nullptr && prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, M, etid);
+      named_barrier_sync(1, 128);  // previous tile's bias reads and column sums are done
+      if (tile_stats != nullptr && prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
       prev_l = l; prev_rb = mt; prev_n = nt * BN;
-      for (int j = etid; j < BN; j += 32 * kEpiWarps) {
+      for (int j = etid; j < BN; j += 128) {
         const int n = nt * BN + j;
         sh->bias[j] = (bias != nullptr && n < N) ? t16_to_float(bias[1LL * l * N + n]) : 0.f;
       }
       // One thread performs the bounded wait and publishes the outcome, so the four warps always
       // take the same branch and nobody is left alone at a named barrier.
       if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-      named_barrier_sync(1, 32 * kEpiWarps);
+      named_barrier_sync(1, 128);
       if (!sh->epi_ok) { ok = false; break; }
       tc_fence_after();
       const int m_base = mt * BM + quarter * 32;
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(quarter * 32) << 16);
-      if (m_base < M) epilogue_slab(taddr, &map_c, epi_stage + (warp - 2) * kEpiStageBytes, sh->bias, half * (BN / kEpiCols / 2), min((half + 1) * (BN / kEpiCols / 2), (N - nt * BN + kEpiCols - 1) / kEpiCols), nt * BN, m_base, l, lane,
-                                    tile_stats != nullptr ? sh->colacc + quarter * 2 * BN : nullptr, BN, min(32, M - m_base));
+      if (m_base < M) epilogue_slab(taddr, &map_c, epi_stage + (warp - 2) * kEpiStageBytes, sh->bias, min(BN, ((N - nt * BN + kEpiCols - 1) / kEpiCols) * kEpiCols), nt * BN, m_base, l, lane,
+                                    tile_stats != nullptr ? sh->colacc : nullptr, BN, min(32, M - m_base));
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->tmem_empty[buf]);
     }
     if (ok && tile_stats != nullptr && prev_l >= 0) {
-      named_barrier_sync(1, 32 * kEpiWarps);
-      flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, M, etid);
+      named_barrier_sync(1, 128);
+      flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
     }
   }
 
@@ -300,20 +283,20 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //   full[s]        leader only: armed by the leader's producer for the bytes of both CTAs
 //   empty[s]       both CTAs: commit (multicast) after the MMAs of the stage
 //   tmem_full[b]   both CTAs: commit (multicast) after the tile's last MMA
-//   tmem_empty[b]  leader only: one arrival per epilogue warp of both CTAs
+//   tmem_empty[b]  leader only: 8 arrivals, four epilogue warps of each CTA
 namespace gemm2 {
 constexpr int BM = 128;       // rows per CTA; the pair covers 256
 constexpr int BN = 256;
 constexpr int BN_HALF = 128;  // weight rows loaded per CTA
 constexpr int BK = 64;
-constexpr int STAGES = 5;
+constexpr int STAGES = 6;
 constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
 constexpr uint32_t B_BYTES = BN_HALF * BK * 2;
 constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int NUM_THREADS = 64 + 32 * kEpiWarps;
+constexpr int NUM_THREADS = 192;
 constexpr uint32_t TMEM_COLS = 512;
-constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + kEpiWarps * 4096 + 1024 + 10240;
+constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + 4 * 4096 + 1024 + 4096;
 }  // namespace gemm2
 
 struct GemmPairShared {
@@ -325,7 +308,7 @@ struct GemmPairShared {
   int abort_flag;
   int epi_ok;
   alignas(16) float bias[gemm2::BN];
-  alignas(16) float colacc[4 * 2 * gemm2::BN];
+  float colacc[2 * gemm2::BN];
 };
 
 __global__ void __launch_bounds__(gemm2::NUM_THREADS, 1)
@@ -337,7 +320,7 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;
-  GemmPairShared* sh = reinterpret_cast<GemmPairShared*>(epi_stage + kEpiWarps * kEpiStageBytes);
+  GemmPairShared* sh = reinterpret_cast<GemmPairShared*>(epi_stage + 4 * kEpiStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -358,11 +341,12 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh->tmem_full[b], 1);
-      mbar_init(&sh->tmem_empty[b], 2 * kEpiWarps);
+      mbar_init(&sh->tmem_empty[b], 8);
     }
     sh->abort_flag = 0;
     fence_barrier_init();
   }
+  for (int j = threadIdx.x; j < 2 * BN; j += NUM_THREADS) sh->colacc[j] = 0.f;
   if (warp == 1) {
     tmem_alloc_pair(&sh->tmem_base, TMEM_COLS);
     tmem_relinquish_pair();
@@ -431,7 +415,6 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   } else {
     // ---------------------------------------------------------------- epilogue (both CTAs)
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;
     const int etid = (warp - 2) * 32 + lane;
     const int row_blocks = (M + 127) / 128;
     int prev_l = -1, prev_rb = 0, prev_n = 0;
@@ -443,28 +426,28 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int l = int(t / (1LL * tiles_m * tiles_n));
       const uint32_t buf = local_tile & 1;
       const uint32_t tph = (local_tile >> 1) & 1;
-      named_barrier_sync(1, 32 * kEpiWarps);
-      if (tile_stats != nullptr && prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, M, etid);
+      named_barrier_sync(1, 128);
+      if (tile_stats != nullptr && prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
       prev_l = l; prev_rb = mt * 2 + int(cta_rank); prev_n = nt * BN;
-      for (int j = etid; j < BN; j += 32 * kEpiWarps) {
+      for (int j = etid; j < BN; j += 128) {
         const int n = nt * BN + j;
         sh->bias[j] = (bias != nullptr && n < N) ? t16_to_float(bias[1LL * l * N + n]) : 0.f;
       }
       if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-      named_barrier_sync(1, 32 * kEpiWarps);
+      named_barrier_sync(1, 128);
       if (!sh->epi_ok) { ok = false; break; }
       tc_fence_after();
       const int m_base = (mt * 2 + int(cta_rank)) * BM + quarter * 32;
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(quarter * 32) << 16);
-      if (m_base < M) epilogue_slab(taddr, &map_c, epi_stage + (warp - 2) * kEpiStageBytes, sh->bias, half * (BN / kEpiCols / 2), min((half + 1) * (BN / kEpiCols / 2), (N - nt * BN + kEpiCols - 1) / kEpiCols), nt * BN, m_base, l, lane,
-                                    tile_stats != nullptr ? sh->colacc + quarter * 2 * BN : nullptr, BN, min(32, M - m_base));
+      if (m_base < M) epilogue_slab(taddr, &map_c, epi_stage + (warp - 2) * kEpiStageBytes, sh->bias, min(BN, ((N - nt * BN + kEpiCols - 1) / kEpiCols) * kEpiCols), nt * BN, m_base, l, lane,
+                                    tile_stats != nullptr ? sh->colacc : nullptr, BN, min(32, M - m_base));
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&sh->tmem_empty[buf]), 0));  // the leader's barrier
     }
     if (ok && tile_stats != nullptr && prev_l >= 0) {
-      named_barrier_sync(1, 32 * kEpiWarps);
-      flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, M, etid);
+      named_barrier_sync(1, 128);
+      flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
     }
   }
 
@@ -513,8 +496,8 @@ static bool make_kmajor_map(CUtensorMap* map, const void* base, int layers, int 
 }  // namespace clt
 
 // Returns 0 on success, a negative value when the arguments cannot be handled (the caller raises).
-// tile_stats (optional): [L][ceil(M / 128)][N][2] fp32, receives per 128-row block and column the mean and the sum of
-// squared deviations of the stored (rounded) outputs; every element is written, nothing has to be cleared.
+// tile_stats (optional): [L][ceil(M / 128)][N][2] fp32, receives per 128-row block and column the sum and the sum of
+// squares of the stored (bf16-rounded) outputs; every element is written, nothing has to be cleared.
 extern "C" int CLT_FN(clt_encoder_gemm)(const void* A, const void* B, const void* bias, void* C, int L, int M, int N, int K,
                                 long long ldc, long long layer_stride_c, int* status, float* tile_stats, int num_sms, cudaStream_t stream) {
   using namespace clt;

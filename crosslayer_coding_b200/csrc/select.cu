@@ -123,8 +123,9 @@ __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x
 }
 
 // Column statistics from the per-block sums that the encoder GEMM's epilogue leaves behind:
-// tile_stats [L][row_blocks][F][2] = (mean, sum of squared deviations) over the rows of one 128-row block.  The blocks are merged
-// with the pairwise update of Chan et al., which keeps the variance accurate when the mean is large against the spread.
+// tile_stats [L][row_blocks][F][2] = (sum, sum of squares) over the rows of one 128-row block.  The blocks are merged
+// with the pairwise update of Chan et al. (block means first), which keeps the variance accurate when the mean is
+// large against the spread.
 __global__ void __launch_bounds__(256) colstats_from_tiles_kernel(const float* __restrict__ tile_stats, float* __restrict__ mean,
                                                                     float* __restrict__ rstd, int B, int F, int row_blocks, long long n) {
   const long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x;
@@ -132,13 +133,14 @@ __global__ void __launch_bounds__(256) colstats_from_tiles_kernel(const float* _
   const int l = int(i / F), c = int(i - 1LL * l * F);
   const float2* src = reinterpret_cast<const float2*>(tile_stats) + (1LL * l * row_blocks) * F + c;
   float cnt = 0.f, mu = 0.f, m2 = 0.f;
-#pragma unroll 8
   for (int rb = 0; rb < row_blocks; ++rb) {
-    const float2 sq = __ldcs(src + 1LL * rb * F);
+    const float2 sq = src[1LL * rb * F];
     const float nb = float(min(128, B - rb * 128));
+    const float mb = sq.x / nb;
+    const float m2b = fmaxf(sq.y - sq.x * mb, 0.f);
     const float tot = cnt + nb;
-    const float delta = sq.x - mu;
-    m2 += sq.y + delta * delta * (cnt * nb / tot);
+    const float delta = mb - mu;
+    m2 += m2b + delta * delta * (cnt * nb / tot);
     mu += delta * (nb / tot);
     cnt = tot;
   }

@@ -80,9 +80,7 @@ class SparseForward:
         self.ent_tok = torch.empty(cap, dtype=i32, device=dev)
         self.ent_col = torch.empty(cap, dtype=i32, device=dev)
         self.ent_val = torch.empty(cap, dtype=f32, device=dev)
-        self.tile_stats = None  # column statistics of the GEMM's 128-row blocks, for the selections that rank z-scores
         if self.fn in ("batchtopk", "topk"):
-            self.tile_stats = torch.empty(L, (B + 127) // 128, Fl, 2, dtype=f32, device=dev)
             self.mean = torch.empty(L, Fl, dtype=f32, device=dev)
             self.rstd = torch.empty(L, Fl, dtype=f32, device=dev)
         if self.fn == "batchtopk":
@@ -140,14 +138,14 @@ class SparseForward:
         e, m = self.ext, self.model
         assert X.dtype == torch.bfloat16 and X.shape == (self.L, self.B, self.d), (X.dtype, tuple(X.shape))
         (self._zeroed if clear_loss else self._zeroed_encode).zero_()
-        e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, self.tile_stats)
-        if self.tile_stats is not None:
-            e.colstats_from_tiles(self.tile_stats, self.mean, self.rstd, self.B)
+        e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, None)
         if self.fn == "batchtopk":
+            e.colstats(self.preact, self.mean, self.rstd)
             e.batchtopk_select(self.preact, self.mean, self.rstd, self.Fl, self.Fl, 0, self.Fl, self.k_total, self.key_lo, self.shift,
                                self.hist, self.ctl, self.ent_tok, self.ent_col, self.ent_val, self.cand[0], self.cand[1], self.cand[2],
                                self.cand[3], self.status, 1, 0, [], [], 0, 0, self.sel_state, self.pool)
         elif self.fn == "topk":
+            e.colstats(self.preact, self.mean, self.rstd)
             e.token_topk_select(self.preact, self.mean, self.rstd, self.Fl, self.k_token, self.ctl, self.ent_tok, self.ent_col,
                                 self.ent_val, self.status)
         else:
