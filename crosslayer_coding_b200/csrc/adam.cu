@@ -368,7 +368,8 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
 // whole rows between global and shared memory with 1-D bulk copies (cp.async.bulk, no multicast): row in
 // (w, m, v and the gradient-seed rows of the feature's first four entries) -> consumers update the row in
 // place in shared memory -> row out.  The ring keeps several rows per CTA in flight in both directions and
-// the consumers never wait on a global load, except for the rare feature with more than four entries.
+// the consumers only wait on global loads for features with more than four entries.
+// Entries beyond the staged ones are gathered by the consumers in batches, see add_entries.
 // Every mbarrier wait is bounded; a timeout sets the status word and drains the copies in flight.
 constexpr int kAdamStages = 4;  // at most; rows above 24 KB per stage run with three so that two CTAs fit an SM
 constexpr int kAdamSlots = 4;  // gradient-seed rows per stage
@@ -449,8 +450,77 @@ __device__ __forceinline__ void stbf(t16* p, const float (&o)[EPT], unsigned int
   }
 }
 
-template <typename WT, bool SR, int EPT, typename MT>
-__global__ void __launch_bounds__(288) decoder_rows_adam_bulk_kernel(const DecAdamParams p, int gthreads, int stage_bytes, int ns, int* status) {
+// Warp sums of N values at once (N a power of two up to 32): every exchange halves the number of values a lane still carries,
+// N - 1 + 5 - log2(N) shuffles instead of 5 N.  Returns the total of value warp_sum_slot<N>(lane); the tree is warp_sum's.
+template <int N>
+__device__ __forceinline__ float warp_sum_many(float (&v)[N], int lane) {
+  int o = 16;
+#pragma unroll
+  for (int half = N / 2; half >= 1; half >>= 1, o >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float send = upper ? v[i] : v[i + half];
+      const float keep = upper ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+    }
+  }
+  float r = v[0];
+#pragma unroll
+  for (int q = 16 / N; q >= 1; q >>= 1) r += __shfl_xor_sync(0xFFFFFFFFu, r, q);
+  return r;
+}
+template <int N>
+__device__ __forceinline__ int warp_sum_slot(int lane) { return lane / (32 / N); }
+
+// g += a_j * seed_j and dL/da of the entries of one batch: lane j of the warp holds entry j (its slot in the CSR arrays, token and
+// activation), cnt of them.  The seed rows come kBatch at a time, so a feature with many entries waits for L2 once per
+// kBatch of them and not twice per entry (eight entries per feature on average, tied Pythia-70m shape: both sweeps of a step
+// 1.81 -> 1.60 ms).  It takes 72 registers; a cap of 64 spills and cost 0.4 ms at the GPT-2 shape.
+template <int EPT>
+__device__ __forceinline__ void add_entries(int cnt, int my_x, int my_tok, float my_a, const t16* gs_t, int d, bool act, int lane, const float (&w)[EPT],
+                                            float (&g)[EPT], float* grad_a, float gsc) {
+  constexpr int kBatch = 4;
+  for (int j0 = 0; j0 < cnt; j0 += kBatch) {
+    uint2 q2[kBatch][EPT / 4];
+    float dot[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const int tok = __shfl_sync(0xFFFFFFFFu, my_tok, j0 + k);
+      if (act && j0 + k < cnt) {
+#pragma unroll
+        for (int z = 0; z < EPT / 4; ++z) q2[k][z] = __ldg(reinterpret_cast<const uint2*>(gs_t + 1LL * tok * d) + z);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) {
+      const float a = __shfl_sync(0xFFFFFFFFu, my_a, j0 + k);
+      dot[k] = 0.f;
+      if (act && j0 + k < cnt) {
+#pragma unroll
+        for (int z = 0; z < EPT / 4; ++z) {
+          const float gv[4] = {t16_lo(q2[k][z].x), t16_hi(q2[k][z].x), t16_lo(q2[k][z].y), t16_hi(q2[k][z].y)};
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            g[4 * z + c] = fmaf(a, gv[c], g[4 * z + c]);
+            dot[k] = fmaf(gv[c], w[4 * z + c], dot[k]);
+          }
+        }
+      }
+    }
+    if (grad_a != nullptr) {
+      const float sdot = warp_sum_many<kBatch>(dot, lane);
+      const int k = j0 + warp_sum_slot<kBatch>(lane);
+      const int x = __shfl_sync(0xFFFFFFFFu, my_x, k);
+      if (lane % (32 / kBatch) == 0 && k < cnt && sdot != 0.f) atomicAdd(&grad_a[x], sdot * gsc);
+    }
+  }
+}
+
+// PT: per-target tied decoders (one row per feature and target layer, shared by the source layers below): the entries of a row
+// come from several CSR segments, so none are staged in slots.
+template <typename WT, bool SR, int EPT, typename MT, bool PT = false>
+__global__ void __launch_bounds__(288, EPT == 4 ? 3 : 2) decoder_rows_adam_bulk_kernel(const DecAdamParams p, int gthreads, int stage_bytes, int ns, int* status) {
   extern __shared__ __align__(128) uint8_t smem_raw_adam[];  // bulk copies need 16-byte alignment only
   uint8_t* ring = smem_raw_adam;
   AdamBulkShared* sh = reinterpret_cast<AdamBulkShared*>(ring + size_t(ns) * stage_bytes);
@@ -512,7 +582,7 @@ __global__ void __launch_bounds__(288) decoder_rows_adam_bulk_kernel(const DecAd
       const int st = i % ns;
       uint8_t* stage = ring + size_t(st) * stage_bytes;
       AdamStageHdr* h = reinterpret_cast<AdamStageHdr*>(stage);
-      const int ne = cur.e - cur.b;
+      const int ne = PT ? 0 : cur.e - cur.b;
       const long long elem_off = (1LL * f * R + r) * d;
       h->ne = ne; h->b = cur.b; h->col = ti * Fp + f; h->ti = ti; h->r = r; h->R = R; h->elem_off = elem_off;
 #pragma unroll
@@ -587,6 +657,7 @@ __global__ void __launch_bounds__(288) decoder_rows_adam_bulk_kernel(const DecAd
         for (int j = 0; j < kAdamSlots; ++j) dacc[j] = 0.f;
         norm2 = 0.f;
         pc = p.pen_coef ? __ldg(p.pen_coef + col) : 0.f;
+        if (PT && p.pen_coef) pc = warp_sum(lane <= ti ? __ldg(p.pen_coef + lane * Fp + col - ti * Fp) : 0.f);  // the row is part of the norms of all sources
       }
       float w[EPT], m[EPT], v[EPT], g[EPT];
 #pragma unroll
@@ -619,21 +690,37 @@ __global__ void __launch_bounds__(288) decoder_rows_adam_bulk_kernel(const DecAd
           }
         }
       }
-      for (int x = b + kAdamSlots; x < b + ne; ++x) {  // rare: features with more entries than slots
-        float dot = 0.f;
-        if (act) {
-          const float a = __ldg(p.fcsr_val + x);
-          float gv[EPT];
-          ldbf_global<EPT>(p.gs + (1LL * (ti + r) * B + __ldg(p.fcsr_tok + x)) * d + e0, gv);
-#pragma unroll
-          for (int q = 0; q < EPT; ++q) {
-            g[q] = fmaf(a, gv[q], g[q]);
-            dot = fmaf(gv[q], w[q], dot);
-          }
+      if (PT) {
+        // the entries of feature f in all source layers s <= ti, one CSR segment per layer: the lanes hold the segments, and
+        // entry j of their concatenation lies in the segment whose inclusive count is the first above j
+        const int f = col - ti * Fp;
+        int seg_b = 0, seg_n = 0;
+        if (lane <= ti) {
+          seg_b = __ldg(p.feat_off + lane * Fp + f);
+          seg_n = __ldg(p.feat_off + lane * Fp + f + 1) - seg_b;
         }
-        if (p.grad_a != nullptr) {
-          dot = warp_sum(dot);
-          if (lane == 0 && dot != 0.f) atomicAdd(&p.grad_a[x], dot * gsc);
+        int incl = seg_n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+          if (lane >= o) incl += up;
+        }
+        const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        for (int j0 = 0; j0 < total; j0 += 32) {
+          const int j = j0 + lane;
+          int seg = 0;
+          for (int s = 0; s < ti; ++s) seg += __shfl_sync(0xFFFFFFFFu, incl, s) <= j ? 1 : 0;
+          const int x = __shfl_sync(0xFFFFFFFFu, seg_b, seg) + j - (__shfl_sync(0xFFFFFFFFu, incl, seg) - __shfl_sync(0xFFFFFFFFu, seg_n, seg));
+          const int my_tok = j < total ? __ldg(p.fcsr_tok + x) : 0;
+          const float my_a = j < total ? __ldg(p.fcsr_val + x) : 0.f;
+          add_entries<EPT>(min(32, total - j0), x, my_tok, my_a, p.gs + 1LL * ti * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
+        }
+      } else {
+        for (int x0 = b + kAdamSlots; x0 < b + ne; x0 += 32) {  // entries beyond the slots
+          const int cnt = min(32, b + ne - x0);
+          const int my_tok = lane < cnt ? __ldg(p.fcsr_tok + x0 + lane) : 0;
+          const float my_a = lane < cnt ? __ldg(p.fcsr_val + x0 + lane) : 0.f;
+          add_entries<EPT>(cnt, x0 + lane, my_tok, my_a, p.gs + 1LL * (ti + r) * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
         }
       }
       if (act) {
@@ -652,11 +739,16 @@ __global__ void __launch_bounds__(288) decoder_rows_adam_bulk_kernel(const DecAd
           float gq = fmaf(pc, w[q], g[q] * gsc);
           if (extra) gq += dg0[q];
           adam1(w[q], m[q], v[q], gq * sc.clip, hr);
-          norm2 = fmaf(w[q], w[q], norm2);
+          if (!PT) norm2 = fmaf(w[q], w[q], norm2);
         }
         const unsigned long long gidx = (unsigned long long)(p.row_start[ti] * d + h->elem_off + e0);
         if (sizeof(WT) == 2) stbf<EPT, SR>(reinterpret_cast<t16*>(w_s), w, p.h.sr_seed, (unsigned int)gidx);
         else stf<EPT>(reinterpret_cast<float*>(w_s), w);
+        if (PT) {  // norms of the stored (rounded) weights
+          ldbf<EPT>(reinterpret_cast<const t16*>(w_s), w);
+#pragma unroll
+          for (int q = 0; q < EPT; ++q) norm2 = fmaf(w[q], w[q], norm2);
+        }
         if (sizeof(MT) == 2) {
           // bf16 moments are always rounded stochastically: with beta2 = 0.999 a nearest rounding would freeze v
           // one hash per thread and row seeds a linear congruential stream: two 16-bit dither values per element
@@ -682,15 +774,10 @@ __global__ void __launch_bounds__(288) decoder_rows_adam_bulk_kernel(const DecAd
         }
       }
       if (r == R - 1) {
-        if (p.grad_a != nullptr) {
-          const int nslot = ne < kAdamSlots ? ne : kAdamSlots;
-#pragma unroll
-          for (int j = 0; j < kAdamSlots; ++j) {
-            if (j < nslot) {
-              const float sdot = warp_sum(dacc[j]);
-              if (lane == 0 && sdot != 0.f) atomicAdd(&p.grad_a[b + j], sdot * gsc);
-            }
-          }
+        if (!PT && p.grad_a != nullptr) {
+          const float sdot = warp_sum_many<kAdamSlots>(dacc, lane);  // the sums of slots without an entry are zero
+          const int j = warp_sum_slot<kAdamSlots>(lane);
+          if (lane % (32 / kAdamSlots) == 0 && j < ne && sdot != 0.f) atomicAdd(&p.grad_a[b + j], sdot * gsc);
         }
         if (p.norm2_out != nullptr) {
           const float sn = warp_sum(norm2);
@@ -1156,20 +1243,25 @@ static bool bulk_rows_adam_fits(int d, int weights_bf16) {
   size_t smem;
   return bulk_rows_adam_geometry(d, weights_bf16 != 0, false, &ept, &gthreads, &stage_bytes, &smem) != 0;
 }
-static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool sr, int num_sms, int* status, cudaStream_t st) {
+static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool sr, int num_sms, int* status, cudaStream_t st, bool per_target = false) {
   int ept, gthreads, stage_bytes;
   size_t smem;
   const bool mb = p.moments_bf16 != 0;
   if (mb && !weights_bf16) return -1;  // bf16 moments go with bf16 weights
   int nstages = kAdamStages;
   if (!bulk_rows_adam_geometry(p.d, weights_bf16, mb, &ept, &gthreads, &stage_bytes, &smem, &nstages)) return -1;
-  int per_sm = int((227 * 1024) / (smem + 1024));
-  const int by_threads = 2048 / (gthreads + 32);
-  per_sm = per_sm > by_threads ? by_threads : per_sm;
-  per_sm = per_sm < 1 ? 1 : (per_sm > 6 ? 6 : per_sm);
-  int bgrid = num_sms * per_sm;
-  if (bgrid > p.F_pitch) bgrid = p.F_pitch;
-  {
+  auto launch = [&](auto kern, int which) -> int {
+    static size_t attr_set[14] = {};
+    if (attr_set[which] < smem) {
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
+      attr_set[which] = smem;
+    }
+    // resident CTAs per SM from the runtime (shared memory, threads and registers together): a grid beyond them would run a
+    // second wave of CTAs over features that were dealt out evenly
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, gthreads + 32, smem) != cudaSuccess || per_sm < 1) return -4;
+    int bgrid = num_sms * (per_sm > 6 ? 6 : per_sm);
+    if (bgrid > p.F_pitch) bgrid = p.F_pitch;
     // CTA b owns the features b, b + grid, ... of every tensor: pick the grid (between half of the resident slots and all
     // of them) that splits the features most evenly, so that no CTA still streams rows when the others are done.  On a
     // narrow shard (3072 features, 888 slots) the naive grid leaves CTAs with 3 and with 4 features per tensor.
@@ -1180,18 +1272,14 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
       const double waste = double(per) * g / double(p.F_pitch);
       if (waste < best_waste - 1e-9) { best_waste = waste; best = g; }
     }
-    bgrid = best;
-  }
-  auto launch = [&](auto kern, int which) -> int {
-    static size_t attr_set[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (attr_set[which] < smem) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
-      attr_set[which] = smem;
-    }
-    kern<<<bgrid, gthreads + 32, smem, st>>>(p, gthreads, stage_bytes, nstages, status);
+    kern<<<best, gthreads + 32, smem, st>>>(p, gthreads, stage_bytes, nstages, status);
     return 0;
   };
   using bf = t16;
+  if (per_target) {
+    if (ept == 4) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, float, true>, 10) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, float, true>, 11);
+    return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, float, true>, 12) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, float, true>, 13);
+  }
   if (mb) {
 #if CLT_T16_IS_HALF
     return -6;  // bf16 moments go with bf16 weights
@@ -1244,6 +1332,11 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   }
   if (a->tying == 0 && a->status != nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16) && acc * a->d < (1LL << 62)) {
     const int rc = launch_rows_adam_bulk(p, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st);
+    if (rc != 0) return rc;
+  } else if (a->tying == 2 && a->status != nullptr && a->weights_bf16 && a->L <= 32 && a->ntensors == a->L && a->feat_offset == nullptr &&
+             a->feat_scale == nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16)) {
+    // per-target tied rows without affine terms: the row pipeline too (their entries are gathered by the consumers)
+    const int rc = launch_rows_adam_bulk(p, true, a->h.sr_seed != 0, num_sms, a->status, st, true);
     if (rc != 0) return rc;
   } else if (a->tying == 0) {
     const bool sr = a->h.sr_seed != 0;

@@ -215,3 +215,64 @@ def test_threshold_statistics_match_the_dense_form(ext, fn):
     assert float((sparse["cnt_min"] != dense["cnt_min"]).float().mean()) < 0.02
     same = sparse["cnt_min"] == dense["cnt_min"]
     assert float(((sparse["sum_min"] - dense["sum_min"]).abs()[same] > 0.05).float().mean()) < 0.02
+
+
+HYPER = [1e-3, 0.9, 0.999, 1e-8, 0.01, 1 - 0.9 ** 3, 1 - 0.999 ** 3, 1.0, 0.5, 0.0, 1.0]
+
+
+# entry counts around the four staged slots, the batches of four and the 32 a warp fetches at once; d with idle lanes, with four
+# and with eight elements per thread
+@pytest.mark.parametrize("tying", [0, 2])
+@pytest.mark.parametrize("L,B,d", [(3, 90, 64), (2, 90, 520), (4, 70, 768), (2, 60, 1536)])
+def test_decoder_row_update(ext, L, B, d, tying):
+    dev = _dev()
+    g = torch.Generator().manual_seed(d + tying)
+    counts = [0, 1, 3, 4, 5, 7, 8, 9, 35, 36, 37, 60, 0, 2]
+    F = len(counts)
+    ent = [(l * F + f, t) for l in range(L) for f, c in enumerate(counts) for t in torch.randperm(B, generator=g)[:c].tolist()]
+    col = torch.tensor([e[0] for e in ent], dtype=I32, device=dev)
+    tok = torch.tensor([e[1] for e in ent], dtype=I32, device=dev)
+    val = torch.randn(len(ent), generator=g).to(dev)
+    c = _csr(ext, tok, col, val, B, L * F, F)
+    rows = [L - s if tying == 0 else 1 for s in range(L)]
+    W = [(torch.randn(F, r, d, generator=g) / 8).bfloat16().to(dev) for r in rows]
+    M = [(torch.randn(F, r, d, generator=g) * 0.01).to(dev) for r in rows]
+    V = [(torch.rand(F, r, d, generator=g) * 1e-3 + 1e-4).to(dev) for r in rows]
+    gs = torch.randn(L, B, d, generator=g).bfloat16().to(dev)
+    pen = (torch.rand(L * F, generator=g) * 0.01).to(dev)
+    acts = torch.zeros(L, B, F, device=dev, dtype=torch.float64)
+    acts[(col // F).long(), tok.long(), (col % F).long()] = val.double()
+    gsc, (lr, b1, b2, eps, wd, bc1, bc2) = HYPER[8], HYPER[:7]
+    want, norm2 = [], []
+    dlda = torch.zeros(L, B, F, device=dev, dtype=torch.float64)
+    for i in range(L):
+        grad = torch.zeros(F, rows[i], d, device=dev, dtype=torch.float64)
+        for r in range(rows[i]):
+            t = i + r if tying == 0 else i
+            for s in ([i] if tying == 0 else range(i + 1)):
+                grad[:, r] += gsc * acts[s].t() @ gs[t].double()
+                dlda[s] += gsc * gs[t].double() @ W[i][:, r].double().t()
+        pc = pen.view(L, F).double()
+        grad += (pc[i] if tying == 0 else pc[: i + 1].sum(0))[:, None, None] * W[i].double()
+        m = b1 * M[i].double() + (1 - b1) * grad
+        v = b2 * V[i].double() + (1 - b2) * grad.square()
+        w = W[i].double() * (1 - lr * wd) - lr / bc1 * m / ((v / bc2).sqrt() + eps)
+        want.append((w, m, v))
+    grad_a = torch.zeros(len(ent), device=dev)
+    n2 = torch.zeros(L * F, device=dev)
+    status = torch.zeros(4, dtype=I32, device=dev)
+    ext.decoder_rows_adam(W, M, V, L, B, d, F, tying, c["feat_off"], c["fcsr_tok"], c["fcsr_val"], gs, grad_a, pen, n2, None, None, None, HYPER, status, None,
+                          None, None, False, None, None)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    for i in range(L):
+        w, m, v = want[i]
+        # m, v: fp32 sums of up to 60 * L products of unit size, 2^-24 each (1 - beta is itself rounded to 2^-24 of one, a relative
+        # 6e-5 of 0.001); w: one bf16 rounding
+        assert (M[i].double() - m).abs().max() < 4e-6 * m.abs().max() and (V[i].double() - v).abs().max() < 1e-4 * v.abs().max()
+        assert ((W[i].double() - w).abs() <= 2 ** -8 * w.abs() + 1e-7).all()
+        # norms of the updated rows: 2^-9 relative rounding per weight, averaged over the row
+        assert torch.allclose(n2.view(L, F)[i].double(), W[i].double().square().sum((1, 2)), rtol=2e-3)
+    order = torch.argsort(col.long() * B + tok.long())
+    got_l, got_f, got_t = (col[order] // F).long(), (col[order] % F).long(), tok[order].long()
+    assert (grad_a.double() - dlda[got_l, got_t, got_f]).abs().max() < 1e-5 * dlda.abs().max()
