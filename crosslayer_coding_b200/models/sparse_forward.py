@@ -129,7 +129,9 @@ class SparseForward:
     # ------------------------------------------------------------------ selection
     def _theta(self) -> torch.Tensor:
         if self.fn == "jumprelu":
-            torch.exp(self.model.log_threshold.data, out=self.theta)  # re-read on every call: the parameter may have changed
+            # re-read on every call: the parameter may have changed.  In fp32 also for a 16-bit parameter: `exp` computes in its
+            # input's type, and a threshold rounded to eight bits moves entries across it
+            torch.exp(self.model.log_threshold.data.float(), out=self.theta)
         return self.theta
 
     @torch.no_grad()

@@ -194,6 +194,26 @@ def test_sparse_forward_with_and_without_targets(ext, fn, tying):
     sf.check_status()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32, torch.float64])
+def test_thresholds_are_computed_in_32_bits(ext, dtype):
+    """``model.bfloat16()`` turns ``log_threshold`` into a 16-bit parameter; the threshold is its exponential in fp32 all the same."""
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model("jumprelu", "none", dev)
+    with torch.no_grad():
+        # a fifth to four times the spread of the pre-activations; the exponentials of 16-bit values lie between 16-bit values
+        model.log_threshold.data = (3.0 * torch.rand(3, 512, device=dev) - 4.0).to(dtype)
+    sf = SparseForward(model, 200)
+    x = torch.randn(3, 200, 64, device=dev).bfloat16()
+    sf.encode(x)
+    sf.check_status()
+    theta = model.log_threshold.data.double().exp()
+    assert ((sf.theta.double() / theta - 1).abs() <= 2.0 ** -22).all()  # fp32: 2^-24, and the error bound of expf (2 ulp)
+    want = torch.where(sf.preact.float() >= model.log_threshold.data.float().exp()[:, None, :], sf.preact.float(), torch.zeros((), device=dev))
+    assert torch.equal(sf.activations_dense(), want)
+
+
 @pytest.mark.parametrize("fn", ["batchtopk", "topk"])
 def test_threshold_statistics_match_the_dense_form(ext, fn):
     from crosslayer_coding_b200.models import theta
