@@ -84,8 +84,25 @@ def accumulate_theta_batch_sparse(sf, X: torch.Tensor, stats: Dict[str, torch.Te
     every feature come from the selection's column statistics, the per-feature minimum of the selected z-scores from the
     feature-major entry list, one kernel - no dense ``[B, L*F]`` selection, which is what the dense path spends its time on."""
     sf.encode(X)
-    sf.ext.theta_accumulate(sf.feat_off, sf.fcsr_val, sf.mean, sf.rstd, act.ZSCORE_EPS, stats["sum_min"], stats["cnt_min"], stats["mean"],
-                            stats["std"], stats["batches"])
+    names = ("sum_min", "cnt_min", "mean", "std")
+
+    def accumulate(into: Dict[str, torch.Tensor]) -> None:
+        sf.ext.theta_accumulate(sf.feat_off, sf.fcsr_val, sf.mean, sf.rstd, act.ZSCORE_EPS, into["sum_min"], into["cnt_min"], into["mean"],
+                                into["std"], into["batches"])
+
+    width = stats["sum_min"].shape[-1]
+    planes = all(stats[n].dtype == torch.float32 and stats[n].is_contiguous() and stats[n].shape == (sf.L, width) for n in names)
+    counts = stats["batches"]
+    if planes and width <= sf.Fl and torch.is_tensor(counts) and counts.dtype == torch.float32 and counts.is_contiguous() and counts.numel() == sf.L:
+        accumulate(stats)
+        return
+    # sums of another type, stride or width (64-bit accumulators, a view of a wider table): this batch's statistics on their own, then added
+    batch = {n: torch.zeros(sf.L, sf.Fl, dtype=torch.float32, device=X.device) for n in names}
+    batch["batches"] = torch.zeros(sf.L, dtype=torch.float32, device=X.device)
+    accumulate(batch)
+    for n in names:
+        stats[n] += batch[n][:, : stats[n].shape[1]]
+    stats["batches"] += 1
 
 
 @torch.no_grad()

@@ -237,6 +237,31 @@ def test_threshold_statistics_match_the_dense_form(ext, fn):
     assert float(((sparse["sum_min"] - dense["sum_min"]).abs()[same] > 0.05).float().mean()) < 0.02
 
 
+def test_threshold_statistics_of_any_type_and_stride(ext):
+    """The sums may be 64-bit, a view of a wider table, or narrower than the shard: every form gets what the fp32 planes get."""
+    from crosslayer_coding_b200.models import theta
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model("batchtopk", "none", dev)
+    sf = SparseForward(model, 150)
+    x = torch.randn(3, 150, 64, device=dev).bfloat16()
+    want = theta._new_stats(model)
+    theta.accumulate_theta_batch_sparse(sf, x, want)
+    names = ("sum_min", "cnt_min", "mean", "std")
+    double = {n: t.double() for n, t in theta._new_stats(model).items()}
+    table = torch.zeros(4, 3, 1024, device=dev)
+    views = {n: table[i][:, 256:768] for i, n in enumerate(names)} | {"batches": torch.zeros(6, device=dev)[::2]}
+    narrow = {n: torch.zeros(3, 200, device=dev, dtype=torch.float64) for n in names} | {"batches": torch.zeros((), device=dev)}
+    for stats, width in ((double, 512), (views, 512), (narrow, 200)):
+        theta.accumulate_theta_batch_sparse(sf, x, stats)
+        for n in names:
+            assert torch.equal(stats[n].float(), want[n][:, :width]), n
+        assert bool((stats["batches"] == 1).all())
+    assert float(table[:, :, :256].abs().sum() + table[:, :, 768:].abs().sum()) == 0.0
+    sf.check_status()
+
+
 HYPER = [1e-3, 0.9, 0.999, 1e-8, 0.01, 1 - 0.9 ** 3, 1 - 0.999 ** 3, 1.0, 0.5, 0.0, 1.0]
 
 
