@@ -488,8 +488,9 @@ void sparse_decode(const std::vector<Tensor>& dec_w, int64_t L, int64_t B, int64
   } else if (mode == 0) {
     TORCH_CHECK(a.yhat_partial != nullptr, "mode 0 needs yhat_partial");
   } else {
-    // without a target there is no loss: the reconstruction is the only output
-    TORCH_CHECK(a.bias_sum && ((a.target && a.gs && a.sq_err) || (!a.target && a.yhat_out)), "mode 1 needs bias_sum and either target, gs, sq_err or yhat_out alone");
+    // without a target there is no loss: the reconstruction is the only output, and outputs that would stay unwritten are refused
+    TORCH_CHECK(a.bias_sum && (a.target ? a.gs && a.sq_err : a.yhat_out && !a.gs && !a.sq_err),
+                "mode 1 needs bias_sum and either target, gs and sq_err, or yhat_out without the three");
   }
   c10::cuda::CUDAGuard guard(tok_off.device());
   check(CLT_PICK(half, clt_sparse_decode)(&a, cur_stream()), "sparse_decode");

@@ -89,6 +89,28 @@ def test_gather_decode_matches_dense(ext, L, B, d, tying, affine):
     assert int(status[0]) == 0
 
 
+def test_decode_refuses_loss_outputs_without_a_target(ext):
+    """Without a target neither the gradient seed nor the error sums are written: a call that hands them in is an error."""
+    dev = _dev()
+    L, B, d, F = 2, 3, 64, 24
+    g = torch.Generator().manual_seed(0)
+    c = _csr(ext, *_entries(g, L, B, F, 20, dev), B, L * F, F)
+    W = [torch.randn(F, L - s, d, generator=g).bfloat16().to(dev) for s in range(L)]
+    bias, yhat = torch.zeros(L, d, device=dev), torch.empty(L, B, d, device=dev)
+    gs, sq = torch.empty(L, B, d, device=dev, dtype=torch.bfloat16), torch.zeros(L, device=dev, dtype=torch.float64)
+    target = torch.zeros(L, B, d, device=dev, dtype=torch.bfloat16)
+
+    def call(target, gs, yhat, sq):
+        ext.sparse_decode(W, L, B, d, F, 0, c["tok_off"], c["tcsr_col"], c["tcsr_val"], None, None, None, bias, None, target, None, gs, yhat, sq, 1, [], 0, 0,
+                          torch.zeros(4, dtype=I32, device=dev))
+
+    for bad in ((None, gs, yhat, sq), (None, gs, yhat, None), (None, None, yhat, sq), (None, None, None, None), (target, None, yhat, sq), (target, gs, yhat, None)):
+        with pytest.raises(RuntimeError, match="mode 1"):
+            call(*bad)
+    call(None, None, yhat, None)
+    call(target, gs, None, sq)
+
+
 # long segments in shared memory, ranges beyond it, one feature per CTA, tokens beyond the token sort's buffer
 @pytest.mark.parametrize("B,L,F,n", [(40, 2, 300, 900), (3000, 1, 8, 20000), (5000, 1, 2, 9000), (9000, 1, 3, 27000), (2, 2, 4000, 9000), (700, 3, 512, 200000)])
 def test_csr_segments_are_sorted(ext, B, L, F, n):
