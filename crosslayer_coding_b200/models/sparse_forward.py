@@ -164,7 +164,10 @@ class SparseForward:
         self.encode(X, clear_loss=True)
         e, m = self.ext, self.model
         yhat = torch.empty(self.L, self.B, self.d, dtype=torch.float32, device=self.dev)
-        e.step_finish(None, None, m.dec_bias.data, self.bias_sel, self.bias_sum)
+        bias = m.dec_bias.data
+        if bias.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not bias.is_contiguous():
+            bias = bias.float().contiguous()  # the types and the layout the kernel reads
+        e.step_finish(None, None, bias, self.bias_sel, self.bias_sum)
         off = scale = None
         if m.feature_offset is not None:
             off = m.feature_offset.data.float().contiguous()

@@ -217,6 +217,26 @@ def test_sparse_forward_with_and_without_targets(ext, fn, tying):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32, torch.float64])
+@pytest.mark.parametrize("strided", [False, True])
+def test_decoder_bias_of_any_type_and_stride(ext, dtype, strided):
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model("jumprelu", "none", dev)
+    bias = model.dec_bias.data.to(dtype)
+    if strided:
+        bias = torch.stack([bias, bias + 1], dim=2)[:, :, 0]
+    model.dec_bias.data = bias
+    sf = SparseForward(model, 200)
+    x = torch.randn(3, 200, 64, device=dev).bfloat16()
+    got = sf.reconstruct(x)
+    model.dec_bias.data = torch.zeros_like(bias).contiguous().float()
+    want = sf.reconstruct(x) + (sf.bias_sel.double() @ bias.double()).float()[:, None]
+    assert torch.allclose(got, want, rtol=0, atol=1e-5)  # fp32 sums of a few terms of about one
+    sf.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32, torch.float64])
 def test_thresholds_are_computed_in_32_bits(ext, dtype):
     """``model.bfloat16()`` turns ``log_threshold`` into a 16-bit parameter; the threshold is its exponential in fp32 all the same."""
     from crosslayer_coding_b200.models.sparse_forward import SparseForward
