@@ -1334,8 +1334,9 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
     const int rc = launch_rows_adam_bulk(p, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st);
     if (rc != 0) return rc;
   } else if (a->tying == 2 && a->status != nullptr && a->weights_bf16 && a->L <= 32 && a->ntensors == a->L && a->feat_offset == nullptr &&
-             a->feat_scale == nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16)) {
-    // per-target tied rows without affine terms: the row pipeline too (their entries are gathered by the consumers)
+             a->feat_scale == nullptr && a->d_feat_offset == nullptr && a->d_feat_scale == nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16)) {
+    // per-target tied rows without affine terms and without gradients of such terms (which the row pipeline does not form): the row
+    // pipeline too (their entries are gathered by the consumers)
     const int rc = launch_rows_adam_bulk(p, true, a->h.sr_seed != 0, num_sms, a->status, st, true);
     if (rc != 0) return rc;
   } else if (a->tying == 0) {

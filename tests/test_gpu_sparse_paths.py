@@ -363,3 +363,31 @@ def test_decoder_row_update(ext, L, B, d, tying):
     order = torch.argsort(col.long() * B + tok.long())
     got_l, got_f, got_t = (col[order] // F).long(), (col[order] % F).long(), tok[order].long()
     assert (grad_a.double() - dlda[got_l, got_t, got_f]).abs().max() < 1e-5 * dlda.abs().max()
+
+
+def test_affine_gradients_without_affine_terms(ext):
+    """The gradients of the offsets and scales of per-target tied rows are formed whenever their accumulators are given, also while the
+    terms themselves are left out (offset 0, scale 1)."""
+    dev = _dev()
+    L, B, d, F = 3, 40, 520, 16
+    g = torch.Generator().manual_seed(5)
+    tok, col, val = _entries(g, L, B, F, 200, dev)
+    c = _csr(ext, tok, col, val, B, L * F, F)
+    W = [(torch.randn(F, 1, d, generator=g) / 8).bfloat16().to(dev) for _ in range(L)]
+    M, V = ([torch.zeros(F, 1, d, device=dev) for _ in range(L)] for _ in range(2))
+    gs = torch.randn(L, B, d, generator=g).bfloat16().to(dev)
+    acts = torch.zeros(L, B, F, device=dev, dtype=torch.float64)
+    acts[(col // F).long(), tok.long(), (col % F).long()] = val.double()
+    want_off, want_sc = (torch.zeros(L, F, device=dev, dtype=torch.float64) for _ in range(2))
+    for t in range(L):
+        dots = HYPER[8] * gs[t].double() @ W[t][:, 0].double().t()
+        want_off[t] = ((acts[: t + 1] != 0) * dots).sum((0, 1))
+        want_sc[t] = (acts[: t + 1] * dots).sum((0, 1))
+    d_off, d_sc = torch.zeros(L, F, device=dev), torch.zeros(L, F, device=dev)
+    status = torch.zeros(4, dtype=I32, device=dev)
+    ext.decoder_rows_adam(W, M, V, L, B, d, F, 2, c["feat_off"], c["fcsr_tok"], c["fcsr_val"], gs, torch.zeros(tok.numel(), device=dev), None, None, None, None,
+                          None, HYPER, status, None, None, None, False, d_off, d_sc)
+    assert int(status[0]) == 0
+    # fp32 sums of some ten thousand products: 2^-24 times the square root of their number, on terms of the size of the result
+    assert (d_off.double() - want_off).abs().max() < 1e-5 * want_off.abs().max()
+    assert (d_sc.double() - want_sc).abs().max() < 1e-5 * want_sc.abs().max()
