@@ -529,9 +529,13 @@ __global__ void __launch_bounds__(288, EPT == 4 ? 3 : 2) decoder_rows_adam_bulk_
   const int tid = threadIdx.x;
   const StepScales sc = read_step_ctl(p.ctl);
   if (sc.skip) return;  // the whole grid sees the same flag: a skipped step touches nothing
+  // Features b, b + grid, ... of every tensor.  PT: rows b, b + grid, ... of all tensors taken as one list, so that the rows of a
+  // feature with many entries (one per target, gathered by the consumers) fall to different CTAs: 90 entries in eight of 1128
+  // features, 8 targets, d = 512: 285 us when one CTA had all rows of a feature, 62 us now.
   const int nf = (Fp - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);  // features of this CTA per tensor
   long long n_rows = 0;
   for (int ti = 0; ti < p.ntensors; ++ti) n_rows += 1LL * (nf > 0 ? nf : 0) * p.rows[ti];
+  if (PT) n_rows = (1LL * p.ntensors * Fp - blockIdx.x + gridDim.x - 1) / gridDim.x;
   const int n = int(n_rows);
   const uint32_t w_bytes = uint32_t(d) * sizeof(WT), mv_bytes = uint32_t(d) * sizeof(MT), gs_bytes = uint32_t(d) * 2u;
   const uint32_t off_w = 64, off_m = off_w + w_bytes, off_v = off_m + mv_bytes, off_gs = off_v + mv_bytes;
@@ -548,7 +552,7 @@ __global__ void __launch_bounds__(288, EPT == 4 ? 3 : 2) decoder_rows_adam_bulk_
 
   if (tid == nconsumer) {
     // ------------------------------------------------------------------ producer / store issuer
-    const int n_feat = nf * p.ntensors;
+    const int n_feat = PT ? n : nf * p.ntensors;
     auto col_of = [&](int k) { const int ti = k / nf; return ti * Fp + int(blockIdx.x) + (k - ti * nf) * int(gridDim.x); };
     auto load_offsets = [&](int k, FeatMeta& mt) {
       if (k < n_feat) { const int c = col_of(k); mt.b = __ldg(p.feat_off + c); mt.e = __ldg(p.feat_off + c + 1); }
@@ -567,14 +571,21 @@ __global__ void __launch_bounds__(288, EPT == 4 ? 3 : 2) decoder_rows_adam_bulk_
     const uint64_t pol_stream = l2_policy_evict_first();
     const uint64_t pol_keep = l2_policy_evict_last();
     FeatMeta cur, nxt, nn;
-    load_offsets(0, cur); load_entries(cur);
-    load_offsets(1, nxt);
+    if (PT) {
+      cur.b = cur.e = 0;
+#pragma unroll
+      for (int j = 0; j < kAdamSlots; ++j) { cur.tok[j] = 0; cur.a[j] = 0.f; }
+    } else {
+      load_offsets(0, cur); load_entries(cur);
+      load_offsets(1, nxt);
+    }
     int k = 0, r = 0;             // feature / row whose loads are issued next
     int ti = 0, R = n_feat > 0 ? p.rows[0] : 0;
     int f = int(blockIdx.x);
+    if (PT) { ti = f / Fp; f -= ti * Fp; R = 1; }
     bool fresh = true;            // first row of a feature: start the prefetch of the following ones
     auto issue_loads = [&](int i) {
-      if (fresh) {
+      if (!PT && fresh) {
         load_entries(nxt);        // offsets of k + 1 were requested one feature ago
         load_offsets(k + 2, nn);
         fresh = false;
@@ -597,7 +608,9 @@ __global__ void __launch_bounds__(288, EPT == 4 ? 3 : 2) decoder_rows_adam_bulk_
       for (int j = 0; j < kAdamSlots; ++j)
         if (j < nslot) bulk_load_1d_hint(stage + off_gs + j * gs_bytes, gs_t + 1LL * cur.tok[j] * d, gs_bytes, &sh->full[st], pol_keep);
       // advance to the next row
-      if (++r == R) {
+      if (PT) {
+        for (f += int(gridDim.x); f >= Fp; f -= Fp) ++ti;
+      } else if (++r == R) {
         r = 0; ++k;
         cur = nxt; nxt.b = nn.b; nxt.e = nn.e;
         fresh = true;
@@ -1250,50 +1263,64 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
   if (mb && !weights_bf16) return -1;  // bf16 moments go with bf16 weights
   int nstages = kAdamStages;
   if (!bulk_rows_adam_geometry(p.d, weights_bf16, mb, &ept, &gthreads, &stage_bytes, &smem, &nstages)) return -1;
-  auto launch = [&](auto kern, int which) -> int {
-    static size_t attr_set[14] = {};
-    if (attr_set[which] < smem) {
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
-      attr_set[which] = smem;
-    }
+  auto launch = [&](auto kern) -> int {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
     // resident CTAs per SM from the runtime (shared memory, threads and registers together): a grid beyond them would run a
     // second wave of CTAs over features that were dealt out evenly
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, gthreads + 32, smem) != cudaSuccess || per_sm < 1) return -4;
     int bgrid = num_sms * (per_sm > 6 ? 6 : per_sm);
-    if (bgrid > p.F_pitch) bgrid = p.F_pitch;
-    // CTA b owns the features b, b + grid, ... of every tensor: pick the grid (between half of the resident slots and all
-    // of them) that splits the features most evenly, so that no CTA still streams rows when the others are done.  On a
-    // narrow shard (3072 features, 888 slots) the naive grid leaves CTAs with 3 and with 4 features per tensor.
     int best = bgrid;
-    double best_waste = double((p.F_pitch + bgrid - 1) / bgrid) * bgrid / double(p.F_pitch) - 0.03;  // a few per cent do not pay for fewer CTAs
-    for (int g = bgrid - 1; g >= (3 * bgrid) / 4 && g >= 1; --g) {
-      const int per = (p.F_pitch + g - 1) / g;
-      const double waste = double(per) * g / double(p.F_pitch);
-      if (waste < best_waste - 1e-9) { best_waste = waste; best = g; }
+    if (per_target) {
+      // one list of all rows: any grid splits it evenly.  The rows of a feature are F_pitch apart; take the grid, among a few at the
+      // upper end, that sends the most of them to CTAs of their own
+      const long long rows = 1LL * p.ntensors * p.F_pitch;
+      if (bgrid > rows) bgrid = int(rows);
+      int best_distinct = 0;
+      for (int g = bgrid; g > bgrid - 8 && g >= 1 && best_distinct < p.ntensors; --g) {
+        int distinct = 0;
+        for (int i = 0; i < p.ntensors; ++i) {
+          bool seen = false;
+          for (int j = 0; j < i && !seen; ++j) seen = (1LL * (i - j) * p.F_pitch) % g == 0;
+          distinct += seen ? 0 : 1;
+        }
+        if (distinct > best_distinct) { best_distinct = distinct; best = g; }
+      }
+    } else {
+      if (bgrid > p.F_pitch) bgrid = p.F_pitch;
+      // CTA b owns the features b, b + grid, ... of every tensor: pick the grid (between three quarters of the resident slots and all
+      // of them) that splits the features most evenly, so that no CTA still streams rows when the others are done.  On a
+      // narrow shard (3072 features, 888 slots) the naive grid leaves CTAs with 3 and with 4 features per tensor.
+      best = bgrid;
+      double best_waste = double((p.F_pitch + bgrid - 1) / bgrid) * bgrid / double(p.F_pitch) - 0.03;  // a few per cent do not pay for fewer CTAs
+      for (int g = bgrid - 1; g >= (3 * bgrid) / 4 && g >= 1; --g) {
+        const int per = (p.F_pitch + g - 1) / g;
+        const double waste = double(per) * g / double(p.F_pitch);
+        if (waste < best_waste - 1e-9) { best_waste = waste; best = g; }
+      }
     }
     kern<<<best, gthreads + 32, smem, st>>>(p, gthreads, stage_bytes, nstages, status);
     return 0;
   };
   using bf = t16;
   if (per_target) {
-    if (ept == 4) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, float, true>, 10) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, float, true>, 11);
-    return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, float, true>, 12) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, float, true>, 13);
+    if (ept == 4) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, float, true>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, float, true>);
+    return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, float, true>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, float, true>);
   }
   if (mb) {
 #if CLT_T16_IS_HALF
     return -6;  // bf16 moments go with bf16 weights
 #else
-    if (ept == 4) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, bf>, 6) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, bf>, 7);
-    return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, bf>, 8) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, bf>, 9);
+    if (ept == 4) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, bf>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, bf>);
+    return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, bf>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, bf>);
 #endif
   }
   if (ept == 4) {
-    if (weights_bf16) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, float>, 0) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, float>, 1);
-    return launch(decoder_rows_adam_bulk_kernel<float, false, 4, float>, 2);
+    if (weights_bf16) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, float>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, float>);
+    return launch(decoder_rows_adam_bulk_kernel<float, false, 4, float>);
   }
-  if (weights_bf16) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, float>, 3) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, float>, 4);
-  return launch(decoder_rows_adam_bulk_kernel<float, false, 8, float>, 5);
+  if (weights_bf16) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, float>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, float>);
+  return launch(decoder_rows_adam_bulk_kernel<float, false, 8, float>);
 }
 
 extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sms, cudaStream_t st) {
@@ -1317,6 +1344,8 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   p.norm_sq_out = a->ctl != nullptr ? a->ctl + SC_GRAD_NORM_SQ : nullptr;
   if (a->moments_bf16 && !(a->tying == 0 && a->status != nullptr && a->weights_bf16)) return -6;  // only the bulk pipeline handles bf16 moments
   if (acc == 0) return 0;
+  bool single_rows = true;
+  for (int i = 0; i < a->ntensors; ++i) single_rows = single_rows && a->rows[i] == 1;
   const int grid = num_sms * 8;
   if (a->norm_only) {
     if (a->ctl == nullptr) return -1;
@@ -1333,10 +1362,14 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   if (a->tying == 0 && a->status != nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16) && acc * a->d < (1LL << 62)) {
     const int rc = launch_rows_adam_bulk(p, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st);
     if (rc != 0) return rc;
-  } else if (a->tying == 2 && a->status != nullptr && a->weights_bf16 && a->L <= 32 && a->ntensors == a->L && a->feat_offset == nullptr &&
-             a->feat_scale == nullptr && a->d_feat_offset == nullptr && a->d_feat_scale == nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16)) {
-    // per-target tied rows without affine terms and without gradients of such terms (which the row pipeline does not form): the row
-    // pipeline too (their entries are gathered by the consumers)
+  } else if (a->tying == 2 && a->status != nullptr && a->weights_bf16 && a->L <= 32 && a->ntensors == a->L && single_rows && a->d > 256 &&
+             a->feat_offset == nullptr && a->feat_scale == nullptr && a->d_feat_offset == nullptr && a->d_feat_scale == nullptr &&
+             bulk_rows_adam_fits(a->d, a->weights_bf16)) {
+    // Per-target tied rows without affine terms and without gradients of such terms (which the row pipeline does not form): the row
+    // pipeline too, its consumers gather the entries.  Up to d = 256 a row is one warp of the general sweep, which keeps several dozen
+    // rows per SM in flight against six here and waits for three dependent loads (offsets, token, seed row) in all of them at once: d =
+    // 256, 8 x 10000 rows, one entry in four features 148 us there against 188 here; d = 264, two warps a row there: 262 against 203.
+    // With 90 entries in a few features 94 against 53 us (8 x 1128 rows, d = 256) and 105 against 55 (d = 264).
     const int rc = launch_rows_adam_bulk(p, true, a->h.sr_seed != 0, num_sms, a->status, st, true);
     if (rc != 0) return rc;
   } else if (a->tying == 0) {

@@ -307,29 +307,39 @@ def test_threshold_statistics_of_any_type_and_stride(ext):
 HYPER = [1e-3, 0.9, 0.999, 1e-8, 0.01, 1 - 0.9 ** 3, 1 - 0.999 ** 3, 1.0, 0.5, 0.0, 1.0]
 
 
-# entry counts around the four staged slots, the batches of four and the 32 a warp fetches at once; d with idle lanes, with four
-# and with eight elements per thread
-@pytest.mark.parametrize("tying", [0, 2])
-@pytest.mark.parametrize("L,B,d", [(3, 90, 64), (2, 90, 520), (4, 70, 768), (2, 60, 1536)])
-def test_decoder_row_update(ext, L, B, d, tying):
+def _row_update(ext, L, B, d, tying, counts, rows_of=None, dtype=torch.bfloat16, ctl=False, extra=False, seed=0):
+    """One call of the decoder sweep against 64 bits: moments, weights, norms and dL/da.  ``counts``: entries per feature (the same
+    in every layer); ``rows_of``: target rows per feature of a tensor; ``ctl``: loss scale and clip coefficient; ``extra``: compact
+    extra gradients of every third feature's first row; ``seed``: stochastic rounding of the weights."""
     dev = _dev()
     g = torch.Generator().manual_seed(d + tying)
-    counts = [0, 1, 3, 4, 5, 7, 8, 9, 35, 36, 37, 60, 0, 2]
     F = len(counts)
     ent = [(l * F + f, t) for l in range(L) for f, c in enumerate(counts) for t in torch.randperm(B, generator=g)[:c].tolist()]
     col = torch.tensor([e[0] for e in ent], dtype=I32, device=dev)
     tok = torch.tensor([e[1] for e in ent], dtype=I32, device=dev)
     val = torch.randn(len(ent), generator=g).to(dev)
     c = _csr(ext, tok, col, val, B, L * F, F)
-    rows = [L - s if tying == 0 else 1 for s in range(L)]
-    W = [(torch.randn(F, r, d, generator=g) / 8).bfloat16().to(dev) for r in rows]
+    rows = [(rows_of or (lambda s: L - s if tying == 0 else 1))(s) for s in range(L)]
+    W = [(torch.randn(F, r, d, generator=g) / 8).to(dtype).to(dev) for r in rows]
     M = [(torch.randn(F, r, d, generator=g) * 0.01).to(dev) for r in rows]
     V = [(torch.rand(F, r, d, generator=g) * 1e-3 + 1e-4).to(dev) for r in rows]
-    gs = torch.randn(L, B, d, generator=g).bfloat16().to(dev)
+    gs = torch.randn(L, B, d, generator=g).to(dtype).to(dev)
     pen = (torch.rand(L * F, generator=g) * 0.01).to(dev)
     acts = torch.zeros(L, B, F, device=dev, dtype=torch.float64)
     acts[(col // F).long(), tok.long(), (col % F).long()] = val.double()
-    gsc, (lr, b1, b2, eps, wd, bc1, bc2) = HYPER[8], HYPER[:7]
+    control, inv_scale, clip = None, 1.0, 1.0
+    if ctl:
+        inv_scale, clip = 0.25, 0.625
+        control = torch.zeros(16, device=dev)
+        control[1], control[2], control[6] = inv_scale, 4.0, clip
+    gsc, (lr, b1, b2, eps, wd, bc1, bc2) = HYPER[8] * inv_scale, HYPER[:7]
+    xi = xr = None
+    if extra:
+        n_extra = (L * F + 2) // 3
+        xi = torch.full((L * F,), -1, dtype=I32)
+        xi[::3] = torch.arange(n_extra, dtype=I32)
+        xr = torch.randn(n_extra, d, generator=g).to(dev)
+        xi = xi.to(dev)
     want, norm2 = [], []
     dlda = torch.zeros(L, B, F, device=dev, dtype=torch.float64)
     for i in range(L):
@@ -341,6 +351,10 @@ def test_decoder_row_update(ext, L, B, d, tying):
                 dlda[s] += gsc * gs[t].double() @ W[i][:, r].double().t()
         pc = pen.view(L, F).double()
         grad += (pc[i] if tying == 0 else pc[: i + 1].sum(0))[:, None, None] * W[i].double()
+        if extra:
+            has = xi[i * F: (i + 1) * F] >= 0
+            grad[has, 0] += xr[xi[i * F: (i + 1) * F][has].long()].double()
+        grad *= clip
         m = b1 * M[i].double() + (1 - b1) * grad
         v = b2 * V[i].double() + (1 - b2) * grad.square()
         w = W[i].double() * (1 - lr * wd) - lr / bc1 * m / ((v / bc2).sqrt() + eps)
@@ -348,21 +362,53 @@ def test_decoder_row_update(ext, L, B, d, tying):
     grad_a = torch.zeros(len(ent), device=dev)
     n2 = torch.zeros(L * F, device=dev)
     status = torch.zeros(4, dtype=I32, device=dev)
-    ext.decoder_rows_adam(W, M, V, L, B, d, F, tying, c["feat_off"], c["fcsr_tok"], c["fcsr_val"], gs, grad_a, pen, n2, None, None, None, HYPER, status, None,
-                          None, None, False, None, None)
+    hyper = HYPER[:9] + [float(seed)] + HYPER[10:]
+    ext.decoder_rows_adam(W, M, V, L, B, d, F, tying, c["feat_off"], c["fcsr_tok"], c["fcsr_val"], gs, grad_a, pen, n2, None, None, None, hyper, status, xi,
+                          xr, control, False, None, None)
     torch.cuda.synchronize()
     assert int(status[0]) == 0
+    ulp = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -11  # half a unit in the last place; all of it when rounded stochastically
     for i in range(L):
         w, m, v = want[i]
-        # m, v: fp32 sums of up to 60 * L products of unit size, 2^-24 each (1 - beta is itself rounded to 2^-24 of one, a relative
-        # 6e-5 of 0.001); w: one bf16 rounding
+        # m, v: fp32 sums of up to 90 * L products of unit size, 2^-24 each (1 - beta is itself rounded to 2^-24 of one, a relative
+        # 6e-5 of 0.001); w: one rounding to 16 bits (below 2^-14 fp16 has a fixed spacing of 2^-24)
         assert (M[i].double() - m).abs().max() < 4e-6 * m.abs().max() and (V[i].double() - v).abs().max() < 1e-4 * v.abs().max()
-        assert ((W[i].double() - w).abs() <= 2 ** -8 * w.abs() + 1e-7).all()
+        assert ((W[i].double() - w).abs() <= (2 if seed else 1) * ulp * w.abs() + 1e-7).all()
         # norms of the updated rows: 2^-9 relative rounding per weight, averaged over the row
         assert torch.allclose(n2.view(L, F)[i].double(), W[i].double().square().sum((1, 2)), rtol=2e-3)
     order = torch.argsort(col.long() * B + tok.long())
     got_l, got_f, got_t = (col[order] // F).long(), (col[order] % F).long(), tok[order].long()
     assert (grad_a.double() - dlda[got_l, got_t, got_f]).abs().max() < 1e-5 * dlda.abs().max()
+
+
+COUNTS = [0, 1, 3, 4, 5, 7, 8, 9, 35, 36, 37, 60, 0, 2]
+
+
+# entry counts around the four staged slots, the batches of four and the 32 a warp fetches at once; d with idle lanes, with four
+# and with eight elements per thread
+@pytest.mark.parametrize("tying", [0, 2])
+@pytest.mark.parametrize("L,B,d", [(3, 90, 64), (2, 90, 520), (4, 70, 768), (2, 60, 1536)])
+def test_decoder_row_update(ext, L, B, d, tying):
+    _row_update(ext, L, B, d, tying, COUNTS)
+
+
+# per-target tied rows on both sides of the width at which they change to the row pipeline; more rows than resident CTAs, so that
+# every CTA has several, of several tensors (600 and 148 features per tensor: a grid that divides the number of features), features
+# with many entries among them
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,d,F", [(3, 256, 600), (5, 264, 600), (12, 512, 148), (2, 1032, 800)])
+def test_per_target_rows_dealt_over_the_grid(ext, L, d, F, dtype):
+    counts = [0] * F
+    for i, n in enumerate([90, 1, 0, 33, 4] * 4):
+        counts[(i * 37) % F] = n
+    _row_update(ext, L, 90, d, 2, counts, dtype=dtype)
+
+
+# what the engine adds to the sweep: loss scale and clip coefficient from the control block, compact extra rows, stochastic rounding
+@pytest.mark.parametrize("tying,d", [(0, 264), (2, 200), (2, 264), (2, 1032)])
+@pytest.mark.parametrize("opts", [dict(ctl=True), dict(extra=True), dict(seed=1234), dict(ctl=True, extra=True, dtype=torch.float16)])
+def test_decoder_row_update_options(ext, tying, d, opts):
+    _row_update(ext, 3, 90, d, tying, COUNTS, **opts)
 
 
 def test_affine_gradients_without_affine_terms(ext):
