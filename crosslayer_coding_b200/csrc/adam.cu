@@ -13,6 +13,8 @@
 // fp32 moments (or fp32 weights).  d must be a multiple of 8.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace clt {
 
 constexpr int kMaxLayersA = 32;
@@ -477,10 +479,9 @@ __device__ __forceinline__ int warp_sum_slot(int lane) { return lane / (32 / N);
 // activation), cnt of them.  The seed rows come kBatch at a time, so a feature with many entries waits for L2 once per
 // kBatch of them and not twice per entry (eight entries per feature on average, tied Pythia-70m shape: both sweeps of a step
 // 1.81 -> 1.60 ms).  It takes 72 registers; a cap of 64 spills and cost 0.4 ms at the GPT-2 shape.
-template <int EPT>
+template <int EPT, int kBatch>
 __device__ __forceinline__ void add_entries(int cnt, int my_x, int my_tok, float my_a, const t16* gs_t, int d, bool act, int lane, const float (&w)[EPT],
                                             float (&g)[EPT], float* grad_a, float gsc) {
-  constexpr int kBatch = 4;
   for (int j0 = 0; j0 < cnt; j0 += kBatch) {
     uint2 q2[kBatch][EPT / 4];
     float dot[kBatch];
@@ -519,8 +520,9 @@ __device__ __forceinline__ void add_entries(int cnt, int my_x, int my_tok, float
 
 // PT: per-target tied decoders (one row per feature and target layer, shared by the source layers below): the entries of a row
 // come from several CSR segments, so none are staged in slots.
-template <typename WT, bool SR, int EPT, typename MT, bool PT = false>
-__global__ void __launch_bounds__(288, EPT == 4 ? 3 : 2) decoder_rows_adam_bulk_kernel(const DecAdamParams p, int gthreads, int stage_bytes, int ns, int* status) {
+// NB: entries beyond the staged ones that are loaded together.  NARROW: 64 registers instead of 72 (d <= 640).
+template <typename WT, bool SR, int EPT, typename MT, bool PT = false, int NB = 4, bool NARROW = false>
+__global__ void __launch_bounds__(NARROW ? 192 : 288, NARROW ? 5 : (EPT == 4 ? 3 : 2)) decoder_rows_adam_bulk_kernel(const DecAdamParams p, int gthreads, int stage_bytes, int ns, int* status) {
   extern __shared__ __align__(128) uint8_t smem_raw_adam[];  // bulk copies need 16-byte alignment only
   uint8_t* ring = smem_raw_adam;
   AdamBulkShared* sh = reinterpret_cast<AdamBulkShared*>(ring + size_t(ns) * stage_bytes);
@@ -726,14 +728,14 @@ __global__ void __launch_bounds__(288, EPT == 4 ? 3 : 2) decoder_rows_adam_bulk_
           const int x = __shfl_sync(0xFFFFFFFFu, seg_b, seg) + j - (__shfl_sync(0xFFFFFFFFu, incl, seg) - __shfl_sync(0xFFFFFFFFu, seg_n, seg));
           const int my_tok = j < total ? __ldg(p.fcsr_tok + x) : 0;
           const float my_a = j < total ? __ldg(p.fcsr_val + x) : 0.f;
-          add_entries<EPT>(min(32, total - j0), x, my_tok, my_a, p.gs + 1LL * ti * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
+          add_entries<EPT, NB>(min(32, total - j0), x, my_tok, my_a, p.gs + 1LL * ti * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
         }
       } else {
         for (int x0 = b + kAdamSlots; x0 < b + ne; x0 += 32) {  // entries beyond the slots
           const int cnt = min(32, b + ne - x0);
           const int my_tok = lane < cnt ? __ldg(p.fcsr_tok + x0 + lane) : 0;
           const float my_a = lane < cnt ? __ldg(p.fcsr_val + x0 + lane) : 0.f;
-          add_entries<EPT>(cnt, x0 + lane, my_tok, my_a, p.gs + 1LL * (ti + r) * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
+          add_entries<EPT, NB>(cnt, x0 + lane, my_tok, my_a, p.gs + 1LL * (ti + r) * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
         }
       }
       if (act) {
@@ -1235,6 +1237,7 @@ struct CltDecAdamArgs {
   float* ctl;        // step control block (skip flag, 1 / loss scale, clip coefficient); may be null
   int norm_only;     // 1: gradient-norm pre-pass (adds to ctl[SC_GRAD_NORM_SQ], writes grad_a, updates nothing)
   float* d_feat_offset; float* d_feat_scale;  // tied decoders: gradient accumulators of the affine terms, see DecAdamParams
+  long long n_entries;  // length of fcsr_tok / fcsr_val
 };
 
 // Launch geometry of the bulk-copy row pipeline (shared by the decoder and the encoder update).
@@ -1256,7 +1259,9 @@ static bool bulk_rows_adam_fits(int d, int weights_bf16) {
   size_t smem;
   return bulk_rows_adam_geometry(d, weights_bf16 != 0, false, &ept, &gthreads, &stage_bytes, &smem) != 0;
 }
-static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool sr, int num_sms, int* status, cudaStream_t st, bool per_target = false) {
+// n_entries: length of the entry list (an upper bound where the number of active entries is not known to the host).
+static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool sr, int num_sms, int* status, cudaStream_t st, long long n_entries,
+                                 bool per_target = false) {
   int ept, gthreads, stage_bytes;
   size_t smem;
   const bool mb = p.moments_bf16 != 0;
@@ -1302,6 +1307,36 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
     kern<<<best, gthreads + 32, smem, st>>>(p, gthreads, stage_bytes, nstages, status);
     return 0;
   };
+  // Registers against batches.  Four entries per batch take 72 registers, which costs rows of 392 to 608 elements a resident CTA per SM
+  // (five for six up to 512, four for five above), and a list of a few entries beyond the staged ones fills no batch.  So the 64-register
+  // form with batches of two runs where it has more resident CTAs and the lists are short or wait little:
+  //  * one row per feature (encoder) up to 512 wide: 6 x 10520 rows of 440, one entry in four features 123 -> 119 us (152 with 72
+  //    registers), eight per feature 246 -> 233 (274); from 520 on the 72-register form is the better one (576 wide, eight per feature
+  //    310 -> 258 us against 304);
+  //  * several rows per feature (untied decoders) with at most three entries per feature on average: 6 x 2864 features 576 wide, one
+  //    entry in four 126 -> 126 us (129 with 72 registers), 2.7 per feature 162 -> 154 (162).
+  // Above 1024 (eight elements per thread) one row per feature takes its entries one by one: 6 x 10520 rows of 1432, five per feature
+  // 478 -> 469 us (488 with batches of four).  The first figure of a pair is the sweep that waited twice per entry.
+  auto per_sm_of = [&](auto kern) -> int {
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, gthreads + 32, smem) != cudaSuccess) return -1;
+    return n > 6 ? 6 : n;
+  };
+  bool single_rows = true;
+  for (int i = 0; i < p.ntensors; ++i) single_rows = single_rows && p.rows[i] == 1;
+  const bool short_lists = single_rows ? gthreads <= 128 : gthreads <= 160 && n_entries <= 3LL * p.F_pitch * p.L;
+  auto pick = [&](auto srv, auto wt, auto mt) -> int {
+    constexpr bool S = decltype(srv)::value;
+    using W = decltype(wt);
+    using M = decltype(mt);
+    if (ept == 8) return single_rows ? launch(decoder_rows_adam_bulk_kernel<W, S, 8, M, false, 1>) : launch(decoder_rows_adam_bulk_kernel<W, S, 8, M>);
+    if (short_lists && per_sm_of(decoder_rows_adam_bulk_kernel<W, S, 4, M, false, 2, true>) > per_sm_of(decoder_rows_adam_bulk_kernel<W, S, 4, M>))
+      return launch(decoder_rows_adam_bulk_kernel<W, S, 4, M, false, 2, true>);
+    return launch(decoder_rows_adam_bulk_kernel<W, S, 4, M>);
+  };
+  using yes = std::true_type;
+  using no = std::false_type;
   using bf = t16;
   if (per_target) {
     if (ept == 4) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, float, true>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, float, true>);
@@ -1311,16 +1346,11 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
 #if CLT_T16_IS_HALF
     return -6;  // bf16 moments go with bf16 weights
 #else
-    if (ept == 4) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, bf>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, bf>);
-    return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, bf>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, bf>);
+    return sr ? pick(yes{}, bf{}, bf{}) : pick(no{}, bf{}, bf{});
 #endif
   }
-  if (ept == 4) {
-    if (weights_bf16) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 4, float>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 4, float>);
-    return launch(decoder_rows_adam_bulk_kernel<float, false, 4, float>);
-  }
-  if (weights_bf16) return sr ? launch(decoder_rows_adam_bulk_kernel<bf, true, 8, float>) : launch(decoder_rows_adam_bulk_kernel<bf, false, 8, float>);
-  return launch(decoder_rows_adam_bulk_kernel<float, false, 8, float>);
+  if (!weights_bf16) return pick(no{}, float{}, float{});
+  return sr ? pick(yes{}, bf{}, float{}) : pick(no{}, bf{}, float{});
 }
 
 extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sms, cudaStream_t st) {
@@ -1360,7 +1390,7 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
   if (a->tying == 0 && a->status != nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16) && acc * a->d < (1LL << 62)) {
-    const int rc = launch_rows_adam_bulk(p, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st);
+    const int rc = launch_rows_adam_bulk(p, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st, a->n_entries);
     if (rc != 0) return rc;
   } else if (a->tying == 2 && a->status != nullptr && a->weights_bf16 && a->L <= 32 && a->ntensors == a->L && single_rows && a->d > 256 &&
              a->feat_offset == nullptr && a->feat_scale == nullptr && a->d_feat_offset == nullptr && a->d_feat_scale == nullptr &&
@@ -1370,7 +1400,7 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
     // rows per SM in flight against six here and waits for three dependent loads (offsets, token, seed row) in all of them at once: d =
     // 256, 8 x 10000 rows, one entry in four features 148 us there against 188 here; d = 264, two warps a row there: 262 against 203.
     // With 90 entries in a few features 94 against 53 us (8 x 1128 rows, d = 256) and 105 against 55 (d = 264).
-    const int rc = launch_rows_adam_bulk(p, true, a->h.sr_seed != 0, num_sms, a->status, st, true);
+    const int rc = launch_rows_adam_bulk(p, true, a->h.sr_seed != 0, num_sms, a->status, st, a->n_entries, true);
     if (rc != 0) return rc;
   } else if (a->tying == 0) {
     const bool sr = a->h.sr_seed != 0;
@@ -1399,6 +1429,7 @@ struct CltEncAdamArgs {
   const int* extra_idx; const float* extra_rows; const float* extra_bias;  // compact extras, see EncAdamParams
   float* ctl;
   int norm_only;
+  long long n_entries;  // length of fcsr_tok / delta
 };
 
 extern "C" int CLT_FN(clt_encoder_rows_adam)(const CltEncAdamArgs* a, int num_sms, cudaStream_t st) {
@@ -1442,7 +1473,7 @@ extern "C" int CLT_FN(clt_encoder_rows_adam)(const CltEncAdamArgs* a, int num_sm
     q.extra_idx = a->dense_grad == nullptr ? a->extra_idx : nullptr; q.extra_rows = a->extra_rows;
     q.ctl = a->ctl; q.use_inv_scale = 0; q.norm_sq_out = nullptr;
     if (a->dense_grad != nullptr && a->extra_idx != nullptr) return -7;  // the row pipeline takes one kind of extra rows
-    const int rc = launch_rows_adam_bulk(q, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st);
+    const int rc = launch_rows_adam_bulk(q, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st, a->n_entries);
     if (rc != 0) return rc;
     if (p.bias != nullptr) {
       const int bgrid = int((1LL * a->L * a->F_pitch + 255) / 256);

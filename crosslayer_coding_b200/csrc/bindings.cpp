@@ -104,6 +104,7 @@ struct CltDecAdamArgs {
   float* ctl;
   int norm_only;
   float* d_feat_offset; float* d_feat_scale;
+  long long n_entries;
 };
 struct CltEncAdamArgs {
   void* w; float* m; float* v; void* bias; float* bias_m; float* bias_v;
@@ -116,6 +117,7 @@ struct CltEncAdamArgs {
   const int* extra_idx; const float* extra_rows; const float* extra_bias;
   float* ctl;
   int norm_only;
+  long long n_entries;
 };
 struct CltStepControlArgs {
   float* ctl; const int* status; double* sq_err; int L; double* scalars; int n_scalars; float* losses; double inv_bd;
@@ -603,6 +605,7 @@ void decoder_rows_adam(std::vector<Tensor>& w, std::vector<Tensor>& m, std::vect
   a.moments_bf16 = m[0].scalar_type() == at::kBFloat16 ? 1 : 0;
   a.ctl = ctl_ptr(ctl);
   a.norm_only = norm_only ? 1 : 0;
+  a.n_entries = fcsr_tok.numel();
   a.d_feat_offset = opt_ptr<float>(d_feat_offset); a.d_feat_scale = opt_ptr<float>(d_feat_scale);
   for (const OptTensor* t : {&d_feat_offset, &d_feat_scale})
     if (t->has_value() && (*t)->defined())
@@ -634,6 +637,7 @@ void encoder_rows_adam(Tensor& w, Tensor& m, Tensor& v, Tensor& bias, Tensor& bi
   a.status = opt_ptr<int>(status);
   a.ctl = ctl_ptr(ctl);
   a.norm_only = norm_only ? 1 : 0;
+  a.n_entries = fcsr_tok.numel();
   c10::cuda::CUDAGuard guard(w.device());
   check(CLT_PICK(half, clt_encoder_rows_adam)(&a, num_sms(), cur_stream()), "encoder_rows_adam");
 }
