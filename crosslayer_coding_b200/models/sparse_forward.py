@@ -137,8 +137,9 @@ class SparseForward:
         return self.theta
 
     @torch.no_grad()
-    def encode(self, X: torch.Tensor, clear_loss: bool = False) -> None:
-        """Pre-activations, selection and the token-major / feature-major CSR views of the active entries."""
+    def encode(self, X: torch.Tensor, clear_loss: bool = False, sort_tokens: bool = True) -> None:
+        """Pre-activations, selection and the token-major / feature-major CSR views of the active entries.  ``sort_tokens``: a token's
+        entries ordered by (layer, feature), which the decode wants; whoever reads the feature-major view alone can do without."""
         e, m = self.ext, self.model
         assert X.dtype == torch.bfloat16 and X.shape == (self.L, self.B, self.d), (X.dtype, tuple(X.shape))
         e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, None)
@@ -157,7 +158,7 @@ class SparseForward:
         (self._zeroed if clear_loss else self._zeroed_encode).zero_()
         e.build_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.feat_cnt, self.tok_off,
                     self.feat_off, self.tok_cursor, self.feat_cursor, self.tcsr_col, self.tcsr_val, self.fcsr_tok, self.fcsr_val,
-                    None, 3, self.Fl)
+                    None, 3 if sort_tokens else 2, self.Fl)
 
     # ------------------------------------------------------------------ decode
     @torch.no_grad()

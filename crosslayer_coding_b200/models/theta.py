@@ -83,7 +83,7 @@ def accumulate_theta_batch_sparse(sf, X: torch.Tensor, stats: Dict[str, torch.Te
     """The same statistic from the sparse forward (``models.sparse_forward.SparseForward``): the batch mean / std of
     every feature come from the selection's column statistics, the per-feature minimum of the selected z-scores from the
     feature-major entry list, one kernel - no dense ``[B, L*F]`` selection, which is what the dense path spends its time on."""
-    sf.encode(X)
+    sf.encode(X, sort_tokens=False)
     names = ("sum_min", "cnt_min", "mean", "std")
 
     def accumulate(into: Dict[str, torch.Tensor]) -> None:
