@@ -39,54 +39,96 @@ def _entries(g, L, B, F, n, dev):
     return (flat // (L * F)).to(I32).to(dev), (flat % (L * F)).to(I32).to(dev), val.to(dev)
 
 
-# d: one, two, three and four 16-byte vectors per lane, partly filled ones, two column chunks; B: the split walk (few
-# (token, target) warps), the walk and (per source) the running sum, each with a last CTA that is not full
-@pytest.mark.parametrize("tying,affine", [(0, False), (1, False), (1, True), (2, False), (2, True)])
-@pytest.mark.parametrize("L,B,d", [(2, 3, 8), (3, 5, 264), (12, 2, 768), (4, 1030, 256), (5, 1027, 520), (2, 2055, 768), (3, 1500, 1024), (2, 2051, 1032), (3, 700, 2048)])
-def test_gather_decode_matches_dense(ext, L, B, d, tying, affine):
+def _dense_decode(L, B, d, F, tying, tok, col, val, W, off, sc, rows_limit=0):
+    """``[L, B, d]`` in 64 bits: the sums over the entries, without biases."""
+    acts = torch.zeros(L, B, F, device=tok.device, dtype=torch.float64)
+    acts[(col // F).long(), tok.long(), (col % F).long()] = val.double()
+    want = torch.zeros(L, B, d, device=tok.device, dtype=torch.float64)
+    for t in range(L):
+        for s in range(t + 1):
+            if rows_limit and t - s >= rows_limit:
+                continue
+            a = acts[s]
+            if off is not None:
+                a = torch.where(a != 0, (a + off[t].double()) * sc[t].double(), a)
+            w = W[s][:, t - s] if tying == 0 else W[s if tying == 1 else t][:, 0]
+            want[t] += a @ w.double()
+    return want
+
+
+def _check_decode(ext, L, B, d, tying, affine, dtype=torch.bfloat16, addend=False, rows_limit=0):
     dev = _dev()
     g = torch.Generator().manual_seed(L * 1000 + B + d)
     F = 24
     tok, col, val = _entries(g, L, B, F, min(B * L * F, 7 * B), dev)
     rows = [L - s if tying == 0 else 1 for s in range(L)]
-    W = [(torch.randn(F, r, d, generator=g) / 4).bfloat16().to(dev) for r in rows]
+    W = [(torch.randn(F, r, d, generator=g) / 4).to(dtype).to(dev) for r in rows]
     off = torch.randn(L, F, generator=g).to(dev) if affine else None
     sc = torch.randn(L, F, generator=g).to(dev) if affine else None
     bias = torch.randn(L, d, generator=g).to(dev)
-    y = torch.randn(L, B, d, generator=g).bfloat16().to(dev)
+    add = torch.randn(L, B, d, generator=g).to(dev) if addend else None
+    y = torch.randn(L, B, d, generator=g).to(dtype).to(dev)
     sigma = (0.5 + torch.rand(L, d, generator=g)).to(dev)
-    acts = torch.zeros(L, B, F, device=dev, dtype=torch.float64)
-    acts[(col // F).long(), tok.long(), (col % F).long()] = val.double()
-    want = torch.zeros(L, B, d, device=dev, dtype=torch.float64)
-    for t in range(L):
-        for s in range(t + 1):
-            a = acts[s]
-            if affine:
-                a = torch.where(a != 0, (a + off[t].double()) * sc[t].double(), a)
-            w = W[s][:, t - s] if tying == 0 else W[s if tying == 1 else t][:, 0]
-            want[t] += a @ w.double()
-    want += bias.double()[:, None, :]
+    want = _dense_decode(L, B, d, F, tying, tok, col, val, W, off, sc, rows_limit) + bias.double()[:, None, :]
+    if addend:
+        want += add.double()
     status = torch.zeros(4, dtype=I32, device=dev)
     for sort in (3, 0):  # the order of a token's entries changes only the order of the sums
         c = _csr(ext, tok, col, val, B, L * F, F, sort)
+
+        def decode(mode, partial=None, bias=None, addend=None, target=None, sigma=None, gs=None, yhat=None, sq=None, peers=(), rows_per_rank=0, rank=0):
+            ext.sparse_decode(W, L, B, d, F, tying, c["tok_off"], c["tcsr_col"], c["tcsr_val"], off, sc, partial, bias, addend, target, sigma, gs, yhat, sq, mode,
+                              list(peers), rows_per_rank, rank, status, None, rows_limit)
+
         yhat = torch.full((L, B, d), float("nan"), device=dev)
-        gs = torch.empty(L, B, d, device=dev, dtype=torch.bfloat16)
+        gs = torch.empty(L, B, d, device=dev, dtype=dtype)
         sq = torch.zeros(L, device=dev, dtype=torch.float64)
-        ext.sparse_decode(W, L, B, d, F, tying, c["tok_off"], c["tcsr_col"], c["tcsr_val"], off, sc, None, bias, None, y, sigma, gs, yhat, sq, 1, [], 0, 0,
-                          status)
+        decode(1, bias=bias, addend=add, target=y, sigma=sigma, gs=gs, yhat=yhat, sq=sq)
         # fp32 sums of at most a few dozen products: 2^-24 each on terms of the size of the result
         scale = want.abs().max()
         assert (yhat.double() - want).abs().max() < 1e-5 * scale
         r = (want - y.double()) * sigma.double()[:, None]
         assert torch.allclose(sq, r.square().sum((1, 2)), rtol=1e-5)
-        # bf16 keeps 8 bits: half a unit in the last place of the value, plus the fp32 error of the sum
+        # bf16 keeps 8 bits (fp16 has 11): half a unit in the last place of the value, plus the fp32 error of the sum
         assert ((gs.double() - r * sigma.double()[:, None]).abs() <= 2 ** -8 * (r * sigma.double()[:, None]).abs() + 1e-4).all()
+        # the reconstruction alone
+        plain = torch.full((L, B, d), float("nan"), device=dev)
+        decode(1, bias=bias, addend=add, yhat=plain)
+        assert torch.equal(plain, yhat) if sort == 3 else (plain.double() - want).abs().max() < 1e-5 * scale
         # partial sums only (the tensor-parallel form before the exchange)
+        sums = want - bias.double()[:, None] - (add.double() if addend else 0)
         part = torch.full((L, B, d), float("nan"), device=dev)
-        ext.sparse_decode(W, L, B, d, F, tying, c["tok_off"], c["tcsr_col"], c["tcsr_val"], off, sc, part, None, None, None, None, None, None, None, 0, [], 0,
-                          0, status)
-        assert (part.double() + bias.double()[:, None] - want).abs().max() < 1e-5 * scale
+        decode(0, partial=part)
+        assert (part.double() - sums).abs().max() < 1e-5 * scale
+        # the same sums pushed to the owners of the tokens, three of them with the last block not full: each holds an area [ranks, L,
+        # rows, d] per sending rank; here all areas lie in this GPU's memory (the kernel only stores, no rank waits for another)
+        world, rank = 3, 1
+        rows_per_rank = (B + world - 1) // world
+        areas = torch.full((world, world, L, rows_per_rank, d), float("nan"), device=dev)
+        decode(2, peers=[areas[o].data_ptr() for o in range(world)], rows_per_rank=rows_per_rank, rank=rank)
+        pushed = torch.cat([areas[o, rank] for o in range(world)], dim=1)
+        assert torch.equal(pushed[:, :B], part) if sort == 3 else (pushed[:, :B].double() - sums).abs().max() < 1e-5 * scale
+        assert bool(pushed[:, B:].isnan().all()) and bool(areas[:, [0, 2]].isnan().all())
     assert int(status[0]) == 0
+
+
+# d: one to four 16-byte vectors per lane, partly filled ones, two column chunks; B: the split walk (few (token, target) warps), the
+# walk, the walk of two rows per step (2048 tokens and three or four vectors) and (per source) the running sum, each with a last
+# CTA that is not full
+@pytest.mark.parametrize("tying,affine", [(0, False), (1, False), (1, True), (2, False), (2, True)])
+@pytest.mark.parametrize("L,B,d", [(2, 3, 8), (3, 5, 264), (12, 2, 768), (2, 3, 1024), (3, 4, 2048), (4, 1030, 256), (4, 1030, 512), (5, 1027, 520), (2, 2055, 768),
+                                   (2, 2051, 1024), (3, 1500, 1024), (2, 2051, 1032), (3, 700, 2048), (2, 2050, 2048)])
+def test_gather_decode_matches_dense(ext, L, B, d, tying, affine):
+    _check_decode(ext, L, B, d, tying, affine)
+
+
+# the half-precision build, the skip connection's addend, a limit on the target rows (which keeps per-source decoders off the
+# running sum), more layers than any other test has
+@pytest.mark.parametrize("tying", [0, 1, 2])
+@pytest.mark.parametrize("L,B,d", [(3, 5, 264), (4, 1100, 512), (2, 2055, 768), (20, 70, 264), (32, 1030, 64)])
+@pytest.mark.parametrize("opts", [dict(dtype=torch.float16), dict(addend=True), dict(rows_limit=1), dict(rows_limit=2, dtype=torch.float16, addend=True)])
+def test_gather_decode_options(ext, L, B, d, tying, opts):
+    _check_decode(ext, L, B, d, tying, False, **opts)
 
 
 def test_decode_refuses_loss_outputs_without_a_target(ext):
@@ -138,6 +180,23 @@ def test_equal_keys_in_a_token_segment_are_all_kept(ext):
     assert torch.equal(torch.sort(c["tcsr_val"]).values, val)
 
 
+def _check_token_topk(ext, x, mean, rstd, k, F, dev):
+    L, B, Fl = x.shape
+    status = torch.zeros(4, dtype=I32, device=dev)
+    ctl = torch.zeros(16, dtype=torch.int64, device=dev)
+    tok, col = torch.zeros(B * k, dtype=I32, device=dev), torch.zeros(B * k, dtype=I32, device=dev)
+    val = torch.zeros(B * k, device=dev)
+    ext.token_topk_select(x, mean, rstd, Fl, k, ctl, tok, col, val, status, F)
+    torch.cuda.synchronize(dev)
+    assert int(status[0]) == 0 and int(ctl[3]) == B * k
+    assert torch.equal(tok.view(B, k), torch.arange(B, device=dev, dtype=I32)[:, None].expand(B, k))
+    assert torch.equal(x.float()[(col // Fl).long(), tok.long(), (col % Fl).long()], val)
+    z = ((x.float() - mean[:, None]) * rstd[:, None])[:, :, :F].permute(1, 0, 2).reshape(B, L * F)
+    order = torch.sort(z, dim=1, descending=True, stable=True).indices[:, :k]
+    want = torch.sort((order // F) * Fl + order % F, dim=1).values.to(I32)
+    assert torch.equal(torch.sort(col.view(B, k), dim=1).values, want)
+
+
 # one, two and four tokens per CTA with a last CTA that is not full; k up to the radix rounds; padding columns
 @pytest.mark.parametrize("L,B,Fl,F,k", [(3, 5, 4096, 4096, 64), (2, 601, 2056, 2050, 24), (4, 1779, 520, 520, 7), (2, 33, 1032, 1030, 513), (1, 9, 64, 64, 64),
                                         (2, 40, 16384, 16384, 300)])
@@ -146,25 +205,47 @@ def test_token_topk(ext, L, B, Fl, F, k):
     torch.manual_seed(k)
     x = torch.randn(L, B, Fl, device=dev).bfloat16()
     if B == 33:
-        x[0, :, 100:400] = 1.5  # equal columns after standardisation: ties at and around the cut
+        x[0, :, 100:400] = 1.5  # equal columns after standardisation: ties at and around the cut of the radix rounds
     mean, rstd = torch.empty(L, Fl, device=dev), torch.empty(L, Fl, device=dev)
     ext.colstats(x, mean, rstd)
     if B == 40:
-        x[1, 3] = 30.0  # a token whose list overflows: half of its keys are far above the bound of the other half
+        x[1, 3] = 30.0  # a token with half of its keys far above the other half: the bound from the sample rises with them
         ext.colstats(x, mean, rstd)
-    status = torch.zeros(4, dtype=I32, device=dev)
-    ctl = torch.zeros(16, dtype=torch.int64, device=dev)
-    tok, col = torch.zeros(B * k, dtype=I32, device=dev), torch.zeros(B * k, dtype=I32, device=dev)
-    val = torch.zeros(B * k, device=dev)
-    ext.token_topk_select(x, mean, rstd, Fl, k, ctl, tok, col, val, status, F)
-    torch.cuda.synchronize()
-    assert int(status[0]) == 0 and int(ctl[3]) == B * k
-    assert torch.equal(tok.view(B, k), torch.arange(B, device=dev, dtype=I32)[:, None].expand(B, k))
-    assert torch.equal(x.float()[(col // Fl).long(), tok.long(), (col % Fl).long()], val)
-    z = ((x.float() - mean[:, None]) * rstd[:, None])[:, :, :F].permute(1, 0, 2).reshape(B, L * F)
-    order = torch.sort(z, dim=1, descending=True, stable=True).indices[:, :k]
-    want = torch.sort((order // F) * Fl + order % F, dim=1).values.to(I32)
-    assert torch.equal(torch.sort(col.view(B, k), dim=1).values, want)
+    _check_token_topk(ext, x, mean, rstd, k, F, dev)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B", [6, 602, 1781])
+def test_token_topk_hands_overflowing_lists_to_the_radix_rounds(ext, B, dtype):
+    """The bound on a token's k-th key comes from every eighth block of 2048 columns here.  Large values in the blocks between stay
+    above it, more of them than the list holds: those tokens are marked for the radix kernel, which takes them and their
+    neighbours in a group of four."""
+    dev = _dev()
+    L, F, k = 2, 65536 if B == 6 else 16384, 16
+    g = torch.Generator().manual_seed(B)
+    x = torch.randn(L, B, F, generator=g).to(dtype).to(dev)
+    step = min(8, L * F // 8 // 2048)  # as the launcher picks it for k = 16: list of 2048, 1024 maxima
+    assert step > 1
+    block = torch.arange(L * F, device=dev).view(L, F) // 2048
+    unsampled = (block % step != 0) & (block < 4)
+    assert int(unsampled.sum()) > 2048
+    for t in {1, B // 2 + 1, B - 1}:
+        x[:, t][unsampled] = (10 + 2 * torch.rand(int(unsampled.sum()), generator=g)).to(dtype).to(dev)  # with ties: 16-bit values
+        assert float(x[:, t][~unsampled].max()) < 10
+    _check_token_topk(ext, x, torch.zeros(L, F, device=dev), torch.ones(L, F, device=dev), k, F, dev)
+
+
+@pytest.mark.parametrize("B,k", [(5, 64), (700, 24), (1800, 7)])
+def test_token_topk_list_takes_ties_by_the_lowest_index(ext, B, k):
+    """Keys with a spacing of a half: dozens of columns share the key at the cut, and the list kernel keeps the first of them."""
+    dev = _dev()
+    L, F = 2, 16384
+    g = torch.Generator().manual_seed(k)
+    x = ((2 * torch.randn(L, B, F, generator=g)).round() / 2).bfloat16().to(dev)
+    z = x.float().permute(1, 0, 2).reshape(B, L * F)
+    cut = torch.topk(z, k, dim=1).values[:, -1:]
+    assert bool(((z >= cut).sum(1) > k).any()) and int((z >= cut - 0.5).sum(1).max()) < 2048  # ties, and a list that holds them
+    _check_token_topk(ext, x, torch.zeros(L, F, device=dev), torch.ones(L, F, device=dev), k, F, dev)
 
 
 def _serving_model(fn, tying, dev, L=3, d=64, F=512):
