@@ -1723,11 +1723,8 @@ extern "C" int CLT_FN(clt_threshold_select)(const CltSelectArgs* a, cudaStream_t
 
 template <int TPC>
 static int launch_token_list(const CltSelectArgs* a, const ScanGeom& g, int f_valid, int k, cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(token_topk_list_kernel<TPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TokenListShared<TPC>))) != cudaSuccess) return -4;
-    attr_set = true;
-  }
+  // per call, not once per process: the attribute belongs to the current device, and four tokens take more than the default limit
+  if (cudaFuncSetAttribute(token_topk_list_kernel<TPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TokenListShared<TPC>))) != cudaSuccess) return -4;
   // sample: at most every eighth block, at least enough groups for all maxima, and an expected list (step * k) of half its room
   const int groups = g.L * (g.F / 8);
   int step = kTkList / 2 / k;

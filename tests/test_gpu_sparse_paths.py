@@ -248,6 +248,16 @@ def test_token_topk_list_takes_ties_by_the_lowest_index(ext, B, k):
     _check_token_topk(ext, x, torch.zeros(L, F, device=dev), torch.ones(L, F, device=dev), k, F, dev)
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_token_topk_on_two_devices_of_one_process(ext):
+    for i in (0, 1):
+        dev = torch.device("cuda", i)
+        x = torch.randn(2, 1800, 512, device=dev).bfloat16()
+        mean, rstd = torch.empty(2, 512, device=dev), torch.empty(2, 512, device=dev)
+        ext.colstats(x, mean, rstd)
+        _check_token_topk(ext, x, mean, rstd, 8, 512, dev)
+
+
 def _serving_model(fn, tying, dev, L=3, d=64, F=512):
     from crosslayer_coding_b200 import CLTConfig, CrossLayerTranscoder
 
