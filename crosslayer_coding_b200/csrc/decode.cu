@@ -123,19 +123,26 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // ------------------------------------------------------------------ gather kernels
 // Both kernels below give a warp one token and one slice of d_model and let it walk the token's active entries with
 // plain 16-byte loads, a few decoder rows at a time; the sums stay in registers.  The work is a read of n_entries * targets
-// decoder rows, several times the size of the touched weights, so what bounds it is how many of those reads L2 serves and how
-// many are in flight.  One warp per (token, target) without a shared-memory ring keeps thousands of tokens resident (the ring
-// of a CTA per token held 444), all at the same target, and because the entries of a token are sorted by (layer, feature) they
-// pass over that target's rows together: 7.9 GB from DRAM become 6.3 GB at the GPT-2 shape.
-// Walk configurations.  Few warps with four rows in flight each finish a short list soonest; with thousands of tokens it is the
-// number of tokens on the chip that counts: seven-warp CTAs of 72 registers, two rows in flight, put 28 warps on an SM.
-// GPT-2 shape, 4096 tokens, k = 200: 2.08 ms with 16 warps of four rows, 1.80 ms with 28 of two; 512 tokens, k = 32: 0.119
-// against 0.151 ms.
-constexpr int kWalkWarps = 8;
-constexpr int kFullWarps = 7;
+// decoder rows, several times the size of the touched weights, by chains of dependent loads (list, row): bound by how many warps
+// are in a chain at any moment, and with thousands of tokens by DRAM (GPT-2 shape, 4096 tokens, k = 200: 7.0 GB in 1.39 ms, 5.2 TB/s,
+// where 2.9 GB are touched; all warps are at the same target and the entries of a token are sorted by (layer, feature), so that L2
+// serves the rest).
+//
+// A walk is a CTA of one warp: lists differ in length (a global selection gives the tokens between none and six times the average),
+// and warps that share a CTA wait for the longest of their lists.  GPT-2 shape, 4096 tokens, BatchTopK k = 200: 1977 us with seven
+// tokens per CTA, 1400 with one; k = 32: 555 and 379 (a CTA per token behind a ring of bulk copies, the form before: 2013 and 475).
+// With equally long lists it is 268 and 238 us (2048 tokens, top-k of 64).
+// Two walk configurations, by rows in flight against warps per SM: four rows and 16 warps (three or four vectors per lane) finish a
+// short list soonest, two rows and 28 (three vectors: 72 registers) or 21 keep more tokens on the chip.  GPT-2 shape, k = 32: 1024 tokens
+// 155 us with four rows against 186 with two, 2048 252 against 264, 3072 324 against 315, 4096 402 against 375; k = 200: 2048 870
+// against 895, 4096 1503 against 1399; equal lists of 64, 2048 tokens: 262 against 238.  So the line is at 2048 tokens.
+// The entries of a token are split over the eight warps of a CTA while there are few (token, target) warps: long lists then
+// decide.  340 tokens, k = 32: 70 us split, 122 not; 512 tokens (6144 warps): 102 and 127; 1024: 181 and 155.  Equal lists gain less
+// from it: top-k of 32, 128 tokens 31 us split against 25 not, 340 tokens 67 against 38; of 200, 128 tokens 76 against 86.
+constexpr int kSplitWarps = 8;
 constexpr long long kRunningMinWarps = 1024;   // below: too few warps, the (token, target) split has L times as many
-constexpr int kFullMinTokens = 2048;             // from here on the chip is full of tokens
-constexpr long long kSplitBelowWarps = 4096;   // fewer (token, target) warps than that leave SMs idle: the entries are split too
+constexpr int kFullMinTokens = 2048;
+constexpr long long kSplitBelowWarps = 4096;
 
 __device__ __forceinline__ int decode_token(const DecodeParams& p, int i) {
   // Tensor-parallel push: rank r starts with the tokens owned by rank r + 1, so that at any moment the ranks
@@ -174,151 +181,142 @@ __device__ __forceinline__ void gather_rows(uint32_t mask, float a, const t16* r
   }
 }
 
-// One warp (SPLIT = 1) or one CTA of kWalkWarps warps (SPLIT = kWalkWarps: few tokens, the entries of a token are dealt to
-// the warps and the partial sums meet in shared memory) per (token, target, column chunk of NV * 256).  Every tying mode:
-// `tying` only decides which row an entry reads.  blockIdx.y counts the targets from the last one down: the longest
-// lists come first, so that the short ones fill the tail.
+// One warp (SPLIT = 1) or one CTA of kSplitWarps warps (few tokens, the entries of a token are dealt to the warps and the
+// partial sums meet in shared memory) per (token, target, column chunk of NV * 256).  Every tying mode: `tying` only decides which
+// row an entry reads.  blockIdx.y counts the targets from the last one down: the longest lists come first, so that the short ones
+// fill the tail.
 template <int NV, int SPLIT, bool FULL = false>
-__global__ void __launch_bounds__(32 * (FULL ? kFullWarps : kWalkWarps), FULL ? (NV == 4 ? 3 : 4) : (NV >= 3 ? 2 : (NV == 2 ? 3 : 4))) decode_walk_kernel(const DecodeParams p) {
+__global__ void __launch_bounds__(32 * SPLIT, SPLIT > 1 ? (NV >= 3 ? 2 : (NV == 2 ? 3 : 4)) : FULL ? (NV == 4 ? 21 : 28) : (NV >= 3 ? 16 : (NV == 2 ? 24 : 32)))
+    decode_walk_kernel(const DecodeParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = p.L - 1 - int(blockIdx.y);
-  constexpr int kWarps = FULL ? kFullWarps : kWalkWarps;
-  const int slot = SPLIT == 1 ? int(blockIdx.x) * kWarps + warp : int(blockIdx.x);
   const int d = p.d;
   const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
   float sq = 0.f;
-  __shared__ float red_s[kWarps];
-  if (slot < p.B) {
-    const int tok = decode_token(p, slot);
-    int e0[NV];
-    bool act[NV];
-    float acc[NV][8];
+  const int tok = decode_token(p, int(blockIdx.x));
+  int e0[NV];
+  bool act[NV];
+  float acc[NV][8];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    e0[v] = ((int(blockIdx.z) * NV + v) * 32 + lane) * 8;
+    act[v] = e0[v] < d;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
+  }
+  const int span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + span - 1 of a source layer s
+  const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
+  int seen = 0;  // SPLIT: entries dealt so far
+  for (int i0 = b; i0 < e; i0 += 32) {
+    const int i = i0 + lane;
+    const int col = i < e ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
+    float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
+    const int s = col >> 24, f = col & 0xFFFFFF;
+    bool use = a != 0.f;
+    if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
+    use = use && s <= t && t - s < span;
+    const t16* row = nullptr;
+    if (use) {
+      const int wi = p.tying == 2 ? t : s;
+      row = p.w[wi] + (p.tying == 0 ? 1LL * f * p.rows[s] + (t - s) : 1LL * f) * d;
+      if (p.tying != 0) {
+        if (p.feat_offset) a += p.feat_offset[1LL * t * p.col_pitch + f];
+        if (p.feat_scale) a *= p.feat_scale[1LL * t * p.col_pitch + f];
+      }
+    }
+    uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
+    if (SPLIT > 1) {
+      const int rank = seen + __popc(mask & ((1u << lane) - 1u));
+      seen += __popc(mask);
+      mask = __ballot_sync(0xFFFFFFFFu, use && rank % SPLIT == warp);
+    }
+    gather_rows<NV, FULL ? 2 : 4>(mask, a, row, e0, act, acc);
+  }
+  if (SPLIT == 1) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+      if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
+  } else {
+    __shared__ __align__(16) float part[SPLIT > 1 ? SPLIT : 1][SPLIT > 1 ? NV * 256 : 4];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      e0[v] = ((int(blockIdx.z) * NV + v) * 32 + lane) * 8;
-      act[v] = e0[v] < d;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
+      float4* dst = reinterpret_cast<float4*>(&part[warp][(v * 32 + lane) * 8]);
+      dst[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+      dst[1] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
     }
-    const int span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + span - 1 of a source layer s
-    const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
-    int seen = 0;  // SPLIT: entries dealt so far
-    for (int i0 = b; i0 < e; i0 += 32) {
-      const int i = i0 + lane;
-      const int col = i < e ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
-      float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
-      const int s = col >> 24, f = col & 0xFFFFFF;
-      bool use = a != 0.f;
-      if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
-      use = use && s <= t && t - s < span;
-      const t16* row = nullptr;
-      if (use) {
-        const int wi = p.tying == 2 ? t : s;
-        row = p.w[wi] + (p.tying == 0 ? 1LL * f * p.rows[s] + (t - s) : 1LL * f) * d;
-        if (p.tying != 0) {
-          if (p.feat_offset) a += p.feat_offset[1LL * t * p.col_pitch + f];
-          if (p.feat_scale) a *= p.feat_scale[1LL * t * p.col_pitch + f];
-        }
+    __syncthreads();
+    for (int c = threadIdx.x; c < NV * 32; c += blockDim.x) {  // one 8-element slice per thread
+      const int ec = (int(blockIdx.z) * NV * 32 + c) * 8;
+      if (ec >= d) continue;
+      float out[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) out[i] = 0.f;
+#pragma unroll
+      for (int w = 0; w < SPLIT; ++w) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[i] += part[w][c * 8 + i];
       }
-      uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
-      if (SPLIT > 1) {
-        const int rank = seen + __popc(mask & ((1u << lane) - 1u));
-        seen += __popc(mask);
-        mask = __ballot_sync(0xFFFFFFFFu, use && rank % SPLIT == warp);
-      }
-      gather_rows<NV, FULL ? 2 : 4>(mask, a, row, e0, act, acc);
-    }
-    if (SPLIT == 1) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v)
-        if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
-    } else {
-      __shared__ __align__(16) float part[SPLIT > 1 ? SPLIT : 1][SPLIT > 1 ? NV * 256 : 4];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        float4* dst = reinterpret_cast<float4*>(&part[warp][(v * 32 + lane) * 8]);
-        dst[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
-        dst[1] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
-      }
-      __syncthreads();
-      for (int c = threadIdx.x; c < NV * 32; c += blockDim.x) {  // one 8-element slice per thread
-        const int ec = (int(blockIdx.z) * NV * 32 + c) * 8;
-        if (ec >= d) continue;
-        float out[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) out[i] = 0.f;
-#pragma unroll
-        for (int w = 0; w < SPLIT; ++w) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) out[i] += part[w][c * 8 + i];
-        }
-        sq += decode_epilogue(p, tok, t, ec, out, loss_scale);
-      }
+      sq += decode_epilogue(p, tok, t, ec, out, loss_scale);
     }
   }
   if (p.mode == 1) {
-    // one shared word per warp and one global atomic per CTA: all warps of the CTA work on the same target
+    // one global atomic per CTA: all warps of the CTA work on the same target
     sq = warp_sum(sq);
-    if (lane == 0) red_s[warp] = sq;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float tot = 0.f;
-      for (int w = 0; w < kWarps; ++w) tot += red_s[w];
-      if (tot != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[t], double(tot));
+    if (SPLIT > 1) {
+      __shared__ float red_s[SPLIT];
+      if (lane == 0) red_s[warp] = sq;
+      __syncthreads();
+      sq = 0.f;
+      for (int w = 0; w < SPLIT; ++w) sq += red_s[w];
     }
+    if (threadIdx.x == 0 && sq != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[t], double(sq));
   }
 }
 
 // Per-source tied decoders without affine terms: the row of feature (s, f) serves every target t >= s with the same weight,
 // so the reconstruction of target t is the one of t - 1 plus the entries of layer t.  One warp per (token, column chunk)
 // reads every row once and finishes a target whenever a layer's entries are in.  The list is scanned once per layer
-// (coalesced, a few hundred bytes), which makes the result independent of how the entries of a token are ordered.
+// (coalesced, a few hundred bytes), so the entries of a token may come in any order (within a layer they are added in the
+// order of the list: bit for bit the same sums take a sorted list).  One warp per CTA, as in the walk: tied Pythia-70m shape, 4096
+// tokens, k = 200: 571 us with eight, 518 with one.
 template <int NV>
-__global__ void __launch_bounds__(32 * kWalkWarps, NV >= 2 ? 2 : 3) decode_running_kernel(const DecodeParams p) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int slot = int(blockIdx.x) * kWalkWarps + warp;
+__global__ void __launch_bounds__(32, NV >= 2 ? 16 : 24) decode_running_kernel(const DecodeParams p) {
+  const int lane = threadIdx.x & 31;
   const int d = p.d;
   const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
-  __shared__ float sq_s[kMaxLayers];
-  if (threadIdx.x < kMaxLayers) sq_s[threadIdx.x] = 0.f;
-  __syncthreads();
-  if (slot < p.B) {
-    const int tok = decode_token(p, slot);
-    int e0[NV];
-    bool act[NV];
-    float acc[NV][8];
+  const int tok = decode_token(p, int(blockIdx.x));
+  int e0[NV];
+  bool act[NV];
+  float acc[NV][8];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      e0[v] = ((int(blockIdx.y) * NV + v) * 32 + lane) * 8;
-      act[v] = e0[v] < d;
+  for (int v = 0; v < NV; ++v) {
+    e0[v] = ((int(blockIdx.y) * NV + v) * 32 + lane) * 8;
+    act[v] = e0[v] < d;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
+    for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
+  }
+  const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
+  for (int t = 0; t < p.L; ++t) {
+    for (int i0 = b; i0 < e; i0 += 32) {
+      const int i = i0 + lane;
+      const int col = i < e ? __ldg(p.tcsr_col + i) : 0;
+      const float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
+      const int f = col & 0xFFFFFF;
+      bool use = a != 0.f;
+      if (use && (!clt_in_bounds(col >> 24, p.L, p.dbg_status, 103) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 104))) use = false;
+      use = use && (col >> 24) == t;
+      const uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
+      if (mask != 0u) gather_rows<NV, 4>(mask, a, p.w[t] + 1LL * f * d, e0, act, acc);
     }
-    const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
-    for (int t = 0; t < p.L; ++t) {
-      for (int i0 = b; i0 < e; i0 += 32) {
-        const int i = i0 + lane;
-        const int col = i < e ? __ldg(p.tcsr_col + i) : 0;
-        const float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
-        const int f = col & 0xFFFFFF;
-        bool use = a != 0.f;
-        if (use && (!clt_in_bounds(col >> 24, p.L, p.dbg_status, 103) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 104))) use = false;
-        use = use && (col >> 24) == t;
-        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
-        if (mask != 0u) gather_rows<NV, 4>(mask, a, p.w[t] + 1LL * f * d, e0, act, acc);
-      }
-      float sq = 0.f;
+    float sq = 0.f;
 #pragma unroll
-      for (int v = 0; v < NV; ++v)
-        if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
-      if (p.mode == 1) {
-        sq = warp_sum(sq);
-        if (lane == 0) atomicAdd(&sq_s[t], sq);
-      }
+    for (int v = 0; v < NV; ++v)
+      if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
+    if (p.mode == 1) {
+      sq = warp_sum(sq);
+      if (lane == 0 && sq != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[t], double(sq));
     }
   }
-  __syncthreads();
-  if (p.mode == 1 && threadIdx.x < p.L && sq_s[threadIdx.x] != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[threadIdx.x], double(sq_s[threadIdx.x]));
 }
 
 // Epilogue for the tensor-parallel path, run after the partial reconstructions were summed across ranks:
@@ -444,7 +442,7 @@ struct CltDecodeArgs {
   void* stage_peers[8];
   int rows_per_rank, rank, world;
   int mode;
-  int* status;  // when given, untied decoders use the bulk-copy pipeline (its bounded waits report here)
+  int* status;  // may be null; the index checks of the debug build report here
   float* ctl;   // optional step control block (loss scale in, found-inf flag out)
   int rows_limit;
 };
@@ -467,28 +465,27 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   const int chunks = a->d > 1024 ? 2 : 1;
   const int nv = (a->d / 8 + 32 * chunks - 1) / (32 * chunks);
   const bool plain_tied = a->tying == 1 && a->feat_offset == nullptr && a->feat_scale == nullptr && a->rows_limit <= 0;
-  auto pick = [&](auto k1, auto k2, auto k3, auto k4, dim3 grid, int block) {
+  auto pick = [&](auto k1, auto k2, auto k3, auto k4, int block) {
+    const dim3 grid(a->B, a->L, chunks);
     if (nv <= 1) k1<<<grid, block, 0, st>>>(p);
     else if (nv == 2) k2<<<grid, block, 0, st>>>(p);
     else if (nv == 3) k3<<<grid, block, 0, st>>>(p);
     else k4<<<grid, block, 0, st>>>(p);
   };
-  const int token_ctas = (a->B + kWalkWarps - 1) / kWalkWarps;
   const int run_chunks = (a->d + 511) / 512;  // at most two vectors per lane: the sums stay live across the epilogues of all targets
-  const int block = 32 * kWalkWarps;
   if (plain_tied && 1LL * a->B * run_chunks >= kRunningMinWarps) {
-    const dim3 grid(token_ctas, run_chunks);
-    if (a->d <= 256) decode_running_kernel<1><<<grid, block, 0, st>>>(p);
-    else decode_running_kernel<2><<<grid, block, 0, st>>>(p);
+    const dim3 grid(a->B, run_chunks);
+    if (a->d <= 256) decode_running_kernel<1><<<grid, 32, 0, st>>>(p);
+    else decode_running_kernel<2><<<grid, 32, 0, st>>>(p);
   } else if (nv >= 3 && a->B >= kFullMinTokens) {
-    const dim3 grid((a->B + kFullWarps - 1) / kFullWarps, a->L, chunks);
-    if (nv == 3) decode_walk_kernel<3, 1, true><<<grid, 32 * kFullWarps, 0, st>>>(p);
-    else decode_walk_kernel<4, 1, true><<<grid, 32 * kFullWarps, 0, st>>>(p);
+    const dim3 grid(a->B, a->L, chunks);
+    if (nv == 3) decode_walk_kernel<3, 1, true><<<grid, 32, 0, st>>>(p);
+    else decode_walk_kernel<4, 1, true><<<grid, 32, 0, st>>>(p);
   } else if (1LL * a->B * a->L * chunks >= kSplitBelowWarps) {
-    pick(decode_walk_kernel<1, 1>, decode_walk_kernel<2, 1>, decode_walk_kernel<3, 1>, decode_walk_kernel<4, 1>, dim3(token_ctas, a->L, chunks), block);
+    pick(decode_walk_kernel<1, 1>, decode_walk_kernel<2, 1>, decode_walk_kernel<3, 1>, decode_walk_kernel<4, 1>, 32);
   } else {
-    pick(decode_walk_kernel<1, kWalkWarps>, decode_walk_kernel<2, kWalkWarps>, decode_walk_kernel<3, kWalkWarps>, decode_walk_kernel<4, kWalkWarps>,
-         dim3(a->B, a->L, chunks), block);
+    pick(decode_walk_kernel<1, kSplitWarps>, decode_walk_kernel<2, kSplitWarps>, decode_walk_kernel<3, kSplitWarps>, decode_walk_kernel<4, kSplitWarps>,
+         32 * kSplitWarps);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -4,7 +4,7 @@
 // flattened tensor (clt/models/activations.py:27-32, 281-357).  Here the same selection is a threshold
 // search over the bf16 pre-activations written by the encoder GEMM:
 //
-//   1. colstats      per-feature batch mean and 1/(std+1e-6) (unbiased std, from the encoder GEMM's row blocks or a pass of its own)
+//   1. colstats      per-feature batch mean and 1/(std+1e-6) (unbiased std, shifted sums)
 //   2. zhist         8192-bin histogram of the order-preserving key of z = (x-mean)*rstd, keys >= key_lo
 //   3. find_bin      bin that contains the k_total-th largest key (after the ranks' histograms were summed)
 //   4. compact       entries above the bin go to the output list, entries inside it to a candidate list
