@@ -128,18 +128,23 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // where 2.9 GB are touched; all warps are at the same target and the entries of a token are sorted by (layer, feature), so that L2
 // serves the rest).
 //
-// A walk is a CTA of one warp: lists differ in length (a global selection gives the tokens between none and six times the average),
-// and warps that share a CTA wait for the longest of their lists.  GPT-2 shape, 4096 tokens, BatchTopK k = 200: 1977 us with seven
-// tokens per CTA, 1400 with one; k = 32: 555 and 379 (a CTA per token behind a ring of bulk copies, the form before: 2013 and 475).
-// With equally long lists it is 268 and 238 us (2048 tokens, top-k of 64).
+// Lists differ in length (a global selection gives the tokens between none and six times the average), and warps that share a CTA
+// wait for the longest of their lists, so a walk of three or four vectors per lane is a CTA of one warp.  GPT-2 shape, 4096
+// tokens, BatchTopK k = 200: 1977 us with seven tokens per CTA, 1400 with one; k = 32: 555 and 379 (a CTA per token behind a ring of
+// bulk copies, the form before: 2013 and 475).  With equally long lists it is 268 and 238 us (2048 tokens, top-k of 64).  Narrow
+// rows are over sooner, and what a CTA costs by itself (its launch, its addition to the error sum, 1.5 ns together) shows: 12 x 6208
+// (token, target) pairs of 136 elements without an entry 116 us with one warp per CTA, 46 with eight, although 8000 tokens of 64 entries
+// (6 x 256) take 289 with one, 305 with two, 322 with four and 348 with eight.  So two vectors per lane go two warps to a CTA, one
+// vector four.
 // Two walk configurations, by rows in flight against warps per SM: four rows and 16 warps (three or four vectors per lane) finish a
-// short list soonest, two rows and 28 (three vectors: 72 registers) or 21 keep more tokens on the chip.  GPT-2 shape, k = 32: 1024 tokens
+// short list soonest, two rows and 28 (three vectors: 72 registers) or 20 (four) keep more tokens on the chip.  GPT-2 shape, k = 32: 1024 tokens
 // 155 us with four rows against 186 with two, 2048 252 against 264, 3072 324 against 315, 4096 402 against 375; k = 200: 2048 870
 // against 895, 4096 1503 against 1399; equal lists of 64, 2048 tokens: 262 against 238.  So the line is at 2048 tokens.
 // The entries of a token are split over the eight warps of a CTA while there are few (token, target) warps: long lists then
 // decide.  340 tokens, k = 32: 70 us split, 122 not; 512 tokens (6144 warps): 102 and 127; 1024: 181 and 155.  Equal lists gain less
 // from it: top-k of 32, 128 tokens 31 us split against 25 not, 340 tokens 67 against 38; of 200, 128 tokens 76 against 86.
 constexpr int kSplitWarps = 8;
+__host__ __device__ constexpr int walk_warps(int nv) { return nv == 1 ? 4 : (nv == 2 ? 2 : 1); }
 constexpr long long kRunningMinWarps = 1024;   // below: too few warps, the (token, target) split has L times as many
 constexpr int kFullMinTokens = 2048;
 constexpr long long kSplitBelowWarps = 4096;
@@ -186,88 +191,93 @@ __device__ __forceinline__ void gather_rows(uint32_t mask, float a, const t16* r
 // row an entry reads.  blockIdx.y counts the targets from the last one down: the longest lists come first, so that the short ones
 // fill the tail.
 template <int NV, int SPLIT, bool FULL = false>
-__global__ void __launch_bounds__(32 * SPLIT, SPLIT > 1 ? (NV >= 3 ? 2 : (NV == 2 ? 3 : 4)) : FULL ? (NV == 4 ? 21 : 28) : (NV >= 3 ? 16 : (NV == 2 ? 24 : 32)))
+__global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : walk_warps(NV)), SPLIT > 1 ? (NV >= 3 ? 2 : (NV == 2 ? 3 : 4))
+                                                                                        : (FULL ? (NV == 4 ? 20 : 28) : (NV >= 3 ? 16 : (NV == 2 ? 24 : 32))) / walk_warps(NV))
     decode_walk_kernel(const DecodeParams p) {
+  constexpr int kWarps = SPLIT > 1 ? SPLIT : walk_warps(NV);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = p.L - 1 - int(blockIdx.y);
+  const int slot = SPLIT > 1 ? int(blockIdx.x) : int(blockIdx.x) * kWarps + warp;
   const int d = p.d;
   const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
   float sq = 0.f;
-  const int tok = decode_token(p, int(blockIdx.x));
-  int e0[NV];
-  bool act[NV];
-  float acc[NV][8];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    e0[v] = ((int(blockIdx.z) * NV + v) * 32 + lane) * 8;
-    act[v] = e0[v] < d;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
-  }
-  const int span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + span - 1 of a source layer s
-  const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
-  int seen = 0;  // SPLIT: entries dealt so far
-  for (int i0 = b; i0 < e; i0 += 32) {
-    const int i = i0 + lane;
-    const int col = i < e ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
-    float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
-    const int s = col >> 24, f = col & 0xFFFFFF;
-    bool use = a != 0.f;
-    if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
-    use = use && s <= t && t - s < span;
-    const t16* row = nullptr;
-    if (use) {
-      const int wi = p.tying == 2 ? t : s;
-      row = p.w[wi] + (p.tying == 0 ? 1LL * f * p.rows[s] + (t - s) : 1LL * f) * d;
-      if (p.tying != 0) {
-        if (p.feat_offset) a += p.feat_offset[1LL * t * p.col_pitch + f];
-        if (p.feat_scale) a *= p.feat_scale[1LL * t * p.col_pitch + f];
-      }
-    }
-    uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
-    if (SPLIT > 1) {
-      const int rank = seen + __popc(mask & ((1u << lane) - 1u));
-      seen += __popc(mask);
-      mask = __ballot_sync(0xFFFFFFFFu, use && rank % SPLIT == warp);
-    }
-    gather_rows<NV, FULL ? 2 : 4>(mask, a, row, e0, act, acc);
-  }
-  if (SPLIT == 1) {
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
-  } else {
-    __shared__ __align__(16) float part[SPLIT > 1 ? SPLIT : 1][SPLIT > 1 ? NV * 256 : 4];
+  if (slot < p.B) {
+    const int tok = decode_token(p, slot);
+    int e0[NV];
+    bool act[NV];
+    float acc[NV][8];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      float4* dst = reinterpret_cast<float4*>(&part[warp][(v * 32 + lane) * 8]);
-      dst[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
-      dst[1] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
+      e0[v] = ((int(blockIdx.z) * NV + v) * 32 + lane) * 8;
+      act[v] = e0[v] < d;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < NV * 32; c += blockDim.x) {  // one 8-element slice per thread
-      const int ec = (int(blockIdx.z) * NV * 32 + c) * 8;
-      if (ec >= d) continue;
-      float out[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) out[i] = 0.f;
-#pragma unroll
-      for (int w = 0; w < SPLIT; ++w) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) out[i] += part[w][c * 8 + i];
+    const int span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + span - 1 of a source layer s
+    const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
+    int seen = 0;  // SPLIT: entries dealt so far
+    for (int i0 = b; i0 < e; i0 += 32) {
+      const int i = i0 + lane;
+      const int col = i < e ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
+      float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
+      const int s = col >> 24, f = col & 0xFFFFFF;
+      bool use = a != 0.f;
+      if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
+      use = use && s <= t && t - s < span;
+      const t16* row = nullptr;
+      if (use) {
+        const int wi = p.tying == 2 ? t : s;
+        row = p.w[wi] + (p.tying == 0 ? 1LL * f * p.rows[s] + (t - s) : 1LL * f) * d;
+        if (p.tying != 0) {
+          if (p.feat_offset) a += p.feat_offset[1LL * t * p.col_pitch + f];
+          if (p.feat_scale) a *= p.feat_scale[1LL * t * p.col_pitch + f];
+        }
       }
-      sq += decode_epilogue(p, tok, t, ec, out, loss_scale);
+      uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
+      if (SPLIT > 1) {
+        const int rank = seen + __popc(mask & ((1u << lane) - 1u));
+        seen += __popc(mask);
+        mask = __ballot_sync(0xFFFFFFFFu, use && rank % SPLIT == warp);
+      }
+      gather_rows<NV, FULL ? 2 : 4>(mask, a, row, e0, act, acc);
+    }
+    if (SPLIT == 1) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v)
+        if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
+    } else {
+      __shared__ __align__(16) float part[SPLIT > 1 ? SPLIT : 1][SPLIT > 1 ? NV * 256 : 4];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        float4* dst = reinterpret_cast<float4*>(&part[warp][(v * 32 + lane) * 8]);
+        dst[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+        dst[1] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
+      }
+      __syncthreads();
+      for (int c = threadIdx.x; c < NV * 32; c += blockDim.x) {  // one 8-element slice per thread
+        const int ec = (int(blockIdx.z) * NV * 32 + c) * 8;
+        if (ec >= d) continue;
+        float out[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[i] = 0.f;
+#pragma unroll
+        for (int w = 0; w < SPLIT; ++w) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) out[i] += part[w][c * 8 + i];
+        }
+        sq += decode_epilogue(p, tok, t, ec, out, loss_scale);
+      }
     }
   }
   if (p.mode == 1) {
     // one global atomic per CTA: all warps of the CTA work on the same target
     sq = warp_sum(sq);
-    if (SPLIT > 1) {
-      __shared__ float red_s[SPLIT];
+    if (kWarps > 1) {
+      __shared__ float red_s[kWarps];
       if (lane == 0) red_s[warp] = sq;
       __syncthreads();
       sq = 0.f;
-      for (int w = 0; w < SPLIT; ++w) sq += red_s[w];
+      for (int w = 0; w < kWarps; ++w) sq += red_s[w];
     }
     if (threadIdx.x == 0 && sq != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[t], double(sq));
   }
@@ -296,6 +306,7 @@ __global__ void __launch_bounds__(32, NV >= 2 ? 16 : 24) decode_running_kernel(c
     for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
   }
   const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
+  float sq_t = 0.f;  // lane t: the sum of target t (at most 32 layers), one addition per CTA and target at the end
   for (int t = 0; t < p.L; ++t) {
     for (int i0 = b; i0 < e; i0 += 32) {
       const int i = i0 + lane;
@@ -314,9 +325,10 @@ __global__ void __launch_bounds__(32, NV >= 2 ? 16 : 24) decode_running_kernel(c
       if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
     if (p.mode == 1) {
       sq = warp_sum(sq);
-      if (lane == 0 && sq != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[t], double(sq));
+      if (lane == t) sq_t = sq;
     }
   }
+  if (p.mode == 1 && sq_t != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[lane], double(sq_t));
 }
 
 // Epilogue for the tensor-parallel path, run after the partial reconstructions were summed across ranks:
@@ -465,27 +477,26 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   const int chunks = a->d > 1024 ? 2 : 1;
   const int nv = (a->d / 8 + 32 * chunks - 1) / (32 * chunks);
   const bool plain_tied = a->tying == 1 && a->feat_offset == nullptr && a->feat_scale == nullptr && a->rows_limit <= 0;
-  auto pick = [&](auto k1, auto k2, auto k3, auto k4, int block) {
-    const dim3 grid(a->B, a->L, chunks);
-    if (nv <= 1) k1<<<grid, block, 0, st>>>(p);
-    else if (nv == 2) k2<<<grid, block, 0, st>>>(p);
-    else if (nv == 3) k3<<<grid, block, 0, st>>>(p);
-    else k4<<<grid, block, 0, st>>>(p);
+  auto pick = [&](auto k1, auto k2, auto k3, auto k4, bool split) {
+    auto go = [&](auto kern, int warps) { kern<<<dim3(split ? a->B : (a->B + warps - 1) / warps, a->L, chunks), 32 * (split ? kSplitWarps : warps), 0, st>>>(p); };
+    if (nv <= 1) go(k1, walk_warps(1));
+    else if (nv == 2) go(k2, walk_warps(2));
+    else if (nv == 3) go(k3, walk_warps(3));
+    else go(k4, walk_warps(4));
   };
   const int run_chunks = (a->d + 511) / 512;  // at most two vectors per lane: the sums stay live across the epilogues of all targets
   if (plain_tied && 1LL * a->B * run_chunks >= kRunningMinWarps) {
     const dim3 grid(a->B, run_chunks);
     if (a->d <= 256) decode_running_kernel<1><<<grid, 32, 0, st>>>(p);
     else decode_running_kernel<2><<<grid, 32, 0, st>>>(p);
+  } else if (1LL * a->B * a->L * chunks < kSplitBelowWarps) {
+    pick(decode_walk_kernel<1, kSplitWarps>, decode_walk_kernel<2, kSplitWarps>, decode_walk_kernel<3, kSplitWarps>, decode_walk_kernel<4, kSplitWarps>, true);
   } else if (nv >= 3 && a->B >= kFullMinTokens) {
     const dim3 grid(a->B, a->L, chunks);
     if (nv == 3) decode_walk_kernel<3, 1, true><<<grid, 32, 0, st>>>(p);
     else decode_walk_kernel<4, 1, true><<<grid, 32, 0, st>>>(p);
-  } else if (1LL * a->B * a->L * chunks >= kSplitBelowWarps) {
-    pick(decode_walk_kernel<1, 1>, decode_walk_kernel<2, 1>, decode_walk_kernel<3, 1>, decode_walk_kernel<4, 1>, 32);
   } else {
-    pick(decode_walk_kernel<1, kSplitWarps>, decode_walk_kernel<2, kSplitWarps>, decode_walk_kernel<3, kSplitWarps>, decode_walk_kernel<4, kSplitWarps>,
-         32 * kSplitWarps);
+    pick(decode_walk_kernel<1, 1>, decode_walk_kernel<2, 1>, decode_walk_kernel<3, 1>, decode_walk_kernel<4, 1>, false);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
