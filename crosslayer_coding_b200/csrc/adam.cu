@@ -520,9 +520,10 @@ __device__ __forceinline__ void add_entries(int cnt, int my_x, int my_tok, float
 
 // PT: per-target tied decoders (one row per feature and target layer, shared by the source layers below): the entries of a row
 // come from several CSR segments, so none are staged in slots.
-// NB: entries beyond the staged ones that are loaded together.  NARROW: 64 registers instead of 72 (d <= 640).
+// NB: entries beyond the staged ones that are loaded together.  NARROW: 64 registers instead of 72 (d <= 640), 80 instead of 96 with
+// eight elements per thread (d <= 1792).
 template <typename WT, bool SR, int EPT, typename MT, bool PT = false, int NB = 4, bool NARROW = false>
-__global__ void __launch_bounds__(NARROW ? 192 : 288, NARROW ? 5 : (EPT == 4 ? 3 : 2)) decoder_rows_adam_bulk_kernel(const DecAdamParams p, int gthreads, int stage_bytes, int ns, int* status) {
+__global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW ? (EPT == 4 ? 5 : 3) : (EPT == 4 ? 3 : 2)) decoder_rows_adam_bulk_kernel(const DecAdamParams p, int gthreads, int stage_bytes, int ns, int* status) {
   extern __shared__ __align__(128) uint8_t smem_raw_adam[];  // bulk copies need 16-byte alignment only
   uint8_t* ring = smem_raw_adam;
   AdamBulkShared* sh = reinterpret_cast<AdamBulkShared*>(ring + size_t(ns) * stage_bytes);
@@ -1316,7 +1317,10 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
   //  * several rows per feature (untied decoders) with at most three entries per feature on average: 6 x 2864 features 576 wide, one
   //    entry in four 126 -> 126 us (129 with 72 registers), 2.7 per feature 162 -> 154 (162).
   // Above 1024 (eight elements per thread) one row per feature takes its entries one by one: 6 x 10520 rows of 1432, five per feature
-  // 478 -> 469 us (488 with batches of four).  The first figure of a pair is the sweep that waited twice per entry.
+  // 478 -> 469 us (488 with batches of four).  Between 1288 and 1408 three CTAs fit an SM with 80 registers and two with 96, and the
+  // 80-register form without batches runs whatever the lists hold: 6 x 10520 rows of 1400, one entry in four features 298 -> 298 us
+  // (355 with 96), untied rows of 6 x 4672 features 458 -> 460 (542), with eight entries per feature 1080 -> 1025 (1062).
+  // The first figure of a pair is the sweep that waited twice per entry.
   auto per_sm_of = [&](auto kern) -> int {
     int n = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
@@ -1330,6 +1334,8 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
     constexpr bool S = decltype(srv)::value;
     using W = decltype(wt);
     using M = decltype(mt);
+    if (ept == 8 && gthreads <= 224 && per_sm_of(decoder_rows_adam_bulk_kernel<W, S, 8, M, false, 1, true>) > per_sm_of(decoder_rows_adam_bulk_kernel<W, S, 8, M>))
+      return launch(decoder_rows_adam_bulk_kernel<W, S, 8, M, false, 1, true>);
     if (ept == 8) return single_rows ? launch(decoder_rows_adam_bulk_kernel<W, S, 8, M, false, 1>) : launch(decoder_rows_adam_bulk_kernel<W, S, 8, M>);
     if (short_lists && per_sm_of(decoder_rows_adam_bulk_kernel<W, S, 4, M, false, 2, true>) > per_sm_of(decoder_rows_adam_bulk_kernel<W, S, 4, M>))
       return launch(decoder_rows_adam_bulk_kernel<W, S, 4, M, false, 2, true>);

@@ -495,11 +495,11 @@ def test_per_target_rows_dealt_over_the_grid(ext, L, d, F, dtype):
     _row_update(ext, L, 90, d, 2, counts, dtype=dtype)
 
 
-# the forms of the row pipeline with 64 registers (one row per feature up to 512 wide, several rows with short lists up to 640) and
-# without batches (one row of more than 1024), next to the widths and lists that keep batches of four
+# the forms of the row pipeline with 64 registers (one row per feature up to 512 wide, several rows with short lists up to 640), with
+# 80 (1288 to 1408 wide) and without batches (one row of more than 1024), next to the widths and lists that keep batches of four
 @pytest.mark.parametrize("opts", [dict(), dict(seed=99), dict(dtype=torch.float16)])
 @pytest.mark.parametrize("single,d,short", [(True, 392, False), (True, 512, False), (True, 520, False), (False, 520, True), (False, 640, True), (False, 520, False),
-                                            (True, 1032, False), (True, 2048, False)])
+                                            (True, 1032, False), (True, 1400, False), (False, 1400, False), (True, 2048, False)])
 def test_decoder_row_update_register_forms(ext, single, d, short, opts):
     _row_update(ext, 3, 90, d, 0, COUNTS + [0] * 100 if short else COUNTS, rows_of=(lambda s: 1) if single else None, **opts)
 
