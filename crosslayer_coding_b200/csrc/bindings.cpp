@@ -5,6 +5,7 @@
 #include <torch/extension.h>
 
 #include <cstring>
+#include <string>
 #include <vector>
 
 using torch::Tensor;
@@ -189,8 +190,10 @@ int num_sms() {
   return n;
 }
 
+// The code goes into the message as text: numbers that TORCH_CHECK formats pass through an ostream of the C++ runtime that torch was
+// built with, and an extension that carries its own copy of that runtime (a statically linked libstdc++) ends with SIGSEGV there.
 void check(int rc, const char* what) {
-  TORCH_CHECK(rc == 0, what, " failed with code ", rc);
+  TORCH_CHECK(rc == 0, what, " failed with code ", std::to_string(rc));
 }
 void need(const Tensor& t, c10::ScalarType ty, const char* name) {
   TORCH_CHECK(t.is_cuda(), name, " must be a CUDA tensor");

@@ -537,3 +537,31 @@ def test_affine_gradients_without_affine_terms(ext):
     # fp32 sums of some ten thousand products: 2^-24 times the square root of their number, on terms of the size of the result
     assert (d_off.double() - want_off).abs().max() < 1e-5 * want_off.abs().max()
     assert (d_sc.double() - want_sc).abs().max() < 1e-5 * want_sc.abs().max()
+
+
+def test_refused_sizes_raise(ext):
+    """Sizes that an entry point refuses on the host (nothing is launched) come back as an exception with the code, not as the end of
+    the process."""
+    dev = _dev()
+    L, B, F = 2, 4, 8
+    off, idx, val = torch.zeros(L * F + 1, dtype=I32, device=dev), torch.zeros(1, dtype=I32, device=dev), torch.zeros(1, device=dev)
+    status = torch.zeros(4, dtype=I32, device=dev)
+
+    def rows(d):
+        W = [torch.zeros(F, 1, d, device=dev, dtype=torch.bfloat16) for _ in range(L)]
+        M, V = ([torch.zeros(F, 1, d, device=dev) for _ in range(L)] for _ in range(2))
+        gs = torch.zeros(L, B, d, device=dev, dtype=torch.bfloat16)
+        ext.decoder_rows_adam(W, M, V, L, B, d, F, 0, off, idx, val, gs, None, None, None, None, None, None, HYPER, status, None, None, None, False, None, None)
+
+    def decode(d):
+        W = [torch.zeros(F, L - s, d, device=dev, dtype=torch.bfloat16) for s in range(L)]
+        ext.sparse_decode(W, L, B, d, F, 0, torch.zeros(B + 1, dtype=I32, device=dev), idx, val, None, None, torch.zeros(L, B, d, device=dev), None, None, None,
+                          None, None, None, None, 0, [], 0, 0, status)
+
+    for call, d in ((rows, 12), (decode, 12), (decode, 2056)):
+        with pytest.raises(RuntimeError, match="failed with code -1"):
+            call(d)
+    rows(16)
+    decode(16)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
