@@ -1269,6 +1269,8 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
   if (mb && !weights_bf16) return -1;  // bf16 moments go with bf16 weights
   int nstages = kAdamStages;
   if (!bulk_rows_adam_geometry(p.d, weights_bf16, mb, &ept, &gthreads, &stage_bytes, &smem, &nstages)) return -1;
+  bool single_rows = true;
+  for (int i = 0; i < p.ntensors; ++i) single_rows = single_rows && p.rows[i] == 1;
   auto launch = [&](auto kern) -> int {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
     // resident CTAs per SM from the runtime (shared memory, threads and registers together): a grid beyond them would run a
@@ -1293,13 +1295,16 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
         if (distinct > best_distinct) { best_distinct = distinct; best = g; }
       }
     } else {
+      // CTA b owns the features b, b + grid, ... of every tensor.  With one row per feature all resident slots run, also where they do
+      // not divide the features: fewer CTAs keep fewer rows in flight (6 x 6144 rows of 592: 104 us on 683 CTAs, 88 on 740; 6 x 3072
+      // of 768: 64 us on 512, 59 on 592).
       if (bgrid > p.F_pitch) bgrid = p.F_pitch;
-      // CTA b owns the features b, b + grid, ... of every tensor: pick the grid (between three quarters of the resident slots and all
-      // of them) that splits the features most evenly, so that no CTA still streams rows when the others are done.  On a
-      // narrow shard (3072 features, 888 slots) the naive grid leaves CTAs with 3 and with 4 features per tensor.
       best = bgrid;
+      // With several rows a feature is a longer piece of work: pick the grid (between three quarters of the resident slots and all of
+      // them) that splits the features most evenly, so that no CTA still streams rows when the others are done.  2864 features of
+      // 6 to 1 rows of 512, 888 slots: 111 us on the 716 CTAs that have four each, 118 on all.
       double best_waste = double((p.F_pitch + bgrid - 1) / bgrid) * bgrid / double(p.F_pitch) - 0.03;  // a few per cent do not pay for fewer CTAs
-      for (int g = bgrid - 1; g >= (3 * bgrid) / 4 && g >= 1; --g) {
+      for (int g = bgrid - 1; !single_rows && g >= (3 * bgrid) / 4 && g >= 1; --g) {
         const int per = (p.F_pitch + g - 1) / g;
         const double waste = double(per) * g / double(p.F_pitch);
         if (waste < best_waste - 1e-9) { best_waste = waste; best = g; }
@@ -1310,26 +1315,25 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
   };
   // Registers against batches.  Four entries per batch take 72 registers, which costs rows of 392 to 608 elements a resident CTA per SM
   // (five for six up to 512, four for five above), and a list of a few entries beyond the staged ones fills no batch.  So the 64-register
-  // form with batches of two runs where it has more resident CTAs and the lists are short or wait little:
-  //  * one row per feature (encoder) up to 512 wide: 6 x 10520 rows of 440, one entry in four features 123 -> 119 us (152 with 72
-  //    registers), eight per feature 246 -> 233 (274); from 520 on the 72-register form is the better one (576 wide, eight per feature
-  //    310 -> 258 us against 304);
-  //  * several rows per feature (untied decoders) with at most three entries per feature on average: 6 x 2864 features 576 wide, one
-  //    entry in four 126 -> 126 us (129 with 72 registers), 2.7 per feature 162 -> 154 (162).
+  // form with batches of two runs where it has more resident CTAs and
+  //  * there is one row per feature (encoder; tied decoders): 6 x 10520 rows of 440, one entry in four features 123 -> 119 us (152 with
+  //    72 registers), eight per feature 246 -> 233 (274); 4 x 11312 rows of 592, one in four 112 -> 105 (133), eight 215 -> 203 (233).
+  //    With sixteen per feature the batches of four are ahead again (6 x 1504 rows of 576: 119 -> 99 us against 88);
+  //  * or untied decoders have at most three entries per feature on average: 6 x 2864 features 576 wide, one entry in four 126 -> 126
+  //    us (129 with 72 registers), 2.7 per feature 162 -> 154 (162).
   // Above 1024 (eight elements per thread) one row per feature takes its entries one by one: 6 x 10520 rows of 1432, five per feature
   // 478 -> 469 us (488 with batches of four).  Between 1288 and 1408 three CTAs fit an SM with 80 registers and two with 96, and the
   // 80-register form without batches runs whatever the lists hold: 6 x 10520 rows of 1400, one entry in four features 298 -> 298 us
   // (355 with 96), untied rows of 6 x 4672 features 458 -> 460 (542), with eight entries per feature 1080 -> 1025 (1062).
-  // The first figure of a pair is the sweep that waited twice per entry.
+  // The first figure of a pair is the sweep that waited twice per entry.  Encoder rows of 1032 to 1280 elements with fewer than three
+  // entries stay 3 to 5 % above it (6 x 10520 rows of 1152: 295 -> 306 us), with five and more they are below.
   auto per_sm_of = [&](auto kern) -> int {
     int n = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, gthreads + 32, smem) != cudaSuccess) return -1;
     return n > 6 ? 6 : n;
   };
-  bool single_rows = true;
-  for (int i = 0; i < p.ntensors; ++i) single_rows = single_rows && p.rows[i] == 1;
-  const bool short_lists = single_rows ? gthreads <= 128 : gthreads <= 160 && n_entries <= 3LL * p.F_pitch * p.L;
+  const bool short_lists = gthreads <= 160 && (single_rows || n_entries <= 3LL * p.F_pitch * p.L);
   auto pick = [&](auto srv, auto wt, auto mt) -> int {
     constexpr bool S = decltype(srv)::value;
     using W = decltype(wt);
