@@ -423,14 +423,6 @@ __device__ __forceinline__ void ldbf(const t16* p, float (&o)[EPT]) {
     o[i] = t16_lo(q.x); o[i + 1] = t16_hi(q.x); o[i + 2] = t16_lo(q.y); o[i + 3] = t16_hi(q.y);
   }
 }
-template <int EPT>
-__device__ __forceinline__ void ldbf_global(const t16* p, float (&o)[EPT]) {
-#pragma unroll
-  for (int i = 0; i < EPT; i += 4) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2*>(p + i));
-    o[i] = t16_lo(q.x); o[i + 1] = t16_hi(q.x); o[i + 2] = t16_lo(q.y); o[i + 3] = t16_hi(q.y);
-  }
-}
 template <int EPT, bool SR>
 __device__ __forceinline__ void stbf(t16* p, const float (&o)[EPT], unsigned int seed, unsigned int idx) {
 #pragma unroll

@@ -1753,8 +1753,15 @@ extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, cudaStream_
   const int grid = (a->B + kTokPerCta - 1) / kTokPerCta;
   const bool list = k <= kTkMaxima / 2;
   if (list) {
-    const int rc = a->B >= 1776 ? launch_token_list<4>(a, g, f_valid, int(k), st) : a->B >= 592 ? launch_token_list<2>(a, g, f_valid, int(k), st)
-                                                                                              : launch_token_list<1>(a, g, f_valid, int(k), st);
+    // Tokens per CTA: what finishes in one wave of 148 SMs with four CTAs each (three of four tokens, whose lists are 64 KB).  More
+    // tokens per CTA share the loads of the column statistics but take longer each, so one token while all fit that way, then
+    // two, then four (from 1332: a second wave of a few CTAs of two costs less than four tokens in a row); beyond that, in several
+    // waves, two.  6 x 32768 columns, k = 64, in us with one / two / four tokens per CTA: 592 tokens 155 / 175 / 224, 1184 288 / 222 /
+    // 257, 1240 - / 255 / 290, 1500 320 / 339 / 298, 1776 355 / 365 / 302, 2368 466 / 427 / 509, 4096 750 / 667 / 765.
+    constexpr int kOneWave = 148 * 4;
+    const int rc = a->B <= kOneWave ? launch_token_list<1>(a, g, f_valid, int(k), st)
+                   : a->B > kOneWave * 9 / 4 && a->B <= kOneWave * 3 ? launch_token_list<4>(a, g, f_valid, int(k), st)
+                                                                   : launch_token_list<2>(a, g, f_valid, int(k), st);
     if (rc != 0) return rc;
   }
   token_topk_kernel<<<grid, 256, sizeof(TokenTopkShared), st>>>(static_cast<const t16*>(a->x), a->mean, a->rstd, g, a->col_pitch,

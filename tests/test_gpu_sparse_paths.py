@@ -198,7 +198,7 @@ def _check_token_topk(ext, x, mean, rstd, k, F, dev):
 
 
 # one, two and four tokens per CTA with a last CTA that is not full; k up to the radix rounds; padding columns
-@pytest.mark.parametrize("L,B,Fl,F,k", [(3, 5, 4096, 4096, 64), (2, 601, 2056, 2050, 24), (4, 1779, 520, 520, 7), (2, 33, 1032, 1030, 513), (1, 9, 64, 64, 64),
+@pytest.mark.parametrize("L,B,Fl,F,k", [(3, 5, 4096, 4096, 64), (2, 601, 2056, 2050, 24), (4, 1779, 520, 520, 7), (4, 1401, 520, 520, 7), (2, 33, 1032, 1030, 513), (1, 9, 64, 64, 64),
                                         (2, 40, 16384, 16384, 300)])
 def test_token_topk(ext, L, B, Fl, F, k):
     dev = _dev()
@@ -215,7 +215,7 @@ def test_token_topk(ext, L, B, Fl, F, k):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("B", [6, 602, 1781])
+@pytest.mark.parametrize("B", [6, 602, 1401, 1781])
 def test_token_topk_hands_overflowing_lists_to_the_radix_rounds(ext, B, dtype):
     """The bound on a token's k-th key comes from every eighth block of 2048 columns here.  Large values in the blocks between stay
     above it, more of them than the list holds: those tokens are marked for the radix kernel, which takes them and their
@@ -235,7 +235,7 @@ def test_token_topk_hands_overflowing_lists_to_the_radix_rounds(ext, B, dtype):
     _check_token_topk(ext, x, torch.zeros(L, F, device=dev), torch.ones(L, F, device=dev), k, F, dev)
 
 
-@pytest.mark.parametrize("B,k", [(5, 64), (700, 24), (1800, 7)])
+@pytest.mark.parametrize("B,k", [(5, 64), (700, 24), (1400, 7)])
 def test_token_topk_list_takes_ties_by_the_lowest_index(ext, B, k):
     """Keys with a spacing of a half: dozens of columns share the key at the cut, and the list kernel keeps the first of them."""
     dev = _dev()
@@ -252,7 +252,7 @@ def test_token_topk_list_takes_ties_by_the_lowest_index(ext, B, k):
 def test_token_topk_on_two_devices_of_one_process(ext):
     for i in (0, 1):
         dev = torch.device("cuda", i)
-        x = torch.randn(2, 1800, 512, device=dev).bfloat16()
+        x = torch.randn(2, 1401, 512, device=dev).bfloat16()
         mean, rstd = torch.empty(2, 512, device=dev), torch.empty(2, 512, device=dev)
         ext.colstats(x, mean, rstd)
         _check_token_topk(ext, x, mean, rstd, 8, 512, dev)
