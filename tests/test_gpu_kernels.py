@@ -387,7 +387,7 @@ def test_dead_counter_and_csr_consistency():
 
 @pytest.mark.parametrize("L,d", [(16, 2048), (6, 1536), (5, 2048)])
 def test_sparse_decode_wide_rows_take_the_bulk_ring(L, d):
-    """d_model above 1024: two column chunks per thread and a ring of fewer, larger stages (64 KB per stage at 16 layers x 2048)."""
+    """d_model above 1024: a row is read in two column chunks."""
     cfg, model, tc, eng, X, Y = _engine_and_model(L=L, d=d, F=256, B=64, k=6, seed=5)
     yhat = eng.forward(X, Y)
     torch.cuda.synchronize()
