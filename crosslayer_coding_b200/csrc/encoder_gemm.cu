@@ -6,9 +6,9 @@
 // Counterpart of the reference's per-layer F.linear calls (clt/models/parallel.py:286 through
 // clt/models/encoder.py:101).
 //
-// Structure: one CTA per SM, 6 warps.  Warp 0 feeds a 4-stage shared-memory ring with TMA tile loads
+// Structure: one CTA per SM, 10 warps.  Warp 0 feeds a 4-stage shared-memory ring with TMA tile loads
 // (no cluster multicast: every CTA fetches its own tiles), warp 1 issues tcgen05.mma 128x256x16 into one
-// of two 256-column TMEM accumulators, warps 2-5 drain the other accumulator with tcgen05.ld, add the
+// of two 256-column TMEM accumulators, warps 2-9 drain the other accumulator with tcgen05.ld, add the
 // bias and store bf16.  Tiles are ordered m-fastest so CTAs that run together share the weight tile in L2.
 // Every mbarrier wait is bounded; on a timeout the CTA records STATUS_WAIT_TIMEOUT, drains its copies,
 // frees its TMEM and returns.
@@ -22,61 +22,75 @@ namespace gemm {
 constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 64;  // 64 bf16 = one 128-byte swizzled row
-constexpr int STAGES = 4;
 constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
 constexpr uint32_t B_BYTES = BN * BK * 2;
 constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int NUM_THREADS = 192;
+constexpr int NUM_THREADS = 320;
 constexpr uint32_t TMEM_COLS = 512;
-// ring + 1024 B alignment slack + barriers/bias
-constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + 4 * 4096 + 1024 + 4096;  // ring + epilogue staging + slack + barriers
 }  // namespace gemm
 
-// Epilogue of one 32-row slab (one warp, lane = row): TMEM -> registers -> + bias -> bf16 -> shared staging
+// Epilogue of 32 rows x 128 columns (one warp, lane = row): TMEM -> registers -> + bias -> 16 bit -> shared staging
 // tile of 32 rows x 64 columns in the 128-byte-swizzled layout -> one TMA store per 64 columns.  Writing
 // full rows through TMA instead of 16 bytes per lane and row keeps the L1/shared data pipe, which the tensor
-// core's operand reads share, almost free.  `stage` is this warp's 4 KB buffer (1024-byte aligned).
+// core's operand reads share, almost free.
+//
+// Eight warps drain a tile (two per TMEM lane quarter), and a warp takes all of its 128 columns into registers before it
+// converts the first: the accumulator goes back to the MMA warp after the TMEM reads, not after the stores.  With four warps,
+// 64 columns at a time, one chain of TMEM read, conversion, staging and store per 64 columns took about 2400 cycles, 9900 a tile,
+// where the MMAs of a tile take 4096 at K = 512 (and 6144 at K = 768): the epilogue was what bounded every K below about 900.
 constexpr int kEpiCols = 64;
+constexpr int kEpiWarps = 8;
+constexpr int kEpiThreads = 32 * kEpiWarps;
+constexpr int kEpiWarpCols = 128;
 constexpr uint32_t kEpiStageBytes = 32 * kEpiCols * 2;
 
-// With `colacc` (shared, [2][BN] floats: sums and sums of squares per tile column) the slab's column statistics
-// of the rounded bf16 values are read back from the staging tile (each lane owns two adjacent columns) and
-// added up over the tile's four slabs; `nrows` masks the rows beyond the matrix.
-__device__ __forceinline__ void epilogue_slab(uint32_t taddr, const CUtensorMap* map_c, uint8_t* stage, const float* bias_s,
-                                              int bn, int n_base, int m_base, int l, int lane, float* colacc, int bn_full, int nrows) {
-  for (int c = 0; c < bn / kEpiCols; ++c) {
-    uint32_t r0[32], r1[32];
-    tmem_ld_32x32(taddr + c * kEpiCols, r0);
-    tmem_ld_32x32(taddr + c * kEpiCols + 32, r1);
-    if (lane == 0) bulk_wait_read<0>();  // the previous store has read the staging tile
+// `stage`: this warp's BUFS staging tiles (1024-byte aligned), used in turn (`turn` counts the stores); `chunks` of the two
+// 64-column chunks are inside the matrix; `release` hands the accumulator back.
+// With `colacc` (shared, [2][BN] floats: sums and sums of squares per tile column) the column statistics of the rounded
+// values are read back from the staging tile (each lane owns two adjacent columns) and added up over the tile's
+// four row slabs; `nrows` masks the rows beyond the matrix.
+template <int BUFS, bool STATS, typename Release>
+__device__ __forceinline__ void epilogue_warp(uint32_t taddr, const CUtensorMap* map_c, uint8_t* stage, uint32_t& turn, const t16* bias_s,
+                                              int chunks, int n_base, int m_base, int l, int lane, float* colacc, int bn_full, int nrows,
+                                              Release release) {
+  uint32_t r[4][32];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) tmem_ld_32x32(taddr + j * 32, r[j]);
+  tmem_ld_wait();
+  release();
+#pragma unroll
+  for (int c = 0; c < kEpiWarpCols / kEpiCols; ++c) {
+    if (c >= chunks) break;
+    uint8_t* tile = stage + (BUFS > 1 ? (turn % BUFS) * kEpiStageBytes : 0u);
+    ++turn;
+    if (lane == 0) bulk_wait_read<BUFS - 1>();  // the store that used this staging tile before has read it
     __syncwarp();
-    tmem_ld_wait();
-    const float4* b4 = reinterpret_cast<const float4*>(bias_s + c * kEpiCols);
+    const uint4* b8 = reinterpret_cast<const uint4*>(bias_s + c * kEpiCols);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {  // 16-byte chunk j of this lane's row: columns [8j, 8j + 8)
-      const uint32_t* r = j < 4 ? &r0[8 * j] : &r1[8 * (j - 4)];
-      const float4 ba = b4[2 * j], bb = b4[2 * j + 1];
+      const uint32_t* v = &r[2 * c + (j >> 2)][8 * (j & 3)];
+      const uint4 b = b8[j];  // the same address in every lane: one broadcast
       uint4 q;
-      q.x = pack_t16x2(__uint_as_float(r[0]) + ba.x, __uint_as_float(r[1]) + ba.y);
-      q.y = pack_t16x2(__uint_as_float(r[2]) + ba.z, __uint_as_float(r[3]) + ba.w);
-      q.z = pack_t16x2(__uint_as_float(r[4]) + bb.x, __uint_as_float(r[5]) + bb.y);
-      q.w = pack_t16x2(__uint_as_float(r[6]) + bb.z, __uint_as_float(r[7]) + bb.w);
-      *reinterpret_cast<uint4*>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) = q;
+      q.x = pack_t16x2(__uint_as_float(v[0]) + t16_lo(b.x), __uint_as_float(v[1]) + t16_hi(b.x));
+      q.y = pack_t16x2(__uint_as_float(v[2]) + t16_lo(b.y), __uint_as_float(v[3]) + t16_hi(b.y));
+      q.z = pack_t16x2(__uint_as_float(v[4]) + t16_lo(b.z), __uint_as_float(v[5]) + t16_hi(b.z));
+      q.w = pack_t16x2(__uint_as_float(v[6]) + t16_lo(b.w), __uint_as_float(v[7]) + t16_hi(b.w));
+      *reinterpret_cast<uint4*>(tile + lane * 128 + ((j ^ (lane & 7)) << 4)) = q;
     }
     fence_proxy_async();
     __syncwarp();
     if (lane == 0) {
-      tma_store_3d(map_c, stage, n_base + c * kEpiCols, m_base, l);
+      tma_store_3d(map_c, tile, n_base + c * kEpiCols, m_base, l);
       bulk_commit();
     }
-    if (colacc != nullptr) {
+    if constexpr (STATS) {
       float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
       const uint32_t chunk = uint32_t(lane >> 2), inner = uint32_t(lane & 3) * 4u;
 #pragma unroll 8
-      for (int r = 0; r < 32; ++r) {
-        if (r < nrows) {
-          const uint32_t u = *reinterpret_cast<const uint32_t*>(stage + r * 128 + ((chunk ^ uint32_t(r & 7)) << 4) + inner);
+      for (int i = 0; i < 32; ++i) {
+        if (i < nrows) {
+          const uint32_t u = *reinterpret_cast<const uint32_t*>(tile + i * 128 + ((chunk ^ uint32_t(i & 7)) << 4) + inner);
           const float a = t16_lo(u), b = t16_hi(u);
           s0 += a; q0 = fmaf(a, a, q0);
           s1 += b; q1 = fmaf(b, b, q1);
@@ -89,10 +103,24 @@ __device__ __forceinline__ void epilogue_slab(uint32_t taddr, const CUtensorMap*
   }
 }
 
+// This warp's 128 bias values in shared memory (four per lane, 16-bit as they are stored); columns beyond N read 0.
+__device__ __forceinline__ void load_bias(t16* bias_s, const t16* bias, long long row, int n_base, int N, int lane) {
+  t16 v[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int n = n_base + 4 * lane + i;
+    v[i] = (bias != nullptr && n < N) ? bias[row + n] : float_to_t16(0.f);
+  }
+  __syncwarp();  // the previous tile's reads are done
+#pragma unroll
+  for (int i = 0; i < 2; ++i) reinterpret_cast<t16x2*>(bias_s)[2 * lane + i] = make_t16x2(v[2 * i], v[2 * i + 1]);
+  __syncwarp();
+}
+
 // Per-tile column statistics -> global partials [L][row blocks of 128][N][2], then cleared for the next tile.
 __device__ __forceinline__ void flush_tile_stats(float* colacc, int bn_full, float* tile_stats, int l, int row_block, int row_blocks,
                                                  int n_base, int N, int etid) {
-  for (int j = etid; j < bn_full; j += 128) {
+  for (int j = etid; j < bn_full; j += kEpiThreads) {
     const int n = n_base + j;
     if (n < N && row_block < row_blocks) {
       float2* dst = reinterpret_cast<float2*>(tile_stats) + (1LL * l * row_blocks + row_block) * N + n;
@@ -103,29 +131,35 @@ __device__ __forceinline__ void flush_tile_stats(float* colacc, int bn_full, flo
   }
 }
 
+template <int STAGES, bool STATS>
 struct GemmShared {
-  uint64_t full[gemm::STAGES];
-  uint64_t empty[gemm::STAGES];
+  uint64_t full[STAGES];
+  uint64_t empty[STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   int abort_flag;
   int epi_ok;
-  alignas(16) float bias[gemm::BN];
-  float colacc[2 * gemm::BN];
+  alignas(16) t16 bias[kEpiWarps][kEpiWarpCols];  // per epilogue warp: no barrier between the warps of a tile
+  float colacc[STATS ? 2 * gemm::BN : 1];
 };
+// ring + epilogue staging + barriers, bias and column sums
+template <int STAGES, int BUFS, bool STATS, uint32_t STAGE_BYTES>
+constexpr size_t kGemmSmem = size_t(STAGES) * STAGE_BYTES + size_t(kEpiWarps) * BUFS * kEpiStageBytes + sizeof(GemmShared<STAGES, STATS>);
+constexpr size_t kMaxDynamicSmem = 227 * 1024;
 
+template <int STAGES, int BUFS, bool STATS>
 __global__ void __launch_bounds__(gemm::NUM_THREADS, 1)
 encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_c, const t16* __restrict__ bias,
                     int L, int M, int N, int K, long long ldc, long long layer_stride_c, int* __restrict__ status,
                     float* __restrict__ tile_stats) {
   using namespace gemm;
-  extern __shared__ uint8_t smem_raw[];
-  // 128-byte-swizzled tiles need 1024-byte alignment
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;  // four 4 KB staging tiles, 1024-byte aligned
-  GemmShared* sh = reinterpret_cast<GemmShared*>(epi_stage + 4 * kEpiStageBytes);
+  extern __shared__ __align__(1024) uint8_t tiles[];  // 128-byte-swizzled tiles need 1024-byte alignment
+  uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;  // 4 KB staging tiles, 1024-byte aligned
+  using Shared = GemmShared<STAGES, STATS>;
+  static_assert(kGemmSmem<STAGES, BUFS, STATS, STAGE_BYTES> <= kMaxDynamicSmem, "shared memory of one CTA");
+  Shared* sh = reinterpret_cast<Shared*>(epi_stage + kEpiWarps * BUFS * kEpiStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -142,12 +176,14 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh->tmem_full[b], 1);
-      mbar_init(&sh->tmem_empty[b], 4);
+      mbar_init(&sh->tmem_empty[b], kEpiWarps);
     }
     sh->abort_flag = 0;
     fence_barrier_init();
   }
-  for (int j = threadIdx.x; j < 2 * BN; j += NUM_THREADS) sh->colacc[j] = 0.f;
+  if constexpr (STATS) {
+    for (int j = threadIdx.x; j < 2 * BN; j += NUM_THREADS) sh->colacc[j] = 0.f;
+  }
   if (warp == 1) {
     tmem_alloc(&sh->tmem_base, TMEM_COLS);
     tmem_relinquish();
@@ -225,10 +261,13 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   } else {
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) belong to this warp
-    const int etid = (warp - 2) * 32 + lane;
+    const int ew = warp - 2;
+    const int col0 = (ew >> 2) * kEpiWarpCols;
+    const int etid = ew * 32 + lane;
     const int row_blocks = (M + 127) / 128;
+    uint8_t* stage = epi_stage + ew * BUFS * kEpiStageBytes;
     int prev_l = -1, prev_rb = 0, prev_n = 0;
-    uint32_t local_tile = 0;
+    uint32_t local_tile = 0, turn = 0;
     bool ok = true;
     for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local_tile) {
       const int mt = int(t % tiles_m);
@@ -236,30 +275,43 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int l = int(t / (1LL * tiles_m * tiles_n));
       const uint32_t buf = local_tile & 1;
       const uint32_t tph = (local_tile >> 1) & 1;
-      named_barrier_sync(1, 128);  // previous tile's bias reads and column sums are done
-      if (tile_stats != nullptr && prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
-      prev_l = l; prev_rb = mt; prev_n = nt * BN;
-      for (int j = etid; j < BN; j += 128) {
-        const int n = nt * BN + j;
-        sh->bias[j] = (bias != nullptr && n < N) ? t16_to_float(bias[1LL * l * N + n]) : 0.f;
+      const int n_base = nt * BN + col0;
+      load_bias(sh->bias[ew], bias, 1LL * l * N, n_base, N, lane);
+      if constexpr (STATS) {
+        named_barrier_sync(1, kEpiThreads);  // the previous tile's column sums are complete
+        if (prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
+        prev_l = l; prev_rb = mt; prev_n = nt * BN;
+        // One thread performs the bounded wait and publishes the outcome, so the warps always
+        // take the same branch and nobody is left alone at a named barrier.
+        if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
+        named_barrier_sync(1, kEpiThreads);
+        ok = sh->epi_ok != 0;
+      } else {
+        int landed = 0;
+        if (lane == 0) landed = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
+        ok = __shfl_sync(0xFFFFFFFFu, landed, 0) != 0;
       }
-      // One thread performs the bounded wait and publishes the outcome, so the four warps always
-      // take the same branch and nobody is left alone at a named barrier.
-      if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-      named_barrier_sync(1, 128);
-      if (!sh->epi_ok) { ok = false; break; }
+      if (!ok) break;
       tc_fence_after();
-      const int m_base = mt * BM + quarter * 32;
-      const uint32_t taddr = tmem_base + buf * BN + (uint32_t(quarter * 32) << 16);
-      if (m_base < M) epilogue_slab(taddr, &map_c, epi_stage + (warp - 2) * kEpiStageBytes, sh->bias, min(BN, ((N - nt * BN + kEpiCols - 1) / kEpiCols) * kEpiCols), nt * BN, m_base, l, lane,
-                                    tile_stats != nullptr ? sh->colacc : nullptr, BN, min(32, M - m_base));
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->tmem_empty[buf]);
+      const int m_base = (mt) * BM + quarter * 32;
+      const uint32_t taddr = tmem_base + buf * BN + col0 + (uint32_t(quarter * 32) << 16);
+      const int chunks = m_base < M ? (N - n_base + kEpiCols - 1) / kEpiCols : 0;
+      const auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh->tmem_empty[buf]);
+      };
+      if (chunks > 0)
+        epilogue_warp<BUFS, STATS>(taddr, &map_c, stage, turn, sh->bias[ew], chunks, n_base, m_base, l, lane,
+                                   STATS ? sh->colacc + col0 : nullptr, BN, min(32, M - m_base), release);
+      else
+        release();
     }
-    if (ok && tile_stats != nullptr && prev_l >= 0) {
-      named_barrier_sync(1, 128);
-      flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
+    if constexpr (STATS) {
+      if (ok && prev_l >= 0) {
+        named_barrier_sync(1, kEpiThreads);
+        flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
+      }
     }
   }
 
@@ -283,44 +335,32 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //   full[s]        leader only: armed by the leader's producer for the bytes of both CTAs
 //   empty[s]       both CTAs: commit (multicast) after the MMAs of the stage
 //   tmem_full[b]   both CTAs: commit (multicast) after the tile's last MMA
-//   tmem_empty[b]  leader only: 8 arrivals, four epilogue warps of each CTA
+//   tmem_empty[b]  leader only: 16 arrivals, eight epilogue warps of each CTA
 namespace gemm2 {
 constexpr int BM = 128;       // rows per CTA; the pair covers 256
 constexpr int BN = 256;
 constexpr int BN_HALF = 128;  // weight rows loaded per CTA
 constexpr int BK = 64;
-constexpr int STAGES = 6;
 constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
 constexpr uint32_t B_BYTES = BN_HALF * BK * 2;
 constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int NUM_THREADS = 192;
+constexpr int NUM_THREADS = 320;
 constexpr uint32_t TMEM_COLS = 512;
-constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + 4 * 4096 + 1024 + 4096;
 }  // namespace gemm2
 
-struct GemmPairShared {
-  uint64_t full[gemm2::STAGES];
-  uint64_t empty[gemm2::STAGES];
-  uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];
-  uint32_t tmem_base;
-  int abort_flag;
-  int epi_ok;
-  alignas(16) float bias[gemm2::BN];
-  float colacc[2 * gemm2::BN];
-};
-
+template <int STAGES, int BUFS, bool STATS>
 __global__ void __launch_bounds__(gemm2::NUM_THREADS, 1)
 encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_c, const t16* __restrict__ bias,
                          int L, int M, int N, int K, long long ldc, long long layer_stride_c, int* __restrict__ status,
                          float* __restrict__ tile_stats) {
   using namespace gemm2;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t tiles[];
   uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;
-  GemmPairShared* sh = reinterpret_cast<GemmPairShared*>(epi_stage + 4 * kEpiStageBytes);
+  using Shared = GemmShared<STAGES, STATS>;
+  static_assert(kGemmSmem<STAGES, BUFS, STATS, STAGE_BYTES> <= kMaxDynamicSmem, "shared memory of one CTA");
+  Shared* sh = reinterpret_cast<Shared*>(epi_stage + kEpiWarps * BUFS * kEpiStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -341,12 +381,14 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh->tmem_full[b], 1);
-      mbar_init(&sh->tmem_empty[b], 8);
+      mbar_init(&sh->tmem_empty[b], 2 * kEpiWarps);
     }
     sh->abort_flag = 0;
     fence_barrier_init();
   }
-  for (int j = threadIdx.x; j < 2 * BN; j += NUM_THREADS) sh->colacc[j] = 0.f;
+  if constexpr (STATS) {
+    for (int j = threadIdx.x; j < 2 * BN; j += NUM_THREADS) sh->colacc[j] = 0.f;
+  }
   if (warp == 1) {
     tmem_alloc_pair(&sh->tmem_base, TMEM_COLS);
     tmem_relinquish_pair();
@@ -414,11 +456,14 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
   } else {
     // ---------------------------------------------------------------- epilogue (both CTAs)
-    const int quarter = warp & 3;
-    const int etid = (warp - 2) * 32 + lane;
+    const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) belong to this warp
+    const int ew = warp - 2;
+    const int col0 = (ew >> 2) * kEpiWarpCols;
+    const int etid = ew * 32 + lane;
     const int row_blocks = (M + 127) / 128;
+    uint8_t* stage = epi_stage + ew * BUFS * kEpiStageBytes;
     int prev_l = -1, prev_rb = 0, prev_n = 0;
-    uint32_t local_tile = 0;
+    uint32_t local_tile = 0, turn = 0;
     bool ok = true;
     for (long long t = pair; t < total_tiles && ok; t += npairs, ++local_tile) {
       const int mt = int(t % tiles_m);
@@ -426,28 +471,43 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int l = int(t / (1LL * tiles_m * tiles_n));
       const uint32_t buf = local_tile & 1;
       const uint32_t tph = (local_tile >> 1) & 1;
-      named_barrier_sync(1, 128);
-      if (tile_stats != nullptr && prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
-      prev_l = l; prev_rb = mt * 2 + int(cta_rank); prev_n = nt * BN;
-      for (int j = etid; j < BN; j += 128) {
-        const int n = nt * BN + j;
-        sh->bias[j] = (bias != nullptr && n < N) ? t16_to_float(bias[1LL * l * N + n]) : 0.f;
+      const int n_base = nt * BN + col0;
+      load_bias(sh->bias[ew], bias, 1LL * l * N, n_base, N, lane);
+      if constexpr (STATS) {
+        named_barrier_sync(1, kEpiThreads);  // the previous tile's column sums are complete
+        if (prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
+        prev_l = l; prev_rb = mt * 2 + int(cta_rank); prev_n = nt * BN;
+        // One thread performs the bounded wait and publishes the outcome, so the warps always
+        // take the same branch and nobody is left alone at a named barrier.
+        if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
+        named_barrier_sync(1, kEpiThreads);
+        ok = sh->epi_ok != 0;
+      } else {
+        int landed = 0;
+        if (lane == 0) landed = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
+        ok = __shfl_sync(0xFFFFFFFFu, landed, 0) != 0;
       }
-      if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-      named_barrier_sync(1, 128);
-      if (!sh->epi_ok) { ok = false; break; }
+      if (!ok) break;
       tc_fence_after();
       const int m_base = (mt * 2 + int(cta_rank)) * BM + quarter * 32;
-      const uint32_t taddr = tmem_base + buf * BN + (uint32_t(quarter * 32) << 16);
-      if (m_base < M) epilogue_slab(taddr, &map_c, epi_stage + (warp - 2) * kEpiStageBytes, sh->bias, min(BN, ((N - nt * BN + kEpiCols - 1) / kEpiCols) * kEpiCols), nt * BN, m_base, l, lane,
-                                    tile_stats != nullptr ? sh->colacc : nullptr, BN, min(32, M - m_base));
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&sh->tmem_empty[buf]), 0));  // the leader's barrier
+      const uint32_t taddr = tmem_base + buf * BN + col0 + (uint32_t(quarter * 32) << 16);
+      const int chunks = m_base < M ? (N - n_base + kEpiCols - 1) / kEpiCols : 0;
+      const auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&sh->tmem_empty[buf]), 0));  // the leader's barrier
+      };
+      if (chunks > 0)
+        epilogue_warp<BUFS, STATS>(taddr, &map_c, stage, turn, sh->bias[ew], chunks, n_base, m_base, l, lane,
+                                   STATS ? sh->colacc + col0 : nullptr, BN, min(32, M - m_base), release);
+      else
+        release();
     }
-    if (ok && tile_stats != nullptr && prev_l >= 0) {
-      named_barrier_sync(1, 128);
-      flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
+    if constexpr (STATS) {
+      if (ok && prev_l >= 0) {
+        named_barrier_sync(1, kEpiThreads);
+        flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
+      }
     }
   }
 
@@ -493,6 +553,57 @@ static bool make_kmajor_map(CUtensorMap* map, const void* base, int layers, int 
   return r == CUDA_SUCCESS;
 }
 
+// Ring stages and staging tiles per epilogue warp of the pair kernel.
+constexpr int kPairStages = 6, kPairBufs = 1;
+
+template <int STAGES, int BUFS, bool STATS>
+static int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const t16* bias, int L, int M, int N, int K,
+                       long long ldc, long long layer_stride_c, int* status, float* tile_stats, int num_sms, cudaStream_t stream) {
+  auto* kernel = encoder_gemm_pair_kernel<STAGES, BUFS, STATS>;
+  constexpr size_t smem = kGemmSmem<STAGES, BUFS, STATS, gemm2::STAGE_BYTES>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * num_sms);
+  cfg.blockDim = dim3(gemm2::NUM_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  static int pair_clusters = -1;  // co-resident clusters of two, probed once
+  if (pair_clusters < 0) {
+    int n = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      n = 0;
+      (void)cudaGetLastError();
+    }
+    pair_clusters = n;
+  }
+  if (pair_clusters <= 0) return 1;
+  const long long pair_tiles = 1LL * L * ((M + 2 * gemm2::BM - 1) / (2 * gemm2::BM)) * ((N + gemm2::BN - 1) / gemm2::BN);
+  cfg.gridDim = dim3(unsigned(2 * (pair_tiles < pair_clusters ? pair_tiles : pair_clusters)));
+  if (cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_c, bias, L, M, N, K, ldc, layer_stride_c, status, tile_stats) != cudaSuccess) return -5;
+  return 0;
+}
+
+template <int STAGES, int BUFS, bool STATS>
+static int launch_single(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const t16* bias, int L, int M, int N, int K,
+                         long long ldc, long long layer_stride_c, int* status, float* tile_stats, int num_sms, cudaStream_t stream) {
+  auto* kernel = encoder_gemm_kernel<STAGES, BUFS, STATS>;
+  constexpr size_t smem = kGemmSmem<STAGES, BUFS, STATS, gemm::STAGE_BYTES>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
+    attr_set = true;
+  }
+  const long long tiles = 1LL * L * ((M + gemm::BM - 1) / gemm::BM) * ((N + gemm::BN - 1) / gemm::BN);
+  const int grid = int(tiles < num_sms ? tiles : num_sms);
+  kernel<<<grid, gemm::NUM_THREADS, smem, stream>>>(map_a, map_b, map_c, bias, L, M, N, K, ldc, layer_stride_c, status, tile_stats);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
 }  // namespace clt
 
 // Returns 0 on success, a negative value when the arguments cannot be handled (the caller raises).
@@ -507,58 +618,19 @@ extern "C" int CLT_FN(clt_encoder_gemm)(const void* A, const void* B, const void
   if (!make_kmajor_map(&map_a, A, L, M, K, K, 1LL * M * K, gemm::BM)) return -3;
   // output map: [L, M, N] with 64-column x 32-row boxes (one epilogue slab store), clipped at M and N
   if (!make_kmajor_map(&map_c, C, L, M, N, ldc, layer_stride_c, 32)) return -3;
-  // ---- CTA pairs when the problem has full 256-row tiles and the device can co-schedule clusters of two
-  static int pair_clusters = -1;  // co-resident clusters of two, probed once
-  if (pair_clusters < 0) {
-    pair_clusters = 0;
-    if (cudaFuncSetAttribute(encoder_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm2::SMEM_BYTES)) == cudaSuccess) {
-      cudaLaunchConfig_t probe = {};
-      probe.gridDim = dim3(2 * num_sms);
-      probe.blockDim = dim3(gemm2::NUM_THREADS);
-      probe.dynamicSmemBytes = gemm2::SMEM_BYTES;
-      cudaLaunchAttribute pattr[1];
-      pattr[0].id = cudaLaunchAttributeClusterDimension;
-      pattr[0].val.clusterDim.x = 2; pattr[0].val.clusterDim.y = 1; pattr[0].val.clusterDim.z = 1;
-      probe.attrs = pattr;
-      probe.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, encoder_gemm_pair_kernel, &probe) == cudaSuccess && n > 0) pair_clusters = n;
-      else (void)cudaGetLastError();
-    } else {
-      (void)cudaGetLastError();
-    }
-  }
-  const long long pair_tiles = 1LL * L * ((M + 2 * gemm2::BM - 1) / (2 * gemm2::BM)) * ((N + gemm2::BN - 1) / gemm2::BN);
   // CLT_GEMM_SINGLE_CTA=1 keeps the single-CTA 128x256 kernel for every shape (for comparisons)
   static const bool force_single = [] { const char* e = getenv("CLT_GEMM_SINGLE_CTA"); return e != nullptr && e[0] == '1'; }();
-  if (pair_clusters > 0 && !force_single && M >= 2 * gemm2::BM && pair_tiles > 0) {
+  if (1LL * L * M * N == 0) return 0;
+  const t16* bias_p = static_cast<const t16*>(bias);
+  if (M >= 2 * gemm2::BM && !force_single) {  // CTA pairs when the problem has full 256-row tiles
     if (!make_kmajor_map(&map_b, B, L, N, K, K, 1LL * N * K, gemm2::BN_HALF)) return -3;
-    const int clusters = int(pair_tiles < pair_clusters ? pair_tiles : pair_clusters);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * clusters);
-    cfg.blockDim = dim3(gemm2::NUM_THREADS);
-    cfg.dynamicSmemBytes = gemm2::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const t16* bias_p = static_cast<const t16*>(bias);
-    if (cudaLaunchKernelEx(&cfg, encoder_gemm_pair_kernel, map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats) != cudaSuccess)
-      return -5;
-    return 0;
+    const int r = tile_stats != nullptr
+                      ? launch_pair<5, 1, true>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats, num_sms, stream)
+                      : launch_pair<kPairStages, kPairBufs, false>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, nullptr, num_sms, stream);
+    if (r <= 0) return r;  // 1: the device cannot co-schedule clusters of two
   }
   if (!make_kmajor_map(&map_b, B, L, N, K, K, 1LL * N * K, gemm::BN)) return -3;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(encoder_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gemm::SMEM_BYTES)) != cudaSuccess) return -4;
-    attr_set = true;
-  }
-  const long long tiles = 1LL * L * ((M + gemm::BM - 1) / gemm::BM) * ((N + gemm::BN - 1) / gemm::BN);
-  if (tiles == 0) return 0;
-  const int grid = int(tiles < num_sms ? tiles : num_sms);
-  encoder_gemm_kernel<<<grid, gemm::NUM_THREADS, gemm::SMEM_BYTES, stream>>>(
-      map_a, map_b, map_c, static_cast<const t16*>(bias), L, M, N, K, ldc, layer_stride_c, status, tile_stats);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return tile_stats != nullptr
+             ? launch_single<3, 1, true>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats, num_sms, stream)
+             : launch_single<4, 1, false>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, nullptr, num_sms, stream);
 }

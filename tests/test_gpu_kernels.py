@@ -51,6 +51,28 @@ def test_encoder_gemm_matches_fp32(ext, L, M, N, K):
     assert rel < 4e-3, rel
 
 
+# without the column sums: rows and columns that end in the first or the second half of a tile, in a 64-column store, in a 32-row slab;
+# one CTA per tile (up to 255 rows) and pairs; more tiles than CTAs
+@pytest.mark.parametrize("M", [1, 33, 200, 256, 300, 520])
+@pytest.mark.parametrize("L,N,K", [(1, 8, 8), (2, 136, 72), (1, 200, 64), (1, 256, 520), (2, 328, 136), (3, 20488, 64)])
+@pytest.mark.parametrize("with_bias", [True, False])
+def test_encoder_gemm_tile_edges(ext, L, M, N, K, with_bias):
+    torch.manual_seed(L + M + N + K)
+    dev = _dev()
+    x = torch.randn(L, M, K, device=dev).bfloat16()
+    w = (torch.randn(L, N, K, device=dev) / math.sqrt(K)).bfloat16()
+    b = torch.randn(L, N, device=dev).bfloat16() if with_bias else None
+    out = torch.full((L, M, N), float("nan"), device=dev, dtype=torch.bfloat16)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    ext.encoder_gemm(x, w, b, out, status, None)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    ref = torch.einsum("lmk,lnk->lmn", x.double(), w.double()) + (b.double()[:, None, :] if with_bias else 0)
+    # half a unit in the last place of bf16 (2^-9) and fp32 sums of K products (2^-24 each, on the sum of their sizes)
+    size = torch.einsum("lmk,lnk->lmn", x.double().abs(), w.double().abs()) + (b.double().abs()[:, None, :] if with_bias else 0)
+    assert ((out.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (K + 1) * 2.0 ** -24 * size + 1e-30).all()
+
+
 @pytest.mark.parametrize("L,B,F", [(3, 257, 72), (2, 1030, 256)])  # the second shape takes the row-split path
 def test_colstats(ext, L, B, F):
     torch.manual_seed(1)
