@@ -43,6 +43,7 @@ struct DecodeParams {
   // seed that leaves the 16-bit range or is NaN raises ctl[SC_FOUND_INF] (the step is then skipped)
   float* ctl;
   int rows_limit;  // > 0: only the first rows_limit target rows of a feature are decoded (auxiliary loss: same layer only)
+  const int* order; // optional [B]: the token of slot i (modes 0 and 1)
   int* dbg_status; // status words for the index checks of the debug build (may be null)
 };
 
@@ -121,38 +122,42 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 }
 
 // ------------------------------------------------------------------ gather kernels
-// Both kernels below give a warp one token and one slice of d_model and let it walk the token's active entries with
-// plain 16-byte loads, a few decoder rows at a time; the sums stay in registers.  The work is a read of n_entries * targets
-// decoder rows, several times the size of the touched weights, by chains of dependent loads (list, row): bound by how many warps
-// are in a chain at any moment, and with thousands of tokens by DRAM (GPT-2 shape, 4096 tokens, k = 200: 7.0 GB in 1.39 ms, 5.2 TB/s,
-// where 2.9 GB are touched; all warps are at the same target and the entries of a token are sorted by (layer, feature), so that L2
-// serves the rest).
+// Both kernels below give a CTA one token and one slice of d_model; its warps share the token's active entries and gather the
+// decoder rows with plain 16-byte loads, a few rows at a time; the sums stay in registers and meet in shared memory.  The work is a
+// read of n_entries * targets decoder rows, several times the size of the touched weights, by chains of dependent loads (list, row).
 //
-// Lists differ in length (a global selection gives the tokens between none and six times the average), and warps that share a CTA
-// wait for the longest of their lists, so a walk of three or four vectors per lane is a CTA of one warp.  GPT-2 shape, 4096
-// tokens, BatchTopK k = 200: 1977 us with seven tokens per CTA, 1400 with one; k = 32: 555 and 379 (a CTA per token behind a ring of
-// bulk copies, the form before: 2013 and 475).  With equally long lists it is 268 and 238 us (2048 tokens, top-k of 64).  Narrow
-// rows are over sooner, and what a CTA costs by itself (its launch, its addition to the error sum, 1.5 ns together) shows: 12 x 6208
-// (token, target) pairs of 136 elements without an entry 116 us with one warp per CTA, 46 with eight, although 8000 tokens of 64 entries
-// (6 x 256) take 289 with one, 305 with two, 322 with four and 348 with eight.  So two vectors per lane go two warps to a CTA, one
-// vector four.
-// Two walk configurations, by rows in flight against warps per SM: four rows and 16 warps (three or four vectors per lane) finish a
-// short list soonest, two rows and 28 (three vectors: 72 registers) or 20 (four) keep more tokens on the chip.  GPT-2 shape, k = 32: 1024 tokens
-// 155 us with four rows against 186 with two, 2048 252 against 264, 3072 324 against 315, 4096 402 against 375; k = 200: 2048 870
-// against 895, 4096 1503 against 1399; equal lists of 64, 2048 tokens: 262 against 238.  So the line is at 2048 tokens.
-// The entries of a token are split over the eight warps of a CTA while there are few (token, target) warps: long lists then
-// decide.  340 tokens, k = 32: 70 us split, 122 not; 512 tokens (6144 warps): 102 and 127; 1024: 181 and 155.  Equal lists gain less
-// from it: top-k of 32, 128 tokens 31 us split against 25 not, 340 tokens 67 against 38; of 200, 128 tokens 76 against 86.
-constexpr int kSplitWarps = 8;
-__host__ __device__ constexpr int walk_warps(int nv) { return nv == 1 ? 4 : (nv == 2 ? 2 : 1); }
-constexpr long long kRunningMinWarps = 1024;   // below: too few warps, the (token, target) split has L times as many
-constexpr int kFullMinTokens = 2048;
-constexpr long long kSplitBelowWarps = 4096;
+// What bounds it: lists differ in length (a global selection gives the tokens between none and six times the average), so a warp
+// per token leaves the chip to the longest lists of every target, and warps that start together drift apart in the feature order, so that
+// L2 serves less.  Four warps per token: GPT-2 shape, 4096 tokens, BatchTopK k = 200, 1435 us with one warp and 1081 with four (8.2 GB of
+// rows at 7.6 TB/s, of which DRAM gives about 6); 512 tokens, k = 32: 124 and 62; 1000 tokens of 16 x 2048, 242 entries: 1138 and 963; 4096
+// tokens of 6 x 512, per-target tied, k = 64: 172 and 132.  Equally long lists lose nothing: 2048 tokens, top-k of 64, 117 and 122; 776
+// tokens of 24 entries 21 and 25.  Eight warps pay where there are too few CTAs to fill the chip (16 tokens 36 us with four, 22
+// with eight; 128 tokens of 200 entries 72 and 67; 256: 102 and 109).
+// Rows in flight against warps per SM: four rows and 20 warps (three vectors per lane) or 16 (four) are best up to some thousands of CTAs
+// (2048 tokens, k = 200: 588 us against 605 with two rows and 28 warps), two rows and more warps beyond (4096 tokens 1164 and 1081; 1000 tokens
+// of 16 x 2048 1003 and 963).  There the tokens are also taken in the order of their list lengths, longest first: warps that
+// run together then end together and stay closer in the feature order (1081 -> 1032 us, 963 -> 913).
+// Short lists over many tokens: the latency of a CTA by itself (offsets, list, rows, sums, targets) is what counts, and two warps keep
+// twice the tokens on the chip.  4096 tokens, entries per token on average: 8 139 us with two and 174 with four, 16 182 and 213, 25 (one
+// eighth of the features) 191 and 224, 32 266 and 287, 66 436 and 437, 100 629 and 606.  Only the caller knows the average without a
+// host synchronisation (its k); a threshold selection does not, and counts as long.
+// Narrow rows: what a CTA costs by itself shows, above all its addition to the error sum (1.5 ns, all CTAs of a target on one
+// address): 12 x 6208 (token, target) pairs of 136 elements without an entry take 116 us with one token per CTA, 60 with two.  So with many
+// tokens one vector per lane goes two tokens and two warps each to a CTA (4096 tokens of 6 x 256, k = 64: 93 us either way).
+// Per-source tied, running sums: 4 warps 340 us, 1 warp 610 (8192 tokens of 6 x 512, k = 200), sorted by length 295.
+constexpr long long kRunningMinWarps = 1024;   // tokens x chunks; below, the (token, target) split has L times as many CTAs
+constexpr long long kEightWarpsBelow = 2048;   // CTAs
+constexpr long long kManyCtas = 28672;         // CTAs
+constexpr long long kPairNarrowFrom = 24576;   // (token, target) pairs
+constexpr int kRunningOrderFrom = 4096;        // tokens
+constexpr int kShortBelow = 64;                // entries per token on average
+constexpr long long kShortFrom = 16384;        // CTAs
 
 __device__ __forceinline__ int decode_token(const DecodeParams& p, int i) {
   // Tensor-parallel push: rank r starts with the tokens owned by rank r + 1, so that at any moment the ranks
   // store into different owners instead of all into the same one.
-  return p.mode == 2 ? int((i + 1LL * ((p.rank + 1) % p.world) * p.rows_per_rank) % p.B) : i;
+  if (p.mode != 2) return p.order != nullptr ? __ldg(p.order + i) : i;
+  return int((i + 1LL * ((p.rank + 1) % p.world) * p.rows_per_rank) % p.B);
 }
 
 // acc += a_j * row_j over the entries whose bits are set in `mask` (lane i of the warp holds entry i of the batch: its
@@ -186,149 +191,251 @@ __device__ __forceinline__ void gather_rows(uint32_t mask, float a, const t16* r
   }
 }
 
-// One warp (SPLIT = 1) or one CTA of kSplitWarps warps (few tokens, the entries of a token are dealt to the warps and the
-// partial sums meet in shared memory) per (token, target, column chunk of NV * 256).  Every tying mode: `tying` only decides which
-// row an entry reads.  blockIdx.y counts the targets from the last one down: the longest lists come first, so that the short ones
-// fill the tail.
-template <int NV, int SPLIT, bool FULL = false>
-__global__ void __launch_bounds__(32 * (SPLIT > 1 ? SPLIT : walk_warps(NV)), SPLIT > 1 ? (NV >= 3 ? 2 : (NV == 2 ? 3 : 4))
-                                                                                        : (FULL ? (NV == 4 ? 20 : 28) : (NV >= 3 ? 16 : (NV == 2 ? 24 : 32))) / walk_warps(NV))
-    decode_walk_kernel(const DecodeParams p) {
-  constexpr int kWarps = SPLIT > 1 ? SPLIT : walk_warps(NV);
+// A warp's sums in shared memory, and the total of the SPLIT warps of a token for one 8-element slice (added in the order of
+// the warps: equal lists give equal bits).  A slice is two 16-byte vectors that lie a row of 16-byte vectors apart, so that the lanes of a
+// warp touch consecutive vectors.
+template <int NV>
+__device__ __forceinline__ void put_partial(float* sums, const float (&acc)[NV][8], int lane) {
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    float4* dst = reinterpret_cast<float4*>(sums) + v * 32 + lane;
+    dst[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+    dst[NV * 32] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
+  }
+}
+template <int NV, int SPLIT>
+__device__ __forceinline__ void sum_partials(const float (*sums)[NV * 256], int slice, float (&out)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) out[i] = 0.f;
+#pragma unroll
+  for (int w = 0; w < SPLIT; ++w) {
+    const float4* src = reinterpret_cast<const float4*>(sums[w]) + slice;
+    const float4 lo = src[0], hi = src[NV * 32];
+    out[0] += lo.x; out[1] += lo.y; out[2] += lo.z; out[3] += lo.w;
+    out[4] += hi.x; out[5] += hi.y; out[6] += hi.z; out[7] += hi.w;
+  }
+}
+
+// acc += the entries first, first + stride, first + 2 * stride, ... below `end` of a token's list for target t, 32 at a time (a lane
+// holds one; the next 32 are loaded while the rows of these are gathered).
+template <int NV, int R>
+__device__ __forceinline__ void walk_list(const DecodeParams& p, int t, int first, int stride, int end, int lane, const int (&e0)[NV], const bool (&act)[NV],
+                                          float (&acc)[NV][8]) {
+  const int span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + span - 1 of a source layer s
+  int i = first + lane * stride;
+  int col = i < end ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
+  float a = i < end ? __ldg(p.tcsr_val + i) : 0.f;
+  for (int i0 = first; i0 < end; i0 += 32 * stride) {
+    i += 32 * stride;
+    const int col_next = i < end ? __ldg(p.tcsr_col + i) : 0;
+    const float a_next = i < end ? __ldg(p.tcsr_val + i) : 0.f;
+    const int s = col >> 24, f = col & 0xFFFFFF;
+    bool use = a != 0.f;
+    if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
+    use = use && s <= t && t - s < span;
+    const t16* row = nullptr;
+    if (use) {
+      const int wi = p.tying == 2 ? t : s;
+      row = p.w[wi] + (p.tying == 0 ? 1LL * f * p.rows[s] + (t - s) : 1LL * f) * p.d;
+      if (p.tying != 0) {
+        if (p.feat_offset) a += p.feat_offset[1LL * t * p.col_pitch + f];
+        if (p.feat_scale) a *= p.feat_scale[1LL * t * p.col_pitch + f];
+      }
+    }
+    gather_rows<NV, R>(__ballot_sync(0xFFFFFFFFu, use), a, row, e0, act, acc);
+    col = col_next;
+    a = a_next;
+  }
+}
+
+// One CTA works on TOK tokens of one target layer and one column chunk of NV * 256, SPLIT warps to a token: the token's entries are
+// dealt to them one by one and the partial sums meet in shared memory.  Every tying mode: `tying` only decides which row an entry reads.
+// blockIdx.y counts the targets from the last one down: the longest lists come first, so that the short ones fill the tail.
+template <int NV, int TOK, int SPLIT, int R, int WARPS_PER_SM>
+__global__ void __launch_bounds__(32 * TOK * SPLIT, WARPS_PER_SM / (TOK * SPLIT)) decode_walk_kernel(const DecodeParams p) {
+  constexpr int kWarps = TOK * SPLIT;
+  __shared__ __align__(16) float sums[kWarps][NV * 256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = p.L - 1 - int(blockIdx.y);
-  const int slot = SPLIT > 1 ? int(blockIdx.x) : int(blockIdx.x) * kWarps + warp;
+  const int slot = int(blockIdx.x) * TOK + warp / SPLIT, part = warp % SPLIT;
   const int d = p.d;
   const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
-  float sq = 0.f;
+  int b = 0, e = 0;
   if (slot < p.B) {
     const int tok = decode_token(p, slot);
-    int e0[NV];
+    b = __ldg(p.tok_off + tok);
+    e = __ldg(p.tok_off + tok + 1);
+    if (p.target != nullptr) {  // the epilogue's row on its way while the entries are gathered
+      const int e0 = (int(blockIdx.z) * NV * 32 + part * 32 + lane) * 8;
+      if (e0 < d && part < NV) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.target + (1LL * t * p.B + tok) * d + e0));
+    }
+    int off[NV];
     bool act[NV];
     float acc[NV][8];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      e0[v] = ((int(blockIdx.z) * NV + v) * 32 + lane) * 8;
-      act[v] = e0[v] < d;
+      off[v] = ((int(blockIdx.z) * NV + v) * 32 + lane) * 8;
+      act[v] = off[v] < d;
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
     }
-    const int span = p.rows_limit > 0 ? p.rows_limit : kMaxLayers;  // targets s .. s + span - 1 of a source layer s
-    const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
-    int seen = 0;  // SPLIT: entries dealt so far
-    for (int i0 = b; i0 < e; i0 += 32) {
-      const int i = i0 + lane;
-      const int col = i < e ? __ldg(p.tcsr_col + i) : 0;  // packed by the CSR build: (layer << 24) | feature
-      float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
-      const int s = col >> 24, f = col & 0xFFFFFF;
-      bool use = a != 0.f;
-      if (use && (!clt_in_bounds(s, p.L, p.dbg_status, 101) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 102))) use = false;
-      use = use && s <= t && t - s < span;
-      const t16* row = nullptr;
-      if (use) {
-        const int wi = p.tying == 2 ? t : s;
-        row = p.w[wi] + (p.tying == 0 ? 1LL * f * p.rows[s] + (t - s) : 1LL * f) * d;
-        if (p.tying != 0) {
-          if (p.feat_offset) a += p.feat_offset[1LL * t * p.col_pitch + f];
-          if (p.feat_scale) a *= p.feat_scale[1LL * t * p.col_pitch + f];
-        }
-      }
-      uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
-      if (SPLIT > 1) {
-        const int rank = seen + __popc(mask & ((1u << lane) - 1u));
-        seen += __popc(mask);
-        mask = __ballot_sync(0xFFFFFFFFu, use && rank % SPLIT == warp);
-      }
-      gather_rows<NV, FULL ? 2 : 4>(mask, a, row, e0, act, acc);
-    }
-    if (SPLIT == 1) {
-#pragma unroll
-      for (int v = 0; v < NV; ++v)
-        if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
-    } else {
-      __shared__ __align__(16) float part[SPLIT > 1 ? SPLIT : 1][SPLIT > 1 ? NV * 256 : 4];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        float4* dst = reinterpret_cast<float4*>(&part[warp][(v * 32 + lane) * 8]);
-        dst[0] = make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
-        dst[1] = make_float4(acc[v][4], acc[v][5], acc[v][6], acc[v][7]);
-      }
-      __syncthreads();
-      for (int c = threadIdx.x; c < NV * 32; c += blockDim.x) {  // one 8-element slice per thread
-        const int ec = (int(blockIdx.z) * NV * 32 + c) * 8;
-        if (ec >= d) continue;
-        float out[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) out[i] = 0.f;
-#pragma unroll
-        for (int w = 0; w < SPLIT; ++w) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) out[i] += part[w][c * 8 + i];
-        }
-        sq += decode_epilogue(p, tok, t, ec, out, loss_scale);
-      }
-    }
+    walk_list<NV, R>(p, t, b + part, SPLIT, e, lane, off, act, acc);
+    if (TOK > 1 || e > b) put_partial<NV>(sums[warp], acc, lane);
   }
-  if (p.mode == 1) {
-    // one global atomic per CTA: all warps of the CTA work on the same target
-    sq = warp_sum(sq);
-    if (kWarps > 1) {
-      __shared__ float red_s[kWarps];
-      if (lane == 0) red_s[warp] = sq;
-      __syncthreads();
-      sq = 0.f;
-      for (int w = 0; w < kWarps; ++w) sq += red_s[w];
+  const bool empty = TOK == 1 && e == b;  // nothing was gathered: no sums to wait for
+  if (!empty) __syncthreads();
+  float sq = 0.f;
+  for (int c = threadIdx.x; c < TOK * NV * 32; c += 32 * kWarps) {  // one 8-element slice per thread
+    const int g = TOK > 1 ? c / (NV * 32) : 0, cv = TOK > 1 ? c % (NV * 32) : c;
+    const int ec = (int(blockIdx.z) * NV * 32 + cv) * 8, slot_c = int(blockIdx.x) * TOK + g;
+    if (ec >= d || slot_c >= p.B) continue;
+    float out[8];
+    if (empty) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) out[i] = 0.f;
+    } else {
+      sum_partials<NV, SPLIT>(&sums[g * SPLIT], cv, out);
     }
-    if (threadIdx.x == 0 && sq != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[t], double(sq));
+    sq += decode_epilogue(p, decode_token(p, slot_c), t, ec, out, loss_scale);
+  }
+  if (p.mode == 1 && p.sq_err != nullptr) {
+    // one global atomic per CTA: all warps of the CTA work on the same target
+    __shared__ float red_s[kWarps];
+    sq = warp_sum(sq);
+    if (lane == 0) red_s[warp] = sq;
+    __syncthreads();
+    sq = 0.f;
+    for (int w = 0; w < kWarps; ++w) sq += red_s[w];
+    if (threadIdx.x == 0 && sq != 0.f) atomicAdd(&p.sq_err[t], double(sq));
   }
 }
 
 // Per-source tied decoders without affine terms: the row of feature (s, f) serves every target t >= s with the same weight,
-// so the reconstruction of target t is the one of t - 1 plus the entries of layer t.  One warp per (token, column chunk)
-// reads every row once and finishes a target whenever a layer's entries are in.  The list is scanned once per layer
-// (coalesced, a few hundred bytes), so the entries of a token may come in any order (within a layer they are added in the
-// order of the list: bit for bit the same sums take a sorted list).  One warp per CTA, as in the walk: tied Pythia-70m shape, 4096
-// tokens, k = 200: 571 us with eight, 518 with one.
-template <int NV>
-__global__ void __launch_bounds__(32, NV >= 2 ? 16 : 24) decode_running_kernel(const DecodeParams p) {
-  const int lane = threadIdx.x & 31;
+// so the reconstruction of target t is the one of t - 1 plus the entries of layer t.  The SPLIT warps of a CTA read every row of a
+// (token, column chunk) once and finish a target whenever a layer's entries are in: their running sums meet in shared memory at every target.
+// A warp holds 32 of its entries at a time and moves on when a layer has used them up, which takes a list whose layers ascend; any other
+// list (the entries of a token may come in any order) is scanned once per layer.
+template <int NV, int SPLIT, int R, int WARPS_PER_SM>
+__global__ void __launch_bounds__(32 * SPLIT, WARPS_PER_SM / SPLIT) decode_running_kernel(const DecodeParams p) {
+  __shared__ __align__(16) float sums[2][SPLIT][NV * 256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.d;
   const float loss_scale = p.ctl != nullptr ? p.ctl[SC_LOSS_SCALE] : 1.f;
   const int tok = decode_token(p, int(blockIdx.x));
-  int e0[NV];
+  const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
+  int off[NV];
   bool act[NV];
   float acc[NV][8];
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    e0[v] = ((int(blockIdx.y) * NV + v) * 32 + lane) * 8;
-    act[v] = e0[v] < d;
+    off[v] = ((int(blockIdx.y) * NV + v) * 32 + lane) * 8;
+    act[v] = off[v] < d;
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[v][i] = 0.f;
   }
-  const int b = __ldg(p.tok_off + tok), e = __ldg(p.tok_off + tok + 1);
-  float sq_t = 0.f;  // lane t: the sum of target t (at most 32 layers), one addition per CTA and target at the end
+  bool in_order = true;
+  for (int i = b + 1 + int(threadIdx.x); i < e; i += 32 * SPLIT) in_order &= (__ldg(p.tcsr_col + i) >> 24) >= (__ldg(p.tcsr_col + i - 1) >> 24);
+  const bool ascending = __syncthreads_and(in_order);
+  float sq_t = 0.f;  // lane t: this warp's share of the sum of target t (at most 32 layers), one addition per CTA and target at the end
+  int base = b + warp;  // position of lane 0's entry
+  int col = 0;
+  float a = 0.f;
+  const auto fetch = [&]() {
+    const int i = base + lane * SPLIT;
+    col = i < e ? __ldg(p.tcsr_col + i) : 0;
+    a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
+    if (a != 0.f && (!clt_in_bounds(col >> 24, p.L, p.dbg_status, 103) || !clt_in_bounds(col & 0xFFFFFF, p.col_pitch, p.dbg_status, 104))) a = 0.f;
+  };
+  fetch();
+#pragma unroll 1
   for (int t = 0; t < p.L; ++t) {
-    for (int i0 = b; i0 < e; i0 += 32) {
-      const int i = i0 + lane;
-      const int col = i < e ? __ldg(p.tcsr_col + i) : 0;
-      const float a = i < e ? __ldg(p.tcsr_val + i) : 0.f;
-      const int f = col & 0xFFFFFF;
-      bool use = a != 0.f;
-      if (use && (!clt_in_bounds(col >> 24, p.L, p.dbg_status, 103) || !clt_in_bounds(f, p.col_pitch, p.dbg_status, 104))) use = false;
-      use = use && (col >> 24) == t;
-      const uint32_t mask = __ballot_sync(0xFFFFFFFFu, use);
-      if (mask != 0u) gather_rows<NV, 4>(mask, a, p.w[t] + 1LL * f * d, e0, act, acc);
+    if (!ascending) {
+      base = b + warp;
+      fetch();
     }
+    for (;;) {
+      const uint32_t mask = __ballot_sync(0xFFFFFFFFu, a != 0.f && (col >> 24) == t);
+      if (mask != 0u) gather_rows<NV, R>(mask, a, p.w[t] + 1LL * (col & 0xFFFFFF) * d, off, act, acc);
+      if (base + 32 * SPLIT >= e) break;                                               // no entries behind these
+      if (ascending && (__shfl_sync(0xFFFFFFFFu, col, 31) >> 24) > t) break;           // the last of these is a later layer's
+      base += 32 * SPLIT;
+      fetch();
+    }
+    // two buffers in turn: a warp that is already at the next target writes the other one, and it cannot be two targets
+    // ahead, because the barrier of the next target needs every warp
+    float(*buf)[NV * 256] = sums[t & 1];
+    put_partial<NV>(buf[warp], acc, lane);
+    __syncthreads();
     float sq = 0.f;
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      if (act[v]) sq += decode_epilogue(p, tok, t, e0[v], acc[v], loss_scale);
-    if (p.mode == 1) {
-      sq = warp_sum(sq);
-      if (lane == t) sq_t = sq;
+    for (int c = threadIdx.x; c < NV * 32; c += 32 * SPLIT) {
+      const int ec = (int(blockIdx.y) * NV * 32 + c) * 8;
+      if (ec >= d) continue;
+      float out[8];
+      sum_partials<NV, SPLIT>(buf, c, out);
+      sq += decode_epilogue(p, tok, t, ec, out, loss_scale);
     }
+    sq = warp_sum(sq);
+    if (lane == t) sq_t = sq;
   }
-  if (p.mode == 1 && sq_t != 0.f && p.sq_err != nullptr) atomicAdd(&p.sq_err[lane], double(sq_t));
+  if (p.mode == 1 && p.sq_err != nullptr) {
+    __shared__ float red_s[SPLIT][kMaxLayers];
+    red_s[warp][lane] = sq_t;
+    __syncthreads();
+    sq_t = 0.f;
+    if (warp == 0)
+      for (int w = 0; w < SPLIT; ++w) sq_t += red_s[w][lane];
+    if (warp == 0 && sq_t != 0.f) atomicAdd(&p.sq_err[lane], double(sq_t));
+  }
+}
+
+// order[0 .. B): the tokens by the length of their lists, longest first (in classes of four; the order inside a class is open).
+// One CTA: a counting sort of a few thousand lengths, 4 us.
+constexpr int kLenClasses = 1024;
+__global__ void __launch_bounds__(kLenClasses) decode_order_kernel(const int* __restrict__ tok_off, int B, int* __restrict__ order) {
+  __shared__ int place[kLenClasses];
+  __shared__ int warp_sums[32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  place[tid] = 0;
+  __syncthreads();
+  const auto class_of = [&](int i) { return kLenClasses - 1 - min((tok_off[i + 1] - tok_off[i]) >> 2, kLenClasses - 1); };
+  // one addition per class and warp: lists of equal length would otherwise queue up at one counter
+  const auto take = [&](int i, bool valid) {
+    const int c = valid ? class_of(i) : kLenClasses;
+    const uint32_t same = __match_any_sync(0xFFFFFFFFu, c);
+    const int leader = __ffs(same) - 1;
+    int first = 0;
+    if (valid && lane == leader) first = atomicAdd(&place[c], __popc(same));
+    return __shfl_sync(0xFFFFFFFFu, first, leader) + __popc(same & ((1u << lane) - 1u));
+  };
+  const int rounds = (B + kLenClasses - 1) / kLenClasses;
+  for (int r = 0; r < rounds; ++r) take(r * kLenClasses + tid, r * kLenClasses + tid < B);
+  __syncthreads();
+  const int mine = place[tid];
+  int x = mine;  // inclusive prefix sum over the warp, then over the warps
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sums[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    int s = warp_sums[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, s, o);
+      if (lane >= o) s += y;
+    }
+    warp_sums[lane] = s;
+  }
+  __syncthreads();
+  place[tid] = x - mine + (warp > 0 ? warp_sums[warp - 1] : 0);
+  __syncthreads();
+  for (int r = 0; r < rounds; ++r) {
+    const int i = r * kLenClasses + tid;
+    const int at = take(i, i < B);
+    if (i < B) order[at] = i;
+  }
 }
 
 // Epilogue for the tensor-parallel path, run after the partial reconstructions were summed across ranks:
@@ -457,7 +564,27 @@ struct CltDecodeArgs {
   int* status;  // may be null; the index checks of the debug build report here
   float* ctl;   // optional step control block (loss scale in, found-inf flag out)
   int rows_limit;
+  int expected; // entries per token that the caller expects (its k), 0: not known
+  int* order;   // scratch of clt_sparse_decode_scratch(args) ints, null where that is 0
 };
+
+// 16-byte vectors per lane: the whole row up to d_model 1024 (a warp then reads an entry's row in one go), half of it above
+static int walk_chunks(const CltDecodeArgs* a) { return a->d > 1024 ? 2 : 1; }
+// at most two vectors per lane: the sums stay live across the epilogues of all targets
+static int running_chunks(const CltDecodeArgs* a) { return (a->d + 511) / 512; }
+static bool takes_running(const CltDecodeArgs* a) {
+  return a->tying == 1 && a->feat_offset == nullptr && a->feat_scale == nullptr && a->rows_limit <= 0 && 1LL * a->B * running_chunks(a) >= kRunningMinWarps;
+}
+
+static long long walk_ctas(const CltDecodeArgs* a) { return 1LL * a->B * a->L * walk_chunks(a); }
+static bool short_lists(const CltDecodeArgs* a) { return a->expected > 0 && a->expected < kShortBelow; }
+
+// Number of ints the call wants in `order`: the tokens are sorted by length where there are so many CTAs that it pays.
+extern "C" long long CLT_FN(clt_sparse_decode_scratch)(const CltDecodeArgs* a) {
+  if (a->mode == 2 || a->B <= 0 || short_lists(a)) return 0;
+  if (takes_running(a)) return a->B >= kRunningOrderFrom ? a->B : 0;
+  return a->d > 512 && walk_ctas(a) >= kManyCtas ? a->B : 0;
+}
 
 extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st) {
   if (a->d % 8 != 0 || a->L > kMaxLayers || a->d > 2048) return -1;
@@ -473,30 +600,42 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   p.rows_per_rank = a->rows_per_rank; p.rank = a->rank; p.world = a->world;
   p.ctl = a->ctl; p.rows_limit = a->rows_limit; p.dbg_status = a->status;
   if (a->B <= 0 || a->L <= 0) return 0;
-  // 16-byte vectors per lane: the whole row up to d_model 1024 (a warp then reads an entry's row in one go), half of it above
-  const int chunks = a->d > 1024 ? 2 : 1;
-  const int nv = (a->d / 8 + 32 * chunks - 1) / (32 * chunks);
-  const bool plain_tied = a->tying == 1 && a->feat_offset == nullptr && a->feat_scale == nullptr && a->rows_limit <= 0;
-  auto pick = [&](auto k1, auto k2, auto k3, auto k4, bool split) {
-    auto go = [&](auto kern, int warps) { kern<<<dim3(split ? a->B : (a->B + warps - 1) / warps, a->L, chunks), 32 * (split ? kSplitWarps : warps), 0, st>>>(p); };
-    if (nv <= 1) go(k1, walk_warps(1));
-    else if (nv == 2) go(k2, walk_warps(2));
-    else if (nv == 3) go(k3, walk_warps(3));
-    else go(k4, walk_warps(4));
-  };
-  const int run_chunks = (a->d + 511) / 512;  // at most two vectors per lane: the sums stay live across the epilogues of all targets
-  if (plain_tied && 1LL * a->B * run_chunks >= kRunningMinWarps) {
-    const dim3 grid(a->B, run_chunks);
-    if (a->d <= 256) decode_running_kernel<1><<<grid, 32, 0, st>>>(p);
-    else decode_running_kernel<2><<<grid, 32, 0, st>>>(p);
-  } else if (1LL * a->B * a->L * chunks < kSplitBelowWarps) {
-    pick(decode_walk_kernel<1, kSplitWarps>, decode_walk_kernel<2, kSplitWarps>, decode_walk_kernel<3, kSplitWarps>, decode_walk_kernel<4, kSplitWarps>, true);
-  } else if (nv >= 3 && a->B >= kFullMinTokens) {
-    const dim3 grid(a->B, a->L, chunks);
-    if (nv == 3) decode_walk_kernel<3, 1, true><<<grid, 32, 0, st>>>(p);
-    else decode_walk_kernel<4, 1, true><<<grid, 32, 0, st>>>(p);
+  if (a->order != nullptr && CLT_FN(clt_sparse_decode_scratch)(a) > 0) {
+    p.order = a->order;
+    decode_order_kernel<<<1, kLenClasses, 0, st>>>(a->tok_off, a->B, a->order);
   } else {
-    pick(decode_walk_kernel<1, 1>, decode_walk_kernel<2, 1>, decode_walk_kernel<3, 1>, decode_walk_kernel<4, 1>, false);
+    p.order = nullptr;
+  }
+  if (takes_running(a)) {
+    const dim3 grid(a->B, running_chunks(a));
+    if (a->d <= 256) decode_running_kernel<1, 4, 4, 24><<<grid, 128, 0, st>>>(p);
+    else decode_running_kernel<2, 4, 4, 20><<<grid, 128, 0, st>>>(p);
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  }
+  const int chunks = walk_chunks(a);
+  const int nv = (a->d / 8 + 32 * chunks - 1) / (32 * chunks);
+  const long long ctas = walk_ctas(a);
+  const dim3 grid(a->B, a->L, chunks);
+  if (ctas < kEightWarpsBelow) {
+    if (nv <= 1) decode_walk_kernel<1, 1, 8, 4, 32><<<grid, 256, 0, st>>>(p);
+    else if (nv == 2) decode_walk_kernel<2, 1, 8, 4, 24><<<grid, 256, 0, st>>>(p);
+    else if (nv == 3) decode_walk_kernel<3, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
+    else decode_walk_kernel<4, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
+  } else if (nv <= 1) {
+    if (ctas >= kPairNarrowFrom) decode_walk_kernel<1, 2, 2, 4, 40><<<dim3((a->B + 1) / 2, a->L), 128, 0, st>>>(p);
+    else decode_walk_kernel<1, 1, 4, 4, 40><<<grid, 128, 0, st>>>(p);
+  } else if (short_lists(a) && ctas >= kShortFrom) {
+    if (nv == 2) decode_walk_kernel<2, 1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
+    else if (nv == 3) decode_walk_kernel<3, 1, 2, 2, 28><<<grid, 64, 0, st>>>(p);
+    else decode_walk_kernel<4, 1, 2, 2, 20><<<grid, 64, 0, st>>>(p);
+  } else if (nv == 2) {
+    decode_walk_kernel<2, 1, 4, 4, 24><<<grid, 128, 0, st>>>(p);
+  } else if (ctas >= kManyCtas) {
+    if (nv == 3) decode_walk_kernel<3, 1, 4, 2, 28><<<grid, 128, 0, st>>>(p);
+    else decode_walk_kernel<4, 1, 4, 2, 20><<<grid, 128, 0, st>>>(p);
+  } else {
+    if (nv == 3) decode_walk_kernel<3, 1, 4, 4, 20><<<grid, 128, 0, st>>>(p);
+    else decode_walk_kernel<4, 1, 4, 4, 16><<<grid, 128, 0, st>>>(p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

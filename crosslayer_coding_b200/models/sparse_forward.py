@@ -74,6 +74,7 @@ class SparseForward:
         else:
             cap = int(min(B * L * Fl, max_active_per_token * B))
         self.cap = cap
+        self.expected_entries = self.k_total // max(B, 1) if self.fn in ("batchtopk", "topk") else 0  # per token; a threshold leaves it open
         self.preact = torch.empty(L, B, Fl, dtype=torch.bfloat16, device=dev)
         self.ctl = torch.zeros(16, dtype=torch.int64, device=dev)
         self.status = torch.zeros(4, dtype=i32, device=dev)
@@ -180,7 +181,8 @@ class SparseForward:
         sg = sigma.to(device=self.dev, dtype=torch.float32).reshape(self.L, self.d).contiguous() if sigma is not None else None
         gs, sq_err = (self.gs, self.sq_err) if Y is not None else (None, None)  # no targets: the reconstruction is the only output
         e.sparse_decode([w.data for w in m.dec_weight], self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col,
-                        self.tcsr_val, off, scale, None, self.bias_sum, None, Y, sg, gs, yhat, sq_err, 1, [], 0, 0, self.status)
+                        self.tcsr_val, off, scale, None, self.bias_sum, None, Y, sg, gs, yhat, sq_err, 1, [], 0, 0, self.status,
+                        expected_entries=self.expected_entries)
         return yhat
 
     def forward_dict(self, inputs: Dict[int, torch.Tensor]) -> Dict[int, torch.Tensor]:

@@ -232,6 +232,8 @@ class FusedBatchTopKEngine:
             # ``fused_max_active_per_token`` entries per token and a step that needs more reports it
             per_tok = int(getattr(training_config, "fused_max_active_per_token", 1024) or 1024) if training_config is not None else 1024
             self.k_total = int(min(B * L * max(self.Fv, 1), per_tok * B))
+        # entries per token of this rank, for the decode's choice of warps per token; a threshold leaves it open
+        self.expected_entries = max(1, self.k_total // (B * self.world)) if self.fn in ("batchtopk", "topk") else 0
         self.key_lo, self.shift = histogram_range(self.k_total, B * L * self.F) if self.fn == "batchtopk" else (0, 19)
         self.preact = torch.empty(L, B, Fl, dtype=self.t16, device=dev)
         self.mean = torch.empty(L, Fl, dtype=f32, device=dev)
@@ -568,7 +570,7 @@ class FusedBatchTopKEngine:
         if self.world == 1:
             e.sparse_decode(dec_w, self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col, self.tcsr_val,
                             self.foff32, self.fsc32, None, bias_sum, addend, Y, self.sigma, self.gs, yhat, self.sq_err, 1, [], 0, 0, self.status,
-                            self.step_ctl)
+                            self.step_ctl, expected_entries=self.expected_entries)
             self.kernel_launches += 1
         else:
             sy = self.symm
@@ -576,7 +578,8 @@ class FusedBatchTopKEngine:
                 yhat.zero_()
             # 1. decode, pushing every token's partial sums into its owner's staging slot (peer stores)
             e.sparse_decode(dec_w, self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col, self.tcsr_val,
-                            self.foff32, self.fsc32, None, None, None, None, None, None, None, None, 2, sy.stage_ptrs, sy.rows_per_rank, self.rank, self.status)
+                            self.foff32, self.fsc32, None, None, None, None, None, None, None, None, 2, sy.stage_ptrs, sy.rows_per_rank, self.rank, self.status,
+                            expected_entries=self.expected_entries)
             sy.barrier(e, self.status)
             # 2. owners reduce their rows, finish their part of the loss and push the gradient seed to every rank; the
             #    exchange inside the step-control kernel that follows is the barrier behind these pushes

@@ -56,11 +56,10 @@ def _dense_decode(L, B, d, F, tying, tok, col, val, W, off, sc, rows_limit=0):
     return want
 
 
-def _check_decode(ext, L, B, d, tying, affine, dtype=torch.bfloat16, addend=False, rows_limit=0):
+def _check_decode(ext, L, B, d, tying, affine, dtype=torch.bfloat16, addend=False, rows_limit=0, F=24, entries=None, expected=0):
     dev = _dev()
     g = torch.Generator().manual_seed(L * 1000 + B + d)
-    F = 24
-    tok, col, val = _entries(g, L, B, F, min(B * L * F, 7 * B), dev)
+    tok, col, val = (entries or _entries)(g, L, B, F, min(B * L * F, 7 * B), dev)
     rows = [L - s if tying == 0 else 1 for s in range(L)]
     W = [(torch.randn(F, r, d, generator=g) / 4).to(dtype).to(dev) for r in rows]
     off = torch.randn(L, F, generator=g).to(dev) if affine else None
@@ -78,7 +77,7 @@ def _check_decode(ext, L, B, d, tying, affine, dtype=torch.bfloat16, addend=Fals
 
         def decode(mode, partial=None, bias=None, addend=None, target=None, sigma=None, gs=None, yhat=None, sq=None, peers=(), rows_per_rank=0, rank=0):
             ext.sparse_decode(W, L, B, d, F, tying, c["tok_off"], c["tcsr_col"], c["tcsr_val"], off, sc, partial, bias, addend, target, sigma, gs, yhat, sq, mode,
-                              list(peers), rows_per_rank, rank, status, None, rows_limit)
+                              list(peers), rows_per_rank, rank, status, None, rows_limit, expected)
 
         yhat = torch.full((L, B, d), float("nan"), device=dev)
         gs = torch.empty(L, B, d, device=dev, dtype=dtype)
@@ -129,6 +128,36 @@ def test_gather_decode_matches_dense(ext, L, B, d, tying, affine):
 @pytest.mark.parametrize("opts", [dict(dtype=torch.float16), dict(addend=True), dict(rows_limit=1), dict(rows_limit=2, dtype=torch.float16, addend=True)])
 def test_gather_decode_options(ext, L, B, d, tying, opts):
     _check_decode(ext, L, B, d, tying, False, **opts)
+
+
+def _uneven_entries(g, L, B, F, n, dev):
+    """Lists of very different length: every 64th token has up to 600 entries, most have a few, every fifth none."""
+    tok, flat = [], []
+    for b in range(B):
+        k = 0 if b % 5 == 4 else (600 if b % 64 == 0 else (130 if b % 64 == 1 else b % 4))
+        pick = torch.randperm(L * F, generator=g)[:k]
+        tok.append(torch.full((pick.numel(),), b))
+        flat.append(pick)
+    tok, flat = torch.cat(tok), torch.cat(flat)
+    mix = torch.randperm(tok.numel(), generator=g)
+    return tok[mix].to(I32).to(dev), flat[mix].to(I32).to(dev), torch.randn(tok.numel(), generator=g).to(dev)
+
+
+# lists of several batches per warp next to empty ones, on both sides of every line of the dispatch: eight warps per token, four, two tokens
+# of narrow rows per CTA, two rows per step with the tokens by length (also with two column chunks), the running sum with and without
+# that order
+@pytest.mark.parametrize("tying", [0, 1, 2])
+@pytest.mark.parametrize("L,B,d", [(3, 70, 264), (3, 70, 1032), (4, 1030, 136), (13, 1900, 136), (4, 1030, 512), (14, 2049, 520), (4, 4097, 512), (7, 2050, 1800)])
+def test_gather_decode_of_uneven_lists(ext, L, B, d, tying):
+    _check_decode(ext, L, B, d, tying, False, F=72, entries=_uneven_entries)
+
+
+# two warps per token, which callers with a small k ask for (and get for many (token, target) pairs): the sums do not depend on how
+# true the expectation is
+@pytest.mark.parametrize("tying", [0, 1, 2])
+@pytest.mark.parametrize("L,B,d", [(13, 1303, 512), (13, 1303, 520), (9, 1001, 1800), (3, 70, 520)])
+def test_gather_decode_with_an_expected_length(ext, L, B, d, tying):
+    _check_decode(ext, L, B, d, tying, tying != 0, F=72, entries=_uneven_entries, expected=20)
 
 
 def test_decode_refuses_loss_outputs_without_a_target(ext):
