@@ -801,6 +801,266 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
   if (tid == 0 && sh->abort_flag && status != nullptr) atomicCAS(status, STATUS_OK, STATUS_WAIT_TIMEOUT);
 }
 
+// ------------------------------------------------------------------ row update, one warp per row
+// Rows of up to 512 elements (16-bit weights, fp32 moments): the row is one warp's alone, NC blocks of 128 elements, four per lane.  A
+// warp has its own ring of kNarrowStages rows in shared memory, filled and drained by bulk copies that its first lane issues, and gathers the
+// seed (input) rows of the row's entries itself, kNarrowBatch at a time; offsets are requested two rows ahead, the first 32 entries one row
+// ahead, the first batch of seed rows before the row itself is waited for.
+// Against the row pipeline above (a CTA per row): that one has five or six rows per SM at its consumers, each of which waits
+// for the lists and seed rows beyond the four staged ones, twice per row and one row after the other; here twenty rows per SM do so at the
+// same time, and the dot products of a row (dL/da) and its norm need no sum across warps.
+template <int NC>
+__device__ __forceinline__ void load_seed_row(const t16* row, int lane, int d, uint2 (&q)[NC]) {
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int e = c * 128 + lane * 4;
+    if (e < d) q[c] = __ldg(reinterpret_cast<const uint2*>(row + e));
+  }
+}
+
+constexpr int kNarrowStages = 2;
+constexpr int kNarrowWarps = 4;
+constexpr int kNarrowBatch = 4;
+
+// Resident CTAs per SM: 128 registers for rows above 256, 96 for 129 to 256, 80 below.  Five CTAs of 96 registers spill at 512 (1069 us
+// against 925 for both sweeps of the tied Pythia-70m shape), and three stages with 14 warps are slower than two with 16 (1063).
+__host__ __device__ constexpr int narrow_ctas(int nc) { return nc >= 3 ? 4 : (nc == 2 ? 5 : 6); }
+
+struct RowAt {
+  long long idx;  // position in the list of all rows
+  int ti, f, r;
+};
+
+template <bool SR, int NC, bool PT>
+__global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_rows_adam_kernel(const DecAdamParams p, long long total_rows, int* status) {
+  extern __shared__ __align__(128) uint8_t smem_narrow[];
+  __shared__ uint64_t full_s[kNarrowWarps][kNarrowStages];
+  __shared__ int abort_s;
+  const StepScales sc = read_step_ctl(p.ctl);
+  if (sc.skip) return;  // the whole grid sees the same flag: a skipped step touches nothing
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int d = p.d, Fp = p.F_pitch;
+  const uint32_t w_bytes = uint32_t(d) * 2u, mv_bytes = uint32_t(d) * 4u, stage_bytes = w_bytes + 2u * mv_bytes;
+  uint8_t* ring = smem_narrow + size_t(warp) * kNarrowStages * stage_bytes;
+  uint64_t* full = full_s[warp];
+  if (threadIdx.x == 0) abort_s = 0;
+  if (lane == 0) {
+    for (int s = 0; s < kNarrowStages; ++s) mbar_init(&full[s], 1);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  volatile int* abort_flag = &abort_s;
+  const HyperRegs hr = make_regs(p.h);
+  const float gsc = hr.gscale * (p.use_inv_scale ? sc.inv_scale : 1.f);
+  const uint64_t pol_stream = l2_policy_evict_first();  // rows are touched once per step
+
+  const long long stride = 1LL * gridDim.x * kNarrowWarps;
+  const auto place = [&](RowAt& at) {  // tensor, feature and row of at.idx (at.ti: at or before the right one)
+    if (at.idx >= total_rows) return;
+    while (at.idx >= p.row_start[at.ti + 1]) ++at.ti;
+    const long long rem = at.idx - p.row_start[at.ti];
+    const int R = p.rows[at.ti];
+    at.f = R == 1 ? int(rem) : int(rem / R);
+    at.r = R == 1 ? 0 : int(rem - 1LL * at.f * R);
+  };
+  const auto elem_of = [&](const RowAt& at) { return (at.idx - p.row_start[at.ti]) * d; };
+  // entries: PT: lane s holds the segment of source layer s <= ti; else all lanes hold the feature's one segment
+  const auto load_offsets = [&](const RowAt& at, int& b, int& n) {
+    b = n = 0;
+    if (at.idx >= total_rows) return;
+    if (PT ? lane <= at.ti : true) {
+      const int* o = p.feat_off + (PT ? lane : at.ti) * Fp + at.f;
+      b = __ldg(o);
+      n = __ldg(o + 1) - b;
+    }
+  };
+  // entry j0 + lane of the row: its place in the CSR arrays, token and activation; returns the number of entries
+  const auto load_list = [&](const RowAt& at, int b, int n, int j0, int& x, int& tok, float& a) -> int {
+    const int j = j0 + lane;
+    int total = n;
+    if (PT) {
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+      int seg = 0;
+      if (total > 0)
+        for (int s = 0; s < at.ti; ++s) seg += __shfl_sync(0xFFFFFFFFu, incl, s) <= j ? 1 : 0;
+      x = __shfl_sync(0xFFFFFFFFu, b, seg) + j - (__shfl_sync(0xFFFFFFFFu, incl, seg) - __shfl_sync(0xFFFFFFFFu, n, seg));
+    } else {
+      x = b + j;
+    }
+    tok = j < total ? __ldg(p.fcsr_tok + x) : 0;
+    a = j < total ? __ldg(p.fcsr_val + x) : 0.f;
+    if (!clt_in_bounds(tok, p.B, status, 202)) { tok = 0; a = 0.f; }
+    return total;
+  };
+  const auto issue_row = [&](const RowAt& at, int st) {
+    if (lane != 0 || at.idx >= total_rows) return;
+    uint8_t* stage = ring + size_t(st) * stage_bytes;
+    const long long eo = elem_of(at);
+    mbar_expect_tx(&full[st], stage_bytes);
+    bulk_load_1d_hint(stage, static_cast<const t16*>(p.w[at.ti]) + eo, w_bytes, &full[st], pol_stream);
+    bulk_load_1d_hint(stage + w_bytes, p.m[at.ti] + eo, mv_bytes, &full[st], pol_stream);
+    bulk_load_1d_hint(stage + w_bytes + mv_bytes, p.v[at.ti] + eo, mv_bytes, &full[st], pol_stream);
+  };
+
+  RowAt cur{1LL * blockIdx.x * kNarrowWarps + warp, 0, 0, 0};
+  place(cur);
+  RowAt nxt{cur.idx + stride, cur.ti, 0, 0};
+  place(nxt);
+  for (int k = 0; k < kNarrowStages; ++k) {
+    RowAt at{cur.idx + k * stride, cur.ti, 0, 0};
+    place(at);
+    issue_row(at, k);
+  }
+  int b = 0, n = 0, b1 = 0, n1 = 0;  // offsets of the current and the next row
+  load_offsets(cur, b, n);
+  load_offsets(nxt, b1, n1);
+  int x, tok;
+  float a;
+  int total = load_list(cur, b, n, 0, x, tok, a);
+  bool ok = true;
+  uint32_t i = 0;
+  for (; cur.idx < total_rows; ++i) {
+    const int st = int(i % kNarrowStages);
+    RowAt nn{nxt.idx + stride, nxt.ti, 0, 0};
+    place(nn);
+    int b2, n2;
+    load_offsets(nn, b2, n2);
+    const t16* gs_t = p.gs + 1LL * (cur.ti + cur.r) * p.B * d;
+    uint2 q[kNarrowBatch][NC];
+#pragma unroll
+    for (int k = 0; k < kNarrowBatch; ++k) {
+      const int tk = __shfl_sync(0xFFFFFFFFu, tok, k);
+      if (k < total) load_seed_row<NC>(gs_t + 1LL * tk * d, lane, d, q[k]);
+    }
+    int x1, tok1;
+    float a1;
+    const int total1 = load_list(nxt, b1, n1, 0, x1, tok1, a1);
+    const int col = cur.ti * Fp + cur.f;
+    float pc = p.pen_coef ? __ldg(p.pen_coef + col) : 0.f;
+    if (PT && p.pen_coef) pc = warp_sum(lane <= cur.ti ? __ldg(p.pen_coef + lane * Fp + cur.f) : 0.f);  // the row is part of the norms of all sources
+    if (!mbar_wait(&full[st], (i / kNarrowStages) & 1, abort_flag)) { ok = false; break; }
+    uint8_t* stage = ring + size_t(st) * stage_bytes;
+    t16* w_s = reinterpret_cast<t16*>(stage);
+    float* m_s = reinterpret_cast<float*>(stage + w_bytes);
+    float* v_s = reinterpret_cast<float*>(stage + w_bytes + mv_bytes);
+    float w[NC][4], g[NC][4];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w[c][k] = g[c][k] = 0.f;
+      if (c * 128 + lane * 4 < d) ldbf<4>(w_s + c * 128 + lane * 4, w[c]);
+    }
+    for (int j0 = 0; j0 < total; j0 += 32) {
+      if (j0 > 0) load_list(cur, b, n, j0, x, tok, a);
+      const int cnt = min(32, total - j0);
+      for (int k0 = 0; k0 < cnt; k0 += kNarrowBatch) {
+        if (j0 + k0 > 0) {
+#pragma unroll
+          for (int k = 0; k < kNarrowBatch; ++k) {
+            const int tk = __shfl_sync(0xFFFFFFFFu, tok, (k0 + k) & 31);
+            if (k0 + k < cnt) load_seed_row<NC>(gs_t + 1LL * tk * d, lane, d, q[k]);
+          }
+        }
+        float dot[kNarrowBatch];
+#pragma unroll
+        for (int k = 0; k < kNarrowBatch; ++k) {
+          const float ak = __shfl_sync(0xFFFFFFFFu, a, (k0 + k) & 31);
+          dot[k] = 0.f;
+          if (k0 + k < cnt) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              if (c * 128 + lane * 4 < d) {
+                const float gv[4] = {t16_lo(q[k][c].x), t16_hi(q[k][c].x), t16_lo(q[k][c].y), t16_hi(q[k][c].y)};
+#pragma unroll
+                for (int z = 0; z < 4; ++z) {
+                  g[c][z] = fmaf(ak, gv[z], g[c][z]);
+                  dot[k] = fmaf(gv[z], w[c][z], dot[k]);
+                }
+              }
+            }
+          }
+        }
+        if (p.grad_a != nullptr) {
+          const float sdot = warp_sum_many<kNarrowBatch>(dot, lane);
+          const int k = k0 + warp_sum_slot<kNarrowBatch>(lane);
+          const int xk = __shfl_sync(0xFFFFFFFFu, x, k & 31);
+          if (lane % (32 / kNarrowBatch) == 0 && k < cnt && sdot != 0.f) atomicAdd(&p.grad_a[xk], sdot * gsc);
+        }
+      }
+    }
+    const float* xrow = cur.r == 0 ? extra_row_ptr(p, col) : nullptr;
+    const long long eo = elem_of(cur);
+    float norm2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int e = c * 128 + lane * 4;
+      if (e < d) {
+        float m[4], v[4], extra[4] = {0.f, 0.f, 0.f, 0.f};
+        ldf<4>(m_s + e, m);
+        ldf<4>(v_s + e, v);
+        if (xrow != nullptr) {
+          const float4 t4 = __ldg(reinterpret_cast<const float4*>(xrow + e));
+          extra[0] = t4.x; extra[1] = t4.y; extra[2] = t4.z; extra[3] = t4.w;
+        }
+#pragma unroll
+        for (int z = 0; z < 4; ++z) {
+          float gq = fmaf(pc, w[c][z], g[c][z] * gsc);
+          if (xrow != nullptr) gq += extra[z];
+          adam1(w[c][z], m[z], v[z], gq * sc.clip, hr);
+          if (!PT) norm2 = fmaf(w[c][z], w[c][z], norm2);
+        }
+        stbf<4, SR>(w_s + e, w[c], p.h.sr_seed, (unsigned int)(unsigned long long)(p.row_start[cur.ti] * d + eo + e));
+        if (PT) {  // norms of the stored (rounded) weights
+          float wr[4];
+          ldbf<4>(w_s + e, wr);
+#pragma unroll
+          for (int z = 0; z < 4; ++z) norm2 = fmaf(wr[z], wr[z], norm2);
+        }
+        stf<4>(m_s + e, m);
+        stf<4>(v_s + e, v);
+      }
+    }
+    if (p.norm2_out != nullptr) {
+      norm2 = warp_sum(norm2);
+      if (lane == 0) atomicAdd(&p.norm2_out[col], norm2);
+    }
+    fence_proxy_async();  // the row written above is read next by the bulk stores (async proxy)
+    __syncwarp();
+    if (lane == 0) {
+      bulk_store_1d_hint(static_cast<t16*>(p.w[cur.ti]) + eo, stage, w_bytes, pol_stream);
+      bulk_store_1d_hint(p.m[cur.ti] + eo, stage + w_bytes, mv_bytes, pol_stream);
+      bulk_store_1d_hint(p.v[cur.ti] + eo, stage + w_bytes + mv_bytes, mv_bytes, pol_stream);
+      bulk_commit();
+      bulk_wait_read<0>();  // the stage is refilled
+    }
+    RowAt far{cur.idx + kNarrowStages * stride, nxt.ti, 0, 0};
+    place(far);
+    issue_row(far, st);
+    cur = nxt; nxt = nn;
+    b = b1; n = n1; b1 = b2; n1 = n2;
+    x = x1; tok = tok1; a = a1; total = total1;
+  }
+  if (lane == 0) {
+    bulk_wait_all();
+    if (!ok) {
+      // rows whose loads were issued but never consumed: give them a bounded chance to land
+      for (uint32_t j = i; j < i + kNarrowStages && cur.idx + (j - i) * stride < total_rows; ++j) {
+        const long long start = clock64();
+        while (!mbar_try_wait(&full[j % kNarrowStages], (j / kNarrowStages) & 1))
+          if (clock64() - start > kWaitTimeoutCycles) break;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && abort_s && status != nullptr) atomicCAS(status, STATUS_OK, STATUS_WAIT_TIMEOUT);
+}
+
 // Tied decoders (per_source / per_target): same structure without the register-resident entries.
 // Work item = (feature of one decoder tensor, 256-element segment): one warp, 8 elements per lane, walking
 // the feature's R rows with the next row's (w, m, v) already in flight while the current row is updated.
@@ -1252,6 +1512,34 @@ static bool bulk_rows_adam_fits(int d, int weights_bf16) {
   size_t smem;
   return bulk_rows_adam_geometry(d, weights_bf16 != 0, false, &ept, &gthreads, &stage_bytes, &smem) != 0;
 }
+// Rows of up to 512 elements, one warp per row.
+constexpr int kNarrowMaxWidth = 512;
+static int launch_narrow_rows(const DecAdamParams& p, bool sr, int num_sms, int* status, cudaStream_t st, bool per_target) {
+  const long long total = p.row_start[p.ntensors];
+  const size_t smem = size_t(kNarrowWarps) * kNarrowStages * p.d * 10;
+  auto launch = [&](auto kern) -> int {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kNarrowWarps, smem) != cudaSuccess || per_sm < 1) return -4;
+    long long grid = 1LL * num_sms * per_sm;
+    const long long ctas = (total + kNarrowWarps - 1) / kNarrowWarps;
+    if (grid > ctas) grid = ctas;
+    kern<<<int(grid), 32 * kNarrowWarps, smem, st>>>(p, total, status);
+    return 0;
+  };
+  auto pick = [&](auto srv, auto ptv) -> int {
+    constexpr bool S = decltype(srv)::value, T = decltype(ptv)::value;
+    if (p.d <= 128) return launch(narrow_rows_adam_kernel<S, 1, T>);
+    if (p.d <= 256) return launch(narrow_rows_adam_kernel<S, 2, T>);
+    if (p.d <= 384) return launch(narrow_rows_adam_kernel<S, 3, T>);
+    return launch(narrow_rows_adam_kernel<S, 4, T>);
+  };
+  using yes = std::true_type;
+  using no = std::false_type;
+  if (per_target) return sr ? pick(yes{}, yes{}) : pick(no{}, yes{});
+  return sr ? pick(yes{}, no{}) : pick(no{}, no{});
+}
+
 // n_entries: length of the entry list (an upper bound where the number of active entries is not known to the host).
 static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool sr, int num_sms, int* status, cudaStream_t st, long long n_entries,
                                  bool per_target = false) {
@@ -1263,6 +1551,13 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
   if (!bulk_rows_adam_geometry(p.d, weights_bf16, mb, &ept, &gthreads, &stage_bytes, &smem, &nstages)) return -1;
   bool single_rows = true;
   for (int i = 0; i < p.ntensors; ++i) single_rows = single_rows && p.rows[i] == 1;
+  // One warp per row up to 512 elements.  Both sweeps of a step, row pipeline -> one warp per row, us: tied Pythia-70m shape (one row of 512,
+  // eight entries per feature) 1557 -> 925; per-target 6 x 16384 rows of 512, nine entries per row 565 -> 284, of 256 (12 per row, general
+  // sweep) 484 -> 231; untied 6 x 12288 features of 512, 3.5 entries 760 -> 590, of 384 608 -> 501, 8 x 12288 of 256 774 -> 597, 8 x 16384 of
+  // 128, six entries 1451 -> 777, one entry in sixteen 694 -> 472.  Where almost no feature has an entry, wide rows are a plain stream and
+  // the deeper ring of the pipeline is ahead by 2 to 3 % (one entry in nine, rows of 512: 569 against 586; one in eight, tied: 348, 353).
+  const bool idle_lists = !per_target && p.d > 384 && 2 * n_entries < 1LL * p.F_pitch * p.L;
+  if (weights_bf16 && !mb && p.d <= kNarrowMaxWidth && !idle_lists) return launch_narrow_rows(p, sr, num_sms, status, st, per_target);
   auto launch = [&](auto kern) -> int {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
     // resident CTAs per SM from the runtime (shared memory, threads and registers together): a grid beyond them would run a
@@ -1394,14 +1689,11 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   if (a->tying == 0 && a->status != nullptr && bulk_rows_adam_fits(a->d, a->weights_bf16) && acc * a->d < (1LL << 62)) {
     const int rc = launch_rows_adam_bulk(p, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st, a->n_entries);
     if (rc != 0) return rc;
-  } else if (a->tying == 2 && a->status != nullptr && a->weights_bf16 && a->L <= 32 && a->ntensors == a->L && single_rows && a->d > 256 &&
+  } else if (a->tying == 2 && a->status != nullptr && a->weights_bf16 && a->L <= 32 && a->ntensors == a->L && single_rows &&
              a->feat_offset == nullptr && a->feat_scale == nullptr && a->d_feat_offset == nullptr && a->d_feat_scale == nullptr &&
              bulk_rows_adam_fits(a->d, a->weights_bf16)) {
-    // Per-target tied rows without affine terms and without gradients of such terms (which the row pipeline does not form): the row
-    // pipeline too, its consumers gather the entries.  Up to d = 256 a row is one warp of the general sweep, which keeps several dozen
-    // rows per SM in flight against six here and waits for three dependent loads (offsets, token, seed row) in all of them at once: d =
-    // 256, 8 x 10000 rows, one entry in four features 148 us there against 188 here; d = 264, two warps a row there: 262 against 203.
-    // With 90 entries in a few features 94 against 53 us (8 x 1128 rows, d = 256) and 105 against 55 (d = 264).
+    // Per-target tied rows without affine terms and without gradients of such terms, which neither form of the row update forms: one
+    // warp per row up to 512 elements, the row pipeline above, whose consumers gather the entries.
     const int rc = launch_rows_adam_bulk(p, true, a->h.sr_seed != 0, num_sms, a->status, st, a->n_entries, true);
     if (rc != 0) return rc;
   } else if (a->tying == 0) {
