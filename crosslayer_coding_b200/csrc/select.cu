@@ -249,7 +249,8 @@ struct Pool {
   unsigned int* count;  // zeroed by the caller together with the histograms
 };
 constexpr int kPoolStage = 512;   // histogram + queue + staging stay inside the 48 KB of static shared memory
-constexpr int kHitQueue = 1024;   // 16-byte groups per CTA that passed the coarse filter
+constexpr int kHitQueue = 1024;   // 16-byte groups per CTA that passed the coarse filter (threshold scan: four times that)
+constexpr int kCollectQueue = 2 * kHitQueue;  // in the histogram scan, whose tile (64 rows, 256 threads) takes 16 bits to number
 constexpr int kHistExtra = 32;    // words after the two histograms: [0] = pool counter
 
 // Phase A streams the matrix with a coarse filter in the input's own format (one packed compare per two
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(256) zhist_collect_kernel(const t16* __restric
   const int shift = int(sel_state[1]);
   const float z_lo = key_to_float(key_lo);
   __shared__ unsigned int sh[kHistBins];
-  __shared__ uint32_t s_queue[kHitQueue];
+  __shared__ uint16_t s_queue[kCollectQueue];
   __shared__ uint32_t s_key[kPoolStage];
   __shared__ int s_tok[kPoolStage];
   __shared__ int s_col[kPoolStage];
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(256) zhist_collect_kernel(const t16* __restric
                              t16x2_ge_mask(v[k].z, thr2[2]) | t16x2_ge_mask(v[k].w, thr2[3]);
         if (hit != 0 && rb + k < r1) {
           const int slot = atomicAdd(&s_q, 1);
-          if (slot < kHitQueue) s_queue[slot] = (uint32_t(rb + k - r0) << 8) | threadIdx.x;
+          if (slot < kCollectQueue) s_queue[slot] = uint16_t((uint32_t(rb + k - r0) << 8) | threadIdx.x);
         }
       }
     }
@@ -317,8 +318,8 @@ __global__ void __launch_bounds__(256) zhist_collect_kernel(const t16* __restric
   __syncthreads();
   // ---- phase B: exact test, histogram and pool staging, one element per thread
   const int nq_all = s_q;
-  if (nq_all > kHitQueue && threadIdx.x == 0) atomicOr(pool.count, 0x80000000u);  // lost groups: force the full-range pass
-  const int nq = min(nq_all, kHitQueue);
+  if (nq_all > kCollectQueue && threadIdx.x == 0) atomicOr(pool.count, 0x80000000u);  // lost groups: force the full-range pass
+  const int nq = nq_all > kCollectQueue ? 0 : nq_all;  // lost groups: nothing of this pass will be used
   for (int e = threadIdx.x; e < nq * 8; e += blockDim.x) {
     const uint32_t item = s_queue[e >> 3];
     const int r = r0 + int(item >> 8);

@@ -91,7 +91,7 @@ class SparseForward:
             cand_cap = int(min(B * L * Fl, max(1 << 20, 4 * self.k_total)))
             self.cand = [torch.empty(cand_cap, dtype=i32, device=dev) for _ in range(3)] + [torch.empty(cand_cap, dtype=f32, device=dev)]
             self.sel_state = torch.tensor([self.key_lo, self.shift], dtype=torch.int64, device=dev) if self.key_lo != 0 else None
-            self.pool = torch.empty(4, int(min(B * L * Fl, 3 * self.k_total + (1 << 16))), dtype=i32, device=dev) if self.key_lo != 0 else None
+            self.pool = torch.empty(4, int(min(B * L * Fl, 10 * self.k_total + (1 << 16))), dtype=i32, device=dev) if self.key_lo != 0 else None
         ncols = self.ncols = L * Fl
         # counters of the CSR build and loss sums in one buffer, cleared by one memset right in front of the build: cleared at the
         # start of the call they have left L2 by then (the encoder's weights and the pre-activations passed through it), and the

@@ -242,7 +242,7 @@ class FusedBatchTopKEngine:
         # tracked histogram range {key_lo, shift} and the pool filled by the single pass over the pre-activations
         self.sel_state = torch.tensor([self.key_lo, self.shift], dtype=torch.int64, device=dev) if self.key_lo != 0 else None
         k_local = -(-self.k_total // max(1, self.world))
-        self.pool = torch.empty(4, int(min(B * L * max(Fl, 1), 3 * k_local + (1 << 16))), dtype=i32, device=dev) if self.key_lo != 0 else None
+        self.pool = torch.empty(4, int(min(B * L * max(Fl, 1), 10 * k_local + (1 << 16))), dtype=i32, device=dev) if self.key_lo != 0 else None
         self.ctl = torch.zeros(16, dtype=torch.int64, device=dev)
         self.status = torch.zeros(4, dtype=i32, device=dev)
         cap = max(self.k_total, 8)
