@@ -80,6 +80,7 @@ struct CltDecodeArgs {
   float* ctl;
   int rows_limit;
   int expected;
+  int equal;
   int* order;
 };
 struct CltPeerTable {
@@ -466,7 +467,7 @@ void sparse_decode(const std::vector<Tensor>& dec_w, int64_t L, int64_t B, int64
                    const OptTensor& yhat_partial, const OptTensor& bias_sum, const OptTensor& addend, const OptTensor& target,
                    const OptTensor& sigma, const OptTensor& gs, const OptTensor& yhat_out, const OptTensor& sq_err, int64_t mode,
                    const std::vector<int64_t>& stage_peers, int64_t rows_per_rank, int64_t rank, const OptTensor& status,
-                   const OptTensor& ctl, int64_t rows_limit, int64_t expected_entries) {
+                   const OptTensor& ctl, int64_t rows_limit, int64_t expected_entries, bool equal_lists) {
   TORCH_CHECK(dec_w.size() >= 1 && dec_w.size() <= 32, "1..32 decoder tensors");
   const bool half = is_half(dec_w[0], "dec_w");
   const auto ty = t16_of(half);
@@ -490,6 +491,7 @@ void sparse_decode(const std::vector<Tensor>& dec_w, int64_t L, int64_t B, int64
   a.ctl = ctl_ptr(ctl);
   a.rows_limit = int(rows_limit);
   a.expected = int(std::clamp<int64_t>(expected_entries, 0, 1 << 30));
+  a.equal = equal_lists ? 1 : 0;
   if (mode == 2) {
     TORCH_CHECK(stage_peers.size() >= 1 && stage_peers.size() <= 8 && rows_per_rank > 0, "mode 2 needs the peers' staging pointers");
     for (size_t i = 0; i < stage_peers.size(); ++i) a.stage_peers[i] = reinterpret_cast<void*>(stage_peers[i]);
@@ -995,7 +997,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("tok_off"), py::arg("tcsr_col"), py::arg("tcsr_val"), py::arg("feat_offset"), py::arg("feat_scale"), py::arg("yhat_partial"),
         py::arg("bias_sum"), py::arg("addend"), py::arg("target"), py::arg("sigma"), py::arg("gs"), py::arg("yhat_out"), py::arg("sq_err"),
         py::arg("mode"), py::arg("stage_peers"), py::arg("rows_per_rank"), py::arg("rank"), py::arg("status"), py::arg("ctl") = none,
-        py::arg("rows_limit") = 0, py::arg("expected_entries") = 0);
+        py::arg("rows_limit") = 0, py::arg("expected_entries") = 0, py::arg("equal_lists") = false);
   m.def("recon_epilogue", &recon_epilogue, py::arg("yhat_sum"), py::arg("bias_sum"), py::arg("addend"), py::arg("target"), py::arg("sigma"),
         py::arg("gs"), py::arg("yhat_out"), py::arg("sq_err"), py::arg("row0"), py::arg("nrows"), py::arg("ctl") = none);
   m.def("gs_colsum", &gs_colsum);

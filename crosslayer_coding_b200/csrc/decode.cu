@@ -130,9 +130,8 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // per token leaves the chip to the longest lists of every target, and warps that start together drift apart in the feature order, so that
 // L2 serves less.  Four warps per token: GPT-2 shape, 4096 tokens, BatchTopK k = 200, 1435 us with one warp and 1081 with four (8.2 GB of
 // rows at 7.6 TB/s, of which DRAM gives about 6); 512 tokens, k = 32: 124 and 62; 1000 tokens of 16 x 2048, 242 entries: 1138 and 963; 4096
-// tokens of 6 x 512, per-target tied, k = 64: 172 and 132.  Equally long lists lose nothing: 2048 tokens, top-k of 64, 117 and 122; 776
-// tokens of 24 entries 21 and 25.  Eight warps pay where there are too few CTAs to fill the chip (16 tokens 36 us with four, 22
-// with eight; 128 tokens of 200 entries 72 and 67; 256: 102 and 109).
+// tokens of 6 x 512, per-target tied, k = 64: 172 and 132.  Eight warps pay where there are too few CTAs to fill the chip
+// (16 tokens 36 us with four, 22 with eight; 128 tokens of 200 entries 72 and 67; 256: 102 and 109).
 // Rows in flight against warps per SM: four rows and 20 warps (three vectors per lane) or 16 (four) are best up to some thousands of CTAs
 // (2048 tokens, k = 200: 588 us against 605 with two rows and 28 warps), two rows and more warps beyond (4096 tokens 1164 and 1081; 1000 tokens
 // of 16 x 2048 1003 and 963).  There the tokens are also taken in the order of their list lengths, longest first: warps that
@@ -141,6 +140,8 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // twice the tokens on the chip.  4096 tokens, entries per token on average: 8 139 us with two and 174 with four, 16 182 and 213, 25 (one
 // eighth of the features) 191 and 224, 32 266 and 287, 66 436 and 437, 100 629 and 606.  Only the caller knows the average without a
 // host synchronisation (its k); a threshold selection does not, and counts as long.
+// Equally long lists (a per-token selection) gain nothing from four warps: 2048 tokens of 6 x 768, k = 64, 82 us with one warp and 100 with
+// four, 3536 of 4 x 856, k = 24, 71 and 104, 776 of 5 x 520, k = 24, 19 and 28.
 // Narrow rows: what a CTA costs by itself shows, above all its addition to the error sum (1.5 ns, all CTAs of a target on one
 // address): 12 x 6208 (token, target) pairs of 136 elements without an entry take 116 us with one token per CTA, 60 with two.  So with many
 // tokens one vector per lane goes two tokens and two warps each to a CTA (4096 tokens of 6 x 256, k = 64: 93 us either way).
@@ -152,6 +153,7 @@ constexpr long long kPairNarrowFrom = 24576;   // (token, target) pairs
 constexpr int kRunningOrderFrom = 4096;        // tokens
 constexpr int kShortBelow = 64;                // entries per token on average
 constexpr long long kShortFrom = 16384;        // CTAs
+constexpr int kOneWarpBelow = 128;               // entries of every token
 
 __device__ __forceinline__ int decode_token(const DecodeParams& p, int i) {
   // Tensor-parallel push: rank r starts with the tokens owned by rank r + 1, so that at any moment the ranks
@@ -565,6 +567,7 @@ struct CltDecodeArgs {
   float* ctl;   // optional step control block (loss scale in, found-inf flag out)
   int rows_limit;
   int expected; // entries per token that the caller expects (its k), 0: not known
+  int equal;    // every token has that many
   int* order;   // scratch of clt_sparse_decode_scratch(args) ints, null where that is 0
 };
 
@@ -621,10 +624,15 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
     else if (nv == 2) decode_walk_kernel<2, 1, 8, 4, 24><<<grid, 256, 0, st>>>(p);
     else if (nv == 3) decode_walk_kernel<3, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
     else decode_walk_kernel<4, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
+  } else if (a->equal != 0 && a->expected > 0 && a->expected < kOneWarpBelow) {
+    if (nv <= 1) decode_walk_kernel<1, 4, 1, 4, 32><<<dim3((a->B + 3) / 4, a->L), 128, 0, st>>>(p);
+    else if (nv == 2) decode_walk_kernel<2, 2, 1, 4, 24><<<dim3((a->B + 1) / 2, a->L), 64, 0, st>>>(p);
+    else if (nv == 3) decode_walk_kernel<3, 1, 1, 2, 28><<<grid, 32, 0, st>>>(p);
+    else decode_walk_kernel<4, 1, 1, 2, 20><<<grid, 32, 0, st>>>(p);
   } else if (nv <= 1) {
     if (ctas >= kPairNarrowFrom) decode_walk_kernel<1, 2, 2, 4, 40><<<dim3((a->B + 1) / 2, a->L), 128, 0, st>>>(p);
     else decode_walk_kernel<1, 1, 4, 4, 40><<<grid, 128, 0, st>>>(p);
-  } else if (short_lists(a) && ctas >= kShortFrom) {
+  } else if (short_lists(a) && (a->equal != 0 || ctas >= kShortFrom) && nv >= 2) {
     if (nv == 2) decode_walk_kernel<2, 1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
     else if (nv == 3) decode_walk_kernel<3, 1, 2, 2, 28><<<grid, 64, 0, st>>>(p);
     else decode_walk_kernel<4, 1, 2, 2, 20><<<grid, 64, 0, st>>>(p);

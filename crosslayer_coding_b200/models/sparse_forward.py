@@ -182,7 +182,7 @@ class SparseForward:
         gs, sq_err = (self.gs, self.sq_err) if Y is not None else (None, None)  # no targets: the reconstruction is the only output
         e.sparse_decode([w.data for w in m.dec_weight], self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col,
                         self.tcsr_val, off, scale, None, self.bias_sum, None, Y, sg, gs, yhat, sq_err, 1, [], 0, 0, self.status,
-                        expected_entries=self.expected_entries)
+                        expected_entries=self.expected_entries, equal_lists=self.fn == "topk")
         return yhat
 
     def forward_dict(self, inputs: Dict[int, torch.Tensor]) -> Dict[int, torch.Tensor]:

@@ -570,7 +570,7 @@ class FusedBatchTopKEngine:
         if self.world == 1:
             e.sparse_decode(dec_w, self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col, self.tcsr_val,
                             self.foff32, self.fsc32, None, bias_sum, addend, Y, self.sigma, self.gs, yhat, self.sq_err, 1, [], 0, 0, self.status,
-                            self.step_ctl, expected_entries=self.expected_entries)
+                            self.step_ctl, expected_entries=self.expected_entries, equal_lists=self.fn == "topk")
             self.kernel_launches += 1
         else:
             sy = self.symm

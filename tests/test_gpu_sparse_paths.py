@@ -56,7 +56,7 @@ def _dense_decode(L, B, d, F, tying, tok, col, val, W, off, sc, rows_limit=0):
     return want
 
 
-def _check_decode(ext, L, B, d, tying, affine, dtype=torch.bfloat16, addend=False, rows_limit=0, F=24, entries=None, expected=0):
+def _check_decode(ext, L, B, d, tying, affine, dtype=torch.bfloat16, addend=False, rows_limit=0, F=24, entries=None, expected=0, equal=False):
     dev = _dev()
     g = torch.Generator().manual_seed(L * 1000 + B + d)
     tok, col, val = (entries or _entries)(g, L, B, F, min(B * L * F, 7 * B), dev)
@@ -77,7 +77,7 @@ def _check_decode(ext, L, B, d, tying, affine, dtype=torch.bfloat16, addend=Fals
 
         def decode(mode, partial=None, bias=None, addend=None, target=None, sigma=None, gs=None, yhat=None, sq=None, peers=(), rows_per_rank=0, rank=0):
             ext.sparse_decode(W, L, B, d, F, tying, c["tok_off"], c["tcsr_col"], c["tcsr_val"], off, sc, partial, bias, addend, target, sigma, gs, yhat, sq, mode,
-                              list(peers), rows_per_rank, rank, status, None, rows_limit, expected)
+                              list(peers), rows_per_rank, rank, status, None, rows_limit, expected, equal)
 
         yhat = torch.full((L, B, d), float("nan"), device=dev)
         gs = torch.empty(L, B, d, device=dev, dtype=dtype)
@@ -156,8 +156,14 @@ def test_gather_decode_of_uneven_lists(ext, L, B, d, tying):
 # true the expectation is
 @pytest.mark.parametrize("tying", [0, 1, 2])
 @pytest.mark.parametrize("L,B,d", [(13, 1303, 512), (13, 1303, 520), (9, 1001, 1800), (3, 70, 520)])
-def test_gather_decode_with_an_expected_length(ext, L, B, d, tying):
-    _check_decode(ext, L, B, d, tying, tying != 0, F=72, entries=_uneven_entries, expected=20)
+@pytest.mark.parametrize("expected,equal", [(20, False), (20, True), (60, True)])
+def test_gather_decode_with_an_expected_length(ext, L, B, d, tying, expected, equal):
+    _check_decode(ext, L, B, d, tying, tying != 0, F=72, entries=_uneven_entries, expected=expected, equal=equal)
+
+
+@pytest.mark.parametrize("L,B,d", [(3, 1303, 200), (3, 1303, 512)])
+def test_gather_decode_of_equal_short_lists_in_narrow_rows(ext, L, B, d):
+    _check_decode(ext, L, B, d, 0, False, F=72, entries=_uneven_entries, expected=20, equal=True)
 
 
 def test_decode_refuses_loss_outputs_without_a_target(ext):
