@@ -143,6 +143,7 @@ extern "C" {
 // type-independent entry points (compiled once)
 int clt_colstats_from_tiles(const float* tile_stats, float* mean, float* rstd, int L, int B, int F, cudaStream_t st);
 int clt_build_csr(const CltCsrArgs* a, cudaStream_t st);
+int clt_build_token_csr(const CltCsrArgs* a, int* layer_cnt, cudaStream_t st);
 int clt_dead_counter_update(long long* counter, unsigned char* fired, int n, cudaStream_t st);
 int clt_peer_barrier(const CltPeerTable* flags, int slot, unsigned int seq, int* status, long long timeout_cycles, cudaStream_t st);
 int clt_sparsity_penalty(const int* feat_off, const float* fcsr_val, const float* norm2, int ncols, float lambda, float c,
@@ -450,6 +451,27 @@ void build_csr(const Tensor& ent_tok, const Tensor& ent_col, const Tensor& ent_v
   TORCH_CHECK(col_pitch > 0 && col_pitch < (1 << 24), "col_pitch must be in (0, 2^24)");
   c10::cuda::CUDAGuard guard(ent_tok.device());
   check(clt_build_csr(&a, cur_stream()), "build_csr");
+}
+
+// The token-major view alone, sorted by (layer, feature); layer_cnt: entries per layer (int32, at least one word per layer).
+void build_token_csr(const Tensor& ent_tok, const Tensor& ent_col, const Tensor& ent_val, const Tensor& ctl, int64_t num_tokens, int64_t num_cols,
+                     Tensor& tok_cnt, Tensor& tok_off, Tensor& tok_cursor, Tensor& tcsr_col, Tensor& tcsr_val, Tensor& layer_cnt, int64_t col_pitch) {
+  need(ent_tok, at::kInt, "ent_tok"); need(ent_col, at::kInt, "ent_col"); need(ent_val, at::kFloat, "ent_val"); need(ctl, at::kLong, "ctl");
+  need(tok_cnt, at::kInt, "tok_cnt"); need(tok_off, at::kInt, "tok_off"); need(tok_cursor, at::kInt, "tok_cursor"); need(layer_cnt, at::kInt, "layer_cnt");
+  need(tcsr_col, at::kInt, "tcsr_col"); need(tcsr_val, at::kFloat, "tcsr_val");
+  TORCH_CHECK(col_pitch > 0 && col_pitch < (1 << 24), "col_pitch must be in (0, 2^24)");
+  TORCH_CHECK(tok_off.numel() >= num_tokens + 1 && tok_cnt.numel() >= num_tokens && tok_cursor.numel() >= num_tokens, "token arrays too small");
+  TORCH_CHECK(ent_col.numel() >= ent_tok.numel() && ent_val.numel() >= ent_tok.numel() && tcsr_col.numel() >= ent_tok.numel() &&
+              tcsr_val.numel() >= ent_tok.numel() && layer_cnt.numel() >= (num_cols + col_pitch - 1) / col_pitch, "entry arrays too small");
+  CltCsrArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.ent_tok = ent_tok.data_ptr<int>(); a.ent_col = ent_col.data_ptr<int>(); a.ent_val = ent_val.data_ptr<float>(); a.ent_cap = ent_tok.numel();
+  a.ctl = reinterpret_cast<const long long*>(ctl.data_ptr<int64_t>());
+  a.num_tokens = int(num_tokens); a.num_cols = int(num_cols); a.col_pitch = int(col_pitch);
+  a.tok_cnt = tok_cnt.data_ptr<int>(); a.tok_off = tok_off.data_ptr<int>(); a.tok_cursor = tok_cursor.data_ptr<int>();
+  a.tcsr_col = tcsr_col.data_ptr<int>(); a.tcsr_val = tcsr_val.data_ptr<float>();
+  c10::cuda::CUDAGuard guard(ent_tok.device());
+  check(clt_build_token_csr(&a, layer_cnt.data_ptr<int>(), cur_stream()), "build_token_csr");
 }
 
 void dead_counter_update(Tensor& counter, Tensor& fired) {
@@ -992,6 +1014,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("theta_grad_gemm", &theta_grad_gemm, py::arg("gs"), py::arg("dec_w"), py::arg("preact"), py::arg("theta"), py::arg("bandwidth"),
         py::arg("S1"), py::arg("S2"), py::arg("status"), py::arg("tying") = 0, py::arg("gs_cum") = none);
   m.def("build_csr", &build_csr);
+  m.def("build_token_csr", &build_token_csr);
   m.def("dead_counter_update", &dead_counter_update);
   m.def("sparse_decode", &sparse_decode, py::arg("dec_w"), py::arg("L"), py::arg("B"), py::arg("d"), py::arg("col_pitch"), py::arg("tying"),
         py::arg("tok_off"), py::arg("tcsr_col"), py::arg("tcsr_val"), py::arg("feat_offset"), py::arg("feat_scale"), py::arg("yhat_partial"),

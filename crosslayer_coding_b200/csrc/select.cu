@@ -1424,6 +1424,45 @@ __global__ void __launch_bounds__(256) csr_scatter_kernel(const int* __restrict_
   }
 }
 
+// The token-major view alone, for callers that decode and update nothing: no counters, scan and scatter over the columns.
+// layer_cnt [number of layers, at most 32]: entries per layer.
+__global__ void __launch_bounds__(256) csr_token_count_kernel(const int* __restrict__ ent_tok, const int* __restrict__ ent_col, long long cap,
+                                                                const long long* __restrict__ ctl, int* __restrict__ tok_cnt, int* __restrict__ layer_cnt,
+                                                                int col_pitch, int num_tokens, int num_cols) {
+  __shared__ int per_layer[32];
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) per_layer[threadIdx.x] = 0;
+  __syncthreads();
+  long long n = ctl[CTL_NUM_ENTRIES];
+  if (n > cap) n = cap;
+  const long long stride = 1LL * gridDim.x * blockDim.x;
+  for (long long i0 = blockIdx.x * 1LL * blockDim.x; i0 < n; i0 += stride) {
+    const long long i = i0 + threadIdx.x;
+    const int t = i < n ? ent_tok[i] : -1, c = i < n ? ent_col[i] : -1;
+    const bool in = t >= 0 && t < num_tokens && c >= 0 && c < num_cols;  // as in csr_count_kernel
+    if (in) atomicAdd(&tok_cnt[t], 1);
+    const int layer = in ? c / col_pitch : 32;
+    const uint32_t same = __match_any_sync(0xFFFFFFFFu, layer);
+    if (layer < 32 && lane == __ffs(same) - 1) atomicAdd(&per_layer[layer], __popc(same));
+  }
+  __syncthreads();
+  if (threadIdx.x < 32 && per_layer[threadIdx.x] != 0) atomicAdd(&layer_cnt[threadIdx.x], per_layer[threadIdx.x]);
+}
+__global__ void __launch_bounds__(256) csr_token_scatter_kernel(const int* __restrict__ ent_tok, const int* __restrict__ ent_col,
+                                                                  const float* __restrict__ ent_val, long long cap, const long long* __restrict__ ctl,
+                                                                  int* __restrict__ tok_cursor, int* __restrict__ tcsr_col, float* __restrict__ tcsr_val,
+                                                                  int col_pitch, int num_tokens, int num_cols) {
+  long long n = ctl[CTL_NUM_ENTRIES];
+  if (n > cap) n = cap;
+  for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
+    const int t = ent_tok[i], c = ent_col[i];
+    if (t < 0 || t >= num_tokens || c < 0 || c >= num_cols) continue;
+    const int p = atomicAdd(&tok_cursor[t], 1);
+    const int layer = c / col_pitch;
+    if (p >= 0 && p < cap) { tcsr_col[p] = (layer << 24) | (c - layer * col_pitch); tcsr_val[p] = ent_val[i]; }
+  }
+}
+
 // Bitonic network on n 64-bit words in shared memory or on (key, value) pairs in global memory, by all threads of the CTA.  Every
 // comparator puts the smaller key at the lower index (the first step of a merge pairs mirrored positions), so the virtual
 // padding to a power of two, which stands for +infinity at the end of the array, never has to move.
@@ -1915,6 +1954,22 @@ extern "C" int clt_build_csr(const CltCsrArgs* a, cudaStream_t st) {
   if ((a->sort_segments & 1) && a->num_tokens > 0)
     csr_sort_token_segments_kernel<<<a->num_tokens, 256, 0, st>>>(a->tok_off, a->tcsr_col, a->tcsr_val);
   if (a->sort_segments & 2) launch_feature_sort(a->feat_off, a->num_cols, a->ent_cap, a->fcsr_tok, a->fcsr_val, st);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+// tok_cnt and layer_cnt are zeroed by the caller, as the counters of clt_build_csr are.
+extern "C" int clt_build_token_csr(const CltCsrArgs* a, int* layer_cnt, cudaStream_t st) {
+  if (a->num_tokens <= 0) return 0;
+  if ((a->num_cols + a->col_pitch - 1) / a->col_pitch > 32) return -1;
+  const int blocks = int((a->ent_cap + 255) / 256 < 592 ? (a->ent_cap + 255) / 256 : 592);
+  csr_token_count_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_cap, a->ctl, a->tok_cnt, layer_cnt, a->col_pitch, a->num_tokens, a->num_cols);
+  const ScanJob job{a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens}, none{nullptr, nullptr, nullptr, 0};
+  const int tiles = (a->num_tokens + 4095) / 4096;
+  if (tiles <= 512 && (reinterpret_cast<uintptr_t>(a->tok_cnt) & 15) == 0) exclusive_scan_tiles_kernel<<<tiles, 1024, 0, st>>>(job, none, tiles);
+  else exclusive_scan_kernel<<<1, 1024, 0, st>>>(job.in, job.out, job.cursor, job.n);
+  csr_token_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->tcsr_col, a->tcsr_val,
+                                                   a->col_pitch, a->num_tokens, a->num_cols);
+  csr_sort_token_segments_kernel<<<a->num_tokens, 256, 0, st>>>(a->tok_off, a->tcsr_col, a->tcsr_val);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -98,21 +98,24 @@ class SparseForward:
         # scan over them takes 21 us instead of 16 at 12 x 24576 features.  The loss sums come last, because only `reconstruct`
         # clears them.
         self.hist = torch.zeros(2 * 8192 + 32, dtype=i32, device=dev) if self.fn == "batchtopk" else None
+        # Order: feature counters (only where that view is built), token and layer counters, loss sums.
         starts = [0]
-        for n in (B, ncols):
+        for n in (ncols, B, L):
             starts.append((starts[-1] + n + 63) // 64 * 64)
         self._zeroed = torch.zeros(starts[-1] + 2 * L, dtype=i32, device=dev)
-        self._zeroed_encode = self._zeroed[: starts[-1]]
-        self.tok_cnt, self.feat_cnt = self._zeroed[:B], self._zeroed[starts[1]: starts[1] + ncols]
+        self._zeroed_encode, self._zeroed_token = self._zeroed[: starts[-1]], self._zeroed[starts[1]:]
+        self.feat_cnt, self.tok_cnt = self._zeroed[:ncols], self._zeroed[starts[1]: starts[1] + B]
+        self.layer_cnt = self._zeroed[starts[2]: starts[2] + L]
         self.sq_err = self._zeroed[starts[-1]:].view(torch.float64)
+        self._feature_view = False  # whether the feature-major arrays belong to the last selection
         self.tok_off = torch.zeros(B + 1, dtype=i32, device=dev)
-        self.feat_off = torch.zeros(ncols + 1, dtype=i32, device=dev)
+        self._feat_off = torch.zeros(ncols + 1, dtype=i32, device=dev)
         self.tok_cursor = torch.zeros(B, dtype=i32, device=dev)
         self.feat_cursor = torch.zeros(ncols, dtype=i32, device=dev)
         self.tcsr_col = torch.zeros(cap, dtype=i32, device=dev)
         self.tcsr_val = torch.zeros(cap, dtype=f32, device=dev)
-        self.fcsr_tok = torch.zeros(cap, dtype=i32, device=dev)
-        self.fcsr_val = torch.zeros(cap, dtype=f32, device=dev)
+        self._fcsr_tok = torch.zeros(cap, dtype=i32, device=dev)
+        self._fcsr_val = torch.zeros(cap, dtype=f32, device=dev)
         self.gs = torch.empty(L, B, d, dtype=torch.bfloat16, device=dev)
         if self.tying == 0:
             from .clt import pair_index
@@ -141,6 +144,29 @@ class SparseForward:
     def encode(self, X: torch.Tensor, clear_loss: bool = False, sort_tokens: bool = True) -> None:
         """Pre-activations, selection and the token-major / feature-major CSR views of the active entries.  ``sort_tokens``: a token's
         entries ordered by (layer, feature), which the decode wants; whoever reads the feature-major view alone can do without."""
+        self._select(X)
+        (self._zeroed if clear_loss else self._zeroed_encode).zero_()
+        self._build_views(sort_tokens)
+
+    def _build_views(self, sort_tokens: bool = True) -> None:
+        self.ext.build_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.feat_cnt, self.tok_off,
+                           self._feat_off, self.tok_cursor, self.feat_cursor, self.tcsr_col, self.tcsr_val, self._fcsr_tok, self._fcsr_val,
+                           None, 3 if sort_tokens else 2, self.Fl)
+        self._feature_view = True
+
+    def _features(self, name: str) -> torch.Tensor:
+        """An array of the feature-major view of the last selection.  ``reconstruct`` reads the token-major view alone and does not
+        build the other; it is built from the entry list when somebody asks for it."""
+        if not self._feature_view:
+            self._zeroed_encode.zero_()
+            self._build_views()
+        return getattr(self, name)
+
+    feat_off = property(lambda self: self._features("_feat_off"))
+    fcsr_tok = property(lambda self: self._features("_fcsr_tok"))
+    fcsr_val = property(lambda self: self._features("_fcsr_val"))
+
+    def _select(self, X: torch.Tensor) -> None:
         e, m = self.ext, self.model
         assert X.dtype == torch.bfloat16 and X.shape == (self.L, self.B, self.d), (X.dtype, tuple(X.shape))
         e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, None)
@@ -156,18 +182,17 @@ class SparseForward:
                                 self.ent_val, self.status)
         else:
             e.threshold_select(self.preact, self._theta(), self.Fl, self.Fl, self.ctl, self.ent_tok, self.ent_col, self.ent_val, self.status)
-        (self._zeroed if clear_loss else self._zeroed_encode).zero_()
-        e.build_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.feat_cnt, self.tok_off,
-                    self.feat_off, self.tok_cursor, self.feat_cursor, self.tcsr_col, self.tcsr_val, self.fcsr_tok, self.fcsr_val,
-                    None, 3 if sort_tokens else 2, self.Fl)
-
     # ------------------------------------------------------------------ decode
     @torch.no_grad()
     def reconstruct(self, X: torch.Tensor, Y: Optional[torch.Tensor] = None, sigma: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Reconstructions ``[L, B, d]`` (fp32).  With targets ``Y`` the per-layer sums of squared errors
         (scaled by ``sigma [L, d]`` when given) are left in ``self.sq_err``."""
-        self.encode(X, clear_loss=True)
+        self._select(X)
+        self._zeroed_token.zero_()
+        self._feature_view = False
         e, m = self.ext, self.model
+        e.build_token_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.tok_off, self.tok_cursor,
+                          self.tcsr_col, self.tcsr_val, self.layer_cnt, self.Fl)
         yhat = torch.empty(self.L, self.B, self.d, dtype=torch.float32, device=self.dev)
         bias = m.dec_bias.data
         if bias.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not bias.is_contiguous():
@@ -187,9 +212,19 @@ class SparseForward:
 
     def forward_dict(self, inputs: Dict[int, torch.Tensor]) -> Dict[int, torch.Tensor]:
         """Same contract as ``CrossLayerTranscoder.forward``: ``{layer: [B, d]}`` in, reconstructions out."""
-        X = torch.stack([inputs[l].reshape(-1, self.d) for l in range(self.L)]).to(torch.bfloat16)
-        yhat = self.reconstruct(X)
+        yhat = self.reconstruct(self._stacked([inputs[l].reshape(-1, self.d) for l in range(self.L)]))
         return {l: yhat[l] for l in range(self.L)}
+
+    def _stacked(self, rows) -> torch.Tensor:
+        """``[L, B, d]`` in bf16.  Layers that already lie one after the other in one tensor (the rows of a batch that a store or a capture
+        filled as ``[L, B, d]``) are taken as they are; anything else is copied."""
+        first, step = rows[0], self.B * self.d
+        base, shape = first.data_ptr(), (self.B, self.d)
+        # consecutive addresses inside the first one's storage: the other tensors are views of the same memory
+        if base % 16 == 0 and first.untyped_storage().nbytes() >= 2 * (first.storage_offset() + self.L * step) and all(
+                r.dtype == torch.bfloat16 and r.shape == shape and r.is_contiguous() and r.data_ptr() == base + 2 * l * step for l, r in enumerate(rows)):
+            return first.detach().as_strided((self.L, self.B, self.d), (step, self.d, 1))
+        return torch.stack(rows).to(torch.bfloat16)
 
     # ------------------------------------------------------------------ views of the last selection
     def num_entries(self) -> int:
@@ -197,8 +232,11 @@ class SparseForward:
 
     def l0_per_layer(self) -> torch.Tensor:
         """Mean number of active features per token and layer of the last ``encode``."""
-        per_col = (self.feat_off[1:] - self.feat_off[:-1]).view(self.L, self.Fl).sum(dim=1)
-        return per_col.float() / self.B
+        if self._feature_view:
+            per_layer = (self.feat_off[1:] - self.feat_off[:-1]).view(self.L, self.Fl).sum(dim=1)
+        else:
+            per_layer = self.layer_cnt
+        return per_layer.float() / self.B
 
     def activations_dense(self) -> torch.Tensor:
         """Dense ``[L, B, F]`` activations of the last ``encode`` (testing)."""

@@ -204,6 +204,52 @@ def test_csr_segments_are_sorted(ext, B, L, F, n):
     assert torch.equal(c["tok_off"].cpu(), torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(tok.cpu().long(), minlength=B).cumsum(0)]).to(I32))
 
 
+# one to four entries per thread by rank, the network beyond, one and several tiles of the scan
+@pytest.mark.parametrize("B,L,F,n", [(1, 2, 4000, 250), (3, 4, 1000, 1530), (2, 4, 1000, 1600), (2, 3, 2000, 4500), (5000, 3, 64, 40000), (700, 32, 16, 90000)])
+def test_token_view_alone(ext, B, L, F, n):
+    """The token-major view without the feature-major one: equal to that of the full build, entries outside the problem left out."""
+    dev = _dev()
+    g = torch.Generator().manual_seed(n)
+    tok, col, val = _entries(g, L, B, F, n, dev)
+    c = _csr(ext, tok, col, val, B, L * F, F)
+    stray = torch.tensor([-1, B, 0, 0], dtype=I32, device=dev), torch.tensor([0, 0, -1, L * F], dtype=I32, device=dev), torch.ones(4, device=dev)
+    tok2, col2, val2 = (torch.cat([a, b]) for a, b in zip((tok, col, val), stray))
+    ctl = torch.zeros(16, dtype=torch.int64, device=dev)
+    ctl[3] = n + 4
+    z = lambda k, dt=I32: torch.zeros(k, dtype=dt, device=dev)  # noqa: E731
+    off, tc, tv, per_layer = z(B + 1), z(n + 4), z(n + 4, F32), z(L)
+    ext.build_token_csr(tok2, col2, val2, ctl, B, L * F, z(B), off, z(B), tc, tv, per_layer, F)
+    assert torch.equal(off, c["tok_off"]) and torch.equal(tc[:n], c["tcsr_col"]) and torch.equal(tv[:n], c["tcsr_val"])
+    assert torch.equal(per_layer.long(), torch.bincount((col // F).long(), minlength=L))
+
+
+@pytest.mark.parametrize("fn", ["batchtopk", "topk", "jumprelu"])
+def test_views_after_a_reconstruction(ext, fn):
+    """``reconstruct`` builds the token-major view; the feature-major one and the counts per layer are those of the same selection, and a
+    batch that lies in one tensor gives what separate tensors give."""
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    sf = SparseForward(_serving_model(fn, "none", dev), 200)
+    x = torch.randn(3, 200, 64, device=dev).bfloat16()
+    sf.encode(x)
+    names = ("tok_off", "tcsr_col", "tcsr_val", "feat_off", "fcsr_tok", "fcsr_val")
+    want, n, l0 = {k: getattr(sf, k).clone() for k in names}, sf.num_entries(), sf.l0_per_layer()
+    sf.encode(torch.randn(3, 200, 64, device=dev).bfloat16())
+    a = sf.forward_dict({l: x[l] for l in range(3)})
+    assert torch.equal(sf.l0_per_layer(), l0)
+    for k in names:  # beyond the entries of this selection the arrays hold what earlier ones left
+        assert torch.equal(getattr(sf, k)[: n if "csr" in k else None], want[k][: n if "csr" in k else None]), k
+    assert torch.equal(sf.l0_per_layer(), l0)
+    y = x.clone()
+    for other in ({l: x[l].clone() for l in range(3)}, {l: x[l].float() for l in range(3)}, {0: x[0], 1: x[1], 2: y[2]}):
+        b = sf.forward_dict(other)
+        assert all(torch.equal(a[l], b[l]) for l in range(3))
+    swapped = sf.forward_dict({0: x[1], 1: x[0], 2: x[2]})
+    assert not torch.equal(swapped[0], a[0])
+    sf.check_status()
+
+
 def test_equal_keys_in_a_token_segment_are_all_kept(ext):
     """A caller's list may name one column twice for a token: both entries stay."""
     dev = _dev()
