@@ -1550,60 +1550,133 @@ __global__ void __launch_bounds__(256) csr_sort_feature_segments_kernel(const in
     for (int i = threadIdx.x; i < range; i += 256) { key[lo + i] = int(w[i] >> 32); val[lo + i] = __uint_as_float((unsigned int)(w[i] & 0xFFFFFFFFULL)); }
 }
 
-// Token segments: one CTA per token sorts its entries by (layer, feature).  Up to kTokenRankCap entries every thread counts how
-// many keys are below its own (broadcast reads of shared memory, no barrier in between: 1 us where the 36 barriers of a
-// network on 256 entries take ten) and stores its entry at that rank; more entries, or equal keys, go through the
-// network in shared memory, and lists beyond its buffer through the one in global memory.  The order lets the decode's tokens
-// pass over the decoder rows together (L2) and fixes the order of its sums.
+// Token segments: one CTA per token sorts its entries by (layer, feature).  Short lists: every thread counts how many keys are below
+// its own (broadcast reads of shared memory, no barrier in between: 1 us where the 36 barriers of a network on 256 entries take ten)
+// and stores its entry at that rank.  Longer ones: the entries are dealt into buckets by layer first, and an entry's place is the number of
+// entries in lower layers plus the number of smaller keys in its own bucket.  Long buckets (kTokenRankCap), or equal keys, go through the
+// network in shared memory, and lists beyond its buffer through the one in global memory.  The order lets the decode's tokens pass over
+// the decoder rows together (L2) and fixes the order of its sums.
+// The buckets take a few more barriers and do n * n / layers instead of n * n comparisons: few tokens, where the latency of one CTA counts,
+// rank up to 512 entries (512 tokens of at most 352: 5.3 us against 10.0 with buckets; 16 tokens of up to 605: 16.4 us with the
+// network above 512, 9.1 with buckets); with many tokens the comparisons count (4096 tokens, 200 entries on average: 60 us with ranks up to
+// 512, 48 with buckets; 8192 tokens: 86 and 77; 4096 tokens of 25: 8.7 and 9.7).
 constexpr int kTokenSortCap = 2048;
-constexpr int kTokenRankCap = 512;
+constexpr int kTokenRankCap = 256;
+constexpr int kTokenBuckets = 128;  // layers, as the packed key can number them
+constexpr int kFewTokens = 768;
+
+// Ranks over the whole list, M entries per thread; false when two keys are equal.
+template <int M>
+__device__ __forceinline__ bool rank_sort_segment(int* __restrict__ key, float* __restrict__ val, int n, int* keys, int* taken) {
+  int mine[M], rank[M];
+  float v[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const int i = threadIdx.x + 256 * m;
+    mine[m] = i < n ? key[i] : 0x7FFFFFFF;
+    v[m] = i < n ? val[i] : 0.f;
+    rank[m] = 0;
+    keys[i] = mine[m];
+    taken[i] = 0;
+  }
+  __syncthreads();
+  const int4* k4 = reinterpret_cast<const int4*>(keys);
+  for (int j = 0; j < (n + 3) / 4; ++j) {
+    const int4 q = k4[j];
+#pragma unroll
+    for (int m = 0; m < M; ++m) rank[m] += (q.x < mine[m]) + (q.y < mine[m]) + (q.z < mine[m]) + (q.w < mine[m]);
+  }
+  bool clash = false;  // equal keys share a rank
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+    if (threadIdx.x + 256 * m < n) clash |= atomicExch(&taken[rank[m]], 1) != 0;
+  if (__syncthreads_or(clash)) return false;
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+    if (threadIdx.x + 256 * m < n) { key[rank[m]] = mine[m]; val[rank[m]] = v[m]; }
+  return true;
+}
+
+// M entries per thread (n <= 256 M); false when the network has to sort them.
+template <int M>
+__device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float* __restrict__ val, int n, int* bucket, int* taken, int* count, int* base) {
+  int mine[M], slot[M];
+  float v[M];
+  if (threadIdx.x < kTokenBuckets) count[threadIdx.x] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const int i = threadIdx.x + 256 * m;
+    if (i < n) {
+      mine[m] = key[i];
+      v[m] = val[i];
+      slot[m] = atomicAdd(&count[(mine[m] >> 24) & (kTokenBuckets - 1)], 1);
+      taken[i] = 0;
+    }
+  }
+  __syncthreads();
+  bool network = false;
+  if (threadIdx.x < 32) {
+    int c[4], sum = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      c[k] = count[4 * threadIdx.x + k];
+      network |= c[k] > kTokenRankCap;
+      sum += c[k];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (int(threadIdx.x) >= o) incl += up;
+    }
+    int run = incl - sum;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { base[4 * threadIdx.x + k] = run; run += c[k]; }
+  }
+  if (__syncthreads_or(network)) return false;
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+    if (threadIdx.x + 256 * m < n) bucket[base[(mine[m] >> 24) & (kTokenBuckets - 1)] + slot[m]] = mine[m];
+  __syncthreads();
+  bool clash = false;  // equal keys share a place
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    if (threadIdx.x + 256 * m < n) {
+      const int l = (mine[m] >> 24) & (kTokenBuckets - 1);
+      const int b = base[l], e = b + count[l];
+      int at = b;
+      for (int j = b; j < e; ++j) at += bucket[j] < mine[m] ? 1 : 0;
+      slot[m] = at;
+      clash |= atomicExch(&taken[at], 1) != 0;
+    }
+  }
+  if (__syncthreads_or(clash)) return false;
+#pragma unroll
+  for (int m = 0; m < M; ++m)
+    if (threadIdx.x + 256 * m < n) { key[slot[m]] = mine[m]; val[slot[m]] = v[m]; }
+  return true;
+}
+
 __global__ void __launch_bounds__(256) csr_sort_token_segments_kernel(const int* __restrict__ off, int* __restrict__ key, float* __restrict__ val) {
-  __shared__ unsigned long long w[kTokenSortCap];
+  __shared__ __align__(16) unsigned long long w[kTokenSortCap];
+  __shared__ int count[kTokenBuckets], base[kTokenBuckets];
   const int b = off[blockIdx.x], n = off[blockIdx.x + 1] - b;
   if (n <= 1) return;
   if (n > kTokenSortCap) {
     sort_pairs_cta(key + b, val + b, n);
     return;
   }
-  if (n <= kTokenRankCap) {
-    __shared__ __align__(16) int keys[kTokenRankCap];
-    __shared__ int taken[kTokenRankCap];
-    int mine[2];
-    float v[2];
-    int rank[2] = {0, 0};
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const int i = threadIdx.x + 256 * m;
-      mine[m] = i < n ? key[b + i] : 0x7FFFFFFF;
-      v[m] = i < n ? val[b + i] : 0.f;
-      keys[i] = mine[m];
-      taken[i] = 0;
-    }
-    __syncthreads();
-    const int4* k4 = reinterpret_cast<const int4*>(keys);
-    if (n <= 256) {
-      for (int j = 0; j < (n + 3) / 4; ++j) {
-        const int4 q = k4[j];
-        rank[0] += (q.x < mine[0]) + (q.y < mine[0]) + (q.z < mine[0]) + (q.w < mine[0]);
-      }
-    } else {
-      for (int j = 0; j < (n + 3) / 4; ++j) {
-        const int4 q = k4[j];
-#pragma unroll
-        for (int m = 0; m < 2; ++m) rank[m] += (q.x < mine[m]) + (q.y < mine[m]) + (q.z < mine[m]) + (q.w < mine[m]);
-      }
-    }
-    bool clash = false;  // equal keys share a rank
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-      if (threadIdx.x + 256 * m < n) clash |= atomicExch(&taken[rank[m]], 1) != 0;
-    if (!__syncthreads_or(clash)) {
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-        if (threadIdx.x + 256 * m < n) { key[b + rank[m]] = mine[m]; val[b + rank[m]] = v[m]; }
-      return;
-    }
-  }
+  int* bucket = reinterpret_cast<int*>(w);  // the buckets share the network's buffer: keys in the first half, marks in the second
+  int* taken = bucket + kTokenSortCap;
+  const bool done = n <= (gridDim.x < kFewTokens ? 512 : 128)
+                        ? (n <= 256 ? rank_sort_segment<1>(key + b, val + b, n, bucket, taken) : rank_sort_segment<2>(key + b, val + b, n, bucket, taken))
+                    : n <= 256  ? bucket_sort_segment<1>(key + b, val + b, n, bucket, taken, count, base)
+                    : n <= 512  ? bucket_sort_segment<2>(key + b, val + b, n, bucket, taken, count, base)
+                    : n <= 1024 ? bucket_sort_segment<4>(key + b, val + b, n, bucket, taken, count, base)
+                                : bucket_sort_segment<8>(key + b, val + b, n, bucket, taken, count, base);
+  if (done) return;
+  __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) w[i] = pack_entry(key[b + i], val[b + i]);
   sort_words_cta(w, n);
   for (int i = threadIdx.x; i < n; i += blockDim.x) { key[b + i] = int(w[i] >> 32); val[b + i] = __uint_as_float((unsigned int)(w[i] & 0xFFFFFFFFULL)); }

@@ -204,8 +204,10 @@ def test_csr_segments_are_sorted(ext, B, L, F, n):
     assert torch.equal(c["tok_off"].cpu(), torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(tok.cpu().long(), minlength=B).cumsum(0)]).to(I32))
 
 
-# one to four entries per thread by rank, the network beyond, one and several tiles of the scan
-@pytest.mark.parametrize("B,L,F,n", [(1, 2, 4000, 250), (3, 4, 1000, 1530), (2, 4, 1000, 1600), (2, 3, 2000, 4500), (5000, 3, 64, 40000), (700, 32, 16, 90000)])
+# ranks over the list and buckets by layer (few and many tokens), one to eight entries per thread, a bucket that is too long, the network
+# beyond, one and several tiles of the scan
+@pytest.mark.parametrize("B,L,F,n", [(1, 2, 4000, 250), (3, 4, 1000, 1530), (2, 4, 1000, 1600), (2, 12, 1000, 3800), (2, 2, 4000, 1700), (2, 3, 2000, 4500),
+                                     (5000, 3, 64, 40000), (700, 32, 16, 90000), (1100, 8, 64, 200000), (1100, 8, 80, 450000), (1100, 5, 300, 900000)])
 def test_token_view_alone(ext, B, L, F, n):
     """The token-major view without the feature-major one: equal to that of the full build, entries outside the problem left out."""
     dev = _dev()
