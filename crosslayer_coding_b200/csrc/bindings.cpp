@@ -363,7 +363,9 @@ void token_topk_select(const Tensor& x, const Tensor& mean, const Tensor& rstd, 
   a.ent_tok = ent_tok.data_ptr<int>(); a.ent_col = ent_col.data_ptr<int>(); a.ent_val = ent_val.data_ptr<float>(); a.ent_cap = ent_tok.numel();
   a.status = status.data_ptr<int>();
   c10::cuda::CUDAGuard guard(x.device());
-  check(CLT_PICK(half, clt_token_topk_select)(&a, cur_stream()), "token_topk_select");
+  Tensor scratch;  // allocated and used on the current stream
+  if (const long long bytes = CLT_PICK(half, clt_token_topk_scratch)(&a)) scratch = at::empty({bytes}, x.options().dtype(at::kByte));
+  check(CLT_PICK(half, clt_token_topk_select)(&a, scratch.defined() ? scratch.data_ptr() : nullptr, cur_stream()), "token_topk_select");
 }
 
 // One phase of the TokenTopK selection across feature shards (0: push the local candidates' keys to the token owners,

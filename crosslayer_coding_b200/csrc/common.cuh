@@ -306,6 +306,12 @@ __device__ __forceinline__ uint32_t t16x2_ge_mask(uint32_t a, uint32_t b) {
   asm("set.ge.u32.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
+// 0xFFFF in every half where a >= b or either is NaN
+__device__ __forceinline__ uint32_t t16x2_not_below_mask(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("set.geu.u32.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 #else
 __device__ __forceinline__ uint32_t pack_t16x2(float lo, float hi) { return pack_bf16x2(lo, hi); }
 __device__ __forceinline__ float t16_lo(uint32_t v) { return bf16_lo(v); }
@@ -317,6 +323,12 @@ __device__ __forceinline__ t16x2 make_t16x2(t16 a, t16 b) { return __halves2bflo
 __device__ __forceinline__ uint32_t t16x2_ge_mask(uint32_t a, uint32_t b) {
   uint32_t r;
   asm("set.ge.u32.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+// 0xFFFF in every half where a >= b or either is NaN
+__device__ __forceinline__ uint32_t t16x2_not_below_mask(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("set.geu.u32.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
 #endif

@@ -857,6 +857,203 @@ __global__ void __launch_bounds__(kTkThreads) token_topk_list_kernel(const t16* 
   }
 }
 
+// The list form for large matrices, in four passes.  The kernel above gives a CTA one to four tokens and reads the column statistics once
+// per such group: 64 bytes of statistics per 16 bytes of a token, a chain of a hundred dependent loads, 350 us at 6 x 2048 x 32768, k = 64;
+// the four passes take 302 (sample 46, bound 29, collect 206, cut 22).  Here a thread owns eight columns and walks 64 tokens, as the histogram scan does:
+//   sample   maxima of groups of eight columns, every step-th run of 32 groups, one word per group and token
+//   bound    per token: a key that at least k of its maxima reach
+//   collect  one scan: what reaches the bound goes to the token's list (about step * k words)
+//   cut      per token (one warp): the exact cut of the list, as above; a token whose list overflows goes to the radix kernel
+constexpr int kWideRows = 64;
+constexpr int kWideMaxima = 4096;   // per token
+constexpr int kWideQueue = 2048;    // groups of a tile that pass the coarse test, numbered with 16 bits
+struct WideTopk {
+  int* n;                        // [B] list lengths (zeroed by the caller)
+  uint32_t* bound;               // [B]
+  uint32_t* maxima;              // [B][ng]
+  unsigned long long* list;      // [B][cap] (key << 32 | inverted column)
+  int ng, cap, step, groups;
+};
+
+__device__ __forceinline__ float t16_of(const uint4& v, int j) {
+  const uint32_t u = j < 2 ? v.x : (j < 4 ? v.y : (j < 6 ? v.z : v.w));
+  return (j & 1) ? t16_hi(u) : t16_lo(u);
+}
+
+__global__ void __launch_bounds__(256) token_sample_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
+                                                             int f_valid, WideTopk wt) {
+  const int sg = blockIdx.x * 256 + threadIdx.x;  // < ng, a multiple of 256
+  const int q = (sg >> 5) * 32 * wt.step + (sg & 31);  // runs of 32 groups: short enough that a sample meets every layer
+  const int r0 = blockIdx.y * kWideRows, r1 = min(g.B, r0 + kWideRows);
+  if (q >= wt.groups) {
+    for (int r = r0; r < r1; ++r) wt.maxima[1LL * r * wt.ng + sg] = 0u;
+    return;
+  }
+  const int per_layer = g.F / 8;
+  const int l = q / per_layer, c0 = (q - l * per_layer) * 8;
+  float mu[8], rs[8];
+  load_cols8(mean + 1LL * l * g.sp + c0, mu);
+  load_cols8(rstd + 1LL * l * g.sp + c0, rs);
+  const int nvalid = f_valid - c0;
+  const t16* base = x + 1LL * l * g.layer_stride + c0;
+  for (int rb = r0; rb < r1; rb += 8) {
+    uint4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __ldg(reinterpret_cast<const uint4*>(base + 1LL * min(rb + k, r1 - 1) * g.ld));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (rb + k >= r1) break;
+      float m = -INFINITY;  // a NaN, which sorts above everything, only makes the bound smaller here
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m = fmaxf(m, j < nvalid ? (t16_of(v[k], j) - mu[j]) * rs[j] : -INFINITY);
+      wt.maxima[1LL * (rb + k) * wt.ng + sg] = m == -INFINITY ? 0u : float_to_key(m);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) token_bound_kernel(WideTopk wt, int k, long long* __restrict__ ctl, long long n_entries) {
+  __shared__ int total[2];
+  const int tok = blockIdx.x;
+  if (tok == 0 && threadIdx.x == 0) ctl[CTL_NUM_ENTRIES] = n_entries;
+  uint32_t mine[kWideMaxima / 256];
+#pragma unroll
+  for (int i = 0; i < kWideMaxima / 256; ++i) {
+    const int at = i * 256 + threadIdx.x;
+    mine[i] = at < wt.ng ? wt.maxima[1LL * tok * wt.ng + at] : 0u;
+  }
+  if (threadIdx.x < 2) total[threadIdx.x] = 0;
+  __syncthreads();
+  uint32_t bound = 0;  // largest key with zero low bits that at least k maxima reach
+  int turn = 0;
+#pragma unroll 1
+  for (int bit = 31; bit >= 12; --bit, turn ^= 1) {
+    const uint32_t trial = bound | (1u << bit);
+    int cnt = 0;
+#pragma unroll
+    for (int i = 0; i < kWideMaxima / 256; ++i) cnt += mine[i] >= trial ? 1 : 0;
+    cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+    if ((threadIdx.x & 31) == 0 && cnt != 0) atomicAdd(&total[turn], cnt);
+    __syncthreads();
+    if (total[turn] >= k) bound = trial;
+    if (threadIdx.x == 0) total[turn ^ 1] = 0;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) wt.bound[tok] = bound;
+}
+
+__global__ void __launch_bounds__(256) token_collect_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
+                                                              int col_pitch, int f_valid, WideTopk wt) {
+  __shared__ uint16_t queue[kWideQueue];
+  __shared__ float z_scaled[kWideRows];
+  __shared__ uint32_t bound[kWideRows];
+  __shared__ int s_q;
+  const int l = blockIdx.z, c0 = (blockIdx.x * 256 + int(threadIdx.x)) * 8;
+  const int r0 = blockIdx.y * kWideRows, r1 = min(g.B, r0 + kWideRows);
+  constexpr float kSlack = 1.f / 256.f;
+  if (threadIdx.x < kWideRows) {
+    const uint32_t b = r0 + int(threadIdx.x) < r1 ? wt.bound[r0 + threadIdx.x] : 0xFFFFFFFFu;
+    const float z = key_to_float(b);  // NaN for a bound of 0: everything passes
+    bound[threadIdx.x] = b;
+    z_scaled[threadIdx.x] = z - kSlack * fabsf(z);
+  }
+  if (threadIdx.x == 0) s_q = 0;
+  __syncthreads();
+  if (c0 < g.F) {
+    // A coarse test in the input's own format (one packed compare per two elements, one FMA per column) lets through what the exact test may
+    // accept: z >= z_b needs x >= mean + z_b / rstd, and the right side, lowered by 2^-8 of its terms, stays below that after
+    // rounding to 16 bits.  "Not below" rather than "at or above": a NaN, in the element or in a column's statistics, is left to the
+    // exact test, where it sorts above everything.
+    float low[8], spread[8];
+    {
+      float mu[8], rs[8];
+      load_cols8(mean + 1LL * l * g.sp + c0, mu);
+      load_cols8(rstd + 1LL * l * g.sp + c0, rs);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        low[j] = mu[j] - fmaf(kSlack, fabsf(mu[j]), kT16Max < 1e5f ? 1e-7f : 1e-30f);  // fp16: below its smallest step
+        spread[j] = __fdividef(1.f, rs[j]);
+      }
+    }
+    const t16* base = x + 1LL * l * g.layer_stride + c0;
+    for (int rb = r0; rb < r1; rb += 8) {
+      uint4 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = __ldcs(reinterpret_cast<const uint4*>(base + 1LL * min(rb + k, r1 - 1) * g.ld));
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float z = z_scaled[min(rb + k, r1 - 1) - r0];
+        uint32_t thr[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) thr[j] = pack_t16x2(fmaf(z, spread[2 * j], low[2 * j]), fmaf(z, spread[2 * j + 1], low[2 * j + 1]));
+        const uint32_t hit = t16x2_not_below_mask(v[k].x, thr[0]) | t16x2_not_below_mask(v[k].y, thr[1]) | t16x2_not_below_mask(v[k].z, thr[2]) |
+                             t16x2_not_below_mask(v[k].w, thr[3]);
+        if (hit != 0u && rb + k < r1) {
+          const int slot = atomicAdd(&s_q, 1);
+          if (slot < kWideQueue) queue[slot] = uint16_t((uint32_t(rb + k - r0) << 8) | threadIdx.x);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  const int nq = s_q;
+  if (nq > kWideQueue) {  // lost groups: the tokens of this tile go to the radix kernel
+    if (int(threadIdx.x) < r1 - r0) atomicMax(&wt.n[r0 + threadIdx.x], 1 << 28);
+    return;
+  }
+  for (int e = threadIdx.x; e < nq * 8; e += 256) {
+    const uint32_t item = queue[e >> 3];
+    const int r = int(item >> 8), c = (blockIdx.x * 256 + int(item & 255u)) * 8 + (e & 7);
+    if (c >= f_valid || c >= g.F) continue;  // padding columns of a shard take no part
+    const float xv = t16_to_float(x[1LL * l * g.layer_stride + 1LL * (r0 + r) * g.ld + c]);
+    const uint32_t key = float_to_key((xv - __ldg(mean + 1LL * l * g.sp + c)) * __ldg(rstd + 1LL * l * g.sp + c));
+    if (key < bound[r]) continue;
+    const int slot = atomicAdd(&wt.n[r0 + r], 1);
+    if (slot >= 0 && slot < wt.cap) wt.list[1LL * (r0 + r) * wt.cap + slot] = ((unsigned long long)key << 32) | (0xFFFFFFFFu - (unsigned int)(l * col_pitch + c));
+  }
+}
+
+// W: words per lane (cap <= 32 W).
+template <int W>
+__global__ void __launch_bounds__(128) token_cut_kernel(const t16* __restrict__ x, ScanGeom g, int col_pitch, int k, WideTopk wt, Lists o) {
+  const int tok = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (tok >= g.B) return;
+  const int n = wt.n[tok];
+  if (n > wt.cap || n < k) {
+    if (lane == 0) o.ent_tok[1LL * tok * k] = -1;  // for the radix kernel
+    return;
+  }
+  unsigned long long w[W];
+#pragma unroll
+  for (int i = 0; i < W; ++i) w[i] = i * 32 + lane < n ? wt.list[1LL * tok * wt.cap + i * 32 + lane] : 0ULL;
+  unsigned long long cut = 0;  // the largest word that exactly k words reach
+#pragma unroll 1
+  for (int bit = 63; bit >= 0; --bit) {
+    const unsigned long long trial = cut | (1ULL << bit);
+    int cnt = 0;
+#pragma unroll
+    for (int i = 0; i < W; ++i) cnt += w[i] >= trial ? 1 : 0;
+    cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+    if (cnt >= k) cut = trial;
+    if (cnt == k) break;
+  }
+  const long long out = 1LL * tok * k;
+  int done = 0;
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    const bool keep = i * 32 + lane < n && w[i] >= cut;
+    const unsigned ball = __ballot_sync(0xFFFFFFFFu, keep);
+    const int slot = done + __popc(ball & ((1u << lane) - 1u));
+    if (keep && slot < k) {
+      const int col = int(0xFFFFFFFFu - (unsigned int)(w[i] & 0xFFFFFFFFULL));
+      const int l = col / col_pitch, c = col - l * col_pitch;
+      o.ent_tok[out + slot] = tok;
+      o.ent_col[out + slot] = col;
+      o.ent_val[out + slot] = t16_to_float(x[1LL * l * g.layer_stride + 1LL * tok * g.ld + c]);
+    }
+    done += __popc(ball);
+  }
+}
+
 // ------------------------------------------------------------------ 3b. split the pool at the threshold bin
 // Runs instead of the full compaction pass when the tracked range contained the cut.
 __global__ void __launch_bounds__(256) classify_pool_kernel(Pool pool, long long* __restrict__ ctl, Lists o,
@@ -1849,10 +2046,38 @@ static int launch_token_list(const CltSelectArgs* a, const ScanGeom& g, int f_va
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
+// Geometry of the wide form, or step = 0 where it does not apply: at least kWideElements elements, and a sample of at least 4 k groups
+// whose expected list (step * k) takes half of its room.  6 x 2048 x 32768, k = 64: 351 us in one kernel, 302 here; 6 x 2048 x 8192, k = 24: about 100
+// and 148, the passes over tokens (bound, cut) do not shrink with the columns.
+constexpr long long kWideElements = 1LL << 28;
+static WideTopk wide_topk(const CltSelectArgs* a, long long k) {
+  WideTopk w = {};
+  w.groups = a->L * (a->F / 8);
+  if (1LL * a->B * a->L * a->F < kWideElements || k > 512) return w;
+  w.cap = k <= 64 ? 1024 : 2048;
+  int step = int(w.cap / 2 / k);
+  step = step > 8 ? 8 : step;
+  const auto sampled = [&](int s) { return ((w.groups + 32 * s - 1) / (32 * s) * 32 + 255) / 256 * 256; };
+  while (step > 1 && sampled(step) < 4 * k) --step;
+  if (step < 1 || sampled(step) > kWideMaxima || sampled(step) < 4 * k) return w;
+  // a tile (64 tokens, 2048 columns) has room for four times the groups expected in it; where k is a larger share of the columns, tokens would
+  // be lost to the radix kernel (6 x 2048 x 8192, k = 64: 494 us)
+  if (1LL * kWideRows * step * k * 2048 > kWideQueue / 4 * 1LL * a->L * a->F) return w;
+  w.step = step;
+  w.ng = sampled(step);
+  return w;
+}
+// Bytes of scratch that clt_token_topk_select uses in its wide form (0: none).
+extern "C" long long CLT_FN(clt_token_topk_scratch)(const CltSelectArgs* a) {
+  const WideTopk w = wide_topk(a, a->k_total);
+  if (w.step == 0 || a->k_total <= 0) return 0;
+  return 1LL * a->B * (8LL * w.cap + 4LL * w.ng + 8);
+}
+
 // Per-token top-k of the batch z-scores (TokenTopK).  Uses x, mean, rstd, L, B, F, stat_pitch, ld, layer_stride,
 // col_pitch, ctl, ent_* (capacity >= B * k), status of the argument block; k_total carries the per-token k and feat_offset
 // (when positive) the number of valid columns per layer (the rest of F is shard padding).
-extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, cudaStream_t st) {
+extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, void* scratch, cudaStream_t st) {
   if (a->ld % 8 != 0 || a->layer_stride % 8 != 0 || a->F % 8 != 0 || a->stat_pitch % 4 != 0 || a->F > a->ld) return -1;
   const long long k = a->k_total;
   const int f_valid = a->feat_offset > 0 && a->feat_offset <= a->F ? a->feat_offset : a->F;  // feat_offset carries the valid column count here
@@ -1864,8 +2089,24 @@ extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, cudaStream_
     attr_set = true;
   }
   const int grid = (a->B + kTokPerCta - 1) / kTokPerCta;
-  const bool list = k <= kTkMaxima / 2;
-  if (list) {
+  const WideTopk shape = wide_topk(a, k);
+  const bool wide = shape.step > 0 && scratch != nullptr;
+  const bool list = wide || k <= kTkMaxima / 2;
+  if (wide) {
+    WideTopk w = shape;
+    w.list = static_cast<unsigned long long*>(scratch);
+    w.maxima = reinterpret_cast<uint32_t*>(w.list + 1LL * a->B * w.cap);
+    w.bound = w.maxima + 1LL * a->B * w.ng;
+    w.n = reinterpret_cast<int*>(w.bound + a->B);
+    const t16* x = static_cast<const t16*>(a->x);
+    const int row_blocks = (a->B + kWideRows - 1) / kWideRows;
+    if (cudaMemsetAsync(w.n, 0, sizeof(int) * size_t(a->B), st) != cudaSuccess) return -5;
+    token_sample_kernel<<<dim3(w.ng / 256, row_blocks), 256, 0, st>>>(x, a->mean, a->rstd, g, f_valid, w);
+    token_bound_kernel<<<a->B, 256, 0, st>>>(w, int(k), a->ctl, 1LL * a->B * k);
+    token_collect_kernel<<<dim3((a->F / 8 + 255) / 256, row_blocks, a->L), 256, 0, st>>>(x, a->mean, a->rstd, g, a->col_pitch, f_valid, w);
+    if (w.cap <= 1024) token_cut_kernel<32><<<(a->B + 3) / 4, 128, 0, st>>>(x, g, a->col_pitch, int(k), w, lists_of(a));
+    else token_cut_kernel<64><<<(a->B + 3) / 4, 128, 0, st>>>(x, g, a->col_pitch, int(k), w, lists_of(a));
+  } else if (list) {
     // Tokens per CTA: what finishes in one wave of 148 SMs with four CTAs each (three of four tokens, whose lists are 64 KB).  More
     // tokens per CTA share the loads of the column statistics but take longer each, so one token while all fit that way, then
     // two, then four (from 1332: a second wave of a few CTAs of two costs less than four tokens in a row); beyond that, in several

@@ -166,6 +166,13 @@ def test_gather_decode_of_equal_short_lists_in_narrow_rows(ext, L, B, d):
     _check_decode(ext, L, B, d, 0, False, F=72, entries=_uneven_entries, expected=20, equal=True)
 
 
+# the running sum with one and with two warps per token
+@pytest.mark.parametrize("d", [200, 520])
+@pytest.mark.parametrize("expected,equal", [(20, False), (40, False), (100, True)])
+def test_running_decode_with_an_expected_length(ext, d, expected, equal):
+    _check_decode(ext, 5, 1303, d, 1, False, F=72, entries=_uneven_entries, expected=expected, equal=equal)
+
+
 def test_decode_refuses_loss_outputs_without_a_target(ext):
     """Without a target neither the gradient seed nor the error sums are written: a call that hands them in is an error."""
     dev = _dev()
@@ -339,6 +346,48 @@ def test_token_topk_on_two_devices_of_one_process(ext):
         mean, rstd = torch.empty(2, 512, device=dev), torch.empty(2, 512, device=dev)
         ext.colstats(x, mean, rstd)
         _check_token_topk(ext, x, mean, rstd, 8, 512, dev)
+
+
+# the four-pass form of large matrices: shard padding, columns and tokens that do not fill a tile, k on both sides of the two list sizes; values
+# with ties at the cut
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,B,Fl,F,k", [(3, 4400, 20488, 20481, 24), (4, 2050, 33000, 33000, 64), (8, 1030, 32768, 32760, 200), (8, 1029, 32776, 32776, 512)])
+def test_token_topk_of_large_matrices(ext, L, B, Fl, F, k, dtype):
+    dev = _dev()
+    assert B * L * Fl >= 1 << 28
+    g = torch.Generator(device=dev).manual_seed(k)
+    x = (torch.randn(L, B, Fl, generator=g, device=dev) * 0.7 + 0.3 * torch.randn(L, 1, Fl, generator=g, device=dev)).to(dtype)
+    mean = torch.stack([x[l].float().mean(0) for l in range(L)])
+    rstd = torch.stack([1.0 / (x[l].float().std(0) + 1e-6) for l in range(L)])
+    _check_token_topk(ext, x, mean, rstd, k, F, dev)
+
+
+def test_token_topk_of_large_matrices_with_values_that_are_not_finite(ext):
+    """A column with a NaN has NaN statistics and sorts above everything in every row, and infinities sort by their sign: as in the form for
+    small matrices, which the same rows are put through a few at a time."""
+    dev = _dev()
+    L, B, F, k = 2, 3328, 41000, 40
+    g = torch.Generator(device=dev).manual_seed(3)
+    x = torch.randn(L, B, F, generator=g, device=dev).bfloat16()
+    x[0, 7, 100] = float("nan")
+    x[1, 9, 200] = float("inf")
+    x[1, 5, 300] = float("-inf")
+    x[:, 11] = 1000.0  # a row far above the others: its whole list reaches the bound
+    x[:, 12, :8192] = 50.0
+    mean, rstd = x.float().mean(1), 1.0 / (x.float().std(1) + 1e-6)
+    rstd[1, 400] = 0.0
+
+    def select(rows):
+        xs = x[:, rows].contiguous()
+        n = xs.shape[1]
+        tok, col = torch.zeros(n * k, dtype=I32, device=dev), torch.zeros(n * k, dtype=I32, device=dev)
+        val, status = torch.zeros(n * k, device=dev), torch.zeros(4, dtype=I32, device=dev)
+        ext.token_topk_select(xs, mean, rstd, F, k, torch.zeros(16, dtype=torch.int64, device=dev), tok, col, val, status, F)
+        return torch.sort(col.view(n, k), dim=1).values, int(status[0])
+
+    want = [select(slice(b, b + 256)) for b in range(0, B, 256)]
+    got = select(slice(0, B))
+    assert torch.equal(got[0], torch.cat([w[0] for w in want])) and got[1] == max(w[1] for w in want)
 
 
 def _serving_model(fn, tying, dev, L=3, d=64, F=512):
