@@ -145,7 +145,8 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // Narrow rows: what a CTA costs by itself shows, above all its addition to the error sum (1.5 ns, all CTAs of a target on one
 // address): 12 x 6208 (token, target) pairs of 136 elements without an entry take 116 us with one token per CTA, 60 with two.  So with many
 // tokens one vector per lane goes two tokens and two warps each to a CTA (4096 tokens of 6 x 256, k = 64: 93 us either way).
-// Per-source tied, running sums: 4 warps 340 us, 1 warp 610 (8192 tokens of 6 x 512, k = 200), sorted by length 295.
+// Per-source tied, running sums: 4 warps 340 us, 1 warp 610 (8192 tokens of 6 x 512, k = 200), sorted by length 295; short or equally long
+// lists are the other way round (5809 tokens of 4 x 600, k = 19: 122 us with four, 77 with one; 2048 of 6 x 512, equal lists of 64: 37, 33).
 constexpr long long kRunningMinWarps = 1024;   // tokens x chunks; below, the (token, target) split has L times as many CTAs
 constexpr long long kEightWarpsBelow = 2048;   // CTAs
 constexpr long long kManyCtas = 28672;         // CTAs
@@ -153,6 +154,7 @@ constexpr long long kPairNarrowFrom = 24576;   // (token, target) pairs
 constexpr int kRunningOrderFrom = 4096;        // tokens
 constexpr int kShortBelow = 64;                // entries per token on average
 constexpr long long kShortFrom = 16384;        // CTAs
+constexpr int kRunningOneWarpBelow = 32;         // entries per token on average
 constexpr int kOneWarpBelow = 128;               // entries of every token
 
 __device__ __forceinline__ int decode_token(const DecodeParams& p, int i) {
@@ -611,8 +613,16 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   }
   if (takes_running(a)) {
     const dim3 grid(a->B, running_chunks(a));
-    if (a->d <= 256) decode_running_kernel<1, 4, 4, 24><<<grid, 128, 0, st>>>(p);
-    else decode_running_kernel<2, 4, 4, 20><<<grid, 128, 0, st>>>(p);
+    if (a->expected > 0 && a->expected < (a->equal != 0 ? kOneWarpBelow : kRunningOneWarpBelow)) {
+      if (a->d <= 256) decode_running_kernel<1, 1, 4, 24><<<grid, 32, 0, st>>>(p);
+      else decode_running_kernel<2, 1, 4, 16><<<grid, 32, 0, st>>>(p);
+    } else if (short_lists(a)) {
+      if (a->d <= 256) decode_running_kernel<1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
+      else decode_running_kernel<2, 2, 4, 20><<<grid, 64, 0, st>>>(p);
+    } else {
+      if (a->d <= 256) decode_running_kernel<1, 4, 4, 24><<<grid, 128, 0, st>>>(p);
+      else decode_running_kernel<2, 4, 4, 20><<<grid, 128, 0, st>>>(p);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
   const int chunks = walk_chunks(a);
