@@ -63,6 +63,7 @@ struct CltCsrArgs {
   unsigned char* fired;
   int sort_segments;
   int col_pitch;
+  int* layer_cnt;
 };
 struct CltDecodeArgs {
   const void* w[32];
@@ -143,7 +144,7 @@ extern "C" {
 // type-independent entry points (compiled once)
 int clt_colstats_from_tiles(const float* tile_stats, float* mean, float* rstd, int L, int B, int F, cudaStream_t st);
 int clt_build_csr(const CltCsrArgs* a, cudaStream_t st);
-int clt_build_token_csr(const CltCsrArgs* a, int* layer_cnt, cudaStream_t st);
+int clt_build_token_csr(const CltCsrArgs* a, cudaStream_t st);
 int clt_dead_counter_update(long long* counter, unsigned char* fired, int n, cudaStream_t st);
 int clt_peer_barrier(const CltPeerTable* flags, int slot, unsigned int seq, int* status, long long timeout_cycles, cudaStream_t st);
 int clt_sparsity_penalty(const int* feat_off, const float* fcsr_val, const float* norm2, int ncols, float lambda, float c,
@@ -435,7 +436,7 @@ void theta_grad_gemm(const Tensor& gs, const std::vector<Tensor>& dec_w, const T
 void build_csr(const Tensor& ent_tok, const Tensor& ent_col, const Tensor& ent_val, const Tensor& ctl, int64_t num_tokens, int64_t num_cols,
                Tensor& tok_cnt, Tensor& feat_cnt, Tensor& tok_off, Tensor& feat_off, Tensor& tok_cursor, Tensor& feat_cursor,
                Tensor& tcsr_col, Tensor& tcsr_val, Tensor& fcsr_tok, Tensor& fcsr_val, const OptTensor& fired, int64_t sort_segments,
-               int64_t col_pitch) {
+               int64_t col_pitch, const OptTensor& layer_cnt) {
   need(ent_tok, at::kInt, "ent_tok"); need(ctl, at::kLong, "ctl");
   need(tok_cnt, at::kInt, "tok_cnt"); need(feat_cnt, at::kInt, "feat_cnt"); need(tok_off, at::kInt, "tok_off"); need(feat_off, at::kInt, "feat_off");
   TORCH_CHECK(tok_off.numel() >= num_tokens + 1 && feat_off.numel() >= num_cols + 1, "offset arrays too small");
@@ -451,6 +452,11 @@ void build_csr(const Tensor& ent_tok, const Tensor& ent_col, const Tensor& ent_v
   a.sort_segments = int(sort_segments);
   a.col_pitch = int(col_pitch);
   TORCH_CHECK(col_pitch > 0 && col_pitch < (1 << 24), "col_pitch must be in (0, 2^24)");
+  a.layer_cnt = opt_ptr<int>(layer_cnt);
+  if (a.layer_cnt != nullptr) {
+    need(*layer_cnt, at::kInt, "layer_cnt");
+    TORCH_CHECK(layer_cnt->numel() >= (num_cols + col_pitch - 1) / col_pitch, "layer_cnt too small");
+  }
   c10::cuda::CUDAGuard guard(ent_tok.device());
   check(clt_build_csr(&a, cur_stream()), "build_csr");
 }
@@ -472,8 +478,9 @@ void build_token_csr(const Tensor& ent_tok, const Tensor& ent_col, const Tensor&
   a.num_tokens = int(num_tokens); a.num_cols = int(num_cols); a.col_pitch = int(col_pitch);
   a.tok_cnt = tok_cnt.data_ptr<int>(); a.tok_off = tok_off.data_ptr<int>(); a.tok_cursor = tok_cursor.data_ptr<int>();
   a.tcsr_col = tcsr_col.data_ptr<int>(); a.tcsr_val = tcsr_val.data_ptr<float>();
+  a.layer_cnt = layer_cnt.data_ptr<int>();
   c10::cuda::CUDAGuard guard(ent_tok.device());
-  check(clt_build_token_csr(&a, layer_cnt.data_ptr<int>(), cur_stream()), "build_token_csr");
+  check(clt_build_token_csr(&a, cur_stream()), "build_token_csr");
 }
 
 void dead_counter_update(Tensor& counter, Tensor& fired) {
@@ -1015,7 +1022,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("token_topk_tp", &token_topk_tp);
   m.def("theta_grad_gemm", &theta_grad_gemm, py::arg("gs"), py::arg("dec_w"), py::arg("preact"), py::arg("theta"), py::arg("bandwidth"),
         py::arg("S1"), py::arg("S2"), py::arg("status"), py::arg("tying") = 0, py::arg("gs_cum") = none);
-  m.def("build_csr", &build_csr);
+  m.def("build_csr", &build_csr, py::arg("ent_tok"), py::arg("ent_col"), py::arg("ent_val"), py::arg("ctl"), py::arg("num_tokens"), py::arg("num_cols"),
+        py::arg("tok_cnt"), py::arg("feat_cnt"), py::arg("tok_off"), py::arg("feat_off"), py::arg("tok_cursor"), py::arg("feat_cursor"),
+        py::arg("tcsr_col"), py::arg("tcsr_val"), py::arg("fcsr_tok"), py::arg("fcsr_val"), py::arg("fired"), py::arg("sort_segments"),
+        py::arg("col_pitch"), py::arg("layer_cnt") = none);
   m.def("build_token_csr", &build_token_csr);
   m.def("dead_counter_update", &dead_counter_update);
   m.def("sparse_decode", &sparse_decode, py::arg("dec_w"), py::arg("L"), py::arg("B"), py::arg("d"), py::arg("col_pitch"), py::arg("tying"),

@@ -1606,7 +1606,12 @@ __global__ void __launch_bounds__(256) csr_scatter_kernel(const int* __restrict_
                                                             const long long* __restrict__ ctl, int* __restrict__ tok_cursor,
                                                             int* __restrict__ feat_cursor, int* __restrict__ tcsr_col,
                                                             float* __restrict__ tcsr_val, int* __restrict__ fcsr_tok,
-                                                            float* __restrict__ fcsr_val, int col_pitch, int num_tokens, int num_cols) {
+                                                            float* __restrict__ fcsr_val, int col_pitch, int num_tokens, int num_cols,
+                                                            const int* __restrict__ feat_off, int* __restrict__ layer_cnt) {
+  if (layer_cnt != nullptr && blockIdx.x == 0) {  // entries per layer: the offsets are complete
+    for (int l = threadIdx.x; 1LL * l * col_pitch < num_cols; l += blockDim.x)
+      layer_cnt[l] = feat_off[min(1LL * (l + 1) * col_pitch, 1LL * num_cols)] - feat_off[1LL * l * col_pitch];
+  }
   long long n = ctl[CTL_NUM_ENTRIES];
   if (n > cap) n = cap;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
@@ -2247,6 +2252,7 @@ struct CltCsrArgs {
   unsigned char* fired;               // optional [num_cols]
   int sort_segments;                  // bit 0: token segments, bit 1: feature segments
   int col_pitch;                      // columns are layer * col_pitch + feature (feature < 2^24)
+  int* layer_cnt;                     // optional: entries per layer
 };
 
 // Features per CTA: as many as fill half of the shared buffer when the list is full, so that small dictionaries with long
@@ -2264,7 +2270,7 @@ extern "C" int clt_build_csr(const CltCsrArgs* a, cudaStream_t st) {
                                            a->num_tokens, a->num_cols);
   launch_exclusive_scans({a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens}, {a->feat_cnt, a->feat_off, a->feat_cursor, a->num_cols}, st);
   csr_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->feat_cursor,
-                                             a->tcsr_col, a->tcsr_val, a->fcsr_tok, a->fcsr_val, a->col_pitch, a->num_tokens, a->num_cols);
+                                             a->tcsr_col, a->tcsr_val, a->fcsr_tok, a->fcsr_val, a->col_pitch, a->num_tokens, a->num_cols, a->feat_off, a->layer_cnt);
   if ((a->sort_segments & 1) && a->num_tokens > 0)
     csr_sort_token_segments_kernel<<<a->num_tokens, 256, 0, st>>>(a->tok_off, a->tcsr_col, a->tcsr_val);
   if (a->sort_segments & 2) launch_feature_sort(a->feat_off, a->num_cols, a->ent_cap, a->fcsr_tok, a->fcsr_val, st);
@@ -2272,11 +2278,11 @@ extern "C" int clt_build_csr(const CltCsrArgs* a, cudaStream_t st) {
 }
 
 // tok_cnt and layer_cnt are zeroed by the caller, as the counters of clt_build_csr are.
-extern "C" int clt_build_token_csr(const CltCsrArgs* a, int* layer_cnt, cudaStream_t st) {
+extern "C" int clt_build_token_csr(const CltCsrArgs* a, cudaStream_t st) {
   if (a->num_tokens <= 0) return 0;
   if ((a->num_cols + a->col_pitch - 1) / a->col_pitch > 32) return -1;
   const int blocks = int((a->ent_cap + 255) / 256 < 592 ? (a->ent_cap + 255) / 256 : 592);
-  csr_token_count_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_cap, a->ctl, a->tok_cnt, layer_cnt, a->col_pitch, a->num_tokens, a->num_cols);
+  csr_token_count_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_cap, a->ctl, a->tok_cnt, a->layer_cnt, a->col_pitch, a->num_tokens, a->num_cols);
   const ScanJob job{a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens}, none{nullptr, nullptr, nullptr, 0};
   const int tiles = (a->num_tokens + 4095) / 4096;
   if (tiles <= 512 && (reinterpret_cast<uintptr_t>(a->tok_cnt) & 15) == 0) exclusive_scan_tiles_kernel<<<tiles, 1024, 0, st>>>(job, none, tiles);
@@ -2355,7 +2361,7 @@ extern "C" int clt_build_csr_static(const int* ent_tok, const int* ent_col, cons
   exclusive_scan_kernel<<<1, 1024, 0, stream>>>(tok_cnt, tok_off, tok_cursor, num_tokens);
   exclusive_scan_kernel<<<1, 1024, 0, stream>>>(feat_cnt, feat_off, feat_cursor, num_cols);
   csr_scatter_kernel<<<blocks, 256, 0, stream>>>(ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cursor, feat_cursor, tcsr_col, tcsr_val,
-                                                 fcsr_tok, fcsr_val, col_pitch, num_tokens, num_cols);
+                                                 fcsr_tok, fcsr_val, col_pitch, num_tokens, num_cols, feat_off, nullptr);
   if (sort_segments & 1) csr_sort_token_segments_kernel<<<num_tokens, 256, 0, stream>>>(tok_off, tcsr_col, tcsr_val);
   if (sort_segments & 2) launch_feature_sort(feat_off, num_cols, ent_cap, fcsr_tok, fcsr_val, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;

@@ -18,6 +18,7 @@ callers use ``CrossLayerTranscoder.forward`` for those.
 """
 from __future__ import annotations
 
+import threading
 from typing import Dict, Optional
 
 import torch
@@ -98,20 +99,22 @@ class SparseForward:
         # scan over them takes 21 us instead of 16 at 12 x 24576 features.  The loss sums come last, because only `reconstruct`
         # clears them.
         self.hist = torch.zeros(2 * 8192 + 32, dtype=i32, device=dev) if self.fn == "batchtopk" else None
-        # Order: feature counters (only where that view is built), token and layer counters, loss sums.
+        # Order: feature counters (cleared only where that view is built), token and layer counters, loss sums.
         starts = [0]
         for n in (ncols, B, L):
             starts.append((starts[-1] + n + 63) // 64 * 64)
         self._zeroed = torch.zeros(starts[-1] + 2 * L, dtype=i32, device=dev)
         self._zeroed_encode, self._zeroed_token = self._zeroed[: starts[-1]], self._zeroed[starts[1]:]
-        self.feat_cnt, self.tok_cnt = self._zeroed[:ncols], self._zeroed[starts[1]: starts[1] + B]
+        self._feat_cnt, self.tok_cnt = self._zeroed[:ncols], self._zeroed[starts[1]: starts[1] + B]
         self.layer_cnt = self._zeroed[starts[2]: starts[2] + L]
         self.sq_err = self._zeroed[starts[-1]:].view(torch.float64)
-        self._feature_view = False  # whether the feature-major arrays belong to the last selection
+        # see `_features`
+        self._features_read = self._features_due = False
+        self._lock = threading.RLock()
         self.tok_off = torch.zeros(B + 1, dtype=i32, device=dev)
         self._feat_off = torch.zeros(ncols + 1, dtype=i32, device=dev)
         self.tok_cursor = torch.zeros(B, dtype=i32, device=dev)
-        self.feat_cursor = torch.zeros(ncols, dtype=i32, device=dev)
+        self._feat_cursor = torch.zeros(ncols, dtype=i32, device=dev)
         self.tcsr_col = torch.zeros(cap, dtype=i32, device=dev)
         self.tcsr_val = torch.zeros(cap, dtype=f32, device=dev)
         self._fcsr_tok = torch.zeros(cap, dtype=i32, device=dev)
@@ -144,25 +147,44 @@ class SparseForward:
     def encode(self, X: torch.Tensor, clear_loss: bool = False, sort_tokens: bool = True) -> None:
         """Pre-activations, selection and the token-major / feature-major CSR views of the active entries.  ``sort_tokens``: a token's
         entries ordered by (layer, feature), which the decode wants; whoever reads the feature-major view alone can do without."""
-        self._select(X)
-        (self._zeroed if clear_loss else self._zeroed_encode).zero_()
-        self._build_views(sort_tokens)
+        with self._lock:
+            self._select(X)
+            self._build_views(clear_loss, sort_tokens)
+            if not self._capturing():
+                self._features_due = False
 
-    def _build_views(self, sort_tokens: bool = True) -> None:
-        self.ext.build_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.feat_cnt, self.tok_off,
-                           self._feat_off, self.tok_cursor, self.feat_cursor, self.tcsr_col, self.tcsr_val, self._fcsr_tok, self._fcsr_val,
-                           None, 3 if sort_tokens else 2, self.Fl)
-        self._feature_view = True
+    def _build_views(self, clear_loss: bool = False, sort_tokens: bool = True) -> None:
+        (self._zeroed if clear_loss else self._zeroed_encode).zero_()
+        self.ext.build_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self._feat_cnt, self.tok_off,
+                           self._feat_off, self.tok_cursor, self._feat_cursor, self.tcsr_col, self.tcsr_val, self._fcsr_tok, self._fcsr_val,
+                           None, 3 if sort_tokens else 2, self.Fl, self.layer_cnt)
+
+    def _capturing(self) -> bool:
+        """Whether calls on this device are being recorded into a graph (taken as true where the current device is another one)."""
+        return self.dev.index not in (None, torch.cuda.current_device()) or torch.cuda.is_current_stream_capturing()
 
     def _features(self, name: str) -> torch.Tensor:
-        """An array of the feature-major view of the last selection.  ``reconstruct`` reads the token-major view alone and does not
-        build the other; it is built from the entry list when somebody asks for it."""
-        if not self._feature_view:
-            self._zeroed_encode.zero_()
-            self._build_views()
-        return getattr(self, name)
+        """An array of the feature-major view.  It belongs to the last selection, as every other array here does, also for a caller that
+        holds it over several calls.  ``reconstruct`` itself reads the token-major view alone and leaves this one out (a fifth of a
+        16-token call) until somebody has asked for one of its arrays: only a caller that has asked before can hold one.  A call that is
+        recorded into a graph always fills it, because nothing here learns of a replay.  The first read after calls that left it out
+        builds it; which streams the list came from and the reader uses is not known here, so that read waits for the device, once
+        in the life of the object."""
+        with self._lock:
+            self._features_read = True
+            if self._features_due:
+                if self._capturing():
+                    self._build_views()  # recorded: every replay builds it from the list of that moment
+                else:
+                    torch.cuda.synchronize(self.dev)
+                    self._build_views()
+                    torch.cuda.synchronize(self.dev)
+                    self._features_due = False
+            return getattr(self, name)
 
     feat_off = property(lambda self: self._features("_feat_off"))
+    feat_cnt = property(lambda self: self._features("_feat_cnt"))
+    feat_cursor = property(lambda self: self._features("_feat_cursor"))
     fcsr_tok = property(lambda self: self._features("_fcsr_tok"))
     fcsr_val = property(lambda self: self._features("_fcsr_val"))
 
@@ -182,17 +204,26 @@ class SparseForward:
                                 self.ent_val, self.status)
         else:
             e.threshold_select(self.preact, self._theta(), self.Fl, self.Fl, self.ctl, self.ent_tok, self.ent_col, self.ent_val, self.status)
+
+    def _select_for_decode(self, X: torch.Tensor) -> None:
+        """Selection and the token-major view; the feature-major one too where somebody may be holding it (see ``_features``)."""
+        with self._lock:
+            if self._features_read or self._capturing():
+                self.encode(X, clear_loss=True)
+                return
+            self._select(X)
+            self._zeroed_token.zero_()
+            self.ext.build_token_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.tok_off,
+                                     self.tok_cursor, self.tcsr_col, self.tcsr_val, self.layer_cnt, self.Fl)
+            self._features_due = True
+
     # ------------------------------------------------------------------ decode
     @torch.no_grad()
     def reconstruct(self, X: torch.Tensor, Y: Optional[torch.Tensor] = None, sigma: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Reconstructions ``[L, B, d]`` (fp32).  With targets ``Y`` the per-layer sums of squared errors
         (scaled by ``sigma [L, d]`` when given) are left in ``self.sq_err``."""
-        self._select(X)
-        self._zeroed_token.zero_()
-        self._feature_view = False
+        self._select_for_decode(X)
         e, m = self.ext, self.model
-        e.build_token_csr(self.ent_tok, self.ent_col, self.ent_val, self.ctl, self.B, self.ncols, self.tok_cnt, self.tok_off, self.tok_cursor,
-                          self.tcsr_col, self.tcsr_val, self.layer_cnt, self.Fl)
         yhat = torch.empty(self.L, self.B, self.d, dtype=torch.float32, device=self.dev)
         bias = m.dec_bias.data
         if bias.dtype not in (torch.bfloat16, torch.float16, torch.float32) or not bias.is_contiguous():
@@ -231,12 +262,8 @@ class SparseForward:
         return int(self.ctl[3].item())
 
     def l0_per_layer(self) -> torch.Tensor:
-        """Mean number of active features per token and layer of the last ``encode``."""
-        if self._feature_view:
-            per_layer = (self.feat_off[1:] - self.feat_off[:-1]).view(self.L, self.Fl).sum(dim=1)
-        else:
-            per_layer = self.layer_cnt
-        return per_layer.float() / self.B
+        """Mean number of active features per token and layer of the last selection."""
+        return self.layer_cnt.float() / self.B
 
     def activations_dense(self) -> torch.Tensor:
         """Dense ``[L, B, F]`` activations of the last ``encode`` (testing)."""

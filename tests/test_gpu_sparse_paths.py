@@ -259,6 +259,117 @@ def test_views_after_a_reconstruction(ext, fn):
     sf.check_status()
 
 
+FEATURE_VIEW = ("feat_off", "feat_cnt", "feat_cursor", "fcsr_tok", "fcsr_val")
+
+
+def _views(sf):
+    """Copies of both views and the counts per layer; the arrays as long as the entry list end where its entries do."""
+    n = sf.num_entries()
+    return [getattr(sf, k)[: n if "csr" in k else None].clone() for k in ("tok_off", "tcsr_col", "tcsr_val") + FEATURE_VIEW] + [sf.l0_per_layer()]
+
+
+def _encoded(model, B, x):
+    """The views of a selection by ``encode`` on an object of its own."""
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    sf = SparseForward(model, B)
+    sf.encode(x)
+    return _views(sf)
+
+
+def _batches(n, dev, B=200, seed=0):
+    g = torch.Generator(device=dev).manual_seed(seed)
+    return [torch.randn(3, B, 64, device=dev, generator=g).bfloat16() for _ in range(n)]
+
+
+@pytest.mark.parametrize("fn", ["batchtopk", "topk", "jumprelu"])
+@pytest.mark.parametrize("taken", ["at the start", "after a call"])
+def test_held_feature_arrays_follow_the_calls(ext, fn, taken):
+    """The feature-major arrays are buffers: whoever holds one has the last selection in it, whichever call made it."""
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model(fn, "none", dev)
+    sf = SparseForward(model, 200)
+    x = _batches(3, dev)
+    if taken == "after a call":
+        sf.reconstruct(x[2])
+    held = {k: getattr(sf, k) for k in FEATURE_VIEW}
+    for b in x:
+        sf.reconstruct(b)
+        want, n = _encoded(model, 200, b), sf.num_entries()
+        for k, w in zip(FEATURE_VIEW, want[3:]):
+            assert torch.equal(held[k][: n if "csr" in k else None], w), k
+        assert all(torch.equal(a, b) for a, b in zip(_views(sf), want))
+
+
+@pytest.mark.parametrize("fn", ["batchtopk", "topk", "jumprelu"])
+@pytest.mark.parametrize("read_before", [False, True])
+def test_feature_view_after_graph_replays(ext, fn, read_before):
+    """Replays of a recorded ``reconstruct``: the views and the counts per layer are those of the replay, before and after the first read
+    and next to eager calls."""
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model(fn, "none", dev)
+    sf = SparseForward(model, 200)
+    x = _batches(4, dev)
+    inp = x[0].clone()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        sf.reconstruct(inp)  # warm-up
+    torch.cuda.current_stream().wait_stream(side)
+    if read_before:
+        sf.feat_off
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        sf.reconstruct(inp)
+    l0 = []
+    for step, b in enumerate(x[1:] + x[:2]):
+        if step == 2:
+            sf.reconstruct(x[0])  # an eager call in between
+            assert all(torch.equal(a, w) for a, w in zip(_views(sf), _encoded(model, 200, x[0])))
+        inp.copy_(b)
+        graph.replay()
+        l0.append(sf.l0_per_layer())
+        if step != 0:  # the first replay passes without a read of the feature-major view
+            assert all(torch.equal(a, w) for a, w in zip(_views(sf), _encoded(model, 200, b)))
+        assert torch.equal(l0[-1], _encoded(model, 200, b)[-1])
+    sf.check_status()
+
+
+def test_feature_view_read_inside_a_recording_and_on_another_stream(ext):
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    model = _serving_model("batchtopk", "none", dev)
+    x = _batches(2, dev, seed=1)
+    want = [_encoded(model, 200, b) for b in x]
+    sf = SparseForward(model, 200)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            sf.reconstruct(x[1])
+        sf.reconstruct(x[0])
+    off = sf.feat_off  # taken on the current stream while the calls run on the other one
+    side.synchronize()
+    assert torch.equal(off, want[0][3])
+    # a recording that only reads, behind an eager call that left the view out: each replay reads the list of its moment
+    sf = SparseForward(model, 200)
+    sf.reconstruct(x[0])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        copy = sf.feat_off.clone()
+    graph.replay()
+    assert torch.equal(copy, want[0][3])
+    sf.reconstruct(x[1])
+    graph.replay()
+    assert torch.equal(copy, want[1][3])
+
+
 def test_equal_keys_in_a_token_segment_are_all_kept(ext):
     """A caller's list may name one column twice for a token: both entries stay."""
     dev = _dev()
