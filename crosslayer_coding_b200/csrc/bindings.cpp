@@ -369,6 +369,15 @@ void token_topk_select(const Tensor& x, const Tensor& mean, const Tensor& rstd, 
   check(CLT_PICK(half, clt_token_topk_select)(&a, scratch.defined() ? scratch.data_ptr() : nullptr, cur_stream()), "token_topk_select");
 }
 
+// Bytes of scratch that the selection of k of L * F columns for B tokens allocates; 0: a form that needs none, or a call that is refused.
+int64_t token_topk_scratch(int64_t L, int64_t B, int64_t F, int64_t k) {
+  TORCH_CHECK(L >= 0 && B >= 0 && F >= 0 && L < (1 << 30) && B < (1LL << 31) && F < (1LL << 31), "sizes out of range");
+  CltSelectArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.L = int(L); a.B = int(B); a.F = int(F); a.k_total = k;
+  return clt_token_topk_scratch(&a);  // the same for both 16-bit types
+}
+
 // One phase of the TokenTopK selection across feature shards (0: push the local candidates' keys to the token owners,
 // 1: owners find the cut of their tokens and publish it, 2: keep the candidates at or above the cut).  The caller separates
 // the phases with peer barriers.  cand_* [B * k]: the local top k of every token (token_topk_select into scratch lists).
@@ -1019,6 +1028,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("threshold_select", &threshold_select);
   m.def("token_topk_select", &token_topk_select, py::arg("x"), py::arg("mean"), py::arg("rstd"), py::arg("col_pitch"), py::arg("k"), py::arg("ctl"),
         py::arg("ent_tok"), py::arg("ent_col"), py::arg("ent_val"), py::arg("status"), py::arg("f_valid") = 0);
+  m.def("token_topk_scratch", &token_topk_scratch, py::arg("L"), py::arg("B"), py::arg("F"), py::arg("k"));
   m.def("token_topk_tp", &token_topk_tp);
   m.def("theta_grad_gemm", &theta_grad_gemm, py::arg("gs"), py::arg("dec_w"), py::arg("preact"), py::arg("theta"), py::arg("bandwidth"),
         py::arg("S1"), py::arg("S2"), py::arg("status"), py::arg("tying") = 0, py::arg("gs_cum") = none);

@@ -2058,7 +2058,7 @@ constexpr long long kWideElements = 1LL << 28;
 static WideTopk wide_topk(const CltSelectArgs* a, long long k) {
   WideTopk w = {};
   w.groups = a->L * (a->F / 8);
-  if (1LL * a->B * a->L * a->F < kWideElements || k > 512) return w;
+  if (k <= 0 || 1LL * a->B * a->L * a->F < kWideElements || k > 512) return w;
   w.cap = k <= 64 ? 1024 : 2048;
   int step = int(w.cap / 2 / k);
   step = step > 8 ? 8 : step;
@@ -2075,7 +2075,7 @@ static WideTopk wide_topk(const CltSelectArgs* a, long long k) {
 // Bytes of scratch that clt_token_topk_select uses in its wide form (0: none).
 extern "C" long long CLT_FN(clt_token_topk_scratch)(const CltSelectArgs* a) {
   const WideTopk w = wide_topk(a, a->k_total);
-  if (w.step == 0 || a->k_total <= 0) return 0;
+  if (w.step == 0) return 0;
   return 1LL * a->B * (8LL * w.cap + 4LL * w.ng + 8);
 }
 

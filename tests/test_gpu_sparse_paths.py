@@ -501,6 +501,16 @@ def test_token_topk_of_large_matrices_with_values_that_are_not_finite(ext):
     assert torch.equal(got[0], torch.cat([w[0] for w in want])) and got[1] == max(w[1] for w in want)
 
 
+@pytest.mark.parametrize("L,B,F", [(2, 40, 64), (6, 2048, 8192), (6, 2048, 32768)])  # the last one is large enough for the four passes
+@pytest.mark.parametrize("k", [0, -1, -(1 << 40)])
+def test_token_topk_refuses_a_count_that_is_not_positive(ext, L, B, F, k):
+    dev = _dev()
+    x = torch.zeros(L, B, F, dtype=torch.bfloat16, device=dev)
+    z = lambda n, dt=I32: torch.zeros(n, dtype=dt, device=dev)  # noqa: E731
+    with pytest.raises(RuntimeError):
+        ext.token_topk_select(x, z((L, F), F32), z((L, F), F32), F, k, z(16, torch.int64), z(B), z(B), z(B, F32), z(4), F)
+
+
 def _serving_model(fn, tying, dev, L=3, d=64, F=512):
     from crosslayer_coding_b200 import CLTConfig, CrossLayerTranscoder
 
