@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
     float norm2 = 0.f, pc = 0.f;
     for (int i = 0; i < n; ++i) {
       const int st = i % ns;
-      if (!mbar_wait(&sh->full[st], (i / ns) & 1, abort_flag)) break;
+      if (!mbar_wait_warp(&sh->full[st], (i / ns) & 1, abort_flag)) break;
       uint8_t* stage = ring + size_t(st) * stage_bytes;
       const AdamStageHdr* h = reinterpret_cast<const AdamStageHdr*>(stage);
       const int ne = h->ne, r = h->r, R = h->R, col = h->col, ti = h->ti, b = h->b;
@@ -944,7 +944,7 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
     const int col = cur.ti * Fp + cur.f;
     float pc = p.pen_coef ? __ldg(p.pen_coef + col) : 0.f;
     if (PT && p.pen_coef) pc = warp_sum(lane <= cur.ti ? __ldg(p.pen_coef + lane * Fp + cur.f) : 0.f);  // the row is part of the norms of all sources
-    if (!mbar_wait(&full[st], (i / kNarrowStages) & 1, abort_flag)) { ok = false; break; }
+    if (!mbar_wait_warp(&full[st], (i / kNarrowStages) & 1, abort_flag)) { ok = false; break; }
     uint8_t* stage = ring + size_t(st) * stage_bytes;
     t16* w_s = reinterpret_cast<t16*>(stage);
     float* m_s = reinterpret_cast<float*>(stage + w_bytes);

@@ -108,6 +108,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
   }
 }
+// The wait of a whole warp, all lanes with one verdict.  Every lane waits, and so sees what the barrier stands for; but
+// a lane can see the barrier turn while another has just seen the abort flag or its limit, and a warp that split there would stand at a
+// shuffle of some lanes and at the CTA's last barrier with the others, without a limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag));
+}
 
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

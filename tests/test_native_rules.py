@@ -1,4 +1,5 @@
 """Host-side rules of the native library, which need no GPU: sizes at which a call takes another form or is refused."""
+import re
 import subprocess
 import sys
 from pathlib import Path
@@ -24,3 +25,30 @@ def test_scratch_of_the_token_topk_for_any_count(ext, k):
     assert r.returncode == 0, r.stderr
     small, large = eval(r.stdout.strip().splitlines()[-1])
     assert small == 0 and (large > 0) == (k > 0)
+
+
+def _waits():
+    """(file, line, openers of the blocks around it) of every plain bounded wait on an mbarrier outside its helpers."""
+    for path in sorted((ROOT / "crosslayer_coding_b200" / "csrc").glob("*.cu")):
+        src = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"\bmbar_wait\(", src):
+            line = src[src.rfind("\n", 0, m.start()) + 1: src.find("\n", m.start())].strip()
+            around, depth = [], 0
+            for i in range(m.start() - 1, -1, -1):
+                if src[i] == "}":
+                    depth += 1
+                elif src[i] == "{" and depth:
+                    depth -= 1
+                elif src[i] == "{":
+                    around.append(src[max(src.rfind(c, 0, i) for c in ";{}") + 1: i].strip())
+            yield path.name, line, around
+
+
+def test_bounded_waits_do_not_split_a_warp():
+    """A lane that gives up at a bounded wait must not leave the others of its warp at a shuffle: a plain wait belongs to one thread, which
+    goes on alone or shares the verdict; a whole warp waits through ``mbar_wait_warp``."""
+    one_thread = re.compile(r"\b(lane|tid|etid) == \w+")
+    waits = list(_waits())
+    assert len(waits) > 10
+    split = [(name, line) for name, line, around in waits if not one_thread.search(line) and not any(one_thread.search(a) for a in around)]
+    assert not split, split
