@@ -115,6 +115,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
   if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
   return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag));
 }
+// The wait of a whole warp by its first lane.  The shuffle hands the verdict on but orders no memory; with __syncwarp behind it what the first
+// lane saw at the barrier is seen by every lane.
+__device__ __forceinline__ bool mbar_wait_leader(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int lane) {
+  int landed = 0;
+  if (lane == 0) landed = mbar_wait(bar, parity, abort_flag) ? 1 : 0;
+  landed = __shfl_sync(0xFFFFFFFFu, landed, 0);
+  __syncwarp();
+  return landed != 0;
+}
 
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -287,9 +287,7 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         named_barrier_sync(1, kEpiThreads);
         ok = sh->epi_ok != 0;
       } else {
-        int landed = 0;
-        if (lane == 0) landed = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-        ok = __shfl_sync(0xFFFFFFFFu, landed, 0) != 0;
+        ok = mbar_wait_leader(&sh->tmem_full[buf], tph, abort_flag, lane);
       }
       if (!ok) break;
       tc_fence_after();
@@ -483,9 +481,7 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         named_barrier_sync(1, kEpiThreads);
         ok = sh->epi_ok != 0;
       } else {
-        int landed = 0;
-        if (lane == 0) landed = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-        ok = __shfl_sync(0xFFFFFFFFu, landed, 0) != 0;
+        ok = mbar_wait_leader(&sh->tmem_full[buf], tph, abort_flag, lane);
       }
       if (!ok) break;
       tc_fence_after();

@@ -46,9 +46,18 @@ def _waits():
 
 def test_bounded_waits_do_not_split_a_warp():
     """A lane that gives up at a bounded wait must not leave the others of its warp at a shuffle: a plain wait belongs to one thread, which
-    goes on alone or shares the verdict; a whole warp waits through ``mbar_wait_warp``."""
+    goes on alone or shares the verdict; a whole warp waits through ``mbar_wait_warp`` or, its first lane for all, ``mbar_wait_leader``."""
     one_thread = re.compile(r"\b(lane|tid|etid) == \w+")
     waits = list(_waits())
     assert len(waits) > 10
     split = [(name, line) for name, line, around in waits if not one_thread.search(line) and not any(one_thread.search(a) for a in around)]
     assert not split, split
+
+
+def test_a_verdict_that_one_lane_brings_home_is_ordered():
+    """What one lane saw at an mbarrier is not seen by the others through a shuffle alone: a lane's own verdict for its warp comes from
+    ``mbar_wait_leader``, which puts a ``__syncwarp`` behind it; a thread's for a whole CTA role through shared memory and a barrier."""
+    alone = [(name, line) for name, line, around in _waits() if re.search(r"\blane == 0\) \w+ = mbar_wait", line)]
+    assert not alone, alone
+    helper = (ROOT / "crosslayer_coding_b200" / "csrc" / "common.cuh").read_text().split("bool mbar_wait_leader(")[1].split("\n}")[0]
+    assert helper.index("mbar_wait(") < helper.index("__shfl_sync") < helper.index("__syncwarp")
