@@ -860,19 +860,20 @@ __global__ void __launch_bounds__(kTkThreads) token_topk_list_kernel(const t16* 
 // The list form for large matrices, in four passes.  The kernel above gives a CTA one to four tokens and reads the column statistics once
 // per such group: 64 bytes of statistics per 16 bytes of a token, a chain of a hundred dependent loads, 350 us at 6 x 2048 x 32768, k = 64;
 // the four passes take 302 (sample 46, bound 29, collect 206, cut 22).  Here a thread owns eight columns and walks 64 tokens, as the histogram scan does:
-//   sample   maxima of groups of eight columns, every step-th run of 32 groups, one word per group and token
+//   sample   maxima of groups of eight columns, every eighth run of 32 groups, one word per group and token
 //   bound    per token: a key that at least k of its maxima reach
-//   collect  one scan: what reaches the bound goes to the token's list (about step * k words)
+//   collect  one scan: what reaches the bound goes to the token's list (about 8 k words)
 //   cut      per token (one warp): the exact cut of the list, as above; a token whose list overflows goes to the radix kernel
 constexpr int kWideRows = 64;
 constexpr int kWideMaxima = 4096;   // per token
 constexpr int kWideQueue = 2048;    // groups of a tile that pass the coarse test, numbered with 16 bits
+constexpr int kWideStep = 8;        // one run of groups in kWideStep is sampled: a list has about kWideStep * k words
 struct WideTopk {
   int* n;                        // [B] list lengths (zeroed by the caller)
   uint32_t* bound;               // [B]
   uint32_t* maxima;              // [B][ng]
   unsigned long long* list;      // [B][cap] (key << 32 | inverted column)
-  int ng, cap, step, groups;
+  int ng, cap, groups;  // maxima per token (0: another form), room of a list, groups of eight columns
 };
 
 __device__ __forceinline__ float t16_of(const uint4& v, int j) {
@@ -883,7 +884,7 @@ __device__ __forceinline__ float t16_of(const uint4& v, int j) {
 __global__ void __launch_bounds__(256) token_sample_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
                                                              int f_valid, WideTopk wt) {
   const int sg = blockIdx.x * 256 + threadIdx.x;  // < ng, a multiple of 256
-  const int q = (sg >> 5) * 32 * wt.step + (sg & 31);  // runs of 32 groups: short enough that a sample meets every layer
+  const int q = (sg >> 5) * 32 * kWideStep + (sg & 31);  // runs of 32 groups: short enough that a sample meets every layer
   const int r0 = blockIdx.y * kWideRows, r1 = min(g.B, r0 + kWideRows);
   if (q >= wt.groups) {
     for (int r = r0; r < r1; ++r) wt.maxima[1LL * r * wt.ng + sg] = 0u;
@@ -2051,31 +2052,32 @@ static int launch_token_list(const CltSelectArgs* a, const ScanGeom& g, int f_va
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-// Geometry of the wide form, or step = 0 where it does not apply: at least kWideElements elements, and a sample of at least 4 k groups
-// whose expected list (step * k) takes half of its room.  6 x 2048 x 32768, k = 64: 351 us in one kernel, 302 here; 6 x 2048 x 8192, k = 24: about 100
-// and 148, the passes over tokens (bound, cut) do not shrink with the columns.
+// The wide form: 131072 to 262144 columns over all layers, at most one column in 2048 kept (so k <= 128), 2^28 elements or more.
+// One kernel / four passes, us:
+//   elements: 6 x 32768 columns, k = 16 and 64, 900 tokens (1.8e8) 167 / 155 and 204 / 199, 1100 (2.2e8) 170 / 167 and 210 / 214, 1400 (2.8e8)
+//     226 / 194 and 288 / 249, 2048 302 / 249 and 370 / 327, 8192 (k = 64) 1183 / 1114.  Below the line k = 90 is slower (1100 tokens 226 / 247,
+//     1300 263 / 276), above it is not (1400 314 / 292).
+//   columns: the passes over the tokens (bound, cut) do not shrink with them.  k = 24: 4 x 16384 x 4200 tokens 255 / 298, 12 x 8192 x 4096 321 / 331,
+//     4 x 32768 x 2100 239 / 224, 12 x 16384 x 2048 325 / 265, 12 x 20480 x 2048 380 / 298; 1 x 4096 x 65600, k = 1: 654 / 1189.  Above 262144 the
+//     maxima of a token (one in 64 columns) have no room in the bound pass.
+//   k: 6 x 32768 x 2048, k = 96: 411 / 414; 8 x 32768 x 2048, k = 128: 539 / 507.  A tile (64 tokens, 2048 columns) has room for four times the
+//     groups that are expected in it at the line; beyond it tokens would be lost to the radix kernel.
 constexpr long long kWideElements = 1LL << 28;
+constexpr long long kWideMinColumns = 1LL << 17, kWideMaxColumns = 1LL * kWideMaxima * 8 * kWideStep;
+static_assert(1LL * kWideRows * kWideStep * 4 <= kWideQueue, "a tile of 2048 columns at the line: one kept column in 2048, kWideStep candidates for each");
 static WideTopk wide_topk(const CltSelectArgs* a, long long k) {
   WideTopk w = {};
-  w.groups = a->L * (a->F / 8);
-  if (k <= 0 || 1LL * a->B * a->L * a->F < kWideElements || k > 512) return w;
-  w.cap = k <= 64 ? 1024 : 2048;
-  int step = int(w.cap / 2 / k);
-  step = step > 8 ? 8 : step;
-  const auto sampled = [&](int s) { return ((w.groups + 32 * s - 1) / (32 * s) * 32 + 255) / 256 * 256; };
-  while (step > 1 && sampled(step) < 4 * k) --step;
-  if (step < 1 || sampled(step) > kWideMaxima || sampled(step) < 4 * k) return w;
-  // a tile (64 tokens, 2048 columns) has room for four times the groups expected in it; where k is a larger share of the columns, tokens would
-  // be lost to the radix kernel (6 x 2048 x 8192, k = 64: 494 us)
-  if (1LL * kWideRows * step * k * 2048 > kWideQueue / 4 * 1LL * a->L * a->F) return w;
-  w.step = step;
-  w.ng = sampled(step);
+  const long long columns = 1LL * a->L * a->F;
+  if (k <= 0 || columns < kWideMinColumns || columns > kWideMaxColumns || 2048 * k > columns || a->B * columns < kWideElements) return w;
+  w.groups = int(columns / 8);
+  w.cap = k <= 64 ? 1024 : 2048;  // twice the expected list
+  w.ng = ((w.groups + 32 * kWideStep - 1) / (32 * kWideStep) * 32 + 255) / 256 * 256;
   return w;
 }
 // Bytes of scratch that clt_token_topk_select uses in its wide form (0: none).
 extern "C" long long CLT_FN(clt_token_topk_scratch)(const CltSelectArgs* a) {
   const WideTopk w = wide_topk(a, a->k_total);
-  if (w.step == 0) return 0;
+  if (w.ng == 0) return 0;
   return 1LL * a->B * (8LL * w.cap + 4LL * w.ng + 8);
 }
 
@@ -2095,7 +2097,7 @@ extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, void* scrat
   }
   const int grid = (a->B + kTokPerCta - 1) / kTokPerCta;
   const WideTopk shape = wide_topk(a, k);
-  const bool wide = shape.step > 0 && scratch != nullptr;
+  const bool wide = shape.ng > 0 && scratch != nullptr;
   const bool list = wide || k <= kTkMaxima / 2;
   if (wide) {
     WideTopk w = shape;

@@ -459,13 +459,15 @@ def test_token_topk_on_two_devices_of_one_process(ext):
         _check_token_topk(ext, x, mean, rstd, 8, 512, dev)
 
 
-# the four-pass form of large matrices: shard padding, columns and tokens that do not fill a tile, k on both sides of the two list sizes; values
-# with ties at the cut
+# the four-pass form of large matrices: shard padding, columns and tokens that do not fill a tile, the smallest and the largest number of columns, k on both
+# sides of the two list sizes and at its largest; and large matrices that keep the other forms (too few columns, too large a k, too many columns)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("L,B,Fl,F,k", [(3, 4400, 20488, 20481, 24), (4, 2050, 33000, 33000, 64), (8, 1030, 32768, 32760, 200), (8, 1029, 32776, 32776, 512)])
-def test_token_topk_of_large_matrices(ext, L, B, Fl, F, k, dtype):
+@pytest.mark.parametrize("L,B,Fl,F,k,passes", [(4, 2050, 32768, 32761, 64, True), (16, 1100, 16376, 16370, 24, True), (8, 1030, 32768, 32765, 65, True), (8, 1031, 32768, 32760, 100, True),
+                                               (8, 1029, 32768, 32761, 128, True), (3, 4400, 20488, 20481, 24, False), (8, 1030, 32768, 32760, 200, False),
+                                               (8, 1029, 32776, 32776, 512, False)])
+def test_token_topk_of_large_matrices(ext, L, B, Fl, F, k, passes, dtype):
     dev = _dev()
-    assert B * L * Fl >= 1 << 28
+    assert B * L * Fl >= 1 << 28 and (ext.token_topk_scratch(L, B, Fl, k) > 0) == passes
     g = torch.Generator(device=dev).manual_seed(k)
     x = (torch.randn(L, B, Fl, generator=g, device=dev) * 0.7 + 0.3 * torch.randn(L, 1, Fl, generator=g, device=dev)).to(dtype)
     mean = torch.stack([x[l].float().mean(0) for l in range(L)])
@@ -477,7 +479,8 @@ def test_token_topk_of_large_matrices_with_values_that_are_not_finite(ext):
     """A column with a NaN has NaN statistics and sorts above everything in every row, and infinities sort by their sign: as in the form for
     small matrices, which the same rows are put through a few at a time."""
     dev = _dev()
-    L, B, F, k = 2, 3328, 41000, 40
+    L, B, F, k = 4, 2048, 33000, 40
+    assert ext.token_topk_scratch(L, B, F, k) > 0  # the four passes; 256 rows at a time take the other form
     g = torch.Generator(device=dev).manual_seed(3)
     x = torch.randn(L, B, F, generator=g, device=dev).bfloat16()
     x[0, 7, 100] = float("nan")

@@ -27,6 +27,17 @@ def test_scratch_of_the_token_topk_for_any_count(ext, k):
     assert small == 0 and (large > 0) == (k > 0)
 
 
+# both sides of every line: elements, columns (fewest and most), count; and counts of list words and maxima by what the scratch holds
+@pytest.mark.parametrize("L,B,F,k,room", [(6, 1365, 32768, 64, 0), (6, 1366, 32768, 64, 1024), (4, 4096, 32760, 24, 0), (4, 4096, 32768, 24, 1024), (8, 2048, 32768, 24, 1024),
+                                          (8, 2048, 32776, 24, 0), (4, 4096, 32768, 64, 1024), (4, 4096, 32768, 65, 0), (8, 2048, 32768, 64, 1024), (8, 2048, 32768, 65, 2048),
+                                          (8, 2048, 32768, 128, 2048), (8, 2048, 32768, 129, 0), (1, 65600, 4096, 1, 0), (1, 1 << 22, 256, 1, 0)])
+def test_sizes_of_the_four_pass_token_topk(ext, L, B, F, k, room):
+    got = ext.token_topk_scratch(L, B, F, k)
+    maxima = -(-(-(-(L * F // 8) // 256) * 32) // 256) * 256  # one group of eight columns in eight, in whole blocks
+    assert got == (B * (8 * room + 4 * maxima + 8) if room else 0)
+    assert got <= B * L * F * 2 // 8  # an eighth of the matrix at most
+
+
 def _waits():
     """(file, line, openers of the blocks around it) of every plain bounded wait on an mbarrier outside its helpers."""
     for path in sorted((ROOT / "crosslayer_coding_b200" / "csrc").glob("*.cu")):
