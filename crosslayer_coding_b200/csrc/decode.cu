@@ -140,8 +140,14 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // twice the tokens on the chip.  4096 tokens, entries per token on average: 8 139 us with two and 174 with four, 16 182 and 213, 25 (one
 // eighth of the features) 191 and 224, 32 266 and 287, 66 436 and 437, 100 629 and 606.  Only the caller knows the average without a
 // host synchronisation (its k); a threshold selection does not, and counts as long.
-// Equally long lists (a per-token selection) gain nothing from four warps: 2048 tokens of 6 x 768, k = 64, 82 us with one warp and 100 with
-// four, 3536 of 4 x 856, k = 24, 71 and 104, 776 of 5 x 520, k = 24, 19 and 28.
+// Equally long lists (a per-token selection) gain nothing from four warps while they are short: 2048 tokens of 6 x 768, k = 64, 82 us with one warp
+// and 100 with four, 3536 of 4 x 856, k = 24, 71 and 104, 776 of 5 x 520, k = 24, 19 and 28.  Long ones (k = 200) do not either where the chip is full of
+// wide rows: 12 x 768, 1024 tokens 227 and 223, 2048 305 and 404, 8192 1128 and 1327; 16 x 2048, 128 tokens 125 and 127, 512 313 and 350; 8 x
+// 512, 4096 tokens of 8192 features 312 and 313, of 32768 385 and 444 (k = 400: 555 and 516, 665 and 722).  Running sums, k = 200: 1024 tokens of 6 x 512 76 and 57,
+// 4096 141 and 159, of 8 x 256 74 and 122; k = 400, 4096 tokens of 12 x 768 509 and 482, of 8 x 256 117 and 165.  Their order by length
+// says nothing: it is not formed.
+// Near-empty lists of a length that the caller does not know take four warps too: 12 x 768, 4096 tokens without an entry 114 us, where two warps take 92
+// and one 84.  Whoever knows that lists are short says so (the expected length).
 // Narrow rows: what a CTA costs by itself shows, above all its addition to the error sum (1.5 ns, all CTAs of a target on one
 // address): 12 x 6208 (token, target) pairs of 136 elements without an entry take 116 us with one token per CTA, 60 with two.  So with many
 // tokens one vector per lane goes two tokens and two warps each to a CTA (4096 tokens of 6 x 256, k = 64: 93 us either way).
@@ -155,7 +161,10 @@ constexpr int kRunningOrderFrom = 4096;        // tokens
 constexpr int kShortBelow = 64;                // entries per token on average
 constexpr long long kShortFrom = 16384;        // CTAs
 constexpr int kRunningOneWarpBelow = 32;         // entries per token on average
-constexpr int kOneWarpBelow = 128;               // entries of every token
+constexpr int kOneWarpBelow = 128;               // entries of every token; above, by one_warp_lists
+constexpr int kOneWarpMediumBelow = 256;        // entries of every token
+constexpr int kOneWarpRunningFrom = 2048;        // tokens
+constexpr long long kOneWarpWalkFrom = 16384, kOneWarpWideWalkFrom = 8192;  // CTAs; the second: four vectors per lane
 
 __device__ __forceinline__ int decode_token(const DecodeParams& p, int i) {
   // Tensor-parallel push: rank r starts with the tokens owned by rank r + 1, so that at any moment the ranks
@@ -582,11 +591,21 @@ static bool takes_running(const CltDecodeArgs* a) {
 }
 
 static long long walk_ctas(const CltDecodeArgs* a) { return 1LL * a->B * a->L * walk_chunks(a); }
+static int walk_vectors(const CltDecodeArgs* a) { return (a->d / 8 + 32 * walk_chunks(a) - 1) / (32 * walk_chunks(a)); }
 static bool short_lists(const CltDecodeArgs* a) { return a->expected > 0 && a->expected < kShortBelow; }
+// Lists of one length that a warp takes alone.
+static bool one_warp_lists(const CltDecodeArgs* a) {
+  if (a->equal == 0 || a->expected <= 0) return false;
+  if (a->expected < kOneWarpBelow) return true;
+  if (takes_running(a)) return a->B >= kOneWarpRunningFrom && (a->expected < kOneWarpMediumBelow || a->d <= 256);
+  const int nv = walk_vectors(a);
+  if (nv == 2) return walk_ctas(a) >= kOneWarpWalkFrom && a->expected < kOneWarpMediumBelow;
+  return nv >= 3 && walk_ctas(a) >= (nv == 3 ? kOneWarpWalkFrom : kOneWarpWideWalkFrom);
+}
 
 // Number of ints the call wants in `order`: the tokens are sorted by length where there are so many CTAs that it pays.
 extern "C" long long CLT_FN(clt_sparse_decode_scratch)(const CltDecodeArgs* a) {
-  if (a->mode == 2 || a->B <= 0 || short_lists(a)) return 0;
+  if (a->mode == 2 || a->B <= 0 || a->equal != 0 || short_lists(a)) return 0;
   if (takes_running(a)) return a->B >= kRunningOrderFrom ? a->B : 0;
   return a->d > 512 && walk_ctas(a) >= kManyCtas ? a->B : 0;
 }
@@ -613,8 +632,8 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   }
   if (takes_running(a)) {
     const dim3 grid(a->B, running_chunks(a));
-    if (a->expected > 0 && a->expected < (a->equal != 0 ? kOneWarpBelow : kRunningOneWarpBelow)) {
-      if (a->d <= 256) decode_running_kernel<1, 1, 4, 24><<<grid, 32, 0, st>>>(p);
+    if (one_warp_lists(a) || (a->equal == 0 && a->expected > 0 && a->expected < kRunningOneWarpBelow)) {
+      if (a->d <= 256) decode_running_kernel<1, 1, 4, 28><<<grid, 32, 0, st>>>(p);
       else decode_running_kernel<2, 1, 4, 16><<<grid, 32, 0, st>>>(p);
     } else if (short_lists(a)) {
       if (a->d <= 256) decode_running_kernel<1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
@@ -625,8 +644,7 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
-  const int chunks = walk_chunks(a);
-  const int nv = (a->d / 8 + 32 * chunks - 1) / (32 * chunks);
+  const int chunks = walk_chunks(a), nv = walk_vectors(a);
   const long long ctas = walk_ctas(a);
   const dim3 grid(a->B, a->L, chunks);
   if (ctas < kEightWarpsBelow) {
@@ -634,7 +652,7 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
     else if (nv == 2) decode_walk_kernel<2, 1, 8, 4, 24><<<grid, 256, 0, st>>>(p);
     else if (nv == 3) decode_walk_kernel<3, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
     else decode_walk_kernel<4, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
-  } else if (a->equal != 0 && a->expected > 0 && a->expected < kOneWarpBelow) {
+  } else if (one_warp_lists(a)) {
     if (nv <= 1) decode_walk_kernel<1, 4, 1, 4, 32><<<dim3((a->B + 3) / 4, a->L), 128, 0, st>>>(p);
     else if (nv == 2) decode_walk_kernel<2, 2, 1, 4, 24><<<dim3((a->B + 1) / 2, a->L), 64, 0, st>>>(p);
     else if (nv == 3) decode_walk_kernel<3, 1, 1, 2, 28><<<grid, 32, 0, st>>>(p);
@@ -642,7 +660,7 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   } else if (nv <= 1) {
     if (ctas >= kPairNarrowFrom) decode_walk_kernel<1, 2, 2, 4, 40><<<dim3((a->B + 1) / 2, a->L), 128, 0, st>>>(p);
     else decode_walk_kernel<1, 1, 4, 4, 40><<<grid, 128, 0, st>>>(p);
-  } else if (short_lists(a) && (a->equal != 0 || ctas >= kShortFrom) && nv >= 2) {
+  } else if (short_lists(a) && ctas >= kShortFrom) {
     if (nv == 2) decode_walk_kernel<2, 1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
     else if (nv == 3) decode_walk_kernel<3, 1, 2, 2, 28><<<grid, 64, 0, st>>>(p);
     else decode_walk_kernel<4, 1, 2, 2, 20><<<grid, 64, 0, st>>>(p);

@@ -161,6 +161,14 @@ def test_gather_decode_with_an_expected_length(ext, L, B, d, tying, expected, eq
     _check_decode(ext, L, B, d, tying, tying != 0, F=72, entries=_uneven_entries, expected=expected, equal=equal)
 
 
+# lists of one length of 128 and more entries: one warp or four per token on either side of the lines, without the order by length
+@pytest.mark.parametrize("tying", [0, 1, 2])
+@pytest.mark.parametrize("L,B,d", [(13, 1303, 520), (9, 1303, 520), (7, 2050, 1800), (3, 600, 1032), (13, 1303, 512), (4, 4100, 200)])
+@pytest.mark.parametrize("expected", [127, 200, 300])
+def test_gather_decode_of_equal_long_lists(ext, tying, L, B, d, expected):
+    _check_decode(ext, L, B, d, tying, False, F=72, entries=_uneven_entries, expected=expected, equal=True)
+
+
 @pytest.mark.parametrize("L,B,d", [(3, 1303, 200), (3, 1303, 512)])
 def test_gather_decode_of_equal_short_lists_in_narrow_rows(ext, L, B, d):
     _check_decode(ext, L, B, d, 0, False, F=72, entries=_uneven_entries, expected=20, equal=True)
