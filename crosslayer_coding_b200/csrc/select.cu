@@ -1756,16 +1756,21 @@ __global__ void __launch_bounds__(256) csr_sort_feature_segments_kernel(const in
 // Token segments: one CTA per token sorts its entries by (layer, feature).  Short lists: every thread counts how many keys are below
 // its own (broadcast reads of shared memory, no barrier in between: 1 us where the 36 barriers of a network on 256 entries take ten)
 // and stores its entry at that rank.  Longer ones: the entries are dealt into buckets by layer first, and an entry's place is the number of
-// entries in lower layers plus the number of smaller keys in its own bucket.  Long buckets (kTokenRankCap), or equal keys, go through the
+// entries in lower layers plus the number of smaller keys in its own bucket.  Long buckets (kTokenBucketCap), or equal keys, go through the
 // network in shared memory, and lists beyond its buffer through the one in global memory.  The order lets the decode's tokens pass over
 // the decoder rows together (L2) and fixes the order of its sums.
 // The buckets take a few more barriers and do n * n / layers instead of n * n comparisons: few tokens, where the latency of one CTA counts,
 // rank up to 512 entries (512 tokens of at most 352: 5.3 us against 10.0 with buckets; 16 tokens of up to 605: 16.4 us with the
 // network above 512, 9.1 with buckets); with many tokens the comparisons count (4096 tokens, 200 entries on average: 60 us with ranks up to
-// 512, 48 with buckets; 8192 tokens: 86 and 77; 4096 tokens of 25: 8.7 and 9.7).
+// 512, 48 with buckets; 8192 tokens: 86 and 77; 4096 tokens of 25: 8.7 and 9.7).  Lists that must have a bucket above the cap, because there are
+// not layers enough, go to the network directly (1024 tokens of 800 entries in two layers: 47 us, 49 behind a count of the buckets), and
+// with one layer there is one bucket: ranks up to 256 entries (4096 tokens of 200: 29 us, 38 as a bucket).
+// The bucket of layer l starts at bank l: the lanes of a warp read the buckets of their layers side by side, and where those lie by the lengths before
+// them they meet at few banks (1024 tokens of 2000 entries, up to 256 in each of eight layers: 594 us, with a bank for every layer 104).
 constexpr int kTokenSortCap = 2048;
-constexpr int kTokenRankCap = 256;
+constexpr int kTokenBucketCap = 256;
 constexpr int kTokenBuckets = 128;  // layers, as the packed key can number them
+constexpr int kTokenBucketRoom = kTokenSortCap + 32 * 31 + kTokenBuckets;  // every bucket of 32 layers with room to the next layer's bank
 constexpr int kFewTokens = 768;
 
 // Ranks over the whole list, M entries per thread; false when two keys are equal.
@@ -1802,7 +1807,7 @@ __device__ __forceinline__ bool rank_sort_segment(int* __restrict__ key, float* 
 
 // M entries per thread (n <= 256 M); false when the network has to sort them.
 template <int M>
-__device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float* __restrict__ val, int n, int* bucket, int* taken, int* count, int* base) {
+__device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float* __restrict__ val, int n, int* bucket, int* taken, int* count, int* base, int* start) {
   int mine[M], slot[M];
   float v[M];
   if (threadIdx.x < kTokenBuckets) count[threadIdx.x] = 0;
@@ -1820,22 +1825,29 @@ __device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float
   __syncthreads();
   bool network = false;
   if (threadIdx.x < 32) {
-    int c[4], sum = 0;
+    int c[4], sum = 0, room = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       c[k] = count[4 * threadIdx.x + k];
-      network |= c[k] > kTokenRankCap;
+      network |= c[k] > kTokenBucketCap;
       sum += c[k];
+      room += c[k] + ((1 - c[k]) & 31);
     }
-    int incl = sum;
+    int incl = sum, incl_room = room;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (int(threadIdx.x) >= o) incl += up;
+      const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o), up_room = __shfl_up_sync(0xFFFFFFFFu, incl_room, o);
+      if (int(threadIdx.x) >= o) { incl += up; incl_room += up_room; }
     }
-    int run = incl - sum;
+    network |= incl_room > kTokenBucketRoom;
+    int run = incl - sum, at = incl_room - room;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) { base[4 * threadIdx.x + k] = run; run += c[k]; }
+    for (int k = 0; k < 4; ++k) {
+      start[4 * threadIdx.x + k] = run;
+      base[4 * threadIdx.x + k] = at;
+      run += c[k];
+      at += c[k] + ((1 - c[k]) & 31);
+    }
   }
   if (__syncthreads_or(network)) return false;
 #pragma unroll
@@ -1848,7 +1860,7 @@ __device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float
     if (threadIdx.x + 256 * m < n) {
       const int l = (mine[m] >> 24) & (kTokenBuckets - 1);
       const int b = base[l], e = b + count[l];
-      int at = b;
+      int at = start[l];
       for (int j = b; j < e; ++j) at += bucket[j] < mine[m] ? 1 : 0;
       slot[m] = at;
       clash |= atomicExch(&taken[at], 1) != 0;
@@ -1861,28 +1873,37 @@ __device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float
   return true;
 }
 
-__global__ void __launch_bounds__(256) csr_sort_token_segments_kernel(const int* __restrict__ off, int* __restrict__ key, float* __restrict__ val) {
-  __shared__ __align__(16) unsigned long long w[kTokenSortCap];
-  __shared__ int count[kTokenBuckets], base[kTokenBuckets];
+__global__ void __launch_bounds__(256) csr_sort_token_segments_kernel(const int* __restrict__ off, int* __restrict__ key, float* __restrict__ val, int rank_up_to,
+                                                                         int bucket_up_to) {
+  __shared__ __align__(16) unsigned long long w[(kTokenBucketRoom + kTokenSortCap) / 2];
+  __shared__ int count[kTokenBuckets], base[kTokenBuckets], start[kTokenBuckets];
   const int b = off[blockIdx.x], n = off[blockIdx.x + 1] - b;
   if (n <= 1) return;
   if (n > kTokenSortCap) {
     sort_pairs_cta(key + b, val + b, n);
     return;
   }
-  int* bucket = reinterpret_cast<int*>(w);  // the buckets share the network's buffer: keys in the first half, marks in the second
-  int* taken = bucket + kTokenSortCap;
-  const bool done = n <= (gridDim.x < kFewTokens ? 512 : 128)
+  int* bucket = reinterpret_cast<int*>(w);  // the buckets share the network's buffer: keys first, marks behind them
+  int* taken = bucket + kTokenBucketRoom;
+  const bool done = n <= rank_up_to
                         ? (n <= 256 ? rank_sort_segment<1>(key + b, val + b, n, bucket, taken) : rank_sort_segment<2>(key + b, val + b, n, bucket, taken))
-                    : n <= 256  ? bucket_sort_segment<1>(key + b, val + b, n, bucket, taken, count, base)
-                    : n <= 512  ? bucket_sort_segment<2>(key + b, val + b, n, bucket, taken, count, base)
-                    : n <= 1024 ? bucket_sort_segment<4>(key + b, val + b, n, bucket, taken, count, base)
-                                : bucket_sort_segment<8>(key + b, val + b, n, bucket, taken, count, base);
+                    : n > bucket_up_to ? false
+                    : n <= 256         ? bucket_sort_segment<1>(key + b, val + b, n, bucket, taken, count, base, start)
+                    : n <= 512         ? bucket_sort_segment<2>(key + b, val + b, n, bucket, taken, count, base, start)
+                    : n <= 1024        ? bucket_sort_segment<4>(key + b, val + b, n, bucket, taken, count, base, start)
+                                       : bucket_sort_segment<8>(key + b, val + b, n, bucket, taken, count, base, start);
   if (done) return;
   __syncthreads();
   for (int i = threadIdx.x; i < n; i += blockDim.x) w[i] = pack_entry(key[b + i], val[b + i]);
   sort_words_cta(w, n);
   for (int i = threadIdx.x; i < n; i += blockDim.x) { key[b + i] = int(w[i] >> 32); val[b + i] = __uint_as_float((unsigned int)(w[i] & 0xFFFFFFFFULL)); }
+}
+
+static void launch_token_sort(const int* off, int* key, float* val, int num_tokens, int num_cols, int col_pitch, cudaStream_t st) {
+  if (num_tokens <= 0) return;
+  const int layers = (num_cols + col_pitch - 1) / col_pitch;
+  const int rank_up_to = num_tokens < kFewTokens ? 512 : (layers <= 1 ? 256 : 128);
+  csr_sort_token_segments_kernel<<<num_tokens, 256, 0, st>>>(off, key, val, rank_up_to, layers < 8 ? layers * kTokenBucketCap : kTokenSortCap);
 }
 
 // Dead-feature counters: +1 per step, reset where the feature fired (reference trainer.py:693-712).
@@ -2273,8 +2294,7 @@ extern "C" int clt_build_csr(const CltCsrArgs* a, cudaStream_t st) {
   launch_exclusive_scans({a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens}, {a->feat_cnt, a->feat_off, a->feat_cursor, a->num_cols}, st);
   csr_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->feat_cursor,
                                              a->tcsr_col, a->tcsr_val, a->fcsr_tok, a->fcsr_val, a->col_pitch, a->num_tokens, a->num_cols, a->feat_off, a->layer_cnt);
-  if ((a->sort_segments & 1) && a->num_tokens > 0)
-    csr_sort_token_segments_kernel<<<a->num_tokens, 256, 0, st>>>(a->tok_off, a->tcsr_col, a->tcsr_val);
+  if (a->sort_segments & 1) launch_token_sort(a->tok_off, a->tcsr_col, a->tcsr_val, a->num_tokens, a->num_cols, a->col_pitch, st);
   if (a->sort_segments & 2) launch_feature_sort(a->feat_off, a->num_cols, a->ent_cap, a->fcsr_tok, a->fcsr_val, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -2291,7 +2311,7 @@ extern "C" int clt_build_token_csr(const CltCsrArgs* a, cudaStream_t st) {
   else exclusive_scan_kernel<<<1, 1024, 0, st>>>(job.in, job.out, job.cursor, job.n);
   csr_token_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->tcsr_col, a->tcsr_val,
                                                    a->col_pitch, a->num_tokens, a->num_cols);
-  csr_sort_token_segments_kernel<<<a->num_tokens, 256, 0, st>>>(a->tok_off, a->tcsr_col, a->tcsr_val);
+  launch_token_sort(a->tok_off, a->tcsr_col, a->tcsr_val, a->num_tokens, a->num_cols, a->col_pitch, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -2364,7 +2384,7 @@ extern "C" int clt_build_csr_static(const int* ent_tok, const int* ent_col, cons
   exclusive_scan_kernel<<<1, 1024, 0, stream>>>(feat_cnt, feat_off, feat_cursor, num_cols);
   csr_scatter_kernel<<<blocks, 256, 0, stream>>>(ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cursor, feat_cursor, tcsr_col, tcsr_val,
                                                  fcsr_tok, fcsr_val, col_pitch, num_tokens, num_cols, feat_off, nullptr);
-  if (sort_segments & 1) csr_sort_token_segments_kernel<<<num_tokens, 256, 0, stream>>>(tok_off, tcsr_col, tcsr_val);
+  if (sort_segments & 1) launch_token_sort(tok_off, tcsr_col, tcsr_val, num_tokens, num_cols, col_pitch, stream);
   if (sort_segments & 2) launch_feature_sort(feat_off, num_cols, ent_cap, fcsr_tok, fcsr_val, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

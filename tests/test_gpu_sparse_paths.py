@@ -240,6 +240,24 @@ def test_token_view_alone(ext, B, L, F, n):
     assert torch.equal(per_layer.long(), torch.bincount((col // F).long(), minlength=L))
 
 
+# the same number of entries in every layer: one layer (ranks, then the network), too few layers for the buckets, buckets that all start at a multiple of 32
+# words, the longest buckets of every number of entries per thread, the last of the 128 layers a key can number
+@pytest.mark.parametrize("B,L,per_layer", [(800, 1, 200), (800, 1, 256), (800, 1, 300), (800, 2, 300), (800, 2, 64), (800, 2, 128), (800, 2, 256), (40, 4, 256), (40, 8, 256), (800, 8, 32),
+                                           (800, 16, 64), (40, 20, 100), (40, 128, 15), (800, 128, 3)])
+def test_token_segments_of_even_layers(ext, B, L, per_layer):
+    dev = _dev()
+    F = 320
+    g = torch.Generator().manual_seed(B + L + per_layer)
+    f = torch.stack([torch.randperm(F, generator=g)[:per_layer] for _ in range(B * L)])  # distinct features of a (token, layer)
+    row = torch.arange(B * L).repeat_interleave(per_layer)
+    tok, col = row // L, (row % L) * F + f.reshape(-1)
+    mix = torch.randperm(tok.numel(), generator=g)
+    tok, col, val = tok[mix].to(I32).to(dev), col[mix].to(I32).to(dev), torch.randn(tok.numel(), generator=g).to(dev)
+    c = _csr(ext, tok, col, val, B, L * F, F)
+    order = torch.argsort(tok.long() * L * F + col.long())
+    assert torch.equal(c["tcsr_col"], ((col[order] // F) << 24) | (col[order] % F)) and torch.equal(c["tcsr_val"], val[order])
+
+
 @pytest.mark.parametrize("fn", ["batchtopk", "topk", "jumprelu"])
 def test_views_after_a_reconstruction(ext, fn):
     """``reconstruct`` builds the token-major view; the feature-major one and the counts per layer are those of the same selection, and a
