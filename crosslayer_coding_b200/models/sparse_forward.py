@@ -49,7 +49,11 @@ def supports(model) -> Optional[str]:
 
 
 class SparseForward:
-    def __init__(self, model, batch_tokens: int, max_active_per_token: int = 2048):
+    def __init__(self, model, batch_tokens: int, max_active_per_token: int = 2048, expected_active_per_token: Optional[int] = None):
+        """``max_active_per_token``: room of the entry list of a threshold selection (a batch that needs more is reported, see
+        ``check_status``).  ``expected_active_per_token``: about how many entries a token has under such a selection; only the speed of the
+        decode depends on it (short lists take two warps per token instead of four: 4096 tokens of 12 x 768 without an entry 92 us instead
+        of 114).  Left out, lists count as long unless the room says that they are not."""
         reason = supports(model)
         if reason is not None:
             raise ValueError(f"SparseForward does not cover this model: {reason}")
@@ -75,7 +79,13 @@ class SparseForward:
         else:
             cap = int(min(B * L * Fl, max_active_per_token * B))
         self.cap = cap
-        self.expected_entries = self.k_total // max(B, 1) if self.fn in ("batchtopk", "topk") else 0  # per token; a threshold leaves it open
+        # entries per token, for the decode's choice of warps per token (0: not known)
+        if self.fn in ("batchtopk", "topk"):
+            self.expected_entries = self.k_total // max(B, 1)
+        elif expected_active_per_token is not None:
+            self.expected_entries = max(1, int(expected_active_per_token))
+        else:
+            self.expected_entries = max(1, int(max_active_per_token)) if max_active_per_token < 64 else 0
         self.preact = torch.empty(L, B, Fl, dtype=torch.bfloat16, device=dev)
         self.ctl = torch.zeros(16, dtype=torch.int64, device=dev)
         self.status = torch.zeros(4, dtype=i32, device=dev)

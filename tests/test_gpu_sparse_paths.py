@@ -303,6 +303,29 @@ def _encoded(model, B, x):
     return _views(sf)
 
 
+def test_expected_length_of_threshold_lists(ext):
+    """What the caller expects of the lists changes the order of the sums and nothing else; a small room says as much."""
+    from crosslayer_coding_b200.models.sparse_forward import SparseForward
+
+    dev = _dev()
+    B = 6000  # enough (token, target) pairs for two warps per token
+    model = _serving_model("jumprelu", "none", dev)
+    with torch.no_grad():
+        model.log_threshold.fill_(0.9)
+    x = _batches(1, dev, B)[0]
+    y = torch.randn(3, B, 64, device=dev).bfloat16()
+    runs = {}
+    for name, kw in (("open", {}), ("short", dict(expected_active_per_token=3)), ("none", dict(expected_active_per_token=0)), ("long", dict(expected_active_per_token=500)),
+                     ("room", dict(max_active_per_token=60))):
+        sf = SparseForward(model, B, **kw)
+        runs[name] = (sf.reconstruct(x, y), sf.sq_err.clone(), sf.expected_entries)
+        sf.check_status()
+    assert [r[2] for r in runs.values()] == [0, 3, 1, 500, 60]
+    scale = runs["open"][0].abs().max()
+    for yhat, sq, _ in runs.values():
+        assert (yhat - runs["open"][0]).abs().max() < 1e-5 * scale and torch.allclose(sq, runs["open"][1], rtol=1e-5)
+
+
 def _batches(n, dev, B=200, seed=0):
     g = torch.Generator(device=dev).manual_seed(seed)
     return [torch.randn(3, B, 64, device=dev, generator=g).bfloat16() for _ in range(n)]
