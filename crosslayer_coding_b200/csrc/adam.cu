@@ -1555,8 +1555,11 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
   // eight entries per feature) 1557 -> 925; per-target 6 x 16384 rows of 512, nine entries per row 565 -> 284, of 256 (12 per row, general
   // sweep) 484 -> 231; untied 6 x 12288 features of 512, 3.5 entries 760 -> 590, of 384 608 -> 501, 8 x 12288 of 256 774 -> 597, 8 x 16384 of
   // 128, six entries 1451 -> 777, one entry in sixteen 694 -> 472.  Where almost no feature has an entry, wide rows are a plain stream and
-  // the deeper ring of the pipeline is ahead by 2 to 3 % (one entry in nine, rows of 512: 569 against 586; one in eight, tied: 348, 353).
-  const bool idle_lists = !per_target && p.d > 384 && 2 * n_entries < 1LL * p.F_pitch * p.L;
+  // the deeper ring of the pipeline is ahead by 2 to 3 % (one entry in nine, rows of 512: 569 against 586; one in eight, tied: 348, 353).  With
+  // several rows per feature that holds up to one entry per feature for the widest of them (6 x 5576 features of 512, six to one row each,
+  // entries per feature: 0.5 208 / 221 us, 0.8 211 / 219, 1 215 / 215; of 480: 0.5 220 / 223, 0.7 225 / 222; of 448: 0.5 223 / 216).
+  const long long features = 1LL * p.F_pitch * p.L;
+  const bool idle_lists = !per_target && ((p.d > 384 && 2 * n_entries < features) || (p.d > 480 && !single_rows && n_entries < features));
   if (weights_bf16 && !mb && p.d <= kNarrowMaxWidth && !idle_lists) return launch_narrow_rows(p, sr, num_sms, status, st, per_target);
   auto launch = [&](auto kern) -> int {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
