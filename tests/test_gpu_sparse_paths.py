@@ -703,7 +703,7 @@ def test_threshold_statistics_of_any_type_and_stride(ext):
 HYPER = [1e-3, 0.9, 0.999, 1e-8, 0.01, 1 - 0.9 ** 3, 1 - 0.999 ** 3, 1.0, 0.5, 0.0, 1.0]
 
 
-def _row_update(ext, L, B, d, tying, counts, rows_of=None, dtype=torch.bfloat16, ctl=False, extra=False, seed=0, norm_rtol=2e-3):
+def _row_update(ext, L, B, d, tying, counts, rows_of=None, dtype=torch.bfloat16, ctl=False, extra=False, seed=0):
     """One call of the decoder sweep against 64 bits: moments, weights, norms and dL/da.  ``counts``: entries per feature (the same
     in every layer); ``rows_of``: target rows per feature of a tensor; ``ctl``: loss scale and clip coefficient; ``extra``: compact
     extra gradients of every third feature's first row; ``seed``: stochastic rounding of the weights."""
@@ -770,8 +770,11 @@ def _row_update(ext, L, B, d, tying, counts, rows_of=None, dtype=torch.bfloat16,
         # 6e-5 of 0.001); w: one rounding to 16 bits (below 2^-14 fp16 has a fixed spacing of 2^-24)
         assert (M[i].double() - m).abs().max() < 4e-6 * m.abs().max() and (V[i].double() - v).abs().max() < 1e-4 * v.abs().max()
         assert ((W[i].double() - w).abs() <= (2 if seed else 1) * ulp * w.abs() + 1e-7).all()
-        # norms of the updated rows: 2^-9 relative rounding per weight, averaged over the row
-        assert torch.allclose(n2.view(L, F)[i].double(), W[i].double().square().sum((1, 2)), rtol=norm_rtol)
+        # norms of the updated rows, of the stored weights in the per-target layout, before they are rounded in the other: fp32 sums of up to 64
+        # squares per thread and a tree over the threads and rows (below 100 additions in a row, 2^-24 each), and in the second case
+        # weights that are themselves fp32 results of a few operations
+        size = (W[i].double() if tying == 2 else w).square().sum((1, 2))
+        assert ((n2.view(L, F)[i].double() - size).abs() <= 1e-5 * size).all()
     order = torch.argsort(col.long() * B + tok.long())
     got_l, got_f, got_t = (col[order] // F).long(), (col[order] % F).long(), tok[order].long()
     assert (grad_a.double() - dlda[got_l, got_t, got_f]).abs().max() < 1e-5 * dlda.abs().max()
@@ -810,16 +813,13 @@ def test_decoder_row_update_register_forms(ext, single, d, short, opts):
 
 
 # one warp per row: every number of 128-element blocks with full and partly filled lanes, more rows than three times the resident
-# warps (a stage is refilled), one and several rows per feature, rows of all tensors of a per-target layout.  The norms may be taken
-# before the weights are rounded: 2^-8 of a weight at most (2^-7 when rounded stochastically), twice that of its square; thousands of rows
-# come nearer to that bound than the fourteen of the other tests
+# warps (a stage is refilled), one and several rows per feature, rows of all tensors of a per-target layout
 @pytest.mark.parametrize("tying,single", [(0, False), (0, True), (2, True)])
 @pytest.mark.parametrize("d", [8, 128, 136, 256, 264, 392, 512])
 @pytest.mark.parametrize("opts", [dict(), dict(ctl=True, extra=True, dtype=torch.float16), dict(seed=7)])
 def test_decoder_row_update_one_warp_per_row(ext, tying, single, d, opts):
     counts = COUNTS + [1, 0, 2] * (900 if d <= 136 else 700)
-    _row_update(ext, 3, 90, d, tying, counts, rows_of=(lambda s: 1) if single else None, norm_rtol=2.0 ** (-6 if "seed" in opts else -7),
-                **opts)
+    _row_update(ext, 3, 90, d, tying, counts, rows_of=(lambda s: 1) if single else None, **opts)
 
 
 # what the engine adds to the sweep: loss scale and clip coefficient from the control block, compact extra rows, stochastic rounding
