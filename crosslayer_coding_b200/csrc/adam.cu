@@ -807,7 +807,7 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
 // seed (input) rows of the row's entries itself, kNarrowBatch at a time; offsets are requested two rows ahead, the first 32 entries one row
 // ahead, the first batch of seed rows before the row itself is waited for.
 // Against the row pipeline above (a CTA per row): that one has five or six rows per SM at its consumers, each of which waits
-// for the lists and seed rows beyond the four staged ones, twice per row and one row after the other; here twenty rows per SM do so at the
+// for the lists and seed rows beyond the four staged ones, twice per row and one row after the other; here 16 to 24 rows per SM do so at the
 // same time, and the dot products of a row (dL/da) and its norm need no sum across warps.
 template <int NC>
 __device__ __forceinline__ void load_seed_row(const t16* row, int lane, int d, uint2 (&q)[NC]) {

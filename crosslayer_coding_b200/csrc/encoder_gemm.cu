@@ -6,7 +6,7 @@
 // Counterpart of the reference's per-layer F.linear calls (clt/models/parallel.py:286 through
 // clt/models/encoder.py:101).
 //
-// Structure: one CTA per SM, 10 warps.  Warp 0 feeds a 4-stage shared-memory ring with TMA tile loads
+// Structure: one CTA per SM, 10 warps.  Warp 0 feeds a 4-stage shared-memory ring (3 with statistics) with TMA tile loads
 // (no cluster multicast: every CTA fetches its own tiles), warp 1 issues tcgen05.mma 128x256x16 into one
 // of two 256-column TMEM accumulators, warps 2-9 drain the other accumulator with tcgen05.ld, add the
 // bias and store bf16.  Tiles are ordered m-fastest so CTAs that run together share the weight tile in L2.
@@ -45,13 +45,13 @@ constexpr int kEpiThreads = 32 * kEpiWarps;
 constexpr int kEpiWarpCols = 128;
 constexpr uint32_t kEpiStageBytes = 32 * kEpiCols * 2;
 
-// `stage`: this warp's BUFS staging tiles (1024-byte aligned), used in turn (`turn` counts the stores); `chunks` of the two
-// 64-column chunks are inside the matrix; `release` hands the accumulator back.
+// `tile`: this warp's staging tile (1024-byte aligned); `chunks` of the two 64-column chunks are inside the matrix; `release` hands the
+// accumulator back.
 // With `colacc` (shared, [2][BN] floats: sums and sums of squares per tile column) the column statistics of the rounded
 // values are read back from the staging tile (each lane owns two adjacent columns) and added up over the tile's
 // four row slabs; `nrows` masks the rows beyond the matrix.
-template <int BUFS, bool STATS, typename Release>
-__device__ __forceinline__ void epilogue_warp(uint32_t taddr, const CUtensorMap* map_c, uint8_t* stage, uint32_t& turn, const t16* bias_s,
+template <bool STATS, typename Release>
+__device__ __forceinline__ void epilogue_warp(uint32_t taddr, const CUtensorMap* map_c, uint8_t* tile, const t16* bias_s,
                                               int chunks, int n_base, int m_base, int l, int lane, float* colacc, int bn_full, int nrows,
                                               Release release) {
   uint32_t r[4][32];
@@ -62,9 +62,7 @@ __device__ __forceinline__ void epilogue_warp(uint32_t taddr, const CUtensorMap*
 #pragma unroll
   for (int c = 0; c < kEpiWarpCols / kEpiCols; ++c) {
     if (c >= chunks) break;
-    uint8_t* tile = stage + (BUFS > 1 ? (turn % BUFS) * kEpiStageBytes : 0u);
-    ++turn;
-    if (lane == 0) bulk_wait_read<BUFS - 1>();  // the store that used this staging tile before has read it
+    if (lane == 0) bulk_wait_read<0>();  // the store that used the staging tile before has read it
     __syncwarp();
     const uint4* b8 = reinterpret_cast<const uint4*>(bias_s + c * kEpiCols);
 #pragma unroll
@@ -144,11 +142,11 @@ struct GemmShared {
   float colacc[STATS ? 2 * gemm::BN : 1];
 };
 // ring + epilogue staging + barriers, bias and column sums
-template <int STAGES, int BUFS, bool STATS, uint32_t STAGE_BYTES>
-constexpr size_t kGemmSmem = size_t(STAGES) * STAGE_BYTES + size_t(kEpiWarps) * BUFS * kEpiStageBytes + sizeof(GemmShared<STAGES, STATS>);
+template <int STAGES, bool STATS, uint32_t STAGE_BYTES>
+constexpr size_t kGemmSmem = size_t(STAGES) * STAGE_BYTES + size_t(kEpiWarps) * kEpiStageBytes + sizeof(GemmShared<STAGES, STATS>);
 constexpr size_t kMaxDynamicSmem = 227 * 1024;
 
-template <int STAGES, int BUFS, bool STATS>
+template <int STAGES, bool STATS>
 __global__ void __launch_bounds__(gemm::NUM_THREADS, 1)
 encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_c, const t16* __restrict__ bias,
@@ -158,8 +156,8 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   extern __shared__ __align__(1024) uint8_t tiles[];  // 128-byte-swizzled tiles need 1024-byte alignment
   uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;  // 4 KB staging tiles, 1024-byte aligned
   using Shared = GemmShared<STAGES, STATS>;
-  static_assert(kGemmSmem<STAGES, BUFS, STATS, STAGE_BYTES> <= kMaxDynamicSmem, "shared memory of one CTA");
-  Shared* sh = reinterpret_cast<Shared*>(epi_stage + kEpiWarps * BUFS * kEpiStageBytes);
+  static_assert(kGemmSmem<STAGES, STATS, STAGE_BYTES> <= kMaxDynamicSmem, "shared memory of one CTA");
+  Shared* sh = reinterpret_cast<Shared*>(epi_stage + kEpiWarps * kEpiStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -265,9 +263,9 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int col0 = (ew >> 2) * kEpiWarpCols;
     const int etid = ew * 32 + lane;
     const int row_blocks = (M + 127) / 128;
-    uint8_t* stage = epi_stage + ew * BUFS * kEpiStageBytes;
+    uint8_t* stage = epi_stage + ew * kEpiStageBytes;
     int prev_l = -1, prev_rb = 0, prev_n = 0;
-    uint32_t local_tile = 0, turn = 0;
+    uint32_t local_tile = 0;
     bool ok = true;
     for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local_tile) {
       const int mt = int(t % tiles_m);
@@ -300,7 +298,7 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (lane == 0) mbar_arrive(&sh->tmem_empty[buf]);
       };
       if (chunks > 0)
-        epilogue_warp<BUFS, STATS>(taddr, &map_c, stage, turn, sh->bias[ew], chunks, n_base, m_base, l, lane,
+        epilogue_warp<STATS>(taddr, &map_c, stage, sh->bias[ew], chunks, n_base, m_base, l, lane,
                                    STATS ? sh->colacc + col0 : nullptr, BN, min(32, M - m_base), release);
       else
         release();
@@ -347,7 +345,7 @@ constexpr int NUM_THREADS = 320;
 constexpr uint32_t TMEM_COLS = 512;
 }  // namespace gemm2
 
-template <int STAGES, int BUFS, bool STATS>
+template <int STAGES, bool STATS>
 __global__ void __launch_bounds__(gemm2::NUM_THREADS, 1)
 encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_c, const t16* __restrict__ bias,
@@ -357,8 +355,8 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   extern __shared__ __align__(1024) uint8_t tiles[];
   uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;
   using Shared = GemmShared<STAGES, STATS>;
-  static_assert(kGemmSmem<STAGES, BUFS, STATS, STAGE_BYTES> <= kMaxDynamicSmem, "shared memory of one CTA");
-  Shared* sh = reinterpret_cast<Shared*>(epi_stage + kEpiWarps * BUFS * kEpiStageBytes);
+  static_assert(kGemmSmem<STAGES, STATS, STAGE_BYTES> <= kMaxDynamicSmem, "shared memory of one CTA");
+  Shared* sh = reinterpret_cast<Shared*>(epi_stage + kEpiWarps * kEpiStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -459,9 +457,9 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     const int col0 = (ew >> 2) * kEpiWarpCols;
     const int etid = ew * 32 + lane;
     const int row_blocks = (M + 127) / 128;
-    uint8_t* stage = epi_stage + ew * BUFS * kEpiStageBytes;
+    uint8_t* stage = epi_stage + ew * kEpiStageBytes;
     int prev_l = -1, prev_rb = 0, prev_n = 0;
-    uint32_t local_tile = 0, turn = 0;
+    uint32_t local_tile = 0;
     bool ok = true;
     for (long long t = pair; t < total_tiles && ok; t += npairs, ++local_tile) {
       const int mt = int(t % tiles_m);
@@ -494,7 +492,7 @@ encoder_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&sh->tmem_empty[buf]), 0));  // the leader's barrier
       };
       if (chunks > 0)
-        epilogue_warp<BUFS, STATS>(taddr, &map_c, stage, turn, sh->bias[ew], chunks, n_base, m_base, l, lane,
+        epilogue_warp<STATS>(taddr, &map_c, stage, sh->bias[ew], chunks, n_base, m_base, l, lane,
                                    STATS ? sh->colacc + col0 : nullptr, BN, min(32, M - m_base), release);
       else
         release();
@@ -549,14 +547,16 @@ static bool make_kmajor_map(CUtensorMap* map, const void* base, int layers, int 
   return r == CUDA_SUCCESS;
 }
 
-// Ring stages and staging tiles per epilogue warp of the pair kernel.
-constexpr int kPairStages = 6, kPairBufs = 1;
+// Ring stages: as many as fit beside the staging tiles (five with two staging tiles per warp were slower, 1419 against 1325 us at 12 x 4096 x
+// 24576 x 768), one less with the column sums.
+constexpr int kPairStages = 6, kPairStatsStages = 5;
+constexpr int kSingleStages = 4, kSingleStatsStages = 3;
 
-template <int STAGES, int BUFS, bool STATS>
+template <int STAGES, bool STATS>
 static int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const t16* bias, int L, int M, int N, int K,
                        long long ldc, long long layer_stride_c, int* status, float* tile_stats, int num_sms, cudaStream_t stream) {
-  auto* kernel = encoder_gemm_pair_kernel<STAGES, BUFS, STATS>;
-  constexpr size_t smem = kGemmSmem<STAGES, BUFS, STATS, gemm2::STAGE_BYTES>;
+  auto* kernel = encoder_gemm_pair_kernel<STAGES, STATS>;
+  constexpr size_t smem = kGemmSmem<STAGES, STATS, gemm2::STAGE_BYTES>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * num_sms);
   cfg.blockDim = dim3(gemm2::NUM_THREADS);
@@ -584,11 +584,11 @@ static int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const
   return 0;
 }
 
-template <int STAGES, int BUFS, bool STATS>
+template <int STAGES, bool STATS>
 static int launch_single(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const t16* bias, int L, int M, int N, int K,
                          long long ldc, long long layer_stride_c, int* status, float* tile_stats, int num_sms, cudaStream_t stream) {
-  auto* kernel = encoder_gemm_kernel<STAGES, BUFS, STATS>;
-  constexpr size_t smem = kGemmSmem<STAGES, BUFS, STATS, gemm::STAGE_BYTES>;
+  auto* kernel = encoder_gemm_kernel<STAGES, STATS>;
+  constexpr size_t smem = kGemmSmem<STAGES, STATS, gemm::STAGE_BYTES>;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
@@ -621,12 +621,12 @@ extern "C" int CLT_FN(clt_encoder_gemm)(const void* A, const void* B, const void
   if (M >= 2 * gemm2::BM && !force_single) {  // CTA pairs when the problem has full 256-row tiles
     if (!make_kmajor_map(&map_b, B, L, N, K, K, 1LL * N * K, gemm2::BN_HALF)) return -3;
     const int r = tile_stats != nullptr
-                      ? launch_pair<5, 1, true>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats, num_sms, stream)
-                      : launch_pair<kPairStages, kPairBufs, false>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, nullptr, num_sms, stream);
+                      ? launch_pair<kPairStatsStages, true>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats, num_sms, stream)
+                      : launch_pair<kPairStages, false>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, nullptr, num_sms, stream);
     if (r <= 0) return r;  // 1: the device cannot co-schedule clusters of two
   }
   if (!make_kmajor_map(&map_b, B, L, N, K, K, 1LL * N * K, gemm::BN)) return -3;
   return tile_stats != nullptr
-             ? launch_single<3, 1, true>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats, num_sms, stream)
-             : launch_single<4, 1, false>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, nullptr, num_sms, stream);
+             ? launch_single<kSingleStatsStages, true>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats, num_sms, stream)
+             : launch_single<kSingleStages, false>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, nullptr, num_sms, stream);
 }
