@@ -345,8 +345,9 @@ void threshold_select(const Tensor& x, const Tensor& theta, int64_t f_valid, int
   check(CLT_PICK(half, clt_threshold_select)(&a, cur_stream()), "threshold_select");
 }
 
-// Per-token top-k of the batch z-scores: exactly k entries per token at [token * k, token * k + k) of the entry list.
-void token_topk_select(const Tensor& x, const Tensor& mean, const Tensor& rstd, int64_t col_pitch, int64_t k, Tensor& ctl, Tensor& ent_tok,
+// Per-token top-k of the batch z-scores: exactly k entries per token at [token * k, token * k + k) of the entry list.  Returns the number of
+// kernels launched.
+int64_t token_topk_select(const Tensor& x, const Tensor& mean, const Tensor& rstd, int64_t col_pitch, int64_t k, Tensor& ctl, Tensor& ent_tok,
                        Tensor& ent_col, Tensor& ent_val, Tensor& status, int64_t f_valid) {
   const bool half = is_half(x, "x");
   need(x, t16_of(half), "x"); need(mean, at::kFloat, "mean"); need(rstd, at::kFloat, "rstd"); need(ctl, at::kLong, "ctl");
@@ -366,7 +367,9 @@ void token_topk_select(const Tensor& x, const Tensor& mean, const Tensor& rstd, 
   c10::cuda::CUDAGuard guard(x.device());
   Tensor scratch;  // allocated and used on the current stream
   if (const long long bytes = CLT_PICK(half, clt_token_topk_scratch)(&a)) scratch = at::empty({bytes}, x.options().dtype(at::kByte));
-  check(CLT_PICK(half, clt_token_topk_select)(&a, scratch.defined() ? scratch.data_ptr() : nullptr, cur_stream()), "token_topk_select");
+  int kernels = 0;
+  check(CLT_PICK(half, clt_token_topk_select)(&a, scratch.defined() ? scratch.data_ptr() : nullptr, &kernels, cur_stream()), "token_topk_select");
+  return kernels;
 }
 
 // Bytes of scratch that the selection of k of L * F columns for B tokens allocates; 0: a form that needs none, or a call that is refused.
@@ -502,7 +505,8 @@ void dead_counter_update(Tensor& counter, Tensor& fired) {
 
 // ctl (optional): step control block; the gradient seed is multiplied by its loss scale and a seed outside the 16-bit range
 // raises its found-inf flag.  rows_limit > 0: only the first rows_limit target rows of every feature are decoded.
-void sparse_decode(const std::vector<Tensor>& dec_w, int64_t L, int64_t B, int64_t d, int64_t col_pitch, int64_t tying, const Tensor& tok_off,
+// Returns the number of kernels launched.
+int64_t sparse_decode(const std::vector<Tensor>& dec_w, int64_t L, int64_t B, int64_t d, int64_t col_pitch, int64_t tying, const Tensor& tok_off,
                    const Tensor& tcsr_col, const Tensor& tcsr_val, const OptTensor& feat_offset, const OptTensor& feat_scale,
                    const OptTensor& yhat_partial, const OptTensor& bias_sum, const OptTensor& addend, const OptTensor& target,
                    const OptTensor& sigma, const OptTensor& gs, const OptTensor& yhat_out, const OptTensor& sq_err, int64_t mode,
@@ -550,6 +554,7 @@ void sparse_decode(const std::vector<Tensor>& dec_w, int64_t L, int64_t B, int64
     a.order = order.data_ptr<int>();
   }
   check(CLT_PICK(half, clt_sparse_decode)(&a, cur_stream()), "sparse_decode");
+  return a.order != nullptr ? 2 : 1;
 }
 
 void recon_epilogue(const Tensor& yhat_sum, const Tensor& bias_sum, const OptTensor& addend, const Tensor& target, const OptTensor& sigma,

@@ -2104,8 +2104,8 @@ extern "C" long long CLT_FN(clt_token_topk_scratch)(const CltSelectArgs* a) {
 
 // Per-token top-k of the batch z-scores (TokenTopK).  Uses x, mean, rstd, L, B, F, stat_pitch, ld, layer_stride,
 // col_pitch, ctl, ent_* (capacity >= B * k), status of the argument block; k_total carries the per-token k and feat_offset
-// (when positive) the number of valid columns per layer (the rest of F is shard padding).
-extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, void* scratch, cudaStream_t st) {
+// (when positive) the number of valid columns per layer (the rest of F is shard padding).  *kernels: how many kernels were launched.
+extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, void* scratch, int* kernels, cudaStream_t st) {
   if (a->ld % 8 != 0 || a->layer_stride % 8 != 0 || a->F % 8 != 0 || a->stat_pitch % 4 != 0 || a->F > a->ld) return -1;
   const long long k = a->k_total;
   const int f_valid = a->feat_offset > 0 && a->feat_offset <= a->F ? a->feat_offset : a->F;  // feat_offset carries the valid column count here
@@ -2120,6 +2120,7 @@ extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, void* scrat
   const WideTopk shape = wide_topk(a, k);
   const bool wide = shape.ng > 0 && scratch != nullptr;
   const bool list = wide || k <= kTkMaxima / 2;
+  *kernels = wide ? 5 : (list ? 2 : 1);
   if (wide) {
     WideTopk w = shape;
     w.list = static_cast<unsigned long long*>(scratch);

@@ -422,8 +422,8 @@ class FusedBatchTopKEngine:
             self._begin_step()
         self._X_last = X
         # The GEMM can leave per-block column sums behind (tile_stats) so that the batch statistics need no second
-        # pass; at K = d_model that epilogue work outlasts the MMAs of a tile (measured: +0.75 ms on the GEMM against
-        # 0.37 ms for the separate pass at the GPT-2 shape), so the separate column-statistics pass is used.
+        # pass; its epilogue then outlasts the MMAs of a tile (1912 against 1330 us at the GPT-2 shape, where the
+        # separate pass takes 421), so the separate column-statistics pass is used.
         e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, self.tile_stats)
         if self.fn in ("jumprelu", "relu"):
             self._ensure_theta()
@@ -436,10 +436,10 @@ class FusedBatchTopKEngine:
         else:
             e.colstats(self.preact, self.mean, self.rstd)
         if self.fn == "topk" and self.world == 1:
-            e.token_topk_select(self.preact, self.mean, self.rstd, self.Fl, self.k_token, self.ctl, self.ent_tok, self.ent_col,
-                                self.ent_val, self.status, self.Fv)
+            self.kernel_launches += e.token_topk_select(self.preact, self.mean, self.rstd, self.Fl, self.k_token, self.ctl, self.ent_tok, self.ent_col,
+                                                        self.ent_val, self.status, self.Fv)
             self._build_csr()
-            self.kernel_launches += 4 + 5  # gemm, colstats, per-token selection (list, radix for overflowed lists), csr (5)
+            self.kernel_launches += 2 + 5  # gemm, colstats, csr (5)
             return
         if self.fn == "topk":
             self._token_topk_sharded()
@@ -570,10 +570,10 @@ class FusedBatchTopKEngine:
         bias_sum = self.bias_sum
         addend = self._skip_term(self._X_last) if m.skip_weight is not None else None
         if self.world == 1:
-            e.sparse_decode(dec_w, self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col, self.tcsr_val,
-                            self.foff32, self.fsc32, None, bias_sum, addend, Y, self.sigma, self.gs, yhat, self.sq_err, 1, [], 0, 0, self.status,
-                            self.step_ctl, expected_entries=self.expected_entries, equal_lists=self.fn == "topk")
-            self.kernel_launches += 1
+            self.kernel_launches += e.sparse_decode(
+                dec_w, self.L, self.B, self.d, self.Fl, self.tying, self.tok_off, self.tcsr_col, self.tcsr_val, self.foff32, self.fsc32, None,
+                bias_sum, addend, Y, self.sigma, self.gs, yhat, self.sq_err, 1, [], 0, 0, self.status, self.step_ctl,
+                expected_entries=self.expected_entries, equal_lists=self.fn == "topk")
         else:
             sy = self.symm
             if yhat is not None:

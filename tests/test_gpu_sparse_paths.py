@@ -553,6 +553,21 @@ def test_token_topk_of_large_matrices_with_values_that_are_not_finite(ext):
     assert torch.equal(got[0], torch.cat([w[0] for w in want])) and got[1] == max(w[1] for w in want)
 
 
+def test_launches_are_counted(ext):
+    """What a caller adds to its count of kernels: the per-token selection by its three forms, the decode with and without the order by length."""
+    dev = _dev()
+    z = lambda n, dt=I32: torch.zeros(n, dtype=dt, device=dev)  # noqa: E731
+    for (L, B, F, k), kernels in (((2, 40, 64, 8), 2), ((2, 40, 1024, 600), 1), ((4, 2050, 32768, 8), 5)):
+        x = torch.randn(L, B, F, device=dev).bfloat16()
+        got = ext.token_topk_select(x, z((L, F), F32), torch.ones(L, F, device=dev), F, k, z(16, torch.int64), z(B * k), z(B * k), z(B * k, F32), z(4), F)
+        assert got == kernels
+    for B, expected, equal, kernels in ((40, 0, False, 1), (10000, 0, False, 2), (10000, 20, False, 1), (10000, 200, False, 2), (10000, 200, True, 1)):
+        L, d = 3, 520
+        got = ext.sparse_decode([z((8, L - s, d), torch.bfloat16) for s in range(L)], L, B, d, 8, 0, z(B + 1), z(8), z(8, F32), None, None, None, z((L, d), F32), None, None, None,
+                                None, z((L, B, d), F32), None, 1, [], 0, 0, z(4), None, 0, expected, equal)
+        assert got == kernels
+
+
 @pytest.mark.parametrize("L,B,F", [(2, 40, 64), (6, 2048, 8192), (6, 2048, 32768)])  # the last one is large enough for the four passes
 @pytest.mark.parametrize("k", [0, -1, -(1 << 40)])
 def test_token_topk_refuses_a_count_that_is_not_positive(ext, L, B, F, k):
