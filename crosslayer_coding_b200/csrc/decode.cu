@@ -152,7 +152,10 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // address): 12 x 6208 (token, target) pairs of 136 elements without an entry take 116 us with one token per CTA, 60 with two.  So with many
 // tokens one vector per lane goes two tokens and two warps each to a CTA (4096 tokens of 6 x 256, k = 64: 93 us either way).
 // Per-source tied, running sums: 4 warps 340 us, 1 warp 610 (8192 tokens of 6 x 512, k = 200), sorted by length 295; short or equally long
-// lists are the other way round (5809 tokens of 4 x 600, k = 19: 122 us with four, 77 with one; 2048 of 6 x 512, equal lists of 64: 37, 33).
+// lists are the other way round (5809 tokens of 4 x 600, k = 19: 122 us with four, 77 with one; 2048 of 6 x 512, equal lists of 64: 37, 33).  Lists
+// of a length that the caller does not know: many tokens keep the chip busy with two warps each, whatever the length (four / two warps: 8192
+// tokens of 6 x 512 without an entry 122 / 83 us, of 12 entries 140 / 97, of 200 288 / 235; 4096 of 12 x 768 198 / 126, 216 / 138, 349 / 259;
+// below the line 4096 of 6 x 512, 48 entries on average but few in most lists, 99 / 130).
 constexpr long long kRunningMinWarps = 1024;   // tokens x chunks; below, the (token, target) split has L times as many CTAs
 constexpr long long kEightWarpsBelow = 2048;   // CTAs
 constexpr long long kManyCtas = 28672;         // CTAs
@@ -161,6 +164,7 @@ constexpr int kRunningOrderFrom = 4096;        // tokens
 constexpr int kShortBelow = 64;                // entries per token on average
 constexpr long long kShortFrom = 16384;        // CTAs
 constexpr int kRunningOneWarpBelow = 32;         // entries per token on average
+constexpr long long kRunningTwoWarpsFrom = 8192; // tokens x chunks
 constexpr int kOneWarpBelow = 128;               // entries of every token; above, by one_warp_lists
 constexpr int kOneWarpMediumBelow = 256;        // entries of every token
 constexpr int kOneWarpRunningFrom = 2048;        // tokens
@@ -635,7 +639,7 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
     if (one_warp_lists(a) || (a->equal == 0 && a->expected > 0 && a->expected < kRunningOneWarpBelow)) {
       if (a->d <= 256) decode_running_kernel<1, 1, 4, 28><<<grid, 32, 0, st>>>(p);
       else decode_running_kernel<2, 1, 4, 16><<<grid, 32, 0, st>>>(p);
-    } else if (short_lists(a)) {
+    } else if (short_lists(a) || (a->expected <= 0 && 1LL * a->B * running_chunks(a) >= kRunningTwoWarpsFrom)) {
       if (a->d <= 256) decode_running_kernel<1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
       else decode_running_kernel<2, 2, 4, 20><<<grid, 64, 0, st>>>(p);
     } else {

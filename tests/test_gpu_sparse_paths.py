@@ -174,6 +174,12 @@ def test_gather_decode_of_equal_short_lists_in_narrow_rows(ext, L, B, d):
     _check_decode(ext, L, B, d, 0, False, F=72, entries=_uneven_entries, expected=20, equal=True)
 
 
+# the running sum over lists of unknown length: on both sides of the line between four and two warps per token, one and two column chunks
+@pytest.mark.parametrize("B,d", [(8191, 200), (8192, 200), (4095, 520), (4096, 520)])
+def test_running_decode_of_many_tokens(ext, B, d):
+    _check_decode(ext, 2, B, d, 1, False, F=72, entries=_uneven_entries)
+
+
 # the running sum with one and with two warps per token
 @pytest.mark.parametrize("d", [200, 520])
 @pytest.mark.parametrize("expected,equal", [(20, False), (40, False), (100, True)])
