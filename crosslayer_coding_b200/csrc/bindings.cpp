@@ -252,6 +252,25 @@ void encoder_gemm(const Tensor& x, const Tensor& w, const OptTensor& bias, Tenso
                                          status.data_ptr<int>(), ts, num_sms(), cur_stream()), "encoder_gemm");
 }
 
+// Pre-activations and their batch statistics mean / rstd [L, N]: what encoder_gemm and colstats give, in one call.  Returns the number of
+// kernels.
+int64_t encoder_gemm_stats(const Tensor& x, const Tensor& w, const OptTensor& bias, Tensor& out, Tensor& mean, Tensor& rstd, Tensor& status) {
+  const bool half = is_half(x, "x");
+  const auto ty = t16_of(half);
+  need(x, ty, "x"); need(w, ty, "w"); need(out, ty, "out"); need(status, at::kInt, "status");
+  need(mean, at::kFloat, "mean"); need(rstd, at::kFloat, "rstd");
+  TORCH_CHECK(x.dim() == 3 && w.dim() == 3 && out.dim() == 3, "expected [L, M, K], [L, N, K], [L, M, N]");
+  const int L = x.size(0), M = x.size(1), K = x.size(2), N = w.size(1);
+  TORCH_CHECK(w.size(0) == L && w.size(2) == K && out.size(0) == L && out.size(1) == M && out.size(2) == N, "shape mismatch");
+  TORCH_CHECK(mean.numel() == 1LL * L * N && rstd.numel() == 1LL * L * N, "mean/rstd must be [L, N]");
+  if (bias.has_value() && bias->defined()) { need(*bias, ty, "bias"); TORCH_CHECK(bias->numel() == 1LL * L * N, "bias must be [L, N]"); }
+  c10::cuda::CUDAGuard guard(x.device());
+  int kernels = 0;
+  check(CLT_PICK(half, clt_encoder_gemm_stats)(x.data_ptr(), w.data_ptr(), opt_ptr<void>(bias), out.data_ptr(), L, M, N, K, status.data_ptr<int>(),
+                                               mean.data_ptr<float>(), rstd.data_ptr<float>(), &kernels, num_sms(), cur_stream()), "encoder_gemm_stats");
+  return kernels;
+}
+
 // mean / rstd [L, F] from the per-block sums written by encoder_gemm (B rows per column).
 void colstats_from_tiles(const Tensor& tile_stats, Tensor& mean, Tensor& rstd, int64_t B) {
   need(tile_stats, at::kFloat, "tile_stats"); need(mean, at::kFloat, "mean"); need(rstd, at::kFloat, "rstd");
@@ -1027,6 +1046,7 @@ void scatter_add_rows(Tensor& dst, const c10::optional<Tensor>& dst_bias, const 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   const auto none = py::none();
   m.def("encoder_gemm", &encoder_gemm);
+  m.def("encoder_gemm_stats", &encoder_gemm_stats);
   m.def("colstats", &colstats);
   m.def("colstats_from_tiles", &colstats_from_tiles);
   m.def("batchtopk_select", &batchtopk_select);

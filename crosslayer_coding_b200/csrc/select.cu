@@ -56,44 +56,66 @@ __device__ bool exchange_sum(const Exchange& ex, int round, uint32_t* vals, int 
 }
 
 // ------------------------------------------------------------------ 1. column statistics
-// x: [L, B, ld] bf16.  Each thread owns 8 adjacent columns; blockDim = (32, 8): 8 row groups.
+// x: [L, B, ld] bf16.  Each thread owns VEC adjacent columns; blockDim = (32, 8): 8 row groups.
 // With gridDim.z > 1 (narrow shards, where one CTA per column block would leave SMs idle) the rows are split
 // over blockIdx.z: the shifted sums are additive because every chunk shifts by the column's first row, so the
 // chunks add them into mean / rstd (zeroed by the launcher) and colstats_finalize_kernel converts in place.
+// blockIdx.x counts blocks of 32 * VEC columns over strips of 256 columns over all layers, from strip `first_strip` on: the encoder GEMM computes the
+// statistics of the strips before it, with the same sums in the same order (eight per column, rows r = y mod 8, added in the order of y).
+// VEC = 8: 64 bytes in flight per thread, for many strips.  VEC = 2: four times the threads with 128 bytes each, for the few strips that the GEMM
+// leaves, where the chip would wait for 8 x 256 chains (28 strips of 8192 rows: 25 us).
+template <int VEC>
+struct ColstatsLoad;
+template <>
+struct ColstatsLoad<8> {
+  using T = uint4;
+  static constexpr int kDepth = 4;
+  __device__ static uint32_t word(const uint4& v, int j) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; }
+};
+template <>
+struct ColstatsLoad<2> {
+  using T = uint32_t;
+  static constexpr int kDepth = 32;
+  __device__ static uint32_t word(const uint32_t& v, int) { return v; }
+};
+template <int VEC>
 __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x, float* __restrict__ mean,
                                                          float* __restrict__ rstd, int B, int F, long long ld,
-                                                         long long layer_stride) {
-  const int l = blockIdx.y;
+                                                         long long layer_stride, long long first_strip) {
+  using Ld = ColstatsLoad<VEC>;
+  constexpr int kBlocks = 8 / VEC;  // of 32 * VEC columns in a strip
+  constexpr int kDepth = Ld::kDepth;
+  const int strips = (F + 255) / 256;
+  const long long strip = first_strip + blockIdx.x / kBlocks;
+  const int l = int(strip / strips);
   const int rows_per_z = (((B + int(gridDim.z) - 1) / int(gridDim.z)) + 31) / 32 * 32;
   const int row_lo = int(blockIdx.z) * rows_per_z;
   const int row_hi = min(B, row_lo + rows_per_z);
-  const int cg = blockIdx.x * 32 + threadIdx.x;  // column group of 8
-  const int c0 = cg * 8;
-  __shared__ float red[8][32][17];
-  float s[8], q[8], shift[8];
+  const int c0 = int(strip % strips) * 256 + (int(blockIdx.x % kBlocks) * 32 + int(threadIdx.x)) * VEC;
+  __shared__ float red[8][32][2 * VEC + 1];
+  float s[VEC], q[VEC], shift[VEC];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) s[j] = q[j] = shift[j] = 0.f;
+  for (int j = 0; j < VEC; ++j) s[j] = q[j] = shift[j] = 0.f;
   const bool active = c0 < F;
   const t16* base = x + 1LL * l * layer_stride + c0;
   if (active) {
-    uint4 v0 = *reinterpret_cast<const uint4*>(base);
-    const uint32_t w[4] = {v0.x, v0.y, v0.z, v0.w};
+    const typename Ld::T v0 = *reinterpret_cast<const typename Ld::T*>(base);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { shift[2 * j] = t16_lo(w[j]); shift[2 * j + 1] = t16_hi(w[j]); }
-    for (int r0 = row_lo + threadIdx.y; r0 < row_hi; r0 += 32) {
-      uint4 v[4];
+    for (int j = 0; j < VEC / 2; ++j) { shift[2 * j] = t16_lo(Ld::word(v0, j)); shift[2 * j + 1] = t16_hi(Ld::word(v0, j)); }
+    for (int r0 = row_lo + threadIdx.y; r0 < row_hi; r0 += 8 * kDepth) {
+      typename Ld::T v[kDepth];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {  // four independent loads in flight
+      for (int k = 0; k < kDepth; ++k) {  // independent loads in flight
         const int r = r0 + 8 * k;
-        v[k] = r < row_hi ? __ldcs(reinterpret_cast<const uint4*>(base + 1LL * r * ld)) : v0;
+        v[k] = r < row_hi ? __ldcs(reinterpret_cast<const typename Ld::T*>(base + 1LL * r * ld)) : v0;
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int k = 0; k < kDepth; ++k) {
         if (r0 + 8 * k >= row_hi) break;
-        const uint32_t u[4] = {v[k].x, v[k].y, v[k].z, v[k].w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float a = t16_lo(u[j]) - shift[2 * j], b = t16_hi(u[j]) - shift[2 * j + 1];
+        for (int j = 0; j < VEC / 2; ++j) {
+          const uint32_t u = Ld::word(v[k], j);
+          const float a = t16_lo(u) - shift[2 * j], b = t16_hi(u) - shift[2 * j + 1];
           s[2 * j] += a; q[2 * j] += a * a;
           s[2 * j + 1] += b; q[2 * j + 1] += b * b;
         }
@@ -101,22 +123,18 @@ __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x
     }
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) { red[threadIdx.y][threadIdx.x][j] = s[j]; red[threadIdx.y][threadIdx.x][8 + j] = q[j]; }
+  for (int j = 0; j < VEC; ++j) { red[threadIdx.y][threadIdx.x][j] = s[j]; red[threadIdx.y][threadIdx.x][VEC + j] = q[j]; }
   __syncthreads();
   if (threadIdx.y == 0 && active) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < VEC; ++j) {
       float ss = 0.f, qq = 0.f;
-      for (int y = 0; y < 8; ++y) { ss += red[y][threadIdx.x][j]; qq += red[y][threadIdx.x][8 + j]; }
+      for (int y = 0; y < 8; ++y) { ss += red[y][threadIdx.x][j]; qq += red[y][threadIdx.x][VEC + j]; }
       if (c0 + j < F && gridDim.z > 1) {
         atomicAdd(&mean[1LL * l * F + c0 + j], ss);
         atomicAdd(&rstd[1LL * l * F + c0 + j], qq);
       } else if (c0 + j < F) {
-        const float mu = ss / float(B);
-        float var = B > 1 ? (qq - ss * mu) / float(B - 1) : 0.f;
-        var = fmaxf(var, 0.f);
-        mean[1LL * l * F + c0 + j] = shift[j] + mu;
-        rstd[1LL * l * F + c0 + j] = 1.f / (sqrtf(var) + 1e-6f);
+        colstats_finish(ss, qq, shift[j], B, &mean[1LL * l * F + c0 + j], &rstd[1LL * l * F + c0 + j]);
       }
     }
   }
@@ -152,17 +170,12 @@ __global__ void __launch_bounds__(256) colstats_from_tiles_kernel(const float* _
 // mean / rstd hold the shifted sum and sum of squares (shift = the column's first row); convert in place.
 __global__ void __launch_bounds__(256) colstats_finalize_kernel(const t16* __restrict__ x, float* __restrict__ mean,
                                                                   float* __restrict__ rstd, int B, int F, long long layer_stride,
-                                                                  long long n) {
-  const long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x;
+                                                                  long long first, long long n) {
+  const long long i = first + blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int l = int(i / F), c = int(i - 1LL * l * F);
   const float shift = t16_to_float(x[1LL * l * layer_stride + c]);
-  const float ss = mean[i], qq = rstd[i];
-  const float mu = ss / float(B);
-  float var = B > 1 ? (qq - ss * mu) / float(B - 1) : 0.f;
-  var = fmaxf(var, 0.f);
-  mean[i] = shift + mu;
-  rstd[i] = 1.f / (sqrtf(var) + 1e-6f);
+  colstats_finish(mean[i], rstd[i], shift, B, &mean[i], &rstd[i]);
 }
 
 // ------------------------------------------------------------------ 2. histogram of z keys
@@ -1919,24 +1932,46 @@ __global__ void __launch_bounds__(256) dead_counter_kernel(long long* __restrict
 // ====================================================================== C launchers
 using namespace clt;
 
-extern "C" int CLT_FN(clt_colstats)(const void* x, float* mean, float* rstd, int L, int B, int F, long long ld, long long layer_stride,
-                            cudaStream_t st) {
-  if (F % 8 != 0 || ld % 8 != 0 || layer_stride % 8 != 0) return -1;
+// Chunks of rows in the statistics of L layers of F columns: one, or as many as fill the chip where the columns alone do not.
+#if !CLT_T16_IS_HALF
+extern "C" int clt_colstats_splits(int L, int B, int F) {
   const int col_blocks = (F / 8 + 31) / 32;
   int zsplit = 1;
   while (1LL * col_blocks * L * zsplit < 592 && zsplit < 16 && B / (zsplit * 2) >= 128) zsplit *= 2;
-  dim3 grid(col_blocks, L, zsplit), block(32, 8);
+  return zsplit;
+}
+#else
+extern "C" int clt_colstats_splits(int L, int B, int F);
+#endif
+
+// The statistics of the strips of 256 columns (counted over all layers) from `first_strip` on.
+extern "C" int CLT_FN(clt_colstats_strips)(const void* x, float* mean, float* rstd, int L, int B, int F, long long ld, long long layer_stride,
+                                           long long first_strip, int* kernels, cudaStream_t st) {
+  *kernels = 0;
+  if (F % 8 != 0 || ld % 8 != 0 || layer_stride % 8 != 0) return -1;
+  const int strips = (F + 255) / 256;
+  const long long todo = 1LL * L * strips - first_strip;
+  if (todo <= 0) return 0;
+  const int zsplit = clt_colstats_splits(L, B, F);
+  const dim3 block(32, 8);
   const t16* xp = static_cast<const t16*>(x);
+  const long long first = first_strip / strips * F + first_strip % strips * 256, n = 1LL * L * F;  // in mean / rstd
   if (zsplit > 1) {
-    if (cudaMemsetAsync(mean, 0, sizeof(float) * size_t(L) * F, st) != cudaSuccess) return -5;
-    if (cudaMemsetAsync(rstd, 0, sizeof(float) * size_t(L) * F, st) != cudaSuccess) return -5;
+    if (cudaMemsetAsync(mean + first, 0, sizeof(float) * size_t(n - first), st) != cudaSuccess) return -5;
+    if (cudaMemsetAsync(rstd + first, 0, sizeof(float) * size_t(n - first), st) != cudaSuccess) return -5;
   }
-  colstats_kernel<<<grid, block, 0, st>>>(xp, mean, rstd, B, F, ld, layer_stride);
-  if (zsplit > 1) {
-    const long long n = 1LL * L * F;
-    colstats_finalize_kernel<<<int((n + 255) / 256), 256, 0, st>>>(xp, mean, rstd, B, F, layer_stride, n);
-  }
+  if (first_strip > 0)  // the rest of a GEMM: less than one strip for each pair of SMs
+    colstats_kernel<2><<<dim3(unsigned(4 * todo), 1, zsplit), block, 0, st>>>(xp, mean, rstd, B, F, ld, layer_stride, first_strip);
+  else
+    colstats_kernel<8><<<dim3(unsigned(todo), 1, zsplit), block, 0, st>>>(xp, mean, rstd, B, F, ld, layer_stride, 0);
+  if (zsplit > 1) colstats_finalize_kernel<<<int((n - first + 255) / 256), 256, 0, st>>>(xp, mean, rstd, B, F, layer_stride, first, n);
+  *kernels = zsplit > 1 ? 2 : 1;
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+extern "C" int CLT_FN(clt_colstats)(const void* x, float* mean, float* rstd, int L, int B, int F, long long ld, long long layer_stride,
+                            cudaStream_t st) {
+  int kernels;
+  return CLT_FN(clt_colstats_strips)(x, mean, rstd, L, B, F, ld, layer_stride, 0, &kernels, st);
 }
 
 #if !CLT_T16_IS_HALF

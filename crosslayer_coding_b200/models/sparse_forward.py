@@ -201,15 +201,16 @@ class SparseForward:
     def _select(self, X: torch.Tensor) -> None:
         e, m = self.ext, self.model
         assert X.dtype == torch.bfloat16 and X.shape == (self.L, self.B, self.d), (X.dtype, tuple(X.shape))
-        e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, None)
+        if self.fn in ("batchtopk", "topk"):
+            e.encoder_gemm_stats(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.mean, self.rstd, self.status)
+        else:
+            e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, None)
         if self.fn == "batchtopk":
-            e.colstats(self.preact, self.mean, self.rstd)
             self.hist.zero_()
             e.batchtopk_select(self.preact, self.mean, self.rstd, self.Fl, self.Fl, 0, self.Fl, self.k_total, self.key_lo, self.shift,
                                self.hist, self.ctl, self.ent_tok, self.ent_col, self.ent_val, self.cand[0], self.cand[1], self.cand[2],
                                self.cand[3], self.status, 1, 0, [], [], 0, 0, self.sel_state, self.pool)
         elif self.fn == "topk":
-            e.colstats(self.preact, self.mean, self.rstd)
             e.token_topk_select(self.preact, self.mean, self.rstd, self.Fl, self.k_token, self.ctl, self.ent_tok, self.ent_col,
                                 self.ent_val, self.status)
         else:

@@ -421,30 +421,29 @@ class FusedBatchTopKEngine:
         if fresh:
             self._begin_step()
         self._X_last = X
-        # The GEMM can leave per-block column sums behind (tile_stats) so that the batch statistics need no second
-        # pass; its epilogue then outlasts the MMAs of a tile (1912 against 1330 us at the GPT-2 shape, where the
-        # separate pass takes 421), so the separate column-statistics pass is used.
-        e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, self.tile_stats)
         if self.fn in ("jumprelu", "relu"):
+            e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, None)
             self._ensure_theta()
             e.threshold_select(self.preact, self.theta, self.Fv, self.Fl, self.ctl, self.ent_tok, self.ent_col, self.ent_val, self.status)
             self._build_csr()
             self.kernel_launches += 2 + 5  # gemm, threshold selection, csr (5)
             return
-        if self.tile_stats is not None:
+        if self.tile_stats is not None:  # statistics from sums per block of 128 tokens
+            e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, self.tile_stats)
             e.colstats_from_tiles(self.tile_stats, self.mean, self.rstd, self.B)
+            self.kernel_launches += 2
         else:
-            e.colstats(self.preact, self.mean, self.rstd)
+            self.kernel_launches += e.encoder_gemm_stats(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.mean, self.rstd, self.status)
         if self.fn == "topk" and self.world == 1:
             self.kernel_launches += e.token_topk_select(self.preact, self.mean, self.rstd, self.Fl, self.k_token, self.ctl, self.ent_tok, self.ent_col,
                                                         self.ent_val, self.status, self.Fv)
             self._build_csr()
-            self.kernel_launches += 2 + 5  # gemm, colstats, csr (5)
+            self.kernel_launches += 5  # csr
             return
         if self.fn == "topk":
             self._token_topk_sharded()
             self._build_csr()
-            self.kernel_launches += 3 + 5 + 5
+            self.kernel_launches += 1 + 5 + 5
             return
         world, rank, dptr, fptr, slot, seq = self._exchange_args()
         if self.world > 1 and self.symm is None:
@@ -456,9 +455,8 @@ class FusedBatchTopKEngine:
             world, rank, dptr, fptr, slot, seq, self.sel_state, self.pool,
         )
         self._build_csr()
-        # gemm, colstats, select (collect, find_bin, classify, fallback x3, refine, finalize | zhist, find_bin, compact,
-        # refine, finalize), csr (5)
-        self.kernel_launches += 2 + (8 if self.key_lo != 0 else 5) + 5
+        # select (collect, find_bin, classify, fallback x3, refine, finalize | zhist, find_bin, compact, refine, finalize), csr (5)
+        self.kernel_launches += (8 if self.key_lo != 0 else 5) + 5
 
     def _token_topk_sharded(self) -> None:
         """TokenTopK across feature shards (reference: clt/models/activations.py:360-491, which gathers the full

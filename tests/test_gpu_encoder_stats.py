@@ -1,0 +1,71 @@
+"""Encoder GEMM with the batch statistics in its epilogue: the outputs of the GEMM without them, the statistics of the separate pass bit for bit."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ext():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from crosslayer_coding_b200.ops import ext as e
+
+    return e.load()
+
+
+def _row_chunks(L, B, F):
+    """Chunks of rows that the separate pass splits its sums into; with more than two, its additions have no fixed order."""
+    z = 1
+    while -(-F // 256) * L * z < 592 and z < 16 and B // (2 * z) >= 128:
+        z *= 2
+    return z
+
+
+# below 256 tokens one CTA per tile; whole strips in one round and in several; strips that are left over; a last tile of 1, 9, 44, 232, 256 tokens;
+# the end of a chunk of rows inside a tile (2 x 264 and 300 rows); a last strip of 8, 72, 136 features; K below and beyond one ring of stages
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize(
+    "L,M,N,K",
+    [(2, 200, 264, 64), (2, 256, 256, 64), (1, 257, 72, 8), (1, 300, 520, 136), (3, 528, 1032, 520), (9, 1000, 8200, 128), (75, 265, 2048, 64),
+     (6, 1536, 16384, 64), (3, 2100, 32768, 72)],
+)
+def test_encoder_gemm_stats(ext, dtype, L, M, N, K):
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(L + M + N + K)
+    x = torch.randn(L, M, K, device=dev, generator=g).to(dtype)
+    w = (torch.randn(L, N, K, device=dev, generator=g) / math.sqrt(K)).to(dtype)
+    b = (3 * torch.randn(L, N, device=dev, generator=g)).to(dtype)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    nan = float("nan")
+    plain, out = (torch.full((L, M, N), nan, device=dev, dtype=dtype) for _ in range(2))
+    mean, rstd, mean_p, rstd_p = (torch.full((L, N), nan, device=dev) for _ in range(4))
+    assert ext.encoder_gemm_stats(x, w, b, out, mean, rstd, status) >= 1
+    ext.encoder_gemm(x, w, b, plain, status, None)
+    ext.colstats(plain, mean_p, rstd_p)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    assert torch.equal(out.view(torch.int16), plain.view(torch.int16))
+    if _row_chunks(L, M, N) <= 2:
+        assert torch.equal(mean, mean_p) and torch.equal(rstd, rstd_p)
+    # fp32 sums of M values (the shift keeps them at the size of the spread): M + 16 roundings of 2^-24 of sums below M times the largest value
+    of = out.double()
+    spread = (of - of[:, :1]).abs().amax(1)
+    eps = (M + 16) * 2.0 ** -24
+    assert ((mean.double() - of.mean(1)).abs() <= eps * spread + 2.0 ** -23 * of.mean(1).abs()).all()
+    var = of.var(1)
+    got = (1 / rstd.double() - 1e-6).square()
+    assert ((got - var).abs() <= 4 * eps * spread.square() + 2.0 ** -20 * var + 1e-12).all()
+
+
+def test_encoder_gemm_stats_refuses_other_shapes(ext):
+    dev = torch.device("cuda:0")
+    x, w = torch.zeros(1, 256, 64, device=dev).bfloat16(), torch.zeros(1, 256, 64, device=dev).bfloat16()
+    out, st = torch.zeros(1, 256, 256, device=dev).bfloat16(), torch.zeros(4, dtype=torch.int32, device=dev)
+    m = torch.zeros(1, 256, device=dev)
+    with pytest.raises(RuntimeError, match="mean/rstd"):
+        ext.encoder_gemm_stats(x, w, None, out, m, torch.zeros(1, 128, device=dev), st)
+    with pytest.raises(RuntimeError, match="dtype"):
+        ext.encoder_gemm_stats(x, w, None, out, m.double(), m, st)
