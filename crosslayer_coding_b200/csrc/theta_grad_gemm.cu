@@ -13,8 +13,12 @@
 // (S2 carries the penalty term, whose G is a per-feature constant outside the active entries).
 // The autograd path computes the same through P dense GEMM pairs and a dense [B, F] backward per layer.
 //
-// Structure: the persistent single-CTA pipeline of encoder_gemm.cu (TMA ring, one MMA thread, two TMEM
-// accumulators, four epilogue warps).  No multicast loads.  Every mbarrier wait is bounded.
+// Structure: a persistent pipeline (TMA ring, one MMA thread, two TMEM accumulators, eight epilogue warps), one CTA on a tile of 128 tokens or
+// a pair of CTAs (cta_group::2) on 256.  What bounds it is the operand traffic: one CTA loads 48 KB for 512 MMA cycles, more than L2 hands an SM
+// (12 x 4096 x 4096 x 768: 1403 us, tensor cores 79 % of the cycles), a CTA of a pair 32 KB (its own tokens, half of the decoder rows).
+// No multicast loads.  Every mbarrier wait is bounded.
+#include <climits>
+
 #include "common.cuh"
 
 namespace clt {
@@ -23,24 +27,31 @@ namespace tg {
 constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 64;
-constexpr int STAGES = 4;
 constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
-constexpr uint32_t B_BYTES = BN * BK * 2;
-constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int NUM_THREADS = 192;
+constexpr int EPI_WARPS = 8;  // two per 32 token rows, each with half of the columns (four: 463 us against 360 at 12 x 4096 x 4096, K = 768)
+constexpr int EPI_THREADS = 32 * EPI_WARPS;
+constexpr int NUM_THREADS = 64 + EPI_THREADS;
 constexpr uint32_t TMEM_COLS = 512;
-constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + 1024 + 4096;
 constexpr int kMaxLayers = 32;
+template <bool PAIR>
+struct Ring {
+  static constexpr int STAGES = PAIR ? 6 : 4;
+  static constexpr int B_ROWS = PAIR ? BN / 2 : BN;  // decoder rows that a CTA loads
+  static constexpr uint32_t B_BYTES = B_ROWS * BK * 2;
+  static constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr size_t SMEM_BYTES = size_t(STAGES) * STAGE_BYTES + 4096;  // barriers, thresholds and sums behind the ring
+};
 }  // namespace tg
 
 struct ThetaGradMaps {
   CUtensorMap b[tg::kMaxLayers];  // decoder tensor of source layer s viewed as [F, (L - s) * d]
 };
 
+template <bool PAIR>
 struct ThetaGradShared {
-  uint64_t full[tg::STAGES];
-  uint64_t empty[tg::STAGES];
+  uint64_t full[tg::Ring<PAIR>::STAGES];   // pairs: the leader's counts the bytes of both CTAs
+  uint64_t empty[tg::Ring<PAIR>::STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
@@ -66,6 +77,7 @@ __device__ __forceinline__ float warp_transpose_sum(float (&v)[32], int lane) {
   return v[0];
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(tg::NUM_THREADS, 1)
 theta_grad_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a_cum,
                        const __grid_constant__ ThetaGradMaps maps_b, int tying,
@@ -73,17 +85,24 @@ theta_grad_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                        const float* __restrict__ theta, int stat_pitch, float half_bw, float* __restrict__ S1,
                        float* __restrict__ S2, int L, int M, int N, int d, int* __restrict__ status) {
   using namespace tg;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  ThetaGradShared* sh = reinterpret_cast<ThetaGradShared*>(tiles + size_t(STAGES) * STAGE_BYTES);
+  using R = Ring<PAIR>;
+  using Shared = ThetaGradShared<PAIR>;
+  constexpr int STAGES = R::STAGES;
+  static_assert(sizeof(Shared) <= 4096 && R::SMEM_BYTES <= 227 * 1024, "shared memory of one CTA");
+  extern __shared__ __align__(1024) uint8_t tiles[];  // 128-byte-swizzled tiles need 1024-byte alignment
+  Shared* sh = reinterpret_cast<Shared*>(tiles + size_t(STAGES) * R::STAGE_BYTES);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int tiles_m = (M + BM - 1) / BM;
+  const int cta_rank = PAIR ? int(cluster_ctarank()) : 0;
+  const bool leader = cta_rank == 0;
+  const int worker = PAIR ? int(blockIdx.x >> 1) : int(blockIdx.x), workers = PAIR ? int(gridDim.x >> 1) : int(gridDim.x);
+  constexpr int kTileRows = PAIR ? 2 * BM : BM;
+  const int tiles_m = (M + kTileRows - 1) / kTileRows;
   const int tiles_n = (N + BN - 1) / BN;
   const int kb_per_layer = (d + BK - 1) / BK;
-  const long long tiles_per_layer = 1LL * tiles_m * tiles_n;
-  const long long total_tiles = 1LL * L * tiles_per_layer;  // source layers in ascending order: longest K first
+  const int tiles_per_layer = tiles_m * tiles_n;
+  const int total_tiles = L * tiles_per_layer;  // source layers in ascending order: longest K first
   volatile int* abort_flag = &sh->abort_flag;
 
   if (threadIdx.x == 0) {
@@ -93,49 +112,65 @@ theta_grad_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh->tmem_full[b], 1);
-      mbar_init(&sh->tmem_empty[b], 4);
+      mbar_init(&sh->tmem_empty[b], (PAIR ? 2 : 1) * EPI_WARPS);
     }
     sh->abort_flag = 0;
     fence_barrier_init();
   }
   for (int j = threadIdx.x; j < BN; j += NUM_THREADS) { sh->acc1[j] = 0.f; sh->acc2[j] = 0.f; }
   if (warp == 1) {
-    tmem_alloc(&sh->tmem_base, TMEM_COLS);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(&sh->tmem_base, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&sh->tmem_base, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
+    // ------------------------------------------------------------ TMA producer (both CTAs of a pair)
     if (lane == 0) {
       tma_prefetch_desc(&map_a);
       uint32_t it = 0;
       bool ok = true;
-      for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        const int src = int(t / tiles_per_layer);
-        const long long rem = t - 1LL * src * tiles_per_layer;
-        const int mt = int(rem % tiles_m);
-        const int nt = int(rem / tiles_m);
+      for (int t = worker; t < total_tiles && ok; t += workers) {
+        const int src = t / tiles_per_layer;
+        const int rem = t - src * tiles_per_layer;
+        const int row = (rem % tiles_m) * kTileRows + cta_rank * BM;
+        const int col = (rem / tiles_m) * BN + cta_rank * R::B_ROWS;
         // K runs over the target layers t >= src (untied: rows of the packed tensor of layer src; per_target: the
         // tensors of the layers t); per_source has one decoder row per feature, its A operand is the seed summed over t
         const int num_kb = (tying == 1 ? 1 : L - src) * kb_per_layer;
+        int tl = 0, kk = 0;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int tl = kb / kb_per_layer, kk = kb - tl * kb_per_layer;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(&sh->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          mbar_expect_tx(&sh->full[s], STAGE_BYTES);
-          uint8_t* a_dst = tiles + size_t(s) * STAGE_BYTES;
-          if (tying == 1) tma_load_3d(a_dst, &map_a_cum, &sh->full[s], kk * BK, mt * BM, src);
-          else tma_load_3d(a_dst, &map_a, &sh->full[s], kk * BK, mt * BM, src + tl);
-          if (tying == 0) tma_load_3d(a_dst + A_BYTES, &maps_b.b[src], &sh->full[s], tl * d + kk * BK, nt * BN, 0);
-          else tma_load_3d(a_dst + A_BYTES, &maps_b.b[tying == 2 ? src + tl : src], &sh->full[s], kk * BK, nt * BN, 0);
+          uint8_t* a_dst = tiles + size_t(s) * R::STAGE_BYTES;
+          const CUtensorMap* a_map = tying == 1 ? &map_a_cum : &map_a;
+          const CUtensorMap* b_map = tying == 2 ? &maps_b.b[src + tl] : &maps_b.b[src];
+          const int a_layer = tying == 1 ? src : src + tl, b_k = tying == 0 ? tl * d + kk * BK : kk * BK;
+          if constexpr (PAIR) {
+            if (leader) mbar_expect_tx(&sh->full[s], 2 * R::STAGE_BYTES);
+            const uint32_t full_leader = mapa_shared(smem_u32(&sh->full[s]), 0);
+            tma_load_3d_pair(a_dst, a_map, full_leader, kk * BK, row, a_layer);
+            tma_load_3d_pair(a_dst + A_BYTES, b_map, full_leader, b_k, col, 0);
+          } else {
+            mbar_expect_tx(&sh->full[s], R::STAGE_BYTES);
+            tma_load_3d(a_dst, a_map, &sh->full[s], kk * BK, row, a_layer);
+            tma_load_3d(a_dst + A_BYTES, b_map, &sh->full[s], b_k, col, 0);
+          }
+          if (++kk == kb_per_layer) { kk = 0; ++tl; }
         }
       }
-      if (!ok) {
+      // (A CTA of a pair that gave up waits at the cluster barrier below until its partner, whose barriers count the copies, is done.)
+      if (!ok && !PAIR) {
         const uint32_t issued = it;
         const uint32_t first = issued > STAGES ? issued - STAGES : 0;
         for (uint32_t j = first; j < issued; ++j) {
@@ -147,64 +182,70 @@ theta_grad_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
     }
   } else if (warp == 1) {
-    // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN);
-      uint32_t it = 0;
-      uint32_t local_tile = 0;
+    // -------------------------------------------------------------- MMA issuer (leader CTA of a pair)
+    if (lane == 0 && leader) {
+      constexpr uint32_t idesc = umma_idesc_bf16(kTileRows, BN);
+      const uint64_t a_desc0 = umma_desc_kmajor_sw128(smem_u32(tiles));
+      const uint64_t b_desc0 = umma_desc_kmajor_sw128(smem_u32(tiles) + A_BYTES);
+      int s = 0;
+      uint32_t ph = 0, buf = 0, tph = 1;
       bool ok = true;
-      for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local_tile) {
-        const int src = int(t / tiles_per_layer);
-        const int num_kb = (tying == 1 ? 1 : L - src) * kb_per_layer;
-        const uint32_t buf = local_tile & 1;
-        const uint32_t tph = (local_tile >> 1) & 1;
-        if (!mbar_wait(&sh->tmem_empty[buf], tph ^ 1, abort_flag)) { ok = false; break; }
+      for (int t = worker; t < total_tiles && ok; t += workers) {
+        const int num_kb = (tying == 1 ? 1 : L - t / tiles_per_layer) * kb_per_layer;
+        if (!mbar_wait(&sh->tmem_empty[buf], tph, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
+        for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&sh->full[s], ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(tiles + size_t(s) * STAGE_BYTES);
-          const uint64_t a_desc = umma_desc_kmajor_sw128(a_addr);
-          const uint64_t b_desc = umma_desc_kmajor_sw128(a_addr + A_BYTES);
+          const uint64_t a_desc = a_desc0 + uint64_t(s * int(R::STAGE_BYTES >> 4));
+          const uint64_t b_desc = b_desc0 + uint64_t(s * int(R::STAGE_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16_ss(d_tmem, a_desc + uint64_t(k * 2), b_desc + uint64_t(k * 2), idesc, (kb | k) != 0);
-          tc_commit(&sh->empty[s]);
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            if constexpr (PAIR) umma_bf16_ss_pair(d_tmem, a_desc + uint64_t(k * 2), b_desc + uint64_t(k * 2), idesc, (kb | k) != 0);
+            else umma_bf16_ss(d_tmem, a_desc + uint64_t(k * 2), b_desc + uint64_t(k * 2), idesc, (kb | k) != 0);
+          }
+          if constexpr (PAIR) tc_commit_pair(&sh->empty[s], 3);
+          else tc_commit(&sh->empty[s]);
+          if (++s == STAGES) { s = 0; ph ^= 1; }
         }
-        if (ok) tc_commit(&sh->tmem_full[buf]);
+        if (ok) {
+          if constexpr (PAIR) tc_commit_pair(&sh->tmem_full[buf], 3);
+          else tc_commit(&sh->tmem_full[buf]);
+        }
+        buf ^= 1;
+        if (buf == 0) tph ^= 1;
       }
     }
   } else {
     // ---------------------------------------------------------------- reducing epilogue
     const int quarter = warp & 3;
+    const int half = (warp - 2) >> 2;
     const int etid = (warp - 2) * 32 + lane;
     uint32_t local_tile = 0;
     bool ok = true;
-    for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local_tile) {
-      const int src = int(t / tiles_per_layer);
-      const long long rem = t - 1LL * src * tiles_per_layer;
-      const int mt = int(rem % tiles_m);
-      const int nt = int(rem / tiles_m);
+    for (int t = worker; t < total_tiles && ok; t += workers, ++local_tile) {
+      const int src = t / tiles_per_layer;
+      const int rem = t - src * tiles_per_layer;
+      const int mt = rem % tiles_m;
+      const int nt = rem / tiles_m;
       const uint32_t buf = local_tile & 1;
       const uint32_t tph = (local_tile >> 1) & 1;
-      named_barrier_sync(1, 128);  // accumulators of the previous tile were flushed and cleared
-      for (int j = etid; j < BN; j += 128) {
+      named_barrier_sync(1, EPI_THREADS);  // accumulators of the previous tile were flushed and cleared
+      for (int j = etid; j < BN; j += EPI_THREADS) {
         const int n = nt * BN + j;
         sh->theta[j] = n < N ? theta[1LL * src * stat_pitch + n] : INFINITY;
       }
       if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-      named_barrier_sync(1, 128);
+      named_barrier_sync(1, EPI_THREADS);
       if (!sh->epi_ok) { ok = false; break; }
       tc_fence_after();
-      const int m = mt * BM + quarter * 32 + lane;
+      const int m = mt * kTileRows + cta_rank * BM + quarter * 32 + lane;
       const bool row_ok = m < M;
       const t16* xrow = preact + 1LL * src * layer_stride_x + 1LL * (row_ok ? m : 0) * ldx + 1LL * nt * BN;
       const uint32_t taddr = tmem_base + buf * BN + (uint32_t(quarter * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = half * (BN / 64); c < (half + 1) * (BN / 64); ++c) {
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
         float wx[32];
@@ -237,9 +278,12 @@ theta_grad_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->tmem_empty[buf]);
-      named_barrier_sync(1, 128);  // all four warps added their rows
-      for (int j = etid; j < BN; j += 128) {
+      if (lane == 0) {
+        if constexpr (PAIR) mbar_arrive_cluster(mapa_shared(smem_u32(&sh->tmem_empty[buf]), 0));  // the leader's barrier
+        else mbar_arrive(&sh->tmem_empty[buf]);
+      }
+      named_barrier_sync(1, EPI_THREADS);  // all warps added their rows
+      for (int j = etid; j < BN; j += EPI_THREADS) {
         const int n = nt * BN + j;
         const float a1 = sh->acc1[j], a2 = sh->acc2[j];
         if (n < N) {
@@ -254,9 +298,11 @@ theta_grad_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();  // neither CTA retires (or frees TMEM) while the other may still use its memory
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
   if (threadIdx.x == 0 && sh->abort_flag && status != nullptr) atomicCAS(status, STATUS_OK, STATUS_WAIT_TIMEOUT);
 }
@@ -308,31 +354,74 @@ struct CltThetaGradArgs {
   const void* gs_cum;      // per_source: [L, B, d] suffix sums of gs over the layers
 };
 
-// Returns 0 on success, a negative value when the arguments cannot be handled (the caller raises).
-extern "C" int CLT_FN(clt_theta_grad_gemm)(const CltThetaGradArgs* a, int num_sms, cudaStream_t stream) {
-  using namespace clt;
-  if (a->d % 8 != 0 || a->ldx % 8 != 0 || a->layer_stride_x % 8 != 0 || a->L > tg::kMaxLayers || a->L < 1) return -1;
+namespace clt {
+
+// 1: the device cannot co-schedule clusters of two
+template <bool PAIR>
+static int tg_launch(const CltThetaGradArgs* a, int num_sms, cudaStream_t stream) {
+  using R = tg::Ring<PAIR>;
   CUtensorMap map_a, map_a_cum;
   ThetaGradMaps maps;
-  if (a->tying < 0 || a->tying > 2 || (a->tying == 1 && a->gs_cum == nullptr)) return -1;
   if (!tg_make_map(&map_a, a->gs, a->L, a->B, a->d, a->d, 1LL * a->B * a->d, tg::BM)) return -3;
   if (!tg_make_map(&map_a_cum, a->tying == 1 ? a->gs_cum : a->gs, a->L, a->B, a->d, a->d, 1LL * a->B * a->d, tg::BM)) return -3;
   for (int s = 0; s < tg::kMaxLayers; ++s) {
     const int src = s < a->L ? s : a->L - 1;
     const long long K = a->tying == 0 ? 1LL * (a->L - src) * a->d : a->d;
     if ((reinterpret_cast<uintptr_t>(a->w[src]) & 15) != 0) return -2;
-    if (!tg_make_map(&maps.b[s], a->w[src], 1, a->F, K, K, 1LL * a->F * K, tg::BN)) return -3;
+    if (!tg_make_map(&maps.b[s], a->w[src], 1, a->F, K, K, 1LL * a->F * K, R::B_ROWS)) return -3;
   }
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(theta_grad_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tg::SMEM_BYTES)) != cudaSuccess) return -4;
-    attr_set = true;
-  }
-  const long long tiles = 1LL * a->L * ((a->B + tg::BM - 1) / tg::BM) * ((a->F + tg::BN - 1) / tg::BN);
+  constexpr int kTileRows = PAIR ? 2 * tg::BM : tg::BM;
+  const long long tiles = 1LL * a->L * ((a->B + kTileRows - 1) / kTileRows) * ((a->F + tg::BN - 1) / tg::BN);
   if (tiles == 0) return 0;
-  const int grid = int(tiles < num_sms ? tiles : num_sms);
-  theta_grad_gemm_kernel<<<grid, tg::NUM_THREADS, tg::SMEM_BYTES, stream>>>(
-      map_a, map_a_cum, maps, a->tying, static_cast<const t16*>(a->preact), a->ldx, a->layer_stride_x, a->theta, a->stat_pitch,
-      0.5f * a->bandwidth, a->S1, a->S2, a->L, a->B, a->F, a->d, a->status);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  if (tiles > INT_MAX / 2) return -1;
+  auto* kernel = theta_grad_gemm_kernel<PAIR>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(PAIR ? 2 * num_sms : num_sms));
+  cfg.blockDim = dim3(tg::NUM_THREADS);
+  cfg.dynamicSmemBytes = R::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = PAIR ? 1 : 0;
+  // co-resident clusters, probed once per device (the kernel's shared memory limit belongs to the device as well)
+  constexpr int kDevices = 64;
+  static int probed[kDevices] = {};  // count + 1, 0: not yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return -5;
+  int n = dev < kDevices ? probed[dev] : 0;
+  if (n == 0) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(R::SMEM_BYTES)) != cudaSuccess) return -4;
+    n = num_sms;
+    if (PAIR && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      n = 0;
+      (void)cudaGetLastError();
+    }
+    ++n;
+    if (dev < kDevices) probed[dev] = n;
+  }
+  const int workers = n - 1;
+  if (workers <= 0) return 1;
+  cfg.gridDim = dim3(unsigned((PAIR ? 2 : 1) * (tiles < workers ? tiles : workers)));
+  if (cudaLaunchKernelEx(&cfg, kernel, map_a, map_a_cum, maps, a->tying, static_cast<const t16*>(a->preact), a->ldx, a->layer_stride_x, a->theta,
+                         a->stat_pitch, 0.5f * a->bandwidth, a->S1, a->S2, a->L, a->B, a->F, a->d, a->status) != cudaSuccess) return -5;
+  return 0;
+}
+
+}  // namespace clt
+
+// Returns 0 on success, a negative value when the arguments cannot be handled (the caller raises).
+extern "C" int CLT_FN(clt_theta_grad_gemm)(const CltThetaGradArgs* a, int num_sms, cudaStream_t stream) {
+  using namespace clt;
+  if (a->d % 8 != 0 || a->ldx % 8 != 0 || a->layer_stride_x % 8 != 0 || a->L > tg::kMaxLayers || a->L < 1) return -1;
+  if (a->tying < 0 || a->tying > 2 || (a->tying == 1 && a->gs_cum == nullptr)) return -1;
+  // a pair multiplies 256 token rows whether they exist or not: with 640 (five times 128) the sixth of it that is for nothing costs more than
+  // pairs gain (7 % slower, where 1024 and 2000 rows are 7 to 25 % faster)
+  const int halves = (a->B + tg::BM - 1) / tg::BM;
+  if (halves % 2 == 0 || halves > 8) {
+    const int r = tg_launch<true>(a, num_sms, stream);
+    if (r <= 0) return r;
+  }
+  return tg_launch<false>(a, num_sms, stream);
 }
