@@ -1335,6 +1335,7 @@ __global__ void __launch_bounds__(256) encoder_rows_adam_kernel(const EncAdamPar
 // Encoder bias update on its own (used with the bulk-copy row pipeline, which handles the weight rows).
 template <typename WT>
 __global__ void __launch_bounds__(256) encoder_bias_adam_kernel(const EncAdamParams p) {
+  if (chain_wait()) return;
   const long long rows = 1LL * p.L * p.F_pitch;
   const StepScales sc = read_step_ctl(p.ctl);
   if (sc.skip) return;
@@ -1371,6 +1372,7 @@ template <typename WT>
 __global__ void __launch_bounds__(256) dense_adam_kernel(WT* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
                                                            const float* __restrict__ grad, long long n, AdamHyper h,
                                                            float* __restrict__ ctl, int seed_scaled, float norm_weight) {
+  if (chain_wait()) return;
   const StepScales sc = read_step_ctl(ctl);
   if (sc.skip) return;
   const float gmul = h.grad_scale * (seed_scaled ? sc.inv_scale : 1.f);
@@ -1400,6 +1402,7 @@ __global__ void __launch_bounds__(256) dense_adam_kernel(WT* __restrict__ w, flo
 // Squared decoder norms per feature: out[ti * F_pitch + f] = sum over the feature's rows and d of w^2.
 template <typename WT>
 __global__ void __launch_bounds__(256) decoder_norm2_kernel(const WT* __restrict__ w, float* __restrict__ out, int F, int R, int d) {
+  if (chain_wait()) return;
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1428,6 +1431,7 @@ __global__ void __launch_bounds__(256) sparsity_penalty_kernel(const int* __rest
                                                                  const float* __restrict__ norm2, int ncols, float lambda, float c,
                                                                  float* __restrict__ grad_a, float* __restrict__ pen_coef,
                                                                  double* __restrict__ penalty_out) {
+  if (chain_wait()) return;
   float local = 0.f;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncols; col += gridDim.x * blockDim.x) {
     const int b = feat_off[col], e = feat_off[col + 1];
@@ -1524,7 +1528,7 @@ static int launch_narrow_rows(const DecAdamParams& p, bool sr, int num_sms, int*
     long long grid = 1LL * num_sms * per_sm;
     const long long ctas = (total + kNarrowWarps - 1) / kNarrowWarps;
     if (grid > ctas) grid = ctas;
-    kern<<<int(grid), 32 * kNarrowWarps, smem, st>>>(p, total, status);
+    launch_alone(kern, int(grid), 32 * kNarrowWarps, smem, st, p, total, status);
     return 0;
   };
   auto pick = [&](auto srv, auto ptv) -> int {
@@ -1600,7 +1604,7 @@ static int launch_rows_adam_bulk(const DecAdamParams& p, bool weights_bf16, bool
         if (waste < best_waste - 1e-9) { best_waste = waste; best = g; }
       }
     }
-    kern<<<best, gthreads + 32, smem, st>>>(p, gthreads, stage_bytes, nstages, status);
+    launch_alone(kern, best, gthreads + 32, smem, st, p, gthreads, stage_bytes, nstages, status);
     return 0;
   };
   // Registers against batches.  Four entries per batch take 72 registers, which costs rows of 392 to 608 elements a resident CTA per SM
@@ -1680,12 +1684,12 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   if (a->norm_only) {
     if (a->ctl == nullptr) return -1;
     if (a->tying == 0) {
-      if (a->weights_bf16) decoder_rows_adam_untied_kernel<t16, false, true><<<grid, 256, 0, st>>>(p);
-      else decoder_rows_adam_untied_kernel<float, false, true><<<grid, 256, 0, st>>>(p);
+      if (a->weights_bf16) launch_alone(decoder_rows_adam_untied_kernel<t16, false, true>, grid, 256, 0, st, p);
+      else launch_alone(decoder_rows_adam_untied_kernel<float, false, true>, grid, 256, 0, st, p);
     } else if (a->weights_bf16) {
-      decoder_rows_adam_kernel<t16, true><<<grid, 256, 0, st>>>(p);
+      launch_alone(decoder_rows_adam_kernel<t16, true>, grid, 256, 0, st, p);
     } else {
-      decoder_rows_adam_kernel<float, true><<<grid, 256, 0, st>>>(p);
+      launch_alone(decoder_rows_adam_kernel<float, true>, grid, 256, 0, st, p);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
@@ -1702,15 +1706,15 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   } else if (a->tying == 0) {
     const bool sr = a->h.sr_seed != 0;
     if (a->weights_bf16) {
-      if (sr) decoder_rows_adam_untied_kernel<t16, true, false><<<grid, 256, 0, st>>>(p);
-      else decoder_rows_adam_untied_kernel<t16, false, false><<<grid, 256, 0, st>>>(p);
+      if (sr) launch_alone(decoder_rows_adam_untied_kernel<t16, true, false>, grid, 256, 0, st, p);
+      else launch_alone(decoder_rows_adam_untied_kernel<t16, false, false>, grid, 256, 0, st, p);
     } else {
-      decoder_rows_adam_untied_kernel<float, false, false><<<grid, 256, 0, st>>>(p);
+      launch_alone(decoder_rows_adam_untied_kernel<float, false, false>, grid, 256, 0, st, p);
     }
   } else if (a->weights_bf16) {
-    decoder_rows_adam_kernel<t16, false><<<grid, 256, 0, st>>>(p);
+    launch_alone(decoder_rows_adam_kernel<t16, false>, grid, 256, 0, st, p);
   } else {
-    decoder_rows_adam_kernel<float, false><<<grid, 256, 0, st>>>(p);
+    launch_alone(decoder_rows_adam_kernel<float, false>, grid, 256, 0, st, p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -1741,8 +1745,8 @@ extern "C" int CLT_FN(clt_encoder_rows_adam)(const CltEncAdamArgs* a, int num_sm
   const int grid = num_sms * 8;
   if (a->norm_only) {
     if (a->ctl == nullptr) return -1;
-    if (a->weights_bf16) encoder_rows_adam_kernel<t16, true><<<grid, 256, 0, st>>>(p);
-    else encoder_rows_adam_kernel<float, true><<<grid, 256, 0, st>>>(p);
+    if (a->weights_bf16) launch_alone(encoder_rows_adam_kernel<t16, true>, grid, 256, 0, st, p);
+    else launch_alone(encoder_rows_adam_kernel<float, true>, grid, 256, 0, st, p);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
   if (a->status != nullptr && a->L <= kMaxLayersA && bulk_rows_adam_fits(a->d, a->weights_bf16)) {
@@ -1774,13 +1778,13 @@ extern "C" int CLT_FN(clt_encoder_rows_adam)(const CltEncAdamArgs* a, int num_sm
     if (rc != 0) return rc;
     if (p.bias != nullptr) {
       const int bgrid = int((1LL * a->L * a->F_pitch + 255) / 256);
-      if (a->weights_bf16) encoder_bias_adam_kernel<t16><<<bgrid, 256, 0, st>>>(p);
-      else encoder_bias_adam_kernel<float><<<bgrid, 256, 0, st>>>(p);
+      if (a->weights_bf16) launch_chained(encoder_bias_adam_kernel<t16>, bgrid, 256, 0, st, p);
+      else launch_chained(encoder_bias_adam_kernel<float>, bgrid, 256, 0, st, p);
     }
   } else if (a->moments_bf16) {
     return -6;  // only the bulk pipeline handles bf16 moments
-  } else if (a->weights_bf16) encoder_rows_adam_kernel<t16, false><<<grid, 256, 0, st>>>(p);
-  else encoder_rows_adam_kernel<float, false><<<grid, 256, 0, st>>>(p);
+  } else if (a->weights_bf16) launch_alone(encoder_rows_adam_kernel<t16, false>, grid, 256, 0, st, p);
+  else launch_alone(encoder_rows_adam_kernel<float, false>, grid, 256, 0, st, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -1788,8 +1792,8 @@ extern "C" int CLT_FN(clt_dense_adam)(void* w, float* m, float* v, const float* 
                                       float* ctl, int seed_scaled, float norm_weight, cudaStream_t st) {
   if (n <= 0) return 0;
   const int grid = int((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-  if (weights_bf16) dense_adam_kernel<t16><<<grid, 256, 0, st>>>(static_cast<t16*>(w), m, v, grad, n, to_hyper(*h), ctl, seed_scaled, norm_weight);
-  else dense_adam_kernel<float><<<grid, 256, 0, st>>>(static_cast<float*>(w), m, v, grad, n, to_hyper(*h), ctl, seed_scaled, norm_weight);
+  if (weights_bf16) launch_chained(dense_adam_kernel<t16>, grid, 256, 0, st, static_cast<t16*>(w), m, v, grad, n, to_hyper(*h), ctl, seed_scaled, norm_weight);
+  else launch_chained(dense_adam_kernel<float>, grid, 256, 0, st, static_cast<float*>(w), m, v, grad, n, to_hyper(*h), ctl, seed_scaled, norm_weight);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -1797,8 +1801,8 @@ extern "C" int CLT_FN(clt_decoder_norm2)(const void* w, float* out, int F, int R
   if ((1LL * R * d) % 8 != 0) return -1;
   const int grid = (F + 7) / 8 < 1184 ? (F + 7) / 8 : 1184;
   if (grid == 0) return 0;
-  if (weights_bf16) decoder_norm2_kernel<t16><<<grid, 256, 0, st>>>(static_cast<const t16*>(w), out, F, R, d);
-  else decoder_norm2_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(w), out, F, R, d);
+  if (weights_bf16) launch_chained(decoder_norm2_kernel<t16>, grid, 256, 0, st, static_cast<const t16*>(w), out, F, R, d);
+  else launch_chained(decoder_norm2_kernel<float>, grid, 256, 0, st, static_cast<const float*>(w), out, F, R, d);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -1807,7 +1811,7 @@ extern "C" int clt_sparsity_penalty(const int* feat_off, const float* fcsr_val, 
                                     float* grad_a, float* pen_coef, double* penalty_out, cudaStream_t st) {
   if (ncols <= 0) return 0;
   const int grid = (ncols + 255) / 256 < 1184 ? (ncols + 255) / 256 : 1184;
-  sparsity_penalty_kernel<<<grid, 256, 0, st>>>(feat_off, fcsr_val, norm2, ncols, lambda, c, grad_a, pen_coef, penalty_out);
+  launch_chained(sparsity_penalty_kernel, grid, 256, 0, st, feat_off, fcsr_val, norm2, ncols, lambda, c, grad_a, pen_coef, penalty_out);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 #endif

@@ -34,6 +34,7 @@ constexpr int kAuxMaxCap = 4096;  // compact dead features per layer that one CT
 __global__ void __launch_bounds__(1024) aux_compact_kernel(const long long* __restrict__ dead_counter, long long window, int F_pitch, int F_valid,
                                                             int nd_cap, int* __restrict__ dead_cols, int* __restrict__ nd, int* __restrict__ nd_all,
                                                             int* __restrict__ extra_idx) {
+  if (chain_wait()) return;
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   const int l = blockIdx.x;
@@ -110,6 +111,7 @@ __device__ __forceinline__ int warp_find_bin_from_top(const unsigned int* hist, 
 __global__ void __launch_bounds__(256) aux_gather_bias_kernel(const void* __restrict__ enc_bias, int bias_is_16, int F_pitch,
                                                                 const int* __restrict__ dead_cols, const int* __restrict__ nd, int nd_cap,
                                                                 float* __restrict__ bias_c) {
+  if (chain_wait()) return;
   const int l = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nd_cap) return;
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256) aux_gather_select_kernel(const t16* __res
                                                                   const int* __restrict__ dead_cols, const int* __restrict__ nd,
                                                                   const int* __restrict__ nd_all, int nd_cap, int k_aux_max, int B,
                                                                   t16* __restrict__ A) {
+  if (chain_wait()) return;
   extern __shared__ __align__(16) uint8_t aux_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tok = blockIdx.x * 8 + warp, l = blockIdx.y;
@@ -225,6 +228,7 @@ struct AuxRowsParams {
 };
 __global__ void __launch_bounds__(256) aux_gather_rows_kernel(AuxRowsParams p, const int* __restrict__ dead_cols, const int* __restrict__ nd,
                                                                 int nd_cap, int d, t16* __restrict__ W0) {
+  if (chain_wait()) return;
   const int l = blockIdx.y;
   const int vec = d / 8;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < 1LL * nd_cap * vec; i += 1LL * gridDim.x * blockDim.x) {
@@ -248,6 +252,7 @@ __global__ void __launch_bounds__(256) aux_residual_kernel(const float* __restri
                                                              t16* __restrict__ gs, t16* __restrict__ g_out, double* __restrict__ loss,
                                                              const int* __restrict__ nd, const float* __restrict__ ctl, int L, int B, int d,
                                                              float factor, int scale_g) {
+  if (chain_wait()) return;
   const int l = blockIdx.y;
   const bool live = nd[l] > 0;  // a layer without dead features has no auxiliary term
   const float scale = ctl != nullptr ? ctl[SC_LOSS_SCALE] : 1.f;
@@ -298,6 +303,7 @@ __global__ void __launch_bounds__(256) aux_residual_kernel(const float* __restri
 
 // buf *= 1 / loss scale (gradients that were formed from a scaled 16-bit factor)
 __global__ void __launch_bounds__(256) unscale_kernel(float* __restrict__ buf, long long n, const float* __restrict__ ctl) {
+  if (chain_wait()) return;
   const float inv = ctl[SC_INV_SCALE];
   for (long long i = (blockIdx.x * 1LL * blockDim.x + threadIdx.x) * 4; i < n; i += 1LL * gridDim.x * blockDim.x * 4) {
     if (i + 4 <= n) {
@@ -312,6 +318,7 @@ __global__ void __launch_bounds__(256) unscale_kernel(float* __restrict__ buf, l
 
 // out[r] = sum of the 16-bit row r of in [rows, n]  (encoder-bias gradient of the dead features: row sums of G^T)
 __global__ void __launch_bounds__(256) rowsum16_kernel(const t16* __restrict__ in, float* __restrict__ out, long long rows, int n) {
+  if (chain_wait()) return;
   const int lane = threadIdx.x & 31;
   const long long warp_global = (blockIdx.x * 1LL * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (gridDim.x * 1LL * blockDim.x) >> 5;
@@ -333,6 +340,7 @@ __global__ void __launch_bounds__(256) rowsum16_kernel(const t16* __restrict__ i
 __global__ void __launch_bounds__(256) scatter_add_rows_kernel(float* __restrict__ dst, float* __restrict__ dst_bias, const float* __restrict__ src,
                                                                  const float* __restrict__ src_bias, const int* __restrict__ extra_idx,
                                                                  long long n_dst_rows, int d) {
+  if (chain_wait()) return;
   const int vec = d / 4;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n_dst_rows * vec; i += 1LL * gridDim.x * blockDim.x) {
     const long long row = i / vec;
@@ -355,7 +363,7 @@ using namespace clt;
 extern "C" int clt_aux_compact(const long long* dead_counter, long long window, int L, int F_pitch, int F_valid, int nd_cap, int* dead_cols,
                                int* nd, int* nd_all, int* extra_idx, cudaStream_t st) {
   if (L <= 0 || nd_cap <= 0) return -1;
-  aux_compact_kernel<<<L, 1024, 0, st>>>(dead_counter, window, F_pitch, F_valid, nd_cap, dead_cols, nd, nd_all, extra_idx);
+  launch_chained(aux_compact_kernel, L, 1024, 0, st, dead_counter, window, F_pitch, F_valid, nd_cap, dead_cols, nd, nd_all, extra_idx);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -364,7 +372,7 @@ extern "C" int clt_unscale(float* buf, long long n, const float* ctl, cudaStream
   if (ctl == nullptr || (reinterpret_cast<uintptr_t>(buf) & 15) != 0) return -1;
   const long long nv = (n + 3) / 4;
   const int grid = int((nv + 255) / 256 < 148 * 16 ? (nv + 255) / 256 : 148 * 16);
-  unscale_kernel<<<grid, 256, 0, st>>>(buf, n, ctl);
+  launch_chained(unscale_kernel, grid, 256, 0, st, buf, n, ctl);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -373,7 +381,7 @@ extern "C" int clt_scatter_add_rows(float* dst, float* dst_bias, const float* sr
   if (d % 4 != 0) return -1;
   const long long n = n_dst_rows * (d / 4);
   const int grid = int((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-  scatter_add_rows_kernel<<<grid, 256, 0, st>>>(dst, dst_bias, src, src_bias, extra_idx, n_dst_rows, d);
+  launch_chained(scatter_add_rows_kernel, grid, 256, 0, st, dst, dst_bias, src, src_bias, extra_idx, n_dst_rows, d);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 #endif
@@ -384,7 +392,7 @@ extern "C" int CLT_FN(clt_aux_gather_select)(const void* pre, long long ld, long
   if (nd_cap > kAuxMaxCap || nd_cap % 8 != 0 || (pre == nullptr) == (enc_bias == nullptr)) return -1;
   if (enc_bias != nullptr) {
     if (bias_c == nullptr) return -1;  // scratch [L, nd_cap] fp32 for the compact bias
-    aux_gather_bias_kernel<<<dim3((nd_cap + 255) / 256, L), 256, 0, st>>>(enc_bias, bias_is_16, F_pitch, dead_cols, nd, nd_cap, bias_c);
+    launch_chained(aux_gather_bias_kernel, dim3((nd_cap + 255) / 256, L), 256, 0, st, enc_bias, bias_is_16, F_pitch, dead_cols, nd, nd_cap, bias_c);
   }
   const size_t smem = 8 * (size_t(nd_cap) * 2 + 1024);
   static size_t attr_smem = 0;
@@ -392,7 +400,7 @@ extern "C" int CLT_FN(clt_aux_gather_select)(const void* pre, long long ld, long
     if (cudaFuncSetAttribute(aux_gather_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
     attr_smem = smem;
   }
-  aux_gather_select_kernel<<<dim3((B + 7) / 8, L), 256, smem, st>>>(static_cast<const t16*>(pre), ld, layer_stride, enc_bias != nullptr ? bias_c : nullptr, dead_cols,
+  launch_chained(aux_gather_select_kernel, dim3((B + 7) / 8, L), 256, smem, st, static_cast<const t16*>(pre), ld, layer_stride, enc_bias != nullptr ? bias_c : nullptr, dead_cols,
                                                         nd, nd_all, nd_cap, k_aux_max, B, static_cast<t16*>(A));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -408,7 +416,7 @@ extern "C" int CLT_FN(clt_aux_gather_rows)(const CltAuxRowsArgs* a, const int* d
   for (int i = 0; i < 32; ++i) { p.w[i] = static_cast<const t16*>(a->w[i]); p.rows[i] = a->rows[i]; }
   const long long n = 1LL * nd_cap * (d / 8);
   const int gx = int((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-  aux_gather_rows_kernel<<<dim3(gx, L), 256, 0, st>>>(p, dead_cols, nd, nd_cap, d, static_cast<t16*>(W0));
+  launch_chained(aux_gather_rows_kernel, dim3(gx, L), 256, 0, st, p, dead_cols, nd, nd_cap, d, static_cast<t16*>(W0));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -418,7 +426,7 @@ extern "C" int CLT_FN(clt_aux_residual)(const float* recon, const void* bias, in
   if (d % 8 != 0) return -1;
   const long long n = 1LL * B * (d / 8);
   const int gx = int((n + 255) / 256 < 592 ? (n + 255) / 256 : 592);
-  aux_residual_kernel<<<dim3(gx, L), 256, 0, st>>>(recon, bias, bias_is_16, bias_row, sigma, static_cast<t16*>(gs), static_cast<t16*>(g_out), loss,
+  launch_chained(aux_residual_kernel, dim3(gx, L), 256, 0, st, recon, bias, bias_is_16, bias_row, sigma, static_cast<t16*>(gs), static_cast<t16*>(g_out), loss,
                                                    nd, ctl, L, B, d, factor, scale_g);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -426,6 +434,6 @@ extern "C" int CLT_FN(clt_aux_residual)(const float* recon, const void* bias, in
 extern "C" int CLT_FN(clt_rowsum16)(const void* in, float* out, long long rows, int n, cudaStream_t st) {
   if (n % 8 != 0) return -1;
   const int grid = int((rows + 7) / 8 < 1184 ? (rows + 7) / 8 : 1184);
-  rowsum16_kernel<<<grid, 256, 0, st>>>(static_cast<const t16*>(in), out, rows, n);
+  launch_chained(rowsum16_kernel, grid, 256, 0, st, static_cast<const t16*>(in), out, rows, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

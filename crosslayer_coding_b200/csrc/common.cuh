@@ -63,6 +63,48 @@ __device__ __forceinline__ bool clt_in_bounds(long long idx, long long limit, in
 __device__ __forceinline__ bool clt_in_bounds(long long, long long, int*, int) { return true; }
 #endif
 
+// ---------------------------------------------------------------- chained launches
+// The kernels of a step follow one another on a stream, many of them for a few microseconds, and between two of them the chip stood idle for 1 to 2.
+// (73 of 474 us in a step of 48 kernels; 26 of those went, a 512-token inference 365 -> 347 us, a 16-token one 147 -> 139).  The small ones are launched as
+// programmatic dependents: their CTAs take their places as soon as all of the kernel before have started and
+// there is room, and wait there until it is complete and its writes are visible.  Every kernel that is launched so calls chain_wait() first in every
+// thread, before it reads or writes anything; one that did not would let its successor run beside its predecessor.
+// The result is never true; the branch on a value that the compiler does not know keeps every load behind the wait, the read-only ones too, which it may
+// move across statements that write memory.
+__device__ __forceinline__ bool chain_wait() {
+  uint32_t sms;
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;\n\tmov.u32 %0, %%nsmid;" : "=r"(sms) :: "memory");
+  return sms == 0xFFFFFFFFu;
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_kernel(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+}
+// Up to eight CTAs per SM.  CTAs that come early take an SM as the kernel before has divided it between L1 and shared memory, and as long as one of them is
+// there it stays so: larger grids, and the persistent kernels below, would run with fewer CTAs per SM for all of their time (a step with
+// long row updates took 1.2 times as long), where the gap in front of them does not count.
+constexpr unsigned long long kChainedCtas = 8 * 148;
+template <typename... Params, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_kernel(1ULL * grid.x * grid.y * grid.z <= kChainedCtas, kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
+}
+// Kernels whose CTAs stay (GEMMs, row updates): neither early themselves, nor with early CTAs of the next one beside them (which cost the row updates of a
+// GPT-2-shape step 2.5 %), so without chain_wait().
+template <typename... Params, typename... Args>
+inline cudaError_t launch_alone(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_kernel(false, kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
+}
+
 // ~1 s at 2 GHz; every spin-wait in this library gives up after this many cycles.
 constexpr long long kWaitTimeoutCycles = 2000000000LL;
 

@@ -270,6 +270,7 @@ __device__ __forceinline__ void walk_list(const DecodeParams& p, int t, int firs
 // blockIdx.y counts the targets from the last one down: the longest lists come first, so that the short ones fill the tail.
 template <int NV, int TOK, int SPLIT, int R, int WARPS_PER_SM>
 __global__ void __launch_bounds__(32 * TOK * SPLIT, WARPS_PER_SM / (TOK * SPLIT)) decode_walk_kernel(const DecodeParams p) {
+  if (chain_wait()) return;
   constexpr int kWarps = TOK * SPLIT;
   __shared__ __align__(16) float sums[kWarps][NV * 256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -334,6 +335,7 @@ __global__ void __launch_bounds__(32 * TOK * SPLIT, WARPS_PER_SM / (TOK * SPLIT)
 // list (the entries of a token may come in any order) is scanned once per layer.
 template <int NV, int SPLIT, int R, int WARPS_PER_SM>
 __global__ void __launch_bounds__(32 * SPLIT, WARPS_PER_SM / SPLIT) decode_running_kernel(const DecodeParams p) {
+  if (chain_wait()) return;
   __shared__ __align__(16) float sums[2][SPLIT][NV * 256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.d;
@@ -409,6 +411,7 @@ __global__ void __launch_bounds__(32 * SPLIT, WARPS_PER_SM / SPLIT) decode_runni
 // One CTA: a counting sort of a few thousand lengths, 4 us.
 constexpr int kLenClasses = 1024;
 __global__ void __launch_bounds__(kLenClasses) decode_order_kernel(const int* __restrict__ tok_off, int B, int* __restrict__ order) {
+  if (chain_wait()) return;
   __shared__ int place[kLenClasses];
   __shared__ int warp_sums[32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -462,6 +465,7 @@ __global__ void __launch_bounds__(256) recon_epilogue_kernel(const float* __rest
                                                                const float* __restrict__ sigma, t16* __restrict__ gs,
                                                                float* __restrict__ yhat_out, double* __restrict__ sq_err, int L, int B,
                                                                int d, int row0, int nrows, float* __restrict__ ctl) {
+  if (chain_wait()) return;
   const int t = blockIdx.y;
   const float loss_scale = ctl != nullptr ? ctl[SC_LOSS_SCALE] : 1.f;
   bool bad = false;
@@ -514,6 +518,7 @@ __global__ void __launch_bounds__(256) recon_epilogue_kernel(const float* __rest
 // threadIdx.y lanes of a block walk the block's row range, shared memory folds them, one atomic per column and block.
 __global__ void __launch_bounds__(1024) gs_colsum_kernel(const t16* __restrict__ gs, float* __restrict__ out, int B, int d,
                                                           int rows_per_block) {
+  if (chain_wait()) return;
   const int t = blockIdx.z;
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   const int r0 = blockIdx.y * rows_per_block, r1 = min(B, r0 + rows_per_block);
@@ -546,6 +551,7 @@ __global__ void __launch_bounds__(1024) gs_colsum_kernel(const t16* __restrict__
 // Suffix sums of the gradient seed over the layers: out[s] = sum over t >= s of gs[t]  (per_source tied decoders:
 // the threshold-gradient GEMM of source layer s needs the seed of all its targets added up).  fp32 accumulation.
 __global__ void __launch_bounds__(256) gs_suffix_sum_kernel(const t16* __restrict__ gs, t16* __restrict__ out, int L, long long per_layer) {
+  if (chain_wait()) return;
   for (long long i = (blockIdx.x * 1LL * blockDim.x + threadIdx.x) * 8; i < per_layer; i += 1LL * gridDim.x * blockDim.x * 8) {
     float acc[8];
 #pragma unroll
@@ -630,21 +636,21 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   if (a->B <= 0 || a->L <= 0) return 0;
   if (a->order != nullptr && CLT_FN(clt_sparse_decode_scratch)(a) > 0) {
     p.order = a->order;
-    decode_order_kernel<<<1, kLenClasses, 0, st>>>(a->tok_off, a->B, a->order);
+    launch_chained(decode_order_kernel, 1, kLenClasses, 0, st, a->tok_off, a->B, a->order);
   } else {
     p.order = nullptr;
   }
   if (takes_running(a)) {
     const dim3 grid(a->B, running_chunks(a));
     if (one_warp_lists(a) || (a->equal == 0 && a->expected > 0 && a->expected < kRunningOneWarpBelow)) {
-      if (a->d <= 256) decode_running_kernel<1, 1, 4, 28><<<grid, 32, 0, st>>>(p);
-      else decode_running_kernel<2, 1, 4, 16><<<grid, 32, 0, st>>>(p);
+      if (a->d <= 256) launch_chained(decode_running_kernel<1, 1, 4, 28>, grid, 32, 0, st, p);
+      else launch_chained(decode_running_kernel<2, 1, 4, 16>, grid, 32, 0, st, p);
     } else if (short_lists(a) || (a->expected <= 0 && 1LL * a->B * running_chunks(a) >= kRunningTwoWarpsFrom)) {
-      if (a->d <= 256) decode_running_kernel<1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
-      else decode_running_kernel<2, 2, 4, 20><<<grid, 64, 0, st>>>(p);
+      if (a->d <= 256) launch_chained(decode_running_kernel<1, 2, 4, 24>, grid, 64, 0, st, p);
+      else launch_chained(decode_running_kernel<2, 2, 4, 20>, grid, 64, 0, st, p);
     } else {
-      if (a->d <= 256) decode_running_kernel<1, 4, 4, 24><<<grid, 128, 0, st>>>(p);
-      else decode_running_kernel<2, 4, 4, 20><<<grid, 128, 0, st>>>(p);
+      if (a->d <= 256) launch_chained(decode_running_kernel<1, 4, 4, 24>, grid, 128, 0, st, p);
+      else launch_chained(decode_running_kernel<2, 4, 4, 20>, grid, 128, 0, st, p);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
@@ -652,30 +658,30 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   const long long ctas = walk_ctas(a);
   const dim3 grid(a->B, a->L, chunks);
   if (ctas < kEightWarpsBelow) {
-    if (nv <= 1) decode_walk_kernel<1, 1, 8, 4, 32><<<grid, 256, 0, st>>>(p);
-    else if (nv == 2) decode_walk_kernel<2, 1, 8, 4, 24><<<grid, 256, 0, st>>>(p);
-    else if (nv == 3) decode_walk_kernel<3, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
-    else decode_walk_kernel<4, 1, 8, 4, 16><<<grid, 256, 0, st>>>(p);
+    if (nv <= 1) launch_chained(decode_walk_kernel<1, 1, 8, 4, 32>, grid, 256, 0, st, p);
+    else if (nv == 2) launch_chained(decode_walk_kernel<2, 1, 8, 4, 24>, grid, 256, 0, st, p);
+    else if (nv == 3) launch_chained(decode_walk_kernel<3, 1, 8, 4, 16>, grid, 256, 0, st, p);
+    else launch_chained(decode_walk_kernel<4, 1, 8, 4, 16>, grid, 256, 0, st, p);
   } else if (one_warp_lists(a)) {
-    if (nv <= 1) decode_walk_kernel<1, 4, 1, 4, 32><<<dim3((a->B + 3) / 4, a->L), 128, 0, st>>>(p);
-    else if (nv == 2) decode_walk_kernel<2, 2, 1, 4, 24><<<dim3((a->B + 1) / 2, a->L), 64, 0, st>>>(p);
-    else if (nv == 3) decode_walk_kernel<3, 1, 1, 2, 28><<<grid, 32, 0, st>>>(p);
-    else decode_walk_kernel<4, 1, 1, 2, 20><<<grid, 32, 0, st>>>(p);
+    if (nv <= 1) launch_chained(decode_walk_kernel<1, 4, 1, 4, 32>, dim3((a->B + 3) / 4, a->L), 128, 0, st, p);
+    else if (nv == 2) launch_chained(decode_walk_kernel<2, 2, 1, 4, 24>, dim3((a->B + 1) / 2, a->L), 64, 0, st, p);
+    else if (nv == 3) launch_chained(decode_walk_kernel<3, 1, 1, 2, 28>, grid, 32, 0, st, p);
+    else launch_chained(decode_walk_kernel<4, 1, 1, 2, 20>, grid, 32, 0, st, p);
   } else if (nv <= 1) {
-    if (ctas >= kPairNarrowFrom) decode_walk_kernel<1, 2, 2, 4, 40><<<dim3((a->B + 1) / 2, a->L), 128, 0, st>>>(p);
-    else decode_walk_kernel<1, 1, 4, 4, 40><<<grid, 128, 0, st>>>(p);
+    if (ctas >= kPairNarrowFrom) launch_chained(decode_walk_kernel<1, 2, 2, 4, 40>, dim3((a->B + 1) / 2, a->L), 128, 0, st, p);
+    else launch_chained(decode_walk_kernel<1, 1, 4, 4, 40>, grid, 128, 0, st, p);
   } else if (short_lists(a) && ctas >= kShortFrom) {
-    if (nv == 2) decode_walk_kernel<2, 1, 2, 4, 24><<<grid, 64, 0, st>>>(p);
-    else if (nv == 3) decode_walk_kernel<3, 1, 2, 2, 28><<<grid, 64, 0, st>>>(p);
-    else decode_walk_kernel<4, 1, 2, 2, 20><<<grid, 64, 0, st>>>(p);
+    if (nv == 2) launch_chained(decode_walk_kernel<2, 1, 2, 4, 24>, grid, 64, 0, st, p);
+    else if (nv == 3) launch_chained(decode_walk_kernel<3, 1, 2, 2, 28>, grid, 64, 0, st, p);
+    else launch_chained(decode_walk_kernel<4, 1, 2, 2, 20>, grid, 64, 0, st, p);
   } else if (nv == 2) {
-    decode_walk_kernel<2, 1, 4, 4, 24><<<grid, 128, 0, st>>>(p);
+    launch_chained(decode_walk_kernel<2, 1, 4, 4, 24>, grid, 128, 0, st, p);
   } else if (ctas >= kManyCtas) {
-    if (nv == 3) decode_walk_kernel<3, 1, 4, 2, 28><<<grid, 128, 0, st>>>(p);
-    else decode_walk_kernel<4, 1, 4, 2, 20><<<grid, 128, 0, st>>>(p);
+    if (nv == 3) launch_chained(decode_walk_kernel<3, 1, 4, 2, 28>, grid, 128, 0, st, p);
+    else launch_chained(decode_walk_kernel<4, 1, 4, 2, 20>, grid, 128, 0, st, p);
   } else {
-    if (nv == 3) decode_walk_kernel<3, 1, 4, 4, 20><<<grid, 128, 0, st>>>(p);
-    else decode_walk_kernel<4, 1, 4, 4, 16><<<grid, 128, 0, st>>>(p);
+    if (nv == 3) launch_chained(decode_walk_kernel<3, 1, 4, 4, 20>, grid, 128, 0, st, p);
+    else launch_chained(decode_walk_kernel<4, 1, 4, 4, 16>, grid, 128, 0, st, p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -686,7 +692,7 @@ extern "C" int CLT_FN(clt_recon_epilogue)(const float* yhat_sum, const float* bi
   if (d % 8 != 0) return -1;
   if (nrows <= 0) return 0;
   dim3 grid(148, L);
-  recon_epilogue_kernel<<<grid, 256, 0, st>>>(yhat_sum, bias_sum, addend, static_cast<const t16*>(target), sigma,
+  launch_chained(recon_epilogue_kernel, grid, 256, 0, st, yhat_sum, bias_sum, addend, static_cast<const t16*>(target), sigma,
                                               static_cast<t16*>(gs), yhat_out, sq_err, L, B, d, row0, nrows, ctl);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -697,7 +703,7 @@ extern "C" int CLT_FN(clt_gs_colsum)(const void* gs, float* out, int L, int B, i
   const int ty = 1024 / tx < 8 ? 1024 / tx : 8;
   const int rpb = 128;
   dim3 grid((d / 8 + tx - 1) / tx, (B + rpb - 1) / rpb, L), block(tx, ty);
-  gs_colsum_kernel<<<grid, block, 0, st>>>(static_cast<const t16*>(gs), out, B, d, rpb);
+  launch_chained(gs_colsum_kernel, grid, block, 0, st, static_cast<const t16*>(gs), out, B, d, rpb);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -706,6 +712,6 @@ extern "C" int CLT_FN(clt_gs_suffix_sum)(const void* gs, void* out, int L, int B
   if (per_layer % 8 != 0) return -1;
   const long long nvec = per_layer / 8;
   const int grid = int(nvec / 256 + 1 < 1184 ? nvec / 256 + 1 : 1184);
-  gs_suffix_sum_kernel<<<grid, 256, 0, st>>>(static_cast<const t16*>(gs), static_cast<t16*>(out), L, per_layer);
+  launch_chained(gs_suffix_sum_kernel, grid, 256, 0, st, static_cast<const t16*>(gs), static_cast<t16*>(out), L, per_layer);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -237,6 +237,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 // out[l][c, r] = in[l][r, c] for 16-bit elements, 64 x 64 tiles through shared memory.
 __global__ void __launch_bounds__(256) transpose16_kernel(const t16* __restrict__ in, t16* __restrict__ out, int R, int C, long long ld_in,
                                                             long long layer_stride_in) {
+  if (chain_wait()) return;
   __shared__ t16 tile[64][66];
   const int l = blockIdx.z;
   const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__(256) transpose16_kernel(const t16* __restrict_
 // selection, applied while the gradient is transposed for the GEMM that consumes it.
 __global__ void __launch_bounds__(256) transpose16_vec_kernel(const t16* __restrict__ in, const t16* __restrict__ mask, t16* __restrict__ out, int R,
                                                                 int C, long long ld_in, long long layer_stride_in) {
+  if (chain_wait()) return;
   __shared__ uint32_t tile[64][33];  // 64 rows x 64 elements, two per word
   const int l = blockIdx.z;
   const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
@@ -305,6 +307,7 @@ __global__ void __launch_bounds__(256) transpose16_vec_kernel(const t16* __restr
 __global__ void __launch_bounds__(256) negative_indicator_kernel(const t16* __restrict__ pre, t16* __restrict__ ind, float* __restrict__ bias_grad,
                                                                    double* __restrict__ loss, int B, int F, int F_valid, long long ld,
                                                                    float coef_over_numel) {
+  if (chain_wait()) return;
   __shared__ t16 tile[64][66];
   __shared__ float colsum[64];
   __shared__ float red[8];
@@ -401,8 +404,8 @@ extern "C" int CLT_FN(clt_dense_gemm)(const void* A, int LA, long long lda, long
   const long long tiles = 1LL * G * ((M + dg::BM - 1) / dg::BM) * ((N + dg::BN - 1) / dg::BN);
   const int grid = int(tiles < num_sms ? tiles : num_sms);
   const int2* sp = reinterpret_cast<const int2*>(segs);
-  if (out_f32) dense_gemm_kernel<true><<<grid, dg::NUM_THREADS, dg::SMEM_BYTES, stream>>>(map_a, map_b, map_c, group_off, sp, G, M, N, K, alpha, status);
-  else dense_gemm_kernel<false><<<grid, dg::NUM_THREADS, dg::SMEM_BYTES, stream>>>(map_a, map_b, map_c, group_off, sp, G, M, N, K, alpha, status);
+  if (out_f32) launch_alone(dense_gemm_kernel<true>, grid, dg::NUM_THREADS, dg::SMEM_BYTES, stream, map_a, map_b, map_c, group_off, sp, G, M, N, K, alpha, status);
+  else launch_alone(dense_gemm_kernel<false>, grid, dg::NUM_THREADS, dg::SMEM_BYTES, stream, map_a, map_b, map_c, group_off, sp, G, M, N, K, alpha, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -413,12 +416,12 @@ extern "C" int CLT_FN(clt_transpose16)(const void* in, void* out, int L, int R, 
   const bool vec = R % 8 == 0 && C % 8 == 0 && ld_in % 8 == 0 && layer_stride_in % 8 == 0 &&
                    ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(mask)) & 15) == 0;
   if (vec) {
-    transpose16_vec_kernel<<<grid, 256, 0, st>>>(static_cast<const t16*>(in), static_cast<const t16*>(mask), static_cast<t16*>(out), R, C, ld_in,
+    launch_chained(transpose16_vec_kernel, grid, 256, 0, st, static_cast<const t16*>(in), static_cast<const t16*>(mask), static_cast<t16*>(out), R, C, ld_in,
                                                  layer_stride_in);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
   if (mask != nullptr) return -1;  // the masked form needs the 16-byte layout
-  transpose16_kernel<<<grid, 256, 0, st>>>(static_cast<const t16*>(in), static_cast<t16*>(out), R, C, ld_in, layer_stride_in);
+  launch_chained(transpose16_kernel, grid, 256, 0, st, static_cast<const t16*>(in), static_cast<t16*>(out), R, C, ld_in, layer_stride_in);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -426,7 +429,7 @@ extern "C" int CLT_FN(clt_negative_indicator)(const void* pre, void* ind, float*
                                               long long ld, float coef_over_numel, cudaStream_t st) {
   if (L <= 0 || B <= 0 || F <= 0) return 0;
   dim3 grid((F + 63) / 64, (B + 63) / 64, L);
-  negative_indicator_kernel<<<grid, 256, 0, st>>>(static_cast<const t16*>(pre), static_cast<t16*>(ind), bias_grad, loss, B, F, F_valid, ld,
+  launch_chained(negative_indicator_kernel, grid, 256, 0, st, static_cast<const t16*>(pre), static_cast<t16*>(ind), bias_grad, loss, B, F, F_valid, ld,
                                                   coef_over_numel);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -822,7 +822,7 @@ static int launch_single(const CUtensorMap& map_a, const CUtensorMap& map_b, con
   }
   const long long tiles = 1LL * L * ((M + gemm::BM - 1) / gemm::BM) * ((N + gemm::BN - 1) / gemm::BN);
   const int grid = int(tiles < num_sms ? tiles : num_sms);
-  kernel<<<grid, gemm::NUM_THREADS, smem, stream>>>(map_a, map_b, map_c, bias, L, M, N, K, ldc, layer_stride_c, status, tile_stats);
+  launch_alone(kernel, grid, gemm::NUM_THREADS, smem, stream, map_a, map_b, map_c, bias, L, M, N, K, ldc, layer_stride_c, status, tile_stats);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

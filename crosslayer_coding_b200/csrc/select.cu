@@ -82,6 +82,7 @@ template <int VEC>
 __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x, float* __restrict__ mean,
                                                          float* __restrict__ rstd, int B, int F, long long ld,
                                                          long long layer_stride, long long first_strip) {
+  if (chain_wait()) return;
   using Ld = ColstatsLoad<VEC>;
   constexpr int kBlocks = 8 / VEC;  // of 32 * VEC columns in a strip
   constexpr int kDepth = Ld::kDepth;
@@ -146,6 +147,7 @@ __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x
 // large against the spread.
 __global__ void __launch_bounds__(256) colstats_from_tiles_kernel(const float* __restrict__ tile_stats, float* __restrict__ mean,
                                                                     float* __restrict__ rstd, int B, int F, int row_blocks, long long n) {
+  if (chain_wait()) return;
   const long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int l = int(i / F), c = int(i - 1LL * l * F);
@@ -171,6 +173,7 @@ __global__ void __launch_bounds__(256) colstats_from_tiles_kernel(const float* _
 __global__ void __launch_bounds__(256) colstats_finalize_kernel(const t16* __restrict__ x, float* __restrict__ mean,
                                                                   float* __restrict__ rstd, int B, int F, long long layer_stride,
                                                                   long long first, long long n) {
+  if (chain_wait()) return;
   const long long i = first + blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int l = int(i / F), c = int(i - 1LL * l * F);
@@ -197,6 +200,7 @@ __global__ void __launch_bounds__(256) zhist_kernel(const t16* __restrict__ x, c
                                                       const float* __restrict__ rstd, ScanGeom g, uint32_t key_lo, int shift,
                                                       unsigned int* __restrict__ hist, const long long* __restrict__ ctl,
                                                       int only_if_retry) {
+  if (chain_wait()) return;
   if (only_if_retry && ctl[CTL_RETRY] == 0) return;
   const float z_lo = key_lo == 0u ? -INFINITY : key_to_float(key_lo);
   __shared__ unsigned int sh[kHistBins];
@@ -273,6 +277,7 @@ __global__ void __launch_bounds__(256) zhist_collect_kernel(const t16* __restric
                                                               const float* __restrict__ rstd, ScanGeom g, int col_pitch,
                                                               const long long* __restrict__ sel_state,
                                                               unsigned int* __restrict__ hist, Pool pool) {
+  if (chain_wait()) return;
   const uint32_t key_lo = uint32_t(sel_state[0]);
   const int shift = int(sel_state[1]);
   const float z_lo = key_to_float(key_lo);
@@ -403,6 +408,7 @@ __global__ void __launch_bounds__(1024) find_bin_kernel(const unsigned int* __re
                                                           long long* __restrict__ sel_state,
                                                           const unsigned int* __restrict__ pool_count, long long pool_cap,
                                                           int* __restrict__ status) {
+  if (chain_wait()) return;
   __shared__ uint32_t vals[kHistBins + kHistExtra];
   __shared__ unsigned long long part[1024];
   __shared__ int timeout;
@@ -518,6 +524,7 @@ __global__ void __launch_bounds__(1024) find_bin_kernel(const unsigned int* __re
 __global__ void __launch_bounds__(256) threshold_collect_kernel(const t16* __restrict__ x, const float* __restrict__ theta,
                                                                   ScanGeom g, int col_pitch, long long* __restrict__ ctl,
                                                                   Lists o, int* __restrict__ status) {
+  if (chain_wait()) return;
   __shared__ uint32_t s_queue[4 * kHitQueue];
   __shared__ int s_tok[2 * kPoolStage];
   __shared__ int s_col[2 * kPoolStage];
@@ -643,6 +650,7 @@ __device__ __forceinline__ void token_rows_scan(const t16* __restrict__ x, const
 __global__ void __launch_bounds__(256) token_topk_kernel(const t16* __restrict__ x, const float* __restrict__ mean,
                                                            const float* __restrict__ rstd, ScanGeom g, int col_pitch, int f_valid, int k,
                                                            long long* __restrict__ ctl, Lists o, int* __restrict__ status, int only_marked) {
+  if (chain_wait()) return;
   extern __shared__ uint8_t tk_smem[];
   TokenTopkShared* sh = reinterpret_cast<TokenTopkShared*>(tk_smem);
   const int tok0 = blockIdx.x * kTokPerCta;
@@ -775,6 +783,7 @@ __device__ __forceinline__ void token_keys_scan(const t16* __restrict__ x, const
 template <int TPC>
 __global__ void __launch_bounds__(kTkThreads) token_topk_list_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd,
                                                                      ScanGeom g, int col_pitch, int f_valid, int k, int step, long long* __restrict__ ctl, Lists o) {
+  if (chain_wait()) return;
   extern __shared__ __align__(16) uint8_t tl_smem[];
   TokenListShared<TPC>* sh = reinterpret_cast<TokenListShared<TPC>*>(tl_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -896,6 +905,7 @@ __device__ __forceinline__ float t16_of(const uint4& v, int j) {
 
 __global__ void __launch_bounds__(256) token_sample_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
                                                              int f_valid, WideTopk wt) {
+  if (chain_wait()) return;
   const int sg = blockIdx.x * 256 + threadIdx.x;  // < ng, a multiple of 256
   const int q = (sg >> 5) * 32 * kWideStep + (sg & 31);  // runs of 32 groups: short enough that a sample meets every layer
   const int r0 = blockIdx.y * kWideRows, r1 = min(g.B, r0 + kWideRows);
@@ -926,6 +936,7 @@ __global__ void __launch_bounds__(256) token_sample_kernel(const t16* __restrict
 }
 
 __global__ void __launch_bounds__(256) token_bound_kernel(WideTopk wt, int k, long long* __restrict__ ctl, long long n_entries) {
+  if (chain_wait()) return;
   __shared__ int total[2];
   const int tok = blockIdx.x;
   if (tok == 0 && threadIdx.x == 0) ctl[CTL_NUM_ENTRIES] = n_entries;
@@ -957,6 +968,7 @@ __global__ void __launch_bounds__(256) token_bound_kernel(WideTopk wt, int k, lo
 
 __global__ void __launch_bounds__(256) token_collect_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
                                                               int col_pitch, int f_valid, WideTopk wt) {
+  if (chain_wait()) return;
   __shared__ uint16_t queue[kWideQueue];
   __shared__ float z_scaled[kWideRows];
   __shared__ uint32_t bound[kWideRows];
@@ -1029,6 +1041,7 @@ __global__ void __launch_bounds__(256) token_collect_kernel(const t16* __restric
 // W: words per lane (cap <= 32 W).
 template <int W>
 __global__ void __launch_bounds__(128) token_cut_kernel(const t16* __restrict__ x, ScanGeom g, int col_pitch, int k, WideTopk wt, Lists o) {
+  if (chain_wait()) return;
   const int tok = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (tok >= g.B) return;
   const int n = wt.n[tok];
@@ -1072,6 +1085,7 @@ __global__ void __launch_bounds__(128) token_cut_kernel(const t16* __restrict__ 
 // Runs instead of the full compaction pass when the tracked range contained the cut.
 __global__ void __launch_bounds__(256) classify_pool_kernel(Pool pool, long long* __restrict__ ctl, Lists o,
                                                               int* __restrict__ status) {
+  if (chain_wait()) return;
   if (ctl[CTL_RETRY] != 0) return;
   const uint32_t tbin = uint32_t(ctl[CTL_BIN]);
   const uint32_t key_lo = uint32_t(ctl[CTL_KEY_LO]);
@@ -1126,6 +1140,7 @@ __global__ void __launch_bounds__(256) compact_kernel(const t16* __restrict__ x,
                                                         const float* __restrict__ rstd, ScanGeom g, int col_pitch,
                                                         long long* __restrict__ ctl, Lists o, int* __restrict__ status,
                                                         int only_if_retry) {
+  if (chain_wait()) return;
   if (only_if_retry && ctl[CTL_RETRY] == 0) return;
   __shared__ int s_tok[kStageCap];
   __shared__ int s_col[kStageCap];
@@ -1261,6 +1276,7 @@ __global__ void __launch_bounds__(1024) refine_kernel(const uint32_t* __restrict
                                                         const int* __restrict__ cand_col, long long cand_cap,
                                                         FlatGeom fg, long long* __restrict__ ctl, Exchange ex,
                                                         int* __restrict__ status) {
+  if (chain_wait()) return;
   const int shift = int(ctl[CTL_SHIFT]);
   const uint32_t key_lo = uint32_t(ctl[CTL_KEY_LO]);  // bins are over (key - key_lo): refine on the same offset
   __shared__ uint32_t hist[kRefineBins];
@@ -1433,6 +1449,7 @@ __global__ void __launch_bounds__(1024) refine_kernel(const uint32_t* __restrict
 // ------------------------------------------------------------------ 6. append the kept candidates
 __global__ void __launch_bounds__(256) finalize_kernel(Lists o, FlatGeom fg, long long* __restrict__ ctl,
                                                          int* __restrict__ status) {
+  if (chain_wait()) return;
   const int shift = int(ctl[CTL_SHIFT]);
   const uint32_t key_lo = uint32_t(ctl[CTL_KEY_LO]);
   long long n = ctl[CTL_NUM_CAND];
@@ -1463,6 +1480,7 @@ __global__ void __launch_bounds__(256) csr_count_kernel(const int* __restrict__ 
                                                           const long long* __restrict__ ctl, int* __restrict__ tok_cnt,
                                                           int* __restrict__ feat_cnt, unsigned char* __restrict__ fired,
                                                           int num_tokens, int num_cols) {
+  if (chain_wait()) return;
   long long n = ctl[CTL_NUM_ENTRIES];
   if (n > cap) n = cap;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
@@ -1481,6 +1499,7 @@ __global__ void __launch_bounds__(256) csr_count_kernel(const int* __restrict__ 
 // entries.  cursor (optional) gets a copy of the offsets for the scatter pass.
 __global__ void __launch_bounds__(1024) exclusive_scan_kernel(const int* __restrict__ in, int* __restrict__ out,
                                                                 int* __restrict__ cursor, int n) {
+  if (chain_wait()) return;
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1538,6 +1557,7 @@ struct ScanJob {
   int n;
 };
 __global__ void __launch_bounds__(1024) exclusive_scan_tiles_kernel(ScanJob ja, ScanJob jb, int tiles_a) {
+  if (chain_wait()) return;
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1608,10 +1628,10 @@ static void launch_exclusive_scans(const ScanJob& a, const ScanJob& b, cudaStrea
   const int ta = (a.n + 4095) / 4096, tb = (b.n + 4095) / 4096;
   const bool aligned = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(b.in)) & 15) == 0;
   if (a.n > 0 && b.n > 0 && ta <= 512 && tb <= 512 && aligned) {
-    exclusive_scan_tiles_kernel<<<ta + tb, 1024, 0, st>>>(a, b, ta);
+    launch_chained(exclusive_scan_tiles_kernel, ta + tb, 1024, 0, st, a, b, ta);
   } else {
-    exclusive_scan_kernel<<<1, 1024, 0, st>>>(a.in, a.out, a.cursor, a.n);
-    exclusive_scan_kernel<<<1, 1024, 0, st>>>(b.in, b.out, b.cursor, b.n);
+    launch_chained(exclusive_scan_kernel, 1, 1024, 0, st, a.in, a.out, a.cursor, a.n);
+    launch_chained(exclusive_scan_kernel, 1, 1024, 0, st, b.in, b.out, b.cursor, b.n);
   }
 }
 
@@ -1622,6 +1642,7 @@ __global__ void __launch_bounds__(256) csr_scatter_kernel(const int* __restrict_
                                                             float* __restrict__ tcsr_val, int* __restrict__ fcsr_tok,
                                                             float* __restrict__ fcsr_val, int col_pitch, int num_tokens, int num_cols,
                                                             const int* __restrict__ feat_off, int* __restrict__ layer_cnt) {
+  if (chain_wait()) return;
   if (layer_cnt != nullptr && blockIdx.x == 0) {  // entries per layer: the offsets are complete
     for (int l = threadIdx.x; 1LL * l * col_pitch < num_cols; l += blockDim.x)
       layer_cnt[l] = feat_off[min(1LL * (l + 1) * col_pitch, 1LL * num_cols)] - feat_off[1LL * l * col_pitch];
@@ -1645,6 +1666,7 @@ __global__ void __launch_bounds__(256) csr_scatter_kernel(const int* __restrict_
 __global__ void __launch_bounds__(256) csr_token_count_kernel(const int* __restrict__ ent_tok, const int* __restrict__ ent_col, long long cap,
                                                                 const long long* __restrict__ ctl, int* __restrict__ tok_cnt, int* __restrict__ layer_cnt,
                                                                 int col_pitch, int num_tokens, int num_cols) {
+  if (chain_wait()) return;
   __shared__ int per_layer[32];
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 32) per_layer[threadIdx.x] = 0;
@@ -1668,6 +1690,7 @@ __global__ void __launch_bounds__(256) csr_token_scatter_kernel(const int* __res
                                                                   const float* __restrict__ ent_val, long long cap, const long long* __restrict__ ctl,
                                                                   int* __restrict__ tok_cursor, int* __restrict__ tcsr_col, float* __restrict__ tcsr_val,
                                                                   int col_pitch, int num_tokens, int num_cols) {
+  if (chain_wait()) return;
   long long n = ctl[CTL_NUM_ENTRIES];
   if (n > cap) n = cap;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
@@ -1724,6 +1747,7 @@ constexpr int kShortSegment = 32;
 constexpr int kFeatSortCap = 4096;
 __global__ void __launch_bounds__(256) csr_sort_feature_segments_kernel(const int* __restrict__ off, int nseg, int per_cta,
                                                                           int* __restrict__ key, float* __restrict__ val) {
+  if (chain_wait()) return;
   __shared__ unsigned long long w[kFeatSortCap];
   __shared__ int long_list[256];
   __shared__ int long_count;
@@ -1888,6 +1912,7 @@ __device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float
 
 __global__ void __launch_bounds__(256) csr_sort_token_segments_kernel(const int* __restrict__ off, int* __restrict__ key, float* __restrict__ val, int rank_up_to,
                                                                          int bucket_up_to) {
+  if (chain_wait()) return;
   __shared__ __align__(16) unsigned long long w[(kTokenBucketRoom + kTokenSortCap) / 2];
   __shared__ int count[kTokenBuckets], base[kTokenBuckets], start[kTokenBuckets];
   const int b = off[blockIdx.x], n = off[blockIdx.x + 1] - b;
@@ -1916,11 +1941,12 @@ static void launch_token_sort(const int* off, int* key, float* val, int num_toke
   if (num_tokens <= 0) return;
   const int layers = (num_cols + col_pitch - 1) / col_pitch;
   const int rank_up_to = num_tokens < kFewTokens ? 512 : (layers <= 1 ? 256 : 128);
-  csr_sort_token_segments_kernel<<<num_tokens, 256, 0, st>>>(off, key, val, rank_up_to, layers < 8 ? layers * kTokenBucketCap : kTokenSortCap);
+  launch_chained(csr_sort_token_segments_kernel, num_tokens, 256, 0, st, off, key, val, rank_up_to, layers < 8 ? layers * kTokenBucketCap : kTokenSortCap);
 }
 
 // Dead-feature counters: +1 per step, reset where the feature fired (reference trainer.py:693-712).
 __global__ void __launch_bounds__(256) dead_counter_kernel(long long* __restrict__ counter, unsigned char* __restrict__ fired, int n) {
+  if (chain_wait()) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     counter[i] = fired[i] ? 0 : counter[i] + 1;
     fired[i] = 0;
@@ -1961,10 +1987,10 @@ extern "C" int CLT_FN(clt_colstats_strips)(const void* x, float* mean, float* rs
     if (cudaMemsetAsync(rstd + first, 0, sizeof(float) * size_t(n - first), st) != cudaSuccess) return -5;
   }
   if (first_strip > 0)  // the rest of a GEMM: less than one strip for each pair of SMs
-    colstats_kernel<2><<<dim3(unsigned(4 * todo), 1, zsplit), block, 0, st>>>(xp, mean, rstd, B, F, ld, layer_stride, first_strip);
+    launch_chained(colstats_kernel<2>, dim3(unsigned(4 * todo), 1, zsplit), block, 0, st, xp, mean, rstd, B, F, ld, layer_stride, first_strip);
   else
-    colstats_kernel<8><<<dim3(unsigned(todo), 1, zsplit), block, 0, st>>>(xp, mean, rstd, B, F, ld, layer_stride, 0);
-  if (zsplit > 1) colstats_finalize_kernel<<<int((n - first + 255) / 256), 256, 0, st>>>(xp, mean, rstd, B, F, layer_stride, first, n);
+    launch_chained(colstats_kernel<8>, dim3(unsigned(todo), 1, zsplit), block, 0, st, xp, mean, rstd, B, F, ld, layer_stride, 0);
+  if (zsplit > 1) launch_chained(colstats_finalize_kernel, int((n - first + 255) / 256), 256, 0, st, xp, mean, rstd, B, F, layer_stride, first, n);
   *kernels = zsplit > 1 ? 2 : 1;
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -1978,7 +2004,7 @@ extern "C" int CLT_FN(clt_colstats)(const void* x, float* mean, float* rstd, int
 extern "C" int clt_colstats_from_tiles(const float* tile_stats, float* mean, float* rstd, int L, int B, int F, cudaStream_t st) {
   const long long n = 1LL * L * F;
   if (n == 0) return 0;
-  colstats_from_tiles_kernel<<<int((n + 255) / 256), 256, 0, st>>>(tile_stats, mean, rstd, B, F, (B + 127) / 128, n);
+  launch_chained(colstats_from_tiles_kernel, int((n + 255) / 256), 256, 0, st, tile_stats, mean, rstd, B, F, (B + 127) / 128, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -2061,24 +2087,24 @@ extern "C" int CLT_FN(clt_batchtopk_select)(const CltSelectArgs* a, const CltExc
     Pool pool;
     pool.key = a->pool_key; pool.tok = a->pool_tok; pool.col = a->pool_col; pool.val = a->pool_val; pool.cap = a->pool_cap;
     pool.count = a->hist + 2 * kHistBins;
-    zhist_collect_kernel<<<grid, 256, 0, st>>>(x, a->mean, a->rstd, g, a->col_pitch, a->sel_state, a->hist, pool);
-    find_bin_kernel<<<1, 1024, 0, st>>>(a->hist, a->k_total, a->ctl, ex, 0u, 0, 0, 0, a->sel_state, pool.count, pool.cap, a->status);
-    classify_pool_kernel<<<592, 256, 0, st>>>(pool, a->ctl, lists_of(a), a->status);
+    launch_chained(zhist_collect_kernel, grid, 256, 0, st, x, a->mean, a->rstd, g, a->col_pitch, a->sel_state, a->hist, pool);
+    launch_chained(find_bin_kernel, 1, 1024, 0, st, a->hist, a->k_total, a->ctl, ex, 0u, 0, 0, 0, a->sel_state, pool.count, pool.cap, a->status);
+    launch_chained(classify_pool_kernel, 592, 256, 0, st, pool, a->ctl, lists_of(a), a->status);
     // fallback, skipped inside the kernels unless the tracked range missed the cut or the pool overflowed
-    zhist_kernel<<<grid, 256, 0, st>>>(x, a->mean, a->rstd, g, 0u, 19, a->hist + kHistBins, a->ctl, 1);
-    find_bin_kernel<<<1, 1024, 0, st>>>(a->hist + kHistBins, a->k_total, a->ctl, ex, 0u, 19, 1, 1, a->sel_state, nullptr, 0, a->status);
-    compact_kernel<<<grid, 256, 0, st>>>(x, a->mean, a->rstd, g, a->col_pitch, a->ctl, lists_of(a), a->status, 1);
+    launch_chained(zhist_kernel, grid, 256, 0, st, x, a->mean, a->rstd, g, 0u, 19, a->hist + kHistBins, a->ctl, 1);
+    launch_chained(find_bin_kernel, 1, 1024, 0, st, a->hist + kHistBins, a->k_total, a->ctl, ex, 0u, 19, 1, 1, a->sel_state, nullptr, 0, a->status);
+    launch_chained(compact_kernel, grid, 256, 0, st, x, a->mean, a->rstd, g, a->col_pitch, a->ctl, lists_of(a), a->status, 1);
   } else {
-    zhist_kernel<<<grid, 256, 0, st>>>(x, a->mean, a->rstd, g, a->key_lo, a->shift, a->hist, a->ctl, 0);
-    find_bin_kernel<<<1, 1024, 0, st>>>(a->hist, a->k_total, a->ctl, ex, a->key_lo, a->shift, 0, 0, nullptr, nullptr, 0, a->status);
+    launch_chained(zhist_kernel, grid, 256, 0, st, x, a->mean, a->rstd, g, a->key_lo, a->shift, a->hist, a->ctl, 0);
+    launch_chained(find_bin_kernel, 1, 1024, 0, st, a->hist, a->k_total, a->ctl, ex, a->key_lo, a->shift, 0, 0, nullptr, nullptr, 0, a->status);
     if (a->key_lo != 0) {
-      zhist_kernel<<<grid, 256, 0, st>>>(x, a->mean, a->rstd, g, 0u, 19, a->hist + kHistBins, a->ctl, 1);
-      find_bin_kernel<<<1, 1024, 0, st>>>(a->hist + kHistBins, a->k_total, a->ctl, ex, 0u, 19, 1, 1, nullptr, nullptr, 0, a->status);
+      launch_chained(zhist_kernel, grid, 256, 0, st, x, a->mean, a->rstd, g, 0u, 19, a->hist + kHistBins, a->ctl, 1);
+      launch_chained(find_bin_kernel, 1, 1024, 0, st, a->hist + kHistBins, a->k_total, a->ctl, ex, 0u, 19, 1, 1, nullptr, nullptr, 0, a->status);
     }
-    compact_kernel<<<grid, 256, 0, st>>>(x, a->mean, a->rstd, g, a->col_pitch, a->ctl, lists_of(a), a->status, 0);
+    launch_chained(compact_kernel, grid, 256, 0, st, x, a->mean, a->rstd, g, a->col_pitch, a->ctl, lists_of(a), a->status, 0);
   }
-  refine_kernel<<<1, 1024, 0, st>>>(a->cand_key, a->cand_tok, a->cand_col, a->cand_cap, flat_geom(a), a->ctl, ex, a->status);
-  finalize_kernel<<<256, 256, 0, st>>>(lists_of(a), flat_geom(a), a->ctl, a->status);
+  launch_chained(refine_kernel, 1, 1024, 0, st, a->cand_key, a->cand_tok, a->cand_col, a->cand_cap, flat_geom(a), a->ctl, ex, a->status);
+  launch_chained(finalize_kernel, 256, 256, 0, st, lists_of(a), flat_geom(a), a->ctl, a->status);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -2089,7 +2115,7 @@ extern "C" int CLT_FN(clt_threshold_select)(const CltSelectArgs* a, cudaStream_t
   const ScanGeom g = scan_geom(a);
   dim3 grid(((a->F + 7) / 8 + 255) / 256, (a->B + g.rows_per_block - 1) / g.rows_per_block, a->L);
   if (cudaMemsetAsync(a->ctl + CTL_NUM_ENTRIES, 0, sizeof(long long), st) != cudaSuccess) return -5;
-  threshold_collect_kernel<<<grid, 256, 0, st>>>(static_cast<const t16*>(a->x), a->rstd, g, a->col_pitch, a->ctl, lists_of(a), a->status);
+  launch_chained(threshold_collect_kernel, grid, 256, 0, st, static_cast<const t16*>(a->x), a->rstd, g, a->col_pitch, a->ctl, lists_of(a), a->status);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -2103,7 +2129,7 @@ static int launch_token_list(const CltSelectArgs* a, const ScanGeom& g, int f_va
   step = step > 8 ? 8 : step;
   if (step > groups / (2 * kTkMaxima)) step = groups / (2 * kTkMaxima);
   if (step < 1) step = 1;
-  token_topk_list_kernel<TPC><<<(a->B + TPC - 1) / TPC, kTkThreads, sizeof(TokenListShared<TPC>), st>>>(
+  launch_chained(token_topk_list_kernel<TPC>, (a->B + TPC - 1) / TPC, kTkThreads, sizeof(TokenListShared<TPC>), st, 
       static_cast<const t16*>(a->x), a->mean, a->rstd, g, a->col_pitch, f_valid, k, step, a->ctl, lists_of(a));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -2165,11 +2191,11 @@ extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, void* scrat
     const t16* x = static_cast<const t16*>(a->x);
     const int row_blocks = (a->B + kWideRows - 1) / kWideRows;
     if (cudaMemsetAsync(w.n, 0, sizeof(int) * size_t(a->B), st) != cudaSuccess) return -5;
-    token_sample_kernel<<<dim3(w.ng / 256, row_blocks), 256, 0, st>>>(x, a->mean, a->rstd, g, f_valid, w);
-    token_bound_kernel<<<a->B, 256, 0, st>>>(w, int(k), a->ctl, 1LL * a->B * k);
-    token_collect_kernel<<<dim3((a->F / 8 + 255) / 256, row_blocks, a->L), 256, 0, st>>>(x, a->mean, a->rstd, g, a->col_pitch, f_valid, w);
-    if (w.cap <= 1024) token_cut_kernel<32><<<(a->B + 3) / 4, 128, 0, st>>>(x, g, a->col_pitch, int(k), w, lists_of(a));
-    else token_cut_kernel<64><<<(a->B + 3) / 4, 128, 0, st>>>(x, g, a->col_pitch, int(k), w, lists_of(a));
+    launch_chained(token_sample_kernel, dim3(w.ng / 256, row_blocks), 256, 0, st, x, a->mean, a->rstd, g, f_valid, w);
+    launch_chained(token_bound_kernel, a->B, 256, 0, st, w, int(k), a->ctl, 1LL * a->B * k);
+    launch_chained(token_collect_kernel, dim3((a->F / 8 + 255) / 256, row_blocks, a->L), 256, 0, st, x, a->mean, a->rstd, g, a->col_pitch, f_valid, w);
+    if (w.cap <= 1024) launch_chained(token_cut_kernel<32>, (a->B + 3) / 4, 128, 0, st, x, g, a->col_pitch, int(k), w, lists_of(a));
+    else launch_chained(token_cut_kernel<64>, (a->B + 3) / 4, 128, 0, st, x, g, a->col_pitch, int(k), w, lists_of(a));
   } else if (list) {
     // Tokens per CTA: what finishes in one wave of 148 SMs with four CTAs each (three of four tokens, whose lists are 64 KB).  More
     // tokens per CTA share the loads of the column statistics but take longer each, so one token while all fit that way, then
@@ -2182,7 +2208,7 @@ extern "C" int CLT_FN(clt_token_topk_select)(const CltSelectArgs* a, void* scrat
                                                                    : launch_token_list<2>(a, g, f_valid, int(k), st);
     if (rc != 0) return rc;
   }
-  token_topk_kernel<<<grid, 256, sizeof(TokenTopkShared), st>>>(static_cast<const t16*>(a->x), a->mean, a->rstd, g, a->col_pitch,
+  launch_chained(token_topk_kernel, grid, 256, sizeof(TokenTopkShared), st, static_cast<const t16*>(a->x), a->mean, a->rstd, g, a->col_pitch,
                                                                  f_valid, int(k), a->ctl, lists_of(a), a->status, list ? 1 : 0);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -2214,6 +2240,7 @@ struct CltTopkTpArgs {
 };
 
 __global__ void __launch_bounds__(256) token_topk_push_kernel(CltTopkTpArgs a) {
+  if (chain_wait()) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl[CTL_NUM_ENTRIES] = 0;  // refilled by the filter pass
   const long long n = 1LL * a.B * a.k;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
@@ -2231,6 +2258,7 @@ __global__ void __launch_bounds__(256) token_topk_push_kernel(CltTopkTpArgs a) {
 
 // One CTA per owned token; dynamic shared memory world * k keys.
 __global__ void __launch_bounds__(256) token_topk_cut_kernel(CltTopkTpArgs a) {
+  if (chain_wait()) return;
   extern __shared__ unsigned long long tk_keys[];
   const int lt = blockIdx.x;
   const int t = a.rank * a.rows_per_rank + lt;
@@ -2255,6 +2283,7 @@ __global__ void __launch_bounds__(256) token_topk_cut_kernel(CltTopkTpArgs a) {
 
 // One warp per token: candidates at or above the cut are appended to the entry list.
 __global__ void __launch_bounds__(256) token_topk_filter_kernel(CltTopkTpArgs a) {
+  if (chain_wait()) return;
   const int lane = threadIdx.x & 31;
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= a.B) return;
@@ -2286,16 +2315,16 @@ extern "C" int clt_token_topk_tp(const CltTopkTpArgs* a, int phase, cudaStream_t
   if (phase == 0) {
     const long long n = 1LL * a->B * a->k;
     const int grid = int((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
-    token_topk_push_kernel<<<grid, 256, 0, st>>>(*a);
+    launch_chained(token_topk_push_kernel, grid, 256, 0, st, *a);
   } else if (phase == 1) {
     static size_t attr_smem = 0;
     if (smem > 48 * 1024 && smem > attr_smem) {
       if (cudaFuncSetAttribute(token_topk_cut_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
       attr_smem = smem;
     }
-    token_topk_cut_kernel<<<a->rows_per_rank, 256, smem, st>>>(*a);
+    launch_chained(token_topk_cut_kernel, a->rows_per_rank, 256, smem, st, *a);
   } else {
-    token_topk_filter_kernel<<<(a->B + 7) / 8, 256, 0, st>>>(*a);
+    launch_chained(token_topk_filter_kernel, (a->B + 7) / 8, 256, 0, st, *a);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -2320,15 +2349,15 @@ static void launch_feature_sort(const int* off, int num_cols, long long ent_cap,
   if (num_cols <= 0) return;
   int per_cta = 256;
   while (per_cta > 1 && double(ent_cap) / num_cols * per_cta > kFeatSortCap / 2) per_cta /= 2;
-  csr_sort_feature_segments_kernel<<<(num_cols + per_cta - 1) / per_cta, 256, 0, st>>>(off, num_cols, per_cta, key, val);
+  launch_chained(csr_sort_feature_segments_kernel, (num_cols + per_cta - 1) / per_cta, 256, 0, st, off, num_cols, per_cta, key, val);
 }
 
 extern "C" int clt_build_csr(const CltCsrArgs* a, cudaStream_t st) {
   const int blocks = 592;
-  csr_count_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cnt, a->feat_cnt, a->fired,
+  launch_chained(csr_count_kernel, blocks, 256, 0, st, a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cnt, a->feat_cnt, a->fired,
                                            a->num_tokens, a->num_cols);
   launch_exclusive_scans({a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens}, {a->feat_cnt, a->feat_off, a->feat_cursor, a->num_cols}, st);
-  csr_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->feat_cursor,
+  launch_chained(csr_scatter_kernel, blocks, 256, 0, st, a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->feat_cursor,
                                              a->tcsr_col, a->tcsr_val, a->fcsr_tok, a->fcsr_val, a->col_pitch, a->num_tokens, a->num_cols, a->feat_off, a->layer_cnt);
   if (a->sort_segments & 1) launch_token_sort(a->tok_off, a->tcsr_col, a->tcsr_val, a->num_tokens, a->num_cols, a->col_pitch, st);
   if (a->sort_segments & 2) launch_feature_sort(a->feat_off, a->num_cols, a->ent_cap, a->fcsr_tok, a->fcsr_val, st);
@@ -2340,19 +2369,19 @@ extern "C" int clt_build_token_csr(const CltCsrArgs* a, cudaStream_t st) {
   if (a->num_tokens <= 0) return 0;
   if ((a->num_cols + a->col_pitch - 1) / a->col_pitch > 32) return -1;
   const int blocks = int((a->ent_cap + 255) / 256 < 592 ? (a->ent_cap + 255) / 256 : 592);
-  csr_token_count_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_cap, a->ctl, a->tok_cnt, a->layer_cnt, a->col_pitch, a->num_tokens, a->num_cols);
+  launch_chained(csr_token_count_kernel, blocks, 256, 0, st, a->ent_tok, a->ent_col, a->ent_cap, a->ctl, a->tok_cnt, a->layer_cnt, a->col_pitch, a->num_tokens, a->num_cols);
   const ScanJob job{a->tok_cnt, a->tok_off, a->tok_cursor, a->num_tokens}, none{nullptr, nullptr, nullptr, 0};
   const int tiles = (a->num_tokens + 4095) / 4096;
-  if (tiles <= 512 && (reinterpret_cast<uintptr_t>(a->tok_cnt) & 15) == 0) exclusive_scan_tiles_kernel<<<tiles, 1024, 0, st>>>(job, none, tiles);
-  else exclusive_scan_kernel<<<1, 1024, 0, st>>>(job.in, job.out, job.cursor, job.n);
-  csr_token_scatter_kernel<<<blocks, 256, 0, st>>>(a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->tcsr_col, a->tcsr_val,
+  if (tiles <= 512 && (reinterpret_cast<uintptr_t>(a->tok_cnt) & 15) == 0) launch_chained(exclusive_scan_tiles_kernel, tiles, 1024, 0, st, job, none, tiles);
+  else launch_chained(exclusive_scan_kernel, 1, 1024, 0, st, job.in, job.out, job.cursor, job.n);
+  launch_chained(csr_token_scatter_kernel, blocks, 256, 0, st, a->ent_tok, a->ent_col, a->ent_val, a->ent_cap, a->ctl, a->tok_cursor, a->tcsr_col, a->tcsr_val,
                                                    a->col_pitch, a->num_tokens, a->num_cols);
   launch_token_sort(a->tok_off, a->tcsr_col, a->tcsr_val, a->num_tokens, a->num_cols, a->col_pitch, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 extern "C" int clt_dead_counter_update(long long* counter, unsigned char* fired, int n, cudaStream_t st) {
-  dead_counter_kernel<<<(n + 255) / 256, 256, 0, st>>>(counter, fired, n);
+  launch_chained(dead_counter_kernel, (n + 255) / 256, 256, 0, st, counter, fired, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -2415,10 +2444,10 @@ extern "C" int clt_build_csr_static(const int* ent_tok, const int* ent_col, cons
   if (cudaMemsetAsync(tok_cnt, 0, sizeof(int) * size_t(num_tokens), stream) != cudaSuccess) return -5;
   if (cudaMemsetAsync(feat_cnt, 0, sizeof(int) * size_t(num_cols), stream) != cudaSuccess) return -5;
   const int blocks = 592;
-  csr_count_kernel<<<blocks, 256, 0, stream>>>(ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cnt, feat_cnt, nullptr, num_tokens, num_cols);
-  exclusive_scan_kernel<<<1, 1024, 0, stream>>>(tok_cnt, tok_off, tok_cursor, num_tokens);
-  exclusive_scan_kernel<<<1, 1024, 0, stream>>>(feat_cnt, feat_off, feat_cursor, num_cols);
-  csr_scatter_kernel<<<blocks, 256, 0, stream>>>(ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cursor, feat_cursor, tcsr_col, tcsr_val,
+  launch_chained(csr_count_kernel, blocks, 256, 0, stream, ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cnt, feat_cnt, nullptr, num_tokens, num_cols);
+  launch_chained(exclusive_scan_kernel, 1, 1024, 0, stream, tok_cnt, tok_off, tok_cursor, num_tokens);
+  launch_chained(exclusive_scan_kernel, 1, 1024, 0, stream, feat_cnt, feat_off, feat_cursor, num_cols);
+  launch_chained(csr_scatter_kernel, blocks, 256, 0, stream, ent_tok, ent_col, ent_val, ent_cap, ctl, tok_cursor, feat_cursor, tcsr_col, tcsr_val,
                                                  fcsr_tok, fcsr_val, col_pitch, num_tokens, num_cols, feat_off, nullptr);
   if (sort_segments & 1) launch_token_sort(tok_off, tcsr_col, tcsr_val, num_tokens, num_cols, col_pitch, stream);
   if (sort_segments & 2) launch_feature_sort(feat_off, num_cols, ent_cap, fcsr_tok, fcsr_val, stream);

@@ -68,6 +68,7 @@ struct StepControlParams {
 };
 
 __global__ void __launch_bounds__(64) step_control_kernel(const StepControlParams p) {
+  if (chain_wait()) return;
   __shared__ double vals[kCtlMaxLayers + kMaxScalars + 2];
   __shared__ int timeout;
   const int tid = threadIdx.x;
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(256) decoder_bias_adam_kernel(WT* __restrict__
                                                                   const float* __restrict__ sel, const float* __restrict__ gs_sum,
                                                                   const float* __restrict__ extra, int n_bias, int L, int d,
                                                                   AdamHyperS h, float* __restrict__ ctl, float norm_weight) {
+  if (chain_wait()) return;
   const StepScales sc = read_step_ctl(ctl);
   if (sc.skip) return;
   const long long n = 1LL * n_bias * d;
@@ -190,6 +192,7 @@ template <typename WT>
 __global__ void __launch_bounds__(256) step_finish_kernel(long long* __restrict__ counter, unsigned char* __restrict__ fired, int ncols,
                                                             const WT* __restrict__ bias, const float* __restrict__ sel,
                                                             float* __restrict__ bias_sum, int n_bias, int L, int d) {
+  if (chain_wait()) return;
   const long long stride = 1LL * gridDim.x * blockDim.x;
   const long long tid = blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   if (counter != nullptr)
@@ -259,6 +262,7 @@ struct ThetaAdamParams {
 
 template <typename WT>
 __global__ void __launch_bounds__(256) theta_adam_kernel(const ThetaAdamParams p) {
+  if (chain_wait()) return;
   const StepScales sc = read_step_ctl(p.ctl);
   if (sc.skip) return;
   const long long n = 1LL * p.L * p.pitch;
@@ -317,6 +321,7 @@ __global__ void __launch_bounds__(256) theta_accumulate_kernel(const int* __rest
                                                                  const float* __restrict__ mean, const float* __restrict__ rstd, int L, int pitch,
                                                                  int width, float eps, float* __restrict__ sum_min, float* __restrict__ cnt_min,
                                                                  float* __restrict__ mean_acc, float* __restrict__ std_acc, float* __restrict__ batches) {
+  if (chain_wait()) return;
   const long long n = 1LL * L * pitch;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
     const int l = int(i / pitch), f = int(i - 1LL * l * pitch);
@@ -366,6 +371,7 @@ __device__ __forceinline__ void load8_in<__half>(const __half* p, float (&o)[8])
 template <typename IT>
 __global__ void __launch_bounds__(256) normalize_cast_kernel(const IT* __restrict__ in, t16* __restrict__ out, const float* __restrict__ mean,
                                                                const float* __restrict__ inv_std, long long rows, int rows_per_stat, int d, float mul) {
+  if (chain_wait()) return;
   const int vec_per_row = d / 8;
   const long long nvec = rows * vec_per_row;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < nvec; i += 1LL * gridDim.x * blockDim.x) {
@@ -395,6 +401,7 @@ constexpr int kMaxScales = 1024;
 __global__ void __launch_bounds__(256) scale_histogram_kernel(const t16* __restrict__ x, const float* __restrict__ theta,
                                                                 const float* __restrict__ scales, int n_scales,
                                                                 unsigned long long* __restrict__ hist, int B, int F, long long ld) {
+  if (chain_wait()) return;
   __shared__ float sc[kMaxScales];
   __shared__ unsigned int sh[kMaxScales + 1];
   for (int i = threadIdx.x; i < n_scales; i += blockDim.x) sc[i] = scales[i];
@@ -421,6 +428,7 @@ __global__ void __launch_bounds__(256) scale_histogram_kernel(const t16* __restr
 // theta = exp(log_theta) (set-up, after a checkpoint load)
 template <typename WT>
 __global__ void __launch_bounds__(256) theta_exp_kernel(const WT* __restrict__ log_theta, float* __restrict__ theta, long long n) {
+  if (chain_wait()) return;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x)
     theta[i] = __expf(load_w<WT>(log_theta + i));
 }
@@ -470,7 +478,7 @@ extern "C" int clt_step_control(const CltStepControlArgs* a, const CltExchangeAr
     p.ex.flags[i] = exa ? static_cast<uint32_t*>(exa->flags[i]) : nullptr;
   }
   if (exa && 2 * (a->L + a->n_scalars + 1) > exa->slot_elems) return -1;
-  step_control_kernel<<<1, 64, 0, st>>>(p);
+  launch_chained(step_control_kernel, 1, 64, 0, st, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 #endif
@@ -481,8 +489,8 @@ extern "C" int CLT_FN(clt_decoder_bias_adam)(void* bias, float* m, float* v, con
   const long long n = 1LL * n_bias * d;
   if (n <= 0) return 0;
   const int grid = int((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-  if (weights_16) decoder_bias_adam_kernel<t16><<<grid, 256, 0, st>>>(static_cast<t16*>(bias), m, v, sel, gs_sum, extra, n_bias, L, d, to_hyper_s(*h), ctl, norm_weight);
-  else decoder_bias_adam_kernel<float><<<grid, 256, 0, st>>>(static_cast<float*>(bias), m, v, sel, gs_sum, extra, n_bias, L, d, to_hyper_s(*h), ctl, norm_weight);
+  if (weights_16) launch_chained(decoder_bias_adam_kernel<t16>, grid, 256, 0, st, static_cast<t16*>(bias), m, v, sel, gs_sum, extra, n_bias, L, d, to_hyper_s(*h), ctl, norm_weight);
+  else launch_chained(decoder_bias_adam_kernel<float>, grid, 256, 0, st, static_cast<float*>(bias), m, v, sel, gs_sum, extra, n_bias, L, d, to_hyper_s(*h), ctl, norm_weight);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -493,8 +501,8 @@ extern "C" int CLT_FN(clt_step_finish)(long long* counter, unsigned char* fired,
   if (work <= 0 && bias_blocks <= 0) return 0;
   int grid = int((work + 255) / 256 < 1184 ? (work + 255) / 256 : 1184);
   if (grid < bias_blocks) grid = bias_blocks;
-  if (weights_16) step_finish_kernel<t16><<<grid, 256, 0, st>>>(counter, fired, ncols, static_cast<const t16*>(bias), sel, bias_sum, n_bias, L, d);
-  else step_finish_kernel<float><<<grid, 256, 0, st>>>(counter, fired, ncols, static_cast<const float*>(bias), sel, bias_sum, n_bias, L, d);
+  if (weights_16) launch_chained(step_finish_kernel<t16>, grid, 256, 0, st, counter, fired, ncols, static_cast<const t16*>(bias), sel, bias_sum, n_bias, L, d);
+  else launch_chained(step_finish_kernel<float>, grid, 256, 0, st, counter, fired, ncols, static_cast<const float*>(bias), sel, bias_sum, n_bias, L, d);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -518,16 +526,16 @@ extern "C" int CLT_FN(clt_theta_adam)(const CltThetaAdamArgs* a, cudaStream_t st
   const long long n = 1LL * a->L * a->pitch;
   if (n <= 0) return 0;
   const int grid = int((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-  if (a->weights_16) theta_adam_kernel<t16><<<grid, 256, 0, st>>>(p);
-  else theta_adam_kernel<float><<<grid, 256, 0, st>>>(p);
+  if (a->weights_16) launch_chained(theta_adam_kernel<t16>, grid, 256, 0, st, p);
+  else launch_chained(theta_adam_kernel<float>, grid, 256, 0, st, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 extern "C" int CLT_FN(clt_theta_exp)(const void* log_theta, float* theta, long long n, int weights_16, cudaStream_t st) {
   if (n <= 0) return 0;
   const int grid = int((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-  if (weights_16) theta_exp_kernel<t16><<<grid, 256, 0, st>>>(static_cast<const t16*>(log_theta), theta, n);
-  else theta_exp_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(log_theta), theta, n);
+  if (weights_16) launch_chained(theta_exp_kernel<t16>, grid, 256, 0, st, static_cast<const t16*>(log_theta), theta, n);
+  else launch_chained(theta_exp_kernel<float>, grid, 256, 0, st, static_cast<const float*>(log_theta), theta, n);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -538,7 +546,7 @@ extern "C" int clt_theta_accumulate(const int* feat_off, const float* fcsr_val, 
   const long long n = 1LL * L * pitch;
   if (n <= 0) return 0;
   const int grid = int((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-  theta_accumulate_kernel<<<grid, 256, 0, st>>>(feat_off, fcsr_val, mean, rstd, L, pitch, width, eps, sum_min, cnt_min, mean_acc, std_acc, batches);
+  launch_chained(theta_accumulate_kernel, grid, 256, 0, st, feat_off, fcsr_val, mean, rstd, L, pitch, width, eps, sum_min, cnt_min, mean_acc, std_acc, batches);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 #endif
@@ -550,9 +558,9 @@ extern "C" int CLT_FN(clt_normalize_cast)(const void* in, int in_type, void* out
   const long long nvec = rows * (d / 8);
   const int grid = int((nvec + 255) / 256 < 148 * 16 ? (nvec + 255) / 256 : 148 * 16);
   t16* o = static_cast<t16*>(out);
-  if (in_type == 0) normalize_cast_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(in), o, mean, inv_std, rows, rows_per_stat, d, mul);
-  else if (in_type == 1) normalize_cast_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(in), o, mean, inv_std, rows, rows_per_stat, d, mul);
-  else if (in_type == 2) normalize_cast_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(in), o, mean, inv_std, rows, rows_per_stat, d, mul);
+  if (in_type == 0) launch_chained(normalize_cast_kernel<float>, grid, 256, 0, st, static_cast<const float*>(in), o, mean, inv_std, rows, rows_per_stat, d, mul);
+  else if (in_type == 1) launch_chained(normalize_cast_kernel<__nv_bfloat16>, grid, 256, 0, st, static_cast<const __nv_bfloat16*>(in), o, mean, inv_std, rows, rows_per_stat, d, mul);
+  else if (in_type == 2) launch_chained(normalize_cast_kernel<__half>, grid, 256, 0, st, static_cast<const __half*>(in), o, mean, inv_std, rows, rows_per_stat, d, mul);
   else return -1;
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -563,6 +571,6 @@ extern "C" int CLT_FN(clt_scale_histogram)(const void* x, const float* theta, co
   if (n_scales < 1 || n_scales > kMaxScales || B <= 0 || F <= 0) return -1;
   const long long n = 1LL * B * F;
   const int grid = int((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
-  scale_histogram_kernel<<<grid, 256, 0, st>>>(static_cast<const t16*>(x), theta, scales, n_scales, hist, B, F, ld);
+  launch_chained(scale_histogram_kernel, grid, 256, 0, st, static_cast<const t16*>(x), theta, scales, n_scales, hist, B, F, ld);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
