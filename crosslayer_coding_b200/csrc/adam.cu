@@ -11,6 +11,8 @@
 //
 // Row layout: decoder tensor s is [F, R_s, d] (feature-major), encoder is [L, F, d]; bf16 weights with
 // fp32 moments (or fp32 weights).  d must be a multiple of 8.
+#include <climits>
+
 #include "common.cuh"
 
 #include <type_traits>
@@ -230,10 +232,7 @@ struct RowRegs {
 // elements per lane, walking the feature's R = L - s target rows with the next row's (w, m, v) already in
 // flight.  The first four entries of the feature stay in registers: their activation, token and the
 // partial dot products for dL/da, which are reduced once per item instead of once per row.
-// NORM_ONLY: the gradient-norm pre-pass of gradient clipping.  Nothing is updated: features without entries (and
-// without an extra row) are skipped, the row gradients of the others are formed as in the update, their squares
-// are summed into p.norm_sq_out and dL/da is written to p.grad_a.
-template <typename WT, bool SR, bool NORM_ONLY>
+template <typename WT, bool SR>
 __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const DecAdamParams p) {
   const int lane = threadIdx.x & 31;
   const int warp_global = int((blockIdx.x * 1LL * blockDim.x + threadIdx.x) >> 5);
@@ -242,7 +241,6 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
   const StepScales sc = read_step_ctl(p.ctl);
   if (sc.skip) return;
   const float gsc = hr.gscale * (p.use_inv_scale ? sc.inv_scale : 1.f);
-  float nsq = 0.f;
   const int d = p.d, B = p.B, Fp = p.F_pitch;
   const int nseg = (d + 255) / 256;
   const int per_tensor = Fp * nseg;
@@ -264,9 +262,8 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
     const int b = __ldg(p.feat_off + col), e = __ldg(p.feat_off + col + 1);
     const int ne = e - b;
     const float* xrow = extra_row_ptr(p, col);
-    if (NORM_ONLY && ne == 0 && xrow == nullptr) continue;
     RowRegs<WT> cur, nxt;
-    if (act) { if (NORM_ONLY) cur.w.load(wbase); else cur.load(wbase, mbase, vbase); }
+    if (act) cur.load(wbase, mbase, vbase);
     int tok4[4];
     float a4[4], dacc[4];
 #pragma unroll
@@ -280,7 +277,7 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
     const unsigned int idx_base = (unsigned int)((p.row_start[ti] + row0) * d + e0);
     for (int r = 0; r < R; ++r) {
       const long long roff = 1LL * r * d;
-      if (act && r + 1 < R) { if (NORM_ONLY) nxt.w.load(wbase + roff + d); else nxt.load(wbase + roff + d, mbase + roff + d, vbase + roff + d); }
+      if (act && r + 1 < R) nxt.load(wbase + roff + d, mbase + roff + d, vbase + roff + d);
       float w[8], g[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) { g[i] = 0.f; w[i] = 0.f; }
@@ -321,29 +318,20 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
         float dg0[8];
         const bool extra = r == 0 && xrow != nullptr;
         if (extra) load8f(xrow + e0, dg0);
-        if (NORM_ONLY) {
+        float m[8], v[8];
+        f4x2_to8(cur.m0, cur.m1, m);
+        f4x2_to8(cur.v0, cur.v1, v);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            float gk = fmaf(pc, w[k], g[k] * gsc);
-            if (extra) gk += dg0[k];
-            nsq = fmaf(gk, gk, nsq);
-          }
-        } else {
-          float m[8], v[8];
-          f4x2_to8(cur.m0, cur.m1, m);
-          f4x2_to8(cur.v0, cur.v1, v);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            float gk = fmaf(pc, w[k], g[k] * gsc);
-            if (extra) gk += dg0[k];
-            adam1(w[k], m[k], v[k], gk * sc.clip, hr);
-            norm2 = fmaf(w[k], w[k], norm2);
-          }
-          stream_store8f(mbase + roff, m);
-          stream_store8f(vbase + roff, v);
-          if (sizeof(WT) == 2) __stcs(reinterpret_cast<uint4*>(wbase + roff), pack8_bf16<SR>(w, p.h.sr_seed, idx_base + (unsigned int)roff));
-          else stream_store8f(reinterpret_cast<float*>(wbase + roff), w);
+        for (int k = 0; k < 8; ++k) {
+          float gk = fmaf(pc, w[k], g[k] * gsc);
+          if (extra) gk += dg0[k];
+          adam1(w[k], m[k], v[k], gk * sc.clip, hr);
+          norm2 = fmaf(w[k], w[k], norm2);
         }
+        stream_store8f(mbase + roff, m);
+        stream_store8f(vbase + roff, v);
+        if (sizeof(WT) == 2) __stcs(reinterpret_cast<uint4*>(wbase + roff), pack8_bf16<SR>(w, p.h.sr_seed, idx_base + (unsigned int)roff));
+        else stream_store8f(reinterpret_cast<float*>(wbase + roff), w);
       }
       cur = nxt;
     }
@@ -356,12 +344,181 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
         }
       }
     }
-    if (!NORM_ONLY && p.norm2_out != nullptr) {
+    if (p.norm2_out != nullptr) {
       norm2 = warp_sum(norm2);
       if (lane == 0) atomicAdd(&p.norm2_out[col], norm2);
     }
   }
-  if (NORM_ONLY) block_add(nsq, p.norm_sq_out);
+}
+
+// ---------------------------------------------------------------- gradient norms (clipping)
+// The pre-pass of gradient clipping: squared norms of all row gradients into p.norm_sq_out and, with DOTS (decoders), dL/da into p.grad_a.  Nothing
+// is updated, so features without entries (and without an extra row) are skipped and neither moments nor, without DOTS, weights are read.
+// A gather of every entry's seed row for every target, which L2 could deliver three times as fast as the one-segment form read it: instructions bound
+// that one (a warp per 256 elements of a feature's rows: divisions, list and reductions for each).  Here a warp takes up to 1024 elements of the rows
+// (NV vectors of eight per lane), kEntries entries at a time, with the list of the next feature and the offsets of the one after it on the way.
+// us before and now, decoder + encoder: 12 x 768, 24576 features, 4096 tokens, k = 200 3243 + 321 / 1750 + 195; 3072 features, k = 25 498 + 48 / 281 + 32;
+// 5 x 520, 2056 features, 776 tokens 62 + 15 / 41 + 11; 12 x 352 tied 114 + 50 / 74 + 37; 6 x 136 145 + 37 / 120 + 35; 4 x 2048 102 + 36 / 82 + 24.
+template <typename WT, bool DOTS, int NV>
+__global__ void __launch_bounds__(256, 2) rows_norm_kernel(const DecAdamParams p) {
+  constexpr int kEntries = NV <= 2 ? 4 : 2;
+  const int lane = threadIdx.x & 31;
+  const int warp_global = int((blockIdx.x * 1LL * blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = int((gridDim.x * 1LL * blockDim.x) >> 5);
+  const StepScales sc = read_step_ctl(p.ctl);
+  if (sc.skip) return;
+  const float gsc = p.h.grad_scale * (p.use_inv_scale ? sc.inv_scale : 1.f);
+  float nsq = 0.f;
+  const int d = p.d, Fp = p.F_pitch;
+  const int nseg = (d + 256 * NV - 1) / (256 * NV), seg_width = (d / 8 + nseg - 1) / nseg * 8;  // even segments
+  const int total_cols = Fp * p.ntensors;
+  const long long total_items = 1LL * total_cols * nseg;
+  struct List {
+    int b, e;
+    int tok[4];
+    float a[4];
+  };
+  const auto load_range = [&](long long item, List& m) {
+    m.b = m.e = 0;
+    if (item >= total_items) return;
+    const int col = nseg == 1 ? int(item) : int(item / nseg);
+    m.b = __ldg(p.feat_off + col);
+    m.e = __ldg(p.feat_off + col + 1);
+  };
+  const auto load_entries = [&](List& m) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool in = m.b + j < m.e;
+      m.tok[j] = in ? __ldg(p.fcsr_tok + m.b + j) : 0;
+      m.a[j] = in ? __ldg(p.fcsr_val + m.b + j) : 0.f;
+    }
+  };
+  List cur, nxt;
+  load_range(warp_global, cur);
+  load_entries(cur);
+  load_range(1LL * warp_global + nwarps, nxt);
+  for (long long item = warp_global; item < total_items; item += nwarps) {
+    List after;
+    load_range(item + 2LL * nwarps, after);
+    load_entries(nxt);
+    const int col = nseg == 1 ? int(item) : int(item / nseg);
+    const int seg0 = nseg == 1 ? 0 : int(item - 1LL * col * nseg) * seg_width, end = min(d, seg0 + seg_width);
+    const int b = cur.b, ne = cur.e - b;
+    const float* xrow = extra_row_ptr(p, col);
+    if (ne > 0 || xrow != nullptr) {
+      const int ti = col / Fp, f = col - ti * Fp;
+      const int R = p.rows[ti];
+      const int e0 = seg0 + lane * 8;
+      const WT* wrow = static_cast<const WT*>(p.w[ti]) + 1LL * f * R * d + e0;
+      const t16* gs_t = p.gs + 1LL * ti * p.B * d + e0;
+      const float pc = DOTS && p.pen_coef ? p.pen_coef[col] : 0.f;
+      float dacc[4] = {0.f, 0.f, 0.f, 0.f};
+      float dx = 0.f;  // dL/da of entry 4 + lane
+#pragma unroll 1
+      for (int r = 0; r < R; ++r, wrow += d, gs_t += 1LL * p.B * d) {
+        WVec<WT> wv[NV];
+        float g[NV][8];
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          if (DOTS && e0 + 256 * n < end) wv[n].load(wrow + 256 * n);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) g[n][k] = 0.f;
+        }
+#pragma unroll
+        for (int j0 = 0; j0 < 4; j0 += kEntries) {  // the first four entries, whose list is in registers
+          if (j0 >= ne) break;
+          uint4 v[kEntries][NV];
+#pragma unroll
+          for (int j = 0; j < kEntries; ++j)
+            if (j0 + j < ne) {
+#pragma unroll
+              for (int n = 0; n < NV; ++n)
+                if (e0 + 256 * n < end) v[j][n] = __ldg(reinterpret_cast<const uint4*>(gs_t + 1LL * cur.tok[j0 + j] * d + 256 * n));
+            }
+#pragma unroll
+          for (int j = 0; j < kEntries; ++j)
+            if (j0 + j < ne) {
+#pragma unroll
+              for (int n = 0; n < NV; ++n)
+                if (e0 + 256 * n < end) {
+                  float gv[8], w[8];
+                  unpack8(v[j][n], gv);
+                  if (DOTS) wv[n].get(w);
+#pragma unroll
+                  for (int k = 0; k < 8; ++k) {
+                    g[n][k] = fmaf(cur.a[j0 + j], gv[k], g[n][k]);
+                    if (DOTS) dacc[j0 + j] = fmaf(gv[k], w[k], dacc[j0 + j]);
+                  }
+                }
+            }
+        }
+#pragma unroll 1
+        for (int i = 4; i < ne; ++i) {
+          const float a = __ldg(p.fcsr_val + b + i);
+          const t16* src = gs_t + 1LL * __ldg(p.fcsr_tok + b + i) * d;
+          uint4 v[NV];
+          float dot = 0.f;
+#pragma unroll
+          for (int n = 0; n < NV; ++n)
+            if (e0 + 256 * n < end) v[n] = __ldg(reinterpret_cast<const uint4*>(src + 256 * n));
+#pragma unroll
+          for (int n = 0; n < NV; ++n)
+            if (e0 + 256 * n < end) {
+              float gv[8], w[8];
+              unpack8(v[n], gv);
+              if (DOTS) wv[n].get(w);
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                g[n][k] = fmaf(a, gv[k], g[n][k]);
+                if (DOTS) dot = fmaf(gv[k], w[k], dot);
+              }
+            }
+          if (DOTS && p.grad_a != nullptr) {
+            dot = warp_sum(dot);
+            if (i < 36) dx += lane == i - 4 ? dot : 0.f;
+            else if (lane == 0 && dot != 0.f) atomicAdd(&p.grad_a[b + i], dot * gsc);
+          }
+        }
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          if (e0 + 256 * n < end) {
+            float w[8], dg0[8];
+            if (DOTS && pc != 0.f) wv[n].get(w);
+            const bool extra = r == 0 && xrow != nullptr;
+            if (extra) load8f(xrow + e0 + 256 * n, dg0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              float gk = g[n][k] * gsc;
+              if (DOTS && pc != 0.f) gk = fmaf(pc, w[k], gk);
+              if (extra) gk += dg0[k];
+              nsq = fmaf(gk, gk, nsq);
+            }
+          }
+        }
+      }
+      if (DOTS && p.grad_a != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (j < ne) {
+            const float sdot = warp_sum(dacc[j]);
+            if (lane == 0 && sdot != 0.f) atomicAdd(&p.grad_a[b + j], sdot * gsc);
+          }
+        }
+        if (4 + lane < ne && dx != 0.f) atomicAdd(&p.grad_a[b + 4 + lane], dx * gsc);
+      }
+    }
+    cur = nxt;
+    nxt = after;
+  }
+  block_add(nsq, p.norm_sq_out);
+}
+template <typename WT, bool DOTS>
+static void launch_rows_norm(const DecAdamParams& p, int num_sms, cudaStream_t st) {
+  const int vecs = (p.d + 255) / 256;  // a warp per row up to 1024 elements, even segments of longer ones
+  if (vecs <= 1) launch_alone(rows_norm_kernel<WT, DOTS, 1>, 2 * num_sms, 256, 0, st, p);
+  else if (vecs == 2) launch_alone(rows_norm_kernel<WT, DOTS, 2>, 2 * num_sms, 256, 0, st, p);
+  else if (vecs == 3 || vecs == 5 || vecs == 6) launch_alone(rows_norm_kernel<WT, DOTS, 3>, 2 * num_sms, 256, 0, st, p);
+  else launch_alone(rows_norm_kernel<WT, DOTS, 4>, 2 * num_sms, 256, 0, st, p);
 }
 
 // ---------------------------------------------------------------- untied decoders, bulk-copy pipeline
@@ -1684,8 +1841,8 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   if (a->norm_only) {
     if (a->ctl == nullptr) return -1;
     if (a->tying == 0) {
-      if (a->weights_bf16) launch_alone(decoder_rows_adam_untied_kernel<t16, false, true>, grid, 256, 0, st, p);
-      else launch_alone(decoder_rows_adam_untied_kernel<float, false, true>, grid, 256, 0, st, p);
+      if (a->weights_bf16) launch_rows_norm<t16, true>(p, num_sms, st);
+      else launch_rows_norm<float, true>(p, num_sms, st);
     } else if (a->weights_bf16) {
       launch_alone(decoder_rows_adam_kernel<t16, true>, grid, 256, 0, st, p);
     } else {
@@ -1706,10 +1863,10 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   } else if (a->tying == 0) {
     const bool sr = a->h.sr_seed != 0;
     if (a->weights_bf16) {
-      if (sr) launch_alone(decoder_rows_adam_untied_kernel<t16, true, false>, grid, 256, 0, st, p);
-      else launch_alone(decoder_rows_adam_untied_kernel<t16, false, false>, grid, 256, 0, st, p);
+      if (sr) launch_alone(decoder_rows_adam_untied_kernel<t16, true>, grid, 256, 0, st, p);
+      else launch_alone(decoder_rows_adam_untied_kernel<t16, false>, grid, 256, 0, st, p);
     } else {
-      launch_alone(decoder_rows_adam_untied_kernel<float, false, false>, grid, 256, 0, st, p);
+      launch_alone(decoder_rows_adam_untied_kernel<float, false>, grid, 256, 0, st, p);
     }
   } else if (a->weights_bf16) {
     launch_alone(decoder_rows_adam_kernel<t16, false>, grid, 256, 0, st, p);
@@ -1742,42 +1899,47 @@ extern "C" int CLT_FN(clt_encoder_rows_adam)(const CltEncAdamArgs* a, int num_sm
   p.dense_grad = a->dense_grad; p.dense_bias_grad = a->dense_bias_grad; p.h = to_hyper(a->h);
   p.extra_idx = a->extra_idx; p.extra_rows = a->extra_rows; p.extra_bias = a->extra_bias; p.ctl = a->ctl;
   p.norm_sq_out = a->ctl != nullptr ? a->ctl + SC_GRAD_NORM_SQ : nullptr; p.norm_only = a->norm_only;
-  const int grid = num_sms * 8;
+  const int grid = num_sms * 8, bgrid = int((1LL * a->L * a->F_pitch + 255) / 256);
+  // the encoder as the one-row-per-feature case of the decoder's kernels: layer l is "tensor" l with R = 1, the layer inputs play the gradient
+  // seed and delta the activation
+  DecAdamParams q;
+  const size_t wsz = a->weights_bf16 ? 2 : 4;
+  const long long per_layer = 1LL * a->F_pitch * a->d;
+  for (int i = 0; i < kMaxLayersA; ++i) {
+    const int l = i < a->L ? i : 0;
+    q.w[i] = static_cast<char*>(a->w) + size_t(l) * per_layer * wsz;
+    const size_t msz = a->moments_bf16 ? 2 : 4;
+    q.m[i] = reinterpret_cast<float*>(reinterpret_cast<char*>(a->m) + size_t(l) * per_layer * msz);
+    q.v[i] = reinterpret_cast<float*>(reinterpret_cast<char*>(a->v) + size_t(l) * per_layer * msz);
+    q.rows[i] = 1;
+    q.row_start[i] = 1LL * (i < a->L ? i : a->L) * a->F_pitch;
+  }
+  q.row_start[kMaxLayersA] = 1LL * a->L * a->F_pitch;
+  q.ntensors = a->L; q.L = a->L; q.B = a->B; q.d = a->d; q.F_pitch = a->F_pitch; q.tying = 0;
+  q.feat_off = a->feat_off; q.fcsr_tok = a->fcsr_tok; q.fcsr_val = a->delta; q.gs = p.x;
+  q.grad_a = nullptr; q.pen_coef = nullptr; q.norm2_out = nullptr; q.feat_offset = nullptr; q.feat_scale = nullptr;
+  q.d_feat_offset = nullptr; q.d_feat_scale = nullptr;
+  q.dgrad_row0 = a->dense_grad; q.h = p.h;
+  q.moments_bf16 = a->moments_bf16;
+  q.extra_idx = a->dense_grad == nullptr ? a->extra_idx : nullptr; q.extra_rows = a->extra_rows;
+  q.ctl = a->ctl; q.use_inv_scale = 0; q.norm_sq_out = p.norm_sq_out;
   if (a->norm_only) {
     if (a->ctl == nullptr) return -1;
-    if (a->weights_bf16) launch_alone(encoder_rows_adam_kernel<t16, true>, grid, 256, 0, st, p);
-    else launch_alone(encoder_rows_adam_kernel<float, true>, grid, 256, 0, st, p);
+    if (a->L <= kMaxLayersA && (a->dense_grad == nullptr || a->extra_idx == nullptr) && 1LL * a->L * a->F_pitch < INT_MAX) {
+      launch_rows_norm<t16, false>(q, num_sms, st);  // the weights' type does not matter: they are not read
+      if (p.bias != nullptr) launch_chained(encoder_bias_adam_kernel<t16>, bgrid, 256, 0, st, p);
+    } else if (a->weights_bf16) {  // two kinds of extra rows
+      launch_alone(encoder_rows_adam_kernel<t16, true>, grid, 256, 0, st, p);
+    } else {
+      launch_alone(encoder_rows_adam_kernel<float, true>, grid, 256, 0, st, p);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
   if (a->status != nullptr && a->L <= kMaxLayersA && bulk_rows_adam_fits(a->d, a->weights_bf16)) {
-    // the encoder is the one-row-per-feature case of the row pipeline: layer l is "tensor" l with R = 1, the
-    // layer inputs play the gradient seed and delta the activation
-    DecAdamParams q;
-    const size_t wsz = a->weights_bf16 ? 2 : 4;
-    const long long per_layer = 1LL * a->F_pitch * a->d;
-    for (int i = 0; i < kMaxLayersA; ++i) {
-      const int l = i < a->L ? i : 0;
-      q.w[i] = static_cast<char*>(a->w) + size_t(l) * per_layer * wsz;
-      const size_t msz = a->moments_bf16 ? 2 : 4;
-      q.m[i] = reinterpret_cast<float*>(reinterpret_cast<char*>(a->m) + size_t(l) * per_layer * msz);
-      q.v[i] = reinterpret_cast<float*>(reinterpret_cast<char*>(a->v) + size_t(l) * per_layer * msz);
-      q.rows[i] = 1;
-      q.row_start[i] = 1LL * (i < a->L ? i : a->L) * a->F_pitch;
-    }
-    q.row_start[kMaxLayersA] = 1LL * a->L * a->F_pitch;
-    q.ntensors = a->L; q.L = a->L; q.B = a->B; q.d = a->d; q.F_pitch = a->F_pitch; q.tying = 0;
-    q.feat_off = a->feat_off; q.fcsr_tok = a->fcsr_tok; q.fcsr_val = a->delta; q.gs = p.x;
-    q.grad_a = nullptr; q.pen_coef = nullptr; q.norm2_out = nullptr; q.feat_offset = nullptr; q.feat_scale = nullptr;
-    q.d_feat_offset = nullptr; q.d_feat_scale = nullptr;
-    q.dgrad_row0 = a->dense_grad; q.h = p.h;
-    q.moments_bf16 = a->moments_bf16;
-    q.extra_idx = a->dense_grad == nullptr ? a->extra_idx : nullptr; q.extra_rows = a->extra_rows;
-    q.ctl = a->ctl; q.use_inv_scale = 0; q.norm_sq_out = nullptr;
     if (a->dense_grad != nullptr && a->extra_idx != nullptr) return -7;  // the row pipeline takes one kind of extra rows
     const int rc = launch_rows_adam_bulk(q, a->weights_bf16 != 0, a->h.sr_seed != 0, num_sms, a->status, st, a->n_entries);
     if (rc != 0) return rc;
     if (p.bias != nullptr) {
-      const int bgrid = int((1LL * a->L * a->F_pitch + 255) / 256);
       if (a->weights_bf16) launch_chained(encoder_bias_adam_kernel<t16>, bgrid, 256, 0, st, p);
       else launch_chained(encoder_bias_adam_kernel<float>, bgrid, 256, 0, st, p);
     }
