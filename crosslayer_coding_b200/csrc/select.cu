@@ -2079,7 +2079,11 @@ static FlatGeom flat_geom(const CltSelectArgs* a) {
 // `hist` holds two histograms of 8192 counters, zeroed by the caller.
 extern "C" int CLT_FN(clt_batchtopk_select)(const CltSelectArgs* a, const CltExchangeArgs* exa, cudaStream_t st) {
   if (a->ld % 8 != 0 || a->layer_stride % 8 != 0 || a->stat_pitch % 4 != 0 || a->F > a->ld) return -1;
-  const ScanGeom g = scan_geom(a);
+  ScanGeom g = scan_geom(a);
+  // Kept densely, half the rows per CTA: a tracked range holds 1.75 k elements, so that of the 16384 pieces of 64 rows 900 may hold one at one kept
+  // element in 256 and 1800 at one in 128, and the queue (2048) must not overflow while the cut moves: every overflow costs the
+  // full-range passes (evaluation of 13 x 2536 features, 1504 tokens, k = 245: 677 us with them, 354 without; 4 x 4096, 4096 tokens, k = 120: 807, 397).
+  if (256 * a->k_total > 1LL * a->B * a->L * a->full_F) g.rows_per_block = 32;
   const Exchange ex = to_exchange(exa);
   dim3 grid(((a->F + 7) / 8 + 255) / 256, (a->B + g.rows_per_block - 1) / g.rows_per_block, a->L);
   const t16* x = static_cast<const t16*>(a->x);
