@@ -338,22 +338,35 @@ __global__ void __launch_bounds__(256) zhist_collect_kernel(const t16* __restric
   const int nq_all = s_q;
   if (nq_all > kCollectQueue && threadIdx.x == 0) atomicOr(pool.count, 0x80000000u);  // lost groups: force the full-range pass
   const int nq = nq_all > kCollectQueue ? 0 : nq_all;  // lost groups: nothing of this pass will be used
-  for (int e = threadIdx.x; e < nq * 8; e += blockDim.x) {
-    const uint32_t item = s_queue[e >> 3];
-    const int r = r0 + int(item >> 8);
-    const int c = (blockIdx.x * blockDim.x + int(item & 255u)) * 8 + (e & 7);
-    if (c >= g.F) continue;
-    const float xv = t16_to_float(x[1LL * l * g.layer_stride + 1LL * r * g.ld + c]);
-    const float z = (xv - __ldg(mean + 1LL * l * g.sp + c)) * __ldg(rstd + 1LL * l * g.sp + c);
-    if (!(z >= z_lo)) continue;
-    const uint32_t key = float_to_key(z);
-    atomicAdd(&sh[min((key - key_lo) >> shift, uint32_t(kHistBins - 1))], 1u);
-    const int slot = atomicAdd(&s_n, 1);
-    if (slot < kPoolStage) {
-      s_key[slot] = key; s_tok[slot] = r; s_col[slot] = l * col_pitch + c; s_val[slot] = xv;
-    } else {  // staging full: append directly
-      const unsigned int q = atomicAdd(pool.count, 1u);
-      if ((long long)q < pool.cap) { pool.key[q] = key; pool.tok[q] = r; pool.col[q] = l * col_pitch + c; pool.val[q] = xv; }
+  // (four elements per thread and round: the loads of one after the other were a seventh of the kernel)
+  for (int e0 = threadIdx.x; e0 < nq * 8; e0 += 4 * 256) {
+    int r[4], c[4];
+    bool in[4];
+    float xv[4], mu[4], rs[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = e0 + 256 * u;
+      const uint32_t item = e < nq * 8 ? s_queue[e >> 3] : 0u;
+      r[u] = r0 + int(item >> 8);
+      c[u] = (blockIdx.x * 256 + int(item & 255u)) * 8 + (e & 7);
+      in[u] = e < nq * 8 && c[u] < g.F;
+      xv[u] = in[u] ? t16_to_float(x[1LL * l * g.layer_stride + 1LL * r[u] * g.ld + c[u]]) : 0.f;
+      mu[u] = in[u] ? __ldg(mean + 1LL * l * g.sp + c[u]) : 0.f;
+      rs[u] = in[u] ? __ldg(rstd + 1LL * l * g.sp + c[u]) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float z = (xv[u] - mu[u]) * rs[u];
+      if (!in[u] || !(z >= z_lo)) continue;
+      const uint32_t key = float_to_key(z);
+      atomicAdd(&sh[min((key - key_lo) >> shift, uint32_t(kHistBins - 1))], 1u);
+      const int slot = atomicAdd(&s_n, 1);
+      if (slot < kPoolStage) {
+        s_key[slot] = key; s_tok[slot] = r[u]; s_col[slot] = l * col_pitch + c[u]; s_val[slot] = xv[u];
+      } else {  // staging full: append directly
+        const unsigned int q = atomicAdd(pool.count, 1u);
+        if ((long long)q < pool.cap) { pool.key[q] = key; pool.tok[q] = r[u]; pool.col[q] = l * col_pitch + c[u]; pool.val[q] = xv[u]; }
+      }
     }
   }
   __syncthreads();
@@ -966,7 +979,7 @@ __global__ void __launch_bounds__(256) token_bound_kernel(WideTopk wt, int k, lo
   if (threadIdx.x == 0) wt.bound[tok] = bound;
 }
 
-__global__ void __launch_bounds__(256) token_collect_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
+__global__ void __launch_bounds__(256, 4) token_collect_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
                                                               int col_pitch, int f_valid, WideTopk wt) {
   if (chain_wait()) return;
   __shared__ uint16_t queue[kWideQueue];
@@ -1026,15 +1039,34 @@ __global__ void __launch_bounds__(256) token_collect_kernel(const t16* __restric
     if (int(threadIdx.x) < r1 - r0) atomicMax(&wt.n[r0 + threadIdx.x], 1 << 28);
     return;
   }
-  for (int e = threadIdx.x; e < nq * 8; e += 256) {
-    const uint32_t item = queue[e >> 3];
-    const int r = int(item >> 8), c = (blockIdx.x * 256 + int(item & 255u)) * 8 + (e & 7);
-    if (c >= f_valid || c >= g.F) continue;  // padding columns of a shard take no part
-    const float xv = t16_to_float(x[1LL * l * g.layer_stride + 1LL * (r0 + r) * g.ld + c]);
-    const uint32_t key = float_to_key((xv - __ldg(mean + 1LL * l * g.sp + c)) * __ldg(rstd + 1LL * l * g.sp + c));
-    if (key < bound[r]) continue;
-    const int slot = atomicAdd(&wt.n[r0 + r], 1);
-    if (slot >= 0 && slot < wt.cap) wt.list[1LL * (r0 + r) * wt.cap + slot] = ((unsigned long long)key << 32) | (0xFFFFFFFFu - (unsigned int)(l * col_pitch + c));
+  // Four elements per thread and round: each is a load of the element, a test and a trip to its token's counter, one after the other.  One at a time
+  // took longer than reading the tile (6 x 2048 x 32768, k = 64: 207 us, DRAM at 54 %).
+  for (int e0 = threadIdx.x; e0 < nq * 8; e0 += 4 * 256) {
+    int r[4], c[4], slot[4];
+    uint32_t key[4];
+    bool in[4];
+    float xv[4], mu[4], rs[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = e0 + 256 * u;
+      const uint32_t item = e < nq * 8 ? queue[e >> 3] : 0u;
+      r[u] = int(item >> 8);
+      c[u] = (blockIdx.x * 256 + int(item & 255u)) * 8 + (e & 7);
+      in[u] = e < nq * 8 && c[u] < f_valid && c[u] < g.F;  // padding columns of a shard take no part
+      xv[u] = in[u] ? t16_to_float(x[1LL * l * g.layer_stride + 1LL * (r0 + r[u]) * g.ld + c[u]]) : 0.f;
+      mu[u] = in[u] ? __ldg(mean + 1LL * l * g.sp + c[u]) : 0.f;
+      rs[u] = in[u] ? __ldg(rstd + 1LL * l * g.sp + c[u]) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      key[u] = float_to_key((xv[u] - mu[u]) * rs[u]);
+      in[u] = in[u] && key[u] >= bound[r[u]];
+      slot[u] = in[u] ? atomicAdd(&wt.n[r0 + r[u]], 1) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (in[u] && slot[u] >= 0 && slot[u] < wt.cap)
+        wt.list[1LL * (r0 + r[u]) * wt.cap + slot[u]] = ((unsigned long long)key[u] << 32) | (0xFFFFFFFFu - (unsigned int)(l * col_pitch + c[u]));
   }
 }
 
