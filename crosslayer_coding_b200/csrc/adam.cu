@@ -79,6 +79,15 @@ __device__ __forceinline__ void adam1(float& w, float& m, float& v, float g, con
   const float denom = fmaf(sqrtf(v), r.isb2, r.eps);
   w = fmaf(-r.step, __fdividef(m, denom), w);
 }
+// The same for two elements (every operation rounds as in adam1).
+__device__ __forceinline__ void adam2(float2& w, float2& m, float2& v, float2 g, const HyperRegs& r) {
+  g = f2_fma(f2_all(r.wd_l2), w, g);
+  w = f2_mul(w, f2_all(r.decay));
+  m = f2_fma(f2_all(r.omb1), f2_sub(g, m), m);
+  v = f2_fma(f2_all(r.omb2), f2_fma(g, g, make_float2(-v.x, -v.y)), v);
+  const float2 denom = f2_fma(make_float2(sqrtf(v.x), sqrtf(v.y)), f2_all(r.isb2), f2_all(r.eps));
+  w = f2_fma(f2_all(-r.step), make_float2(__fdividef(m.x, denom.x), __fdividef(m.y, denom.y)), w);
+}
 __device__ __forceinline__ void adam_update8(float (&w)[8], float (&m)[8], float (&v)[8], const float (&g)[8], const AdamHyper& h) {
   const HyperRegs r = make_regs(h);
 #pragma unroll
@@ -966,6 +975,8 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
 // Against the row pipeline above (a CTA per row): that one has five or six rows per SM at its consumers, each of which waits
 // for the lists and seed rows beyond the four staged ones, twice per row and one row after the other; here 16 to 24 rows per SM do so at the
 // same time, and the dot products of a row (dL/da) and its norm need no sum across warps.
+// With sixteen warps per SM what counts is the instructions of a row (issue slots 60 % full, DRAM at 45 %), so the arithmetic is two-wide: tied
+// Pythia-70m shape, both sweeps 933 -> 860 us; per-target decoders of 6 x 16384 x 512, 9 entries per row, 284 -> 254; rows with three entries unchanged.
 template <int NC>
 __device__ __forceinline__ void load_seed_row(const t16* row, int lane, int d, uint2 (&q)[NC]) {
 #pragma unroll
@@ -1106,12 +1117,16 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
     t16* w_s = reinterpret_cast<t16*>(stage);
     float* m_s = reinterpret_cast<float*>(stage + w_bytes);
     float* v_s = reinterpret_cast<float*>(stage + w_bytes + mv_bytes);
-    float w[NC][4], g[NC][4];
+    float2 w[NC][2], g[NC][2];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) w[c][k] = g[c][k] = 0.f;
-      if (c * 128 + lane * 4 < d) ldbf<4>(w_s + c * 128 + lane * 4, w[c]);
+      for (int k = 0; k < 2; ++k) w[c][k] = g[c][k] = f2_all(0.f);
+      if (c * 128 + lane * 4 < d) {
+        const uint2 u = *reinterpret_cast<const uint2*>(w_s + c * 128 + lane * 4);
+        w[c][0] = make_float2(t16_lo(u.x), t16_hi(u.x));
+        w[c][1] = make_float2(t16_lo(u.y), t16_hi(u.y));
+      }
     }
     for (int j0 = 0; j0 < total; j0 += 32) {
       if (j0 > 0) load_list(cur, b, n, j0, x, tok, a);
@@ -1127,21 +1142,22 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
         float dot[kNarrowBatch];
 #pragma unroll
         for (int k = 0; k < kNarrowBatch; ++k) {
-          const float ak = __shfl_sync(0xFFFFFFFFu, a, (k0 + k) & 31);
-          dot[k] = 0.f;
+          const float2 ak = f2_all(__shfl_sync(0xFFFFFFFFu, a, (k0 + k) & 31));
+          float2 dot2 = f2_all(0.f);
           if (k0 + k < cnt) {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
               if (c * 128 + lane * 4 < d) {
-                const float gv[4] = {t16_lo(q[k][c].x), t16_hi(q[k][c].x), t16_lo(q[k][c].y), t16_hi(q[k][c].y)};
+                const float2 gv[2] = {make_float2(t16_lo(q[k][c].x), t16_hi(q[k][c].x)), make_float2(t16_lo(q[k][c].y), t16_hi(q[k][c].y))};
 #pragma unroll
-                for (int z = 0; z < 4; ++z) {
-                  g[c][z] = fmaf(ak, gv[z], g[c][z]);
-                  dot[k] = fmaf(gv[z], w[c][z], dot[k]);
+                for (int z = 0; z < 2; ++z) {
+                  g[c][z] = f2_fma(ak, gv[z], g[c][z]);
+                  dot2 = f2_fma(gv[z], w[c][z], dot2);
                 }
               }
             }
           }
+          dot[k] = dot2.x + dot2.y;
         }
         if (p.grad_a != nullptr) {
           const float sdot = warp_sum_many<kNarrowBatch>(dot, lane);
@@ -1153,39 +1169,37 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
     }
     const float* xrow = cur.r == 0 ? extra_row_ptr(p, col) : nullptr;
     const long long eo = elem_of(cur);
-    float norm2 = 0.f;
+    float2 norm2 = f2_all(0.f);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const int e = c * 128 + lane * 4;
       if (e < d) {
-        float m[4], v[4], extra[4] = {0.f, 0.f, 0.f, 0.f};
-        ldf<4>(m_s + e, m);
-        ldf<4>(v_s + e, v);
-        if (xrow != nullptr) {
-          const float4 t4 = __ldg(reinterpret_cast<const float4*>(xrow + e));
-          extra[0] = t4.x; extra[1] = t4.y; extra[2] = t4.z; extra[3] = t4.w;
-        }
+        const float4 m4 = *reinterpret_cast<const float4*>(m_s + e), v4 = *reinterpret_cast<const float4*>(v_s + e);
+        float2 m[2] = {make_float2(m4.x, m4.y), make_float2(m4.z, m4.w)}, v[2] = {make_float2(v4.x, v4.y), make_float2(v4.z, v4.w)};
+        float4 extra = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (xrow != nullptr) extra = __ldg(reinterpret_cast<const float4*>(xrow + e));
 #pragma unroll
-        for (int z = 0; z < 4; ++z) {
-          float gq = fmaf(pc, w[c][z], g[c][z] * gsc);
-          if (xrow != nullptr) gq += extra[z];
-          adam1(w[c][z], m[z], v[z], gq * sc.clip, hr);
-          if (!PT) norm2 = fmaf(w[c][z], w[c][z], norm2);
+        for (int z = 0; z < 2; ++z) {
+          float2 gq = f2_fma(f2_all(pc), w[c][z], f2_mul(g[c][z], f2_all(gsc)));
+          if (xrow != nullptr) gq = f2_add(gq, z == 0 ? make_float2(extra.x, extra.y) : make_float2(extra.z, extra.w));
+          adam2(w[c][z], m[z], v[z], f2_mul(gq, f2_all(sc.clip)), hr);
+          if (!PT) norm2 = f2_fma(w[c][z], w[c][z], norm2);
         }
-        stbf<4, SR>(w_s + e, w[c], p.h.sr_seed, (unsigned int)(unsigned long long)(p.row_start[cur.ti] * d + eo + e));
+        const float wn[4] = {w[c][0].x, w[c][0].y, w[c][1].x, w[c][1].y};
+        stbf<4, SR>(w_s + e, wn, p.h.sr_seed, (unsigned int)(unsigned long long)(p.row_start[cur.ti] * d + eo + e));
         if (PT) {  // norms of the stored (rounded) weights
           float wr[4];
           ldbf<4>(w_s + e, wr);
 #pragma unroll
-          for (int z = 0; z < 4; ++z) norm2 = fmaf(wr[z], wr[z], norm2);
+          for (int z = 0; z < 2; ++z) norm2 = f2_fma(make_float2(wr[2 * z], wr[2 * z + 1]), make_float2(wr[2 * z], wr[2 * z + 1]), norm2);
         }
-        stf<4>(m_s + e, m);
-        stf<4>(v_s + e, v);
+        *reinterpret_cast<float4*>(m_s + e) = make_float4(m[0].x, m[0].y, m[1].x, m[1].y);
+        *reinterpret_cast<float4*>(v_s + e) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
       }
     }
     if (p.norm2_out != nullptr) {
-      norm2 = warp_sum(norm2);
-      if (lane == 0) atomicAdd(&p.norm2_out[col], norm2);
+      const float sn = warp_sum(norm2.x + norm2.y);
+      if (lane == 0) atomicAdd(&p.norm2_out[col], sn);
     }
     fence_proxy_async();  // the row written above is read next by the bulk stores (async proxy)
     __syncwarp();

@@ -407,6 +407,27 @@ __device__ __forceinline__ float key_to_float(uint32_t k) {
   return __uint_as_float(u);
 }
 
+// Two-wide fp32 instructions: the rounding of the one-wide ones (round to nearest, subnormals flushed as in the rest of the build), half the issue slots.
+#define CLT_F2_BINARY(name, op)                                                                                                        \
+  __device__ __forceinline__ float2 name(float2 x, float2 y) {                                                                         \
+    float2 r;                                                                                                                          \
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" op " d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"        \
+        : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));                                                              \
+    return r;                                                                                                                          \
+  }
+CLT_F2_BINARY(f2_add, "add.rn.ftz.f32x2")
+CLT_F2_BINARY(f2_sub, "sub.rn.ftz.f32x2")
+CLT_F2_BINARY(f2_mul, "mul.rn.ftz.f32x2")
+#undef CLT_F2_BINARY
+__device__ __forceinline__ float2 f2_fma(float2 x, float2 y, float2 z) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.ftz.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
+  return r;
+}
+__device__ __forceinline__ float2 f2_all(float v) { return make_float2(v, v); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);

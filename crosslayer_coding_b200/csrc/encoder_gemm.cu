@@ -428,19 +428,6 @@ struct StripSums {
   float ta, ua, tb, ub;     // over the chunks before it (see colstats_kernel: rows split over blockIdx.z)
   float shift_a, shift_b;   // the first token's value
 };
-__device__ __forceinline__ float2 f2_add(float2 x, float2 y) {
-  float2 r;
-  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.ftz.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
-  return r;
-}
-__device__ __forceinline__ float2 f2_fma(float2 x, float2 y, float2 z) {
-  float2 r;
-  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
-      "fma.rn.ftz.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
-  return r;
-}
 // Two stored values (tokens t and t + 1 of a feature); `valid` of them are rows of the matrix, the others add nothing.
 template <bool MASKED>
 __device__ __forceinline__ void add_pair(float2& s, float2& q, uint32_t u, float shift, int valid) {
