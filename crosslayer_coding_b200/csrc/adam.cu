@@ -610,6 +610,12 @@ __device__ __forceinline__ void stbf(t16* p, const float (&o)[EPT], unsigned int
   }
 }
 
+// Elements i and i + 1 of a register array.
+template <int N>
+__device__ __forceinline__ float2 f2_get(const float (&x)[N], int i) { return make_float2(x[i], x[i + 1]); }
+template <int N>
+__device__ __forceinline__ void f2_put(float (&x)[N], int i, float2 v) { x[i] = v.x; x[i + 1] = v.y; }
+
 // Warp sums of N values at once (N a power of two up to 32): every exchange halves the number of values a lane still carries,
 // N - 1 + 5 - log2(N) shuffles instead of 5 N.  Returns the total of value warp_sum_slot<N>(lane); the tree is warp_sum's.
 template <int N>
@@ -637,7 +643,7 @@ __device__ __forceinline__ int warp_sum_slot(int lane) { return lane / (32 / N);
 // activation), cnt of them.  The seed rows come kBatch at a time, so a feature with many entries waits for L2 once per
 // kBatch of them and not twice per entry (eight entries per feature on average, tied Pythia-70m shape: both sweeps of a step
 // 1.81 -> 1.60 ms).  It takes 72 registers; a cap of 64 spills and cost 0.4 ms at the GPT-2 shape.
-template <int EPT, int kBatch>
+template <int EPT, int kBatch, bool kPairs>
 __device__ __forceinline__ void add_entries(int cnt, int my_x, int my_tok, float my_a, const t16* gs_t, int d, bool act, int lane, const float (&w)[EPT],
                                             float (&g)[EPT], float* grad_a, float gsc) {
   for (int j0 = 0; j0 < cnt; j0 += kBatch) {
@@ -654,18 +660,25 @@ __device__ __forceinline__ void add_entries(int cnt, int my_x, int my_tok, float
 #pragma unroll
     for (int k = 0; k < kBatch; ++k) {
       const float a = __shfl_sync(0xFFFFFFFFu, my_a, j0 + k);
-      dot[k] = 0.f;
+      float2 dot2 = f2_all(0.f);
       if (act && j0 + k < cnt) {
 #pragma unroll
         for (int z = 0; z < EPT / 4; ++z) {
-          const float gv[4] = {t16_lo(q2[k][z].x), t16_hi(q2[k][z].x), t16_lo(q2[k][z].y), t16_hi(q2[k][z].y)};
+          const float2 gv[2] = {make_float2(t16_lo(q2[k][z].x), t16_hi(q2[k][z].x)), make_float2(t16_lo(q2[k][z].y), t16_hi(q2[k][z].y))};
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            g[4 * z + c] = fmaf(a, gv[c], g[4 * z + c]);
-            dot[k] = fmaf(gv[c], w[4 * z + c], dot[k]);
+          for (int c = 0; c < 2; ++c) {
+            const int e = 4 * z + 2 * c;
+            if constexpr (kPairs) {
+              f2_put(g, e, f2_fma(f2_all(a), gv[c], f2_get(g, e)));
+              dot2 = f2_fma(gv[c], f2_get(w, e), dot2);
+            } else {
+              g[e] = fmaf(a, gv[c].x, g[e]); g[e + 1] = fmaf(a, gv[c].y, g[e + 1]);
+              dot2.x = fmaf(gv[c].y, w[e + 1], fmaf(gv[c].x, w[e], dot2.x));
+            }
           }
         }
       }
+      dot[k] = dot2.x + dot2.y;
     }
     if (grad_a != nullptr) {
       const float sdot = warp_sum_many<kBatch>(dot, lane);
@@ -682,6 +695,9 @@ __device__ __forceinline__ void add_entries(int cnt, int my_x, int my_tok, float
 // eight elements per thread (d <= 1792).
 template <typename WT, bool SR, int EPT, typename MT, bool PT = false, int NB = 4, bool NARROW = false>
 __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW ? (EPT == 4 ? 5 : 3) : (EPT == 4 ? 3 : 2)) decoder_rows_adam_bulk_kernel(const DecAdamParams p, int gthreads, int stage_bytes, int ns, int* status) {
+  // Two-wide arithmetic (12 x 768, 24576 features: both sweeps 5987 -> 5932 us, 3072 features 820 -> 794; 4 x 640, 25 entries per feature 1335 -> 1276),
+  // except in the form whose registers it overflows (6 x 2048: 861 us without, 869 with it).
+  constexpr bool kPairs = EPT == 4 || NB != 4 || PT;
   extern __shared__ __align__(128) uint8_t smem_raw_adam[];  // bulk copies need 16-byte alignment only
   uint8_t* ring = smem_raw_adam;
   AdamBulkShared* sh = reinterpret_cast<AdamBulkShared*>(ring + size_t(ns) * stage_bytes);
@@ -857,9 +873,19 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
             float gv[EPT];
             ldbf<EPT>(gs_s + j * d, gv);
 #pragma unroll
-            for (int q = 0; q < EPT; ++q) {
-              g[q] = fmaf(a, gv[q], g[q]);
-              dacc[j] = fmaf(gv[q], w[q], dacc[j]);
+            for (int q = 0; q < EPT; q += 2) {
+              if constexpr (kPairs) {
+                f2_put(g, q, f2_fma(f2_all(a), f2_get(gv, q), f2_get(g, q)));
+              } else {
+                g[q] = fmaf(a, gv[q], g[q]); g[q + 1] = fmaf(a, gv[q + 1], g[q + 1]);
+                dacc[j] = fmaf(gv[q + 1], w[q + 1], fmaf(gv[q], w[q], dacc[j]));
+              }
+            }
+            if constexpr (kPairs) {
+              float2 dot = f2_mul(f2_get(gv, 0), f2_get(w, 0));
+#pragma unroll
+              for (int q = 2; q < EPT; q += 2) dot = f2_fma(f2_get(gv, q), f2_get(w, q), dot);
+              dacc[j] += dot.x + dot.y;
             }
           }
         }
@@ -887,14 +913,14 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
           const int x = __shfl_sync(0xFFFFFFFFu, seg_b, seg) + j - (__shfl_sync(0xFFFFFFFFu, incl, seg) - __shfl_sync(0xFFFFFFFFu, seg_n, seg));
           const int my_tok = j < total ? __ldg(p.fcsr_tok + x) : 0;
           const float my_a = j < total ? __ldg(p.fcsr_val + x) : 0.f;
-          add_entries<EPT, NB>(min(32, total - j0), x, my_tok, my_a, p.gs + 1LL * ti * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
+          add_entries<EPT, NB, kPairs>(min(32, total - j0), x, my_tok, my_a, p.gs + 1LL * ti * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
         }
       } else {
         for (int x0 = b + kAdamSlots; x0 < b + ne; x0 += 32) {  // entries beyond the slots
           const int cnt = min(32, b + ne - x0);
           const int my_tok = lane < cnt ? __ldg(p.fcsr_tok + x0 + lane) : 0;
           const float my_a = lane < cnt ? __ldg(p.fcsr_val + x0 + lane) : 0.f;
-          add_entries<EPT, NB>(cnt, x0 + lane, my_tok, my_a, p.gs + 1LL * (ti + r) * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
+          add_entries<EPT, NB, kPairs>(cnt, x0 + lane, my_tok, my_a, p.gs + 1LL * (ti + r) * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
         }
       }
       if (act) {
@@ -908,12 +934,25 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
             dg0[q] = t4.x; dg0[q + 1] = t4.y; dg0[q + 2] = t4.z; dg0[q + 3] = t4.w;
           }
         }
+        float2 row2 = f2_all(0.f);
 #pragma unroll
-        for (int q = 0; q < EPT; ++q) {
-          float gq = fmaf(pc, w[q], g[q] * gsc);
-          if (extra) gq += dg0[q];
-          adam1(w[q], m[q], v[q], gq * sc.clip, hr);
-          if (!PT) norm2 = fmaf(w[q], w[q], norm2);
+        for (int q = 0; q < EPT; q += 2) {
+          if constexpr (kPairs) {
+            float2 w2 = f2_get(w, q), m2 = f2_get(m, q), v2 = f2_get(v, q);
+            float2 gq = f2_fma(f2_all(pc), w2, f2_mul(f2_get(g, q), f2_all(gsc)));
+            if (extra) gq = f2_add(gq, f2_get(dg0, q));
+            adam2(w2, m2, v2, f2_mul(gq, f2_all(sc.clip)), hr);
+            f2_put(w, q, w2); f2_put(m, q, m2); f2_put(v, q, v2);
+            if (!PT) row2 = f2_fma(w2, w2, row2);
+          } else {
+#pragma unroll
+            for (int z = q; z < q + 2; ++z) {
+              float gq = fmaf(pc, w[z], g[z] * gsc);
+              if (extra) gq += dg0[z];
+              adam1(w[z], m[z], v[z], gq * sc.clip, hr);
+              if (!PT) row2.x = fmaf(w[z], w[z], row2.x);
+            }
+          }
         }
         const unsigned long long gidx = (unsigned long long)(p.row_start[ti] * d + h->elem_off + e0);
         if (sizeof(WT) == 2) stbf<EPT, SR>(reinterpret_cast<t16*>(w_s), w, p.h.sr_seed, (unsigned int)gidx);
@@ -921,8 +960,9 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
         if (PT) {  // norms of the stored (rounded) weights
           ldbf<EPT>(reinterpret_cast<const t16*>(w_s), w);
 #pragma unroll
-          for (int q = 0; q < EPT; ++q) norm2 = fmaf(w[q], w[q], norm2);
+          for (int q = 0; q < EPT; q += 2) row2 = f2_fma(f2_get(w, q), f2_get(w, q), row2);
         }
+        norm2 += row2.x + row2.y;
         if (sizeof(MT) == 2) {
           // bf16 moments are always rounded stochastically: with beta2 = 0.999 a nearest rounding would freeze v
           // one hash per thread and row seeds a linear congruential stream: two 16-bit dither values per element
