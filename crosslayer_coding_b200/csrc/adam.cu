@@ -1017,12 +1017,16 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
 // same time, and the dot products of a row (dL/da) and its norm need no sum across warps.
 // With sixteen warps per SM what counts is the instructions of a row (issue slots 60 % full, DRAM at 45 %), so the arithmetic is two-wide: tied
 // Pythia-70m shape, both sweeps 933 -> 860 us; per-target decoders of 6 x 16384 x 512, 9 entries per row, 284 -> 254; rows with three entries unchanged.
+// A row's stage is refilled in the next row's turn, behind the requests for its seed rows, when the store has long read it: waiting for
+// the store at the end of the row, and a test per block of 128 although only the last can be short, cost 3 to 7 % (6 x 32768 x 512 with 4 entries
+// per row 677 -> 655 us, per-target decoders 230 -> 213, 8 x 8192 x 256 untied 358 -> 344).  Rows of up to 128 elements are over too
+// soon for that (277 us, refilled late 283): they wait for the store.  Per-target encoder rows with two entries lose 1 to 2 % (177 -> 179).
 template <int NC>
 __device__ __forceinline__ void load_seed_row(const t16* row, int lane, int d, uint2 (&q)[NC]) {
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const int e = c * 128 + lane * 4;
-    if (e < d) q[c] = __ldg(reinterpret_cast<const uint2*>(row + e));
+    if (c + 1 < NC || e < d) q[c] = __ldg(reinterpret_cast<const uint2*>(row + e));
   }
 }
 
@@ -1041,6 +1045,8 @@ struct RowAt {
 
 template <bool SR, int NC, bool PT>
 __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_rows_adam_kernel(const DecAdamParams p, long long total_rows, int* status) {
+  static_assert(kNarrowStages == 2, "the late refill is for the next row");
+  constexpr bool kRefillLate = NC > 1;
   extern __shared__ __align__(128) uint8_t smem_narrow[];
   __shared__ uint64_t full_s[kNarrowWarps][kNarrowStages];
   __shared__ int abort_s;
@@ -1149,6 +1155,10 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
     int x1, tok1;
     float a1;
     const int total1 = load_list(nxt, b1, n1, 0, x1, tok1, a1);
+    if (kRefillLate && i > 0) {  // the stage of the row before; its store has read it by now
+      if (lane == 0) bulk_wait_read<0>();
+      issue_row(nxt, int((i + 1) % kNarrowStages));
+    }
     const int col = cur.ti * Fp + cur.f;
     float pc = p.pen_coef ? __ldg(p.pen_coef + col) : 0.f;
     if (PT && p.pen_coef) pc = warp_sum(lane <= cur.ti ? __ldg(p.pen_coef + lane * Fp + cur.f) : 0.f);  // the row is part of the norms of all sources
@@ -1162,7 +1172,7 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
     for (int c = 0; c < NC; ++c) {
 #pragma unroll
       for (int k = 0; k < 2; ++k) w[c][k] = g[c][k] = f2_all(0.f);
-      if (c * 128 + lane * 4 < d) {
+      if (c + 1 < NC || c * 128 + lane * 4 < d) {
         const uint2 u = *reinterpret_cast<const uint2*>(w_s + c * 128 + lane * 4);
         w[c][0] = make_float2(t16_lo(u.x), t16_hi(u.x));
         w[c][1] = make_float2(t16_lo(u.y), t16_hi(u.y));
@@ -1187,7 +1197,7 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
           if (k0 + k < cnt) {
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-              if (c * 128 + lane * 4 < d) {
+              if (c + 1 < NC || c * 128 + lane * 4 < d) {
                 const float2 gv[2] = {make_float2(t16_lo(q[k][c].x), t16_hi(q[k][c].x)), make_float2(t16_lo(q[k][c].y), t16_hi(q[k][c].y))};
 #pragma unroll
                 for (int z = 0; z < 2; ++z) {
@@ -1213,7 +1223,7 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       const int e = c * 128 + lane * 4;
-      if (e < d) {
+      if (c + 1 < NC || e < d) {
         const float4 m4 = *reinterpret_cast<const float4*>(m_s + e), v4 = *reinterpret_cast<const float4*>(v_s + e);
         float2 m[2] = {make_float2(m4.x, m4.y), make_float2(m4.z, m4.w)}, v[2] = {make_float2(v4.x, v4.y), make_float2(v4.z, v4.w)};
         float4 extra = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1248,11 +1258,13 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
       bulk_store_1d_hint(p.m[cur.ti] + eo, stage + w_bytes, mv_bytes, pol_stream);
       bulk_store_1d_hint(p.v[cur.ti] + eo, stage + w_bytes + mv_bytes, mv_bytes, pol_stream);
       bulk_commit();
-      bulk_wait_read<0>();  // the stage is refilled
+      if (!kRefillLate) bulk_wait_read<0>();  // the stage is refilled
     }
-    RowAt far{cur.idx + kNarrowStages * stride, nxt.ti, 0, 0};
-    place(far);
-    issue_row(far, st);
+    if (!kRefillLate) {
+      RowAt far{cur.idx + kNarrowStages * stride, nxt.ti, 0, 0};
+      place(far);
+      issue_row(far, st);
+    }
     cur = nxt; nxt = nn;
     b = b1; n = n1; b1 = b2; n1 = n2;
     x = x1; tok = tok1; a = a1; total = total1;
