@@ -132,6 +132,11 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // rows at 7.6 TB/s, of which DRAM gives about 6); 512 tokens, k = 32: 124 and 62; 1000 tokens of 16 x 2048, 242 entries: 1138 and 963; 4096
 // tokens of 6 x 512, per-target tied, k = 64: 172 and 132.  Eight warps pay where there are too few CTAs to fill the chip
 // (16 tokens 36 us with four, 22 with eight; 128 tokens of 200 entries 72 and 67; 256: 102 and 109).
+// With so few that their slices of 256 columns are all on the chip at once (four CTAs of eight warps per SM), a CTA takes a slice and its warps eight
+// rows at a time: three or four times the loads in flight, and the chain of a warp is half as long.  16 tokens of 12 x 768, 200 entries, 29.2 -> 21.5 us
+// (lists of 100: 22.1 -> 15.4), 8 of 12 x 1024 14.4 -> 10.4, 140 of 1 x 1024 21.7 -> 14.9; near-empty lists 4.0 -> 4.3 and 5.2 -> 4.6.  Beyond one round of
+// CTAs it wins only with long lists (64 tokens of 12 x 768, 200 entries 70 -> 59, six entries 12 -> 14; 64 of 12 x 1024 32 and 33); short equal lists (8 to
+// 24 entries 0.4 us), rows of up to 512 (12 x 24 tokens, 50 entries: 6.2 and 6.7) and above 1024 (60 tokens of 16 x 2048: 64 and 76) stay whole.
 // Rows in flight against warps per SM: four rows and 20 warps (three vectors per lane) or 16 (four) are best up to some thousands of CTAs
 // (2048 tokens, k = 200: 588 us against 605 with two rows and 28 warps), two rows and more warps beyond (4096 tokens 1164 and 1081; 1000 tokens
 // of 16 x 2048 1003 and 963).  There the tokens are also taken in the order of their list lengths, longest first: warps that
@@ -158,6 +163,7 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // below the line 4096 of 6 x 512, 48 entries on average but few in most lists, 99 / 130).
 constexpr long long kRunningMinWarps = 1024;   // tokens x chunks; below, the (token, target) split has L times as many CTAs
 constexpr long long kEightWarpsBelow = 2048;   // CTAs
+constexpr long long kSlicesUpTo = 592;         // CTAs of 256 columns: 148 SMs x 4
 constexpr long long kManyCtas = 28672;         // CTAs
 constexpr long long kPairNarrowFrom = 24576;   // (token, target) pairs
 constexpr int kRunningOrderFrom = 4096;        // tokens
@@ -603,6 +609,10 @@ static bool takes_running(const CltDecodeArgs* a) {
 static long long walk_ctas(const CltDecodeArgs* a) { return 1LL * a->B * a->L * walk_chunks(a); }
 static int walk_vectors(const CltDecodeArgs* a) { return (a->d / 8 + 32 * walk_chunks(a) - 1) / (32 * walk_chunks(a)); }
 static bool short_lists(const CltDecodeArgs* a) { return a->expected > 0 && a->expected < kShortBelow; }
+static int slices(const CltDecodeArgs* a) { return (a->d + 255) / 256; }
+static bool takes_slices(const CltDecodeArgs* a) {
+  return a->d > 512 && a->d <= 1024 && !short_lists(a) && 1LL * a->B * a->L * slices(a) <= kSlicesUpTo;
+}
 // Lists of one length that a warp takes alone.
 static bool one_warp_lists(const CltDecodeArgs* a) {
   if (a->equal == 0 || a->expected <= 0) return false;
@@ -657,7 +667,9 @@ extern "C" int CLT_FN(clt_sparse_decode)(const CltDecodeArgs* a, cudaStream_t st
   const int chunks = walk_chunks(a), nv = walk_vectors(a);
   const long long ctas = walk_ctas(a);
   const dim3 grid(a->B, a->L, chunks);
-  if (ctas < kEightWarpsBelow) {
+  if (takes_slices(a)) {
+    launch_chained(decode_walk_kernel<1, 1, 8, 8, 32>, dim3(a->B, a->L, slices(a)), 256, 0, st, p);
+  } else if (ctas < kEightWarpsBelow) {
     if (nv <= 1) launch_chained(decode_walk_kernel<1, 1, 8, 4, 32>, grid, 256, 0, st, p);
     else if (nv == 2) launch_chained(decode_walk_kernel<2, 1, 8, 4, 24>, grid, 256, 0, st, p);
     else if (nv == 3) launch_chained(decode_walk_kernel<3, 1, 8, 4, 16>, grid, 256, 0, st, p);

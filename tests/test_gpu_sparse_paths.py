@@ -169,6 +169,34 @@ def test_gather_decode_of_equal_long_lists(ext, tying, L, B, d, expected):
     _check_decode(ext, L, B, d, tying, False, F=72, entries=_uneven_entries, expected=expected, equal=True)
 
 
+# slices of 256 columns per CTA where all of them are on the chip at once, at most 592: on both sides of the line, the last slice with one vector,
+# half and whole, next to short expected lists, which keep whole rows
+@pytest.mark.parametrize("tying", [0, 1, 2])
+@pytest.mark.parametrize("L,B,d", [(2, 98, 520), (2, 99, 520), (4, 37, 1024), (4, 38, 1024), (12, 16, 768), (3, 2, 776), (1, 197, 640)])
+@pytest.mark.parametrize("opts", [dict(), dict(expected=20), dict(expected=200, equal=True, dtype=torch.float16), dict(addend=True, rows_limit=2)])
+def test_gather_decode_of_few_tokens(ext, tying, L, B, d, opts):
+    _check_decode(ext, L, B, d, tying, tying != 0 and opts.get("rows_limit") is None, F=300, entries=_uneven_entries, **opts)
+
+
+@pytest.mark.parametrize("d", [520, 768, 1024])
+def test_decode_in_slices_equals_whole_rows(ext, d):
+    """An element's sum takes the same entries in the same order in both forms: few tokens (slices) give the bits that they give among many."""
+    dev = _dev()
+    g = torch.Generator().manual_seed(d)
+    L, F, few, many = 3, 400, 16, 512
+    tok, col, val = _uneven_entries(g, L, many, F, 0, dev)
+    W = [(torch.randn(F, L - s, d, generator=g) / 4).to(torch.bfloat16).to(dev) for s in range(L)]
+    out = []
+    for B in (few, many):
+        keep = tok < B
+        c = _csr(ext, tok[keep].contiguous(), col[keep].contiguous(), val[keep].contiguous(), B, L * F, F)
+        part = torch.full((L, B, d), float("nan"), device=dev)
+        ext.sparse_decode(W, L, B, d, F, 0, c["tok_off"], c["tcsr_col"], c["tcsr_val"], None, None, part, None, None, None, None, None, None, None, 0, [], 0, 0,
+                          torch.zeros(4, dtype=I32, device=dev), None, 0, 0, False)
+        out.append(part[:, :few])
+    assert torch.equal(*out)
+
+
 @pytest.mark.parametrize("L,B,d", [(3, 1303, 200), (3, 1303, 512)])
 def test_gather_decode_of_equal_short_lists_in_narrow_rows(ext, L, B, d):
     _check_decode(ext, L, B, d, 0, False, F=72, entries=_uneven_entries, expected=20, equal=True)
