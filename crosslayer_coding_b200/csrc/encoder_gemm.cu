@@ -8,10 +8,9 @@
 //
 // Two kernels: CTA pairs on transposed tiles (below; from 256 tokens on), and the one here, one CTA per tile, for fewer.
 //
-// Structure of both: one CTA per SM (the pairs have two more warps, for the stores).  Warp 0 feeds a 4-stage shared-memory ring (3 with sums per tile) with TMA tile loads
-// (no cluster multicast: every CTA fetches its own tiles), warp 1 issues tcgen05.mma 128x256x16 into one
-// of two 256-column TMEM accumulators, warps 2-9 drain the other accumulator with tcgen05.ld, add the
-// bias and store bf16.  Tiles are ordered m-fastest so CTAs that run together share the weight tile in L2.
+// Structure of both: one CTA per SM.  Warp 0 feeds a shared-memory ring (here four stages, three with sums per tile) with TMA tile loads (no cluster
+// multicast: every CTA fetches its own tiles), warp 1 issues tcgen05.mma into one of two 256-column TMEM accumulators, eight warps drain the
+// other one with tcgen05.ld, add the bias, convert to 16 bit and hand staging tiles to TMA stores (which two more warps issue in the pairs).
 // Every mbarrier wait is bounded; on a timeout the CTA records STATUS_WAIT_TIMEOUT, drains its copies,
 // frees its TMEM and returns.
 #include <cstdlib>

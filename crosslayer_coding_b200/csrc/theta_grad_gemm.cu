@@ -14,8 +14,10 @@
 // The autograd path computes the same through P dense GEMM pairs and a dense [B, F] backward per layer.
 //
 // Structure: a persistent pipeline (TMA ring, one MMA thread, two TMEM accumulators, eight epilogue warps), one CTA on a tile of 128 tokens or
-// a pair of CTAs (cta_group::2) on 256.  What bounds it is the operand traffic: one CTA loads 48 KB for 512 MMA cycles, more than L2 hands an SM
-// (12 x 4096 x 4096 x 768: 1403 us, tensor cores 79 % of the cycles), a CTA of a pair 32 KB (its own tokens, half of the decoder rows).
+// a pair of CTAs (cta_group::2) on 256.  One CTA loads 48 KB for 512 MMA cycles, more than L2 hands an SM, and stood still for operands; a CTA
+// of a pair loads 32 KB (its own tokens, half of the decoder rows).  With one row per feature the epilogue comes as often as every 12 k-steps, which
+// eight warps keep up with.  12 x 4096 x 4096 x 768: untied 1450 -> 1300 us (2.0 TFLOP, 1.57 PFLOP/s: the rate of the tensor cores
+// under the power cap bounds it now), one row per feature 463 -> 360; 2 x 8192 x 16384 x 136 603 -> 427.
 // No multicast loads.  Every mbarrier wait is bounded.
 #include <climits>
 

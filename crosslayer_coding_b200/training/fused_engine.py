@@ -7,7 +7,8 @@ One step is a fixed sequence of hand-written kernels and never materialises a de
  #    kernel (csrc/)                         replaces in the reference
 ====  =====================================  ============================================
  1    encoder_gemm  (tcgen05 + TMA)          L x F.linear + all_gather, run 2-4x per step
- 2    colstats                               per-layer mean/std temporaries
+ 2    its column sums; colstats for strips   per-layer mean/std temporaries
+      that no CTA pair takes whole
  3    batchtopk_select                       torch.topk over B*L*F + mask + multiply
  4    build_csr                              (dense mask is the reference's data structure)
  5    sparse_decode (+ loss epilogue)        P dense decoder GEMMs + P all-reduces + MSELoss
@@ -240,7 +241,7 @@ class FusedBatchTopKEngine:
         self.preact = torch.empty(L, B, Fl, dtype=self.t16, device=dev)
         self.mean = torch.empty(L, Fl, dtype=f32, device=dev)
         self.rstd = torch.empty(L, Fl, dtype=f32, device=dev)
-        self.tile_stats = None  # [L, ceil(B / 128), Fl, 2] fp32 switches the statistics into the GEMM epilogue
+        self.tile_stats = None  # [L, ceil(B / 128), Fl, 2] fp32: statistics from sums per block of 128 tokens
         # tracked histogram range {key_lo, shift} and the pool filled by the single pass over the pre-activations
         self.sel_state = torch.tensor([self.key_lo, self.shift], dtype=torch.int64, device=dev) if self.key_lo != 0 else None
         k_local = -(-self.k_total // max(1, self.world))
