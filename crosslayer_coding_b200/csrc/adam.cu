@@ -1559,6 +1559,7 @@ __global__ void __launch_bounds__(256) encoder_rows_adam_kernel(const EncAdamPar
 template <typename WT>
 __global__ void __launch_bounds__(256) encoder_bias_adam_kernel(const EncAdamParams p) {
   if (chain_wait()) return;
+  chain_release();
   const long long rows = 1LL * p.L * p.F_pitch;
   const StepScales sc = read_step_ctl(p.ctl);
   if (sc.skip) return;
@@ -1596,6 +1597,7 @@ __global__ void __launch_bounds__(256) dense_adam_kernel(WT* __restrict__ w, flo
                                                            const float* __restrict__ grad, long long n, AdamHyper h,
                                                            float* __restrict__ ctl, int seed_scaled, float norm_weight) {
   if (chain_wait()) return;
+  chain_release();
   const StepScales sc = read_step_ctl(ctl);
   if (sc.skip) return;
   const float gmul = h.grad_scale * (seed_scaled ? sc.inv_scale : 1.f);
@@ -1626,6 +1628,7 @@ __global__ void __launch_bounds__(256) dense_adam_kernel(WT* __restrict__ w, flo
 template <typename WT>
 __global__ void __launch_bounds__(256) decoder_norm2_kernel(const WT* __restrict__ w, float* __restrict__ out, int F, int R, int d) {
   if (chain_wait()) return;
+  chain_release();
   const int lane = threadIdx.x & 31;
   const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1655,6 +1658,7 @@ __global__ void __launch_bounds__(256) sparsity_penalty_kernel(const int* __rest
                                                                  float* __restrict__ grad_a, float* __restrict__ pen_coef,
                                                                  double* __restrict__ penalty_out) {
   if (chain_wait()) return;
+  chain_release();
   float local = 0.f;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncols; col += gridDim.x * blockDim.x) {
     const int b = feat_off[col], e = feat_off[col + 1];

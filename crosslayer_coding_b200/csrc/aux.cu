@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(1024) aux_compact_kernel(const long long* __re
                                                             int nd_cap, int* __restrict__ dead_cols, int* __restrict__ nd, int* __restrict__ nd_all,
                                                             int* __restrict__ extra_idx) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   const int l = blockIdx.x;
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(256) aux_gather_bias_kernel(const void* __rest
                                                                 const int* __restrict__ dead_cols, const int* __restrict__ nd, int nd_cap,
                                                                 float* __restrict__ bias_c) {
   if (chain_wait()) return;
+  chain_release();
   const int l = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nd_cap) return;
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(256) aux_gather_select_kernel(const t16* __res
                                                                   const int* __restrict__ nd_all, int nd_cap, int k_aux_max, int B,
                                                                   t16* __restrict__ A) {
   if (chain_wait()) return;
+  chain_release();
   extern __shared__ __align__(16) uint8_t aux_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tok = blockIdx.x * 8 + warp, l = blockIdx.y;
@@ -229,6 +232,7 @@ struct AuxRowsParams {
 __global__ void __launch_bounds__(256) aux_gather_rows_kernel(AuxRowsParams p, const int* __restrict__ dead_cols, const int* __restrict__ nd,
                                                                 int nd_cap, int d, t16* __restrict__ W0) {
   if (chain_wait()) return;
+  chain_release();
   const int l = blockIdx.y;
   const int vec = d / 8;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < 1LL * nd_cap * vec; i += 1LL * gridDim.x * blockDim.x) {
@@ -253,6 +257,7 @@ __global__ void __launch_bounds__(256) aux_residual_kernel(const float* __restri
                                                              const int* __restrict__ nd, const float* __restrict__ ctl, int L, int B, int d,
                                                              float factor, int scale_g) {
   if (chain_wait()) return;
+  chain_release();
   const int l = blockIdx.y;
   const bool live = nd[l] > 0;  // a layer without dead features has no auxiliary term
   const float scale = ctl != nullptr ? ctl[SC_LOSS_SCALE] : 1.f;
@@ -304,6 +309,7 @@ __global__ void __launch_bounds__(256) aux_residual_kernel(const float* __restri
 // buf *= 1 / loss scale (gradients that were formed from a scaled 16-bit factor)
 __global__ void __launch_bounds__(256) unscale_kernel(float* __restrict__ buf, long long n, const float* __restrict__ ctl) {
   if (chain_wait()) return;
+  chain_release();
   const float inv = ctl[SC_INV_SCALE];
   for (long long i = (blockIdx.x * 1LL * blockDim.x + threadIdx.x) * 4; i < n; i += 1LL * gridDim.x * blockDim.x * 4) {
     if (i + 4 <= n) {
@@ -319,6 +325,7 @@ __global__ void __launch_bounds__(256) unscale_kernel(float* __restrict__ buf, l
 // out[r] = sum of the 16-bit row r of in [rows, n]  (encoder-bias gradient of the dead features: row sums of G^T)
 __global__ void __launch_bounds__(256) rowsum16_kernel(const t16* __restrict__ in, float* __restrict__ out, long long rows, int n) {
   if (chain_wait()) return;
+  chain_release();
   const int lane = threadIdx.x & 31;
   const long long warp_global = (blockIdx.x * 1LL * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = (gridDim.x * 1LL * blockDim.x) >> 5;
@@ -341,6 +348,7 @@ __global__ void __launch_bounds__(256) scatter_add_rows_kernel(float* __restrict
                                                                  const float* __restrict__ src_bias, const int* __restrict__ extra_idx,
                                                                  long long n_dst_rows, int d) {
   if (chain_wait()) return;
+  chain_release();
   const int vec = d / 4;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n_dst_rows * vec; i += 1LL * gridDim.x * blockDim.x) {
     const long long row = i / vec;

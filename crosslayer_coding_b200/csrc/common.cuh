@@ -73,9 +73,13 @@ __device__ __forceinline__ bool clt_in_bounds(long long, long long, int*, int) {
 // move across statements that write memory.
 __device__ __forceinline__ bool chain_wait() {
   uint32_t sms;
-  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;\n\tmov.u32 %0, %%nsmid;" : "=r"(sms) :: "memory");
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%nsmid;" : "=r"(sms) :: "memory");
   return sms == 0xFFFFFFFFu;
 }
+// Lets the next kernel's CTAs take their places; second statement of a chained kernel.  Not in one that waits for another rank: up to 1184
+// CTAs would hold the threads of all SMs until that rank arrives, and kernels of other streams (staging of the next batch) could not start.  There
+// the next kernel comes when this one has ended.
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Params, typename... Args>
 inline cudaError_t launch_kernel(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchAttribute attr = {};

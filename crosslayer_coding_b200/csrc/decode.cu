@@ -277,6 +277,7 @@ __device__ __forceinline__ void walk_list(const DecodeParams& p, int t, int firs
 template <int NV, int TOK, int SPLIT, int R, int WARPS_PER_SM>
 __global__ void __launch_bounds__(32 * TOK * SPLIT, WARPS_PER_SM / (TOK * SPLIT)) decode_walk_kernel(const DecodeParams p) {
   if (chain_wait()) return;
+  chain_release();
   constexpr int kWarps = TOK * SPLIT;
   __shared__ __align__(16) float sums[kWarps][NV * 256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -342,6 +343,7 @@ __global__ void __launch_bounds__(32 * TOK * SPLIT, WARPS_PER_SM / (TOK * SPLIT)
 template <int NV, int SPLIT, int R, int WARPS_PER_SM>
 __global__ void __launch_bounds__(32 * SPLIT, WARPS_PER_SM / SPLIT) decode_running_kernel(const DecodeParams p) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ __align__(16) float sums[2][SPLIT][NV * 256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.d;
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(32 * SPLIT, WARPS_PER_SM / SPLIT) decode_runni
 constexpr int kLenClasses = 1024;
 __global__ void __launch_bounds__(kLenClasses) decode_order_kernel(const int* __restrict__ tok_off, int B, int* __restrict__ order) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ int place[kLenClasses];
   __shared__ int warp_sums[32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -472,6 +475,7 @@ __global__ void __launch_bounds__(256) recon_epilogue_kernel(const float* __rest
                                                                float* __restrict__ yhat_out, double* __restrict__ sq_err, int L, int B,
                                                                int d, int row0, int nrows, float* __restrict__ ctl) {
   if (chain_wait()) return;
+  chain_release();
   const int t = blockIdx.y;
   const float loss_scale = ctl != nullptr ? ctl[SC_LOSS_SCALE] : 1.f;
   bool bad = false;
@@ -525,6 +529,7 @@ __global__ void __launch_bounds__(256) recon_epilogue_kernel(const float* __rest
 __global__ void __launch_bounds__(1024) gs_colsum_kernel(const t16* __restrict__ gs, float* __restrict__ out, int B, int d,
                                                           int rows_per_block) {
   if (chain_wait()) return;
+  chain_release();
   const int t = blockIdx.z;
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
   const int r0 = blockIdx.y * rows_per_block, r1 = min(B, r0 + rows_per_block);
@@ -558,6 +563,7 @@ __global__ void __launch_bounds__(1024) gs_colsum_kernel(const t16* __restrict__
 // the threshold-gradient GEMM of source layer s needs the seed of all its targets added up).  fp32 accumulation.
 __global__ void __launch_bounds__(256) gs_suffix_sum_kernel(const t16* __restrict__ gs, t16* __restrict__ out, int L, long long per_layer) {
   if (chain_wait()) return;
+  chain_release();
   for (long long i = (blockIdx.x * 1LL * blockDim.x + threadIdx.x) * 8; i < per_layer; i += 1LL * gridDim.x * blockDim.x * 8) {
     float acc[8];
 #pragma unroll

@@ -238,6 +238,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 __global__ void __launch_bounds__(256) transpose16_kernel(const t16* __restrict__ in, t16* __restrict__ out, int R, int C, long long ld_in,
                                                             long long layer_stride_in) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ t16 tile[64][66];
   const int l = blockIdx.z;
   const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(256) transpose16_kernel(const t16* __restrict_
 __global__ void __launch_bounds__(256) transpose16_vec_kernel(const t16* __restrict__ in, const t16* __restrict__ mask, t16* __restrict__ out, int R,
                                                                 int C, long long ld_in, long long layer_stride_in) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ uint32_t tile[64][33];  // 64 rows x 64 elements, two per word
   const int l = blockIdx.z;
   const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
@@ -308,6 +310,7 @@ __global__ void __launch_bounds__(256) negative_indicator_kernel(const t16* __re
                                                                    double* __restrict__ loss, int B, int F, int F_valid, long long ld,
                                                                    float coef_over_numel) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ t16 tile[64][66];
   __shared__ float colsum[64];
   __shared__ float red[8];

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x
                                                          float* __restrict__ rstd, int B, int F, long long ld,
                                                          long long layer_stride, long long first_strip) {
   if (chain_wait()) return;
+  chain_release();
   using Ld = ColstatsLoad<VEC>;
   constexpr int kBlocks = 8 / VEC;  // of 32 * VEC columns in a strip
   constexpr int kDepth = Ld::kDepth;
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x
 __global__ void __launch_bounds__(256) colstats_from_tiles_kernel(const float* __restrict__ tile_stats, float* __restrict__ mean,
                                                                     float* __restrict__ rstd, int B, int F, int row_blocks, long long n) {
   if (chain_wait()) return;
+  chain_release();
   const long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int l = int(i / F), c = int(i - 1LL * l * F);
@@ -174,6 +176,7 @@ __global__ void __launch_bounds__(256) colstats_finalize_kernel(const t16* __res
                                                                   float* __restrict__ rstd, int B, int F, long long layer_stride,
                                                                   long long first, long long n) {
   if (chain_wait()) return;
+  chain_release();
   const long long i = first + blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int l = int(i / F), c = int(i - 1LL * l * F);
@@ -201,6 +204,7 @@ __global__ void __launch_bounds__(256) zhist_kernel(const t16* __restrict__ x, c
                                                       unsigned int* __restrict__ hist, const long long* __restrict__ ctl,
                                                       int only_if_retry) {
   if (chain_wait()) return;
+  chain_release();
   if (only_if_retry && ctl[CTL_RETRY] == 0) return;
   const float z_lo = key_lo == 0u ? -INFINITY : key_to_float(key_lo);
   __shared__ unsigned int sh[kHistBins];
@@ -278,6 +282,7 @@ __global__ void __launch_bounds__(256) zhist_collect_kernel(const t16* __restric
                                                               const long long* __restrict__ sel_state,
                                                               unsigned int* __restrict__ hist, Pool pool) {
   if (chain_wait()) return;
+  chain_release();
   const uint32_t key_lo = uint32_t(sel_state[0]);
   const int shift = int(sel_state[1]);
   const float z_lo = key_to_float(key_lo);
@@ -422,6 +427,7 @@ __global__ void __launch_bounds__(1024) find_bin_kernel(const unsigned int* __re
                                                           const unsigned int* __restrict__ pool_count, long long pool_cap,
                                                           int* __restrict__ status) {
   if (chain_wait()) return;
+  if (ex.world <= 1) chain_release();  // else it waits for the other ranks below
   __shared__ uint32_t vals[kHistBins + kHistExtra];
   __shared__ unsigned long long part[1024];
   __shared__ int timeout;
@@ -538,6 +544,7 @@ __global__ void __launch_bounds__(256) threshold_collect_kernel(const t16* __res
                                                                   ScanGeom g, int col_pitch, long long* __restrict__ ctl,
                                                                   Lists o, int* __restrict__ status) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ uint32_t s_queue[4 * kHitQueue];
   __shared__ int s_tok[2 * kPoolStage];
   __shared__ int s_col[2 * kPoolStage];
@@ -664,6 +671,7 @@ __global__ void __launch_bounds__(256) token_topk_kernel(const t16* __restrict__
                                                            const float* __restrict__ rstd, ScanGeom g, int col_pitch, int f_valid, int k,
                                                            long long* __restrict__ ctl, Lists o, int* __restrict__ status, int only_marked) {
   if (chain_wait()) return;
+  chain_release();
   extern __shared__ uint8_t tk_smem[];
   TokenTopkShared* sh = reinterpret_cast<TokenTopkShared*>(tk_smem);
   const int tok0 = blockIdx.x * kTokPerCta;
@@ -797,6 +805,7 @@ template <int TPC>
 __global__ void __launch_bounds__(kTkThreads) token_topk_list_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd,
                                                                      ScanGeom g, int col_pitch, int f_valid, int k, int step, long long* __restrict__ ctl, Lists o) {
   if (chain_wait()) return;
+  chain_release();
   extern __shared__ __align__(16) uint8_t tl_smem[];
   TokenListShared<TPC>* sh = reinterpret_cast<TokenListShared<TPC>*>(tl_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -919,6 +928,7 @@ __device__ __forceinline__ float t16_of(const uint4& v, int j) {
 __global__ void __launch_bounds__(256) token_sample_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
                                                              int f_valid, WideTopk wt) {
   if (chain_wait()) return;
+  chain_release();
   const int sg = blockIdx.x * 256 + threadIdx.x;  // < ng, a multiple of 256
   const int q = (sg >> 5) * 32 * kWideStep + (sg & 31);  // runs of 32 groups: short enough that a sample meets every layer
   const int r0 = blockIdx.y * kWideRows, r1 = min(g.B, r0 + kWideRows);
@@ -950,6 +960,7 @@ __global__ void __launch_bounds__(256) token_sample_kernel(const t16* __restrict
 
 __global__ void __launch_bounds__(256) token_bound_kernel(WideTopk wt, int k, long long* __restrict__ ctl, long long n_entries) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ int total[2];
   const int tok = blockIdx.x;
   if (tok == 0 && threadIdx.x == 0) ctl[CTL_NUM_ENTRIES] = n_entries;
@@ -982,6 +993,7 @@ __global__ void __launch_bounds__(256) token_bound_kernel(WideTopk wt, int k, lo
 __global__ void __launch_bounds__(256, 4) token_collect_kernel(const t16* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, ScanGeom g,
                                                               int col_pitch, int f_valid, WideTopk wt) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ uint16_t queue[kWideQueue];
   __shared__ float z_scaled[kWideRows];
   __shared__ uint32_t bound[kWideRows];
@@ -1074,6 +1086,7 @@ __global__ void __launch_bounds__(256, 4) token_collect_kernel(const t16* __rest
 template <int W>
 __global__ void __launch_bounds__(128) token_cut_kernel(const t16* __restrict__ x, ScanGeom g, int col_pitch, int k, WideTopk wt, Lists o) {
   if (chain_wait()) return;
+  chain_release();
   const int tok = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (tok >= g.B) return;
   const int n = wt.n[tok];
@@ -1121,6 +1134,7 @@ constexpr int kClassifyInFlight = 4;
 __global__ void __launch_bounds__(256) classify_pool_kernel(Pool pool, long long* __restrict__ ctl, Lists o,
                                                               int* __restrict__ status) {
   if (chain_wait()) return;
+  chain_release();
   if (ctl[CTL_RETRY] != 0) return;
   const uint32_t tbin = uint32_t(ctl[CTL_BIN]);
   const uint32_t key_lo = uint32_t(ctl[CTL_KEY_LO]);
@@ -1205,6 +1219,7 @@ __global__ void __launch_bounds__(256) compact_kernel(const t16* __restrict__ x,
                                                         long long* __restrict__ ctl, Lists o, int* __restrict__ status,
                                                         int only_if_retry) {
   if (chain_wait()) return;
+  chain_release();
   if (only_if_retry && ctl[CTL_RETRY] == 0) return;
   __shared__ int s_tok[kStageCap];
   __shared__ int s_col[kStageCap];
@@ -1341,6 +1356,7 @@ __global__ void __launch_bounds__(1024) refine_kernel(const uint32_t* __restrict
                                                         FlatGeom fg, long long* __restrict__ ctl, Exchange ex,
                                                         int* __restrict__ status) {
   if (chain_wait()) return;
+  if (ex.world <= 1) chain_release();  // else it waits for the other ranks below
   const int shift = int(ctl[CTL_SHIFT]);
   const uint32_t key_lo = uint32_t(ctl[CTL_KEY_LO]);  // bins are over (key - key_lo): refine on the same offset
   __shared__ uint32_t hist[kRefineBins];
@@ -1514,6 +1530,7 @@ __global__ void __launch_bounds__(1024) refine_kernel(const uint32_t* __restrict
 __global__ void __launch_bounds__(256) finalize_kernel(Lists o, FlatGeom fg, long long* __restrict__ ctl,
                                                          int* __restrict__ status) {
   if (chain_wait()) return;
+  chain_release();
   const int shift = int(ctl[CTL_SHIFT]);
   const uint32_t key_lo = uint32_t(ctl[CTL_KEY_LO]);
   long long n = ctl[CTL_NUM_CAND];
@@ -1545,6 +1562,7 @@ __global__ void __launch_bounds__(256) csr_count_kernel(const int* __restrict__ 
                                                           int* __restrict__ feat_cnt, unsigned char* __restrict__ fired,
                                                           int num_tokens, int num_cols) {
   if (chain_wait()) return;
+  chain_release();
   long long n = ctl[CTL_NUM_ENTRIES];
   if (n > cap) n = cap;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
@@ -1564,6 +1582,7 @@ __global__ void __launch_bounds__(256) csr_count_kernel(const int* __restrict__ 
 __global__ void __launch_bounds__(1024) exclusive_scan_kernel(const int* __restrict__ in, int* __restrict__ out,
                                                                 int* __restrict__ cursor, int n) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1622,6 +1641,7 @@ struct ScanJob {
 };
 __global__ void __launch_bounds__(1024) exclusive_scan_tiles_kernel(ScanJob ja, ScanJob jb, int tiles_a) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ int warp_tot[32];
   __shared__ int carry_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1707,6 +1727,7 @@ __global__ void __launch_bounds__(256) csr_scatter_kernel(const int* __restrict_
                                                             float* __restrict__ fcsr_val, int col_pitch, int num_tokens, int num_cols,
                                                             const int* __restrict__ feat_off, int* __restrict__ layer_cnt) {
   if (chain_wait()) return;
+  chain_release();
   if (layer_cnt != nullptr && blockIdx.x == 0) {  // entries per layer: the offsets are complete
     for (int l = threadIdx.x; 1LL * l * col_pitch < num_cols; l += blockDim.x)
       layer_cnt[l] = feat_off[min(1LL * (l + 1) * col_pitch, 1LL * num_cols)] - feat_off[1LL * l * col_pitch];
@@ -1731,6 +1752,7 @@ __global__ void __launch_bounds__(256) csr_token_count_kernel(const int* __restr
                                                                 const long long* __restrict__ ctl, int* __restrict__ tok_cnt, int* __restrict__ layer_cnt,
                                                                 int col_pitch, int num_tokens, int num_cols) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ int per_layer[32];
   const int lane = threadIdx.x & 31;
   if (threadIdx.x < 32) per_layer[threadIdx.x] = 0;
@@ -1755,6 +1777,7 @@ __global__ void __launch_bounds__(256) csr_token_scatter_kernel(const int* __res
                                                                   int* __restrict__ tok_cursor, int* __restrict__ tcsr_col, float* __restrict__ tcsr_val,
                                                                   int col_pitch, int num_tokens, int num_cols) {
   if (chain_wait()) return;
+  chain_release();
   long long n = ctl[CTL_NUM_ENTRIES];
   if (n > cap) n = cap;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
@@ -1812,6 +1835,7 @@ constexpr int kFeatSortCap = 4096;
 __global__ void __launch_bounds__(256) csr_sort_feature_segments_kernel(const int* __restrict__ off, int nseg, int per_cta,
                                                                           int* __restrict__ key, float* __restrict__ val) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ unsigned long long w[kFeatSortCap];
   __shared__ int long_list[256];
   __shared__ int long_count;
@@ -1977,6 +2001,7 @@ __device__ __forceinline__ bool bucket_sort_segment(int* __restrict__ key, float
 __global__ void __launch_bounds__(256) csr_sort_token_segments_kernel(const int* __restrict__ off, int* __restrict__ key, float* __restrict__ val, int rank_up_to,
                                                                          int bucket_up_to) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ __align__(16) unsigned long long w[(kTokenBucketRoom + kTokenSortCap) / 2];
   __shared__ int count[kTokenBuckets], base[kTokenBuckets], start[kTokenBuckets];
   const int b = off[blockIdx.x], n = off[blockIdx.x + 1] - b;
@@ -2011,6 +2036,7 @@ static void launch_token_sort(const int* off, int* key, float* val, int num_toke
 // Dead-feature counters: +1 per step, reset where the feature fired (reference trainer.py:693-712).
 __global__ void __launch_bounds__(256) dead_counter_kernel(long long* __restrict__ counter, unsigned char* __restrict__ fired, int n) {
   if (chain_wait()) return;
+  chain_release();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     counter[i] = fired[i] ? 0 : counter[i] + 1;
     fired[i] = 0;
@@ -2309,6 +2335,7 @@ struct CltTopkTpArgs {
 
 __global__ void __launch_bounds__(256) token_topk_push_kernel(CltTopkTpArgs a) {
   if (chain_wait()) return;
+  chain_release();
   if (blockIdx.x == 0 && threadIdx.x == 0) a.ctl[CTL_NUM_ENTRIES] = 0;  // refilled by the filter pass
   const long long n = 1LL * a.B * a.k;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
@@ -2327,6 +2354,7 @@ __global__ void __launch_bounds__(256) token_topk_push_kernel(CltTopkTpArgs a) {
 // One CTA per owned token; dynamic shared memory world * k keys.
 __global__ void __launch_bounds__(256) token_topk_cut_kernel(CltTopkTpArgs a) {
   if (chain_wait()) return;
+  chain_release();
   extern __shared__ unsigned long long tk_keys[];
   const int lt = blockIdx.x;
   const int t = a.rank * a.rows_per_rank + lt;
@@ -2352,6 +2380,7 @@ __global__ void __launch_bounds__(256) token_topk_cut_kernel(CltTopkTpArgs a) {
 // One warp per token: candidates at or above the cut are appended to the entry list.
 __global__ void __launch_bounds__(256) token_topk_filter_kernel(CltTopkTpArgs a) {
   if (chain_wait()) return;
+  chain_release();
   const int lane = threadIdx.x & 31;
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= a.B) return;

@@ -69,6 +69,7 @@ struct StepControlParams {
 
 __global__ void __launch_bounds__(64) step_control_kernel(const StepControlParams p) {
   if (chain_wait()) return;
+  if (p.ex.world <= 1) chain_release();  // else it waits for the other ranks below
   __shared__ double vals[kCtlMaxLayers + kMaxScalars + 2];
   __shared__ int timeout;
   const int tid = threadIdx.x;
@@ -152,6 +153,7 @@ __global__ void __launch_bounds__(256) decoder_bias_adam_kernel(WT* __restrict__
                                                                   const float* __restrict__ extra, int n_bias, int L, int d,
                                                                   AdamHyperS h, float* __restrict__ ctl, float norm_weight) {
   if (chain_wait()) return;
+  chain_release();
   const StepScales sc = read_step_ctl(ctl);
   if (sc.skip) return;
   const long long n = 1LL * n_bias * d;
@@ -193,6 +195,7 @@ __global__ void __launch_bounds__(256) step_finish_kernel(long long* __restrict_
                                                             const WT* __restrict__ bias, const float* __restrict__ sel,
                                                             float* __restrict__ bias_sum, int n_bias, int L, int d) {
   if (chain_wait()) return;
+  chain_release();
   const long long stride = 1LL * gridDim.x * blockDim.x;
   const long long tid = blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   if (counter != nullptr)
@@ -263,6 +266,7 @@ struct ThetaAdamParams {
 template <typename WT>
 __global__ void __launch_bounds__(256) theta_adam_kernel(const ThetaAdamParams p) {
   if (chain_wait()) return;
+  chain_release();
   const StepScales sc = read_step_ctl(p.ctl);
   if (sc.skip) return;
   const long long n = 1LL * p.L * p.pitch;
@@ -322,6 +326,7 @@ __global__ void __launch_bounds__(256) theta_accumulate_kernel(const int* __rest
                                                                  int width, float eps, float* __restrict__ sum_min, float* __restrict__ cnt_min,
                                                                  float* __restrict__ mean_acc, float* __restrict__ std_acc, float* __restrict__ batches) {
   if (chain_wait()) return;
+  chain_release();
   const long long n = 1LL * L * pitch;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x) {
     const int l = int(i / pitch), f = int(i - 1LL * l * pitch);
@@ -372,6 +377,7 @@ template <typename IT>
 __global__ void __launch_bounds__(256) normalize_cast_kernel(const IT* __restrict__ in, t16* __restrict__ out, const float* __restrict__ mean,
                                                                const float* __restrict__ inv_std, long long rows, int rows_per_stat, int d, float mul) {
   if (chain_wait()) return;
+  chain_release();
   const int vec_per_row = d / 8;
   const long long nvec = rows * vec_per_row;
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < nvec; i += 1LL * gridDim.x * blockDim.x) {
@@ -402,6 +408,7 @@ __global__ void __launch_bounds__(256) scale_histogram_kernel(const t16* __restr
                                                                 const float* __restrict__ scales, int n_scales,
                                                                 unsigned long long* __restrict__ hist, int B, int F, long long ld) {
   if (chain_wait()) return;
+  chain_release();
   __shared__ float sc[kMaxScales];
   __shared__ unsigned int sh[kMaxScales + 1];
   for (int i = threadIdx.x; i < n_scales; i += blockDim.x) sc[i] = scales[i];
@@ -429,6 +436,7 @@ __global__ void __launch_bounds__(256) scale_histogram_kernel(const t16* __restr
 template <typename WT>
 __global__ void __launch_bounds__(256) theta_exp_kernel(const WT* __restrict__ log_theta, float* __restrict__ theta, long long n) {
   if (chain_wait()) return;
+  chain_release();
   for (long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x; i < n; i += 1LL * gridDim.x * blockDim.x)
     theta[i] = __expf(load_w<WT>(log_theta + i));
 }
