@@ -18,6 +18,8 @@
 // buffers by the kernels below with bounded flag waits.
 #include "common.cuh"
 
+#include <type_traits>
+
 namespace clt {
 
 constexpr int kHistBins = 8192;
@@ -104,16 +106,16 @@ __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x
     const typename Ld::T v0 = *reinterpret_cast<const typename Ld::T*>(base);
 #pragma unroll
     for (int j = 0; j < VEC / 2; ++j) { shift[2 * j] = t16_lo(Ld::word(v0, j)); shift[2 * j + 1] = t16_hi(Ld::word(v0, j)); }
-    for (int r0 = row_lo + threadIdx.y; r0 < row_hi; r0 += 8 * kDepth) {
+    // kDepth independent loads in flight; only the last batch tests its rows
+    const auto batch = [&](int r0, auto last) {
+      constexpr bool kLast = decltype(last)::value;
       typename Ld::T v[kDepth];
 #pragma unroll
-      for (int k = 0; k < kDepth; ++k) {  // independent loads in flight
-        const int r = r0 + 8 * k;
-        v[k] = r < row_hi ? __ldcs(reinterpret_cast<const typename Ld::T*>(base + 1LL * r * ld)) : v0;
-      }
+      for (int k = 0; k < kDepth; ++k)
+        v[k] = !kLast || r0 + 8 * k < row_hi ? __ldcs(reinterpret_cast<const typename Ld::T*>(base + 1LL * (r0 + 8 * k) * ld)) : v0;
 #pragma unroll
       for (int k = 0; k < kDepth; ++k) {
-        if (r0 + 8 * k >= row_hi) break;
+        if (kLast && r0 + 8 * k >= row_hi) break;
 #pragma unroll
         for (int j = 0; j < VEC / 2; ++j) {
           const uint32_t u = Ld::word(v[k], j);
@@ -122,7 +124,10 @@ __global__ void __launch_bounds__(256) colstats_kernel(const t16* __restrict__ x
           s[2 * j + 1] += b; q[2 * j + 1] += b * b;
         }
       }
-    }
+    };
+    int r0 = row_lo + threadIdx.y;
+    for (; r0 + 8 * (kDepth - 1) < row_hi; r0 += 8 * kDepth) batch(r0, std::false_type{});
+    if (r0 < row_hi) batch(r0, std::true_type{});
   }
 #pragma unroll
   for (int j = 0; j < VEC; ++j) { red[threadIdx.y][threadIdx.x][j] = s[j]; red[threadIdx.y][threadIdx.x][VEC + j] = q[j]; }
