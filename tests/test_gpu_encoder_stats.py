@@ -69,3 +69,31 @@ def test_encoder_gemm_stats_refuses_other_shapes(ext):
         ext.encoder_gemm_stats(x, w, None, out, m, torch.zeros(1, 128, device=dev), st)
     with pytest.raises(RuntimeError, match="dtype"):
         ext.encoder_gemm_stats(x, w, None, out, m.double(), m, st)
+
+
+# few strips with many rows, whose tiles would go one after the other on a part of the chip while the rest of it stood idle: no strip is taken whole.  A full
+# round of strips and a few more: the few are not.  Rounds that are nearly full: all of them are.
+@pytest.mark.parametrize("L,M,N,K,way", [(2, 4100, 2056, 72, "none"), (1, 8192, 2048, 64, "none"), (79, 4100, 256, 8, "full rounds"), (297, 3000, 256, 8, "full rounds"), (3, 4096, 5120, 64, "all")])
+def test_encoder_gemm_stats_of_few_strips(ext, L, M, N, K, way):
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(M + N)
+    x = torch.randn(L, M, K, device=dev, generator=g).bfloat16()
+    w = (torch.randn(L, N, K, device=dev, generator=g) / math.sqrt(K)).bfloat16()
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    plain, out = (torch.full((L, M, N), float("nan"), device=dev, dtype=torch.bfloat16) for _ in range(2))
+    mean, rstd = (torch.full((L, N), float("nan"), device=dev) for _ in range(2))
+    kernels = ext.encoder_gemm_stats(x, w, None, out, mean, rstd, status)
+    ext.encoder_gemm(x, w, None, plain, status, None)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0 and kernels == (1 if way == "all" else 3)  # the pass over the others: sums of row chunks, conversion
+    assert torch.equal(out.view(torch.int16), plain.view(torch.int16))
+    if _row_chunks(L, M, N) <= 2:
+        mean_p, rstd_p = torch.empty_like(mean), torch.empty_like(rstd)
+        ext.colstats(plain, mean_p, rstd_p)
+        assert torch.equal(mean, mean_p) and torch.equal(rstd, rstd_p)
+    of = out.double()
+    spread = (of - of[:, :1]).abs().amax(1)
+    eps = (M + 16) * 2.0 ** -24  # as above
+    assert ((mean.double() - of.mean(1)).abs() <= eps * spread + 2.0 ** -23 * of.mean(1).abs()).all()
+    var = of.var(1)
+    assert (((1 / rstd.double() - 1e-6).square() - var).abs() <= 4 * eps * spread.square() + 2.0 ** -20 * var + 1e-12).all()
