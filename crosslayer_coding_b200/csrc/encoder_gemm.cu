@@ -748,25 +748,25 @@ static int rows_per_chunk(int L, int B, int F) {
 // How many strips of 256 features the pairs take whole, with the statistics: all of them, in ceil(strips / pairs) rounds, the last of which
 // may leave pairs idle; full rounds only, the rest tile by tile over all pairs with a separate pass for its statistics; or none, with a pass over
 // everything.  Estimates in us, fitted to 4 to 600 strips of 256 to 8192 rows with K = 64 to 2048, taken all three ways (the choice is
-// within 5 % of the best for all but a dozen of 1150 shapes, and at most 5 % behind the third, with K = 2048):
-//  * a tile of a whole strip takes a pair 1.5 + 0.0053 K, 0.0046 K in a round that is not full (clocks are higher then), at least the 3.2 of its
-//    epilogue; a tile without sums 0.85 + 0.005 K, at least 2.1;
-//  * a pass takes 10 (clears, sums, conversion; 7 where the rows are one chunk) and 0.024 per tile, or 0.038 with two columns per thread, as behind
-//    whole strips, and 0.0035 or 0.012 for each row of a chunk, which one thread waits for in turn.
+// within 5 % of the best for all but 16 of 1150 shapes, and 2 to 9 % behind the third for four, with K = 2048):
+//  * a tile of a whole strip takes a pair 1.2 + 0.0057 K, 0.0048 K in a round that is not full (clocks are higher then), at least the 3.4 of its
+//    epilogue; a tile without sums 1.2 + 0.005 K, at least 2.5;
+//  * a pass takes 10 (clears, sums, conversion) and 0.024 per tile, or 0.047 with two columns per thread, as behind whole strips, and 0.003 or
+//    0.007 for each row of a chunk, which one thread waits for in turn.
 // 16 strips of 8192 rows, K = 64: whole 100 us, none 46; 32, K = 768: 146 and 106; 64 of 4096, K = 768: 84 and 104; 130, K = 2048: whole 383, full
 // rounds only 452, none 415; 80 of 8192, K = 2048: 739, 484 and 508; 96: 793, 669 and 636.
-static long long whole_strips(long long strips, int npairs, int tiles_m, int K, int rows_per_fold, bool chunks) {
+static long long whole_strips(long long strips, int npairs, int tiles_m, int K, int rows_per_fold) {
   const long long full = strips / npairs * npairs, tail = (strips - full) * tiles_m;
   if (tail == 0) return strips;
   const auto at_least = [](double least, double t) { return t < least ? least : t; };
-  const double rounds = at_least(3.2, 1.5 + 0.0053 * K) * double(full / npairs) * tiles_m;
-  const double plain_tile = at_least(2.1, 0.85 + 0.005 * K), pass = chunks ? 10.0 : 7.0;
+  const double rounds = at_least(3.4, 1.2 + 0.0057 * K) * double(full / npairs) * tiles_m;
+  const double plain_tile = at_least(2.5, 1.2 + 0.005 * K);
   const auto plain = [&](long long tiles) { return plain_tile * double((tiles + npairs - 1) / npairs); };
-  const double all = rounds + at_least(3.2, 1.5 + 0.0046 * K) * tiles_m;
-  const double split = rounds + plain(tail) + pass + 0.038 * double(tail) + 0.012 * rows_per_fold;
-  const double none = plain(strips * tiles_m) + pass + 0.024 * double(strips * tiles_m) + 0.0035 * rows_per_fold;
+  const double all = rounds + at_least(3.4, 1.2 + 0.0048 * K) * tiles_m;
+  const double split = rounds + plain(tail) + 10.0 + 0.047 * double(tail) + 0.007 * rows_per_fold;
+  const double none = plain(strips * tiles_m) + 10.0 + 0.024 * double(strips * tiles_m) + 0.003 * rows_per_fold;
   const double other = split < none ? split : none;
-  return all <= 1.03 * other ? strips : split < none ? full : 0;
+  return all <= 1.01 * other ? strips : split < none ? full : 0;
 }
 
 template <bool STATS>
@@ -804,7 +804,7 @@ static int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, const
   const long long strips = 1LL * L * ((N + 2 * gemm2::BF - 1) / (2 * gemm2::BF));
   const int npairs = int(strips * tiles_m < pair_clusters ? strips * tiles_m : pair_clusters);
   const int rows_per_fold = STATS ? rows_per_chunk(L, M, N) : 0;
-  *whole = STATS ? whole_strips(strips, npairs, tiles_m, K, rows_per_fold, rows_per_fold < M) : 0;
+  *whole = STATS ? whole_strips(strips, npairs, tiles_m, K, rows_per_fold) : 0;
   if constexpr (STATS) {
     if (*whole == 0) return launch_pair<false>(map_w, map_x, map_c, bias, L, M, N, K, status, nullptr, nullptr, whole, num_sms, stream);
   }
