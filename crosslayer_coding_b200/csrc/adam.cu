@@ -1020,7 +1020,8 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
 // A row's stage is refilled in the next row's turn, behind the requests for its seed rows, when the store has long read it: waiting for
 // the store at the end of the row, and a test per block of 128 although only the last can be short, cost 3 to 7 % (6 x 32768 x 512 with 4 entries
 // per row 677 -> 655 us, per-target decoders 230 -> 213, 8 x 8192 x 256 untied 358 -> 344).  Rows of up to 128 elements are over too
-// soon for that (277 us, refilled late 283): they wait for the store.  Per-target encoder rows with two entries lose 1 to 2 % (177 -> 179).
+// soon for that (277 us, refilled late 283): they wait for the store.  With few entries wide rows of this form ask for more than DRAM takes; the
+// launcher then lets fewer CTAs work.
 template <int NC>
 __device__ __forceinline__ void load_seed_row(const t16* row, int lane, int d, uint2 (&q)[NC]) {
 #pragma unroll
@@ -1044,14 +1045,24 @@ struct RowAt {
 };
 
 template <bool SR, int NC, bool PT>
-__global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_rows_adam_kernel(const DecAdamParams p, long long total_rows, int* status) {
+__global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC))
+narrow_rows_adam_kernel(const DecAdamParams p, long long total_rows, float ctas_empty, float ctas_per_entry, int* status) {
   static_assert(kNarrowStages == 2, "the late refill is for the next row");
   constexpr bool kRefillLate = NC > 1;
   extern __shared__ __align__(128) uint8_t smem_narrow[];
   __shared__ uint64_t full_s[kNarrowWarps][kNarrowStages];
   __shared__ int abort_s;
+  const int n_entries = NC >= 3 ? __ldg(p.feat_off + p.L * p.F_pitch) : 0;
   const StepScales sc = read_step_ctl(p.ctl);
   if (sc.skip) return;  // the whole grid sees the same flag: a skipped step touches nothing
+  int grid = int(gridDim.x);
+  if (NC >= 3) {  // of the resident CTAs, as many as keep DRAM busy with these lists
+    float per_row = float(n_entries) / float(p.L * p.F_pitch);
+    if (PT) per_row *= 0.5f * float(p.L + 1);  // an entry is in the rows of all later targets
+    const float enough = ctas_empty + ctas_per_entry * per_row;
+    if (enough < 0.93f * float(grid)) grid = int(enough);
+    if (int(blockIdx.x) >= grid) return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.d, Fp = p.F_pitch;
   const uint32_t w_bytes = uint32_t(d) * 2u, mv_bytes = uint32_t(d) * 4u, stage_bytes = w_bytes + 2u * mv_bytes;
@@ -1068,7 +1079,7 @@ __global__ void __launch_bounds__(32 * kNarrowWarps, narrow_ctas(NC)) narrow_row
   const float gsc = hr.gscale * (p.use_inv_scale ? sc.inv_scale : 1.f);
   const uint64_t pol_stream = l2_policy_evict_first();  // rows are touched once per step
 
-  const long long stride = 1LL * gridDim.x * kNarrowWarps;
+  const long long stride = 1LL * grid * kNarrowWarps;
   const auto place = [&](RowAt& at) {  // tensor, feature and row of at.idx (at.ti: at or before the right one)
     if (at.idx >= total_rows) return;
     while (at.idx >= p.row_start[at.ti + 1]) ++at.ti;
@@ -1748,6 +1759,16 @@ constexpr int kNarrowMaxWidth = 512;
 static int launch_narrow_rows(const DecAdamParams& p, bool sr, int num_sms, int* status, cudaStream_t st, bool per_target) {
   const long long total = p.row_start[p.ntensors];
   const size_t smem = size_t(kNarrowWarps) * kNarrowStages * p.d * 10;
+  // Rows above 256 elements with few entries leave more requests in flight than DRAM takes, and then it falls behind its own rate (one row of 512 per
+  // feature, 0.6 entries each: 530 us with 16 warps per SM, 457 with 12; 2.6 entries: 476 and 506).  So many warps run as 6.55 TB/s need and 5 %
+  // more, or all when that is nearly all of them: a warp takes 2.3 us for a row of up to 384 elements, 1.35 + 0.00258 d for a longer one, and 0.23 for
+  // each of its entries (2.17 + 0.00125 d and 0.25 with the lists of several layers); a row moves 20 d bytes.  The kernel knows how many entries
+  // there are, the host often only a bound.  us with all warps / with the rule (and of the form before two-wide arithmetic and late refills), rows of
+  // 512, one per feature, by entries: 0.6 535 / 499 (548), 1 543 / 486 (542), 1.6 530 / 481 (471), 2 524 / 475 (474), 2.6 482 / 476 (492); of 448, 1
+  // entry: 525 / 484 (484); of 384, six to one per feature, 0.6: 498 / 469 (472); per target, 0.1 per row: of 512 538 / 478 (538).
+  const float ctas_per_us = 1.05f * 6.55e6f / float(20 * p.d * kNarrowWarps);
+  const float row_us = per_target ? 2.17f + 0.00125f * float(p.d) : p.d <= 384 ? 2.3f : 1.35f + 0.00258f * float(p.d);
+  const float ctas_empty = ctas_per_us * row_us, ctas_per_entry = ctas_per_us * (per_target ? 0.25f : 0.23f);
   auto launch = [&](auto kern) -> int {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
     int per_sm = 0;
@@ -1755,7 +1776,7 @@ static int launch_narrow_rows(const DecAdamParams& p, bool sr, int num_sms, int*
     long long grid = 1LL * num_sms * per_sm;
     const long long ctas = (total + kNarrowWarps - 1) / kNarrowWarps;
     if (grid > ctas) grid = ctas;
-    launch_alone(kern, int(grid), 32 * kNarrowWarps, smem, st, p, total, status);
+    launch_alone(kern, int(grid), 32 * kNarrowWarps, smem, st, p, total, ctas_empty, ctas_per_entry, status);
     return 0;
   };
   auto pick = [&](auto srv, auto ptv) -> int {

@@ -871,6 +871,14 @@ def test_decoder_row_update_one_warp_per_row(ext, tying, single, d, opts):
     _row_update(ext, 3, 90, d, tying, counts, rows_of=(lambda s: 1) if single else None, **opts)
 
 
+# rows of more than 256 elements: as many of the resident CTAs as the lists need, from almost empty ones to more than need all of them
+@pytest.mark.parametrize("tying,single", [(0, False), (0, True), (2, True)])
+@pytest.mark.parametrize("d", [264, 384, 512])
+@pytest.mark.parametrize("more", [[0, 0, 0], [2, 1, 2], [7, 5, 9]])
+def test_decoder_row_update_by_the_length_of_the_lists(ext, tying, single, d, more):
+    _row_update(ext, 2, 90, d, tying, COUNTS + more * 700, rows_of=(lambda s: 1) if single else None)
+
+
 # what the engine adds to the sweep: loss scale and clip coefficient from the control block, compact extra rows, stochastic rounding
 @pytest.mark.parametrize("tying,d", [(0, 264), (2, 200), (2, 264), (2, 1032)])
 @pytest.mark.parametrize("opts", [dict(ctl=True), dict(extra=True), dict(seed=1234), dict(ctl=True, extra=True, dtype=torch.float16)])
