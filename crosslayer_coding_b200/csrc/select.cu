@@ -18,6 +18,8 @@
 // buffers by the kernels below with bounded flag waits.
 #include "common.cuh"
 
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 namespace clt {
@@ -2171,24 +2173,48 @@ static FlatGeom flat_geom(const CltSelectArgs* a) {
   return fg;
 }
 
+// Rows per CTA, 64 to begin with.  With more than one kept element in 256 half as many in the passes without a tracked range (one in five: 1041 us, 1312 with
+// 64 of 100000 tokens x 264; 16 x 300 x 1024: 281, 493).
+static int rows_halved(const CltSelectArgs* a, int rows) {  // the grid's second dimension has its limit
+  return rows > 8 && (a->B + rows / 2 - 1) / (rows / 2) <= 65535 ? rows / 2 : rows;
+}
+static bool densely_kept(const CltSelectArgs* a) { return 256 * a->k_total > 1LL * a->B * a->L * a->full_F; }
+
+// The collecting pass: its queue holds 2048 pieces of eight elements, of 16384 in 64 rows of 2048 columns, and must not overflow while the cut moves: every
+// overflow costs the full-range passes (evaluation of 13 x 2536 features, 1504 tokens, k = 245: 677 us with them, 354 without).  A tracked range
+// holds 1.75 k elements; rows are halved until, spread evenly, the pieces with one of them fill at most 0.35 of the queue (eight rows cannot overflow
+// it), and once for densely kept elements where 64 rows make fewer than eight CTAs per SM.  us by rows per CTA (64, 32, 16, 8; + with full-range
+// passes), 6 x 4096 tokens x 2048: one in 400 69 71 72 82; 250 91 81 80 87; 150 317+ 101 92 98; 90 484+ 157 111 113; 60 642+ 799+ 174 131; 30 836+ 726+
+// 1119+ 252; 8 1801+ 1494+ 1814+ 882.
+static int collect_rows(const CltSelectArgs* a) {
+  const double q = kPoolFactor * double(a->k_total) / (double(a->B) * a->L * a->full_F);  // share of the elements
+  const int pieces = (a->F + 7) / 8;
+  const double per_row = (1.0 - std::pow(1.0 - std::min(q, 1.0), 8.0)) * std::min(pieces, 256);
+  int rows = 64;
+  if (densely_kept(a) && 1LL * ((pieces + 255) / 256) * ((a->B + 63) / 64) * a->L < 8 * 148) rows = rows_halved(a, rows);
+  while (rows * per_row > 0.35 * kCollectQueue && rows_halved(a, rows) < rows) rows = rows_halved(a, rows);
+  return rows;
+}
+
 // Steps 2-6.  `exa` may be null (single rank).  The histogram first covers keys >= key_lo only (the
 // caller's guess of where the cut lies); if the cut is not inside, a full-range pass repeats it.
 // `hist` holds two histograms of 8192 counters, zeroed by the caller.
 extern "C" int CLT_FN(clt_batchtopk_select)(const CltSelectArgs* a, const CltExchangeArgs* exa, cudaStream_t st) {
   if (a->ld % 8 != 0 || a->layer_stride % 8 != 0 || a->stat_pitch % 4 != 0 || a->F > a->ld) return -1;
   ScanGeom g = scan_geom(a);
-  // Kept densely, half the rows per CTA: a tracked range holds 1.75 k elements, so that of the 16384 pieces of 64 rows 900 may hold one at one kept
-  // element in 256 and 1800 at one in 128, and the queue (2048) must not overflow while the cut moves: every overflow costs the
-  // full-range passes (evaluation of 13 x 2536 features, 1504 tokens, k = 245: 677 us with them, 354 without; 4 x 4096, 4096 tokens, k = 120: 807, 397).
-  if (256 * a->k_total > 1LL * a->B * a->L * a->full_F) g.rows_per_block = 32;
+  const bool tracked = a->sel_state != nullptr && a->key_lo != 0;
+  if (!tracked && densely_kept(a)) g.rows_per_block = rows_halved(a, g.rows_per_block);
   const Exchange ex = to_exchange(exa);
-  dim3 grid(((a->F + 7) / 8 + 255) / 256, (a->B + g.rows_per_block - 1) / g.rows_per_block, a->L);
+  const auto grid_of = [&](const ScanGeom& s) { return dim3(((a->F + 7) / 8 + 255) / 256, (a->B + s.rows_per_block - 1) / s.rows_per_block, a->L); };
+  const dim3 grid = grid_of(g);
   const t16* x = static_cast<const t16*>(a->x);
-  if (a->sel_state != nullptr && a->key_lo != 0) {
+  if (tracked) {
     Pool pool;
     pool.key = a->pool_key; pool.tok = a->pool_tok; pool.col = a->pool_col; pool.val = a->pool_val; pool.cap = a->pool_cap;
     pool.count = a->hist + 2 * kHistBins;
-    launch_chained(zhist_collect_kernel, grid, 256, 0, st, x, a->mean, a->rstd, g, a->col_pitch, a->sel_state, a->hist, pool);
+    ScanGeom gc = g;
+    gc.rows_per_block = collect_rows(a);
+    launch_chained(zhist_collect_kernel, grid_of(gc), 256, 0, st, x, a->mean, a->rstd, gc, a->col_pitch, a->sel_state, a->hist, pool);
     launch_chained(find_bin_kernel, 1, 1024, 0, st, a->hist, a->k_total, a->ctl, ex, 0u, 0, 0, 0, a->sel_state, pool.count, pool.cap, a->status);
     launch_chained(classify_pool_kernel, 592, 256, 0, st, pool, a->ctl, lists_of(a), a->status);
     // fallback, skipped inside the kernels unless the tracked range missed the cut or the pool overflowed
