@@ -8,11 +8,12 @@
 //
 // Two kernels: CTA pairs on transposed tiles (below; from 256 tokens on), and the one here, one CTA per tile, for fewer.
 //
-// Structure of both: one CTA per SM.  Warp 0 feeds a shared-memory ring (here four stages, three with sums per tile) with TMA tile loads (no cluster
+// Structure of both: one CTA per SM.  Warp 0 feeds a shared-memory ring (here four stages) with TMA tile loads (no cluster
 // multicast: every CTA fetches its own tiles), warp 1 issues tcgen05.mma into one of two 256-column TMEM accumulators, eight warps drain the
 // other one with tcgen05.ld, add the bias, convert to 16 bit and hand staging tiles to TMA stores (which two more warps issue in the pairs).
 // Every mbarrier wait is bounded; on a timeout the CTA records STATUS_WAIT_TIMEOUT, drains its copies,
 // frees its TMEM and returns.
+#include <climits>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -27,6 +28,7 @@ constexpr int UMMA_K = 16;
 constexpr uint32_t A_BYTES = BM * BK * 2;
 constexpr uint32_t B_BYTES = BN * BK * 2;
 constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int STAGES = 4;  // as many as fit beside the staging tiles
 constexpr int NUM_THREADS = 320;
 constexpr uint32_t TMEM_COLS = 512;
 }  // namespace gemm
@@ -42,19 +44,14 @@ constexpr uint32_t TMEM_COLS = 512;
 // where the MMAs of a tile take 4096 at K = 512 (and 6144 at K = 768): the epilogue was what bounded every K below about 900.
 constexpr int kEpiCols = 64;
 constexpr int kEpiWarps = 8;
-constexpr int kEpiThreads = 32 * kEpiWarps;
 constexpr int kEpiWarpCols = 128;
 constexpr uint32_t kEpiStageBytes = 32 * kEpiCols * 2;
 
 // `tile`: this warp's staging tile (1024-byte aligned); `chunks` of the two 64-column chunks are inside the matrix; `release` hands the
 // accumulator back.
-// With `colacc` (shared, [2][BN] floats: sums and sums of squares per tile column) the column statistics of the rounded
-// values are read back from the staging tile (each lane owns two adjacent columns) and added up over the tile's
-// four row slabs; `nrows` masks the rows beyond the matrix.
-template <bool STATS, typename Release>
+template <typename Release>
 __device__ __forceinline__ void epilogue_warp(uint32_t taddr, const CUtensorMap* map_c, uint8_t* tile, const t16* bias_s,
-                                              int chunks, int n_base, int m_base, int l, int lane, float* colacc, int bn_full, int nrows,
-                                              Release release) {
+                                              int chunks, int n_base, int m_base, int l, int lane, Release release) {
   uint32_t r[4][32];
 #pragma unroll
   for (int j = 0; j < 4; ++j) tmem_ld_32x32(taddr + j * 32, r[j]);
@@ -83,22 +80,6 @@ __device__ __forceinline__ void epilogue_warp(uint32_t taddr, const CUtensorMap*
       tma_store_3d(map_c, tile, n_base + c * kEpiCols, m_base, l);
       bulk_commit();
     }
-    if constexpr (STATS) {
-      float s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
-      const uint32_t chunk = uint32_t(lane >> 2), inner = uint32_t(lane & 3) * 4u;
-#pragma unroll 8
-      for (int i = 0; i < 32; ++i) {
-        if (i < nrows) {
-          const uint32_t u = *reinterpret_cast<const uint32_t*>(tile + i * 128 + ((chunk ^ uint32_t(i & 7)) << 4) + inner);
-          const float a = t16_lo(u), b = t16_hi(u);
-          s0 += a; q0 = fmaf(a, a, q0);
-          s1 += b; q1 = fmaf(b, b, q1);
-        }
-      }
-      const int col = c * kEpiCols + 2 * lane;
-      atomicAdd(&colacc[col], s0); atomicAdd(&colacc[col + 1], s1);
-      atomicAdd(&colacc[bn_full + col], q0); atomicAdd(&colacc[bn_full + col + 1], q1);
-    }
   }
 }
 
@@ -116,49 +97,28 @@ __device__ __forceinline__ void load_bias(t16* bias_s, const t16* bias, long lon
   __syncwarp();
 }
 
-// Per-tile column statistics -> global partials [L][row blocks of 128][N][2], then cleared for the next tile.
-__device__ __forceinline__ void flush_tile_stats(float* colacc, int bn_full, float* tile_stats, int l, int row_block, int row_blocks,
-                                                 int n_base, int N, int etid) {
-  for (int j = etid; j < bn_full; j += kEpiThreads) {
-    const int n = n_base + j;
-    if (n < N && row_block < row_blocks) {
-      float2* dst = reinterpret_cast<float2*>(tile_stats) + (1LL * l * row_blocks + row_block) * N + n;
-      *dst = make_float2(colacc[j], colacc[bn_full + j]);
-    }
-    colacc[j] = 0.f;
-    colacc[bn_full + j] = 0.f;
-  }
-}
-
-template <int STAGES, bool STATS>
 struct GemmShared {
-  uint64_t full[STAGES];
-  uint64_t empty[STAGES];
+  uint64_t full[gemm::STAGES];
+  uint64_t empty[gemm::STAGES];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   int abort_flag;
-  int epi_ok;
   alignas(16) t16 bias[kEpiWarps][kEpiWarpCols];  // per epilogue warp: no barrier between the warps of a tile
-  float colacc[STATS ? 2 * gemm::BN : 1];
 };
-// ring + epilogue staging + barriers, bias and column sums
-template <int STAGES, bool STATS, uint32_t STAGE_BYTES>
-constexpr size_t kGemmSmem = size_t(STAGES) * STAGE_BYTES + size_t(kEpiWarps) * kEpiStageBytes + sizeof(GemmShared<STAGES, STATS>);
+// ring + epilogue staging + barriers and bias
+constexpr size_t kGemmSmem = size_t(gemm::STAGES) * gemm::STAGE_BYTES + size_t(kEpiWarps) * kEpiStageBytes + sizeof(GemmShared);
 constexpr size_t kMaxDynamicSmem = 227 * 1024;
+static_assert(kGemmSmem <= kMaxDynamicSmem, "shared memory of one CTA");
 
-template <int STAGES, bool STATS>
 __global__ void __launch_bounds__(gemm::NUM_THREADS, 1)
 encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_c, const t16* __restrict__ bias,
-                    int L, int M, int N, int K, long long ldc, long long layer_stride_c, int* __restrict__ status,
-                    float* __restrict__ tile_stats) {
+                    int L, int M, int N, int K, int* __restrict__ status) {
   using namespace gemm;
   extern __shared__ __align__(1024) uint8_t tiles[];  // 128-byte-swizzled tiles need 1024-byte alignment
   uint8_t* epi_stage = tiles + size_t(STAGES) * STAGE_BYTES;  // 4 KB staging tiles, 1024-byte aligned
-  using Shared = GemmShared<STAGES, STATS>;
-  static_assert(kGemmSmem<STAGES, STATS, STAGE_BYTES> <= kMaxDynamicSmem, "shared memory of one CTA");
-  Shared* sh = reinterpret_cast<Shared*>(epi_stage + kEpiWarps * kEpiStageBytes);
+  GemmShared* sh = reinterpret_cast<GemmShared*>(epi_stage + kEpiWarps * kEpiStageBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -179,9 +139,6 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     sh->abort_flag = 0;
     fence_barrier_init();
-  }
-  if constexpr (STATS) {
-    for (int j = threadIdx.x; j < 2 * BN; j += NUM_THREADS) sh->colacc[j] = 0.f;
   }
   if (warp == 1) {
     tmem_alloc(&sh->tmem_base, TMEM_COLS);
@@ -262,10 +219,7 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter+32) belong to this warp
     const int ew = warp - 2;
     const int col0 = (ew >> 2) * kEpiWarpCols;
-    const int etid = ew * 32 + lane;
-    const int row_blocks = (M + 127) / 128;
     uint8_t* stage = epi_stage + ew * kEpiStageBytes;
-    int prev_l = -1, prev_rb = 0, prev_n = 0;
     uint32_t local_tile = 0;
     bool ok = true;
     for (long long t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++local_tile) {
@@ -276,18 +230,7 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const uint32_t tph = (local_tile >> 1) & 1;
       const int n_base = nt * BN + col0;
       load_bias(sh->bias[ew], bias, 1LL * l * N, n_base, N, lane);
-      if constexpr (STATS) {
-        named_barrier_sync(1, kEpiThreads);  // the previous tile's column sums are complete
-        if (prev_l >= 0) flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
-        prev_l = l; prev_rb = mt; prev_n = nt * BN;
-        // One thread performs the bounded wait and publishes the outcome, so the warps always
-        // take the same branch and nobody is left alone at a named barrier.
-        if (etid == 0) sh->epi_ok = mbar_wait(&sh->tmem_full[buf], tph, abort_flag) ? 1 : 0;
-        named_barrier_sync(1, kEpiThreads);
-        ok = sh->epi_ok != 0;
-      } else {
-        ok = mbar_wait_leader(&sh->tmem_full[buf], tph, abort_flag, lane);
-      }
+      ok = mbar_wait_leader(&sh->tmem_full[buf], tph, abort_flag, lane);
       if (!ok) break;
       tc_fence_after();
       const int m_base = (mt) * BM + quarter * 32;
@@ -299,16 +242,9 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (lane == 0) mbar_arrive(&sh->tmem_empty[buf]);
       };
       if (chunks > 0)
-        epilogue_warp<STATS>(taddr, &map_c, stage, sh->bias[ew], chunks, n_base, m_base, l, lane,
-                                   STATS ? sh->colacc + col0 : nullptr, BN, min(32, M - m_base), release);
+        epilogue_warp(taddr, &map_c, stage, sh->bias[ew], chunks, n_base, m_base, l, lane, release);
       else
         release();
-    }
-    if constexpr (STATS) {
-      if (ok && prev_l >= 0) {
-        named_barrier_sync(1, kEpiThreads);
-        flush_tile_stats(sh->colacc, BN, tile_stats, prev_l, prev_rb, row_blocks, prev_n, N, etid);
-      }
     }
   }
 
@@ -735,9 +671,6 @@ static bool make_kmajor_map(CUtensorMap* map, const void* base, int layers, int 
   return r == CUDA_SUCCESS;
 }
 
-// Ring stages: as many as fit beside the staging tiles.
-constexpr int kSingleStages = 4, kSingleStatsStages = 3;
-
 // Rows that colstats_kernel puts into one chunk of its sums (one chunk unless the columns alone leave SMs idle).
 extern "C" int clt_colstats_splits(int L, int B, int F);
 static int rows_per_chunk(int L, int B, int F) {
@@ -813,24 +746,21 @@ static int launch_pair(const CUtensorMap& map_w, const CUtensorMap& map_x, const
   return 0;
 }
 
-template <int STAGES, bool STATS>
-static int launch_single(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const t16* bias, int L, int M, int N, int K,
-                         long long ldc, long long layer_stride_c, int* status, float* tile_stats, int num_sms, cudaStream_t stream) {
-  auto* kernel = encoder_gemm_kernel<STAGES, STATS>;
-  constexpr size_t smem = kGemmSmem<STAGES, STATS, gemm::STAGE_BYTES>;
+static int launch_single(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c, const t16* bias, int L, int M, int N, int K, int* status,
+                         int num_sms, cudaStream_t stream) {
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) return -4;
+    if (cudaFuncSetAttribute(encoder_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGemmSmem)) != cudaSuccess) return -4;
     attr_set = true;
   }
   const long long tiles = 1LL * L * ((M + gemm::BM - 1) / gemm::BM) * ((N + gemm::BN - 1) / gemm::BN);
   const int grid = int(tiles < num_sms ? tiles : num_sms);
-  launch_alone(kernel, grid, gemm::NUM_THREADS, smem, stream, map_a, map_b, map_c, bias, L, M, N, K, ldc, layer_stride_c, status, tile_stats);
+  launch_alone(encoder_gemm_kernel, grid, gemm::NUM_THREADS, kGemmSmem, stream, map_a, map_b, map_c, bias, L, M, N, K, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 static int encoder_gemm(const void* A, const void* B, const void* bias, void* C, int L, int M, int N, int K, long long ldc, long long layer_stride_c,
-                        int* status, float* tile_stats, float* mean, float* rstd, long long* whole, int num_sms, cudaStream_t stream) {
+                        int* status, float* mean, float* rstd, long long* whole, int num_sms, cudaStream_t stream) {
   *whole = 0;
   if (K % 8 != 0 || ldc % 8 != 0 || layer_stride_c % 8 != 0) return -1;  // 16-byte TMA strides / vector stores
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -2;
@@ -840,7 +770,7 @@ static int encoder_gemm(const void* A, const void* B, const void* bias, void* C,
   static const bool force_single = [] { const char* e = getenv("CLT_GEMM_SINGLE_CTA"); return e != nullptr && e[0] == '1'; }();
   if (1LL * L * M * N == 0) return 0;
   const t16* bias_p = static_cast<const t16*>(bias);
-  if (M >= gemm2::BT && !force_single && tile_stats == nullptr) {  // CTA pairs when the problem has full tiles of 256 tokens
+  if (M >= gemm2::BT && !force_single) {  // CTA pairs when the problem has full tiles of 256 tokens
     if (!make_kmajor_map(&map_b, B, L, N, K, K, 1LL * N * K, gemm2::BF)) return -3;
     // output map: [L, M, N] with boxes of 64 features x 64 tokens (one store), clipped at M and N
     if (!make_kmajor_map(&map_c, C, L, M, N, ldc, layer_stride_c, gemm2::kChunk)) return -3;
@@ -852,9 +782,43 @@ static int encoder_gemm(const void* A, const void* B, const void* bias, void* C,
   if (!make_kmajor_map(&map_b, B, L, N, K, K, 1LL * N * K, gemm::BN)) return -3;
   // output map: boxes of 64 columns x 32 rows (one epilogue slab store)
   if (!make_kmajor_map(&map_c, C, L, M, N, ldc, layer_stride_c, 32)) return -3;
-  return tile_stats != nullptr
-             ? launch_single<kSingleStatsStages, true>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, tile_stats, num_sms, stream)
-             : launch_single<kSingleStages, false>(map_a, map_b, map_c, bias_p, L, M, N, K, ldc, layer_stride_c, status, nullptr, num_sms, stream);
+  return launch_single(map_a, map_b, map_c, bias_p, L, M, N, K, status, num_sms, stream);
+}
+
+// Sums and sums of squares of the stored outputs per block of 128 rows: one CTA for a block of 256 columns, 16 rows per thread, eight columns each.
+__global__ void __launch_bounds__(256) block_sums_kernel(const t16* __restrict__ C, float2* __restrict__ sums, int M, int N, long long ldc, long long layer_stride_c) {
+  if (chain_wait()) return;
+  chain_release();
+  const int col_blocks = (N + 255) / 256, row_blocks = (M + 127) / 128;
+  const int cb = int(blockIdx.x % col_blocks), rest = int(blockIdx.x / col_blocks), rb = rest % row_blocks, l = rest / row_blocks;
+  const int c0 = (cb * 32 + int(threadIdx.x)) * 8, r1 = min(M, (rb + 1) * 128);
+  __shared__ float red[8][32][17];
+  float s[8], q[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s[j] = q[j] = 0.f;
+  if (c0 < N) {
+    const t16* base = C + 1LL * l * layer_stride_c + c0;
+#pragma unroll 8
+    for (int r = rb * 128 + int(threadIdx.y); r < r1; r += 8) {
+      const uint4 v = __ldcs(reinterpret_cast<const uint4*>(base + 1LL * r * ldc));
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float a = t16_lo(u[j]), b = t16_hi(u[j]);
+        s[2 * j] += a; q[2 * j] = fmaf(a, a, q[2 * j]);
+        s[2 * j + 1] += b; q[2 * j + 1] = fmaf(b, b, q[2 * j + 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { red[threadIdx.y][threadIdx.x][j] = s[j]; red[threadIdx.y][threadIdx.x][8 + j] = q[j]; }
+  __syncthreads();
+  const int col = int(threadIdx.y) * 32 + int(threadIdx.x), n = cb * 256 + col;
+  if (n >= N) return;
+  float ss = 0.f, qq = 0.f;
+#pragma unroll
+  for (int y = 0; y < 8; ++y) { ss += red[y][col >> 3][col & 7]; qq += red[y][col >> 3][8 + (col & 7)]; }
+  sums[(1LL * l * row_blocks + rb) * N + n] = make_float2(ss, qq);
 }
 
 }  // namespace clt
@@ -864,8 +828,15 @@ static int encoder_gemm(const void* A, const void* B, const void* bias, void* C,
 // squares of the stored (16-bit-rounded) outputs; every element is written, nothing has to be cleared.
 extern "C" int CLT_FN(clt_encoder_gemm)(const void* A, const void* B, const void* bias, void* C, int L, int M, int N, int K,
                                 long long ldc, long long layer_stride_c, int* status, float* tile_stats, int num_sms, cudaStream_t stream) {
+  using namespace clt;
   long long whole;
-  return clt::encoder_gemm(A, B, bias, C, L, M, N, K, ldc, layer_stride_c, status, tile_stats, nullptr, nullptr, &whole, num_sms, stream);
+  const int r = encoder_gemm(A, B, bias, C, L, M, N, K, ldc, layer_stride_c, status, nullptr, nullptr, &whole, num_sms, stream);
+  if (r != 0 || tile_stats == nullptr || 1LL * L * M * N == 0) return r;
+  const long long ctas = 1LL * L * ((M + 127) / 128) * ((N + 255) / 256);
+  if (ctas > INT_MAX) return -1;
+  launch_chained(block_sums_kernel, dim3(unsigned(ctas)), dim3(32, 8), 0, stream, static_cast<const t16*>(C), reinterpret_cast<float2*>(tile_stats), M, N,
+                 ldc, layer_stride_c);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 extern "C" int CLT_FN(clt_colstats_strips)(const void* x, float* mean, float* rstd, int L, int B, int F, long long ld, long long layer_stride,
@@ -877,7 +848,7 @@ extern "C" int CLT_FN(clt_encoder_gemm_stats)(const void* A, const void* B, cons
                                       int* status, float* mean, float* rstd, int* kernels, int num_sms, cudaStream_t stream) {
   long long whole;
   *kernels = 0;
-  const int r = clt::encoder_gemm(A, B, bias, C, L, M, N, K, N, 1LL * M * N, status, nullptr, mean, rstd, &whole, num_sms, stream);
+  const int r = clt::encoder_gemm(A, B, bias, C, L, M, N, K, N, 1LL * M * N, status, mean, rstd, &whole, num_sms, stream);
   if (r != 0 || 1LL * L * M * N == 0) return r;
   const int rs = CLT_FN(clt_colstats_strips)(C, mean, rstd, L, M, N, N, 1LL * M * N, whole, kernels, stream);
   *kernels += 1;

@@ -241,7 +241,6 @@ class FusedBatchTopKEngine:
         self.preact = torch.empty(L, B, Fl, dtype=self.t16, device=dev)
         self.mean = torch.empty(L, Fl, dtype=f32, device=dev)
         self.rstd = torch.empty(L, Fl, dtype=f32, device=dev)
-        self.tile_stats = None  # [L, ceil(B / 128), Fl, 2] fp32: statistics from sums per block of 128 tokens
         # tracked histogram range {key_lo, shift} and the pool filled by the single pass over the pre-activations
         self.sel_state = torch.tensor([self.key_lo, self.shift], dtype=torch.int64, device=dev) if self.key_lo != 0 else None
         k_local = -(-self.k_total // max(1, self.world))
@@ -429,12 +428,7 @@ class FusedBatchTopKEngine:
             self._build_csr()
             self.kernel_launches += 2 + 5  # gemm, threshold selection, csr (5)
             return
-        if self.tile_stats is not None:  # statistics from sums per block of 128 tokens
-            e.encoder_gemm(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.status, self.tile_stats)
-            e.colstats_from_tiles(self.tile_stats, self.mean, self.rstd, self.B)
-            self.kernel_launches += 2
-        else:
-            self.kernel_launches += e.encoder_gemm_stats(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.mean, self.rstd, self.status)
+        self.kernel_launches += e.encoder_gemm_stats(X, m.enc_weight.data, m.enc_bias.data, self.preact, self.mean, self.rstd, self.status)
         if self.fn == "topk" and self.world == 1:
             self.kernel_launches += e.token_topk_select(self.preact, self.mean, self.rstd, self.Fl, self.k_token, self.ctl, self.ent_tok, self.ent_col,
                                                         self.ent_val, self.status, self.Fv)

@@ -97,3 +97,32 @@ def test_encoder_gemm_stats_of_few_strips(ext, L, M, N, K, way):
     assert ((mean.double() - of.mean(1)).abs() <= eps * spread + 2.0 ** -23 * of.mean(1).abs()).all()
     var = of.var(1)
     assert (((1 / rstd.double() - 1e-6).square() - var).abs() <= 4 * eps * spread.square() + 2.0 ** -20 * var + 1e-12).all()
+
+
+# the GEMM by CTA pairs with and without sums against 64 bits, with tiles of all 256 tokens, and the sums per block of 128 rows of both GEMMs
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("L,M,N,K", [(1, 4096, 1024, 768), (2, 300, 520, 136), (2, 1025, 264, 520), (3, 200, 136, 72), (1, 128, 8, 8)])
+def test_encoder_gemm_forms_against_64_bits(ext, dtype, L, M, N, K):
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    x = torch.randn(L, M, K, device=dev, generator=g).to(dtype)
+    w = (torch.randn(L, N, K, device=dev, generator=g) / math.sqrt(K)).to(dtype)
+    b = torch.randn(L, N, device=dev, generator=g).to(dtype)
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    want = torch.einsum("lmk,lnk->lmn", x.double(), w.double()) + b.double()[:, None]
+    size = torch.einsum("lmk,lnk->lmn", x.double().abs(), w.double().abs()) + b.double().abs()[:, None]
+    half_ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    mean, rstd = (torch.full((L, N), float("nan"), device=dev) for _ in range(2))
+    sums = torch.full((L, (M + 127) // 128, N, 2), float("nan"), device=dev)
+    calls = [lambda o: ext.encoder_gemm(x, w, b, o, status, None), lambda o: ext.encoder_gemm_stats(x, w, b, o, mean, rstd, status),
+             lambda o: ext.encoder_gemm(x, w, b, o, status, sums)]
+    for call in calls:
+        out = torch.full((L, M, N), float("nan"), device=dev, dtype=dtype)
+        call(out)
+        torch.cuda.synchronize()
+        assert int(status[0]) == 0
+        # an fp32 sum of K products and the bias, then one rounding to 16 bits (fp16: at least 2^-25 apart)
+        assert ((out.double() - want).abs() <= 1.01 * half_ulp * want.abs() + (K + 2) * 2.0 ** -23 * size + 2.0 ** -25).all()
+    of = torch.nn.functional.pad(out.double(), (0, 0, 0, -M % 128)).view(L, -1, 128, N)
+    for got, terms in ((sums[..., 0], of), (sums[..., 1], of.square())):
+        assert ((got.double() - terms.sum(2)).abs() <= 130 * 2.0 ** -24 * terms.abs().sum(2)).all()  # 128 additions in fp32
