@@ -176,8 +176,14 @@ struct DecAdamParams {
   const float* ctl;            // optional step control block (skip flag, 1 / loss scale, clip coefficient)
   int use_inv_scale;           // the "gradient seed" operand carries the loss scale (decoder: yes; encoder inputs: no)
   float* norm_sq_out;          // norm-only pass: squared norm of all row gradients is added here
+  int* status;                 // for the index checks of the debug build; may be null
   AdamHyper h;
 };
+
+// The debug build reports a token (from the feature-major lists) outside the batch; row 0 with activation 0 is taken in its place.
+__device__ __forceinline__ void check_token(int& tok, float& a, int B, int* status, int site) {
+  if (!clt_in_bounds(tok, B, status, site)) { tok = 0; a = 0.f; }
+}
 
 // Extra gradient of a feature's first row (dense buffer or compact rows through an index), or null.
 __device__ __forceinline__ const float* extra_row_ptr(const DecAdamParams& p, int col) {
@@ -280,6 +286,7 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
       tok4[j] = j < ne ? __ldg(p.fcsr_tok + b + j) : 0;
       a4[j] = j < ne ? __ldg(p.fcsr_val + b + j) : 0.f;
       dacc[j] = 0.f;
+      check_token(tok4[j], a4[j], B, p.status, 203);
     }
     const float pc = p.pen_coef ? p.pen_coef[col] : 0.f;
     float norm2 = 0.f;
@@ -309,9 +316,10 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
       for (int i = b + 4; i < e; ++i) {  // rare: features with more than four entries
         float dot = 0.f;
         if (act) {
-          const float a = __ldg(p.fcsr_val + i);
-          float gv[8];
-          unpack8(__ldg(reinterpret_cast<const uint4*>(gs + (1LL * (ti + r) * B + __ldg(p.fcsr_tok + i)) * d + e0)), gv);
+          int tok = __ldg(p.fcsr_tok + i);
+          float a = __ldg(p.fcsr_val + i), gv[8];
+          check_token(tok, a, B, p.status, 204);
+          unpack8(__ldg(reinterpret_cast<const uint4*>(gs + (1LL * (ti + r) * B + tok) * d + e0)), gv);
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             g[k] = fmaf(a, gv[k], g[k]);
@@ -400,6 +408,7 @@ __global__ void __launch_bounds__(256, 2) rows_norm_kernel(const DecAdamParams p
       const bool in = m.b + j < m.e;
       m.tok[j] = in ? __ldg(p.fcsr_tok + m.b + j) : 0;
       m.a[j] = in ? __ldg(p.fcsr_val + m.b + j) : 0.f;
+      check_token(m.tok[j], m.a[j], p.B, p.status, 205);
     }
   };
   List cur, nxt;
@@ -463,8 +472,10 @@ __global__ void __launch_bounds__(256, 2) rows_norm_kernel(const DecAdamParams p
         }
 #pragma unroll 1
         for (int i = 4; i < ne; ++i) {
-          const float a = __ldg(p.fcsr_val + b + i);
-          const t16* src = gs_t + 1LL * __ldg(p.fcsr_tok + b + i) * d;
+          float a = __ldg(p.fcsr_val + b + i);
+          int tok = __ldg(p.fcsr_tok + b + i);
+          check_token(tok, a, p.B, p.status, 206);
+          const t16* src = gs_t + 1LL * tok * d;
           uint4 v[NV];
           float dot = 0.f;
 #pragma unroll
@@ -911,15 +922,17 @@ __global__ void __launch_bounds__(NARROW ? (EPT == 4 ? 192 : 256) : 288, NARROW 
           int seg = 0;
           for (int s = 0; s < ti; ++s) seg += __shfl_sync(0xFFFFFFFFu, incl, s) <= j ? 1 : 0;
           const int x = __shfl_sync(0xFFFFFFFFu, seg_b, seg) + j - (__shfl_sync(0xFFFFFFFFu, incl, seg) - __shfl_sync(0xFFFFFFFFu, seg_n, seg));
-          const int my_tok = j < total ? __ldg(p.fcsr_tok + x) : 0;
-          const float my_a = j < total ? __ldg(p.fcsr_val + x) : 0.f;
+          int my_tok = j < total ? __ldg(p.fcsr_tok + x) : 0;
+          float my_a = j < total ? __ldg(p.fcsr_val + x) : 0.f;
+          check_token(my_tok, my_a, B, status, 207);
           add_entries<EPT, NB, kPairs>(min(32, total - j0), x, my_tok, my_a, p.gs + 1LL * ti * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
         }
       } else {
         for (int x0 = b + kAdamSlots; x0 < b + ne; x0 += 32) {  // entries beyond the slots
           const int cnt = min(32, b + ne - x0);
-          const int my_tok = lane < cnt ? __ldg(p.fcsr_tok + x0 + lane) : 0;
-          const float my_a = lane < cnt ? __ldg(p.fcsr_val + x0 + lane) : 0.f;
+          int my_tok = lane < cnt ? __ldg(p.fcsr_tok + x0 + lane) : 0;
+          float my_a = lane < cnt ? __ldg(p.fcsr_val + x0 + lane) : 0.f;
+          check_token(my_tok, my_a, B, status, 208);
           add_entries<EPT, NB, kPairs>(cnt, x0 + lane, my_tok, my_a, p.gs + 1LL * (ti + r) * B * d + e0, d, act, lane, w, g, p.grad_a, gsc);
         }
       }
@@ -1358,8 +1371,9 @@ __global__ void __launch_bounds__(256) decoder_rows_adam_kernel(const DecAdamPar
         const int col = s * p.F_pitch + f;
         const int b = __ldg(p.feat_off + col), e = __ldg(p.feat_off + col + 1);
         for (int i = b; i < e; ++i) {
-          const int tok = __ldg(p.fcsr_tok + i);
-          const float a = __ldg(p.fcsr_val + i);
+          int tok = __ldg(p.fcsr_tok + i);
+          float a = __ldg(p.fcsr_val + i);
+          check_token(tok, a, p.B, p.status, 209);
           const int t_begin = t_fixed >= 0 ? t_fixed : s;
           const int t_end = t_fixed >= 0 ? t_fixed : p.L - 1;
           float dot = 0.f;
@@ -1466,6 +1480,7 @@ struct EncAdamParams {
   const float* ctl;             // optional step control block
   float* norm_sq_out;           // norm-only pass
   int norm_only;                // bias kernel: 1 = only add the squared bias gradients to norm_sq_out
+  int* status;                  // see DecAdamParams
   AdamHyper h;                  // grad_scale applies to the sparse part
 };
 __device__ __forceinline__ int enc_extra_index(const EncAdamParams& p, long long row) {
@@ -1506,9 +1521,10 @@ __global__ void __launch_bounds__(256) encoder_rows_adam_kernel(const EncAdamPar
 #pragma unroll
       for (int i = 0; i < 8; ++i) g[i] = 0.f;
       for (int i = b; i < e; ++i) {
-        const float dl = __ldg(p.delta + i);
-        float xv[8];
-        unpack8(__ldg(reinterpret_cast<const uint4*>(p.x + (1LL * l * p.B + __ldg(p.fcsr_tok + i)) * p.d + e0)), xv);
+        int tok = __ldg(p.fcsr_tok + i);
+        float dl = __ldg(p.delta + i), xv[8];
+        check_token(tok, dl, p.B, p.status, 210);
+        unpack8(__ldg(reinterpret_cast<const uint4*>(p.x + (1LL * l * p.B + tok) * p.d + e0)), xv);
 #pragma unroll
         for (int k = 0; k < 8; ++k) g[k] = fmaf(dl, xv[k], g[k]);
       }
@@ -1924,6 +1940,7 @@ extern "C" int CLT_FN(clt_decoder_rows_adam)(const CltDecAdamArgs* a, int num_sm
   p.moments_bf16 = a->moments_bf16;
   p.extra_idx = a->extra_idx; p.extra_rows = a->extra_rows; p.ctl = a->ctl; p.use_inv_scale = 1;
   p.norm_sq_out = a->ctl != nullptr ? a->ctl + SC_GRAD_NORM_SQ : nullptr;
+  p.status = a->status;
   if (a->moments_bf16 && !(a->tying == 0 && a->status != nullptr && a->weights_bf16)) return -6;  // only the bulk pipeline handles bf16 moments
   if (acc == 0) return 0;
   bool single_rows = true;
@@ -1990,6 +2007,7 @@ extern "C" int CLT_FN(clt_encoder_rows_adam)(const CltEncAdamArgs* a, int num_sm
   p.dense_grad = a->dense_grad; p.dense_bias_grad = a->dense_bias_grad; p.h = to_hyper(a->h);
   p.extra_idx = a->extra_idx; p.extra_rows = a->extra_rows; p.extra_bias = a->extra_bias; p.ctl = a->ctl;
   p.norm_sq_out = a->ctl != nullptr ? a->ctl + SC_GRAD_NORM_SQ : nullptr; p.norm_only = a->norm_only;
+  p.status = a->status;
   const int grid = num_sms * 8, bgrid = int((1LL * a->L * a->F_pitch + 255) / 256);
   // the encoder as the one-row-per-feature case of the decoder's kernels: layer l is "tensor" l with R = 1, the layer inputs play the gradient
   // seed and delta the activation
@@ -2014,6 +2032,7 @@ extern "C" int CLT_FN(clt_encoder_rows_adam)(const CltEncAdamArgs* a, int num_sm
   q.moments_bf16 = a->moments_bf16;
   q.extra_idx = a->dense_grad == nullptr ? a->extra_idx : nullptr; q.extra_rows = a->extra_rows;
   q.ctl = a->ctl; q.use_inv_scale = 0; q.norm_sq_out = p.norm_sq_out;
+  q.status = a->status;
   if (a->norm_only) {
     if (a->ctl == nullptr) return -1;
     if (a->L <= kMaxLayersA && (a->dense_grad == nullptr || a->extra_idx == nullptr) && 1LL * a->L * a->F_pitch < INT_MAX) {

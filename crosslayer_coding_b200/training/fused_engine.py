@@ -913,12 +913,12 @@ class FusedBatchTopKEngine:
             # without entries have none), dL/da is written on the way; step_control turns the norm into the coefficient
             rep = 1.0 / self.world  # replicated parameters are counted once over the ranks
             e.decoder_rows_adam(dec_w, self.dec_m, self.dec_v, L, B, d, self.Fl, tying_dec, self.feat_off, self.fcsr_tok, self.fcsr_val,
-                                gs_dec, self.grad_a, pen, None, self.foff32, self.fsc32, dec0_dense, h_dec, None, dec_x_idx, dec_x_rows, ctl, True,
+                                gs_dec, self.grad_a, pen, None, self.foff32, self.fsc32, dec0_dense, h_dec, self.status, dec_x_idx, dec_x_rows, ctl, True,
                                 self.d_foff, self.d_fsc)
             self._affine_adam(h_enc, ctl, norm_weight=1.0)
             e.decoder_bias_adam(m.dec_bias.data, self.decb_m, self.decb_v, self.bias_sel, self.gs_sum, extra_bias_grad, h_dec, ctl, rep)
             e.encoder_rows_adam(m.enc_weight.data, self.enc_m, self.enc_v, m.enc_bias.data, self.encb_m, self.encb_v, self.feat_off,
-                                self.fcsr_tok, self.grad_a, X, enc_dense, encb_dense, h_enc, None, enc_x_idx, enc_x_rows, enc_x_bias, ctl, True)
+                                self.fcsr_tok, self.grad_a, X, enc_dense, encb_dense, h_enc, self.status, enc_x_idx, enc_x_rows, enc_x_bias, ctl, True)
             if skip_grad is not None:
                 e.dense_adam(m.skip_weight.data, self.skip_m, self.skip_v, skip_grad, h_dec, ctl, True, rep)
             if jr:
