@@ -374,8 +374,8 @@ __global__ void __launch_bounds__(256, 2) decoder_rows_adam_untied_kernel(const 
 // A gather of every entry's seed row for every target, which L2 could deliver three times as fast as the one-segment form read it: instructions bound
 // that one (a warp per 256 elements of a feature's rows: divisions, list and reductions for each).  Here a warp takes up to 1024 elements of the rows
 // (NV vectors of eight per lane), kEntries entries at a time, with the list of the next feature and the offsets of the one after it on the way.
-// us before and now, decoder + encoder: 12 x 768, 24576 features, 4096 tokens, k = 200 3243 + 321 / 1750 + 195; 3072 features, k = 25 498 + 48 / 281 + 32;
-// 5 x 520, 2056 features, 776 tokens 62 + 15 / 41 + 11; 12 x 352 tied 114 + 50 / 74 + 37; 6 x 136 145 + 37 / 120 + 35; 4 x 2048 102 + 36 / 82 + 24.
+// us before and now, decoder + encoder: 12 x 768, 24576 features, 4096 tokens, k = 200 3243 + 321 / 1638 + 196; 3072 features, k = 25 498 + 48 / 262 + 33;
+// 5 x 520, 2056 features, 776 tokens 62 + 15 / 41 + 11; 12 x 352 tied 114 + 50 / 68 + 37; 6 x 136 145 + 37 / 118 + 35; 4 x 2048 102 + 36 / 76 + 26.
 template <typename WT, bool DOTS, int NV>
 __global__ void __launch_bounds__(256, 2) rows_norm_kernel(const DecAdamParams p) {
   constexpr int kEntries = NV <= 2 ? 4 : 2;
@@ -503,13 +503,13 @@ __global__ void __launch_bounds__(256, 2) rows_norm_kernel(const DecAdamParams p
         for (int n = 0; n < NV; ++n) {
           if (e0 + 256 * n < end) {
             float w[8], dg0[8];
-            if (DOTS && pc != 0.f) wv[n].get(w);
+            if (DOTS) wv[n].get(w);
             const bool extra = r == 0 && xrow != nullptr;
             if (extra) load8f(xrow + e0 + 256 * n, dg0);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               float gk = g[n][k] * gsc;
-              if (DOTS && pc != 0.f) gk = fmaf(pc, w[k], gk);
+              if (DOTS) gk = fmaf(pc, w[k], gk);  // without a penalty too, as in the update: a weight that is not finite shows in the norm
               if (extra) gk += dg0[k];
               nsq = fmaf(gk, gk, nsq);
             }

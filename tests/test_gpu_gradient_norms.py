@@ -84,3 +84,33 @@ def test_decoder_and_encoder_norms(ext, dtype, extra, L, F, B, d):
     gb = torch.zeros(L * F, device=dev, dtype=torch.float64).index_add_(0, owner, val.double()) * 0.7
     norm = float(grad.square().sum() + gb.square().sum())
     assert abs(float(ctl[SC_GRAD_NORM_SQ]) - norm) <= (2 * 64 + 2048) * eps * norm
+
+
+# weights that are not finite make the norm so, without a sparsity penalty too (the update forms 0 x w as well), wherever the row is touched at all: the step
+# is then skipped
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d", [8, 264, 1032])
+@pytest.mark.parametrize("touched", ["extra row", "entry", "none"])
+def test_decoder_norm_of_weights_that_are_not_finite(ext, dtype, d, touched):
+    dev = torch.device("cuda:0")
+    L, F, B = 2, 16, 20
+    g = torch.Generator(device=dev).manual_seed(d)
+    w = [torch.randn(F, L - s, d, device=dev, generator=g).to(dtype) for s in range(L)]
+    w[1][5, 0, d - 1] = float("inf")
+    n = torch.ones(L * F, dtype=torch.int64)
+    n[F + 5] = 1 if touched == "entry" else 0
+    off = torch.zeros(L * F + 1, dtype=torch.int32, device=dev)
+    off[1:] = n.cumsum(0).int().to(dev)
+    total = int(off[-1])
+    tok, val = torch.zeros(total, dtype=torch.int32, device=dev), torch.ones(total, device=dev)
+    gs = torch.randn(L, B, d, device=dev, generator=g).bfloat16()
+    idx = torch.full((L * F,), -1, dtype=torch.int32, device=dev)
+    if touched == "extra row":
+        idx[F + 5] = 0
+    ctl = torch.zeros(16, device=dev)
+    ctl[SC_INV_SCALE] = ctl[SC_CLIP] = 1.0
+    zero = [torch.zeros(F, L - s, d, device=dev) for s in range(L)]
+    ext.decoder_rows_adam(w, zero, zero, L, B, d, F, 0, off, tok, val, gs, torch.zeros(total, device=dev), None, None, None, None, None, HYPER,
+                          torch.zeros(4, dtype=torch.int32, device=dev), idx, torch.ones(1, d, device=dev), ctl, True)
+    assert bool(torch.isnan(ctl[SC_GRAD_NORM_SQ])) == (touched != "none")
+    assert touched != "none" or float(ctl[SC_GRAD_NORM_SQ]) > 0
