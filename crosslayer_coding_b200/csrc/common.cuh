@@ -80,6 +80,17 @@ __device__ __forceinline__ bool chain_wait() {
 // CTAs would hold the threads of all SMs until that rank arrives, and kernels of other streams (staging of the next batch) could not start.  There
 // the next kernel comes when this one has ended.
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// SMs of the current device, asked once per device.
+inline int device_sms() {
+  constexpr int kDevices = 64;
+  static int sms[kDevices] = {};
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;  // a whole B200; the launch will say what is wrong
+  if (dev < kDevices && sms[dev] > 0) return sms[dev];
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+  if (dev < kDevices) sms[dev] = n;
+  return n;
+}
 template <typename... Params, typename... Args>
 inline cudaError_t launch_kernel(bool chained, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchAttribute attr = {};
@@ -97,10 +108,10 @@ inline cudaError_t launch_kernel(bool chained, void (*kernel)(Params...), dim3 g
 // Up to eight CTAs per SM.  CTAs that come early take an SM as the kernel before has divided it between L1 and shared memory, and as long as one of them is
 // there it stays so: larger grids, and the persistent kernels below, would run with fewer CTAs per SM for all of their time (a step with
 // long row updates took 1.2 times as long), where the gap in front of them does not count.
-constexpr unsigned long long kChainedCtas = 8 * 148;
+constexpr unsigned long long kChainedCtasPerSm = 8;
 template <typename... Params, typename... Args>
 inline cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
-  return launch_kernel(1ULL * grid.x * grid.y * grid.z <= kChainedCtas, kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
+  return launch_kernel(1ULL * grid.x * grid.y * grid.z <= kChainedCtasPerSm * device_sms(), kernel, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 // Kernels whose CTAs stay (GEMMs, row updates): neither early themselves, nor with early CTAs of the next one beside them (which cost the row updates of a
 // GPT-2-shape step 2.5 %), so without chain_wait().

@@ -163,7 +163,7 @@ __device__ __forceinline__ float decode_epilogue(const DecodeParams& p, int tok,
 // below the line 4096 of 6 x 512, 48 entries on average but few in most lists, 99 / 130).
 constexpr long long kRunningMinWarps = 1024;   // tokens x chunks; below, the (token, target) split has L times as many CTAs
 constexpr long long kEightWarpsBelow = 2048;   // CTAs
-constexpr long long kSlicesUpTo = 592;         // CTAs of 256 columns: 148 SMs x 4
+constexpr long long kSliceCtasPerSm = 4;       // CTAs of 256 columns
 constexpr long long kManyCtas = 28672;         // CTAs
 constexpr long long kPairNarrowFrom = 24576;   // (token, target) pairs
 constexpr int kRunningOrderFrom = 4096;        // tokens
@@ -617,7 +617,7 @@ static int walk_vectors(const CltDecodeArgs* a) { return (a->d / 8 + 32 * walk_c
 static bool short_lists(const CltDecodeArgs* a) { return a->expected > 0 && a->expected < kShortBelow; }
 static int slices(const CltDecodeArgs* a) { return (a->d + 255) / 256; }
 static bool takes_slices(const CltDecodeArgs* a) {
-  return a->d > 512 && a->d <= 1024 && !short_lists(a) && 1LL * a->B * a->L * slices(a) <= kSlicesUpTo;
+  return a->d > 512 && a->d <= 1024 && !short_lists(a) && 1LL * a->B * a->L * slices(a) <= kSliceCtasPerSm * device_sms();
 }
 // Lists of one length that a warp takes alone.
 static bool one_warp_lists(const CltDecodeArgs* a) {

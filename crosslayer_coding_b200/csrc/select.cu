@@ -2191,7 +2191,7 @@ static int collect_rows(const CltSelectArgs* a) {
   const int pieces = (a->F + 7) / 8;
   const double per_row = (1.0 - std::pow(1.0 - std::min(q, 1.0), 8.0)) * std::min(pieces, 256);
   int rows = 64;
-  if (densely_kept(a) && 1LL * ((pieces + 255) / 256) * ((a->B + 63) / 64) * a->L < 8 * 148) rows = rows_halved(a, rows);
+  if (densely_kept(a) && 1LL * ((pieces + 255) / 256) * ((a->B + 63) / 64) * a->L < 8LL * device_sms()) rows = rows_halved(a, rows);
   while (rows * per_row > 0.35 * kCollectQueue && rows_halved(a, rows) < rows) rows = rows_halved(a, rows);
   return rows;
 }

@@ -77,3 +77,11 @@ def test_the_kernels_that_poll_are_known():
     # the wait alone does not release anything
     wait = (CSRC / "common.cuh").read_text().split("bool chain_wait()")[1].split("\n}")[0]
     assert "griddepcontrol.wait" in wait and "launch_dependents" not in wait
+
+
+def test_rules_on_resident_ctas_ask_the_device():
+    """What is launched early, and which decodes are taken in slices, depends on the SMs of the device at hand, not on those of one product."""
+    common, decode = ((CSRC / n).read_text() for n in ("common.cuh", "decode.cu"))
+    assert "kChainedCtasPerSm * device_sms()" in common and "kSliceCtasPerSm * device_sms()" in decode
+    rules = common.split("inline cudaError_t launch_chained")[1].split("\n}")[0] + decode.split("static bool takes_slices")[1].split("\n}")[0]
+    assert not re.search(r"\b(148|592|1184)\b", rules)
