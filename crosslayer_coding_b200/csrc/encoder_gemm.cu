@@ -6,7 +6,7 @@
 // Counterpart of the reference's per-layer F.linear calls (clt/models/parallel.py:286 through
 // clt/models/encoder.py:101).
 //
-// Two kernels: CTA pairs on transposed tiles (below; from 256 tokens on), and the one here, one CTA per tile, for fewer.
+// Two kernels: CTA pairs on transposed tiles (below; from 256 tokens on), and the one here, one CTA per tile, for fewer tokens or few tiles.
 //
 // Structure of both: one CTA per SM.  Warp 0 feeds a shared-memory ring (here four stages) with TMA tile loads (no cluster
 // multicast: every CTA fetches its own tiles), warp 1 issues tcgen05.mma into one of two 256-column TMEM accumulators, eight warps drain the
@@ -770,7 +770,11 @@ static int encoder_gemm(const void* A, const void* B, const void* bias, void* C,
   static const bool force_single = [] { const char* e = getenv("CLT_GEMM_SINGLE_CTA"); return e != nullptr && e[0] == '1'; }();
   if (1LL * L * M * N == 0) return 0;
   const t16* bias_p = static_cast<const t16*>(bias);
-  if (M >= gemm2::BT && !force_single) {  // CTA pairs when the problem has full tiles of 256 tokens
+  // CTA pairs when the problem has full tiles of 256 tokens, and without statistics more tiles than one round of the single CTAs, which start
+  // and end sooner (us in pairs / alone: 1 x 256 x 2048, K = 64 8.3 / 6.5; 1 x 256 x 8192, K = 256 10.3 / 8.3; 9 x 256 x 2048, K = 1024 14.4 / 12.4, K = 2048
+  // 20.6 / 20.6); with two to three rounds they are level up to K = 512 and pairs ahead beyond it (9 x 600 x 2048, K = 2048 45 / 53).
+  const long long singles = 1LL * L * ((M + gemm::BM - 1) / gemm::BM) * ((N + gemm::BN - 1) / gemm::BN);
+  if (M >= gemm2::BT && !force_single && (mean != nullptr || singles > num_sms)) {
     if (!make_kmajor_map(&map_b, B, L, N, K, K, 1LL * N * K, gemm2::BF)) return -3;
     // output map: [L, M, N] with boxes of 64 features x 64 tokens (one store), clipped at M and N
     if (!make_kmajor_map(&map_c, C, L, M, N, ldc, layer_stride_c, gemm2::kChunk)) return -3;

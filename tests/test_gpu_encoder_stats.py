@@ -126,3 +126,24 @@ def test_encoder_gemm_forms_against_64_bits(ext, dtype, L, M, N, K):
     of = torch.nn.functional.pad(out.double(), (0, 0, 0, -M % 128)).view(L, -1, 128, N)
     for got, terms in ((sums[..., 0], of), (sums[..., 1], of.square())):
         assert ((got.double() - terms.sum(2)).abs() <= 130 * 2.0 ** -24 * terms.abs().sum(2)).all()  # 128 additions in fp32
+
+
+# pairs without sums take more tiles than there are CTAs: many layers of few tiles, whose last one ends in its first or second half of features, in a store of 64, in the
+# first or second half of tokens, in a chunk of 64; the same matrices with few layers go one CTA per tile
+@pytest.mark.parametrize("L", [80, 3])
+@pytest.mark.parametrize("M,N", [(256, 8), (257, 136), (300, 200), (520, 328), (400, 72)])
+@pytest.mark.parametrize("K", [8, 72, 520])
+def test_encoder_gemm_of_many_small_layers(ext, L, M, N, K):
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(M + N + K)
+    x = torch.randn(L, M, K, device=dev, generator=g).bfloat16()
+    w = (torch.randn(L, N, K, device=dev, generator=g) / math.sqrt(K)).bfloat16()
+    b = torch.randn(L, N, device=dev, generator=g).bfloat16()
+    status = torch.zeros(4, dtype=torch.int32, device=dev)
+    out = torch.full((L, M, N), float("nan"), device=dev, dtype=torch.bfloat16)
+    ext.encoder_gemm(x, w, b, out, status, None)
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    want = torch.einsum("lmk,lnk->lmn", x.double(), w.double()) + b.double()[:, None]
+    size = torch.einsum("lmk,lnk->lmn", x.double().abs(), w.double().abs()) + b.double().abs()[:, None]
+    assert ((out.double() - want).abs() <= 1.01 * 2.0 ** -8 * want.abs() + (K + 2) * 2.0 ** -23 * size).all()  # fp32 sums, one rounding to bf16

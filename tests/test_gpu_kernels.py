@@ -52,7 +52,7 @@ def test_encoder_gemm_matches_fp32(ext, L, M, N, K):
 
 
 # without the column sums: rows and columns that end in the first or the second half of a tile, in a 64-column store, in a 32-row slab;
-# one CTA per tile (up to 255 rows) and pairs; more tiles than CTAs
+# one CTA per tile (up to 255 rows, or few tiles) and pairs (more tiles than CTAs)
 @pytest.mark.parametrize("M", [1, 33, 200, 256, 300, 520])
 @pytest.mark.parametrize("L,N,K", [(1, 8, 8), (2, 136, 72), (1, 200, 64), (1, 256, 520), (2, 328, 136), (3, 20488, 64)])
 @pytest.mark.parametrize("with_bias", [True, False])
