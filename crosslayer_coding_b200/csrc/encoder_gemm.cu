@@ -276,7 +276,8 @@ encoder_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // and tcgen05.ld.16x256b, whose thread holds tokens 2q and 2q + 1 of every eight for two features, each of the eight sums per feature that
 // colstats_kernel keeps (rows r = y mod 8, in order) lies in one register of one thread.  A pair takes the token tiles of a strip of 256
 // features one after the other and carries the sums along: no shuffle, no shared memory and no partial sums per tile, and the same
-// additions in the same order as in the separate pass, so that the statistics are the same bit for bit.  (Sums per tile, in another
+// additions in the same order as in the separate pass, so that the statistics are the same bit for bit (where that pass takes the rows in at most two
+// chunks; the sums of more chunks it adds by atomics, in no fixed order).  (Sums per tile, in another
 // order, were tried before: +0.15 ms at K = 768, and a last bit that moves single entries across the cut of the selection.)
 // Strips that do not fill a round of all pairs are taken tile by tile, and their statistics by colstats_kernel.
 namespace gemm2 {
@@ -846,7 +847,8 @@ extern "C" int CLT_FN(clt_encoder_gemm)(const void* A, const void* B, const void
 extern "C" int CLT_FN(clt_colstats_strips)(const void* x, float* mean, float* rstd, int L, int B, int F, long long ld, long long layer_stride,
                                            long long first_strip, int* kernels, cudaStream_t st);
 
-// The GEMM and the batch statistics mean / rstd [L, N] of its stored outputs (C contiguous), equal bit for bit to clt_colstats on C.
+// The GEMM and the batch statistics mean / rstd [L, N] of its stored outputs (C contiguous), equal bit for bit to clt_colstats on C where
+// that takes the rows in at most two chunks.
 // *kernels: how many kernels were launched.
 extern "C" int CLT_FN(clt_encoder_gemm_stats)(const void* A, const void* B, const void* bias, void* C, int L, int M, int N, int K,
                                       int* status, float* mean, float* rstd, int* kernels, int num_sms, cudaStream_t stream) {

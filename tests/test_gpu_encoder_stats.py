@@ -1,4 +1,5 @@
-"""Encoder GEMM with the batch statistics in its epilogue: the outputs of the GEMM without them, the statistics of the separate pass bit for bit."""
+"""Encoder GEMM with the batch statistics in its epilogue: the outputs of the GEMM without them, the statistics of the separate pass, bit
+for bit where its additions have a fixed order (rows in at most two chunks)."""
 import math
 
 import pytest
