@@ -1092,7 +1092,7 @@ narrow_rows_adam_kernel(const DecAdamParams p, long long total_rows, float ctas_
   const float gsc = hr.gscale * (p.use_inv_scale ? sc.inv_scale : 1.f);
   const uint64_t pol_stream = l2_policy_evict_first();  // rows are touched once per step
 
-  const long long stride = 1LL * grid * kNarrowWarps;
+  const int stride = grid * kNarrowWarps;
   const auto place = [&](RowAt& at) {  // tensor, feature and row of at.idx (at.ti: at or before the right one)
     if (at.idx >= total_rows) return;
     while (at.idx >= p.row_start[at.ti + 1]) ++at.ti;
@@ -1297,7 +1297,7 @@ narrow_rows_adam_kernel(const DecAdamParams p, long long total_rows, float ctas_
     bulk_wait_all();
     if (!ok) {
       // rows whose loads were issued but never consumed: give them a bounded chance to land
-      for (uint32_t j = i; j < i + kNarrowStages && cur.idx + (j - i) * stride < total_rows; ++j) {
+      for (uint32_t j = i; j < i + kNarrowStages && cur.idx + 1LL * (j - i) * stride < total_rows; ++j) {
         const long long start = clock64();
         while (!mbar_try_wait(&full[j % kNarrowStages], (j / kNarrowStages) & 1))
           if (clock64() - start > kWaitTimeoutCycles) break;
