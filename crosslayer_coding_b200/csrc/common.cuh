@@ -76,9 +76,9 @@ __device__ __forceinline__ bool chain_wait() {
   asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%nsmid;" : "=r"(sms) :: "memory");
   return sms == 0xFFFFFFFFu;
 }
-// Lets the next kernel's CTAs take their places; second statement of a chained kernel.  Not in one that waits for another rank: up to 1184
-// CTAs would hold the threads of all SMs until that rank arrives, and kernels of other streams (staging of the next batch) could not start.  There
-// the next kernel comes when this one has ended.
+// Lets the next kernel's CTAs take their places; second statement of a chained kernel.  Not in one that waits for another rank: up to eight
+// CTAs per SM would hold the threads of all SMs until that rank arrives, and kernels of other streams (staging of the next batch) could not start.
+// There the next kernel comes when this one has ended.
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // SMs of the current device, asked once per device.
 inline int device_sms() {
